@@ -6,23 +6,26 @@
 // (expert, 128-token tile) reading the bool map column-wise, and writes the [T,P]
 // outputs twice (zero-fill, then scatter): csrc/kernels/reroute.cu:21-51, 138-264 and
 // csrc/ultra_ep.cpp:891-892 of the reference. Here:
-//   * pass 1 counts keys per (tile, expert) from coalesced row reads;
-//   * pass 2 turns the counts of the preceding tiles into a base per expert, resolves
-//     ordinals inside the tile in row-major order (sparse: per-warp sub-counts, then match.any
-//     inside the warp; dense: the map tile is staged in shared memory, one thread per expert
-//     walks its column only to count, and the replica arithmetic runs over the marked cells
-//     spread over the CTA), and writes every output element exactly once with coalesced
-//     vector stores (zeros included), so no pre-zeroing pass exists.
+//   * sparse: one launch (ordinals.cuh); a cluster of CTAs keeps its entries in registers and
+//     counts again what lies in front of it;
+//   * dense: pass 1 counts per (tile, expert) from coalesced row reads; pass 2 turns the counts of
+//     the preceding tiles into a base per expert, resolves ordinals inside the tile in row-major
+//     order (the map tile is staged in shared memory, one thread per expert walks its column only
+//     to count, and the replica arithmetic runs over the marked cells spread over the CTA), and
+//     writes every output element exactly once with coalesced vector stores (zeros included), so no
+//     pre-zeroing pass exists.
 // Results equal the reference's dense rule bit for bit; the sparse form applies the same
 // rule per (token, k) entry and therefore is deterministic, which the reference's
 // atomic-counter sparse kernel (reroute.cu:492-515) is not.
 
+#include <climits>
 #include <cstdlib>
 #include <mutex>
 #include <string>
 #include <utility>
 
 #include "internal.h"
+#include "ordinals.cuh"
 
 namespace uep {
 
@@ -30,15 +33,15 @@ namespace {
 
 constexpr int kRerouteThreads = 256;
 constexpr int kDenseTileRows = 64;
-constexpr int kSparseTileEntries = 2048;  // 8 warps x 256 entries
+constexpr int kSparseTileEntries = 2048;  // entries of a row of the count table (at least)
 
-__device__ __forceinline__ int gcd_int(int a, int b) {
-    while (b != 0) {
-        const int t = a % b;
-        a = b;
-        b = t;
-    }
-    return a;
+// The interleave's stride for a total of two or more: the first number from total/2 + 1 upwards that has no factor in
+// common with the total (csrc/kernels/reroute.cu:21-51 of the reference searches for it). With h = total/2,
+// gcd(h + 1, 2h + 1) = 1 and gcd(h + 1, 2h) = gcd(h + 1, 2): only an odd h of an even total needs the next number, and
+// gcd(h + 2, 2h) = gcd(h + 2, 4) = 1 then. A total of two leaves 1.
+__device__ __forceinline__ int interleave_stride(int total) {
+    const int h = total / 2;
+    return total == 2 ? 1 : h + 1 + (((total & 1) == 0 && (h & 1)) ? 1 : 0);
 }
 
 // Per-expert routing parameters (csrc/kernels/reroute.cu:182-209 of the reference).
@@ -98,25 +101,11 @@ __device__ __forceinline__ void stage_expert(int e, const int32_t* __restrict__ 
     r.stride = 0;  // marks "no interleave"
     r.offset = 0;
     if (quota_mode && interleave && r.total > 1) {
-        int st = r.total / 2 + 1;
-        if (st >= r.total) st = r.total - 1;
-        if (st < 1) st = 1;
-        while (gcd_int(st, r.total) != 1) {
-            ++st;
-            if (st >= r.total) st = 1;
-        }
-        r.stride = st;
+        r.stride = interleave_stride(r.total);
         r.offset = e % r.total;
     }
     routers[e] = r;
 }
-
-// Programmatic dependent launch: the second kernel of a pair is launched with the stream-serialisation
-// attribute, so its prologue (everything that does not read the first kernel's output) overlaps the first
-// kernel. `pdl_wait` returns once the first kernel has completed and its writes are visible; without the
-// launch attribute both instructions do nothing.
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ----------------------------------------------------------------------------- dense
 // Copies rows [r0, r1) of the bool map into shared memory, 16 bytes per thread when the tile starts on a
@@ -485,235 +474,222 @@ __global__ void __launch_bounds__(kRerouteThreads) dense_backward_kernel(Batch<D
 }
 
 // ---------------------------------------------------------------------------- sparse
-// bucket of a key: itself when in [0,nb_valid), else the last bucket (if there is one) or none
 template <typename IdT>
-__device__ __forceinline__ int key_bucket(IdT key, int nb_valid, bool tail_bucket) {
-    if (key >= 0 && key < nb_valid) return static_cast<int>(key);
-    return tail_bucket ? nb_valid : -1;
-}
-
-template <typename IdT>
-__global__ void __launch_bounds__(kRerouteThreads) key_count_kernel(const IdT* __restrict__ keys, int64_t n,
-                                                                    int nb_valid, int tail_bucket,
-                                                                    int32_t* __restrict__ tile_counts) {
-    pdl_launch_dependents();
-    extern __shared__ __align__(128) char smem_raw[];
-    int32_t* hist = reinterpret_cast<int32_t*>(smem_raw);
-    const int nb = nb_valid + (tail_bucket ? 1 : 0);
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) hist[i] = 0;
-    __syncthreads();
-    const int64_t begin = static_cast<int64_t>(blockIdx.x) * kSparseTileEntries;
-    const int64_t end = min(begin + kSparseTileEntries, n);
-    for (int64_t i = begin + threadIdx.x; i < end; i += blockDim.x) {
-        const int b = key_bucket<IdT>(keys[i], nb_valid, tail_bucket != 0);
-        if (b >= 0) atomicAdd(hist + b, 1);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) tile_counts[static_cast<int64_t>(blockIdx.x) * nb + i] = hist[i];
-}
-
-// Row-major ordinal of every entry of this CTA's tile inside its bucket, in two steps so that the first
-// one (which reads only the keys) can run before the count kernel has finished:
-//   tile_warp_counts: warp_base[w][b] = entries of bucket b in warp w's part of the tile;
-//   tile_resolve:     with base[b] = entries of bucket b in front of this tile, turns the counts into
-//                     running offsets and hands every entry to emit(i, bucket, ordinal).
-// warp_base holds (blockDim/32) * nb ints.
-template <typename IdT>
-__device__ void tile_warp_counts(const IdT* keys, int64_t n, int nb_valid, bool tail_bucket, int32_t* warp_base) {
-    const int nb = nb_valid + (tail_bucket ? 1 : 0);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    const int per_warp = kSparseTileEntries / nwarps;
-    const int64_t tile_begin = static_cast<int64_t>(blockIdx.x) * kSparseTileEntries;
-    const int64_t wbegin = min(tile_begin + static_cast<int64_t>(warp) * per_warp, n);
-    const int64_t wend = min(wbegin + per_warp, n);
-    for (int i = threadIdx.x; i < nwarps * nb; i += blockDim.x) warp_base[i] = 0;
-    __syncthreads();
-    for (int64_t i = wbegin + lane; i < wend; i += kWarp) {
-        const int b = key_bucket<IdT>(keys[i], nb_valid, tail_bucket);
-        if (b >= 0) atomicAdd(warp_base + warp * nb + b, 1);
-    }
-    __syncthreads();
-}
-
-template <typename IdT, typename Emit>
-__device__ void tile_resolve(const IdT* keys, int64_t n, int nb_valid, bool tail_bucket, const int32_t* base,
-                             int32_t* warp_base, Emit emit) {
-    const int nb = nb_valid + (tail_bucket ? 1 : 0);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    const int per_warp = kSparseTileEntries / nwarps;
-    const int64_t tile_begin = static_cast<int64_t>(blockIdx.x) * kSparseTileEntries;
-    const int64_t wbegin = min(tile_begin + static_cast<int64_t>(warp) * per_warp, n);
-    const int64_t wend = min(wbegin + per_warp, n);
-    // exclusive scan over warps, seeded with the tile base
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-        int run = base[b];
-        for (int w = 0; w < nwarps; ++w) {
-            const int c = warp_base[w * nb + b];
-            warp_base[w * nb + b] = run;
-            run += c;
-        }
-    }
-    __syncthreads();
-    // in-order resolution inside the warp
-    int32_t* mine = warp_base + warp * nb;
-    for (int64_t i0 = wbegin; i0 < wend; i0 += kWarp) {
-        const int64_t i = i0 + lane;
-        const bool in = i < wend;
-        const int b = in ? key_bucket<IdT>(keys[i], nb_valid, tail_bucket) : -1;
-        const unsigned active = __ballot_sync(kFullMask, b >= 0);
-        int ordinal = -1;
-        if (b >= 0) {
-            const unsigned peers = __match_any_sync(active, b);
-            const int before = __popc(peers & ((1u << lane) - 1u));
-            ordinal = mine[b] + before;
-            __syncwarp(active);
-            if (before == 0) mine[b] += __popc(peers);
-        }
-        __syncwarp();
-        if (in) emit(i, b, ordinal);
-    }
-}
-
-template <typename IdT>
-__global__ void __launch_bounds__(kRerouteThreads) sparse_count_kernel(Batch<SparseArgs> batch, int K, int L) {
-    pdl_launch_dependents();  // the reroute kernel may start its prologue now
-    extern __shared__ __align__(128) char smem_raw[];
+__global__ void __launch_bounds__(kOrdThreads) sparse_count_kernel(Batch<SparseArgs> batch, int K, int L, int tile_entries) {
+    pdl_launch_dependents();  // the reroute kernel may start on everything that does not read the table
     const SparseArgs& a = batch.a[blockIdx.y];
-    const IdT* keys = static_cast<const IdT*>(a.ids);
-    const int64_t n = static_cast<int64_t>(a.T) * K;
-    const int64_t begin = static_cast<int64_t>(blockIdx.x) * kSparseTileEntries;
-    // (a tile behind this rank's entries: the second pass launches the same grid and returns at the same test, so
-    // every count it reads has been written by this pass, whatever the scratch buffer held before)
-    if (begin >= n) return;
-    int32_t* hist = reinterpret_cast<int32_t*>(smem_raw);
-    for (int i = threadIdx.x; i < L; i += blockDim.x) hist[i] = 0;
-    __syncthreads();
-    const int64_t end = min(begin + kSparseTileEntries, n);
-    for (int64_t i = begin + threadIdx.x; i < end; i += blockDim.x) {
-        const int b = key_bucket<IdT>(keys[i], L, false);
-        if (b >= 0) atomicAdd(hist + b, 1);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < L; i += blockDim.x) a.scratch[static_cast<int64_t>(blockIdx.x) * L + i] = hist[i];
+    count_tile<IdT>(static_cast<const IdT*>(a.ids), static_cast<int64_t>(a.T) * K, L, false, tile_entries, a.scratch);
 }
 
-template <typename IdT>
-__global__ void __launch_bounds__(kRerouteThreads)
-sparse_reroute_kernel(Batch<SparseArgs> batch, int K, int L, int D, int interleave, int overlapped) {
+// Routing parameters of an expert as the resolution wants them: a reciprocal for the remainder, and a staged prefix row
+// whose unused entries are never reached, so that the replica index is eight comparisons without a loop bound.
+struct FastRouter {
+    int C;              // instances
+    int total, stride, offset;  // stride 0: no interleave
+    uint32_t recip;     // floor((2^32 - 1) / total)
+};
+
+// Rows of the plan of every expert into shared memory, asynchronously: all of them are asked for at once, whether
+// the expert has that many instances or not (the rows are there), so that they cost one round trip beside the
+// entries' own. The instance counts go where the routers will stand.
+__device__ __forceinline__ void stage_plan_rows_async(const int32_t* __restrict__ lcnts, const int32_t* __restrict__ rqp,
+                                                      const int32_t* __restrict__ l2p, int L, int D, bool quota_mode,
+                                                      FastRouter* routers, int32_t* prefix_s, int32_t* l2p_s) {
+    const int tid = threadIdx.x, nt = blockDim.x;
+    for (int e = tid; e < L; e += nt) cp_async_4(&routers[e].C, lcnts + e);
+    const bool vec = D >= kStagedReps && (D % 4) == 0 &&
+                     ((reinterpret_cast<uintptr_t>(l2p) | reinterpret_cast<uintptr_t>(quota_mode ? rqp : l2p)) & 15u) == 0;
+    if (vec) {
+        for (int i = tid; i < L * (kStagedReps / 4); i += nt) {
+            const int e = i / (kStagedReps / 4), j = i % (kStagedReps / 4) * 4;
+            cp_async_16(l2p_s + e * kStagedReps + j, l2p + static_cast<int64_t>(e) * D + j);
+            if (quota_mode) cp_async_16(prefix_s + e * kStagedReps + j, rqp + static_cast<int64_t>(e) * D + j);
+        }
+        return;
+    }
+    for (int i = tid; i < L * kStagedReps; i += nt) {
+        const int e = i / kStagedReps, j = i % kStagedReps;
+        if (j < D) {
+            cp_async_4(l2p_s + i, l2p + static_cast<int64_t>(e) * D + j);
+            if (quota_mode) cp_async_4(prefix_s + i, rqp + static_cast<int64_t>(e) * D + j);
+        }
+    }
+}
+
+// prefix_row: the expert's staged row (rewritten here), or null where rows are not staged.
+__device__ __forceinline__ FastRouter make_fast_router(int e, int C, const int32_t* __restrict__ rqp, int D, bool quota_mode,
+                                                       bool interleave, int32_t* prefix_row) {
+    FastRouter r{C, 0, 0, 0, 0};
+    if (C <= 1 || !quota_mode) return r;
+    if (prefix_row != nullptr && C <= kStagedReps) {
+        r.total = C <= D ? prefix_row[C - 1] : 0;
+#pragma unroll
+        for (int j = 0; j < kStagedReps; ++j) {
+            if (j >= C - 1) prefix_row[j] = INT_MAX;  // the index ends at C - 1 whatever the last prefix says
+            else if (j >= D) prefix_row[j] = 0;
+        }
+    } else {
+        r.total = rqp[static_cast<int64_t>(e) * D + C - 1];
+    }
+    if (interleave && r.total > 1) {
+        r.stride = interleave_stride(r.total);
+        r.offset = e % r.total;
+        r.recip = 0xFFFFFFFFu / static_cast<uint32_t>(r.total);
+    }
+    return r;
+}
+
+__device__ __noinline__ int mod_wide(unsigned long long x, int total) { return static_cast<int>(x % static_cast<unsigned long long>(total)); }
+
+// ordinal -> replica index, for an expert with two or more instances.
+__device__ __forceinline__ int fast_replica_index(const FastRouter& r, int ordinal, const int32_t* prefix_row,
+                                                  const int32_t* __restrict__ rqp_row, bool quota_mode) {
+    if (!quota_mode) return ordinal % r.C;
+    int qr = ordinal;
+    if (r.stride != 0) {
+        const unsigned long long prod = static_cast<unsigned long long>(static_cast<unsigned>(ordinal)) * static_cast<unsigned>(r.stride) +
+                                        static_cast<unsigned>(r.offset);
+        if ((prod >> 32) == 0) {
+            // x * recip >> 32 is the quotient or one less: 2^32 / total - recip <= 1, so the product falls short by less than 2^32
+            const uint32_t x = static_cast<uint32_t>(prod), t = static_cast<uint32_t>(r.total);
+            uint32_t rem = x - __umulhi(x, r.recip) * t;
+            if (rem >= t) rem -= t;
+            qr = static_cast<int>(rem);
+        } else {
+            qr = mod_wide(prod, r.total);
+        }
+    }
+    int idx = 0;
+    if (prefix_row != nullptr && r.C <= kStagedReps) {
+        const int4 a = reinterpret_cast<const int4*>(prefix_row)[0], b = reinterpret_cast<const int4*>(prefix_row)[1];
+        idx = (qr >= a.x) + (qr >= a.y) + (qr >= a.z) + (qr >= a.w) + (qr >= b.x) + (qr >= b.y) + (qr >= b.z) + (qr >= b.w);
+    } else {
+        for (int j = 0; j < r.C - 1; ++j) idx += (qr >= rqp_row[j]) ? 1 : 0;
+    }
+    return idx;
+}
+
+// shared memory: prefix rows [L][8] i32 | l2p rows [L][8] i32 (both only where they fit) | ordinals | routers[L]
+size_t sparse_smem_bytes(int L, bool rows_staged) {
+    return (rows_staged ? static_cast<size_t>(L) * 2 * kStagedReps * 4 : 0) + ord_smem_bytes(L, kOrdThreads) + sizeof(FastRouter) * static_cast<size_t>(L);
+}
+
+// ids may alias out (every entry is read and written by the same thread, and nobody else reads it once the first is written).
+// 512 threads at <= 96 registers and ~144*L bytes of shared memory leave room for this CTA on an SM that a weight_sync
+// CTA occupies.
+template <int EPT, typename IdT>
+__global__ void __launch_bounds__(kOrdThreads) __maxnreg__(EPT > 4 ? 96 : 64)
+sparse_reroute_kernel(Batch<SparseArgs> batch, int ctas, int K, int L, int D, int interleave, int rows_staged, int use_table) {
     extern __shared__ __align__(128) char smem_raw[];
     const SparseArgs& a = batch.a[blockIdx.y];
     const IdT* ids = static_cast<const IdT*>(a.ids);
     IdT* out = static_cast<IdT*>(a.out);
-    const int32_t* __restrict__ l2p = a.l2p;
-    const int32_t* __restrict__ lcnts = a.lcnts;
-    const int32_t* __restrict__ rqp = a.rqp;
-    const int32_t* __restrict__ tile_counts = a.scratch;
     const int64_t n = static_cast<int64_t>(a.T) * K;
-    if (static_cast<int64_t>(blockIdx.x) * kSparseTileEntries >= n) return;
-    // layout: base[L] | routers[L] | prefix rows [L][8] | l2p rows [L][8] | warp_base[nwarps][L]
-    int32_t* base = reinterpret_cast<int32_t*>(smem_raw);
-    Router* routers = reinterpret_cast<Router*>(base + L);
-    int32_t* prefix_s = reinterpret_cast<int32_t*>(routers + L);
+    if (n == 0) return;  // every CTA of the rank
+    const bool quota_mode = interleave != 2;  // 2: round-robin (legacy placement)
+    int32_t* prefix_s = reinterpret_cast<int32_t*>(smem_raw);
     int32_t* l2p_s = prefix_s + static_cast<size_t>(L) * kStagedReps;
-    int32_t* warp_base = l2p_s + static_cast<size_t>(L) * kStagedReps;
-    const int tile = blockIdx.x;
-    auto sum_earlier_tiles = [&]() {
-        for (int e = threadIdx.x; e < L; e += blockDim.x) {
-            int b = 0;
-#pragma unroll 8
-            for (int tl = 0; tl < tile; ++tl) b += __ldcg(tile_counts + static_cast<int64_t>(tl) * L + e);
-            base[e] = b;
+    const OrdShared o = carve_ord_smem(rows_staged ? reinterpret_cast<char*>(l2p_s + static_cast<size_t>(L) * kStagedReps) : smem_raw, L);
+    FastRouter* routers = reinterpret_cast<FastRouter*>(o.counters + kOrdWarps * ord_row(L));
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (rows_staged) stage_plan_rows_async(a.lcnts, a.rqp, a.l2p, L, D, quota_mode, routers, prefix_s, l2p_s);
+
+    int64_t begin, end;
+    int iters;
+    uint32_t packed[EPT];
+    cluster_ordinals<EPT, false, IdT>(
+        ids, n, L, false, ctas, use_table ? a.scratch : nullptr, o, begin, end, iters, packed,
+        [&]() {
+            for (int e = tid; e < L; e += kOrdThreads) {
+                const int C = rows_staged ? routers[e].C : a.lcnts[e];
+                routers[e] = make_fast_router(e, C, a.rqp, D, quota_mode, interleave == 1, rows_staged ? prefix_s + e * kStagedReps : nullptr);
+            }
+        },
+        [&](int b, int base, int) { o.base[b] = base; });
+    if (ctas > 1) cluster_arrive();
+#pragma unroll
+    for (int i = 0; i < EPT; ++i) {
+        const int64_t at = begin + i * kWarp + lane;
+        if (i >= iters || at >= end) continue;
+        const uint32_t p = packed[i];
+        const int b = static_cast<int>(p & 0xFFFFu);
+        const int C = p != 0xFFFFFFFFu ? routers[b].C : 0;
+        if (C <= 0) {  // an id outside [0, L), or an expert that maps nothing: the id stays
+            if (out != ids) out[at] = ids[at];
+            continue;
         }
-    };
-    // Launched behind the count kernel in the ordinary way, its counts are complete already: their loads go out
-    // together with those of the plan rows. Launched as a dependent kernel, everything up to the wait reads the
-    // plan and the ids only.
-    if (!overlapped) sum_earlier_tiles();
-    for (int e = threadIdx.x; e < L; e += blockDim.x) {
-        stage_expert(e, lcnts, rqp, l2p, D, interleave != 2, interleave == 1, routers, prefix_s, l2p_s);  // 2: round-robin (legacy placement)
+        int j = 0;
+        if (C > 1) {
+            const int ordinal = o.base[b] + o.counters[warp * ord_row(L) + b] + static_cast<int>(p >> 16);
+            j = fast_replica_index(routers[b], ordinal, rows_staged ? prefix_s + b * kStagedReps : nullptr,
+                                   a.rqp + static_cast<int64_t>(b) * D, quota_mode);
+        }
+        out[at] = static_cast<IdT>(rows_staged && j < kStagedReps ? l2p_s[b * kStagedReps + j] : a.l2p[static_cast<int64_t>(b) * D + j]);
     }
-    tile_warp_counts<IdT>(ids, n, L, false, warp_base);
-    if (overlapped) {
-        pdl_wait();  // the tile counts of the first kernel are complete from here on
-        sum_earlier_tiles();
-        __syncthreads();
-    }
-    // ids may alias out: every entry is read and written by the same lane, the write comes
-    // last, and tiles do not overlap.
-    tile_resolve<IdT>(ids, n, L, false, base, warp_base, [&](int64_t i, int b, int ordinal) {
-        if (b < 0) {
-            out[i] = ids[i];
-            return;
-        }
-        const Router r = routers[b];
-        if (r.C <= 0) {
-            out[i] = ids[i];
-            return;
-        }
-        const int32_t* prefix = r.C <= kStagedReps ? prefix_s + b * kStagedReps : rqp + static_cast<int64_t>(b) * D;
-        const int j = replica_index(r, ordinal, prefix, interleave != 2);
-        out[i] = static_cast<IdT>(j < kStagedReps ? l2p_s[b * kStagedReps + j] : l2p[static_cast<int64_t>(b) * D + j]);
-    });
+    if (ctas > 1) cluster_wait();
 }
 
-// Experts with C <= 0 keep their id but still consume ordinals in the count pass; the
-// reference skips them before taking an ordinal (reroute.cu:505-509), which is equivalent
-// because such an expert never maps anything.
+// Experts with C <= 0 keep their id but still consume ordinals; the reference skips them before taking an ordinal
+// (reroute.cu:505-509), which is equivalent because such an expert never maps anything.
 
-__global__ void __launch_bounds__(kRerouteThreads)
-dispatch_positions_kernel(const int32_t* __restrict__ phys, int64_t n, int P, const int32_t* __restrict__ tile_counts,
-                          int num_tiles, int32_t* __restrict__ pos, int32_t* __restrict__ expert_offsets) {
+// ------------------------------------------------------------- dispatch positions
+__global__ void __launch_bounds__(kOrdThreads) dispatch_count_kernel(const int32_t* __restrict__ phys, int64_t n, int P, int tile_entries,
+                                                                     int32_t* __restrict__ table) {
+    pdl_launch_dependents();
+    count_tile<int32_t>(phys, n, P, true, tile_entries, table);
+}
+
+// Positions of the (token, k) entries once grouped by physical expert (stable) and the experts' row offsets: the
+// same ordinals, plus a scan of the grand totals over the experts. Keys outside [0, P) go to a group at the end.
+template <int EPT>
+__global__ void __launch_bounds__(kOrdThreads) __maxnreg__(EPT > 4 ? 128 : 80)
+dispatch_positions_kernel(const int32_t* __restrict__ phys, int64_t n, int ctas, int P, const int32_t* __restrict__ table,
+                          int32_t* __restrict__ pos, int32_t* __restrict__ expert_offsets) {
     extern __shared__ __align__(128) char smem_raw[];
+    __shared__ int warp_tot[kOrdWarps];
     const int nb = P + 1;
-    // layout: base[nb] | totals[nb] | warp_base[nwarps][nb]
-    int32_t* base = reinterpret_cast<int32_t*>(smem_raw);
-    int32_t* totals = base + nb;
-    int32_t* warp_base = totals + nb;
-    __shared__ int s_carry;
-    const int tile = blockIdx.x;
-    tile_warp_counts<int32_t>(phys, n, P, true, warp_base);
-    pdl_wait();
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-        int before = 0, total = 0;
-#pragma unroll 8
-        for (int tl = 0; tl < num_tiles; ++tl) {
-            const int c = __ldcg(tile_counts + static_cast<int64_t>(tl) * nb + b);
-            if (tl < tile) before += c;
-            total += c;
-        }
-        base[b] = before;
-        totals[b] = total;
-    }
-    if (threadIdx.x == 0) s_carry = 0;
-    __syncthreads();
-    // exclusive scan of totals over buckets (blocked: 256 buckets per round, warp shuffles)
-    for (int b0 = 0; b0 < nb; b0 += blockDim.x) {
-        const int b = b0 + threadIdx.x;
-        const int v = b < nb ? totals[b] : 0;
-        int incl = v;
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const OrdShared o = carve_ord_smem(smem_raw, nb);
+    int32_t* all_of = o.behind;  // free once the totals are out
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nthreads = blockDim.x;
+    int64_t begin, end;
+    int iters;
+    uint32_t packed[EPT];
+    cluster_ordinals<EPT, true, int32_t>(
+        phys, n, P, true, ctas, table, o, begin, end, iters, packed, []() {},
+        [&](int b, int base, int all) {
+            o.base[b] = base;
+            all_of[b] = all;
+        });
+    if (ctas > 1) cluster_arrive();
+    int carry = 0;
+    for (int b0 = 0; b0 < nb; b0 += nthreads) {
+        const int b = b0 + tid;
+        const int all = b < nb ? all_of[b] : 0;
+        int incl = all;
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int o = __shfl_up_sync(kFullMask, incl, d);
-            if (lane >= d) incl += o;
+        for (int d = 1; d < kWarp; d <<= 1) {
+            const int t = __shfl_up_sync(kFullMask, incl, d);
+            if (lane >= d) incl += t;
         }
-        __shared__ int warp_tot[kRerouteThreads / 32];
-        if (lane == 31) warp_tot[warp] = incl;
+        if (lane == kWarp - 1) warp_tot[warp] = incl;
         __syncthreads();
-        int woff = 0;
-        for (int w = 0; w < warp; ++w) woff += warp_tot[w];
-        const int carry = s_carry;
-        const int excl = carry + woff + incl - v;
+        const int wt = lane < nthreads / kWarp ? warp_tot[lane] : 0;
+        const int excl = carry + __reduce_add_sync(kFullMask, lane < warp ? wt : 0) + incl - all;
         if (b < nb) {
-            base[b] += excl;
-            if (tile == 0 && expert_offsets != nullptr) expert_offsets[b] = excl;
+            o.base[b] += excl;
+            if (blockIdx.x == 0 && expert_offsets != nullptr) expert_offsets[b] = excl;
         }
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) s_carry = carry + woff + incl;
+        carry += __reduce_add_sync(kFullMask, wt);
         __syncthreads();
     }
-    tile_resolve<int32_t>(phys, n, P, true, base, warp_base,
-                          [&](int64_t i, int, int ordinal) { pos[i] = ordinal; });
+#pragma unroll
+    for (int i = 0; i < EPT; ++i) {
+        const int64_t at = begin + i * kWarp + lane;
+        if (i >= iters || at >= end) continue;
+        const int b = static_cast<int>(packed[i] & 0xFFFFu);
+        pos[at] = o.base[b] + o.counters[warp * ord_row(nb) + b] + static_cast<int>(packed[i] >> 16);
+    }
+    if (ctas > 1) cluster_wait();
 }
 
 // ------------------------------------------------------------------- row gather (HBM)
@@ -803,8 +779,8 @@ cudaError_t ensure_smem_attr(const void* fn, size_t bytes) {
     // kernels run next to weight_sync, whose CTAs need most of an SM's shared memory, and an SM that was set up
     // with a small carve-out for a reroute CTA cannot take a weight_sync CTA until it has drained.
     static std::mutex mu;
-    static const void* fns[16];
-    static size_t granted[16];
+    static const void* fns[32];
+    static size_t granted[32];
     static int n = 0;
     std::lock_guard<std::mutex> lock(mu);
     int i = 0;
@@ -812,16 +788,16 @@ cudaError_t ensure_smem_attr(const void* fn, size_t bytes) {
     if (i == n) {
         cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         if (e != cudaSuccess) return e;
-        if (n < 16) {
+        if (n < 32) {
             fns[n] = fn;
             granted[n] = 48 * 1024;
             ++n;
         }
     }
-    if (bytes <= 48 * 1024 || (i < 16 && granted[i] >= bytes)) return cudaSuccess;
+    if (bytes <= 48 * 1024 || (i < 32 && granted[i] >= bytes)) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
     if (e != cudaSuccess) return e;
-    if (i < 16) granted[i] = bytes;
+    if (i < 32) granted[i] = bytes;
     return cudaSuccess;
 }
 
@@ -907,30 +883,109 @@ cudaError_t launch_dense_backward(const Batch<DenseBwdArgs>& b, int L, int P, in
     return cudaGetLastError();
 }
 
+// How an input of n entries is cut: a cluster of CTAs with at most per_lane entries a thread, and as many clusters as it
+// takes. Measured on one rank's int32 ids, 128 experts (us; the count + reroute pair that this replaces: 14.8 at 65536):
+//   * the cluster grows to eight CTAs before a thread takes a second entry: 2048 entries 4.5 on four CTAs, 5.7 on one;
+//   * up to 16384 entries one cluster (6.9; two clusters the same), behind it two entries a thread up to eight clusters
+//     (65536 entries 7.8; four entries a thread 8.5, one 9.6) and four beyond (131072: 9.6 against 11.4 with two);
+//   * behind kOrdRecountMax entries the repeated counting is more than a count kernel, and tiles of sixteen entries a
+//     thread keep its table short;
+//   * several ranks in one launch with more than a cluster each: the count kernel and single CTAs. The launch runs beside
+//     weight_sync, which leaves every SM a quarter of its shared memory: single CTAs find room anywhere, clusters of
+//     eight wait for it or keep weight_sync out (65536 entries of eight ranks: the step took 69 us with clusters).
+constexpr int64_t kOrdRecountMax = 1 << 18;
+constexpr size_t kOrdMaxSmem = 225 * 1024;
+
+struct OrdGrid {
+    int threads, ctas, clusters, per_lane;
+    bool table;
+};
+OrdGrid ord_grid(int64_t n, int ranks, bool in_place, int threads) {
+    OrdGrid g{threads, 1, 1, 1, false};
+    while (g.ctas < kOrdMaxCluster && n > static_cast<int64_t>(g.ctas) * threads) g.ctas *= 2;
+    int64_t row = static_cast<int64_t>(g.ctas) * threads;  // one entry per thread of a cluster
+    if (n <= row) return g;
+    g.per_lane = n > kOrdRecountMax ? 16 : 4;
+    g.table = n > 4 * row && (in_place || ranks > 1 || n > kOrdRecountMax);
+    if (g.table && ranks > 1) {
+        g.ctas = 1;
+        row = threads;
+    }
+    // (tiles of the table: per_lane entries a thread)
+    const int64_t chunk = row * (g.table ? g.per_lane : (n > 4 * row && n <= 16 * row ? 2 : 4));
+    g.clusters = static_cast<int>((n + chunk - 1) / chunk);
+    return g;
+}
+
+// Launch of clusters of `g.ctas` CTAs; `overlap`: as a programmatic dependent launch behind the count kernel.
+template <typename... Params, typename... Args>
+cudaError_t launch_clusters(void (*kernel)(Params...), const OrdGrid& g, int ranks, size_t smem, cudaStream_t stream, bool overlap, Args&&... args) {
+    cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(kernel), smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(g.ctas) * g.clusters, ranks);
+    cfg.blockDim = dim3(g.threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    int na = 0;
+    if (g.ctas > 1) {
+        attr[na].id = cudaLaunchAttributeClusterDimension;
+        attr[na].val.clusterDim.x = g.ctas;
+        attr[na].val.clusterDim.y = 1;
+        attr[na].val.clusterDim.z = 1;
+        ++na;
+    }
+    if (overlap) {
+        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[na].val.programmaticStreamSerializationAllowed = 1;
+        ++na;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = na;
+    count_launch();
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+// `launch` with the compile-time number of entries a thread holds.
+template <typename Launch>
+cudaError_t with_lanes(const OrdGrid& g, Launch launch) {
+    if (g.per_lane == 1) return launch(std::integral_constant<int, 1>{});
+    if (g.per_lane == 4) return launch(std::integral_constant<int, 4>{});
+    return launch(std::integral_constant<int, 16>{});
+}
+
 template <typename IdT>
 static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L, int D, int interleave,
                                        cudaStream_t stream) {
     int64_t max_n = 0;
+    bool in_place = false;
     for (int i = 0; i < b.n; ++i) {
         const int64_t n = static_cast<int64_t>(b.a[i].T) * K;
         max_n = n > max_n ? n : max_n;
+        const uintptr_t x = reinterpret_cast<uintptr_t>(b.a[i].ids), y = reinterpret_cast<uintptr_t>(b.a[i].out);
+        const uintptr_t bytes = static_cast<uintptr_t>(n) * sizeof(IdT);
+        in_place = in_place || (n > 0 && x < y + bytes && y < x + bytes);
     }
     if (max_n == 0) return cudaSuccess;
-    const dim3 grid(static_cast<unsigned>(sparse_tiles(max_n)), b.n);
-    const size_t smem1 = sizeof(int32_t) * L;
-    const size_t smem2 = sizeof(int32_t) * L + sizeof(Router) * L + 2 * sizeof(int32_t) * kStagedReps * L +
-                         sizeof(int32_t) * (kRerouteThreads / 32) * L;
-    cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(sparse_count_kernel<IdT>), smem1);
-    if (e != cudaSuccess) return e;
-    e = ensure_smem_attr(reinterpret_cast<const void*>(sparse_reroute_kernel<IdT>), smem2);
-    if (e != cudaSuccess) return e;
-    count_launch(2);
-    sparse_count_kernel<IdT><<<grid, kRerouteThreads, smem1, stream>>>(b, K, L);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    const bool overlap = b.n == 1 && pdl_enabled();
-    return launch_dependent(sparse_reroute_kernel<IdT>, grid, dim3(kRerouteThreads), smem2, stream, overlap, b, K, L, D, interleave,
-                            overlap ? 1 : 0);
+    const int staged = sparse_smem_bytes(L, true) <= kOrdMaxSmem ? 1 : 0;
+    const size_t smem = sparse_smem_bytes(L, staged != 0);
+    const OrdGrid g = ord_grid(max_n, b.n, in_place, kOrdThreads);
+    // One rank per launch is latency-bound and the overlap with the count kernel pays; several ranks fill the device
+    // with the first kernel alone.
+    const bool overlap = g.table && b.n == 1 && pdl_enabled();
+    if (g.table) {
+        cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(sparse_count_kernel<IdT>), sizeof(int32_t) * L);
+        if (e != cudaSuccess) return e;
+        count_launch();
+        sparse_count_kernel<IdT><<<dim3(g.ctas * g.clusters, b.n), kOrdThreads, sizeof(int32_t) * L, stream>>>(b, K, L, g.per_lane * kOrdThreads);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return with_lanes(g, [&](auto per_lane) {
+        return launch_clusters(sparse_reroute_kernel<decltype(per_lane)::value, IdT>, g, b.n, smem, stream, overlap, b, g.ctas, K, L, D,
+                               interleave, staged, g.table ? 1 : 0);
+    });
 }
 
 cudaError_t launch_sparse_reroute(const Batch<SparseArgs>& b, int ids_kind, int K, int L, int D, int interleave,
@@ -1073,17 +1128,20 @@ int uep_dispatch_positions(const int32_t* phys_ids, int64_t num_entries, int P, 
         return UEP_OK;
     }
     if (!phys_ids || !pos || !scratch) return fail(UEP_ERR_INVALID, "dispatch_positions: null pointer");
-    const int tiles = static_cast<int>(sparse_tiles(num_entries));
-    const int nb = P + 1;
-    const size_t smem1 = sizeof(int32_t) * nb;
-    const size_t smem2 = sizeof(int32_t) * nb * (2 + kRerouteThreads / 32);
-    UEP_CUDA_TRY(ensure_smem_attr(reinterpret_cast<const void*>(key_count_kernel<int32_t>), smem1));
-    UEP_CUDA_TRY(ensure_smem_attr(reinterpret_cast<const void*>(dispatch_positions_kernel), smem2));
-    count_launch(2);
-    key_count_kernel<int32_t><<<tiles, kRerouteThreads, smem1, stream>>>(phys_ids, num_entries, P, 1, scratch);
-    UEP_CUDA_TRY(cudaGetLastError());
-    UEP_CUDA_TRY(launch_dependent(dispatch_positions_kernel, dim3(tiles), dim3(kRerouteThreads), smem2, stream, true, phys_ids,
-                                  num_entries, P, static_cast<const int32_t*>(scratch), tiles, pos, expert_offsets));
+    const OrdGrid g = ord_grid(num_entries, 1, false, ord_smem_bytes(P + 1, kOrdThreads) <= kOrdMaxSmem ? kOrdThreads : kOrdFewThreads);
+    const size_t smem = ord_smem_bytes(P + 1, g.threads), smem1 = sizeof(int32_t) * (P + 1);
+    const bool overlap = g.table && pdl_enabled();
+    if (g.table) {
+        UEP_CUDA_TRY(ensure_smem_attr(reinterpret_cast<const void*>(dispatch_count_kernel), smem1));
+        count_launch();
+        dispatch_count_kernel<<<g.ctas * g.clusters, g.threads, smem1, stream>>>(phys_ids, num_entries, P, g.per_lane * g.threads, scratch);
+        UEP_CUDA_TRY(cudaGetLastError());
+    }
+    const int32_t* table = g.table ? scratch : nullptr;
+    UEP_CUDA_TRY(with_lanes(g, [&](auto per_lane) {
+        return launch_clusters(dispatch_positions_kernel<decltype(per_lane)::value>, g, 1, smem, stream, overlap, phys_ids, num_entries, g.ctas, P,
+                               table, pos, expert_offsets);
+    }));
     return UEP_OK;
 }
 
