@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -23,9 +24,67 @@ using namespace uep;
 
 struct uep_event {
     cudaEvent_t ev = nullptr;
+    int device = 0;
 };
 
 namespace {
+
+// Ordering events that calls hand out and take back: at most kEventsKept idle ones per device are kept (a create and a
+// destroy per call cost about a microsecond of host time). An idle event may still be waited for by a stream: a wait holds on
+// to the record it was made for, so the event can be recorded anew. Any thread.
+class EventPool {
+    static constexpr int kEventsKept = 32, kDevices = 64;
+    std::mutex mu_;
+    std::vector<cudaEvent_t> idle_[kDevices];
+
+public:
+    cudaError_t take(uep_event* out) {
+        cudaError_t e = cudaGetDevice(&out->device);
+        if (e != cudaSuccess) return e;
+        if (out->device < kDevices) {
+            std::lock_guard<std::mutex> lock(mu_);
+            auto& idle = idle_[out->device];
+            if (!idle.empty()) {
+                out->ev = idle.back();
+                idle.pop_back();
+                return cudaSuccess;
+            }
+        }
+        return cudaEventCreateWithFlags(&out->ev, cudaEventDisableTiming);
+    }
+    void give_back(uep_event* ev) {
+        if (ev->ev == nullptr) return;
+        if (ev->device < kDevices) {
+            std::lock_guard<std::mutex> lock(mu_);
+            auto& idle = idle_[ev->device];
+            if (idle.size() < kEventsKept) {
+                idle.push_back(ev->ev);
+                ev->ev = nullptr;
+                return;
+            }
+        }
+        cudaEventDestroy(ev->ev);
+        ev->ev = nullptr;
+    }
+};
+EventPool& event_pool() {
+    static EventPool* pool = new EventPool();  // never destroyed: events may be given back while the process exits
+    return *pool;
+}
+
+// A recorded event, or the error (then nothing is left behind).
+cudaError_t record_event(cudaStream_t stream, uep_event** out) {
+    uep_event* ev = new uep_event();
+    cudaError_t e = event_pool().take(ev);
+    if (e == cudaSuccess) e = cudaEventRecord(ev->ev, stream);
+    if (e != cudaSuccess) {
+        event_pool().give_back(ev);
+        delete ev;
+        return e;
+    }
+    *out = ev;
+    return cudaSuccess;
+}
 
 struct ArenaLayout {
     size_t gather, sync_flags, reduce_flags, relay_flags, replica_weight, replica_scale, replica_grad, total;
@@ -188,15 +247,8 @@ void free_rank(RankHost& r, int my_rank_count) {
 int finish_sync_op(uep_manager* m, int async_finish, cudaStream_t current, uep_event** done_event) {
     if (async_finish) {
         if (done_event == nullptr) return fail(UEP_ERR_INVALID, "async_finish requires done_event");
-        uep_event* ev = new uep_event();
-        cudaError_t e = cudaEventCreateWithFlags(&ev->ev, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaEventRecord(ev->ev, m->comm_stream);
-        if (e != cudaSuccess) {
-            if (ev->ev) cudaEventDestroy(ev->ev);
-            delete ev;
-            return fail_cuda(e, "event for async_finish");
-        }
-        *done_event = ev;
+        const cudaError_t e = record_event(m->comm_stream, done_event);
+        if (e != cudaSuccess) return fail_cuda(e, "event for async_finish");
     } else {
         if (done_event != nullptr) *done_event = nullptr;
         return order_after(m, current, m->comm_stream);
@@ -635,7 +687,8 @@ int uep_weight_sync(uep_manager* m, int layer_id, const int64_t* const* fc1_ptrs
     call.relay_cap = m->relay_cap;
     call.sync_epoch = m->ranks[0].epochs + 1;
     call.trace = m->sync_trace;
-    if (m->R > 0) UEP_CUDA_TRY(launch_weight_sync(call, m->comm_stream));
+    // a group of one rank has nobody to send to
+    if (m->R > 0 && m->N > 1) UEP_CUDA_TRY(launch_weight_sync(call, m->comm_stream));
     return finish_sync_op(m, async_finish, current, done_event);
 }
 
@@ -672,7 +725,8 @@ int uep_grad_reduce(uep_manager* m, int layer_id, const int64_t* const* fc1_grad
     call.ctas_per_rank = std::max(1, std::min(m->grad_reduce_ctas, m->num_sms / m->nlocal));
     call.trace = m->sync_trace;
     call.reduce_epoch = m->ranks[0].epochs + 2;
-    if (m->R > 0 && m->total_numel > 0) UEP_CUDA_TRY(launch_grad_reduce(call, m->comm_stream));
+    // a group of one rank has no replicas
+    if (m->R > 0 && m->N > 1 && m->total_numel > 0) UEP_CUDA_TRY(launch_grad_reduce(call, m->comm_stream));
     return finish_sync_op(m, async_finish, current, done_event);
 }
 
@@ -763,16 +817,8 @@ int uep_set_grad_reduce_deterministic(uep_manager* m, int deterministic, int num
 
 int uep_event_record(void* stream, uep_event** out) {
     if (out == nullptr) return fail(UEP_ERR_INVALID, "event_record: null output");
-    uep_event* ev = new uep_event();
-    cudaError_t e = cudaEventCreateWithFlags(&ev->ev, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventRecord(ev->ev, static_cast<cudaStream_t>(stream));
-    if (e != cudaSuccess) {
-        if (ev->ev) cudaEventDestroy(ev->ev);
-        delete ev;
-        return fail_cuda(e, "event_record");
-    }
-    *out = ev;
-    return UEP_OK;
+    const cudaError_t e = record_event(static_cast<cudaStream_t>(stream), out);
+    return e == cudaSuccess ? UEP_OK : fail_cuda(e, "event_record");
 }
 
 int uep_event_stream_wait(uep_event* ev, void* stream) {
@@ -789,7 +835,7 @@ int uep_event_synchronize(uep_event* ev) {
 
 void uep_event_destroy(uep_event* ev) {
     if (ev == nullptr) return;
-    if (ev->ev) cudaEventDestroy(ev->ev);
+    event_pool().give_back(ev);
     delete ev;
 }
 

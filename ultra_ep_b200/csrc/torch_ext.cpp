@@ -7,11 +7,17 @@
 // destroy(), as in the reference) and turns status codes into Python exceptions.
 
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
+#include <nvtx3/nvToolsExt.h>
 #include <pybind11/functional.h>
 #include <pybind11/stl.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/python_variable.h>
 #include <torch/extension.h>
 
+#include <cstdio>
 #include <cstring>
 #include <memory>
 #include <optional>
@@ -77,6 +83,22 @@ const int64_t* ptr_table(const torch::Tensor& t, int expect, const char* name) {
         throw std::runtime_error(std::string(name) + " must be a cuda int64 tensor with one entry per local master expert");
     return t.data_ptr<int64_t>();
 }
+
+// Output tensors straight from the caching allocator: a call makes up to sixteen of them, and the dispatcher's empty()
+// costs about twice as much host time each.
+torch::Tensor empty_2d(int64_t rows, int64_t cols, torch::ScalarType dtype, const torch::Device& device) {
+    return at::detail::empty_cuda({rows, cols}, dtype, device, std::nullopt);
+}
+
+// Profiler range around one call.
+struct Range {
+    Range(const char* what, int layer) {
+        char name[64];
+        std::snprintf(name, sizeof(name), "%s (layer %d)", what, layer);
+        nvtxRangePushA(name);
+    }
+    ~Range() { nvtxRangePop(); }
+};
 
 class Manager {
     uep_manager* m_ = nullptr;
@@ -203,6 +225,7 @@ public:
     bool is_available() const { return available_; }
 
     void update_placement(int layer_id, torch::Tensor& routing_map) {
+        const Range range("Update placement", layer_id);
         UEP_ASSERT(available_);
         UEP_ASSERT(routing_map.is_cuda() && routing_map.dim() == 2 && routing_map.size(1) == L_ &&
                    routing_map.dtype() == torch::kBool);
@@ -222,7 +245,7 @@ public:
         uep_event* ev = nullptr;
         check(uep_event_record(current_stream(), &ev), "update_placement_sparse");
         const int rc = uep_event_stream_wait(ev, comm);
-        uep_event_destroy(ev);
+        uep_event_destroy(ev);  // (back to the library's pool)
         check(rc, "update_placement_sparse");
         const void* in = ids.data_ptr();
         const int T = static_cast<int>(ids.size(0));
@@ -245,6 +268,7 @@ public:
 
     std::tuple<torch::Tensor, torch::Tensor> dense_reroute_forward(int layer_id, torch::Tensor& probs,
                                                                    torch::Tensor& routing_map) {
+        const Range range("Dense reroute forward", layer_id);
         UEP_ASSERT(available_);
         UEP_ASSERT(routing_map.is_cuda() && probs.is_cuda());
         UEP_ASSERT(routing_map.dtype() == torch::kBool);
@@ -255,8 +279,8 @@ public:
         const int T = static_cast<int>(routing_map.size(0));
         auto dev = routing_map.device();
         // every element is written by the kernel: no zero-fill pass
-        auto expanded_probs = torch::empty({T, P_}, torch::TensorOptions().dtype(torch::kFloat32).device(dev));
-        auto expanded_rmap = torch::empty({T, P_}, torch::TensorOptions().dtype(torch::kBool).device(dev));
+        auto expanded_probs = empty_2d(T, P_, torch::kFloat32, dev);
+        auto expanded_rmap = empty_2d(T, P_, torch::kBool, dev);
         const uint8_t* maps = reinterpret_cast<const uint8_t*>(routing_map.data_ptr());
         const float* pr = probs.data_ptr<float>();
         uint8_t* om = reinterpret_cast<uint8_t*>(expanded_rmap.data_ptr());
@@ -275,7 +299,7 @@ public:
         auto em = expanded_routing_map.contiguous();
         const int T = static_cast<int>(routing_map.size(0));
         const int P = static_cast<int>(grad_expanded_probs.size(1));
-        auto grad_probs = torch::empty({T, L_}, torch::TensorOptions().dtype(torch::kFloat32).device(routing_map.device()));
+        auto grad_probs = empty_2d(T, L_, torch::kFloat32, routing_map.device());
         const float* g = grad_expanded_probs.data_ptr<float>();
         const uint8_t* maps = reinterpret_cast<const uint8_t*>(routing_map.data_ptr());
         const uint8_t* emaps = reinterpret_cast<const uint8_t*>(em.data_ptr());
@@ -300,6 +324,7 @@ public:
     std::optional<EventHandle> weight_sync(int layer_id, torch::Tensor& fc1_ptrs, torch::Tensor& fc2_ptrs,
                                            torch::Tensor& fc1_scale_ptrs, torch::Tensor& fc2_scale_ptrs,
                                            std::optional<EventHandle>& previous_event, bool async_finish) {
+        const Range range("Launch weight_sync", layer_id);
         UEP_ASSERT(available_);
         const int64_t* a = ptr_table(fc1_ptrs, M_, "local_master_fc1_weight_ptr_tensor");
         const int64_t* b = ptr_table(fc2_ptrs, M_, "local_master_fc2_weight_ptr_tensor");
@@ -340,6 +365,148 @@ public:
         return buf(id, torch::kFloat32);
     }
 };
+
+// Backward node of the differentiable dense reroute: [T,P] gradients of the expanded probabilities back to [T,L]. A node of
+// its own rather than a Python autograd.Function: the engine calls it without taking the interpreter lock, and the
+// (non-differentiable) expanded map asks for no zero-filled gradient.
+struct DenseRerouteBackward : public torch::autograd::Node {
+    std::shared_ptr<Manager> manager;
+    int layer_id = 0;
+    torch::Tensor routing_map, expanded_map;
+
+    torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+        torch::Tensor grad = grads[0];
+        if (!grad.defined()) grad = torch::zeros(expanded_map.sizes(), expanded_map.options().dtype(torch::kFloat32));
+        at::AutoDispatchBelowADInplaceOrView guard;
+        return {manager->dense_reroute_backward(layer_id, grad, routing_map, expanded_map)};
+    }
+    std::string name() const override { return "DenseRerouteBackward"; }
+};
+
+std::tuple<torch::Tensor, torch::Tensor> dense_reroute(const std::shared_ptr<Manager>& manager, int layer_id, torch::Tensor probs,
+                                                       torch::Tensor routing_map) {
+    torch::Tensor in = probs, map = routing_map;
+    std::tuple<torch::Tensor, torch::Tensor> out;
+    {
+        at::AutoDispatchBelowADInplaceOrView guard;
+        out = manager->dense_reroute_forward(layer_id, in, map);
+    }
+    if (at::GradMode::is_enabled() && probs.requires_grad()) {
+        std::shared_ptr<DenseRerouteBackward> node(new DenseRerouteBackward(), torch::autograd::deleteNode);
+        node->manager = manager;
+        node->layer_id = layer_id;
+        node->routing_map = routing_map;
+        node->expanded_map = std::get<1>(out);
+        node->set_next_edges(torch::autograd::collect_next_edges(probs));
+        torch::autograd::set_history(std::get<0>(out), node);
+    }
+    return out;
+}
+
+// ---- groups hosted on one device (ultra_ep_b200/sim.py) -------------------------------------
+// The same C ABI entry points with one list element per hosted rank. They return the status code (the caller raises
+// with the library's message); building the pointer arrays in Python cost more than the launches.
+constexpr int kMaxHosted = 8;
+
+struct RankList {
+    const void* ptr[kMaxHosted] = {nullptr};
+    int rows[kMaxHosted] = {0};
+    at::Tensor first;
+    int n = 0;
+
+    explicit RankList(const py::handle& seq) {
+        if (seq.is_none()) return;
+        const py::sequence items = py::reinterpret_borrow<py::sequence>(seq);
+        n = static_cast<int>(py::len(items));
+        if (n > kMaxHosted) throw std::runtime_error("at most 8 ranks can be hosted on one device");
+        for (int i = 0; i < n; ++i) {
+            const py::object item = items[i];
+            if (!THPVariable_Check(item.ptr())) throw py::type_error("expected one tensor per hosted rank");
+            const at::Tensor& t = THPVariable_Unpack(item.ptr());
+            if (i == 0) first = t;
+            ptr[i] = t.data_ptr();
+            rows[i] = t.dim() > 0 ? static_cast<int>(t.size(0)) : 0;
+        }
+    }
+};
+uep_manager* group_of(uintptr_t handle) { return reinterpret_cast<uep_manager*>(handle); }
+// int64 device tables of raw addresses, or null where there are none
+const int64_t* const* tables_of(const RankList& l) { return l.n > 0 ? reinterpret_cast<const int64_t* const*>(l.ptr) : nullptr; }
+
+int group_update_placement(uintptr_t handle, int layer, const py::object& inputs) {
+    const RankList in(inputs);
+    const int kind = in.first.scalar_type() == torch::kBool ? 0 : (in.first.scalar_type() == torch::kInt32 ? 1 : 2);
+    return uep_update_placement(group_of(handle), layer, kind, in.ptr, in.rows, static_cast<int>(in.first.size(1)), current_stream());
+}
+
+std::tuple<int, uintptr_t> group_weight_sync(uintptr_t handle, int layer, const py::object& fc1, const py::object& fc2,
+                                             const py::object& fc1_scale, const py::object& fc2_scale, bool async_finish) {
+    const RankList a(fc1), b(fc2), c(fc1_scale), d(fc2_scale);
+    uep_event* done = nullptr;
+    const int rc = uep_weight_sync(group_of(handle), layer, tables_of(a), tables_of(b), tables_of(c), tables_of(d), nullptr, async_finish,
+                                   current_stream(), &done);
+    return {rc, reinterpret_cast<uintptr_t>(done)};
+}
+
+std::tuple<int, uintptr_t> group_grad_reduce(uintptr_t handle, int layer, const py::object& fc1, const py::object& fc2, bool async_finish) {
+    const RankList a(fc1), b(fc2);
+    uep_event* done = nullptr;
+    const int rc = uep_grad_reduce(group_of(handle), layer, tables_of(a), tables_of(b), nullptr, async_finish, current_stream(), &done);
+    return {rc, reinterpret_cast<uintptr_t>(done)};
+}
+
+int group_wait_event(uintptr_t event) {
+    uep_event* ev = reinterpret_cast<uep_event*>(event);
+    const int rc = uep_event_stream_wait(ev, current_stream());
+    if (rc == UEP_OK) uep_event_destroy(ev);
+    return rc;
+}
+
+std::tuple<int, py::object> group_reroute_sparse(uintptr_t handle, int layer, const py::object& ids, py::object out) {
+    const RankList in(ids);
+    if (out.is_none()) {
+        py::list made;
+        for (const auto& item : py::reinterpret_borrow<py::sequence>(ids)) made.append(torch::empty_like(THPVariable_Unpack(item.ptr())));
+        out = made;
+    }
+    const RankList to(out);
+    const int kind = in.first.scalar_type() == torch::kInt32 ? 1 : 2;
+    const int rc = uep_reroute_sparse(group_of(handle), layer, kind, in.ptr, const_cast<void* const*>(to.ptr), in.rows,
+                                      static_cast<int>(in.first.size(1)), current_stream());
+    return {rc, out};
+}
+
+// One tensor [rows[i], cols] per hosted rank.
+py::list empty_like_ranks(const RankList& like, int64_t cols, torch::ScalarType dtype) {
+    py::list made;
+    for (int i = 0; i < like.n; ++i) made.append(empty_2d(like.rows[i], cols, dtype, like.first.device()));
+    return made;
+}
+
+std::tuple<int, py::object, py::object> group_reroute_dense(uintptr_t handle, int layer, int P, const py::object& maps, const py::object& probs,
+                                                            py::object out_probs, py::object out_maps) {
+    const RankList m(maps), p(probs);
+    if (out_probs.is_none()) {
+        out_maps = empty_like_ranks(m, P, torch::kBool);
+        out_probs = empty_like_ranks(m, P, torch::kFloat32);
+    }
+    const RankList op(out_probs), om(out_maps);
+    const int rc = uep_reroute_dense_forward(group_of(handle), layer, reinterpret_cast<const uint8_t* const*>(m.ptr),
+                                             reinterpret_cast<const float* const*>(p.ptr), reinterpret_cast<uint8_t* const*>(const_cast<void* const*>(om.ptr)),
+                                             reinterpret_cast<float* const*>(const_cast<void* const*>(op.ptr)), m.rows, current_stream());
+    return {rc, out_probs, out_maps};
+}
+
+std::tuple<int, py::object> group_reroute_dense_backward(uintptr_t handle, int layer, int L, int P, const py::object& grads, const py::object& maps,
+                                                         const py::object& expanded_maps) {
+    const RankList g(grads), m(maps), em(expanded_maps);
+    py::object out = empty_like_ranks(m, L, torch::kFloat32);
+    const RankList to(out);
+    const int rc = uep_reroute_dense_backward(group_of(handle), layer, reinterpret_cast<const float* const*>(g.ptr),
+                                              reinterpret_cast<const uint8_t* const*>(m.ptr), reinterpret_cast<const uint8_t* const*>(em.ptr),
+                                              reinterpret_cast<float* const*>(const_cast<void* const*>(to.ptr)), m.rows, P, current_stream());
+    return {rc, out};
+}
 
 // Single-GPU test hooks with the reference's signatures (csrc/ultra_ep.hpp:427-612).
 std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor>
@@ -486,7 +653,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
 
     py::class_<EventHandle>(m, "EventHandle").def(py::init<>()).def("current_stream_wait", &EventHandle::current_stream_wait);
 
-    py::class_<Manager>(m, "Manager")
+    m.def("group_update_placement", &group_update_placement);
+    m.def("group_weight_sync", &group_weight_sync);
+    m.def("group_grad_reduce", &group_grad_reduce);
+    m.def("group_wait_event", &group_wait_event);
+    m.def("group_reroute_sparse", &group_reroute_sparse);
+    m.def("group_reroute_dense", &group_reroute_dense);
+    m.def("group_reroute_dense_backward", &group_reroute_dense_backward);
+
+    py::class_<Manager, std::shared_ptr<Manager>>(m, "Manager")
         .def(py::init<int, int, int, int64_t, int64_t, int, int, int64_t, int64_t, int, bool, bool, bool, float, bool,
                       int32_t, bool, float, int, bool, int, bool, int, int, int, int>(),
              py::arg("num_layers"), py::arg("num_local_master_experts"), py::arg("num_local_redundant_experts"),
@@ -507,6 +682,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def("update_placement_sparse", &Manager::update_placement_sparse)
         .def("reroute_sparse", &Manager::reroute_sparse)
         .def("dense_reroute_forward", &Manager::dense_reroute_forward)
+        .def("dense_reroute", &dense_reroute, "dense_reroute_forward, differentiable with respect to the probabilities")
         .def("dense_reroute_backward", &Manager::dense_reroute_backward)
         .def("grad_reduce", &Manager::grad_reduce, py::arg("layer_id"), py::arg("local_master_fc1_grad_ptr_tensor"),
              py::arg("local_master_fc2_grad_ptr_tensor"), py::arg("previous_event"), py::arg("async_finish"))

@@ -19,7 +19,6 @@ from .config import load_tuning_from_env
 from .event import EventHandle
 from .native import load
 from .profiling import ExpertLoadProfiler, load_profile_config
-from .reroute import _DenseRerouteFunction
 from .runtime import init_runtime
 from .util import check_dtype, dtype_element_size
 
@@ -317,11 +316,10 @@ class Manager:
                 and self.local_master_fc2_weight_ptr_pool[real] is not None
                 and self.local_master_fc1_weight_scale_ptr_pool[real] is not None
                 and self.local_master_fc2_weight_scale_ptr_pool[real] is not None)
-        with torch.cuda.nvtx.range(f"Launch weight_sync (layer {layer_id})"):
-            event = self.runtime.weight_sync(
-                layer_id, self.local_master_fc1_weight_ptr_pool[real], self.local_master_fc2_weight_ptr_pool[real],
-                self.local_master_fc1_weight_scale_ptr_pool[real], self.local_master_fc2_weight_scale_ptr_pool[real],
-                getattr(previous_event, "event", None), async_finish)
+        event = self.runtime.weight_sync(
+            layer_id, self.local_master_fc1_weight_ptr_pool[real], self.local_master_fc2_weight_ptr_pool[real],
+            self.local_master_fc1_weight_scale_ptr_pool[real], self.local_master_fc2_weight_scale_ptr_pool[real],
+            getattr(previous_event, "event", None), async_finish)
         return EventHandle(event)
 
     def set_weight_sync_plan_mode(self, plan_mode: str):
@@ -340,8 +338,7 @@ class Manager:
         """New replication plan of one virtual layer from this microbatch's routing.
         routing_map: bool [tokens, logical experts]. Collective; every rank derives the same plan."""
         assert layer_id < self.num_alloc_layers
-        with torch.cuda.nvtx.range(f"Update placement (layer {layer_id})"):
-            self.runtime.update_placement(layer_id, routing_map)
+        self.runtime.update_placement(layer_id, routing_map)
         self._record_loads(layer_id)
         if verify_reduced_loads:
             loads = routing_map.sum(dim=0, dtype=torch.int32)
@@ -374,9 +371,8 @@ class Manager:
         if backend != "cuda":
             raise ValueError("Only backend='cuda' is supported; CPU reroute has been removed")
         if self.is_train and probs.requires_grad:
-            return _DenseRerouteFunction.apply(probs, routing_map, self.runtime, layer_id)
-        with torch.cuda.nvtx.range(f"Dense reroute forward (layer {layer_id})"):
-            return self.runtime.dense_reroute_forward(layer_id, probs, routing_map)
+            return self.runtime.dense_reroute(layer_id, probs, routing_map)
+        return self.runtime.dense_reroute_forward(layer_id, probs, routing_map)
 
     def reroute_sparse(self, layer_id: int, topk_ids: torch.Tensor):
         """In place: logical ids [tokens, k] -> physical ids (deterministic, row-major ordinals)."""

@@ -14,6 +14,7 @@ from typing import List, Optional, Sequence
 import torch
 
 from . import capi
+from .native import load
 
 _TYPESTR = {torch.int32: "<i4", torch.uint8: "|u1", torch.float32: "<f4"}
 
@@ -106,6 +107,7 @@ class SimGroup:
         if not torch.cuda.is_available():
             raise capi.UepError("a CUDA device is required; there is no CPU implementation of this library")
         self.lib = capi.lib()
+        self._C = load()
         self.cfg = cfg
         self.N = cfg.num_ranks
         self.M = cfg.num_local_master_experts
@@ -132,18 +134,13 @@ class SimGroup:
         return {k: self.buffer(rank, b)[layer] for k, b in self.PLAN_BUFFERS.items()}
 
     # -- operations ------------------------------------------------------------------
-    @staticmethod
-    def _stream() -> int:
-        return torch.cuda.current_stream().cuda_stream
+    def _address(self) -> int:
+        """The native group, 0 once it is destroyed (which the library refuses)."""
+        return self.handle.value if self.handle else 0
 
     def update_placement(self, layer: int, inputs: Sequence[torch.Tensor]):
         """inputs[r]: bool [T,L] routing map, or int32/int64 [T,K] ids, of rank r."""
-        x0 = inputs[0]
-        kind = 0 if x0.dtype == torch.bool else (1 if x0.dtype == torch.int32 else 2)
-        ptrs = capi.ptr_array([x.data_ptr() for x in inputs])
-        Ts = capi.int_array([int(x.shape[0]) for x in inputs])
-        capi.check(self.lib.uep_update_placement(self.handle, layer, kind, ptrs, Ts, int(x0.shape[1]), self._stream()),
-                   "uep_update_placement")
+        capi.check(self._C.group_update_placement(self._address(), layer, inputs), "uep_update_placement")
 
     def pointer_tables(self, tensors_per_rank: Sequence[Sequence[torch.Tensor]]) -> List[torch.Tensor]:
         """int64 device tables of raw addresses, one per rank (what construct_local_master_ptr_pool builds)."""
@@ -152,57 +149,37 @@ class SimGroup:
 
     def weight_sync(self, layer: int, fc1_tables, fc2_tables, fc1_scale_tables=None, fc2_scale_tables=None,
                     async_finish: bool = False):
-        args = [capi.ptr_array([t.data_ptr() for t in tabs]) if tabs is not None else None
-                for tabs in (fc1_tables, fc2_tables, fc1_scale_tables, fc2_scale_tables)]
         self._keep = [fc1_tables, fc2_tables, fc1_scale_tables, fc2_scale_tables]
-        done = C.c_void_p()
-        capi.check(self.lib.uep_weight_sync(self.handle, layer, args[0], args[1], args[2], args[3], None,
-                                            int(async_finish), self._stream(), C.byref(done)), "uep_weight_sync")
-        return done if async_finish else None
+        rc, done = self._C.group_weight_sync(self._address(), layer, fc1_tables, fc2_tables, fc1_scale_tables,
+                                             fc2_scale_tables, async_finish)
+        capi.check(rc, "uep_weight_sync")
+        return C.c_void_p(done) if async_finish else None
 
     def grad_reduce(self, layer: int, fc1_grad_tables, fc2_grad_tables, async_finish: bool = False):
-        a = capi.ptr_array([t.data_ptr() for t in fc1_grad_tables])
-        b = capi.ptr_array([t.data_ptr() for t in fc2_grad_tables])
         self._keep = [fc1_grad_tables, fc2_grad_tables]
-        done = C.c_void_p()
-        capi.check(self.lib.uep_grad_reduce(self.handle, layer, a, b, None, int(async_finish), self._stream(),
-                                            C.byref(done)), "uep_grad_reduce")
-        return done if async_finish else None
+        rc, done = self._C.group_grad_reduce(self._address(), layer, fc1_grad_tables, fc2_grad_tables, async_finish)
+        capi.check(rc, "uep_grad_reduce")
+        return C.c_void_p(done) if async_finish else None
 
     def wait_event(self, ev):
-        capi.check(self.lib.uep_event_stream_wait(ev, self._stream()), "uep_event_stream_wait")
-        self.lib.uep_event_destroy(ev)
+        capi.check(self._C.group_wait_event(ev.value or 0), "uep_event_stream_wait")
 
     def reroute_sparse(self, layer: int, ids: Sequence[torch.Tensor], out: Optional[Sequence[torch.Tensor]] = None):
-        out = [torch.empty_like(x) for x in ids] if out is None else out
-        kind = 1 if ids[0].dtype == torch.int32 else 2
-        capi.check(self.lib.uep_reroute_sparse(
-            self.handle, layer, kind, capi.ptr_array([x.data_ptr() for x in ids]),
-            capi.ptr_array([x.data_ptr() for x in out]), capi.int_array([int(x.shape[0]) for x in ids]),
-            int(ids[0].shape[1]), self._stream()), "uep_reroute_sparse")
+        rc, out = self._C.group_reroute_sparse(self._address(), layer, ids, out)
+        capi.check(rc, "uep_reroute_sparse")
         return out
 
     def reroute_dense(self, layer: int, maps: Sequence[torch.Tensor], probs: Sequence[torch.Tensor], out=None):
         """out: optional (out_probs, out_maps) lists to write into instead of allocating."""
-        if out is None:
-            out_maps = [torch.empty((m.shape[0], self.P), dtype=torch.bool, device=self.device) for m in maps]
-            out_probs = [torch.empty((m.shape[0], self.P), dtype=torch.float32, device=self.device) for m in maps]
-        else:
-            out_probs, out_maps = out
-        capi.check(self.lib.uep_reroute_dense_forward(
-            self.handle, layer, capi.ptr_array([x.data_ptr() for x in maps]),
-            capi.ptr_array([x.data_ptr() for x in probs]), capi.ptr_array([x.data_ptr() for x in out_maps]),
-            capi.ptr_array([x.data_ptr() for x in out_probs]), capi.int_array([int(x.shape[0]) for x in maps]),
-            self._stream()), "uep_reroute_dense_forward")
+        out_probs, out_maps = out if out is not None else (None, None)
+        rc, out_probs, out_maps = self._C.group_reroute_dense(self._address(), layer, self.P, maps, probs, out_probs,
+                                                              out_maps)
+        capi.check(rc, "uep_reroute_dense_forward")
         return out_probs, out_maps
 
     def reroute_dense_backward(self, layer: int, grads, maps, expanded_maps):
-        outs = [torch.empty((m.shape[0], self.L), dtype=torch.float32, device=self.device) for m in maps]
-        capi.check(self.lib.uep_reroute_dense_backward(
-            self.handle, layer, capi.ptr_array([x.data_ptr() for x in grads]),
-            capi.ptr_array([x.data_ptr() for x in maps]), capi.ptr_array([x.data_ptr() for x in expanded_maps]),
-            capi.ptr_array([x.data_ptr() for x in outs]), capi.int_array([int(x.shape[0]) for x in maps]), self.P,
-            self._stream()), "uep_reroute_dense_backward")
+        rc, outs = self._C.group_reroute_dense_backward(self._address(), layer, self.L, self.P, grads, maps, expanded_maps)
+        capi.check(rc, "uep_reroute_dense_backward")
         return outs
 
     def status(self, rank: int = 0):
