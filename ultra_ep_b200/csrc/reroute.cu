@@ -9,15 +9,14 @@
 //   * sparse: one launch (ordinals.cuh); a cluster of CTAs keeps its entries in registers and
 //     counts again what lies in front of it;
 //   * dense: pass 1 counts per (tile, expert) from coalesced row reads; pass 2 turns the counts of
-//     the preceding tiles into a base per expert, resolves ordinals inside the tile in row-major
-//     order (the map tile is staged in shared memory, one thread per expert walks its column only
-//     to count, and the replica arithmetic runs over the marked cells spread over the CTA), and
-//     writes every output element exactly once with coalesced vector stores (zeros included), so no
-//     pre-zeroing pass exists.
+//     the preceding tiles into a base per expert, holds the tile as bit columns, turns logical
+//     columns into physical ones and writes every output element exactly once out of registers
+//     (zeros included), so no pre-zeroing pass exists.
 // Results equal the reference's dense rule bit for bit; the sparse form applies the same
 // rule per (token, k) entry and therefore is deterministic, which the reference's
 // atomic-counter sparse kernel (reroute.cu:492-515) is not.
 
+#include <algorithm>
 #include <climits>
 #include <cstdlib>
 #include <mutex>
@@ -32,6 +31,7 @@ namespace uep {
 namespace {
 
 constexpr int kRerouteThreads = 256;
+constexpr size_t kMaxCtaSmem = 225 * 1024;  // of a CTA
 constexpr int kDenseTileRows = 64;
 constexpr int kSparseTileEntries = 2048;  // entries of a row of the count table (at least)
 
@@ -44,442 +44,10 @@ __device__ __forceinline__ int interleave_stride(int total) {
     return total == 2 ? 1 : h + 1 + (((total & 1) == 0 && (h & 1)) ? 1 : 0);
 }
 
-// Per-expert routing parameters (csrc/kernels/reroute.cu:182-209 of the reference).
-struct Router {
-    int C, total, stride, offset;
-};
-
-// (ordinal * stride + offset) mod total; all operands are non-negative. The product fits 32 bits for every
-// realistic token count, where the remainder is one hardware-assisted division instead of the 64-bit routine.
-__device__ __forceinline__ int mod_product(int ordinal, int stride, int offset, int total) {
-    const unsigned long long prod = static_cast<unsigned long long>(static_cast<unsigned>(ordinal)) * static_cast<unsigned>(stride) +
-                                    static_cast<unsigned>(offset);
-    if ((prod >> 32) == 0) return static_cast<int>(static_cast<unsigned>(prod) % static_cast<unsigned>(total));
-    return static_cast<int>(prod % static_cast<unsigned long long>(total));
-}
-
-// ordinal -> replica index (reroute.cu:239-254 of the reference; round-robin: :126). `prefix` is the expert's
-// row of inclusive rank-quota prefixes (at least C entries).
-__device__ __forceinline__ int replica_index(const Router& r, int ordinal, const int32_t* prefix, bool quota_mode) {
-    if (r.C <= 1) return 0;  // one instance: every branch below ends at index 0
-    if (!quota_mode) return ordinal % r.C;
-    int qr = ordinal;
-    if (r.stride != 0) qr = mod_product(ordinal, r.stride, r.offset, r.total);
-    int idx = 0;
-    for (int j = 0; j < r.C; ++j) idx += (qr >= prefix[j]) ? 1 : 0;
-    return min(idx, max(r.C - 1, 0));
-}
-
 // The first kStagedReps entries of every expert's plan rows (rank-quota prefixes and physical ids) are copied
 // into shared memory once per CTA: resolving an entry then costs no global load. Experts with more instances
 // than that read their rows from global memory.
 constexpr int kStagedReps = 8;
-
-// Thread-per-expert set-up: routing parameters and the staged rows; every global load of an expert is issued
-// before the first one is used (two dependent round trips in all: the count, then the rows).
-__device__ __forceinline__ void stage_expert(int e, const int32_t* __restrict__ lcnts, const int32_t* __restrict__ rqp,
-                                             const int32_t* __restrict__ l2p, int D, bool quota_mode, bool interleave,
-                                             Router* routers, int32_t* prefix_s, int32_t* l2p_s) {
-    Router r;
-    r.C = lcnts[e];
-    const int n = min(min(r.C, D), kStagedReps);
-    int32_t pre[kStagedReps], phys[kStagedReps];
-    int last = 0;
-#pragma unroll
-    for (int j = 0; j < kStagedReps; ++j) {
-        pre[j] = (j < n && quota_mode) ? rqp[static_cast<int64_t>(e) * D + j] : 0;
-        phys[j] = j < n ? l2p[static_cast<int64_t>(e) * D + j] : -1;
-    }
-    if (quota_mode && r.C > kStagedReps) last = rqp[static_cast<int64_t>(e) * D + r.C - 1];
-#pragma unroll
-    for (int j = 0; j < kStagedReps; ++j) {
-        prefix_s[e * kStagedReps + j] = pre[j];
-        l2p_s[e * kStagedReps + j] = phys[j];
-        if (j == r.C - 1) last = pre[j];
-    }
-    r.total = (quota_mode && r.C > 0) ? last : 0;
-    r.stride = 0;  // marks "no interleave"
-    r.offset = 0;
-    if (quota_mode && interleave && r.total > 1) {
-        r.stride = interleave_stride(r.total);
-        r.offset = e % r.total;
-    }
-    routers[e] = r;
-}
-
-// ----------------------------------------------------------------------------- dense
-// Copies rows [r0, r1) of the bool map into shared memory, 16 bytes per thread when the tile starts on a
-// 16-byte boundary. The per-expert walks below then run over shared memory: walking a column of the map in
-// global memory costs one dependent memory round trip per row.
-__device__ __forceinline__ void stage_map_tile(const uint8_t* __restrict__ map, int r0, int r1, int L, uint8_t* smap) {
-    const int64_t first = static_cast<int64_t>(r0) * L;
-    const int bytes = (r1 - r0) * L;
-    const uint8_t* src = map + first;
-    int done = 0;
-    if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
-        const int nvec = bytes / 16;
-        for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
-            reinterpret_cast<uint4*>(smap)[i] = ld_global_nc_v4(src + static_cast<int64_t>(i) * 16);
-        }
-        done = nvec * 16;
-    }
-    for (int i = done + threadIdx.x; i < bytes; i += blockDim.x) smap[i] = src[i];
-}
-
-// The count of a (tile, expert) pair is at most kDenseTileRows = 64: it is kept in ONE BYTE, row-major
-// [tile][L] in the scratch buffer, so that the second kernel can add up the tiles in front of it sixteen
-// experts per load. `fast`: L is a multiple of 16 with L/16 in {1,2,4,...,32}, the map and the scratch are
-// 16-byte aligned: a thread then always meets the same sixteen columns and can add map bytes as packed words.
-__device__ __forceinline__ bool dense_fast_path(const uint8_t* map, const void* scratch, int L) {
-    const int G = L / 16;
-    return (L % 16 == 0) && G <= 32 && (G & (G - 1)) == 0 &&
-           ((reinterpret_cast<uintptr_t>(map) | reinterpret_cast<uintptr_t>(scratch)) & 15u) == 0;
-}
-
-__global__ void __launch_bounds__(kRerouteThreads) dense_count_kernel(Batch<DenseFwdArgs> batch, int L) {
-    pdl_launch_dependents();  // the scatter kernel may start its prologue now
-    extern __shared__ __align__(128) char smem_raw[];  // fast: [L/4] packed words; else [kDenseTileRows][L] bytes
-    const DenseFwdArgs& a = batch.a[blockIdx.y];
-    const int T = a.T;
-    const int tile = blockIdx.x;
-    const int r0 = tile * kDenseTileRows, r1 = min(r0 + kDenseTileRows, T);
-    if (r0 >= T) return;
-    uint8_t* counts = reinterpret_cast<uint8_t*>(a.scratch) + static_cast<int64_t>(tile) * L;
-    if (dense_fast_path(a.map, a.scratch, L)) {
-        const int G = L / 16;
-        uint32_t* cnt = reinterpret_cast<uint32_t*>(smem_raw);
-        for (int i = threadIdx.x; i < L / 4; i += blockDim.x) cnt[i] = 0;
-        __syncthreads();
-        // vector i of the tile covers row i / G, columns 16 * (i % G) ..; blockDim is a multiple of G, so a
-        // thread always meets the same column group and adds the 0/1 bytes of its rows as packed words
-        const uint8_t* src = a.map + static_cast<int64_t>(r0) * L;
-        const int nvec = (r1 - r0) * G;
-        uint4 acc = make_uint4(0, 0, 0, 0);
-        for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
-            const uint4 v = ld_global_nc_v4(src + static_cast<int64_t>(i) * 16);
-            acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-        }
-        // lanes with the same column group inside the warp
-        for (int d = G; d < 32; d <<= 1) {
-            acc.x += __shfl_xor_sync(kFullMask, acc.x, d); acc.y += __shfl_xor_sync(kFullMask, acc.y, d);
-            acc.z += __shfl_xor_sync(kFullMask, acc.z, d); acc.w += __shfl_xor_sync(kFullMask, acc.w, d);
-        }
-        const int lane = threadIdx.x & 31;
-        if (lane < G) {  // a byte never exceeds 64, so packed adds cannot carry into the next byte
-            atomicAdd(cnt + lane * 4 + 0, acc.x); atomicAdd(cnt + lane * 4 + 1, acc.y);
-            atomicAdd(cnt + lane * 4 + 2, acc.z); atomicAdd(cnt + lane * 4 + 3, acc.w);
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < L / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(counts)[i] = cnt[i];
-        return;
-    }
-    uint8_t* smap = reinterpret_cast<uint8_t*>(smem_raw);
-    stage_map_tile(a.map, r0, r1, L, smap);
-    __syncthreads();
-    for (int e = threadIdx.x; e < L; e += blockDim.x) {
-        int c = 0;
-        for (int t = 0; t < r1 - r0; ++t) c += smap[t * L + e] ? 1 : 0;
-        counts[e] = static_cast<uint8_t>(c);
-    }
-}
-
-// Second kernel: one CTA per tile of 64 tokens builds the tile of both outputs in shared memory (zeros,
-// then the tile's routed cells: 64 x top-k of them, against 64 x P output elements) and writes it out with
-// bulk stores. Only the probabilities of routed cells are read. Outputs wider than kDenseMaxChunkCols
-// columns are produced in column chunks.
-constexpr int kDenseMaxChunkCols = 512;
-
-// Row stride of the staged map tile: 16 bytes of padding keep the row starts 16-byte aligned and spread the
-// rows over the shared-memory banks when a thread per row walks across the columns.
-__host__ __device__ __forceinline__ int dense_row_stride(int L) { return (L + 15) / 16 * 16 + 16; }
-
-__global__ void __launch_bounds__(kRerouteThreads)
-dense_scatter_kernel(Batch<DenseFwdArgs> batch, int L, int P, int D, int quota_mode, int interleave, int chunk_cols,
-                     int overlapped) {
-    const DenseFwdArgs& a = batch.a[blockIdx.y];
-    const uint8_t* __restrict__ map = a.map;
-    const float* __restrict__ probs = a.probs;
-    const int32_t* __restrict__ l2p = a.l2p;
-    const int32_t* __restrict__ lcnts = a.lcnts;
-    const int32_t* __restrict__ rqp = a.rqp;
-    uint8_t* __restrict__ out_map = a.out_map;
-    float* __restrict__ out_probs = a.out_probs;
-    const int T = a.T;
-    if (static_cast<int>(blockIdx.x) * kDenseTileRows >= T) return;
-    extern __shared__ __align__(128) char smem_raw[];
-    // layout: probs tile [64][chunk] f32 | map tile [64][chunk] u8 | choice [64][Ls] u8 | routers[L] | base[L] i32 |
-    //         prefix rows [L][8] i32 | l2p rows [L][8] i32
-    const int Ls = dense_row_stride(L);
-    float* tile_probs = reinterpret_cast<float*>(smem_raw);
-    uint8_t* tile_map = reinterpret_cast<uint8_t*>(tile_probs + static_cast<size_t>(kDenseTileRows) * chunk_cols);
-    uint8_t* choice = tile_map + (static_cast<size_t>(kDenseTileRows) * chunk_cols + 15) / 16 * 16;
-    Router* routers = reinterpret_cast<Router*>(choice + static_cast<size_t>(kDenseTileRows) * Ls);
-    int32_t* base_of = reinterpret_cast<int32_t*>(routers + L);
-    int32_t* prefix_s = base_of + (L + 3) / 4 * 4;
-    int32_t* l2p_s = prefix_s + static_cast<size_t>(L) * kStagedReps;
-
-    const int tile = blockIdx.x;
-    const int r0 = tile * kDenseTileRows, r1 = min(r0 + kDenseTileRows, T);
-    const int rows = r1 - r0;
-    const int tid = threadIdx.x;
-
-    auto zero_tile = [&](int cols) {  // both output tiles of the chunk (16-byte stores; the regions are padded)
-        uint4* z = reinterpret_cast<uint4*>(tile_probs);
-        const int n1 = (rows * cols * 4 + 15) / 16;
-        for (int i = tid; i < n1; i += blockDim.x) z[i] = make_uint4(0, 0, 0, 0);
-        uint4* zm = reinterpret_cast<uint4*>(tile_map);
-        const int n2 = (rows * cols + 15) / 16;
-        for (int i = tid; i < n2; i += blockDim.x) zm[i] = make_uint4(0, 0, 0, 0);
-    };
-
-    // ---- prologue: nothing here depends on the count kernel ---------------------------------
-    // the map tile, row by row into the padded rows (the passes below turn each map byte into its replica choice in place)
-    {
-        const uint8_t* src = map + static_cast<int64_t>(r0) * L;
-        if ((L % 16) == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
-            const int G = L / 16;
-            for (int i = tid; i < rows * G; i += blockDim.x) {
-                const int t = i / G, g = i - t * G;
-                *reinterpret_cast<uint4*>(choice + t * Ls + g * 16) = ld_global_nc_v4(src + static_cast<int64_t>(i) * 16);
-            }
-        } else {
-            for (int i = tid; i < rows * L; i += blockDim.x) {
-                const int t = i / L, e = i - t * L;
-                choice[t * Ls + e] = src[i];
-            }
-        }
-    }
-    for (int e = tid; e < L; e += blockDim.x) {
-        stage_expert(e, lcnts, rqp, l2p, D, quota_mode != 0, interleave != 0, routers, prefix_s, l2p_s);
-        base_of[e] = 0;
-    }
-    {   // the tile's probabilities are needed only after the wait below: ask for their lines now
-        const char* pbase = reinterpret_cast<const char*>(probs + static_cast<int64_t>(r0) * L);
-        const int64_t pbytes = static_cast<int64_t>(rows) * L * 4;
-        for (int64_t off = static_cast<int64_t>(tid) * 128; off < pbytes; off += static_cast<int64_t>(blockDim.x) * 128) {
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(pbase + off));
-        }
-    }
-    zero_tile(min(chunk_cols, P));
-    __syncthreads();
-    // ---- ordinal base of every expert: tokens routed to it in the tiles in front of this one ---
-    const uint8_t* counts = reinterpret_cast<const uint8_t*>(a.scratch);
-    auto sum_earlier_tiles = [&]() {
-    if (dense_fast_path(map, a.scratch, L)) {
-        const int G = L / 16;
-        const int g = tid % G, sub = tid / G, nsub = blockDim.x / G;
-        // bytes are widened to 16-bit lanes; a lane overflows after 1024 tiles of 64 rows, so it is spilled before
-        uint32_t lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
-        const int lane = tid & 31;
-        auto spill = [&]() {
-            // lanes of the warp that hold the same sixteen columns first (their sum stays below 2^16), then one
-            // shared-memory add per column from the first of them
-            for (int d = G; d < 32; d <<= 1) {
-#pragma unroll
-                for (int w = 0; w < 4; ++w) {
-                    lo[w] += __shfl_xor_sync(kFullMask, lo[w], d);
-                    hi[w] += __shfl_xor_sync(kFullMask, hi[w], d);
-                }
-            }
-            if (lane < G) {
-#pragma unroll
-                for (int w = 0; w < 4; ++w) {
-                    const int e = g * 16 + w * 4;
-                    if (lo[w] & 0xFFFFu) atomicAdd(base_of + e, static_cast<int>(lo[w] & 0xFFFFu));
-                    if (hi[w] & 0xFFFFu) atomicAdd(base_of + e + 1, static_cast<int>(hi[w] & 0xFFFFu));
-                    if (lo[w] >> 16) atomicAdd(base_of + e + 2, static_cast<int>(lo[w] >> 16));
-                    if (hi[w] >> 16) atomicAdd(base_of + e + 3, static_cast<int>(hi[w] >> 16));
-                }
-            }
-#pragma unroll
-            for (int w = 0; w < 4; ++w) lo[w] = hi[w] = 0;
-        };
-        // every thread runs the same number of rounds (the shuffles above need the whole warp)
-        const int rounds = (tile + 4 * nsub - 1) / (4 * nsub);
-        int since = 0;
-        for (int rd = 0; rd < rounds; ++rd) {
-            const int tl0 = sub + rd * 4 * nsub;
-            uint4 v[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {  // four independent loads in flight
-                const int tl = tl0 + u * nsub;
-                v[u] = tl < tile ? __ldcg(reinterpret_cast<const uint4*>(counts + static_cast<int64_t>(tl) * L) + g)
-                                 : make_uint4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const uint32_t w4[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
-#pragma unroll
-                for (int w = 0; w < 4; ++w) {
-                    lo[w] += w4[w] & 0x00FF00FFu;
-                    hi[w] += (w4[w] >> 8) & 0x00FF00FFu;
-                }
-            }
-            since += 4;
-            if (since >= 4 * G) {  // at most (4G + 4) counts of at most 64 per lane, times 32 / G lanes in the shuffle: < 2^15
-                spill();
-                since = 0;
-            }
-        }
-        spill();
-    } else {
-        for (int e = tid; e < L; e += blockDim.x) {
-            int b = 0;
-#pragma unroll 8
-            for (int tl = 0; tl < tile; ++tl) b += __ldcg(counts + static_cast<int64_t>(tl) * L + e);
-            base_of[e] = b;
-        }
-    }
-    };
-    // Launched behind the count kernel in the ordinary way, its counts are complete already and their loads go out
-    // before the column walk; launched as a dependent kernel, everything up to the wait reads the map and the plan only.
-    if (!overlapped) sum_earlier_tiles();
-    // one thread per expert walks its column only to count: a routed cell of an expert with several instances
-    // is marked 0x80 | (its rank among the tile's routed rows, < 64); with one instance the choice is 0 at once
-    for (int e = tid; e < L; e += blockDim.x) {
-        const int C = routers[e].C;
-        int seen = 0;
-        for (int t = 0; t < rows; ++t) {
-            uint8_t c = 0xFF;
-            if (choice[t * Ls + e]) {
-                c = C <= 1 ? 0 : static_cast<uint8_t>(0x80 | seen);
-                ++seen;
-            }
-            choice[t * Ls + e] = c;
-        }
-    }
-
-    if (overlapped) {
-        pdl_wait();
-        sum_earlier_tiles();
-    }
-    __syncthreads();
-
-    // ---- resolve the marked cells and scatter the routed cells into the output tile. A thread owns one row
-    //      and every (blockDim / rows)-th word of it: a row has top-k routed cells, so the work is even however
-    //      skewed the experts are (a hot expert's column is spread over all rows' threads). --------------------
-    const int words_per_row = (L + 3) / 4;
-    const int row_threads = blockDim.x / kDenseTileRows;  // 4
-    const int my_row = tid % kDenseTileRows, my_first = tid / kDenseTileRows;
-    for (int p_lo = 0; p_lo < P; p_lo += chunk_cols) {
-        const int cols = min(chunk_cols, P - p_lo);
-        if (p_lo > 0) {
-            __syncthreads();  // the previous chunk has left the tile
-            zero_tile(cols);
-            __syncthreads();
-        }
-        if (my_row < rows) {
-            const float* prow = probs + static_cast<int64_t>(r0 + my_row) * L;
-            for (int wd = my_first; wd < words_per_row; wd += row_threads) {
-                const uint32_t word = *reinterpret_cast<const uint32_t*>(choice + my_row * Ls + wd * 4);
-                if (word == 0xFFFFFFFFu) continue;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    uint8_t c = static_cast<uint8_t>(word >> (8 * k));
-                    const int e = wd * 4 + k;
-                    if (c == 0xFF || e >= L) continue;
-                    const float pv = prow[e];  // issued before the arithmetic below
-                    const Router r = routers[e];
-                    if (p_lo == 0 && c >= 0x80) {
-                        const int32_t* prefix = r.C <= kStagedReps ? prefix_s + e * kStagedReps : rqp + static_cast<int64_t>(e) * D;
-                        c = static_cast<uint8_t>(replica_index(r, base_of[e] + (c & 0x3F), prefix, quota_mode != 0));
-                        choice[my_row * Ls + e] = c;
-                    }
-                    const int phys = c < kStagedReps ? l2p_s[e * kStagedReps + c] : l2p[static_cast<int64_t>(e) * D + c];
-                    const int p = phys - p_lo;
-                    if (p >= 0 && p < cols) {
-                        tile_probs[my_row * cols + p] = pv;
-                        tile_map[my_row * cols + p] = 1;
-                    }
-                }
-            }
-        }
-        fence_proxy_async_smem();  // the tile was written with ordinary stores and may leave through bulk stores
-        __syncthreads();
-        // ---- the tile leaves: one bulk store per output when it is a contiguous, 16-byte aligned block ----
-        const int64_t o = static_cast<int64_t>(r0) * P;
-        const bool whole = cols == P;
-        const bool bulk_p = whole && ((rows * P) % 4 == 0) && ((reinterpret_cast<uintptr_t>(out_probs + o) & 15u) == 0);
-        const bool bulk_m = whole && ((rows * P) % 16 == 0) && ((reinterpret_cast<uintptr_t>(out_map + o) & 15u) == 0);
-        if ((bulk_p || bulk_m) && tid == 0) {
-            if (bulk_p) bulk_store(out_probs + o, tile_probs, static_cast<uint32_t>(rows * P * 4));
-            if (bulk_m) bulk_store(out_map + o, tile_map, static_cast<uint32_t>(rows * P));
-            bulk_commit();
-        }
-        if (!bulk_p) {
-            for (int i = tid; i < rows * cols; i += blockDim.x) {
-                const int t = i / cols, p = i - t * cols;
-                out_probs[o + static_cast<int64_t>(t) * P + p_lo + p] = tile_probs[i];
-            }
-        }
-        if (!bulk_m) {
-            for (int i = tid; i < rows * cols; i += blockDim.x) {
-                const int t = i / cols, p = i - t * cols;
-                out_map[o + static_cast<int64_t>(t) * P + p_lo + p] = tile_map[i];
-            }
-        }
-        if ((bulk_p || bulk_m) && tid == 0) bulk_wait_read<0>();  // shared memory must outlive the stores' reads
-    }
-}
-
-__device__ __forceinline__ float routed_grad(const float* __restrict__ grad_expanded, const uint8_t* __restrict__ expanded_map,
-                                             const int32_t* __restrict__ l2p, const int32_t* __restrict__ lcnts, int64_t t,
-                                             int l, int P, int D) {
-    const int C = lcnts[l];
-    for (int r = 0; r < C; ++r) {
-        const int phys = l2p[static_cast<int64_t>(l) * D + r];
-        if (expanded_map[t * P + phys]) return grad_expanded[t * P + phys];
-    }
-    return 0.f;
-}
-
-// One thread per four logical experts of a token when the rows allow it (L a multiple of 4, map rows 4-byte and
-// gradient rows 16-byte aligned): the routing map is read a word at a time and the gradients leave as float4.
-// Most entries are not routed, so the kernel is a zero fill plus a few gathers.
-__global__ void __launch_bounds__(kRerouteThreads) dense_backward_kernel(Batch<DenseBwdArgs> batch, int L, int P, int D) {
-    const DenseBwdArgs& a = batch.a[blockIdx.y];
-    const float* __restrict__ grad_expanded = a.grad_expanded;
-    const uint8_t* __restrict__ map = a.map;
-    const uint8_t* __restrict__ expanded_map = a.expanded_map;
-    const int32_t* __restrict__ l2p = a.l2p;
-    const int32_t* __restrict__ lcnts = a.lcnts;
-    float* __restrict__ grad_probs = a.grad_probs;
-    const int64_t total = static_cast<int64_t>(a.T) * L;
-    const int64_t gtid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int64_t gsize = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    const bool vec = (L % 4 == 0) && ((reinterpret_cast<uintptr_t>(map) & 3u) == 0) &&
-                     ((reinterpret_cast<uintptr_t>(grad_probs) & 15u) == 0);
-    if (vec) {
-        const int groups = L / 4;
-        for (int64_t q = gtid; q < total / 4; q += gsize) {
-            const uint32_t m = __ldg(reinterpret_cast<const uint32_t*>(map) + q);
-            float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (m != 0) {
-                const int64_t t = q / groups;
-                const int l0 = static_cast<int>(q % groups) * 4;
-                if (m & 0x000000FFu) g.x = routed_grad(grad_expanded, expanded_map, l2p, lcnts, t, l0, P, D);
-                if (m & 0x0000FF00u) g.y = routed_grad(grad_expanded, expanded_map, l2p, lcnts, t, l0 + 1, P, D);
-                if (m & 0x00FF0000u) g.z = routed_grad(grad_expanded, expanded_map, l2p, lcnts, t, l0 + 2, P, D);
-                if (m & 0xFF000000u) g.w = routed_grad(grad_expanded, expanded_map, l2p, lcnts, t, l0 + 3, P, D);
-            }
-            reinterpret_cast<float4*>(grad_probs)[q] = g;
-        }
-        return;
-    }
-    for (int64_t idx = gtid; idx < total; idx += gsize) {
-        float g = 0.f;
-        if (map[idx]) g = routed_grad(grad_expanded, expanded_map, l2p, lcnts, idx / L, static_cast<int>(idx % L), P, D);
-        grad_probs[idx] = g;
-    }
-}
-
-// ---------------------------------------------------------------------------- sparse
-template <typename IdT>
-__global__ void __launch_bounds__(kOrdThreads) sparse_count_kernel(Batch<SparseArgs> batch, int K, int L, int tile_entries) {
-    pdl_launch_dependents();  // the reroute kernel may start on everything that does not read the table
-    const SparseArgs& a = batch.a[blockIdx.y];
-    count_tile<IdT>(static_cast<const IdT*>(a.ids), static_cast<int64_t>(a.T) * K, L, false, tile_entries, a.scratch);
-}
 
 // Routing parameters of an expert as the resolution wants them: a reciprocal for the remainder, and a staged prefix row
 // whose unused entries are never reached, so that the replica index is eight comparisons without a loop bound.
@@ -567,6 +135,550 @@ __device__ __forceinline__ int fast_replica_index(const FastRouter& r, int ordin
         for (int j = 0; j < r.C - 1; ++j) idx += (qr >= rqp_row[j]) ? 1 : 0;
     }
     return idx;
+}
+
+// ----------------------------------------------------------------------------- dense
+// A tile is 64 rows. Its bool map is held as bit columns: byte [s][c] has bit i set where row 8s + i marks column c.
+// Four columns of eight rows come from eight independent 4-byte loads and fit one word, so the map is read once,
+// coalesced, and never staged; the rank of a cell among its column's marked rows is a population count.
+constexpr int kDenseSegs = kDenseTileRows / 8;
+static_assert(kDenseTileRows == 64, "a byte of counts and the 64-bit columns rely on it");
+
+__device__ __forceinline__ uint32_t nonzero_bytes(uint32_t w) {  // 0x01 where a byte of w is not zero
+    return ((((w & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | w) >> 7) & 0x01010101u;
+}
+
+__host__ __device__ __forceinline__ int pad4(int n) { return (n + 3) & ~3; }
+
+// Rows 8s .. 8s+7 (those below `rows`) of columns 4q .. 4q+3 as four bytes of row bits, read with loads of W's size, which
+// the address of the tile's first row and `cols` are multiples of.
+template <typename W>
+__device__ __forceinline__ uint32_t segment_bits(const uint8_t* __restrict__ tile, int rows, int cols, int s, int q) {
+    constexpr int kLoads = 4 / sizeof(W);
+    uint32_t acc = 0;
+#pragma unroll
+    for (int k = 0; k < kLoads; ++k) {
+        const int c = 4 * q + k * static_cast<int>(sizeof(W));
+        W w[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            w[i] = (8 * s + i < rows && c < cols) ? __ldg(reinterpret_cast<const W*>(tile + static_cast<int64_t>(8 * s + i) * cols + c)) : W(0);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc |= nonzero_bytes(static_cast<uint32_t>(w[i]) << (8 * sizeof(W) * k)) << i;
+    }
+    return acc;
+}
+__device__ __forceinline__ int map_load_bytes(const uint8_t* map, int cols) {
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(map) | static_cast<uintptr_t>(cols);
+    return (bits & 3u) == 0 ? 4 : ((bits & 1u) == 0 ? 2 : 1);
+}
+__device__ __forceinline__ uint32_t segment_bits_any(int load_bytes, const uint8_t* __restrict__ tile, int rows, int cols, int s, int q) {
+    if (load_bytes == 4) return segment_bits<uint32_t>(tile, rows, cols, s, q);
+    if (load_bytes == 2) return segment_bits<uint16_t>(tile, rows, cols, s, q);
+    return segment_bits<uint8_t>(tile, rows, cols, s, q);
+}
+
+// The bit columns of a tile of up to 8 * segs rows into bits[segs][pad4(cols)] (shared memory), all threads of the CTA.
+__device__ __forceinline__ void tile_bit_columns(const uint8_t* __restrict__ tile, int rows, int segs, int cols, uint8_t* bits) {
+    const int quads = pad4(cols) / 4, load_bytes = map_load_bytes(tile, cols);
+    for (int i = threadIdx.x; i < quads * segs; i += blockDim.x) {
+        const int s = i / quads, q = i - s * quads;
+        reinterpret_cast<uint32_t*>(bits)[i] = segment_bits_any(load_bytes, tile, rows, cols, s, q);
+    }
+}
+
+// The count of a (tile, expert) pair is at most kDenseTileRows = 64: it is kept in ONE BYTE, row-major
+// [tile][L] in the scratch buffer, so that the second kernel can add up the tiles in front of it sixteen
+// experts per load. `fast`: L is a multiple of 16 with L/16 in {1,2,4,...,32}, the map and the scratch are
+// 16-byte aligned: a thread then always meets the same sixteen columns and can add map bytes as packed words.
+__device__ __forceinline__ bool dense_fast_path(const uint8_t* map, const void* scratch, int L) {
+    const int G = L / 16;
+    return (L % 16 == 0) && G <= 32 && (G & (G - 1)) == 0 &&
+           ((reinterpret_cast<uintptr_t>(map) | reinterpret_cast<uintptr_t>(scratch)) & 15u) == 0;
+}
+
+__global__ void __launch_bounds__(kRerouteThreads) dense_count_kernel(Batch<DenseFwdArgs> batch, int L) {
+    pdl_launch_dependents();  // the scatter kernel may start its prologue now
+    extern __shared__ __align__(128) char smem_raw[];  // [pad4(L)] counts, one byte each
+    const DenseFwdArgs& a = batch.a[blockIdx.y];
+    const int T = a.T;
+    const int tile = blockIdx.x;
+    const int r0 = tile * kDenseTileRows, r1 = min(r0 + kDenseTileRows, T);
+    if (r0 >= T) return;
+    uint8_t* counts = reinterpret_cast<uint8_t*>(a.scratch) + static_cast<int64_t>(tile) * L;
+    const uint8_t* src = a.map + static_cast<int64_t>(r0) * L;
+    uint32_t* cnt = reinterpret_cast<uint32_t*>(smem_raw);
+    for (int i = threadIdx.x; i < pad4(L) / 4; i += blockDim.x) cnt[i] = 0;
+    __syncthreads();
+    // a byte never exceeds 64, so the packed adds below cannot carry into the next byte
+    if (dense_fast_path(a.map, a.scratch, L)) {
+        const int G = L / 16;
+        // vector i of the tile covers row i / G, columns 16 * (i % G) ..; blockDim is a multiple of G, so a
+        // thread always meets the same column group and adds the 0/1 bytes of its rows as packed words
+        const int nvec = (r1 - r0) * G;
+        uint4 acc = make_uint4(0, 0, 0, 0);
+#pragma unroll 4
+        for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
+            const uint4 v = ld_global_nc_v4(src + static_cast<int64_t>(i) * 16);
+            acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+        }
+        // lanes with the same column group inside the warp
+        for (int d = G; d < 32; d <<= 1) {
+            acc.x += __shfl_xor_sync(kFullMask, acc.x, d); acc.y += __shfl_xor_sync(kFullMask, acc.y, d);
+            acc.z += __shfl_xor_sync(kFullMask, acc.z, d); acc.w += __shfl_xor_sync(kFullMask, acc.w, d);
+        }
+        const int lane = threadIdx.x & 31;
+        if (lane < G) {
+            atomicAdd(cnt + lane * 4 + 0, acc.x); atomicAdd(cnt + lane * 4 + 1, acc.y);
+            atomicAdd(cnt + lane * 4 + 2, acc.z); atomicAdd(cnt + lane * 4 + 3, acc.w);
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < L / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(counts)[i] = cnt[i];
+        return;
+    }
+    const int quads = pad4(L) / 4;
+    const int load_bytes = map_load_bytes(src, L);
+    for (int i = threadIdx.x; i < quads * kDenseSegs; i += blockDim.x) {
+        const int s = i / quads, q = i - s * quads;
+        const uint32_t b = segment_bits_any(load_bytes, src, r1 - r0, L, s, q);
+        uint32_t packed = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) packed |= static_cast<uint32_t>(__popc((b >> (8 * k)) & 0xFFu)) << (8 * k);
+        if (packed) atomicAdd(cnt + q, packed);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < L; e += blockDim.x) counts[e] = reinterpret_cast<const uint8_t*>(cnt)[e];
+}
+
+// Adds the counts of the tiles in front of `tile` to base_of[L] (shared memory, zeroed), all threads of the CTA.
+__device__ __forceinline__ void sum_earlier_tiles(const DenseFwdArgs& a, int L, int tile, int32_t* base_of) {
+    const uint8_t* counts = reinterpret_cast<const uint8_t*>(a.scratch);
+    const int tid = threadIdx.x;
+    if (dense_fast_path(a.map, a.scratch, L)) {
+        const int G = L / 16;
+        const int g = tid % G, sub = tid / G, nsub = blockDim.x / G;
+        // bytes are widened to 16-bit lanes; a lane overflows after 1024 tiles of 64 rows, so it is spilled before
+        uint32_t lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
+        const int lane = tid & 31;
+        auto spill = [&]() {
+            // lanes of the warp that hold the same sixteen columns first (their sum stays below 2^16), then one
+            // shared-memory add per column from the first of them
+            for (int d = G; d < 32; d <<= 1) {
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    lo[w] += __shfl_xor_sync(kFullMask, lo[w], d);
+                    hi[w] += __shfl_xor_sync(kFullMask, hi[w], d);
+                }
+            }
+            if (lane < G) {
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    const int e = g * 16 + w * 4;
+                    if (lo[w] & 0xFFFFu) atomicAdd(base_of + e, static_cast<int>(lo[w] & 0xFFFFu));
+                    if (hi[w] & 0xFFFFu) atomicAdd(base_of + e + 1, static_cast<int>(hi[w] & 0xFFFFu));
+                    if (lo[w] >> 16) atomicAdd(base_of + e + 2, static_cast<int>(lo[w] >> 16));
+                    if (hi[w] >> 16) atomicAdd(base_of + e + 3, static_cast<int>(hi[w] >> 16));
+                }
+            }
+#pragma unroll
+            for (int w = 0; w < 4; ++w) lo[w] = hi[w] = 0;
+        };
+        // every thread runs the same number of rounds (the shuffles above need the whole warp)
+        const int rounds = (tile + 4 * nsub - 1) / (4 * nsub);
+        int since = 0;
+        for (int rd = 0; rd < rounds; ++rd) {
+            const int tl0 = sub + rd * 4 * nsub;
+            uint4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {  // four independent loads in flight
+                const int tl = tl0 + u * nsub;
+                v[u] = tl < tile ? __ldcg(reinterpret_cast<const uint4*>(counts + static_cast<int64_t>(tl) * L) + g)
+                                 : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint32_t w4[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    lo[w] += w4[w] & 0x00FF00FFu;
+                    hi[w] += (w4[w] >> 8) & 0x00FF00FFu;
+                }
+            }
+            since += 4;
+            if (since >= 4 * G) {  // at most (4G + 4) counts of at most 64 per lane, times 32 / G lanes in the shuffle: < 2^15
+                spill();
+                since = 0;
+            }
+        }
+        spill();
+        return;
+    }
+    if (L % 4 == 0 && (reinterpret_cast<uintptr_t>(counts) & 3u) == 0) {
+        // other widths: a word of four columns per thread, the tiles shared among the threads of a word. A thread per
+        // column that walked all tiles was 16 round trips of eight tiles at 8192 rows.
+        const int quads = L / 4, parts = max(static_cast<int>(blockDim.x) / quads, 1);
+        for (int i = tid; i < quads * parts; i += blockDim.x) {
+            const int q = i % quads, part = i / quads;
+            for (int t0 = part; t0 < tile; t0 += 512 * parts) {  // 512 counts of at most 64 fit a 16-bit lane
+                const int t1 = min(t0 + 512 * parts, tile);
+                uint32_t lo = 0, hi = 0;
+                for (int t = t0; t < t1; t += 8 * parts) {
+                    uint32_t v[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        const int tl = t + u * parts;
+                        v[u] = tl < t1 ? __ldcg(reinterpret_cast<const uint32_t*>(counts + static_cast<int64_t>(tl) * L) + q) : 0u;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        lo += v[u] & 0x00FF00FFu;
+                        hi += (v[u] >> 8) & 0x00FF00FFu;
+                    }
+                }
+                atomicAdd(base_of + 4 * q, static_cast<int>(lo & 0xFFFFu));
+                atomicAdd(base_of + 4 * q + 1, static_cast<int>(hi & 0xFFFFu));
+                atomicAdd(base_of + 4 * q + 2, static_cast<int>(lo >> 16));
+                atomicAdd(base_of + 4 * q + 3, static_cast<int>(hi >> 16));
+            }
+        }
+        return;
+    }
+    for (int e = tid; e < L; e += blockDim.x) {
+        int b = 0;
+#pragma unroll 8
+        for (int tl = 0; tl < tile; ++tl) b += __ldcg(counts + static_cast<int64_t>(tl) * L + e);
+        base_of[e] = b;
+    }
+}
+
+// Second kernel: one CTA per tile of 64 tokens. The logical bit columns become physical ones (an expert with one
+// instance: its column is copied; with several: a warp resolves the column's marked rows), and then a thread owns four
+// physical columns of eight rows and writes them out of its registers: a probability is read where its bit is set,
+// zeros are written elsewhere. Shared memory holds bits and plan rows only (15 KB at 128 experts), so eight CTAs fit an
+// SM, and several still do beside a weight_sync CTA. Outputs wider than kDenseMaxChunkCols go in column chunks.
+// Building the output tile in shared memory took 71 KB per CTA and a walk of every column. Kernel time, before and after:
+// 8191 tokens, 256 experts, one rank 18.4 -> 10.3 us; eight ranks of 8192 tokens, 128 experts, beside weight_sync
+// 53..70 -> 38 us (the two share the memory); 4096 tokens, 64 experts 10.4 -> 5.9 us.
+constexpr int kDenseMaxChunkCols = 4096;
+constexpr int kDenseMaxExperts = 1340;
+constexpr int kDenseMaxThreads = 512;
+
+struct DenseShared {
+    int32_t *prefix, *l2p;  // [L][kStagedReps]
+    FastRouter* routers;    // [L]
+    int32_t* base;          // [L] tokens routed to the expert in front of the tile
+    uint8_t* bits;          // [kDenseSegs][pad4(L)]
+    uint8_t* phys_bits;     // [kDenseSegs][pad4(chunk)]
+    uint16_t* expert_of;    // [pad4(chunk)] valid where a bit is set
+    uint16_t* several;      // [L] experts with several instances that the tile routes to
+};
+__host__ __device__ inline size_t dense_smem_bytes(int L, int chunk_cols) {
+    const size_t Lq = pad4(L), Cq = pad4(chunk_cols);
+    return Lq * (2 * kStagedReps * 4 + sizeof(FastRouter) + 4 + kDenseSegs + 2) + Cq * (kDenseSegs + 2);
+}
+__device__ __forceinline__ DenseShared carve_dense_smem(char* raw, int L, int chunk_cols) {
+    const int Lq = pad4(L), Cq = pad4(chunk_cols);
+    DenseShared s;
+    s.prefix = reinterpret_cast<int32_t*>(raw);
+    s.l2p = s.prefix + Lq * kStagedReps;
+    s.routers = reinterpret_cast<FastRouter*>(s.l2p + Lq * kStagedReps);
+    s.base = reinterpret_cast<int32_t*>(s.routers + Lq);
+    s.bits = reinterpret_cast<uint8_t*>(s.base + Lq);
+    s.phys_bits = s.bits + Lq * kDenseSegs;
+    s.expert_of = reinterpret_cast<uint16_t*>(s.phys_bits + Cq * kDenseSegs);
+    s.several = s.expert_of + Cq;
+    return s;
+}
+
+template <int V>
+struct DenseVec;
+template <>
+struct DenseVec<4> {
+    using F = float4;
+    using B = uint32_t;
+};
+template <>
+struct DenseVec<2> {
+    using F = float2;
+    using B = uint16_t;
+};
+template <>
+struct DenseVec<1> {
+    using F = float;
+    using B = uint8_t;
+};
+
+// Columns [p_lo, p_lo + cols) of the tile's rows, V columns and eight rows per thread and turn.
+template <int V>
+__device__ __forceinline__ void write_dense_chunk(const DenseShared& s, const float* __restrict__ probs, float* __restrict__ out_probs,
+                                                  uint8_t* __restrict__ out_map, int rows, int L, int P, int p_lo, int cols) {
+    const int groups = cols / V, Cq = pad4(cols);
+    const int segs = (rows + 7) / 8;
+    for (int i = threadIdx.x; i < groups * segs; i += blockDim.x) {
+        const int seg = i / groups, c = (i - seg * groups) * V;
+        uint32_t bits[V];
+        int e[V];
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+            bits[k] = s.phys_bits[seg * Cq + c + k];
+            e[k] = s.expert_of[c + k];
+        }
+        float v[8][V];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const float* row = probs + static_cast<int64_t>(8 * seg + r) * L;
+#pragma unroll
+            for (int k = 0; k < V; ++k) v[r][k] = (bits[k] >> r) & 1u ? __ldg(row + e[k]) : 0.f;
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            if (8 * seg + r < rows) {
+                const int64_t at = static_cast<int64_t>(8 * seg + r) * P + p_lo + c;
+                uint32_t m = 0;
+#pragma unroll
+                for (int k = 0; k < V; ++k) m |= ((bits[k] >> r) & 1u) << (8 * k);
+                typename DenseVec<V>::F f;
+#pragma unroll
+                for (int k = 0; k < V; ++k) reinterpret_cast<float*>(&f)[k] = v[r][k];
+                *reinterpret_cast<typename DenseVec<V>::F*>(out_probs + at) = f;
+                *reinterpret_cast<typename DenseVec<V>::B*>(out_map + at) = static_cast<typename DenseVec<V>::B>(m);
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kDenseMaxThreads, 2)
+dense_scatter_kernel(Batch<DenseFwdArgs> batch, int L, int P, int D, int quota_mode, int interleave, int chunk_cols,
+                     int overlapped) {
+    const DenseFwdArgs& a = batch.a[blockIdx.y];
+    const int T = a.T;
+    const int tile = blockIdx.x;
+    const int r0 = tile * kDenseTileRows, rows = min(T - r0, kDenseTileRows);
+    if (rows <= 0) return;
+    extern __shared__ __align__(128) char smem_raw[];
+    __shared__ int n_several;
+    const DenseShared s = carve_dense_smem(smem_raw, L, chunk_cols);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, Lq = pad4(L);
+
+    // ---- nothing here depends on the count kernel ------------------------------------------------
+    stage_plan_rows_async(a.lcnts, a.rqp, a.l2p, L, D, quota_mode != 0, s.routers, s.prefix, s.l2p);
+    for (int e = tid; e < L; e += blockDim.x) s.base[e] = 0;
+    for (int i = tid; i < pad4(chunk_cols) / 4 * kDenseSegs; i += blockDim.x) reinterpret_cast<uint32_t*>(s.phys_bits)[i] = 0;
+    if (tid == 0) n_several = 0;
+    tile_bit_columns(a.map + static_cast<int64_t>(r0) * L, rows, kDenseSegs, L, s.bits);
+    cp_async_wait();
+    __syncthreads();
+    for (int e = tid; e < L; e += blockDim.x) {
+        const int C = s.routers[e].C;
+        s.routers[e] = make_fast_router(e, C, a.rqp, D, quota_mode != 0, interleave != 0, s.prefix + e * kStagedReps);
+        if (C > 1) {
+            uint32_t any = 0;
+#pragma unroll
+            for (int g = 0; g < kDenseSegs; ++g) any |= s.bits[g * Lq + e];
+            if (any) s.several[atomicAdd(&n_several, 1)] = static_cast<uint16_t>(e);
+        }
+    }
+    if (overlapped) pdl_wait();
+    sum_earlier_tiles(a, L, tile, s.base);
+    __syncthreads();
+
+    const float* probs = a.probs + static_cast<int64_t>(r0) * L;
+    float* out_probs = a.out_probs + static_cast<int64_t>(r0) * P;
+    uint8_t* out_map = a.out_map + static_cast<int64_t>(r0) * P;
+    for (int p_lo = 0; p_lo < P; p_lo += chunk_cols) {
+        const int cols = min(chunk_cols, P - p_lo), Cq = pad4(cols);
+        if (p_lo > 0) {
+            __syncthreads();
+            for (int i = tid; i < Cq / 4 * kDenseSegs; i += blockDim.x) reinterpret_cast<uint32_t*>(s.phys_bits)[i] = 0;
+            __syncthreads();
+        }
+        for (int i = tid; i < L * kDenseSegs; i += blockDim.x) {  // experts with one instance
+            const int g = i / L, e = i - g * L;
+            if (s.routers[e].C != 1) continue;
+            const int p = s.l2p[e * kStagedReps] - p_lo;
+            const uint8_t b = s.bits[g * Lq + e];
+            if (b != 0 && p >= 0 && p < cols) {
+                s.phys_bits[g * Cq + p] = b;
+                s.expert_of[p] = static_cast<uint16_t>(e);
+            }
+        }
+        __syncthreads();  // the bytes above share words with the atomics below
+        for (int i = warp; i < n_several; i += blockDim.x / kWarp) {
+            const int e = s.several[i];
+            const FastRouter router = s.routers[e];
+            int before = s.base[e];
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {  // lane t: row 32 * half + t
+                uint32_t m = 0;
+#pragma unroll
+                for (int g = 0; g < 4; ++g) m |= static_cast<uint32_t>(s.bits[(4 * half + g) * Lq + e]) << (8 * g);
+                if ((m >> lane) & 1u) {
+                    const int ordinal = before + __popc(m & ((1u << lane) - 1u));
+                    const int j = fast_replica_index(router, ordinal, s.prefix + e * kStagedReps, a.rqp + static_cast<int64_t>(e) * D,
+                                                     quota_mode != 0);
+                    const int p = (j < kStagedReps ? s.l2p[e * kStagedReps + j] : a.l2p[static_cast<int64_t>(e) * D + j]) - p_lo;
+                    if (p >= 0 && p < cols) {
+                        const int seg = 4 * half + lane / 8;
+                        atomicOr(reinterpret_cast<uint32_t*>(s.phys_bits + seg * Cq) + p / 4, 1u << (8 * (p & 3) + (lane & 7)));
+                        s.expert_of[p] = static_cast<uint16_t>(e);
+                    }
+                }
+                before += __popc(m);
+            }
+        }
+        __syncthreads();
+        const uintptr_t fp = reinterpret_cast<uintptr_t>(out_probs), mp = reinterpret_cast<uintptr_t>(out_map);
+        if (P % 4 == 0 && (fp & 15u) == 0 && (mp & 3u) == 0) write_dense_chunk<4>(s, probs, out_probs, out_map, rows, L, P, p_lo, cols);
+        else if (P % 2 == 0 && (fp & 7u) == 0 && (mp & 1u) == 0) write_dense_chunk<2>(s, probs, out_probs, out_map, rows, L, P, p_lo, cols);
+        else write_dense_chunk<1>(s, probs, out_probs, out_map, rows, L, P, p_lo, cols);
+    }
+}
+
+__device__ __forceinline__ float routed_grad(const float* __restrict__ grad_expanded, const uint8_t* __restrict__ expanded_map,
+                                             const int32_t* __restrict__ l2p, const int32_t* __restrict__ lcnts, int64_t t,
+                                             int l, int P, int D) {
+    const int C = lcnts[l];
+    for (int r = 0; r < C; ++r) {
+        const int phys = l2p[static_cast<int64_t>(l) * D + r];
+        if (expanded_map[t * P + phys]) return grad_expanded[t * P + phys];
+    }
+    return 0.f;
+}
+
+// Backward of a tile of `tile_rows` tokens (a multiple of eight, at most 64): the expanded map as bit columns, then four
+// logical columns of eight rows per thread. Which instance a row took is found for eight rows at a time, an AND per
+// instance, and kept as the bit planes of the instance number, so all the gradients a thread needs are asked for at once.
+// It reads the expanded map as a stream where the kernel below fetches a sector per routed cell and instance: 26 us against
+// 35 for eight ranks of 8192 tokens and 128 experts, behind a gradient reduce. (Walking only the set cells of a thread: 33.)
+// Needs L a multiple of four, a 4-byte aligned map and 16-byte aligned gradients.
+constexpr int kDenseBwdThreads = 128;
+constexpr int64_t kDenseBwdTileCells = 1 << 22;
+
+__host__ __device__ inline size_t dense_bwd_smem_bytes(int L, int P) {
+    return static_cast<size_t>(pad4(L)) * (kStagedReps + 1) * 4 + static_cast<size_t>(pad4(P)) * kDenseSegs;
+}
+__global__ void __launch_bounds__(kDenseBwdThreads, 8)
+dense_backward_tile_kernel(Batch<DenseBwdArgs> batch, int L, int P, int D, int tile_rows) {
+    const DenseBwdArgs& a = batch.a[blockIdx.y];
+    const int64_t r0 = static_cast<int64_t>(blockIdx.x) * tile_rows;
+    if (r0 >= a.T) return;
+    const int rows = min(static_cast<int>(a.T - r0), tile_rows);
+    extern __shared__ __align__(128) char smem_raw[];
+    int32_t* l2p_s = reinterpret_cast<int32_t*>(smem_raw);
+    int32_t* count_s = l2p_s + pad4(L) * kStagedReps;
+    uint8_t* bits = reinterpret_cast<uint8_t*>(count_s + pad4(L));
+    const int Pq = pad4(P), quads = L / 4, tasks = quads * ((rows + 7) / 8);  // (the last tile may have fewer)
+    const uint8_t* map = a.map + r0 * L;
+    for (int e = threadIdx.x; e < L; e += blockDim.x) cp_async_4(count_s + e, a.lcnts + e);
+    if (D >= kStagedReps && D % 4 == 0 && (reinterpret_cast<uintptr_t>(a.l2p) & 15u) == 0) {
+        for (int i = threadIdx.x; i < L * (kStagedReps / 4); i += blockDim.x) {
+            cp_async_16(l2p_s + i * 4, a.l2p + static_cast<int64_t>(i / (kStagedReps / 4)) * D + i % (kStagedReps / 4) * 4);
+        }
+    } else {
+        for (int i = threadIdx.x; i < L * kStagedReps; i += blockDim.x) {
+            if (i % kStagedReps < D) cp_async_4(l2p_s + i, a.l2p + static_cast<int64_t>(i / kStagedReps) * D + i % kStagedReps);
+        }
+    }
+    uint32_t word = threadIdx.x < tasks ? segment_bits<uint32_t>(map, rows, L, threadIdx.x / quads, threadIdx.x % quads) : 0u;
+    tile_bit_columns(a.expanded_map + r0 * P, rows, tile_rows / 8, P, bits);
+    cp_async_wait();
+    __syncthreads();
+    for (int i = threadIdx.x; i < tasks; i += blockDim.x) {
+        const int seg = i / quads, q = i - seg * quads;
+        if (i != threadIdx.x) word = segment_bits<uint32_t>(map, rows, L, seg, q);
+        const float* grads = a.grad_expanded + (r0 + 8 * seg) * P;
+        float v[8][4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int l = 4 * q + k;
+            const int32_t* phys_of = l2p_s + l * kStagedReps;
+            uint32_t open = (word >> (8 * k)) & 0xFFu;  // rows that have not found their instance
+            uint32_t found = 0, plane[3] = {0, 0, 0};
+            const int C = open ? count_s[l] : 0;
+#pragma unroll
+            for (int j = 0; j < kStagedReps; ++j) {
+                if (j < C && open) {
+                    const int phys = phys_of[j];
+                    const uint32_t hit = phys >= 0 && phys < P ? open & bits[seg * Pq + phys] : 0u;
+                    open &= ~hit;
+                    found |= hit;
+#pragma unroll
+                    for (int b = 0; b < 3; ++b) plane[b] |= (j >> b) & 1 ? hit : 0u;
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                v[r][k] = 0.f;
+                if ((found >> r) & 1u) {
+                    const int j = ((plane[0] >> r) & 1u) | ((plane[1] >> r) & 1u) << 1 | ((plane[2] >> r) & 1u) << 2;
+                    v[r][k] = __ldg(grads + static_cast<int64_t>(r) * P + phys_of[j]);
+                }
+            }
+            for (int j = kStagedReps; j < C && open; ++j) {  // instances behind the staged ones
+                const int phys = __ldg(a.l2p + static_cast<int64_t>(l) * D + j);
+                const uint32_t hit = phys >= 0 && phys < P ? open & bits[seg * Pq + phys] : 0u;
+                open &= ~hit;
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    if ((hit >> r) & 1u) v[r][k] = __ldg(grads + static_cast<int64_t>(r) * P + phys);
+                }
+            }
+        }
+        float* out = a.grad_probs + (r0 + 8 * seg) * L + 4 * q;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            if (8 * seg + r < rows) *reinterpret_cast<float4*>(out + static_cast<int64_t>(r) * L) = make_float4(v[r][0], v[r][1], v[r][2], v[r][3]);
+        }
+    }
+}
+
+// One thread per four logical experts of a token when the rows allow it (L a multiple of 4, map rows 4-byte and
+// gradient rows 16-byte aligned): the routing map is read a word at a time and the gradients leave as float4.
+// Most entries are not routed, so the kernel is a zero fill plus a few gathers.
+__global__ void __launch_bounds__(kRerouteThreads) dense_backward_kernel(Batch<DenseBwdArgs> batch, int L, int P, int D) {
+    const DenseBwdArgs& a = batch.a[blockIdx.y];
+    const float* __restrict__ grad_expanded = a.grad_expanded;
+    const uint8_t* __restrict__ map = a.map;
+    const uint8_t* __restrict__ expanded_map = a.expanded_map;
+    const int32_t* __restrict__ l2p = a.l2p;
+    const int32_t* __restrict__ lcnts = a.lcnts;
+    float* __restrict__ grad_probs = a.grad_probs;
+    const int64_t total = static_cast<int64_t>(a.T) * L;
+    const int64_t gtid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int64_t gsize = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    const bool vec = (L % 4 == 0) && ((reinterpret_cast<uintptr_t>(map) & 3u) == 0) &&
+                     ((reinterpret_cast<uintptr_t>(grad_probs) & 15u) == 0);
+    if (vec) {
+        const int groups = L / 4;
+        for (int64_t q = gtid; q < total / 4; q += gsize) {
+            const uint32_t m = __ldg(reinterpret_cast<const uint32_t*>(map) + q);
+            float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (m != 0) {
+                const int64_t t = q / groups;
+                const int l0 = static_cast<int>(q % groups) * 4;
+                if (m & 0x000000FFu) g.x = routed_grad(grad_expanded, expanded_map, l2p, lcnts, t, l0, P, D);
+                if (m & 0x0000FF00u) g.y = routed_grad(grad_expanded, expanded_map, l2p, lcnts, t, l0 + 1, P, D);
+                if (m & 0x00FF0000u) g.z = routed_grad(grad_expanded, expanded_map, l2p, lcnts, t, l0 + 2, P, D);
+                if (m & 0xFF000000u) g.w = routed_grad(grad_expanded, expanded_map, l2p, lcnts, t, l0 + 3, P, D);
+            }
+            reinterpret_cast<float4*>(grad_probs)[q] = g;
+        }
+        return;
+    }
+    for (int64_t idx = gtid; idx < total; idx += gsize) {
+        float g = 0.f;
+        if (map[idx]) g = routed_grad(grad_expanded, expanded_map, l2p, lcnts, idx / L, static_cast<int>(idx % L), P, D);
+        grad_probs[idx] = g;
+    }
+}
+
+// ---------------------------------------------------------------------------- sparse
+template <typename IdT>
+__global__ void __launch_bounds__(kOrdThreads) sparse_count_kernel(Batch<SparseArgs> batch, int K, int L, int tile_entries) {
+    pdl_launch_dependents();  // the reroute kernel may start on everything that does not read the table
+    const SparseArgs& a = batch.a[blockIdx.y];
+    count_tile<IdT>(static_cast<const IdT*>(a.ids), static_cast<int64_t>(a.T) * K, L, false, tile_entries, a.scratch);
 }
 
 // shared memory: prefix rows [L][8] i32 | l2p rows [L][8] i32 (both only where they fit) | ordinals | routers[L]
@@ -842,19 +954,11 @@ cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int
     int max_T = 0;
     for (int i = 0; i < b.n; ++i) max_T = b.a[i].T > max_T ? b.a[i].T : max_T;
     if (max_T == 0) return cudaSuccess;
+    // (the limit dates from a kernel that staged the map; a wider one is still refused)
+    if (L > kDenseMaxExperts) return cudaErrorInvalidValue;
     const dim3 grid(dense_tiles(max_T), b.n);
-    static_assert(kDenseTileRows <= 64, "a routed cell's rank inside its tile is kept in six bits");
-    const size_t smem_count = static_cast<size_t>(kDenseTileRows) * L + 16;
-    // shared memory of the scatter kernel: the map tile, the per-expert tables, and as many output columns
-    // (five bytes per row and column) as fit beside them
-    const size_t fixed = static_cast<size_t>(kDenseTileRows) * dense_row_stride(L) + sizeof(Router) * L +
-                         sizeof(int32_t) * ((L + 3) / 4 * 4) + 2 * sizeof(int32_t) * kStagedReps * L + 64;
-    const size_t budget = 200 * 1024;
-    if (fixed + static_cast<size_t>(kDenseTileRows) * 5 * 16 > budget) return cudaErrorInvalidValue;  // L in the thousands
-    int chunk = static_cast<int>((budget - fixed) / (static_cast<size_t>(kDenseTileRows) * 5));
-    chunk = chunk > kDenseMaxChunkCols ? kDenseMaxChunkCols : chunk;
-    chunk = chunk >= P ? P : chunk / 16 * 16;
-    const size_t smem = static_cast<size_t>(kDenseTileRows) * chunk * 4 + (static_cast<size_t>(kDenseTileRows) * chunk + 15) / 16 * 16 + fixed;
+    const int chunk = P > kDenseMaxChunkCols ? kDenseMaxChunkCols : P;
+    const size_t smem_count = pad4(L), smem = dense_smem_bytes(L, chunk);
     cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(dense_scatter_kernel), smem);
     if (e != cudaSuccess) return e;
     e = ensure_smem_attr(reinterpret_cast<const void*>(dense_count_kernel), smem_count);
@@ -866,7 +970,10 @@ cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int
     // With one rank per launch the pair is latency-bound and the overlap pays; a launch that hosts several ranks
     // fills the device with the first kernel alone, and early CTAs of the second only get in its way.
     const bool overlap = b.n == 1 && pdl_enabled();
-    return launch_dependent(dense_scatter_kernel, grid, dim3(kRerouteThreads), smem, stream, overlap, b, L, P, D, quota_mode,
+    // up to two tiles per SM the kernel is a chain of phases: more threads shorten each
+    const int sms = std::max(device_sm_count(), 1);
+    const int threads = static_cast<int64_t>(grid.x) * b.n <= 2 * sms ? kDenseMaxThreads : kRerouteThreads;
+    return launch_dependent(dense_scatter_kernel, grid, dim3(threads), smem, stream, overlap, b, L, P, D, quota_mode,
                             interleave, chunk, overlap ? 1 : 0);
 }
 
@@ -874,11 +981,29 @@ cudaError_t launch_dense_backward(const Batch<DenseBwdArgs>& b, int L, int P, in
     int max_T = 0;
     for (int i = 0; i < b.n; ++i) max_T = b.a[i].T > max_T ? b.a[i].T : max_T;
     if (max_T == 0) return cudaSuccess;
+    // The tile kernel pays for its staging where the launch is bound by memory; below, the thread-per-four-cells kernel has
+    // the shorter chain (events around one cold launch, tiles against cells: 16384 tokens x 256 experts 18.6 and 22.6 us,
+    // 16384 x 128 15.4 and 14.6, 8192 x 128 14.4 and 12.2).
+    int64_t cells = 0;
+    for (int i = 0; i < b.n; ++i) cells += static_cast<int64_t>(b.a[i].T) * L;
+    bool tiles = cells >= kDenseBwdTileCells && L % 4 == 0 && dense_bwd_smem_bytes(L, P) <= kMaxCtaSmem;
+    for (int i = 0; i < b.n; ++i) {
+        tiles = tiles && ((reinterpret_cast<uintptr_t>(b.a[i].map) & 3u) == 0) && ((reinterpret_cast<uintptr_t>(b.a[i].grad_probs) & 15u) == 0);
+    }
+    count_launch();
+    if (tiles) {
+        const size_t smem = dense_bwd_smem_bytes(L, P);
+        cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(dense_backward_tile_kernel), smem);
+        if (e != cudaSuccess) return e;
+        // a task (four columns, eight rows) per thread; wide layers get short tiles
+        const int segs = std::min(std::max(kDenseBwdThreads / (L / 4), 1), kDenseSegs), rows = 8 * segs;
+        dense_backward_tile_kernel<<<dim3((max_T + rows - 1) / rows, b.n), kDenseBwdThreads, smem, stream>>>(b, L, P, D, rows);
+        return cudaGetLastError();
+    }
     int64_t blocks = (static_cast<int64_t>(max_T) * L / 4 + kRerouteThreads - 1) / kRerouteThreads + 1;
     const int64_t sms = device_sm_count() > 0 ? device_sm_count() : 1;
     const int64_t cap = (sms * 16) / b.n > 1 ? (sms * 16) / b.n : 1;
     if (blocks > cap) blocks = cap;
-    count_launch();
     dense_backward_kernel<<<dim3(static_cast<unsigned>(blocks), b.n), kRerouteThreads, 0, stream>>>(b, L, P, D);
     return cudaGetLastError();
 }
@@ -894,7 +1019,6 @@ cudaError_t launch_dense_backward(const Batch<DenseBwdArgs>& b, int L, int P, in
 //     weight_sync, which leaves every SM a quarter of its shared memory: single CTAs find room anywhere, clusters of
 //     eight wait for it or keep weight_sync out (65536 entries of eight ranks: the step took 69 us with clusters).
 constexpr int64_t kOrdRecountMax = 1 << 18;
-constexpr size_t kOrdMaxSmem = 225 * 1024;
 
 struct OrdGrid {
     int threads, ctas, clusters, per_lane;
@@ -968,7 +1092,7 @@ static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L,
         in_place = in_place || (n > 0 && x < y + bytes && y < x + bytes);
     }
     if (max_n == 0) return cudaSuccess;
-    const int staged = sparse_smem_bytes(L, true) <= kOrdMaxSmem ? 1 : 0;
+    const int staged = sparse_smem_bytes(L, true) <= kMaxCtaSmem ? 1 : 0;
     const size_t smem = sparse_smem_bytes(L, staged != 0);
     const OrdGrid g = ord_grid(max_n, b.n, in_place, kOrdThreads);
     // One rank per launch is latency-bound and the overlap with the count kernel pays; several ranks fill the device
@@ -1128,7 +1252,7 @@ int uep_dispatch_positions(const int32_t* phys_ids, int64_t num_entries, int P, 
         return UEP_OK;
     }
     if (!phys_ids || !pos || !scratch) return fail(UEP_ERR_INVALID, "dispatch_positions: null pointer");
-    const OrdGrid g = ord_grid(num_entries, 1, false, ord_smem_bytes(P + 1, kOrdThreads) <= kOrdMaxSmem ? kOrdThreads : kOrdFewThreads);
+    const OrdGrid g = ord_grid(num_entries, 1, false, ord_smem_bytes(P + 1, kOrdThreads) <= kMaxCtaSmem ? kOrdThreads : kOrdFewThreads);
     const size_t smem = ord_smem_bytes(P + 1, g.threads), smem1 = sizeof(int32_t) * (P + 1);
     const bool overlap = g.table && pdl_enabled();
     if (g.table) {
