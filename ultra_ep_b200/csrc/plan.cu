@@ -25,6 +25,9 @@
 
 #include <algorithm>
 #include <cstring>
+#include <map>
+#include <mutex>
+#include <utility>
 
 #include "internal.h"
 #include "solver.cuh"
@@ -34,6 +37,10 @@ namespace uep {
 namespace {
 
 constexpr int kPlanThreads = 256;
+constexpr int kSolveThreads = 512;
+constexpr size_t kSolveMaxSmem = 200 * 1024;
+constexpr size_t kPlanMatrixBytes = 16 * 1024;  // of the load matrix, where the plan kernel keeps it in shared memory
+constexpr int kPartBatch = 9;  // partial counts a thread asks for at once: two threads an expert cover 18 CTAs
 
 __device__ __forceinline__ void hist_add_swar(uint32_t word, int32_t* hist, int col) {
     // four byte-wide counters packed in `word`
@@ -54,19 +61,28 @@ __device__ __noinline__ void histogram_slice(int input_kind, const void* input, 
         const uint8_t* map = static_cast<const uint8_t*>(input);
         const int rows_per = ceil_div_i(T, nparts);
         const int r0 = min(part * rows_per, T), r1 = min(r0 + rows_per, T);
-        const bool vec_ok = (L % 16 == 0) && ((reinterpret_cast<uintptr_t>(map) & 15u) == 0) && (nthreads % (L / 16) == 0);
+        const int groups = L / 16;
+        const bool vec_ok = (L % 16 == 0) && ((reinterpret_cast<uintptr_t>(map) & 15u) == 0) && groups <= nthreads;
         if (vec_ok) {
-            // one thread owns a 16-column group and walks rows; 0/1 bytes are summed four at a
-            // time inside 32-bit words and spilled to the histogram before a byte can overflow
-            const int groups = L / 16;
+            // one thread owns a 16-column group and walks rows, eight loads in flight; 0/1 bytes are summed four at a
+            // time inside 32-bit words and spilled to the histogram before a byte can overflow. (One load at a time: the
+            // plan kernel of eight ranks of 8192 x 128 took 28 us, against 22 with this and the present solver.)
             const int g = tid % groups;
             const int row_lane = tid / groups, row_lanes = nthreads / groups;
             uint4 acc = make_uint4(0, 0, 0, 0);
             int pending = 0;
-            for (int r = r0 + row_lane; r < r1; r += row_lanes) {
-                const uint4 v = ld_global_nc_v4(map + static_cast<int64_t>(r) * L + g * 16);
-                acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-                if (++pending == 255) {
+            for (int r = row_lane < row_lanes ? r0 + row_lane : r1; r < r1; r += 8 * row_lanes) {
+                uint4 v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int row = r + u * row_lanes;
+                    v[u] = row < r1 ? ld_global_nc_v4(map + static_cast<int64_t>(row) * L + g * 16) : make_uint4(0, 0, 0, 0);
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w;
+                }
+                if ((pending += 8) == 248) {
                     hist_add_swar(acc.x, hist, g * 16); hist_add_swar(acc.y, hist, g * 16 + 4);
                     hist_add_swar(acc.z, hist, g * 16 + 8); hist_add_swar(acc.w, hist, g * 16 + 12);
                     acc = make_uint4(0, 0, 0, 0);
@@ -158,20 +174,40 @@ __global__ void __launch_bounds__(kPlanThreads) histogram_kernel(int input_kind,
 }
 
 // Stateless solve: one CTA per NVLink domain.
-__global__ void __launch_bounds__(kPlanThreads) solve_kernel(SolveArgs a, int32_t* global_loads_out, int reduce_loads,
-                                                             DeviceStatus* status) {
+__global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(SolveArgs a, int32_t* global_loads_out, int reduce_loads, int staged,
+                                                                 DeviceStatus* status) {
     extern __shared__ __align__(128) char smem_raw[];
     const int domain = blockIdx.x;
     const int E = a.G * a.M, L = a.N * a.M;
     if (reduce_loads) {
-        // total load of this domain's experts over all ranks
-        for (int i = threadIdx.x; i < E; i += blockDim.x) {
-            const int l = domain * E + i;
+        // Total load of this domain's experts over all ranks, and this rank's own, straight to where the solver keeps
+        // them. The rows are shared by all the threads an expert can have, 16 loads of each in flight.
+        const SolverSmem sm = carve_solver_smem(smem_raw, E, a.G);
+        const int parts = max(static_cast<int>(blockDim.x) / E, 1);
+        int32_t* matrix = reinterpret_cast<int32_t*>(smem_raw + solver_smem_bytes(E, a.G));
+        for (int i = threadIdx.x; i < E; i += blockDim.x) sm.loads[i] = 0;
+        __syncthreads();
+        for (int i = threadIdx.x; i < E * parts; i += blockDim.x) {
+            const int e = i % E, part = i / E;
+            const int32_t* column = a.loads_per_rank + domain * E + e;
+            if (part == 0) sm.my_loads[e] = __ldcg(column + static_cast<int64_t>(a.my_rank) * L);
             int32_t total = 0;
-            for (int r = 0; r < a.N; ++r) total += __ldcg(a.loads_per_rank + static_cast<int64_t>(r) * L + l);
-            global_loads_out[l] = total;
+            for (int r0 = part; r0 < a.N; r0 += 16 * parts) {
+                int32_t v[16];
+#pragma unroll
+                for (int u = 0; u < 16; ++u) v[u] = r0 + u * parts < a.N ? __ldcg(column + static_cast<int64_t>(r0 + u * parts) * L) : 0;
+#pragma unroll
+                for (int u = 0; u < 16; ++u) {
+                    total += v[u];
+                    if (staged && r0 + u * parts < a.N) matrix[(r0 + u * parts) * L + e] = v[u];
+                }
+            }
+            atomicAdd(sm.loads + e, total);
         }
         __syncthreads();
+        for (int i = threadIdx.x; i < E; i += blockDim.x) global_loads_out[domain * E + i] = sm.loads[i];
+        a.preloaded = 1;
+        a.staged_loads = staged ? matrix : nullptr;
     }
     solve_domain_dispatch(a, domain, smem_raw, status);
 }
@@ -195,8 +231,13 @@ __global__ void __launch_bounds__(256) init_master_kernel(int32_t* p2l, int32_t*
     for (int i = gtid; i < L; i += gsize) lcnts[i] = 1;
 }
 
+__host__ __device__ inline size_t plan_matrix_bytes(int N, int L) {
+    const size_t bytes = sizeof(int32_t) * N * static_cast<size_t>(L);
+    return bytes <= kPlanMatrixBytes ? bytes : 0;
+}
+
 // The fused per-layer plan kernel. gridDim.x = nlocal * ctas_per_rank.
-__global__ void __launch_bounds__(kPlanThreads) plan_kernel(PlanCall call) {
+__global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(PlanCall call) {
     extern __shared__ __align__(128) char smem_raw[];
     __shared__ int s_timeout_peer;
     __shared__ uint64_t s_epoch;
@@ -239,28 +280,35 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(PlanCall call) {
         if (call.trace != nullptr && tid == 0) call.trace[local * 8 + slot] = global_timer_ns();
     };
     if (call.trace != nullptr && tid == 0) call.trace[local * 8 + 5] = t_start;  // when this CTA started
-    for (int i = tid; i < L; i += blockDim.x) {
-        int32_t total = hist[i];
-        for (int c0 = 1; c0 < call.ctas_per_rank; c0 += 8) {
-            uint64_t w[8];
+    {   // an expert's partials are shared by all the threads it can have, so that one round of loads fetches them
+        const int rest = call.ctas_per_rank - 1;
+        const int parts = max(min(static_cast<int>(blockDim.x) / L, rest), 1);
+        for (int idx = tid; idx < L * parts; idx += blockDim.x) {
+            const int i = idx % L, part = idx / L;
+            int32_t total = 0;
+            for (int c0 = 1 + part; c0 <= rest; c0 += kPartBatch * parts) {
+                uint64_t w[kPartBatch];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                if (c0 + u < call.ctas_per_rank) w[u] = ld_relaxed_sys_u64(rk.hist_parts + static_cast<int64_t>(c0 + u) * Lpad + i);
-            }
+                for (int u = 0; u < kPartBatch; ++u) {
+                    const int c = c0 + u * parts;
+                    if (c <= rest) w[u] = ld_relaxed_sys_u64(rk.hist_parts + static_cast<int64_t>(c) * Lpad + i);
+                }
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                if (c0 + u < call.ctas_per_rank) {
-                    if (static_cast<uint32_t>(w[u] >> 32) != tag &&
-                        !wait_tagged_word(rk.hist_parts + static_cast<int64_t>(c0 + u) * Lpad + i, tag,
-                                          *reinterpret_cast<volatile int*>(&s_timeout_peer) >= 0 ? 0 : call.timeout_ns, w[u])) {
-                        atomicMax(&s_timeout_peer, rk.my_rank);
-                        w[u] = 0;
+                for (int u = 0; u < kPartBatch; ++u) {
+                    const int c = c0 + u * parts;
+                    if (c <= rest) {
+                        if (static_cast<uint32_t>(w[u] >> 32) != tag &&
+                            !wait_tagged_word(rk.hist_parts + static_cast<int64_t>(c) * Lpad + i, tag,
+                                              *reinterpret_cast<volatile int*>(&s_timeout_peer) >= 0 ? 0 : call.timeout_ns, w[u])) {
+                            atomicMax(&s_timeout_peer, rk.my_rank);
+                            w[u] = 0;
+                        }
+                        total += static_cast<int32_t>(static_cast<uint32_t>(w[u]));
                     }
-                    total += static_cast<int32_t>(static_cast<uint32_t>(w[u]));
                 }
             }
+            if (rest > 0) atomicAdd(hist + i, total);
         }
-        hist[i] = total;
     }
     __syncthreads();
     if (tid == 0) *rk.epochs = epoch;  // every CTA of the launch has read the old value: its partial carried the tag
@@ -283,6 +331,12 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(PlanCall call) {
         }
     }
 
+    // With one domain the solver finds the loads in shared memory where it keeps them: its loads are where hist was.
+    const bool preload = call.G == N && !call.legacy;
+    const SolverSmem solver_sm = carve_solver_smem(smem_raw, L, N);
+    const bool staged = preload && plan_matrix_bytes(N, L) > 0;
+    int32_t* matrix = reinterpret_cast<int32_t*>(smem_raw + solver_smem_bytes(L, N));
+    __syncthreads();  // hist has been read by every thread
     stamp(1);
     // 3. collect every rank's row (bounded), expose the matrix, reduce. A thread owns one expert:
     //    it first issues the loads of eight ranks' words together and only then looks at them,
@@ -308,11 +362,16 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(PlanCall call) {
                     }
                     const int32_t v = static_cast<int32_t>(static_cast<uint32_t>(w[u]));
                     rk.loads_per_rank[static_cast<int64_t>(r0 + u) * L + i] = v;
+                    if (staged) matrix[(r0 + u) * L + i] = v;
                     total += v;
                 }
             }
         }
         rk.global_loads[i] = total;
+        if (preload) {
+            solver_sm.my_loads[i] = hist[i];
+            solver_sm.loads[i] = total;  // (hist[i] itself)
+        }
     }
     __threadfence_block();
     __syncthreads();
@@ -338,6 +397,8 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(PlanCall call) {
     a.eps = call.params.oracle_eps;
     a.my_rank = me;
     a.legacy = call.legacy;
+    a.preloaded = preload ? 1 : 0;
+    a.staged_loads = staged ? matrix : nullptr;
     a.trace = call.trace != nullptr ? call.trace + (kMaxLocalRanks + local) * 8 : nullptr;
     const int num_domains = N / call.G;
     for (int d = 0; d < num_domains; ++d) solve_domain_dispatch(a, d, smem_raw, rk.status);
@@ -345,14 +406,25 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(PlanCall call) {
 }
 
 size_t plan_smem_bytes(int N, int G, int M) {
-    const size_t solver = std::max(solver_smem_bytes(G * M, G), legacy_smem_bytes(G * M, G));
+    const size_t solver = std::max(solver_smem_bytes(G * M, G) + (G == N ? plan_matrix_bytes(N, N * M) : 0), legacy_smem_bytes(G * M, G));
     const size_t hist = sizeof(int32_t) * static_cast<size_t>(N) * M;
     return (solver > hist ? solver : hist) + 16;
 }
 
 cudaError_t ensure_smem(const void* fn, size_t bytes) {
     if (bytes <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    // remembered per kernel and device: the call costs about as much as a launch
+    static std::mutex mu;
+    static std::map<std::pair<const void*, int>, size_t> granted;
+    int dev = -1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mu);
+    size_t& have = granted[{fn, dev}];
+    if (have >= bytes) return cudaSuccess;
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    if (e == cudaSuccess) have = bytes;
+    return e;
 }
 
 std::atomic<int64_t> g_launches{0};
@@ -454,12 +526,18 @@ int uep_solve_placement(const int32_t* loads_per_rank, int32_t* global_loads_out
     a.eps = params->oracle_eps;
     a.my_rank = my_rank;
     a.legacy = 0;
+    a.preloaded = 0;
+    a.staged_loads = nullptr;
     a.trace = nullptr;
-    const size_t smem = solver_smem_bytes(nvl_ranks * M, nvl_ranks) + 16;
+    size_t smem = solver_smem_bytes(nvl_ranks * M, nvl_ranks) + 16;
+    // with one domain the solver also keeps the load matrix it adds up, where that fits
+    const size_t matrix = sizeof(int32_t) * num_ranks * num_ranks * static_cast<size_t>(M);
+    const int staged = nvl_ranks == num_ranks && smem + matrix <= kSolveMaxSmem ? 1 : 0;
+    if (staged) smem += matrix;
     UEP_CUDA_TRY(ensure_smem(reinterpret_cast<const void*>(solve_kernel), smem));
     count_launch();
-    solve_kernel<<<num_ranks / nvl_ranks, kPlanThreads, smem, stream>>>(a, global_loads_out, 1,
-                                                                        reinterpret_cast<DeviceStatus*>(status));
+    solve_kernel<<<num_ranks / nvl_ranks, kSolveThreads, smem, stream>>>(a, global_loads_out, 1, staged,
+                                                                          reinterpret_cast<DeviceStatus*>(status));
     UEP_CUDA_TRY(cudaGetLastError());
     return UEP_OK;
 }
@@ -486,7 +564,7 @@ int uep_legacy_solve_placement(const int32_t* global_loads, int32_t* p2l, int32_
     const size_t smem = legacy_smem_bytes(nvl_ranks * M, nvl_ranks) + 16;
     UEP_CUDA_TRY(ensure_smem(reinterpret_cast<const void*>(solve_kernel), smem));
     count_launch();
-    solve_kernel<<<num_ranks / nvl_ranks, kPlanThreads, smem, stream>>>(a, nullptr, 0, reinterpret_cast<DeviceStatus*>(status));
+    solve_kernel<<<num_ranks / nvl_ranks, kSolveThreads, smem, stream>>>(a, nullptr, 0, 0, reinterpret_cast<DeviceStatus*>(status));
     UEP_CUDA_TRY(cudaGetLastError());
     return UEP_OK;
 }

@@ -5,13 +5,19 @@
 // (csrc/kernels/placement.cu:788-1482 of the reference): same fp32 threshold
 // arithmetic, same tie-breaks, same probe schedule of the threshold search, same
 // largest-remainder splits. The execution is different:
-//   * one lane per rank with slack / slot counters in registers for any domain size
-//     (1-3 ranks per lane), warp-wide redux instructions instead of shuffle trees,
-//     occupancy of an expert as a ballot word;
+//   * the ranks with slack are kept sorted in the lanes of a warp (1-3 per lane), and one step
+//     makes all the exports of an expert;
+//   * an expert is drained once, from its one home rank, so a build keeps no occupancy table
+//     and no exported sums: a source's masters sit in the lanes, and the walk over the sources
+//     ends at the first one below the threshold;
+//   * the three builds of the fast path and the capacity pre-check run side by side on four
+//     warps (the serial search takes the first that is feasible), while the other warps clear
+//     the outputs;
 //   * each rank's masters are ranked by counting instead of a serial insertion sort;
 //   * the per-rank load matrix is read through L2 where it is needed instead of being
-//     staged in shared memory, so shared memory stays under 48 KB at the static limits;
-//   * output arrays are cleared by the same CTA instead of six memsets.
+//     staged in shared memory, so shared memory stays under 48 KB at the static limits.
+// All of it is latency of one CTA. Kernel time of uep_solve_placement on one B200: 64 ranks x 4 experts x 2 slots 25.3 us
+// (39.5 with the outputs cleared first, one build after another and one warp maximum per export), of which the build 14.
 #pragma once
 
 #include <climits>
@@ -43,6 +49,8 @@ struct SolveArgs {
     int locality;
     float eps;
     int my_rank;
+    const int32_t* staged_loads;  // loads_per_rank[N, L] in shared memory, or null
+    int preloaded;  // 1: the shared-memory loads and my_loads of the (only) domain are in place already
     int legacy;  // 1: legacy placement (counts-only greedy, round-robin reroute) instead of the quota solver
     unsigned long long* trace;  // optional: 8 globaltimer stamps of the solver phases (tuning aid), or null
 };
@@ -51,10 +59,11 @@ constexpr int kSolverProbeWarps = 4;
 
 // Control words in shared memory.
 enum SolverCtrl {
-    kCtlLo = 0, kCtlHi, kCtlPrecheckDone, kCtlFastDone, kCtlNumExports, kCtlSmallRange,
+    kCtlLo = 0, kCtlHi, kCtlStop0, kCtlNumExports = kCtlStop0 + kSolverProbeWarps, kCtlSmallRange,
     kCtlProbe0, kCtlValid0 = kCtlProbe0 + kSolverProbeWarps, kCtlFeasible0 = kCtlValid0 + kSolverProbeWarps,
-    kCtlMultiCount = kCtlFeasible0 + kSolverProbeWarps, kCtlCount
+    kCtlExports0 = kCtlFeasible0 + kSolverProbeWarps, kCtlMultiCount = kCtlExports0 + kSolverProbeWarps, kCtlCount
 };
+static_assert(kCtlCount <= 32, "control words");
 
 struct SolverSmem {
     int32_t* loads;           // [E]
@@ -62,25 +71,23 @@ struct SolverSmem {
     int32_t* sorted_experts;  // [E]
     int32_t* expert_slot;     // [E]
     int32_t* rank_load;       // [Gp]
-    int32_t* source_order;    // [Gp]
+    int32_t* source_order;    // [Gp] ranks by load, largest first, ties to the lower one
+    int32_t* sink_order;      // [Gp] smallest first, likewise
     int32_t* next_slot;       // [Gp]
-    int32_t* export_sum;      // [4][E]
-    uint32_t* occ;            // [4][E*NS]
-    ExportEntry* plan;        // [kMaxExportsPerDomain]
+    int32_t* export_sum;      // [4][E] of the four warps that build plans
+    ExportEntry* plan;        // [4][kMaxExportsPerDomain]
     int* ctrl;                // [kCtlCount]
 };
 
 __host__ __device__ inline int solver_ns(int G) { return (G + 31) / 32; }
 __host__ __device__ inline int solver_gpad(int G) { return (G + 3) / 4 * 4; }
 __host__ __device__ inline size_t solver_smem_bytes(int E, int G) {
-    const int ns = solver_ns(G), gp = solver_gpad(G);
-    return sizeof(int32_t) * (4 * static_cast<size_t>(E) + 3 * gp + kSolverProbeWarps * static_cast<size_t>(E) +
-                              kSolverProbeWarps * static_cast<size_t>(E) * ns) +
-           sizeof(ExportEntry) * kMaxExportsPerDomain + sizeof(int) * 32;
+    return sizeof(int32_t) * (4 * static_cast<size_t>(E) + 4 * solver_gpad(G) + kSolverProbeWarps * static_cast<size_t>(E)) +
+           kSolverProbeWarps * sizeof(ExportEntry) * kMaxExportsPerDomain + sizeof(int) * 32;
 }
 
 __device__ inline SolverSmem carve_solver_smem(char* raw, int E, int G) {
-    const int ns = solver_ns(G), gp = solver_gpad(G);
+    const int gp = solver_gpad(G);
     SolverSmem s;
     int32_t* p = reinterpret_cast<int32_t*>(raw);
     s.loads = p; p += E;
@@ -89,133 +96,194 @@ __device__ inline SolverSmem carve_solver_smem(char* raw, int E, int G) {
     s.expert_slot = p; p += E;
     s.rank_load = p; p += gp;
     s.source_order = p; p += gp;
+    s.sink_order = p; p += gp;
     s.next_slot = p; p += gp;
     s.export_sum = p; p += kSolverProbeWarps * E;
-    s.occ = reinterpret_cast<uint32_t*>(p); p += kSolverProbeWarps * E * ns;
-    s.plan = reinterpret_cast<ExportEntry*>(p); p += 3 * kMaxExportsPerDomain;
+    s.plan = reinterpret_cast<ExportEntry*>(p); p += kSolverProbeWarps * 3 * kMaxExportsPerDomain;
     s.ctrl = reinterpret_cast<int*>(p);
     return s;
 }
 
+__device__ __forceinline__ int warp_inclusive_scan(int v, int lane) {
+#pragma unroll
+    for (int off = 1; off < kWarp; off <<= 1) {
+        const int t = __shfl_up_sync(kFullMask, v, off);
+        if (lane >= off) v += t;
+    }
+    return v;
+}
+
 // Greedy export plan for one threshold, by one warp. Returns feasibility (uniform over
 // the warp). Semantics of csrc/kernels/placement.cu:337-667 of the reference.
+//
+// An expert's exports go to the ranks by slack, largest first, ties to the lower rank, each rank once; every one of them is
+// filled up except the last. So the ranks are kept sorted in the lanes (slot 32 s + lane), with inclusive sums of their
+// slack, and one step per expert finds all its exports: lane i takes part while the slack in front of it is less than what
+// is to be moved and its share passes the floor. The filled ranks leave at the front, and the last one, if slack and
+// slots are left, moves back to its place. (One export at a time, a warp maximum each: 325 ns an export.)
+// `stop`: raised by a warp whose result makes this build pointless.
 template <int NS, bool STORE>
-__device__ bool warp_build_plan(const SolverSmem& sm, int32_t* export_sum, uint32_t* occ, ExportEntry* plan,
-                                int& num_exports, int thr, int E, int G, int M, int R, int min_tokens,
-                                bool allow_zero_master, bool dynamic_floor, int lane) {
+__device__ bool warp_build_plan(const SolverSmem& sm, int32_t* export_sum, ExportEntry* plan, int& num_exports, int thr, int E,
+                                int G, int M, int R, int min_tokens, bool allow_zero_master, bool dynamic_floor, int lane,
+                                const volatile int* stop = nullptr) {
     num_exports = 0;
-    // state init (:86-109)
-    for (int e = lane; e < E; e += kWarp) {
-        export_sum[e] = 0;
-        const int home = e / M;
-#pragma unroll
-        for (int s = 0; s < NS; ++s) occ[e * NS + s] = ((home >> 5) == s) ? (1u << (home & 31)) : 0u;
+    if (STORE) {
+        __syncwarp();  // an earlier build of this warp may still be storing its sums
+        for (int e = lane; e < E; e += kWarp) export_sum[e] = 0;
+        __syncwarp();
     }
-    int slack[NS], slots[NS];
-    int local_excess = 0, local_slack = 0;
+    int slack[NS], meta[NS], upto[NS];  // meta: free slots << 8 | rank; upto: slack of this slot and all in front of it
+    int order[NS], order_load[NS];      // the sources
+    int end = 0;                        // slots with slack are [head, end)
+    int local_excess = 0, total_slack = 0;
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-        const int r = lane + kWarp * s;
-        const int rl = (r < G) ? sm.rank_load[r] : thr;
-        slack[s] = max(thr - rl, 0);
-        slots[s] = 0;
-        local_excess += max(rl - thr, 0);
-        local_slack += slack[s];
+        const int i = lane + kWarp * s;
+        const int sink = i < G ? sm.sink_order[i] : 0;
+        slack[s] = i < G ? max(thr - sm.rank_load[sink], 0) : 0;
+        meta[s] = R << 8 | sink;
+        order[s] = i < G ? sm.source_order[i] : 0;
+        order_load[s] = i < G ? sm.rank_load[order[s]] : thr;
+        local_excess += max(order_load[s] - thr, 0);
+        end += __popc(__ballot_sync(kFullMask, slack[s] > 0));
+        upto[s] = warp_inclusive_scan(slack[s], lane) + total_slack;
+        total_slack = __shfl_sync(kFullMask, upto[s], kWarp - 1);
     }
-    __syncwarp();
     const int total_excess = warp_sum(local_excess);
-    const int total_slack = warp_sum(local_slack);
     if (total_excess == 0) return true;
+    // Every export takes the same from both, so the slack left always covers the excess left.
     if (total_excess > total_slack) return false;
 
-    int running_excess = total_excess;
-    int running_slack = total_slack;
+    auto at = [&](const int (&v)[NS], int slot) {
+        int x = __shfl_sync(kFullMask, v[0], slot & 31);
+#pragma unroll
+        for (int s = 1; s < NS; ++s) {
+            const int y = __shfl_sync(kFullMask, v[s], slot & 31);
+            x = slot >> 5 == s ? y : x;
+        }
+        return x;
+    };
+    auto masters = [&](int src, int base, int& e, int& load) {  // 32 of the source's masters, one per lane
+        e = base + lane < M ? sm.sorted_experts[src * M + base + lane] : 0;
+        load = base + lane < M ? sm.loads[e] : 0;
+    };
+    int head = 0, gone = 0;  // gone: slack in front of slot `head`, as `upto` counts it
+    int src = at(order, 0), src_load = at(order_load, 0), first_e, first_load;
+    masters(src, 0, first_e, first_load);
     for (int ord = 0; ord < G; ++ord) {
-        const int src = sm.source_order[ord];
-        int need = max(sm.rank_load[src] - thr, 0);
-        if (need <= 0) continue;
-        if (need > running_slack) return false;
-
-        for (int pos = 0; pos < M; ++pos) {
-            const int e = sm.sorted_experts[src * M + pos];
-            const int load_e = sm.loads[e];
-            const int keep = (!allow_zero_master && load_e > 0) ? 1 : 0;
-            int es = export_sum[e];
-            int avail = max(load_e - keep - es, 0);
-            if (avail <= 0) continue;
-
-            bool my_occ[NS];
-#pragma unroll
-            for (int s = 0; s < NS; ++s) my_occ[s] = ((occ[e * NS + s] >> lane) & 1u) != 0u;
-            bool changed = false;
-
-            while (need > 0 && avail > 0) {
-                bool ok[NS];
-#pragma unroll
-                for (int s = 0; s < NS; ++s) {
-                    ok[s] = (lane + kWarp * s < G) && slack[s] > 0 && slots[s] < R && !my_occ[s];
+        int need = src_load - thr;
+        if (need <= 0) break;  // sources come by load: no later one is above the threshold
+        if (stop != nullptr && __shfl_sync(kFullMask, *stop, 0) != 0) return false;
+        const int this_src = src;
+        int my_e = first_e, my_load = first_load;
+        const int next_ord = min(ord + 1, G - 1);  // fetched while this one is drained
+        src = at(order, next_ord);
+        src_load = at(order_load, next_ord);
+        masters(src, 0, first_e, first_load);
+        bool drained = false;  // the masters come by load too: no later one has anything to give
+        for (int base = 0; base < M && need > 0 && !drained; base += kWarp) {
+            if (base > 0) masters(this_src, base, my_e, my_load);
+            const int in_chunk = min(M - base, kWarp);
+            for (int pos = 0; pos < in_chunk && need > 0; ++pos) {
+                const int load_e = __shfl_sync(kFullMask, my_load, pos);
+                const int avail = load_e - ((!allow_zero_master && load_e > 0) ? 1 : 0);
+                if (avail <= 0) {
+                    drained = true;
+                    break;
                 }
-                int floor_tokens = min_tokens;
-                if (dynamic_floor) {
-                    int feasible = 0;
+                const int move = min(need, avail);
+                int q[NS], next_slack[NS], next_meta[NS], next_upto[NS];
+                int first_out = kWarp * NS;  // the first slot from `head` on that takes nothing
+#pragma unroll
+                for (int s = NS - 1; s >= 0; --s) {
+                    const int slot = lane + kWarp * s;
+                    const int before = upto[s] - gone - slack[s];
+                    q[s] = min(slack[s], move - before);
+                    // dynamic floor: ceil(what is still needed / the ranks that could still take part)
+                    const bool enough = dynamic_floor ? static_cast<long long>(q[s]) * (end - slot) >= need - before : q[s] >= min_tokens;
+                    const unsigned out = __ballot_sync(kFullMask, slot >= head && !(slot < end && before < move && enough));
+                    if (out != 0u) first_out = kWarp * s + __ffs(out) - 1;
+                    next_slack[s] = __shfl_down_sync(kFullMask, slack[s], 1);
+                    next_meta[s] = __shfl_down_sync(kFullMask, meta[s], 1);
+                    next_upto[s] = __shfl_down_sync(kFullMask, upto[s], 1);
+                    if (s + 1 < NS) {
+                        const int a = __shfl_sync(kFullMask, slack[s + 1 < NS ? s + 1 : s], 0), b = __shfl_sync(kFullMask, meta[s + 1 < NS ? s + 1 : s], 0),
+                                  c = __shfl_sync(kFullMask, upto[s + 1 < NS ? s + 1 : s], 0);
+                        if (lane == kWarp - 1) {
+                            next_slack[s] = a;
+                            next_meta[s] = b;
+                            next_upto[s] = c;
+                        }
+                    }
+                }
+                const int exports = first_out - head;
+                if (exports == 0) continue;
+                const int last = first_out - 1;
+                const int last_upto = at(upto, last), last_meta = at(meta, last);
+                const int moved = min(last_upto - gone, move);
+                const int rest = last_upto - gone - moved;  // slack that the last rank keeps
+                const bool stays = rest > 0 && last_meta >> 8 > 1;
+                if (STORE) {
+                    if (num_exports + exports > kMaxExportsPerDomain) return false;
+                    const int e = __shfl_sync(kFullMask, my_e, pos);
 #pragma unroll
                     for (int s = 0; s < NS; ++s) {
-                        feasible += __popc(__ballot_sync(kFullMask, ok[s] && min(min(need, slack[s]), avail) > 0));
+                        const int slot = lane + kWarp * s;
+                        if (slot >= head && slot < first_out) plan[num_exports + slot - head] = ExportEntry{e, meta[s] & 255, q[s]};
                     }
-                    if (feasible <= 0) break;
-                    floor_tokens = max(1, (need + feasible - 1) / feasible);
+                    if (lane == 0) export_sum[e] = moved;
+                    num_exports += exports;
                 }
-                int cands[NS];
-                int cand = -1;
+                int ahead = 0;  // slots that come in front of the last rank now
 #pragma unroll
                 for (int s = 0; s < NS; ++s) {
-                    cands[s] = (ok[s] && min(min(need, slack[s]), avail) >= floor_tokens) ? slack[s] : -1;
-                    cand = max(cand, cands[s]);
-                }
-                const int best_cap = warp_max(cand);
-                if (best_cap < 0) break;
-                int best = -1;  // largest slack, ties to the lower rank
-#pragma unroll
-                for (int s = 0; s < NS; ++s) {
-                    const unsigned b = __ballot_sync(kFullMask, cands[s] == best_cap);
-                    if (best < 0 && b != 0u) best = (__ffs(b) - 1) + kWarp * s;
-                }
-                if (STORE && num_exports >= kMaxExportsPerDomain) return false;
-                const int q = min(min(need, best_cap), avail);
-                if (STORE) {
-                    if (lane == 0) plan[num_exports] = ExportEntry{e, best, q};
-                    num_exports += 1;
+                    const int slot = lane + kWarp * s;
+                    ahead += __popc(__ballot_sync(kFullMask, slot > last && slot < end && (slack[s] > rest || (slack[s] == rest &&
+                                                                                           (meta[s] & 255) < (last_meta & 255)))));
                 }
 #pragma unroll
                 for (int s = 0; s < NS; ++s) {
-                    if (lane + kWarp * s == best) {
-                        slack[s] -= q;
-                        slots[s] += 1;
-                        my_occ[s] = true;
+                    const int slot = lane + kWarp * s;
+                    if (stays && slot >= last && slot < last + ahead) {
+                        slack[s] = next_slack[s];
+                        meta[s] = next_meta[s];
+                        upto[s] = next_upto[s] - rest;
+                    } else if (stays && slot == last + ahead) {
+                        slack[s] = rest;
+                        meta[s] = last_meta - 256;
                     }
                 }
-                es += q;
-                running_excess -= q;
-                running_slack -= q;
-                need -= q;
-                avail -= q;
-                changed = true;
+                head = stays ? last : first_out;
+                gone = stays ? gone + moved : last_upto;
+                need -= moved;
             }
-            if (changed) {
-#pragma unroll
-                for (int s = 0; s < NS; ++s) {
-                    const unsigned w = __ballot_sync(kFullMask, my_occ[s]);
-                    if (lane == 0) occ[e * NS + s] = w;
-                }
-                if (lane == 0) export_sum[e] = es;
-                __syncwarp();
-            }
-            if (need == 0) break;
         }
         if (need > 0) return false;
-        if (running_excess > running_slack) return false;
     }
     return true;
+}
+
+// x = a * b over d, for a, b >= 0 and d > 0: quotient and remainder. A float estimate of a quotient below 2^20 is off by
+// one at most (six roundings of 2^-24 each), which the remainder shows.
+__device__ __forceinline__ void product_over(int a, int b, int d, int& quotient, int& remainder) {
+    const long long x = static_cast<long long>(a) * b;
+    const float estimate = static_cast<float>(a) * static_cast<float>(b) * __frcp_rn(static_cast<float>(d));
+    if (estimate < 1048576.f) {
+        int q = static_cast<int>(estimate);
+        long long r = x - static_cast<long long>(q) * d;
+        if (r < 0) {
+            --q;
+            r += d;
+        } else if (r >= d) {
+            ++q;
+            r -= d;
+        }
+        quotient = q;
+        remainder = static_cast<int>(r);
+    } else {
+        quotient = static_cast<int>(x / d);
+        remainder = static_cast<int>(x % d);
+    }
 }
 
 // Split of this rank's tokens of one expert over the expert's replicas, as an inclusive
@@ -320,30 +388,20 @@ __device__ void build_rank_quota_prefix(const SolveArgs& a, int l_global, int C,
     }
 }
 
-__device__ __forceinline__ int warp_inclusive_scan(int v, int lane) {
-#pragma unroll
-    for (int off = 1; off < kWarp; off <<= 1) {
-        const int t = __shfl_up_sync(kFullMask, v, off);
-        if (lane >= off) v += t;
-    }
-    return v;
-}
-
 // The split of build_rank_quota_prefix for an expert with 2..32 replicas, by one warp: lane j
-// holds replica j, the sums and arg-max searches are warp reductions, and the hosts' own loads
-// are fetched by all lanes at once. Returns false (nothing written) when two replicas share a
-// host rank, which the sequential bookkeeping of the general version is needed for.
-__device__ __forceinline__ bool warp_rank_quota_prefix(const SolveArgs& a, int l_global, int C, int my_load, int phys,
-                                                       int q, int Lp, int L, int lane) {
+// holds replica j on rank `host`, which has `own` tokens for the expert itself, and the sums and
+// arg-max searches are warp reductions. The hosts differ: an export never goes to a rank that
+// holds the expert already.
+__device__ __forceinline__ void warp_rank_quota_prefix(const SolveArgs& a, int l_global, int C, int my_load, int host,
+                                                       int q, int own, int lane) {
     const bool active = lane < C;
-    const int host = active ? phys / Lp : -1 - lane;
     int my_alloc = 0;
     if (!a.locality) {
         const int total_quota = __reduce_add_sync(kFullMask, active ? q : 0);
         if (my_load > 0 && total_quota > 0) {
-            const long long scaled = static_cast<long long>(my_load) * (active ? q : 0);
-            const int share = static_cast<int>(scaled / total_quota);
-            int rem = active ? static_cast<int>(scaled % total_quota) : INT_MIN;
+            int share, rem;
+            product_over(my_load, active ? q : 0, total_quota, share, rem);
+            if (!active) rem = INT_MIN;
             my_alloc = share;
             int remaining = my_load - __reduce_add_sync(kFullMask, share);  // < C: a sum of C fractional parts
             for (int it = 0; it < C && remaining > 0; ++it) {
@@ -357,9 +415,6 @@ __device__ __forceinline__ bool warp_rank_quota_prefix(const SolveArgs& a, int l
             }
         }
     } else {
-        const unsigned same_host = __match_any_sync(kFullMask, host);  // all 32 lanes take part: not under `active &&`
-        if (__any_sync(kFullMask, active && __popc(same_host) > 1)) return false;
-        const int own = active ? __ldcg(a.loads_per_rank + static_cast<int64_t>(host) * L + l_global) : 0;
         const int local_fill = active ? min(own, q) : 0;
         const int remote_cap = active ? q - local_fill : 0;
         const int total_remote_cap = __reduce_add_sync(kFullMask, remote_cap);
@@ -368,9 +423,9 @@ __device__ __forceinline__ bool warp_rank_quota_prefix(const SolveArgs& a, int l
         const int rem_my = max(my_load - __reduce_add_sync(kFullMask, mine ? local_fill : 0), 0);
         if (rem_my > 0 && total_remote_cap > 0) {
             const bool eligible = active && !mine && remote_cap > 0;
-            const long long scaled = static_cast<long long>(rem_my) * (eligible ? remote_cap : 0);
-            const int share = static_cast<int>(scaled / total_remote_cap);
-            int rem = eligible ? static_cast<int>(scaled % total_remote_cap) : INT_MIN;
+            int share, rem;
+            product_over(rem_my, eligible ? remote_cap : 0, total_remote_cap, share, rem);
+            if (!eligible) rem = INT_MIN;
             my_alloc += share;
             int remaining = rem_my - __reduce_add_sync(kFullMask, share);  // < number of eligible replicas
             for (int it = 0; it < C && remaining > 0; ++it) {
@@ -390,7 +445,6 @@ __device__ __forceinline__ bool warp_rank_quota_prefix(const SolveArgs& a, int l
     }
     const int prefix = warp_inclusive_scan(my_alloc, lane);
     if (active) a.rank_quota_prefix[static_cast<int64_t>(l_global) * a.D + lane] = prefix;
-    return true;
 }
 
 // Solve one NVLink domain. All threads of the CTA must call it (blockDim.x >= 128,
@@ -409,109 +463,123 @@ __device__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, Dev
     };
     stamp(0);
 
-    // Clear this domain's slice of every output, then place the masters.
-    for (int i = tid; i < G * Lp; i += nthreads) {
-        a.p2l[domain_start_rank * Lp + i] = -1;
-        if (a.physical_loads != nullptr) a.physical_loads[domain_start_rank * Lp + i] = 0;
-    }
-    for (int i = tid; i < E * D; i += nthreads) {
-        const int64_t idx = static_cast<int64_t>(domain_start_log) * D + i;
-        a.l2p[idx] = -1;
-        a.quota[idx] = 0;
-        a.quota_prefix[idx] = 0;
-        a.rank_quota_prefix[idx] = 0;
-    }
-    __syncthreads();
+    // Every output of this domain as it is without replicas; run by `n` threads.
+    auto clear_outputs = [&](int t, int n) {
+        for (int i = t; i < G * Lp; i += n) {
+            const int local = i % Lp;
+            a.p2l[domain_start_rank * Lp + i] = local < M ? domain_start_log + i / Lp * M + local : -1;
+            if (a.physical_loads != nullptr) a.physical_loads[domain_start_rank * Lp + i] = 0;
+        }
+        const int64_t first = static_cast<int64_t>(domain_start_log) * D;
+        auto master = [&](int e) { return (domain_start_rank + e / M) * Lp + e % M; };
+        const uintptr_t align = reinterpret_cast<uintptr_t>(a.l2p) | reinterpret_cast<uintptr_t>(a.quota) |
+                                reinterpret_cast<uintptr_t>(a.quota_prefix) | reinterpret_cast<uintptr_t>(a.rank_quota_prefix);
+        if (D % 4 == 0 && (align & 15u) == 0) {
+            const int vecs = D / 4;
+            const int4 none = make_int4(0, 0, 0, 0);
+            for (int i = t; i < E * vecs; i += n) {
+                const int e = i / vecs;
+                reinterpret_cast<int4*>(a.l2p + first)[i] = make_int4(i - e * vecs == 0 ? master(e) : -1, -1, -1, -1);
+                reinterpret_cast<int4*>(a.quota + first)[i] = none;
+                reinterpret_cast<int4*>(a.quota_prefix + first)[i] = none;
+                reinterpret_cast<int4*>(a.rank_quota_prefix + first)[i] = none;
+            }
+        } else {
+            for (int i = t; i < E * D; i += n) {
+                const int e = i / D;
+                a.l2p[first + i] = i - e * D == 0 ? master(e) : -1;
+                a.quota[first + i] = 0;
+                a.quota_prefix[first + i] = 0;
+                a.rank_quota_prefix[first + i] = 0;
+            }
+        }
+    };
     for (int i = tid; i < E; i += nthreads) {
-        const int l_global = domain_start_log + i;
-        sm.loads[i] = __ldcg(a.global_loads + l_global);
-        sm.my_loads[i] = __ldcg(a.loads_per_rank + static_cast<int64_t>(a.my_rank) * L + l_global);
+        if (!a.preloaded) {
+            sm.loads[i] = __ldcg(a.global_loads + domain_start_log + i);
+            sm.my_loads[i] = __ldcg(a.loads_per_rank + static_cast<int64_t>(a.my_rank) * L + domain_start_log + i);
+        }
         sm.expert_slot[i] = 1;
-        const int phys = (domain_start_rank + i / M) * Lp + i % M;
-        a.p2l[phys] = l_global;
-        a.l2p[static_cast<int64_t>(l_global) * D] = phys;
     }
-    __syncthreads();
-    stamp(1);
-    for (int r = tid; r < G; r += nthreads) {
-        int sum = 0;
-        for (int m = 0; m < M; ++m) sum += sm.loads[r * M + m];
-        sm.rank_load[r] = sum;
-        sm.next_slot[r] = 0;
-    }
-    __syncthreads();
-    // ranks by load descending, ties to the lower index; each rank's masters likewise
-    for (int i = tid; i < G; i += nthreads) {
-        const int mine = sm.rank_load[i];
-        int pos = 0;
-        for (int j = 0; j < G; ++j) {
-            const int other = sm.rank_load[j];
-            pos += (other > mine || (other == mine && j < i)) ? 1 : 0;
-        }
-        sm.source_order[pos] = i;
-    }
-    for (int i = tid; i < E; i += nthreads) {
-        const int base = (i / M) * M;
-        const int mine = sm.loads[i];
-        int pos = 0;
-        for (int j = base; j < base + M; ++j) {
-            const int other = sm.loads[j];
-            pos += (other > mine || (other == mine && j < i)) ? 1 : 0;
-        }
-        sm.sorted_experts[base + pos] = i;
-    }
+    if (tid == 0) sm.ctrl[kCtlNumExports] = 0;
+    if (tid < kSolverProbeWarps) sm.ctrl[kCtlStop0 + tid] = 0;
     const bool do_search = (R > 0 && G > 1);
-    if (tid == 0) {
-        sm.ctrl[kCtlNumExports] = 0;
-        sm.ctrl[kCtlFastDone] = 0;
-        sm.ctrl[kCtlPrecheckDone] = 0;
-        if (do_search) {
+    stamp(1);
+    if (!do_search) {
+        clear_outputs(tid, nthreads);
+    } else {
+        __syncthreads();
+        for (int r = tid; r < G; r += nthreads) {
+            int sum = 0;
+#pragma unroll 8
+            for (int m = 0; m < M; ++m) sum += sm.loads[r * M + m];
+            sm.rank_load[r] = sum;
+            sm.next_slot[r] = 0;
+        }
+        for (int i = tid; i < E; i += nthreads) {  // each rank's masters by load descending, ties to the lower index
+            const int base = (i / M) * M;
+            const int mine = sm.loads[i];
+            int pos = 0;
+#pragma unroll 8
+            for (int j = base; j < base + M; ++j) {
+                const int other = sm.loads[j];
+                pos += (other > mine || (other == mine && j < i)) ? 1 : 0;
+            }
+            sm.sorted_experts[base + pos] = i;
+        }
+        __syncthreads();
+        for (int i = tid; i < G; i += nthreads) {  // the ranks likewise
+            const int mine = sm.rank_load[i];
+            int above = 0, below = 0, equal = 0;
+#pragma unroll 8
+            for (int j = 0; j < G; ++j) {
+                const int other = sm.rank_load[j];
+                above += other > mine ? 1 : 0;
+                below += other < mine ? 1 : 0;
+                equal += (other == mine && j < i) ? 1 : 0;
+            }
+            sm.source_order[above + equal] = i;
+            sm.sink_order[below + equal] = i;
+        }
+        if (warp == 0) {
             int total = 0, mx = 0;
-            for (int r = 0; r < G; ++r) {
+            for (int r = lane; r < G; r += kWarp) {
                 total += sm.rank_load[r];
                 mx = max(mx, sm.rank_load[r]);
             }
+            total = warp_sum(total);
+            mx = warp_max(mx);
             // fp32, in the reference's order: ceilf((float(total) / G) * bt)
             const float bt = fmaxf(a.balance_threshold, 1.0f);
             const float mean = __fdiv_rn(static_cast<float>(total), static_cast<float>(G));
             const int lo = static_cast<int>(ceilf(__fmul_rn(mean, bt)));
-            sm.ctrl[kCtlLo] = lo;
-            sm.ctrl[kCtlHi] = max(mx, lo);
-        }
-    }
-    __syncthreads();
-
-    stamp(2);
-    const bool allow0 = a.allow_zero_master != 0;
-    if (do_search) {
-        if (warp == 0) {  // fast path: up to three builds with the dynamic floor
-            const int lo = sm.ctrl[kCtlLo], hi = sm.ctrl[kCtlHi];
-            const float eps = fmaxf(a.eps, 0.0f);
-            int thr = static_cast<int>(ceilf(__fmul_rn(static_cast<float>(lo), __fadd_rn(1.0f, eps))));
-            thr = max(thr, lo);
-            const int step = max(1, (hi + 99) / 100);
-            bool done = false;
-            for (int retry = 0; retry <= 2 && !done; ++retry) {
-                int n = 0;
-                done = warp_build_plan<NS, true>(sm, sm.export_sum, sm.occ, sm.plan, n, thr, E, G, M, R, a.min_tokens,
-                                                 allow0, true, lane);
-                if (done) {
-                    if (lane == 0) {
-                        sm.ctrl[kCtlNumExports] = n;
-                        sm.ctrl[kCtlFastDone] = 1;
-                        sm.ctrl[kCtlLo] = thr;
-                    }
-                } else {
-                    thr = min(hi, thr + step);
-                }
-                __syncwarp();
+            if (lane == 0) {
+                sm.ctrl[kCtlLo] = lo;
+                sm.ctrl[kCtlHi] = max(mx, lo);
             }
         }
         __syncthreads();
-        if (!sm.ctrl[kCtlFastDone]) {
-            if (warp == 0) {
-                int lo = sm.ctrl[kCtlLo], hi = sm.ctrl[kCtlHi];
-                while (lo < hi) {  // capacity bisection
+    }
+    stamp(2);
+    const bool allow0 = a.allow_zero_master != 0;
+    int winner = 0;  // the warp whose plan is taken
+    if (do_search) {
+        // The serial search is: up to three builds with the dynamic floor at rising thresholds; then one build at the
+        // smallest threshold the capacities allow; then the probes below. The first four run at once, one warp each; one that
+        // succeeds stops those behind it.
+        const int lo0 = sm.ctrl[kCtlLo], hi0 = sm.ctrl[kCtlHi];
+        if (warp < kSolverProbeWarps) {
+            int thr;
+            const volatile int* stop = sm.ctrl + kCtlStop0 + warp;
+            const bool fast = warp < kSolverProbeWarps - 1;
+            if (fast) {
+                const float eps = fmaxf(a.eps, 0.0f);
+                thr = max(static_cast<int>(ceilf(__fmul_rn(static_cast<float>(lo0), __fadd_rn(1.0f, eps)))), lo0);
+                const int step = max(1, (hi0 + 99) / 100);
+                for (int i = 0; i < warp; ++i) thr = min(hi0, thr + step);
+            } else {
+                int lo = lo0, hi = hi0;
+                while (lo < hi && __shfl_sync(kFullMask, *stop, 0) == 0) {  // capacity bisection
                     const int probe = lo + ((hi - lo) >> 1);
                     int ex = 0, sl = 0;
                     for (int r = lane; r < G; r += kWarp) {
@@ -521,22 +589,37 @@ __device__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, Dev
                     if (warp_sum(ex) <= warp_sum(sl)) hi = probe;
                     else lo = probe + 1;
                 }
-                int n = 0;
-                const bool ok = warp_build_plan<NS, true>(sm, sm.export_sum, sm.occ, sm.plan, n, lo, E, G, M, R,
-                                                          a.min_tokens, allow0, false, lane);
-                if (lane == 0) {
-                    sm.ctrl[kCtlPrecheckDone] = ok ? 1 : 0;
-                    if (ok) {
-                        sm.ctrl[kCtlNumExports] = n;
-                        sm.ctrl[kCtlLo] = lo;
-                    } else {
-                        sm.ctrl[kCtlLo] = min(lo + 1, sm.ctrl[kCtlHi]);
-                    }
-                }
+                thr = lo;
             }
+            int n = 0;
+            const bool ok = warp_build_plan<NS, true>(sm, sm.export_sum + warp * E, sm.plan + warp * kMaxExportsPerDomain, n, thr, E, G,
+                                                      M, R, a.min_tokens, allow0, fast, lane, stop);
+            if (ok && lane > warp && lane < kSolverProbeWarps) *(sm.ctrl + kCtlStop0 + lane) = 1;
+            if (lane == 0) {
+                sm.ctrl[kCtlProbe0 + warp] = thr;
+                sm.ctrl[kCtlFeasible0 + warp] = ok ? 1 : 0;
+                sm.ctrl[kCtlExports0 + warp] = n;
+            }
+        } else {
+            clear_outputs(tid - kSolverProbeWarps * kWarp, nthreads - kSolverProbeWarps * kWarp);
+        }
+        if (nthreads == kSolverProbeWarps * kWarp) clear_outputs(tid, nthreads);
+        __syncthreads();
+        winner = -1;
+        for (int w = kSolverProbeWarps - 1; w >= 0; --w) {
+            if (sm.ctrl[kCtlFeasible0 + w]) winner = w;
+        }
+        const int precheck_thr = sm.ctrl[kCtlProbe0 + kSolverProbeWarps - 1];
+        const int num_exports = winner >= 0 ? sm.ctrl[kCtlExports0 + winner] : 0;
+        __syncthreads();  // everyone has read the four results
+        if (winner >= 0) {
+            if (tid == 0) sm.ctrl[kCtlNumExports] = num_exports;
+        } else {
+            if (tid == 0) sm.ctrl[kCtlLo] = min(precheck_thr + 1, hi0);
+            winner = 0;
             __syncthreads();
             while (true) {
-                if (sm.ctrl[kCtlPrecheckDone] || sm.ctrl[kCtlLo] >= sm.ctrl[kCtlHi]) break;
+                if (sm.ctrl[kCtlLo] >= sm.ctrl[kCtlHi]) break;
                 __syncthreads();  // everyone has read lo/hi before thread 0 rewrites the probe table
                 if (tid == 0) {
                     const int lo = sm.ctrl[kCtlLo], hi = sm.ctrl[kCtlHi];
@@ -558,8 +641,7 @@ __device__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, Dev
                 __syncthreads();
                 if (warp < kSolverProbeWarps && sm.ctrl[kCtlValid0 + warp]) {
                     int n = 0;
-                    const bool ok = warp_build_plan<NS, false>(sm, sm.export_sum + warp * E, sm.occ + warp * E * NS,
-                                                               nullptr, n, sm.ctrl[kCtlProbe0 + warp], E, G, M, R,
+                    const bool ok = warp_build_plan<NS, false>(sm, nullptr, nullptr, n, sm.ctrl[kCtlProbe0 + warp], E, G, M, R,
                                                                a.min_tokens, allow0, false, lane);
                     if (lane == 0) sm.ctrl[kCtlFeasible0 + warp] = ok ? 1 : 0;
                 }
@@ -597,31 +679,31 @@ __device__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, Dev
                 }
                 __syncthreads();
             }
-            if (!sm.ctrl[kCtlPrecheckDone]) {
-                if (warp == 0) {
-                    int n = 0;
-                    const bool ok = warp_build_plan<NS, true>(sm, sm.export_sum, sm.occ, sm.plan, n, sm.ctrl[kCtlLo], E,
-                                                              G, M, R, a.min_tokens, allow0, false, lane);
-                    if (lane == 0) {
-                        sm.ctrl[kCtlNumExports] = ok ? n : 0;
-                        if (!ok) report_error(status, UEP_DEV_SOLVER_INFEASIBLE, sm.ctrl[kCtlLo]);
-                    }
+            if (warp == 0) {
+                int n = 0;
+                const bool ok = warp_build_plan<NS, true>(sm, sm.export_sum, sm.plan, n, sm.ctrl[kCtlLo], E, G, M, R, a.min_tokens,
+                                                          allow0, false, lane);
+                if (lane == 0) {
+                    sm.ctrl[kCtlNumExports] = ok ? n : 0;
+                    if (!ok) report_error(status, UEP_DEV_SOLVER_INFEASIBLE, sm.ctrl[kCtlLo]);
                 }
-                __syncthreads();
             }
         }
     }
+    __syncthreads();
+    const int32_t* export_sum = sm.export_sum + winner * E;
+    ExportEntry* plan = sm.plan + winner * kMaxExportsPerDomain;
 
     stamp(3);
     // Emit: master quotas, then replicas in plan order. Two tables of the search are free by now
     // and are reused: sorted_experts becomes "first plan entry of this expert" (an expert's
     // exports are consecutive in the plan: they are all made while its one source rank is being
-    // drained), and the probe warps' scratch becomes the list of experts that have replicas.
+    // drained), and another warp's sums become the list of experts that have replicas.
     int* first_entry = sm.sorted_experts;
-    int* multi_list = sm.export_sum + E;
+    int* multi_list = sm.export_sum + (winner + 1) % kSolverProbeWarps * E;
     for (int e = tid; e < E; e += nthreads) {
         const int64_t row = static_cast<int64_t>(domain_start_log + e) * D;
-        const int master_quota = do_search ? (sm.loads[e] - sm.export_sum[e]) : sm.loads[e];
+        const int master_quota = do_search ? (sm.loads[e] - export_sum[e]) : sm.loads[e];
         a.quota[row] = master_quota;
         if (a.physical_loads != nullptr) a.physical_loads[(domain_start_rank + e / M) * Lp + e % M] = master_quota;
     }
@@ -637,7 +719,7 @@ __device__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, Dev
             const bool active = k < n;
             const unsigned amask = __ballot_sync(kFullMask, active);
             if (active) {
-                const ExportEntry entry = sm.plan[k];
+                const ExportEntry entry = plan[k];
                 const unsigned same_e = __match_any_sync(amask, entry.expert_local);
                 const unsigned same_t = __match_any_sync(amask, entry.target_rank_local);
                 const unsigned below = (1u << lane) - 1u;
@@ -657,7 +739,7 @@ __device__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, Dev
                     a.l2p[row + slot] = phys;
                     a.quota[row + slot] = entry.quota;
                     if (a.physical_loads != nullptr) a.physical_loads[phys] = entry.quota;
-                    sm.plan[k].target_rank_local = phys;  // from here on the entry carries the physical id
+                    plan[k].target_rank_local = phys;  // from here on the entry carries the physical id
                 }
             }
             __syncwarp();
@@ -674,7 +756,7 @@ __device__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, Dev
         const int C = min(sm.expert_slot[e], D);
         a.lcnts[l_global] = C;
         if (C == 1) {
-            a.quota_prefix[row] = do_search ? (sm.loads[e] - sm.export_sum[e]) : sm.loads[e];
+            a.quota_prefix[row] = do_search ? (sm.loads[e] - export_sum[e]) : sm.loads[e];
             a.rank_quota_prefix[row] = sm.my_loads[e];
         } else {
             multi_list[atomicAdd(&sm.ctrl[kCtlMultiCount], 1)] = e;
@@ -682,38 +764,51 @@ __device__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, Dev
     }
     __syncthreads();
     const int n_multi = sm.ctrl[kCtlMultiCount];
+    // A lane's replica of the warp's next expert, its host's own load already on the way from L2.
+    struct Replica {
+        int e, C, phys, host, q, own;
+    };
+    auto fetch = [&](int idx) {
+        Replica r{-1, 0, 0, -1 - lane, 0, 0};
+        if (idx >= n_multi) return r;
+        r.e = multi_list[idx];
+        r.C = min(sm.expert_slot[r.e], D);
+        if (lane == 0) {
+            r.phys = (domain_start_rank + r.e / M) * Lp + r.e % M;
+            r.q = sm.loads[r.e] - export_sum[r.e];
+        } else if (lane < r.C && r.C <= kWarp) {
+            const ExportEntry entry = plan[first_entry[r.e] + lane - 1];
+            r.phys = entry.target_rank_local;
+            r.q = entry.quota;
+        }
+        if (lane < r.C && r.C <= kWarp) {
+            r.host = r.phys / Lp;
+            const int64_t at = static_cast<int64_t>(r.host) * L + domain_start_log + r.e;
+            if (a.locality) r.own = a.staged_loads != nullptr ? a.staged_loads[at] : __ldcg(a.loads_per_rank + at);
+        }
+        return r;
+    };
+    Replica next = fetch(warp);
     for (int idx = warp; idx < n_multi; idx += nthreads / kWarp) {
-        const int e = multi_list[idx];
+        const Replica r = next;
+        next = fetch(idx + nthreads / kWarp);
+        const int e = r.e, C = r.C;
         const int l_global = domain_start_log + e;
         const int64_t row = static_cast<int64_t>(l_global) * D;
-        const int C = min(sm.expert_slot[e], D);
-        const int master_quota = sm.loads[e] - sm.export_sum[e];
-        const int master_phys = (domain_start_rank + e / M) * Lp + e % M;
-        const int first = first_entry[e];
-        bool done = false;
         if (C <= kWarp) {
-            int phys = 0, q = 0;
-            if (lane == 0) {
-                phys = master_phys;
-                q = master_quota;
-            } else if (lane < C) {
-                const ExportEntry entry = sm.plan[first + lane - 1];
-                phys = entry.target_rank_local;
-                q = entry.quota;
-            }
-            const int qp = warp_inclusive_scan(q, lane);
+            const int qp = warp_inclusive_scan(r.q, lane);
             if (lane < C) a.quota_prefix[row + lane] = qp;
-            done = warp_rank_quota_prefix(a, l_global, C, sm.my_loads[e], phys, q, Lp, L, lane);
-        }
-        if (!done && lane == 0) {  // more than 32 replicas, or two replicas on one rank: the serial version
+            warp_rank_quota_prefix(a, l_global, C, sm.my_loads[e], r.host, r.q, r.own, lane);
+        } else if (lane == 0) {  // more than 32 replicas: the serial version
             int phys[kMaxRanksPerDomain], q[kMaxRanksPerDomain];
-            phys[0] = master_phys;
-            q[0] = master_quota;
+            phys[0] = r.phys;
+            q[0] = r.q;
             int prefix = 0;
+            const int first = first_entry[e];
             for (int j = 0; j < C; ++j) {
                 if (j > 0) {
-                    phys[j] = sm.plan[first + j - 1].target_rank_local;
-                    q[j] = sm.plan[first + j - 1].quota;
+                    phys[j] = plan[first + j - 1].target_rank_local;
+                    q[j] = plan[first + j - 1].quota;
                 }
                 prefix += q[j];
                 a.quota_prefix[row + j] = prefix;
