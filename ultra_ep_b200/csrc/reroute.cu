@@ -561,14 +561,18 @@ __host__ __device__ inline size_t dense_bwd_smem_bytes(int L, int P) {
 __global__ void __launch_bounds__(kDenseBwdThreads, 8)
 dense_backward_tile_kernel(Batch<DenseBwdArgs> batch, int L, int P, int D, int tile_rows) {
     const DenseBwdArgs& a = batch.a[blockIdx.y];
-    const int64_t r0 = static_cast<int64_t>(blockIdx.x) * tile_rows;
-    if (r0 >= a.T) return;
-    const int rows = min(static_cast<int>(a.T - r0), tile_rows);
+    const int first = static_cast<int>(blockIdx.x) * tile_rows;
+    // Rows from here to the rank's last one, not cut to the tile: everything below compares with it and none of it goes beyond
+    // tile_rows. With min(a.T - r0, tile_rows) and a 64-bit r0 the compiler (12.9.86, under this launch bound) took
+    // tile_rows for the last tile too, so that a height that is no multiple of the tile's wrote behind the output.
+    const int rows = a.T - first;
+    if (rows <= 0) return;
+    const int64_t r0 = first;
     extern __shared__ __align__(128) char smem_raw[];
     int32_t* l2p_s = reinterpret_cast<int32_t*>(smem_raw);
     int32_t* count_s = l2p_s + pad4(L) * kStagedReps;
     uint8_t* bits = reinterpret_cast<uint8_t*>(count_s + pad4(L));
-    const int Pq = pad4(P), quads = L / 4, tasks = quads * ((rows + 7) / 8);  // (the last tile may have fewer)
+    const int Pq = pad4(P), quads = L / 4, tasks = quads * (tile_rows / 8);
     const uint8_t* map = a.map + r0 * L;
     for (int e = threadIdx.x; e < L; e += blockDim.x) cp_async_4(count_s + e, a.lcnts + e);
     if (D >= kStagedReps && D % 4 == 0 && (reinterpret_cast<uintptr_t>(a.l2p) & 15u) == 0) {
