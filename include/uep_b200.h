@@ -140,7 +140,7 @@ int uep_sparse_reroute_i32_static(const int32_t* ids, int32_t* out, int T, int K
                                   void* stream);
 
 /* Row order of the (token,k) entries once grouped by physical expert (stable), and the
- * per-expert row offsets [P+1]. No counterpart in the reference (its dispatcher is external). */
+ * per-expert row offsets [P+1]. pos may be phys_ids. No counterpart in the reference (its dispatcher is external). */
 int uep_dispatch_positions(const int32_t* phys_ids, int64_t num_entries, int P, int32_t* pos,
                            int32_t* expert_offsets, int32_t* scratch, void* stream);
 int64_t uep_dispatch_scratch_elems(int64_t num_entries, int P);

@@ -108,10 +108,10 @@ def cuda_histogram(x, L, kind):
     return loads
 
 
-def cuda_dispatch_positions(phys, P):
+def cuda_dispatch_positions(phys, P, in_place=False):
     L_ = capi.lib()
     n = phys.numel()
-    pos = torch.full((n,), -1, dtype=torch.int32, device=phys.device)
+    pos = phys if in_place else torch.full((n,), -1, dtype=torch.int32, device=phys.device)
     offsets = torch.full((P + 1,), -1, dtype=torch.int32, device=phys.device)
     scratch = torch.empty(int(L_.uep_dispatch_scratch_elems(n, P)), dtype=torch.int32, device=phys.device)
     capi.check(L_.uep_dispatch_positions(phys.data_ptr(), n, P, pos.data_ptr(), offsets.data_ptr(),

@@ -65,12 +65,13 @@ def test_interleave_of_large_products(native_lib, cuda_device):
         assert np.array_equal(got.cpu().numpy(), O.sparse_reroute(ids, plan, True)), total
 
 
-@pytest.mark.parametrize("n,P", [(512, 31), (513, 32), (16385, 80), (65537, 160), (262145, 80), (40000, 4500)])
-def test_dispatch_positions_split_edges(native_lib, cuda_device, n, P):
+@pytest.mark.parametrize("n,P", [(512, 31), (513, 32), (16385, 80), (65537, 160), (262145, 80), (40000, 4500), (4097, 5000)])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_dispatch_positions_split_edges(native_lib, cuda_device, n, P, in_place):
     rng = np.random.default_rng(n)
     phys = np.minimum(rng.zipf(1.3, size=n) - 1, P + 3).astype(np.int32)  # hot experts first, some keys outside [0, P)
     phys[n // 3] = -7
     exp_pos, exp_off = O.dispatch_positions(phys, P)
-    pos, off = G.cuda_dispatch_positions(torch.from_numpy(phys).to(cuda_device), P)
+    pos, off = G.cuda_dispatch_positions(torch.from_numpy(phys).to(cuda_device), P, in_place)
     assert np.array_equal(pos.cpu().numpy(), exp_pos)
     assert np.array_equal(off.cpu().numpy(), exp_off)

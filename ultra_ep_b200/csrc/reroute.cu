@@ -756,11 +756,12 @@ __global__ void __launch_bounds__(kOrdThreads) dispatch_count_kernel(const int32
 }
 
 // Positions of the (token, k) entries once grouped by physical expert (stable) and the experts' row offsets: the
-// same ordinals, plus a scan of the grand totals over the experts. Keys outside [0, P) go to a group at the end.
+// same ordinals, plus a scan of the grand totals over the experts. Keys outside [0, P) go to a group at the end. pos may be
+// phys itself, as in the sparse reroute.
 template <int EPT>
 __global__ void __launch_bounds__(kOrdThreads) __maxnreg__(EPT > 4 ? 128 : 80)
-dispatch_positions_kernel(const int32_t* __restrict__ phys, int64_t n, int ctas, int P, const int32_t* __restrict__ table,
-                          int32_t* __restrict__ pos, int32_t* __restrict__ expert_offsets) {
+dispatch_positions_kernel(const int32_t* phys, int64_t n, int ctas, int P, const int32_t* __restrict__ table, int32_t* pos,
+                          int32_t* __restrict__ expert_offsets) {
     extern __shared__ __align__(128) char smem_raw[];
     __shared__ int warp_tot[kOrdWarps];
     const int nb = P + 1;
@@ -1080,6 +1081,7 @@ OrdGrid ord_grid(int64_t n, int ranks, bool in_place, int threads) {
     if (n <= row) return g;
     g.per_lane = n > kOrdRecountMax ? 16 : 4;
     g.table = n > 4 * row && (in_place || ranks > 1 || n > kOrdRecountMax);
+    if (g.table && threads < kOrdThreads) g.per_lane = 16;  // the scratch buffer has room for tiles of kSparseTileEntries
     if (g.table && ranks > 1) {
         g.ctas = 1;
         row = threads;
@@ -1301,7 +1303,9 @@ int uep_dispatch_positions(const int32_t* phys_ids, int64_t num_entries, int P, 
         return UEP_OK;
     }
     if (!phys_ids || !pos || !scratch) return fail(UEP_ERR_INVALID, "dispatch_positions: null pointer");
-    const OrdGrid g = ord_grid(num_entries, 1, false, ord_smem_bytes(P + 1, kOrdThreads) <= kMaxCtaSmem ? kOrdThreads : kOrdFewThreads);
+    const uintptr_t x = reinterpret_cast<uintptr_t>(phys_ids), y = reinterpret_cast<uintptr_t>(pos), bytes = sizeof(int32_t) * num_entries;
+    const bool in_place = x < y + bytes && y < x + bytes;
+    const OrdGrid g = ord_grid(num_entries, 1, in_place, ord_smem_bytes(P + 1, kOrdThreads) <= kMaxCtaSmem ? kOrdThreads : kOrdFewThreads);
     const size_t smem = ord_smem_bytes(P + 1, g.threads), smem1 = sizeof(int32_t) * (P + 1);
     const bool overlap = g.table && pdl_enabled();
     if (g.table) {
