@@ -385,6 +385,11 @@ struct DenseRerouteBackward : public torch::autograd::Node {
 
 std::tuple<torch::Tensor, torch::Tensor> dense_reroute(const std::shared_ptr<Manager>& manager, int layer_id, torch::Tensor probs,
                                                        torch::Tensor routing_map) {
+    // the node knows the backward only, and the outputs are built below autograd, where a tangent would be lost without a word
+    if (probs._fw_grad(/*level=*/0).defined()) {
+        PyErr_SetString(PyExc_NotImplementedError, "reroute: forward-mode differentiation is not implemented");
+        throw py::error_already_set();
+    }
     torch::Tensor in = probs, map = routing_map;
     std::tuple<torch::Tensor, torch::Tensor> out;
     {
