@@ -410,7 +410,9 @@ std::tuple<torch::Tensor, torch::Tensor> dense_reroute(const std::shared_ptr<Man
 
 // ---- groups hosted on one device (ultra_ep_b200/sim.py) -------------------------------------
 // The same C ABI entry points with one list element per hosted rank. They return the status code (the caller raises
-// with the library's message); building the pointer arrays in Python cost more than the launches.
+// with the library's message); building the pointer arrays in Python cost more than the launches. Each lets go of the
+// interpreter lock for the library's call and for allocations: both can wait for the device (a full launch queue, a
+// scratch buffer that grows).
 constexpr int kMaxHosted = 8;
 
 struct RankList {
@@ -434,6 +436,11 @@ struct RankList {
         }
     }
 };
+template <typename F>
+auto unlocked(F f) {
+    py::gil_scoped_release released;
+    return f();
+}
 uep_manager* group_of(uintptr_t handle) { return reinterpret_cast<uep_manager*>(handle); }
 // int64 device tables of raw addresses, or null where there are none
 const int64_t* const* tables_of(const RankList& l) { return l.n > 0 ? reinterpret_cast<const int64_t* const*>(l.ptr) : nullptr; }
@@ -441,50 +448,66 @@ const int64_t* const* tables_of(const RankList& l) { return l.n > 0 ? reinterpre
 int group_update_placement(uintptr_t handle, int layer, const py::object& inputs) {
     const RankList in(inputs);
     const int kind = in.first.scalar_type() == torch::kBool ? 0 : (in.first.scalar_type() == torch::kInt32 ? 1 : 2);
-    return uep_update_placement(group_of(handle), layer, kind, in.ptr, in.rows, static_cast<int>(in.first.size(1)), current_stream());
+    const int cols = static_cast<int>(in.first.size(1));
+    return unlocked([&] { return uep_update_placement(group_of(handle), layer, kind, in.ptr, in.rows, cols, current_stream()); });
 }
 
 std::tuple<int, uintptr_t> group_weight_sync(uintptr_t handle, int layer, const py::object& fc1, const py::object& fc2,
                                              const py::object& fc1_scale, const py::object& fc2_scale, bool async_finish) {
     const RankList a(fc1), b(fc2), c(fc1_scale), d(fc2_scale);
     uep_event* done = nullptr;
-    const int rc = uep_weight_sync(group_of(handle), layer, tables_of(a), tables_of(b), tables_of(c), tables_of(d), nullptr, async_finish,
-                                   current_stream(), &done);
+    const int rc = unlocked([&] {
+        return uep_weight_sync(group_of(handle), layer, tables_of(a), tables_of(b), tables_of(c), tables_of(d), nullptr, async_finish,
+                               current_stream(), &done);
+    });
     return {rc, reinterpret_cast<uintptr_t>(done)};
 }
 
 std::tuple<int, uintptr_t> group_grad_reduce(uintptr_t handle, int layer, const py::object& fc1, const py::object& fc2, bool async_finish) {
     const RankList a(fc1), b(fc2);
     uep_event* done = nullptr;
-    const int rc = uep_grad_reduce(group_of(handle), layer, tables_of(a), tables_of(b), nullptr, async_finish, current_stream(), &done);
+    const int rc = unlocked([&] {
+        return uep_grad_reduce(group_of(handle), layer, tables_of(a), tables_of(b), nullptr, async_finish, current_stream(), &done);
+    });
     return {rc, reinterpret_cast<uintptr_t>(done)};
 }
 
 int group_wait_event(uintptr_t event) {
     uep_event* ev = reinterpret_cast<uep_event*>(event);
-    const int rc = uep_event_stream_wait(ev, current_stream());
-    if (rc == UEP_OK) uep_event_destroy(ev);
-    return rc;
+    return unlocked([&] {
+        const int rc = uep_event_stream_wait(ev, current_stream());
+        if (rc == UEP_OK) uep_event_destroy(ev);
+        return rc;
+    });
 }
 
 std::tuple<int, py::object> group_reroute_sparse(uintptr_t handle, int layer, const py::object& ids, py::object out) {
     const RankList in(ids);
     if (out.is_none()) {
-        py::list made;
-        for (const auto& item : py::reinterpret_borrow<py::sequence>(ids)) made.append(torch::empty_like(THPVariable_Unpack(item.ptr())));
-        out = made;
+        std::vector<torch::Tensor> tensors;
+        for (const auto& item : py::reinterpret_borrow<py::sequence>(ids)) tensors.push_back(THPVariable_Unpack(item.ptr()));
+        unlocked([&] {
+            for (auto& t : tensors) t = torch::empty_like(t);
+        });
+        out = py::cast(tensors);
     }
     const RankList to(out);
     const int kind = in.first.scalar_type() == torch::kInt32 ? 1 : 2;
-    const int rc = uep_reroute_sparse(group_of(handle), layer, kind, in.ptr, const_cast<void* const*>(to.ptr), in.rows,
-                                      static_cast<int>(in.first.size(1)), current_stream());
+    const int cols = static_cast<int>(in.first.size(1));
+    const int rc = unlocked([&] {
+        return uep_reroute_sparse(group_of(handle), layer, kind, in.ptr, const_cast<void* const*>(to.ptr), in.rows, cols, current_stream());
+    });
     return {rc, out};
 }
 
 // One tensor [rows[i], cols] per hosted rank.
 py::list empty_like_ranks(const RankList& like, int64_t cols, torch::ScalarType dtype) {
+    std::vector<torch::Tensor> tensors(like.n);
+    unlocked([&] {
+        for (int i = 0; i < like.n; ++i) tensors[i] = empty_2d(like.rows[i], cols, dtype, like.first.device());
+    });
     py::list made;
-    for (int i = 0; i < like.n; ++i) made.append(empty_2d(like.rows[i], cols, dtype, like.first.device()));
+    for (const auto& t : tensors) made.append(t);
     return made;
 }
 
@@ -496,9 +519,11 @@ std::tuple<int, py::object, py::object> group_reroute_dense(uintptr_t handle, in
         out_probs = empty_like_ranks(m, P, torch::kFloat32);
     }
     const RankList op(out_probs), om(out_maps);
-    const int rc = uep_reroute_dense_forward(group_of(handle), layer, reinterpret_cast<const uint8_t* const*>(m.ptr),
-                                             reinterpret_cast<const float* const*>(p.ptr), reinterpret_cast<uint8_t* const*>(const_cast<void* const*>(om.ptr)),
-                                             reinterpret_cast<float* const*>(const_cast<void* const*>(op.ptr)), m.rows, current_stream());
+    const int rc = unlocked([&] {
+        return uep_reroute_dense_forward(group_of(handle), layer, reinterpret_cast<const uint8_t* const*>(m.ptr),
+                                         reinterpret_cast<const float* const*>(p.ptr), reinterpret_cast<uint8_t* const*>(const_cast<void* const*>(om.ptr)),
+                                         reinterpret_cast<float* const*>(const_cast<void* const*>(op.ptr)), m.rows, current_stream());
+    });
     return {rc, out_probs, out_maps};
 }
 
@@ -507,9 +532,11 @@ std::tuple<int, py::object> group_reroute_dense_backward(uintptr_t handle, int l
     const RankList g(grads), m(maps), em(expanded_maps);
     py::object out = empty_like_ranks(m, L, torch::kFloat32);
     const RankList to(out);
-    const int rc = uep_reroute_dense_backward(group_of(handle), layer, reinterpret_cast<const float* const*>(g.ptr),
-                                              reinterpret_cast<const uint8_t* const*>(m.ptr), reinterpret_cast<const uint8_t* const*>(em.ptr),
-                                              reinterpret_cast<float* const*>(const_cast<void* const*>(to.ptr)), m.rows, P, current_stream());
+    const int rc = unlocked([&] {
+        return uep_reroute_dense_backward(group_of(handle), layer, reinterpret_cast<const float* const*>(g.ptr),
+                                          reinterpret_cast<const uint8_t* const*>(m.ptr), reinterpret_cast<const uint8_t* const*>(em.ptr),
+                                          reinterpret_cast<float* const*>(const_cast<void* const*>(to.ptr)), m.rows, P, current_stream());
+    });
     return {rc, out};
 }
 
