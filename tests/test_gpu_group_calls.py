@@ -50,3 +50,41 @@ def test_other_threads_run_while_a_call_waits(group, cuda_device):
     assert end - begin > 0.1, "the call did not wait: this test shows nothing"
     inside = [b for b in beats if begin < b < end]
     assert len(inside) > 0.1 * (end - begin) / 0.002
+
+
+def test_any_iterable_of_tensors_is_taken(group, cuda_device):
+    tokens = [33, 70]
+    ids = _ids(tokens, cuda_device)
+    maps = [torch.zeros((t, L), dtype=torch.bool, device=cuda_device).scatter_(1, x.long(), True) for t, x in zip(tokens, ids)]
+    probs = [torch.rand(m.shape, device=cuda_device) * m for m in maps]
+    group.update_placement(0, maps)
+    exp_probs, exp_maps = group.reroute_dense(0, maps, probs)
+    exp_grads = group.reroute_dense_backward(0, exp_probs, maps, exp_maps)
+    exp_ids = group.reroute_sparse(0, ids)
+    as_dict = lambda ts: dict(enumerate(ts)).values()  # noqa: E731
+    host = lambda ts: [t.cpu().pin_memory() for t in ts]  # noqa: E731
+    spare = [torch.zeros((4, L), dtype=torch.bool, device=cuda_device)] * 9
+    for got_probs, got_maps in (group.reroute_dense(0, tuple(maps), (p for p in probs)), group.reroute_dense(0, as_dict(maps), probs),
+                                group.reroute_dense(0, maps + spare, probs + [s.float() for s in spare]),
+                                group.reroute_dense(0, host(maps), host(probs))):
+        assert all(torch.equal(a, b) for a, b in zip(got_probs, exp_probs)) and all(torch.equal(a, b) for a, b in zip(got_maps, exp_maps))
+        assert got_probs[0].is_cuda and got_maps[0].is_cuda
+    grads = group.reroute_dense_backward(0, as_dict(exp_probs), (m for m in maps), tuple(exp_maps))
+    assert all(torch.equal(a, b) for a, b in zip(grads, exp_grads))
+    assert all(torch.equal(a, b) for a, b in zip(group.reroute_sparse(0, tuple(ids), tuple(torch.empty_like(x) for x in ids)), exp_ids))
+    same = torch.stack([ids[0], ids[0]])
+    assert torch.equal(group.reroute_sparse(0, same)[0], exp_ids[0])
+    with pytest.raises(TypeError):
+        group.reroute_sparse(0, [ids[0], 3])
+    for call in (lambda: group.reroute_sparse(0, ids[:1]), lambda: group.update_placement(0, ids[:1]), lambda: group.reroute_dense(0, maps, probs[:1])):
+        with pytest.raises(ValueError):
+            call()
+
+
+def test_events_are_waited_for_by_address_too(group, cuda_device):
+    group.update_placement(0, _ids([8, 8], cuda_device))
+    tables = group.pointer_tables([[torch.zeros(1, device=cuda_device)] * (L // 2)] * 2)
+    group.wait_event(group.weight_sync(0, tables, tables, async_finish=True))
+    group.wait_event(group.weight_sync(0, iter(tables), tables, async_finish=True).value)
+    with pytest.raises(RuntimeError):
+        group.wait_event(None)

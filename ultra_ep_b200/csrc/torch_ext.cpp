@@ -16,6 +16,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/extension.h>
+#include <c10/util/SmallVector.h>
 
 #include <cstdio>
 #include <cstring>
@@ -415,25 +416,36 @@ std::tuple<torch::Tensor, torch::Tensor> dense_reroute(const std::shared_ptr<Man
 // scratch buffer that grows).
 constexpr int kMaxHosted = 8;
 
+// The tensors of any iterable, one per hosted rank; what comes behind the last rank's is ignored.
 struct RankList {
-    const void* ptr[kMaxHosted] = {nullptr};
-    int rows[kMaxHosted] = {0};
+    c10::SmallVector<const void*, kMaxHosted> ptr;
+    c10::SmallVector<int, kMaxHosted> rows;
+    py::object items;
     at::Tensor first;
     int n = 0;
 
-    explicit RankList(const py::handle& seq) {
+    RankList(uintptr_t group, const py::handle& seq) : ptr(kMaxHosted, nullptr), rows(kMaxHosted, 0) {
         if (seq.is_none()) return;
-        const py::sequence items = py::reinterpret_borrow<py::sequence>(seq);
-        n = static_cast<int>(py::len(items));
-        if (n > kMaxHosted) throw std::runtime_error("at most 8 ranks can be hosted on one device");
+        items = py::reinterpret_steal<py::object>(PySequence_Fast(seq.ptr(), "expected one tensor per hosted rank"));
+        if (!items) throw py::error_already_set();
+        n = static_cast<int>(PySequence_Fast_GET_SIZE(items.ptr()));
+        if (group != 0 && n < uep_manager_num_local(reinterpret_cast<uep_manager*>(group)))
+            throw py::value_error("fewer tensors than hosted ranks");
+        if (n > kMaxHosted) {
+            ptr.resize(n);
+            rows.resize(n);
+        }
         for (int i = 0; i < n; ++i) {
-            const py::object item = items[i];
-            if (!THPVariable_Check(item.ptr())) throw py::type_error("expected one tensor per hosted rank");
-            const at::Tensor& t = THPVariable_Unpack(item.ptr());
+            const at::Tensor& t = at(i);
             if (i == 0) first = t;
             ptr[i] = t.data_ptr();
             rows[i] = t.dim() > 0 ? static_cast<int>(t.size(0)) : 0;
         }
+    }
+    const at::Tensor& at(int i) const {
+        PyObject* item = PySequence_Fast_GET_ITEM(items.ptr(), i);
+        if (!THPVariable_Check(item)) throw py::type_error("expected one tensor per hosted rank");
+        return THPVariable_Unpack(item);
     }
 };
 template <typename F>
@@ -443,18 +455,18 @@ auto unlocked(F f) {
 }
 uep_manager* group_of(uintptr_t handle) { return reinterpret_cast<uep_manager*>(handle); }
 // int64 device tables of raw addresses, or null where there are none
-const int64_t* const* tables_of(const RankList& l) { return l.n > 0 ? reinterpret_cast<const int64_t* const*>(l.ptr) : nullptr; }
+const int64_t* const* tables_of(const RankList& l) { return l.n > 0 ? reinterpret_cast<const int64_t* const*>(l.ptr.data()) : nullptr; }
 
 int group_update_placement(uintptr_t handle, int layer, const py::object& inputs) {
-    const RankList in(inputs);
+    const RankList in(handle, inputs);
     const int kind = in.first.scalar_type() == torch::kBool ? 0 : (in.first.scalar_type() == torch::kInt32 ? 1 : 2);
     const int cols = static_cast<int>(in.first.size(1));
-    return unlocked([&] { return uep_update_placement(group_of(handle), layer, kind, in.ptr, in.rows, cols, current_stream()); });
+    return unlocked([&] { return uep_update_placement(group_of(handle), layer, kind, in.ptr.data(), in.rows.data(), cols, current_stream()); });
 }
 
 std::tuple<int, uintptr_t> group_weight_sync(uintptr_t handle, int layer, const py::object& fc1, const py::object& fc2,
                                              const py::object& fc1_scale, const py::object& fc2_scale, bool async_finish) {
-    const RankList a(fc1), b(fc2), c(fc1_scale), d(fc2_scale);
+    const RankList a(handle, fc1), b(handle, fc2), c(handle, fc1_scale), d(handle, fc2_scale);
     uep_event* done = nullptr;
     const int rc = unlocked([&] {
         return uep_weight_sync(group_of(handle), layer, tables_of(a), tables_of(b), tables_of(c), tables_of(d), nullptr, async_finish,
@@ -464,7 +476,7 @@ std::tuple<int, uintptr_t> group_weight_sync(uintptr_t handle, int layer, const 
 }
 
 std::tuple<int, uintptr_t> group_grad_reduce(uintptr_t handle, int layer, const py::object& fc1, const py::object& fc2, bool async_finish) {
-    const RankList a(fc1), b(fc2);
+    const RankList a(handle, fc1), b(handle, fc2);
     uep_event* done = nullptr;
     const int rc = unlocked([&] {
         return uep_grad_reduce(group_of(handle), layer, tables_of(a), tables_of(b), nullptr, async_finish, current_stream(), &done);
@@ -482,60 +494,61 @@ int group_wait_event(uintptr_t event) {
 }
 
 std::tuple<int, py::object> group_reroute_sparse(uintptr_t handle, int layer, const py::object& ids, py::object out) {
-    const RankList in(ids);
+    const RankList in(handle, ids);
     if (out.is_none()) {
-        std::vector<torch::Tensor> tensors;
-        for (const auto& item : py::reinterpret_borrow<py::sequence>(ids)) tensors.push_back(THPVariable_Unpack(item.ptr()));
+        std::vector<torch::Tensor> tensors(in.n);
         unlocked([&] {
-            for (auto& t : tensors) t = torch::empty_like(t);
+            for (int i = 0; i < in.n; ++i) tensors[i] = torch::empty_like(in.at(i));
         });
         out = py::cast(tensors);
     }
-    const RankList to(out);
+    const RankList to(handle, out);
     const int kind = in.first.scalar_type() == torch::kInt32 ? 1 : 2;
     const int cols = static_cast<int>(in.first.size(1));
     const int rc = unlocked([&] {
-        return uep_reroute_sparse(group_of(handle), layer, kind, in.ptr, const_cast<void* const*>(to.ptr), in.rows, cols, current_stream());
+        return uep_reroute_sparse(group_of(handle), layer, kind, in.ptr.data(), const_cast<void* const*>(to.ptr.data()), in.rows.data(), cols, current_stream());
     });
     return {rc, out};
 }
 
-// One tensor [rows[i], cols] per hosted rank.
-py::list empty_like_ranks(const RankList& like, int64_t cols, torch::ScalarType dtype) {
+// One tensor [rows[i], cols] per hosted rank, on the group's device (the inputs may lie in mapped host memory).
+py::list empty_like_ranks(const RankList& like, int64_t cols, torch::ScalarType dtype, const torch::Device& device) {
     std::vector<torch::Tensor> tensors(like.n);
     unlocked([&] {
-        for (int i = 0; i < like.n; ++i) tensors[i] = empty_2d(like.rows[i], cols, dtype, like.first.device());
+        for (int i = 0; i < like.n; ++i) tensors[i] = empty_2d(like.rows[i], cols, dtype, device);
     });
     py::list made;
     for (const auto& t : tensors) made.append(t);
     return made;
 }
 
-std::tuple<int, py::object, py::object> group_reroute_dense(uintptr_t handle, int layer, int P, const py::object& maps, const py::object& probs,
-                                                            py::object out_probs, py::object out_maps) {
-    const RankList m(maps), p(probs);
+std::tuple<int, py::object, py::object> group_reroute_dense(uintptr_t handle, int layer, int P, int device_index, const py::object& maps,
+                                                            const py::object& probs, py::object out_probs, py::object out_maps) {
+    const torch::Device device(torch::kCUDA, static_cast<c10::DeviceIndex>(device_index));
+    const RankList m(handle, maps), p(handle, probs);
     if (out_probs.is_none()) {
-        out_maps = empty_like_ranks(m, P, torch::kBool);
-        out_probs = empty_like_ranks(m, P, torch::kFloat32);
+        out_maps = empty_like_ranks(m, P, torch::kBool, device);
+        out_probs = empty_like_ranks(m, P, torch::kFloat32, device);
     }
-    const RankList op(out_probs), om(out_maps);
+    const RankList op(handle, out_probs), om(handle, out_maps);
     const int rc = unlocked([&] {
-        return uep_reroute_dense_forward(group_of(handle), layer, reinterpret_cast<const uint8_t* const*>(m.ptr),
-                                         reinterpret_cast<const float* const*>(p.ptr), reinterpret_cast<uint8_t* const*>(const_cast<void* const*>(om.ptr)),
-                                         reinterpret_cast<float* const*>(const_cast<void* const*>(op.ptr)), m.rows, current_stream());
+        return uep_reroute_dense_forward(group_of(handle), layer, reinterpret_cast<const uint8_t* const*>(m.ptr.data()),
+                                         reinterpret_cast<const float* const*>(p.ptr.data()), reinterpret_cast<uint8_t* const*>(const_cast<void* const*>(om.ptr.data())),
+                                         reinterpret_cast<float* const*>(const_cast<void* const*>(op.ptr.data())), m.rows.data(), current_stream());
     });
     return {rc, out_probs, out_maps};
 }
 
-std::tuple<int, py::object> group_reroute_dense_backward(uintptr_t handle, int layer, int L, int P, const py::object& grads, const py::object& maps,
-                                                         const py::object& expanded_maps) {
-    const RankList g(grads), m(maps), em(expanded_maps);
-    py::object out = empty_like_ranks(m, L, torch::kFloat32);
-    const RankList to(out);
+std::tuple<int, py::object> group_reroute_dense_backward(uintptr_t handle, int layer, int L, int P, int device_index, const py::object& grads,
+                                                         const py::object& maps, const py::object& expanded_maps) {
+    const torch::Device device(torch::kCUDA, static_cast<c10::DeviceIndex>(device_index));
+    const RankList g(handle, grads), m(handle, maps), em(handle, expanded_maps);
+    py::object out = empty_like_ranks(m, L, torch::kFloat32, device);
+    const RankList to(handle, out);
     const int rc = unlocked([&] {
-        return uep_reroute_dense_backward(group_of(handle), layer, reinterpret_cast<const float* const*>(g.ptr),
-                                          reinterpret_cast<const uint8_t* const*>(m.ptr), reinterpret_cast<const uint8_t* const*>(em.ptr),
-                                          reinterpret_cast<float* const*>(const_cast<void* const*>(to.ptr)), m.rows, P, current_stream());
+        return uep_reroute_dense_backward(group_of(handle), layer, reinterpret_cast<const float* const*>(g.ptr.data()),
+                                          reinterpret_cast<const uint8_t* const*>(m.ptr.data()), reinterpret_cast<const uint8_t* const*>(em.ptr.data()),
+                                          reinterpret_cast<float* const*>(const_cast<void* const*>(to.ptr.data())), m.rows.data(), P, current_stream());
     });
     return {rc, out};
 }

@@ -162,7 +162,7 @@ class SimGroup:
         return C.c_void_p(done) if async_finish else None
 
     def wait_event(self, ev):
-        capi.check(self._C.group_wait_event(ev.value or 0), "uep_event_stream_wait")
+        capi.check(self._C.group_wait_event(getattr(ev, "value", ev) or 0), "uep_event_stream_wait")
 
     def reroute_sparse(self, layer: int, ids: Sequence[torch.Tensor], out: Optional[Sequence[torch.Tensor]] = None):
         rc, out = self._C.group_reroute_sparse(self._address(), layer, ids, out)
@@ -172,13 +172,14 @@ class SimGroup:
     def reroute_dense(self, layer: int, maps: Sequence[torch.Tensor], probs: Sequence[torch.Tensor], out=None):
         """out: optional (out_probs, out_maps) lists to write into instead of allocating."""
         out_probs, out_maps = out if out is not None else (None, None)
-        rc, out_probs, out_maps = self._C.group_reroute_dense(self._address(), layer, self.P, maps, probs, out_probs,
-                                                              out_maps)
+        rc, out_probs, out_maps = self._C.group_reroute_dense(self._address(), layer, self.P, self.device.index, maps, probs,
+                                                              out_probs, out_maps)
         capi.check(rc, "uep_reroute_dense_forward")
         return out_probs, out_maps
 
     def reroute_dense_backward(self, layer: int, grads, maps, expanded_maps):
-        rc, outs = self._C.group_reroute_dense_backward(self._address(), layer, self.L, self.P, grads, maps, expanded_maps)
+        rc, outs = self._C.group_reroute_dense_backward(self._address(), layer, self.L, self.P, self.device.index, grads, maps,
+                                                        expanded_maps)
         capi.check(rc, "uep_reroute_dense_backward")
         return outs
 
