@@ -40,6 +40,27 @@ def test_no_compute_without_gpu_but_clean_errors(native_lib):
     assert native_lib.uep_reroute_scratch_elems(8192, 0, 128) == 128 * 128 + 4
 
 
+def test_shared_memory_grants_belong_to_a_kernel_and_a_device(tmp_path):
+    """What one device's kernel was granted says nothing about the next device's."""
+    src, exe = tmp_path / "grants.cpp", tmp_path / "grants"
+    src.write_text('''
+#include "smem_grants.h"
+int main() {
+    static uep::SmemGrants g;
+    int a, b;
+    g.grant(&a, 0, 96 << 10);
+    if (g.granted(&a, 0) != 96u << 10) return 1;
+    if (g.granted(&a, 1) != 0 || g.granted(&b, 0) != 0) return 2;
+    g.grant(&a, 1, 64 << 10);
+    g.grant(&a, 0, 128 << 10);
+    if (g.granted(&a, 0) != 128u << 10 || g.granted(&a, 1) != 64u << 10) return 3;
+    for (int dev = 2; dev < 1000; ++dev) g.grant(&b, dev, 1);  // a full table forgets, it does not overflow
+    return g.granted(&a, 0) == 128u << 10 && g.granted(&b, 999) == 0 ? 0 : 4;
+}''')
+    subprocess.check_call(["g++", "-std=c++17", "-I", os.path.join(ROOT, "ultra_ep_b200", "csrc"), str(src), "-o", str(exe)])
+    assert subprocess.call([str(exe)]) == 0
+
+
 def test_tuning_defaults_and_validation(monkeypatch):
     from ultra_ep_b200.config import load_tuning_from_env
 

@@ -26,7 +26,7 @@ LIB_PATH = os.path.join(LIB_DIR, "libuep_b200.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 CUDA_SOURCES = ["host_common.cu", "plan.cu", "reroute.cu", "weight_sync.cu", "grad_reduce.cu", "manager.cu"]
-HEADERS = ["common.cuh", "ordinals.cuh", "solver.cuh", "internal.h", os.path.join(INCLUDE, "uep_b200.h")]
+HEADERS = ["common.cuh", "ordinals.cuh", "solver.cuh", "internal.h", "smem_grants.h", os.path.join(INCLUDE, "uep_b200.h")]
 
 NVCC_FLAGS = [
     "-std=c++17", "-O3", "-lineinfo",

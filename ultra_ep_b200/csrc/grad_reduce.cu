@@ -500,13 +500,8 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
 
 cudaError_t launch_grad_reduce(const ReduceCall& call, cudaStream_t stream) {
     const size_t smem = static_cast<size_t>(kReduceStages + kMasterStages) * kReduceTileBytes + kReduceZeroBytes;
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(grad_reduce_kernel),
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
-        attr_set = true;
-    }
+    cudaError_t e = allow_smem(reinterpret_cast<const void*>(grad_reduce_kernel), smem);
+    if (e != cudaSuccess) return e;
     if (call.nlocal * call.R > kMaxOwned) return cudaErrorInvalidValue;  // more replica slots per launch than the kernel's table holds
     count_launch();
     const dim3 grid(call.nlocal * call.ctas_per_rank), block(kReduceThreads);

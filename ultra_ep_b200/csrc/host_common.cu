@@ -1,9 +1,12 @@
 // Error reporting shared by every C-ABI entry point: integer return codes plus a
 // thread-local message (no exceptions cross the ABI).
+#include <algorithm>
 #include <cstdio>
+#include <mutex>
 #include <string>
 
 #include "internal.h"
+#include "smem_grants.h"
 
 namespace uep {
 namespace {
@@ -29,6 +32,29 @@ int device_sm_count() {
         if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) cached[dev] = n;
     }
     return cached[dev];
+}
+
+// Remembered, because each setting costs about as much as a launch.
+cudaError_t allow_smem(const void* fn, size_t bytes, bool largest_carveout) {
+    if (bytes <= SmemGrants::kDefault && !largest_carveout) return cudaSuccess;
+    static std::mutex mu;
+    static SmemGrants grants;
+    int dev = -1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mu);
+    const size_t have = grants.granted(fn, dev);
+    if (have >= std::max(bytes, SmemGrants::kDefault)) return cudaSuccess;
+    if (have == 0 && largest_carveout) {
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        if (e != cudaSuccess) return e;
+    }
+    if (bytes > SmemGrants::kDefault) {
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+        if (e != cudaSuccess) return e;
+    }
+    grants.grant(fn, dev, std::max(bytes, SmemGrants::kDefault));
+    return cudaSuccess;
 }
 }  // namespace uep
 

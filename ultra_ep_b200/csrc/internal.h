@@ -152,6 +152,8 @@ cudaError_t launch_sparse_reroute(const Batch<SparseArgs>& b, int ids_kind, int 
                                   cudaStream_t stream);
 
 int device_sm_count();  // of the current device; launch sizes are multiples of it
+// Lets a kernel use that much dynamic shared memory on the current device (and, once, ask for the largest carve-out).
+cudaError_t allow_smem(const void* fn, size_t bytes, bool largest_carveout = false);
 void set_error(const std::string& msg);
 int fail(int code, const std::string& msg);
 int fail_cuda(cudaError_t e, const char* what);

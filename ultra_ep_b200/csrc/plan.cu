@@ -25,9 +25,6 @@
 
 #include <algorithm>
 #include <cstring>
-#include <map>
-#include <mutex>
-#include <utility>
 
 #include "internal.h"
 #include "solver.cuh"
@@ -411,22 +408,6 @@ size_t plan_smem_bytes(int N, int G, int M) {
     return (solver > hist ? solver : hist) + 16;
 }
 
-cudaError_t ensure_smem(const void* fn, size_t bytes) {
-    if (bytes <= 48 * 1024) return cudaSuccess;
-    // remembered per kernel and device: the call costs about as much as a launch
-    static std::mutex mu;
-    static std::map<std::pair<const void*, int>, size_t> granted;
-    int dev = -1;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> lock(mu);
-    size_t& have = granted[{fn, dev}];
-    if (have >= bytes) return cudaSuccess;
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-    if (e == cudaSuccess) have = bytes;
-    return e;
-}
-
 std::atomic<int64_t> g_launches{0};
 
 }  // namespace
@@ -444,7 +425,7 @@ int plan_ctas_per_rank(int input_kind, int max_T, int K_or_L, int nlocal, int nu
 
 cudaError_t launch_plan(const PlanCall& call, cudaStream_t stream) {
     const size_t smem = plan_smem_bytes(call.N, call.G, call.M);
-    cudaError_t e = ensure_smem(reinterpret_cast<const void*>(plan_kernel), smem);
+    cudaError_t e = allow_smem(reinterpret_cast<const void*>(plan_kernel), smem);
     if (e != cudaSuccess) return e;
     const dim3 grid(call.nlocal * call.ctas_per_rank), block(kPlanThreads);
     count_launch();
@@ -479,7 +460,7 @@ static int histogram_common(int kind, const void* input, int T, int K_or_L, int 
     if (input == nullptr) return fail(UEP_ERR_INVALID, "histogram: null input");
     const int ctas = plan_ctas_per_rank(kind, T, K_or_L, 1, std::max(device_sm_count(), 1));
     const size_t smem = sizeof(int32_t) * L;
-    UEP_CUDA_TRY(ensure_smem(reinterpret_cast<const void*>(histogram_kernel), smem));
+    UEP_CUDA_TRY(allow_smem(reinterpret_cast<const void*>(histogram_kernel), smem));
     count_launch();
     histogram_kernel<<<ctas, kPlanThreads, smem, stream>>>(kind, input, T, K_or_L, L, loads);
     UEP_CUDA_TRY(cudaGetLastError());
@@ -534,7 +515,7 @@ int uep_solve_placement(const int32_t* loads_per_rank, int32_t* global_loads_out
     const size_t matrix = sizeof(int32_t) * num_ranks * num_ranks * static_cast<size_t>(M);
     const int staged = nvl_ranks == num_ranks && smem + matrix <= kSolveMaxSmem ? 1 : 0;
     if (staged) smem += matrix;
-    UEP_CUDA_TRY(ensure_smem(reinterpret_cast<const void*>(solve_kernel), smem));
+    UEP_CUDA_TRY(allow_smem(reinterpret_cast<const void*>(solve_kernel), smem));
     count_launch();
     solve_kernel<<<num_ranks / nvl_ranks, kSolveThreads, smem, stream>>>(a, global_loads_out, 1, staged,
                                                                           reinterpret_cast<DeviceStatus*>(status));
@@ -562,7 +543,7 @@ int uep_legacy_solve_placement(const int32_t* global_loads, int32_t* p2l, int32_
     a.balance_threshold = balance_threshold;
     a.legacy = 1;
     const size_t smem = legacy_smem_bytes(nvl_ranks * M, nvl_ranks) + 16;
-    UEP_CUDA_TRY(ensure_smem(reinterpret_cast<const void*>(solve_kernel), smem));
+    UEP_CUDA_TRY(allow_smem(reinterpret_cast<const void*>(solve_kernel), smem));
     count_launch();
     solve_kernel<<<num_ranks / nvl_ranks, kSolveThreads, smem, stream>>>(a, nullptr, 0, 0, reinterpret_cast<DeviceStatus*>(status));
     UEP_CUDA_TRY(cudaGetLastError());

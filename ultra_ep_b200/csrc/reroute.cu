@@ -936,32 +936,10 @@ __global__ void __launch_bounds__(256) gather_rows_plain_kernel(const uint8_t* _
     }
 }
 
-cudaError_t ensure_smem_attr(const void* fn, size_t bytes) {
-    // Remembered per kernel. On first use the kernel also asks for the largest shared-memory carve-out: these
-    // kernels run next to weight_sync, whose CTAs need most of an SM's shared memory, and an SM that was set up
-    // with a small carve-out for a reroute CTA cannot take a weight_sync CTA until it has drained.
-    static std::mutex mu;
-    static const void* fns[32];
-    static size_t granted[32];
-    static int n = 0;
-    std::lock_guard<std::mutex> lock(mu);
-    int i = 0;
-    while (i < n && fns[i] != fn) ++i;
-    if (i == n) {
-        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        if (e != cudaSuccess) return e;
-        if (n < 32) {
-            fns[n] = fn;
-            granted[n] = 48 * 1024;
-            ++n;
-        }
-    }
-    if (bytes <= 48 * 1024 || (i < 32 && granted[i] >= bytes)) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-    if (e != cudaSuccess) return e;
-    if (i < 32) granted[i] = bytes;
-    return cudaSuccess;
-}
+// These kernels also ask for the largest shared-memory carve-out: they run next to weight_sync, whose CTAs need most of an
+// SM's shared memory, and an SM that was set up with a small carve-out for a reroute CTA cannot take a weight_sync CTA
+// until it has drained.
+cudaError_t ensure_smem_attr(const void* fn, size_t bytes) { return allow_smem(fn, bytes, true); }
 
 int dense_tiles(int T) { return (T + kDenseTileRows - 1) / kDenseTileRows; }
 int64_t sparse_tiles(int64_t n) { return (n + kSparseTileEntries - 1) / kSparseTileEntries; }

@@ -955,12 +955,8 @@ cudaError_t launch_weight_sync(const SyncCall& call, cudaStream_t stream) {
     // compact kernel is the same on every rank because N is
     const bool relay = call.relay_min_replicas > 0 && call.N > 2;
     const void* fn = relay ? g.fn_relay : g.fn;
-    static const void* attr_set_for[2] = {nullptr, nullptr};
-    if (attr_set_for[relay] != fn) {
-        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
-        attr_set_for[relay] = fn;
-    }
+    cudaError_t e = allow_smem(fn, smem);
+    if (e != cudaSuccess) return e;
     // Hosted ranks pool their work over all CTAs. Without relaying, the only waits are those of the
     // last CTA, on flags that peers on other devices write. With relaying, CTAs that forward wait for
     // CTAs that send; when both are in this launch (ranks hosted together) they must be co-resident,
@@ -969,7 +965,7 @@ cudaError_t launch_weight_sync(const SyncCall& call, cudaStream_t stream) {
     count_launch();
     SyncCall copy = call;
     void* args[] = {&copy};
-    cudaError_t e = (call.nlocal > 1 && relay) ? cudaLaunchCooperativeKernel(fn, grid, block, args, smem, stream)
+    e = (call.nlocal > 1 && relay) ? cudaLaunchCooperativeKernel(fn, grid, block, args, smem, stream)
                                                : cudaLaunchKernel(fn, grid, block, args, smem, stream);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
