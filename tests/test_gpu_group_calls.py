@@ -1,13 +1,14 @@
 """The calls of a group hosted on one device as Python sees them: what they accept in the place of a list, and that other
 Python threads run while one of them waits for the device."""
 
+import ctypes as C
 import threading
 import time
 
 import pytest
 import torch
 
-from ultra_ep_b200 import sim
+from ultra_ep_b200 import capi, sim
 
 pytestmark = pytest.mark.gpu
 L = 16
@@ -88,3 +89,36 @@ def test_events_are_waited_for_by_address_too(group, cuda_device):
     group.wait_event(group.weight_sync(0, iter(tables), tables, async_finish=True).value)
     with pytest.raises(RuntimeError):
         group.wait_event(None)
+
+
+@pytest.mark.parametrize("managers", [0, 1])
+def test_events_in_flight_and_used_again(native_lib, cuda_device, managers):
+    """More events than the library keeps, given back while another stream still waits for their record, and recorded anew."""
+    held = [sim.SimGroup(sim.make_config(2, 2, 0, 1, is_train=False, sim=True)) for _ in range(managers)]
+    first, second, other = (torch.cuda.Stream() for _ in range(3))
+    n = 40
+    marks, copies = torch.zeros(n, dtype=torch.int64, device=cuda_device), torch.zeros(n, dtype=torch.int64, device=cuda_device)
+    torch.cuda.synchronize()
+    for _ in range(2):
+        marks.zero_()
+        torch.cuda.synchronize()
+        events = []
+        for i in range(n):
+            with torch.cuda.stream(first):
+                torch.cuda._sleep(200_000)
+                marks[i] = i + 1
+            events.append(C.c_void_p())
+            capi.check(native_lib.uep_event_record(first.cuda_stream, C.byref(events[i])))
+        for i, ev in enumerate(events):
+            capi.check(native_lib.uep_event_stream_wait(ev, second.cuda_stream))
+            native_lib.uep_event_destroy(ev)
+            again = C.c_void_p()
+            capi.check(native_lib.uep_event_record(other.cuda_stream, C.byref(again)))
+            capi.check(native_lib.uep_event_synchronize(again))
+            native_lib.uep_event_destroy(again)
+            with torch.cuda.stream(second):
+                copies[i] = marks[i]
+        torch.cuda.synchronize()
+        assert copies.tolist() == list(range(1, n + 1))
+    for g in held:
+        g.destroy()

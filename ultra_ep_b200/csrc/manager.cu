@@ -15,6 +15,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -30,12 +31,14 @@ struct uep_event {
 namespace {
 
 // Ordering events that calls hand out and take back: at most kEventsKept idle ones per device are kept (a create and a
-// destroy per call cost about a microsecond of host time). An idle event may still be waited for by a stream: a wait holds on
-// to the record it was made for, so the event can be recorded anew. Any thread.
+// destroy per call cost about a microsecond of host time) while there is a manager. An idle event may still be waited
+// for by a stream: a wait holds on to the record it was made for, so the event can be recorded anew. Any thread.
 class EventPool {
     static constexpr int kEventsKept = 32, kDevices = 64;
     std::mutex mu_;
-    std::vector<cudaEvent_t> idle_[kDevices];
+    cudaEvent_t idle_[kDevices][kEventsKept];
+    int n_[kDevices] = {0};
+    int managers_ = 0;
 
 public:
     cudaError_t take(uep_event* out) {
@@ -43,10 +46,9 @@ public:
         if (e != cudaSuccess) return e;
         if (out->device < kDevices) {
             std::lock_guard<std::mutex> lock(mu_);
-            auto& idle = idle_[out->device];
-            if (!idle.empty()) {
-                out->ev = idle.back();
-                idle.pop_back();
+            int& n = n_[out->device];
+            if (n > 0) {
+                out->ev = idle_[out->device][--n];
                 return cudaSuccess;
             }
         }
@@ -56,9 +58,9 @@ public:
         if (ev->ev == nullptr) return;
         if (ev->device < kDevices) {
             std::lock_guard<std::mutex> lock(mu_);
-            auto& idle = idle_[ev->device];
-            if (idle.size() < kEventsKept) {
-                idle.push_back(ev->ev);
+            int& n = n_[ev->device];
+            if (managers_ > 0 && n < kEventsKept) {
+                idle_[ev->device][n++] = ev->ev;
                 ev->ev = nullptr;
                 return;
             }
@@ -66,19 +68,34 @@ public:
         cudaEventDestroy(ev->ev);
         ev->ev = nullptr;
     }
+    void manager_made() {
+        std::lock_guard<std::mutex> lock(mu_);
+        ++managers_;
+    }
+    void manager_gone() {
+        std::lock_guard<std::mutex> lock(mu_);
+        if (--managers_ > 0) return;
+        for (int d = 0; d < kDevices; ++d) {
+            while (n_[d] > 0) cudaEventDestroy(idle_[d][--n_[d]]);
+        }
+    }
 };
 EventPool& event_pool() {
-    static EventPool* pool = new EventPool();  // never destroyed: events may be given back while the process exits
+    alignas(EventPool) static char place[sizeof(EventPool)];
+    static EventPool* pool = new (place) EventPool();  // never destroyed: events may be given back while the process exits
     return *pool;
 }
 
 // A recorded event, or the error (then nothing is left behind).
 cudaError_t record_event(cudaStream_t stream, uep_event** out) {
-    uep_event* ev = new uep_event();
+    uep_event* ev = new (std::nothrow) uep_event();
+    if (ev == nullptr) return cudaErrorMemoryAllocation;
     cudaError_t e = event_pool().take(ev);
-    if (e == cudaSuccess) e = cudaEventRecord(ev->ev, stream);
+    if (e == cudaSuccess) {
+        e = cudaEventRecord(ev->ev, stream);
+        if (e != cudaSuccess) cudaEventDestroy(ev->ev);
+    }
     if (e != cudaSuccess) {
-        event_pool().give_back(ev);
         delete ev;
         return e;
     }
@@ -416,6 +433,7 @@ int uep_manager_create(const uep_config* cfg, uep_manager** out) {
     }
     UEP_TRY_BAIL(cudaDeviceSynchronize());
 #undef UEP_TRY_BAIL
+    event_pool().manager_made();
     *out = m;
     return UEP_OK;
 }
@@ -472,6 +490,7 @@ int uep_manager_destroy(uep_manager* m) {
     for (auto e : m->plan_ready) cudaEventDestroy(e);
     cudaFree(m->sync_trace);
     delete m;
+    event_pool().manager_gone();
     return UEP_OK;
 }
 
