@@ -40,6 +40,16 @@ def test_no_compute_without_gpu_but_clean_errors(native_lib):
     assert native_lib.uep_reroute_scratch_elems(8192, 0, 128) == 128 * 128 + 4
 
 
+def test_widths_beyond_shared_memory_are_refused_with_a_message(native_lib):
+    x = 4096  # any address: nothing is launched
+    assert native_lib.uep_sparse_reroute_i32(x, x, 8, 8, 3200, x, x, x, 8, 1, x, None) == -1
+    assert b"too many experts" in native_lib.uep_last_error()
+    assert native_lib.uep_sparse_reroute_i32_static(x, x, 8, 8, 3200, x, x, x, 8, 1, None) == -1
+    assert b"too many experts" in native_lib.uep_last_error()
+    assert native_lib.uep_dispatch_positions(x, 64, 7400, x, x, x, None) == -1
+    assert b"too many experts" in native_lib.uep_last_error()
+
+
 def test_shared_memory_grants_belong_to_a_kernel_and_a_device(tmp_path):
     """What one device's kernel was granted says nothing about the next device's."""
     src, exe = tmp_path / "grants.cpp", tmp_path / "grants"

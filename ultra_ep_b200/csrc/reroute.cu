@@ -32,6 +32,7 @@ namespace {
 
 constexpr int kRerouteThreads = 256;
 constexpr size_t kMaxCtaSmem = 225 * 1024;  // of a CTA
+constexpr size_t kSmemLimit = 227 * 1024;   // what the device gives to one
 constexpr int kDenseTileRows = 64;
 constexpr int kSparseTileEntries = 2048;  // entries of a row of the count table (at least)
 
@@ -1189,12 +1190,18 @@ int uep_dense_reroute_backward(const float* grad_expanded, const uint8_t* routin
     return UEP_OK;
 }
 
+// One message for what would otherwise end in a failed launch.
+static int check_width(size_t smem, const char* what) {
+    return smem <= kSmemLimit ? UEP_OK : fail(UEP_ERR_INVALID, std::string(what) + ": too many experts for the kernel's shared memory");
+}
+
 static int sparse_common(int kind, const void* ids, void* out, int T, int K, int L, const int32_t* l2p,
                          const int32_t* lcnts, const int32_t* rqp, int D, int interleave, int32_t* scratch,
                          void* stream_) {
     if (T < 0 || K < 0 || L <= 0 || D < 1) return fail(UEP_ERR_INVALID, "sparse_reroute: bad sizes");
     if (static_cast<int64_t>(T) * K == 0) return UEP_OK;
     if (!ids || !out || !scratch || !l2p || !lcnts || (interleave != 2 && !rqp)) return fail(UEP_ERR_INVALID, "sparse_reroute: null pointer");
+    if (const int rc = check_width(sparse_smem_bytes(L, false), "sparse_reroute")) return rc;
     Batch<SparseArgs> b{};
     b.n = 1;
     b.a[0] = SparseArgs{ids, out, l2p, lcnts, rqp, scratch, T};
@@ -1225,9 +1232,9 @@ int uep_sparse_reroute_i64(const int64_t* ids, int64_t* out, int T, int K, int L
 //
 // Limits and rules:
 //   * the per-tile counts must fit the array: ceil(T*K / 2048) * L + 4 <= 262144 int32 (1 MiB);
-//     e.g. 131072 entries (16384 tokens x top-8) with up to 4095 experts, or 511 tiles (1,046,528
-//     entries) with 512 experts: the four spare words count against the limit.
-//     Larger problems are refused with UEP_ERR_INVALID and a message, nothing is launched;
+//     e.g. 131072 entries (16384 tokens x top-8) with as many experts as the kernel takes (about 3050, whose counters
+//     fill a CTA's shared memory), or 511 tiles (1,046,528 entries) with 512 experts: the four spare words count against
+//     the limit. Larger problems are refused with UEP_ERR_INVALID and a message, nothing is launched;
 //   * the array is shared by every call on a device and keeps the previous call's counts. The
 //     count pass overwrites every element the second pass reads, so nothing has to start at
 //     zero; but two calls that can overlap on the GPU (different streams without an ordering
@@ -1249,6 +1256,7 @@ int uep_sparse_reroute_i32_static(const int32_t* ids, int32_t* out, int T, int K
                                          std::to_string(kStaticRerouteScratchElems) +
                                          " (use uep_sparse_reroute_i32 with your own scratch)");
     }
+    if (const int rc = check_width(sparse_smem_bytes(L, false), "sparse_reroute_static")) return rc;
     // In host code the array's name is only a handle for the runtime: the address a kernel can
     // use has to be asked for, per device, while that device is current.
     constexpr int kMaxDevices = 64;
@@ -1281,6 +1289,7 @@ int uep_dispatch_positions(const int32_t* phys_ids, int64_t num_entries, int P, 
         return UEP_OK;
     }
     if (!phys_ids || !pos || !scratch) return fail(UEP_ERR_INVALID, "dispatch_positions: null pointer");
+    if (const int rc = check_width(ord_smem_bytes(P + 1, kOrdFewThreads) + sizeof(int32_t) * kOrdWarps, "dispatch_positions")) return rc;
     const uintptr_t x = reinterpret_cast<uintptr_t>(phys_ids), y = reinterpret_cast<uintptr_t>(pos), bytes = sizeof(int32_t) * num_entries;
     const bool in_place = x < y + bytes && y < x + bytes;
     const OrdGrid g = ord_grid(num_entries, 1, in_place, ord_smem_bytes(P + 1, kOrdThreads) <= kMaxCtaSmem ? kOrdThreads : kOrdFewThreads);
