@@ -21,7 +21,7 @@ def _plan(N, M, R, nvl, seed):
     return O.solve_placement(lpr, M, R, nvl, 1 % N, O.SolverParams(min_tokens_per_replica=1)), p
 
 
-@pytest.mark.parametrize("n", [1, 31, 512, 513, 4096, 4097, 16384, 16385, 32769, 65537, 262144, 262145, 300007])
+@pytest.mark.parametrize("n", [1, 31, 512, 513, 4096, 4097, 16384, 16385, 32769, 65537, 262144, 262145, 300007, 1048577])
 @pytest.mark.parametrize("dtype", [np.int32, np.int64])
 def test_sparse_reroute_split_edges(native_lib, cuda_device, n, dtype):
     plan, p = _plan(8, 9, 3, 8, 5)  # 72 experts: not a power of two

@@ -1042,30 +1042,36 @@ cudaError_t launch_dense_backward(const Batch<DenseBwdArgs>& b, int L, int P, in
 //   * the cluster grows to eight CTAs before a thread takes a second entry: 2048 entries 4.5 on four CTAs, 5.7 on one;
 //   * up to 16384 entries one cluster (6.9; two clusters the same), behind it two entries a thread up to eight clusters
 //     (65536 entries 7.8; four entries a thread 8.5, one 9.6) and four beyond (131072: 9.6 against 11.4 with two);
-//   * behind kOrdRecountMax entries the repeated counting is more than a count kernel, and tiles of sixteen entries a
-//     thread keep its table short;
-//   * several ranks in one launch with more than a cluster each: the count kernel and single CTAs. The launch runs beside
-//     weight_sync, which leaves every SM a quarter of its shared memory: single CTAs find room anywhere, clusters of
-//     eight wait for it or keep weight_sync out (65536 entries of eight ranks: the step took 69 us with clusters).
+//   * behind kOrdRecountMax entries, or in place behind one cluster's, a count kernel in front instead of the repeated
+//     counting. The reroute then goes in single CTAs of four entries a thread: they find room anywhere beside weight_sync,
+//     which leaves every SM a quarter of its shared memory. (524288 entries alone and beside weight_sync: 19.5 and 25, with
+//     clusters of sixteen entries a thread 33.8 and 49; 131072 in place 13.3 and 16.4, 17.4 and 18.6 with clusters of four.) The tiles in front of
+//     a CTA are a sum that grows with the square of the input: behind kOrdShortTiles entries tiles of sixteen entries
+//     (2^21 entries 50, tiles of four 58). The positions need every tile's counts: sixteen entries in clusters at any size
+//     (524288 entries 21.5; four 44, single CTAs 30).
 constexpr int64_t kOrdRecountMax = 1 << 18;
+constexpr int64_t kOrdShortTiles = 1 << 20;
 
 struct OrdGrid {
     int threads, ctas, clusters, per_lane;
     bool table;
 };
-OrdGrid ord_grid(int64_t n, int ranks, bool in_place, int threads) {
+// `totals`: the grand totals are wanted too (the positions).
+OrdGrid ord_grid(int64_t n, int ranks, bool in_place, int threads, bool totals) {
     OrdGrid g{threads, 1, 1, 1, false};
     while (g.ctas < kOrdMaxCluster && n > static_cast<int64_t>(g.ctas) * threads) g.ctas *= 2;
     int64_t row = static_cast<int64_t>(g.ctas) * threads;  // one entry per thread of a cluster
     if (n <= row) return g;
-    g.per_lane = n > kOrdRecountMax ? 16 : 4;
+    g.per_lane = 4;
     g.table = n > 4 * row && (in_place || ranks > 1 || n > kOrdRecountMax);
-    if (g.table && threads < kOrdThreads) g.per_lane = 16;  // the scratch buffer has room for tiles of kSparseTileEntries
-    if (g.table && ranks > 1) {
+    if (g.table && totals) {
+        g.per_lane = 16;
+    } else if (g.table) {
         g.ctas = 1;
         row = threads;
+        g.per_lane = n > kOrdShortTiles ? 16 : 4;
     }
-    // (tiles of the table: per_lane entries a thread)
+    // (tiles of the table: per_lane entries a thread, at least kSparseTileEntries a tile)
     const int64_t chunk = row * (g.table ? g.per_lane : (n > 4 * row && n <= 16 * row ? 2 : 4));
     g.clusters = static_cast<int>((n + chunk - 1) / chunk);
     return g;
@@ -1124,7 +1130,7 @@ static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L,
     if (max_n == 0) return cudaSuccess;
     const int staged = sparse_smem_bytes(L, true) <= kMaxCtaSmem ? 1 : 0;
     const size_t smem = sparse_smem_bytes(L, staged != 0);
-    const OrdGrid g = ord_grid(max_n, b.n, in_place, kOrdThreads);
+    const OrdGrid g = ord_grid(max_n, b.n, in_place, kOrdThreads, false);
     // One rank per launch is latency-bound and the overlap with the count kernel pays; several ranks fill the device
     // with the first kernel alone.
     const bool overlap = g.table && b.n == 1 && pdl_enabled();
@@ -1292,7 +1298,7 @@ int uep_dispatch_positions(const int32_t* phys_ids, int64_t num_entries, int P, 
     if (const int rc = check_width(ord_smem_bytes(P + 1, kOrdFewThreads) + sizeof(int32_t) * kOrdWarps, "dispatch_positions")) return rc;
     const uintptr_t x = reinterpret_cast<uintptr_t>(phys_ids), y = reinterpret_cast<uintptr_t>(pos), bytes = sizeof(int32_t) * num_entries;
     const bool in_place = x < y + bytes && y < x + bytes;
-    const OrdGrid g = ord_grid(num_entries, 1, in_place, ord_smem_bytes(P + 1, kOrdThreads) <= kMaxCtaSmem ? kOrdThreads : kOrdFewThreads);
+    const OrdGrid g = ord_grid(num_entries, 1, in_place, ord_smem_bytes(P + 1, kOrdThreads) <= kMaxCtaSmem ? kOrdThreads : kOrdFewThreads, true);
     const size_t smem = ord_smem_bytes(P + 1, g.threads), smem1 = sizeof(int32_t) * (P + 1);
     const bool overlap = g.table && pdl_enabled();
     if (g.table) {
