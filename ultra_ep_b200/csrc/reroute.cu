@@ -834,26 +834,44 @@ __global__ void __launch_bounds__(32) gather_rows_kernel(const uint8_t* __restri
     }
 
     // either several rows per item or several items (chunks) per row; rows_per_item is a power of two
-    const int64_t total = chunks_per_row > 1 ? num_rows * chunks_per_row : (num_rows + rows_per_item - 1) / rows_per_item;
+    const int shift = 31 - __clz(rows_per_item);
+    const int64_t total = chunks_per_row > 1 ? num_rows * chunks_per_row : (num_rows + rows_per_item - 1) >> shift;
     const int64_t first = blockIdx.x, step = gridDim.x;
     const int count = first < total ? static_cast<int>((total - first + step - 1) / step) : 0;
-    const int items = kGatherBatch / rows_per_item;  // of a batch
-    auto first_row = [&](int k) {
-        const int64_t item = first + k * step;
-        return chunks_per_row == 1 ? item * rows_per_item : item / chunks_per_row;
+    const int items = kGatherBatch >> shift;  // of a batch
+    // Where an item lies. A cursor goes from item to item by additions: the divisions (64 bits, several an item) made rows of
+    // two chunks 1.27 times as slow as one thread without them.
+    struct Cursor {
+        int64_t row;
+        int chunk;
     };
-    auto offset = [&](int k) { return chunks_per_row == 1 ? int64_t{0} : (first + k * step) % chunks_per_row * kGatherChunk; };
-    auto row_part = [&](int k) -> uint32_t {  // bytes of each of its rows
-        return static_cast<uint32_t>(min(row_bytes - offset(k), static_cast<int64_t>(kGatherChunk)));
+    const bool whole = chunks_per_row == 1;
+    const int64_t row_step = whole ? step << shift : step / chunks_per_row;
+    const int chunk_step = whole ? 0 : static_cast<int>(step % chunks_per_row);
+    auto advance = [&](Cursor& c) {
+        c.row += row_step;
+        c.chunk += chunk_step;
+        if (c.chunk >= chunks_per_row) {
+            c.chunk -= chunks_per_row;
+            ++c.row;
+        }
     };
-    auto rows_of = [&](int k) { return static_cast<int>(min(num_rows - first_row(k), static_cast<int64_t>(rows_per_item))); };
+    auto offset = [&](const Cursor& c) { return static_cast<int64_t>(c.chunk) * kGatherChunk; };
+    auto row_part = [&](const Cursor& c) -> uint32_t {  // bytes of each of its rows
+        return static_cast<uint32_t>(min(row_bytes - offset(c), static_cast<int64_t>(kGatherChunk)));
+    };
+    auto rows_of = [&](const Cursor& c) { return static_cast<int>(min(num_rows - c.row, static_cast<int64_t>(rows_per_item))); };
 
     auto fetch = [&](int batch, int32_t (&p)[kGatherBatch / 32]) {
 #pragma unroll
         for (int u = 0; u < kGatherBatch / 32; ++u) {
             const int i = u * 32 + lane;
-            const int k = batch * items + i / rows_per_item;
-            const int64_t row = k < count ? first_row(k) + i % rows_per_item : num_rows;
+            const int k = batch * items + (i >> shift);
+            int64_t row = num_rows;
+            if (k < count) {
+                const int64_t item = first + k * step;
+                row = whole ? (item << shift) + (i & (rows_per_item - 1)) : item / chunks_per_row;
+            }
             p[u] = row < num_rows ? __ldg(pos + row) : 0;
         }
     };
@@ -861,50 +879,63 @@ __global__ void __launch_bounds__(32) gather_rows_kernel(const uint8_t* __restri
 #pragma unroll
         for (int u = 0; u < kGatherBatch / 32; ++u) pos_s[batch & 1][u * 32 + lane] = p[u];
     };
-    auto issue_load = [&](int k) {
-        const int s = k % kGatherStages, n = rows_of(k);
-        const uint32_t bytes = row_part(k);
-        if (lane == 0) mbar_expect_tx(&bars[s], n * bytes);
+    Cursor load = whole ? Cursor{first << shift, 0} : Cursor{first / chunks_per_row, static_cast<int>(first % chunks_per_row)};
+    Cursor store = load;
+    int issued = 0, load_stage = 0, load_slot = 0, load_half = 0;
+    auto issue_load = [&]() {
+        const int n = rows_of(load);
+        const uint32_t bytes = row_part(load);
+        if (lane == 0) mbar_expect_tx(&bars[load_stage], n * bytes);
         __syncwarp();
         if (lane < n) {
-            int64_t src_row = pos_s[(k / items) & 1][k % items * rows_per_item + lane];
+            int64_t src_row = pos_s[load_half][(load_slot << shift) + lane];
             if (src_row < 0 || src_row >= num_src_rows) {  // never read out of bounds: record and clamp
-                report_error(status, UEP_DEV_BAD_PLAN, static_cast<int>(first_row(k) + lane));
+                report_error(status, UEP_DEV_BAD_PLAN, static_cast<int>(load.row + lane));
                 src_row = 0;
             }
-            bulk_load(smem_raw + s * kGatherChunk + lane * bytes, in + src_row * row_bytes + offset(k), bytes, &bars[s]);
+            bulk_load(smem_raw + load_stage * kGatherChunk + lane * bytes, in + src_row * row_bytes + offset(load), bytes, &bars[load_stage]);
+        }
+        advance(load);
+        ++issued;
+        if (++load_stage == kGatherStages) load_stage = 0;
+        if (++load_slot == items) {
+            load_slot = 0;
+            load_half ^= 1;
         }
     };
 
     int32_t ahead[kGatherBatch / 32];
     fetch(0, ahead);
     keep(0, ahead);
+    __syncwarp();
+    // Loads run at most kGatherStages - 1 items ahead: the first ones stay within batch 0, and batch b + 1 is in shared memory
+    // while the items of batch b are stored.
+    static_assert(kGatherBatch / 32 >= kGatherStages - 1, "the loads of a batch's items stay within the next batch");
+    while (issued < count && issued < kGatherStages - 1) issue_load();
     fetch(1, ahead);
     keep(1, ahead);
     __syncwarp();
-    int issued = count < kGatherStages - 1 ? count : kGatherStages - 1;
-    for (int k = 0; k < issued; ++k) issue_load(k);
-    int k = 0;
+    int k = 0, stage = 0;
+    uint32_t parity = 0;
     bool ok = true;
-    // Batch b + 1 is in shared memory while the items of batch b are stored: loads run at most kGatherStages - 1 items ahead.
-    static_assert(kGatherBatch / 32 >= kGatherStages - 1, "the loads of a batch's items stay within the next batch");
     for (int batch = 0; ok && k < count; ++batch) {
         fetch(batch + 2, ahead);
         const int batch_end = min((batch + 1) * items, count);
         for (; k < batch_end; ++k) {
-            const int s = k % kGatherStages;
-            ok = __all_sync(kFullMask, mbar_wait(&bars[s], static_cast<uint32_t>((k / kGatherStages) & 1), timeout_ns));
+            ok = __all_sync(kFullMask, mbar_wait(&bars[stage], parity, timeout_ns));
             if (!ok) break;
             if (lane == 0) {
-                bulk_store(out + first_row(k) * row_bytes + offset(k), smem_raw + s * kGatherChunk, rows_of(k) * row_part(k));
+                bulk_store(out + store.row * row_bytes + offset(store), smem_raw + stage * kGatherChunk, rows_of(store) * row_part(store));
                 bulk_commit();
                 if (issued < count && k >= 1) bulk_wait_read<1>();
             }
             __syncwarp();
-            if (issued < count) {
-                issue_load(issued);
-                ++issued;
+            advance(store);
+            if (++stage == kGatherStages) {
+                stage = 0;
+                parity ^= 1u;
             }
+            if (issued < count) issue_load();
         }
         __syncwarp();
         keep(batch + 2, ahead);  // over batch b, whose loads have all been issued
