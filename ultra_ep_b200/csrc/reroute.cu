@@ -1046,7 +1046,9 @@ cudaError_t launch_dense_backward(const Batch<DenseBwdArgs>& b, int L, int P, in
     // 16384 x 128 15.4 and 14.6, 8192 x 128 14.4 and 12.2).
     int64_t cells = 0;
     for (int i = 0; i < b.n; ++i) cells += static_cast<int64_t>(b.a[i].T) * L;
-    bool tiles = cells >= kDenseBwdTileCells && L % 4 == 0 && dense_bwd_smem_bytes(L, P) <= kMaxCtaSmem;
+    // Wider layers than a task a thread: the staged plan rows are more than the eight rows that share them (1000 experts,
+    // 8192 and 16384 tokens: tiles 31.5 and 48, cells 26.7 and 43).
+    bool tiles = cells >= kDenseBwdTileCells && L % 4 == 0 && L <= 4 * kDenseBwdThreads && dense_bwd_smem_bytes(L, P) <= kMaxCtaSmem;
     for (int i = 0; i < b.n; ++i) {
         tiles = tiles && ((reinterpret_cast<uintptr_t>(b.a[i].map) & 3u) == 0) && ((reinterpret_cast<uintptr_t>(b.a[i].grad_probs) & 15u) == 0);
     }
@@ -1055,8 +1057,8 @@ cudaError_t launch_dense_backward(const Batch<DenseBwdArgs>& b, int L, int P, in
         const size_t smem = dense_bwd_smem_bytes(L, P);
         cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(dense_backward_tile_kernel), smem);
         if (e != cudaSuccess) return e;
-        // a task (four columns, eight rows) per thread; wide layers get short tiles
-        const int segs = std::min(std::max(kDenseBwdThreads / (L / 4), 1), kDenseSegs), rows = 8 * segs;
+        // a task (four columns, eight rows) per thread
+        const int segs = std::min(kDenseBwdThreads / (L / 4), kDenseSegs), rows = 8 * segs;
         dense_backward_tile_kernel<<<dim3((max_T + rows - 1) / rows, b.n), kDenseBwdThreads, smem, stream>>>(b, L, P, D, rows);
         return cudaGetLastError();
     }
