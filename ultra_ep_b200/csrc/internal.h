@@ -148,7 +148,8 @@ int64_t sparse_scratch_elems(int64_t entries, int L);
 cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int D, int quota_mode, int interleave,
                                  cudaStream_t stream);
 cudaError_t launch_dense_backward(const Batch<DenseBwdArgs>& b, int L, int P, int D, cudaStream_t stream);
-cudaError_t launch_sparse_reroute(const Batch<SparseArgs>& b, int ids_kind, int K, int L, int D, int interleave,
+// beside_sync: a weight_sync was launched beside it
+cudaError_t launch_sparse_reroute(const Batch<SparseArgs>& b, int ids_kind, int K, int L, int D, int interleave, bool beside_sync,
                                   cudaStream_t stream);
 
 int device_sm_count();  // of the current device; launch sizes are multiples of it

@@ -147,6 +147,7 @@ struct uep_manager {
     std::vector<cudaEvent_t> plan_ready;
     std::vector<cudaStream_t> plan_stream;
     std::vector<char> plan_recorded;
+    std::vector<char> sync_beside;  // per plan slot: an asynchronous weight_sync of the plan was launched
     uint64_t timeout_ns = 0;
     bool connected = false;
     int grad_reduce_ctas = 42;
@@ -383,6 +384,7 @@ int uep_manager_create(const uep_config* cfg, uep_manager** out) {
     m->plan_ready.assign(slots, nullptr);
     m->plan_stream.assign(slots, nullptr);
     m->plan_recorded.assign(slots, 0);
+    m->sync_beside.assign(slots, 0);
     for (int i = 0; i < slots; ++i) UEP_TRY_BAIL(cudaEventCreateWithFlags(&m->plan_ready[i], cudaEventDisableTiming));
 
     m->ranks.resize(nlocal);
@@ -651,6 +653,7 @@ int uep_update_placement(uep_manager* m, int layer_id, int input_kind, const voi
     UEP_CUDA_TRY(cudaEventRecord(m->plan_ready[slot], stream));
     m->plan_stream[slot] = stream;
     m->plan_recorded[slot] = 1;
+    m->sync_beside[slot] = 0;
     return UEP_OK;
 }
 
@@ -707,7 +710,10 @@ int uep_weight_sync(uep_manager* m, int layer_id, const int64_t* const* fc1_ptrs
     call.sync_epoch = m->ranks[0].epochs + 1;
     call.trace = m->sync_trace;
     // a group of one rank has nobody to send to
-    if (m->R > 0 && m->N > 1) UEP_CUDA_TRY(launch_weight_sync(call, m->comm_stream));
+    if (m->R > 0 && m->N > 1) {
+        UEP_CUDA_TRY(launch_weight_sync(call, m->comm_stream));
+        m->sync_beside[plan_slot(m, layer_id)] = async_finish ? 1 : 0;
+    }
     return finish_sync_op(m, async_finish, current, done_event);
 }
 
@@ -813,7 +819,8 @@ int uep_reroute_sparse(uep_manager* m, int layer_id, int ids_kind, const void* c
         const PlanPtrs p = plan_ptrs(m, m->ranks[i], layer_id);
         b.a[i] = SparseArgs{ids[i], out[i], p.l2p, p.lcnts, p.rank_quota_prefix, m->ranks[i].scratch[1], T[i]};
     }
-    UEP_CUDA_TRY(launch_sparse_reroute(b, ids_kind, K, m->L, m->D, m->cfg.legacy_placement ? 2 : m->cfg.solver.reroute_interleave, stream));
+    UEP_CUDA_TRY(launch_sparse_reroute(b, ids_kind, K, m->L, m->D, m->cfg.legacy_placement ? 2 : m->cfg.solver.reroute_interleave,
+                                       m->sync_beside[plan_slot(m, layer_id)] != 0, stream));
     return UEP_OK;
 }
 

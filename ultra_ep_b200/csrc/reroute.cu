@@ -746,6 +746,120 @@ sparse_reroute_kernel(Batch<SparseArgs> batch, int ctas, int K, int L, int D, in
     if (ctas > 1) cluster_wait();
 }
 
+// Several ranks in one launch beside weight_sync: a warp walks its entries, 32 at a time. Slower by itself than the kernel
+// above, but thin: plain loads where they are needed, one after another. The kernel above finishes within the microseconds in
+// which weight_sync's CTAs read their tables, and its burst of loads and asynchronous copies made that set-up 6.5 us
+// instead of 4.2 (walk 4.9), and everything behind it slower. Whole step of eight ranks, 128 experts, fp8 weights (us):
+// 8192 int32 ids a rank 70.0 with the walk, 75.0 without (the same with 256 threads and eight entries each, and with the
+// reroute held back until weight_sync's launch), 4096 tokens 71.1 and 74.6.
+constexpr int kWalkThreads = 256, kWalkWarps = kWalkThreads / kWarp;
+__host__ __device__ __forceinline__ size_t walk_smem_bytes(int L) {
+    return static_cast<size_t>(L) * (2 * kStagedReps * 4 + sizeof(FastRouter) + 4 + kWalkWarps * 4);
+}
+template <typename IdT>
+__global__ void __launch_bounds__(kWalkThreads) sparse_walk_count_kernel(Batch<SparseArgs> batch, int K, int L) {
+    extern __shared__ __align__(128) char smem_raw[];
+    const SparseArgs& a = batch.a[blockIdx.y];
+    const IdT* keys = static_cast<const IdT*>(a.ids);
+    const int64_t n = static_cast<int64_t>(a.T) * K;
+    const int64_t begin = static_cast<int64_t>(blockIdx.x) * kSparseTileEntries;
+    if (begin >= n) return;  // a tile behind this rank's entries is read by nobody
+    int32_t* hist = reinterpret_cast<int32_t*>(smem_raw);
+    for (int i = threadIdx.x; i < L; i += blockDim.x) hist[i] = 0;
+    __syncthreads();
+    const int64_t end = min(begin + kSparseTileEntries, n);
+    for (int64_t i = begin + threadIdx.x; i < end; i += blockDim.x) {
+        const int b = key_bucket<IdT>(keys[i], L, false);
+        if (b >= 0) atomicAdd(hist + b, 1);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < L; i += blockDim.x) a.scratch[static_cast<int64_t>(blockIdx.x) * L + i] = hist[i];
+}
+
+template <typename IdT>
+__global__ void __launch_bounds__(kWalkThreads) sparse_walk_kernel(Batch<SparseArgs> batch, int K, int L, int D, int interleave) {
+    extern __shared__ __align__(128) char smem_raw[];
+    const SparseArgs& a = batch.a[blockIdx.y];
+    const IdT* ids = static_cast<const IdT*>(a.ids);
+    IdT* out = static_cast<IdT*>(a.out);
+    const int64_t n = static_cast<int64_t>(a.T) * K;
+    const int64_t tile_begin = static_cast<int64_t>(blockIdx.x) * kSparseTileEntries;
+    if (tile_begin >= n) return;
+    const bool quota_mode = interleave != 2;
+    int32_t* prefix_s = reinterpret_cast<int32_t*>(smem_raw);
+    int32_t* l2p_s = prefix_s + static_cast<size_t>(L) * kStagedReps;
+    FastRouter* routers = reinterpret_cast<FastRouter*>(l2p_s + static_cast<size_t>(L) * kStagedReps);
+    int32_t* base = reinterpret_cast<int32_t*>(routers + L);
+    int32_t* warp_base = base + L;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    constexpr int kPerWarp = kSparseTileEntries / kWalkWarps;
+    const int64_t begin = min(tile_begin + warp * kPerWarp, n), end = min(begin + kPerWarp, n);
+    for (int e = tid; e < L; e += kWalkThreads) {
+        int b = 0;
+#pragma unroll 8
+        for (int t = 0; t < static_cast<int>(blockIdx.x); ++t) b += __ldcg(a.scratch + static_cast<int64_t>(t) * L + e);
+        base[e] = b;
+    }
+    for (int e = tid; e < L; e += kWalkThreads) {
+        const int C = a.lcnts[e];
+        const int m = min(min(C, D), kStagedReps);
+        int32_t pre[kStagedReps], phys[kStagedReps];
+#pragma unroll
+        for (int j = 0; j < kStagedReps; ++j) {
+            pre[j] = (j < m && quota_mode) ? a.rqp[static_cast<int64_t>(e) * D + j] : 0;
+            phys[j] = j < m ? a.l2p[static_cast<int64_t>(e) * D + j] : -1;
+        }
+#pragma unroll
+        for (int j = 0; j < kStagedReps; ++j) {
+            prefix_s[e * kStagedReps + j] = pre[j];
+            l2p_s[e * kStagedReps + j] = phys[j];
+        }
+        routers[e] = make_fast_router(e, C, a.rqp, D, quota_mode, interleave == 1, prefix_s + e * kStagedReps);
+    }
+    for (int i = tid; i < kWalkWarps * L; i += kWalkThreads) warp_base[i] = 0;
+    __syncthreads();
+    int32_t* mine = warp_base + warp * L;
+    for (int64_t i = begin + lane; i < end; i += kWarp) {
+        const int b = key_bucket<IdT>(ids[i], L, false);
+        if (b >= 0) atomicAdd(mine + b, 1);
+    }
+    __syncthreads();
+    for (int e = tid; e < L; e += kWalkThreads) {  // exclusive scan over the warps, behind the tiles in front
+        int run = base[e];
+#pragma unroll
+        for (int w = 0; w < kWalkWarps; ++w) {
+            const int c = warp_base[w * L + e];
+            warp_base[w * L + e] = run;
+            run += c;
+        }
+    }
+    __syncthreads();
+    for (int64_t i0 = begin; i0 < end; i0 += kWarp) {
+        const int64_t i = i0 + lane;
+        const bool in = i < end;
+        const IdT id = in ? ids[i] : static_cast<IdT>(-1);
+        const int b = key_bucket<IdT>(id, L, false);
+        const unsigned active = __ballot_sync(kFullMask, b >= 0);
+        int ordinal = 0;
+        if (b >= 0) {
+            const unsigned peers = __match_any_sync(active, b);
+            const int before = __popc(peers & ((1u << lane) - 1u));
+            ordinal = mine[b] + before;
+            __syncwarp(active);
+            if (before == 0) mine[b] += __popc(peers);
+        }
+        __syncwarp();
+        if (!in) continue;
+        const int C = b >= 0 ? routers[b].C : 0;
+        if (C <= 0) {
+            out[i] = id;
+            continue;
+        }
+        const int j = C > 1 ? fast_replica_index(routers[b], ordinal, prefix_s + b * kStagedReps, a.rqp + static_cast<int64_t>(b) * D, quota_mode) : 0;
+        out[i] = static_cast<IdT>(j < kStagedReps ? l2p_s[b * kStagedReps + j] : a.l2p[static_cast<int64_t>(b) * D + j]);
+    }
+}
+
 // Experts with C <= 0 keep their id but still consume ordinals; the reference skips them before taking an ordinal
 // (reroute.cu:505-509), which is equivalent because such an expert never maps anything.
 
@@ -1148,8 +1262,19 @@ cudaError_t with_lanes(const OrdGrid& g, Launch launch) {
     return launch(std::integral_constant<int, 16>{});
 }
 
+// Several ranks in one launch, n entries of the longest (up to one cluster's the other kernel is one launch): does the walk
+// pay? Beside weight_sync while the walk's sums over the earlier tiles stay short, n / 2048 * L up to 4096 (whole step, walk
+// and table: 128 experts, 65536 entries 72.5 and 75.2, 131072 80 and 74; 256 experts, 32768 entries 76.7 and 78.7, 65536 int64
+// 84.9 and 81.3; 64 experts, 131072 entries 57.8 and 60.1). Alone from 65536 entries on, where the launch fills the device
+// either way (131072 entries of 128 experts 27.6 and 31.7; 32768 entries 18 and 14.3). Behind kOrdRecountMax always
+// (524288 entries 69 and 87).
+bool walk_pays(int64_t n, int L, bool beside_sync) {
+    if (n <= 4LL * kOrdMaxCluster * kOrdThreads) return false;
+    return n > kOrdRecountMax || (beside_sync ? n * L <= 1 << 23 : n > 1 << 16);
+}
+
 template <typename IdT>
-static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L, int D, int interleave,
+static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L, int D, int interleave, bool beside_sync,
                                        cudaStream_t stream) {
     int64_t max_n = 0;
     bool in_place = false;
@@ -1161,6 +1286,19 @@ static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L,
         in_place = in_place || (n > 0 && x < y + bytes && y < x + bytes);
     }
     if (max_n == 0) return cudaSuccess;
+    if (b.n > 1 && walk_pays(max_n, L, beside_sync) && walk_smem_bytes(L) <= kMaxCtaSmem) {
+        const dim3 grid(static_cast<unsigned>(sparse_tiles(max_n)), b.n);
+        cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(sparse_walk_count_kernel<IdT>), sizeof(int32_t) * L);
+        if (e != cudaSuccess) return e;
+        e = ensure_smem_attr(reinterpret_cast<const void*>(sparse_walk_kernel<IdT>), walk_smem_bytes(L));
+        if (e != cudaSuccess) return e;
+        count_launch(2);
+        sparse_walk_count_kernel<IdT><<<grid, kWalkThreads, sizeof(int32_t) * L, stream>>>(b, K, L);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        sparse_walk_kernel<IdT><<<grid, kWalkThreads, walk_smem_bytes(L), stream>>>(b, K, L, D, interleave);
+        return cudaGetLastError();
+    }
     const int staged = sparse_smem_bytes(L, true) <= kMaxCtaSmem ? 1 : 0;
     const size_t smem = sparse_smem_bytes(L, staged != 0);
     const OrdGrid g = ord_grid(max_n, b.n, in_place, kOrdThreads, false);
@@ -1181,10 +1319,10 @@ static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L,
     });
 }
 
-cudaError_t launch_sparse_reroute(const Batch<SparseArgs>& b, int ids_kind, int K, int L, int D, int interleave,
+cudaError_t launch_sparse_reroute(const Batch<SparseArgs>& b, int ids_kind, int K, int L, int D, int interleave, bool beside_sync,
                                   cudaStream_t stream) {
-    if (ids_kind == 2) return launch_sparse_typed<long long>(b, K, L, D, interleave, stream);
-    return launch_sparse_typed<int32_t>(b, K, L, D, interleave, stream);
+    if (ids_kind == 2) return launch_sparse_typed<long long>(b, K, L, D, interleave, beside_sync, stream);
+    return launch_sparse_typed<int32_t>(b, K, L, D, interleave, beside_sync, stream);
 }
 
 }  // namespace uep
@@ -1244,7 +1382,7 @@ static int sparse_common(int kind, const void* ids, void* out, int T, int K, int
     Batch<SparseArgs> b{};
     b.n = 1;
     b.a[0] = SparseArgs{ids, out, l2p, lcnts, rqp, scratch, T};
-    UEP_CUDA_TRY(launch_sparse_reroute(b, kind, K, L, D, interleave, static_cast<cudaStream_t>(stream_)));
+    UEP_CUDA_TRY(launch_sparse_reroute(b, kind, K, L, D, interleave, false, static_cast<cudaStream_t>(stream_)));
     return UEP_OK;
 }
 
