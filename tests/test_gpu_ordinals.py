@@ -65,7 +65,8 @@ def test_interleave_of_large_products(native_lib, cuda_device):
         assert np.array_equal(got.cpu().numpy(), O.sparse_reroute(ids, plan, True)), total
 
 
-@pytest.mark.parametrize("n,P", [(512, 31), (513, 32), (16385, 80), (65537, 160), (262145, 80), (40000, 4500), (4097, 7255)])
+@pytest.mark.parametrize("n,P", [(512, 31), (513, 32), (16385, 80), (65537, 160), (262145, 80), (40000, 4500), (4097, 7255), (2048, 256), (2049, 255), (4096, 1023),
+                                 (8193, 1024)])
 @pytest.mark.parametrize("in_place", [False, True])
 def test_dispatch_positions_split_edges(native_lib, cuda_device, n, P, in_place):
     rng = np.random.default_rng(n)
