@@ -6,7 +6,8 @@ import torch
 import torch.autograd.forward_ad as fwAD
 import torch.distributed as dist
 
-from ultra_ep_b200 import Manager
+from ultra_ep_b200 import EventHandle, Manager
+from ultra_ep_b200.native import load
 
 pytestmark = pytest.mark.gpu
 T, L, R = 70, 16, 2
@@ -40,3 +41,56 @@ def test_forward_mode_is_refused(manager, inputs):
         dual = fwAD.make_dual(probs, torch.ones_like(probs))
         with pytest.raises(NotImplementedError):
             manager.reroute(layer, dual, rmap)
+
+
+def test_functional_transforms_are_refused(manager, inputs):
+    layer, probs, rmap = inputs
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda p: manager.reroute(layer, p, rmap)[0].sum())(probs)
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(lambda p: manager.reroute(layer, p, rmap)[0])(torch.stack([probs, probs]))
+
+
+def test_gradients_that_reach_the_node(manager, inputs, cuda_device):
+    """Contiguous, expanded (stride 0), through a slice, twice through one graph, and none at all."""
+    layer, probs, rmap = inputs
+    out, emap = manager.reroute(layer, probs, rmap)
+    assert torch.equal(out, manager.reroute(layer, probs.detach(), rmap)[0]) and not emap.requires_grad
+    upstream = torch.randn(out.shape, device=cuda_device)
+    p2l = manager.physical_to_logical_map[layer].long()
+    want = torch.zeros((T, L), device=cuda_device).index_add_(1, p2l[p2l >= 0], torch.where(emap, upstream, 0.0)[:, p2l >= 0])
+    (first,) = torch.autograd.grad(out, probs, upstream, retain_graph=True)
+    (second,) = torch.autograd.grad(out, probs, upstream.t().contiguous().t(), retain_graph=True)
+    assert torch.equal(first, want) and torch.equal(second, want)
+    (ones,) = torch.autograd.grad(out.sum(), probs, retain_graph=True)
+    assert torch.equal(ones, rmap.float())
+    (part,) = torch.autograd.grad(out[:, :3].sum(), probs)
+    assert torch.equal(part[:, 3:], torch.zeros_like(part[:, 3:])) and torch.equal(part[:, :3], rmap[:, :3].float())
+    with torch.no_grad():
+        assert not manager.reroute(layer, probs, rmap)[0].requires_grad
+    other = torch.zeros(3, device=cuda_device, requires_grad=True)
+    unused, _ = manager.reroute(layer, probs, rmap)
+    assert torch.autograd.grad(other.sum() + 0 * emap.float().sum(), [probs], allow_unused=True) == (None,)
+    del unused
+
+
+def test_one_rank_orders_behind_a_previous_event(manager, inputs, cuda_device):
+    """Nothing is launched for a group of one rank, and the order it promises still holds."""
+    layer, _, _ = inputs
+    side = torch.cuda.Stream()
+    mark = torch.zeros(1, dtype=torch.int64, device=cuda_device)
+    torch.cuda.synchronize()
+    for call in (manager.weight_sync, manager.grad_reduce):
+        for asynchronous in (True, False):
+            mark.zero_()
+            torch.cuda.synchronize()
+            with torch.cuda.stream(side):
+                torch.cuda._sleep(20_000_000)
+                mark += 1
+                before = EventHandle(load().EventHandle())
+            done = call(layer, previous_event=before, async_finish=asynchronous)
+            if asynchronous:
+                done.current_stream_wait()
+            seen = mark.clone()
+            torch.cuda.synchronize()
+            assert seen.item() == 1
