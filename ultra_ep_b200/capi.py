@@ -149,23 +149,3 @@ def check(rc: int, what: str = "") -> None:
     if rc != UEP_OK:
         msg = lib().uep_last_error().decode(errors="replace")
         raise UepError(f"{what or 'uep call'} failed ({rc}): {msg}")
-
-
-def ptr(t) -> int:
-    """Device (or host) address of a torch tensor / numpy array, 0 for None."""
-    if t is None:
-        return 0
-    if hasattr(t, "data_ptr"):
-        return t.data_ptr()
-    return t.ctypes.data
-
-
-def ptr_array(values):
-    arr = (C.c_void_p * max(1, len(values)))()
-    for i, v in enumerate(values):
-        arr[i] = v if isinstance(v, int) else ptr(v)
-    return arr
-
-
-def int_array(values):
-    return (C.c_int * max(1, len(values)))(*values)

@@ -8,7 +8,7 @@
 //     64-byte handles between processes, so this library has no transport of its own;
 //   * a manager can host all ranks of a group on one device ("simulated EP"): the same
 //     kernels then serve every rank in one launch, and the peers are plain device buffers.
-// Per layer it issues one launch for the plan, one for weight_sync, two for reroute and
+// Per layer it issues one launch for the plan, one for weight_sync, one or two for reroute and
 // one for the Wgrad reduce; the reference issues about twenty stream operations.
 
 #include <algorithm>

@@ -36,8 +36,12 @@ namespace {
 constexpr int kPlanThreads = 256;
 constexpr int kSolveThreads = 512;
 constexpr size_t kSolveMaxSmem = 200 * 1024;
-constexpr size_t kPlanMatrixBytes = 16 * 1024;  // of the load matrix, where the plan kernel keeps it in shared memory
-constexpr int kPartBatch = 9;  // partial counts a thread asks for at once: two threads an expert cover 18 CTAs
+// Of the load matrix, where the plan kernel keeps it in shared memory: eight ranks of 512 experts, the largest group that one
+// device can host and the plan kernel could be timed with. The solver's own kernel has its SM to itself and takes what fits.
+constexpr size_t kPlanMatrixBytes = 16 * 1024;
+// Partial counts a thread asks for at once. The CTAs behind a rank's first one are shared by as many threads as an expert
+// can have: 17 of them (eight hosted ranks) by two threads up to 128 experts, one round each; other numbers take more rounds.
+constexpr int kPartBatch = 9;
 
 __device__ __forceinline__ void hist_add_swar(uint32_t word, int32_t* hist, int col) {
     // four byte-wide counters packed in `word`

@@ -7,7 +7,8 @@
 // outputs twice (zero-fill, then scatter): csrc/kernels/reroute.cu:21-51, 138-264 and
 // csrc/ultra_ep.cpp:891-892 of the reference. Here:
 //   * sparse: one launch (ordinals.cuh); a cluster of CTAs keeps its entries in registers and
-//     counts again what lies in front of it;
+//     counts again what lies in front of it. In place, with several ranks or with very many
+//     entries a count kernel goes in front;
 //   * dense: pass 1 counts per (tile, expert) from coalesced row reads; pass 2 turns the counts of
 //     the preceding tiles into a base per expert, holds the tile as bit columns, turns logical
 //     columns into physical ones and writes every output element exactly once out of registers

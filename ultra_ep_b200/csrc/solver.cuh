@@ -14,8 +14,9 @@
 //     warps (the serial search takes the first that is feasible), while the other warps clear
 //     the outputs;
 //   * each rank's masters are ranked by counting instead of a serial insertion sort;
-//   * the per-rank load matrix is read through L2 where it is needed instead of being
-//     staged in shared memory, so shared memory stays under 48 KB at the static limits.
+//   * the loads come in shared memory from the caller, and with one domain the per-rank load matrix
+//     too where it fits (plan.cu); else the few entries of it that are needed are read through L2.
+//     Without the matrix shared memory stays under 48 KB at the static limits.
 // All of it is latency of one CTA. Kernel time of uep_solve_placement on one B200: 64 ranks x 4 experts x 2 slots 25.3 us
 // (39.5 with the outputs cleared first, one build after another and one warp maximum per export), of which the build 14.
 #pragma once

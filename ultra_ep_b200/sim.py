@@ -1,9 +1,10 @@
 """Simulated expert-parallel group: all N ranks of a group hosted on ONE device.
 
-The C-ABI manager runs the same kernels as in the one-rank-per-process case, once for all
-hosted ranks (one launch each); "peers" are buffers on the same device, so weight_sync and the
-Wgrad reduce are bounded by HBM here, not by NVLink. Used for single-GPU parity tests and for
-the single-GPU leg of the benchmark.
+The manager of the C ABI, made and read through ctypes and called through the extension module,
+runs the same kernels as in the one-rank-per-process case, once for all hosted ranks (one launch
+each); "peers" are buffers on the same device, so weight_sync and the Wgrad reduce are bounded by
+HBM here, not by NVLink. Used for single-GPU parity tests and for the single-GPU leg of the
+benchmark.
 """
 
 from __future__ import annotations
@@ -98,7 +99,7 @@ def make_config(num_ranks: int, masters: int, redundant: int, num_layers: int = 
 
 
 class SimGroup:
-    """All ranks of one EP group on the current CUDA device, driven through the C ABI."""
+    """All ranks of one EP group on the current CUDA device."""
 
     PLAN_BUFFERS = {"p2l": capi.BUF_P2L, "l2p": capi.BUF_L2P, "lcnts": capi.BUF_LCNTS, "quota": capi.BUF_QUOTA,
                     "quota_prefix": capi.BUF_QUOTA_PREFIX, "rank_quota_prefix": capi.BUF_RANK_QUOTA_PREFIX}
