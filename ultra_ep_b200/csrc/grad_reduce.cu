@@ -296,9 +296,12 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
         const int n_owned = sm.n_owned;
         const bool vec_zero = ((fc1 & 3) == 0) && ((fc2 & 3) == 0);
         bool ok = true;
-        for (int u = 0; u < n_owned && ok; ++u) {
-            float* base = sm.own_base[u];
-            for (int sg = 0; sg < kReduceSegments && ok; ++sg) {
+        // Segment by segment over all slots: their masters' launches pull all of them at about the same pace. (Slot by slot,
+        // the last segment of the first slot held the clearing of all the others back until the pulls were over: backward of
+        // eight hosted ranks, 128 experts of 4.7 M elements, 189 us; 143 like this. Experts of 18.9 M: 350 and 310.)
+        for (int sg = 0; sg < kReduceSegments && ok; ++sg) {
+            for (int u = 0; u < n_owned && ok; ++u) {
+                float* base = sm.own_base[u];
                 int go = 1;
                 if (lane == 0 && !wait_flag_ge_relaxed(sm.own_flag[u], epoch * kReduceFlagRadix + static_cast<uint64_t>(sg + 1), call.timeout_ns)) {
                     report_error(status0, UEP_DEV_TIMEOUT_SYNC, u);  // the slot keeps what it holds; no further wait runs
