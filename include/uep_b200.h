@@ -301,7 +301,9 @@ int uep_clear_status(uep_manager* m);
  * completes its work but does not publish its load row / completion flags, so the ranks
  * that wait for it run into their time limit and report UEP_DEV_TIMEOUT_*; -1 switches the
  * hook off. No device fault is involved. No counterpart in the reference (its waits are
- * unbounded, csrc/kernels/weight_sync.cu:666-677, csrc/kernels/ptx.cuh:73-86). */
+ * unbounded, csrc/kernels/weight_sync.cu:666-677, csrc/kernels/ptx.cuh:73-86). While the hook is on
+ * (with any rank, one outside the group too), hosted ranks treat each other as ranks of other devices do:
+ * completion flags are written and waited for, and a replica's gradient is cleared by its owner. */
 int uep_debug_withhold_rank(uep_manager* m, int rank);
 
 /* Tuning aid: with UEP_SYNC_TRACE=1 in the environment when the manager is created, the

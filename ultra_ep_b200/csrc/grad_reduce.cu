@@ -9,7 +9,7 @@
 // replica sub-tile at a time through a single shared-memory buffer (load, wait, add, zero
 // with per-thread stores, repeat). Here:
 //   * no task list: every CTA derives the pull list from the plan rows with a block scan;
-//   * a consumed replica region is not zeroed over the link. Pulling 75 MB and pushing 75 MB of
+//   * a replica region consumed from another device is not zeroed over the link. Pulling 75 MB and pushing 75 MB of
 //     zeros back at the same time measured 450 GB/s against 660 GB/s for the pull alone (the link
 //     is full duplex, but one kernel reading from a peer and writing to it through the same SMs
 //     did not get both directions at full rate). Instead the rank that HOSTS a replica
@@ -18,7 +18,8 @@
 //     the CTA that completes a segment stores "epoch, segments done" into a flag word on every
 //     rank it pulls from), and the host rank's launch, once its own pulls are done, clears each
 //     segment of its used slots as soon as the flag allows, from a warp of its own that runs beside
-//     the pulls (bulk stores from a zero tile into local memory);
+//     the pulls (bulk stores from a zero tile into local memory). A replica that lies on a rank
+//     of the same launch needs none of that: the CTA that pulled a tile clears it;
 //   * roles are split. Two producer warps (one lane each) only issue bulk loads: one feeds the
 //     ring of replica tiles, the other the ring of master tiles. Eight
 //     consumer warps wait on a stage's "full" mbarrier, add it into accumulators in registers
@@ -29,7 +30,8 @@
 //     several MB) and three for the local master tiles. In one common ring a master tile would
 //     hold a stage as long as a remote tile does, and with one replica per master half of the
 //     ring would be taken away from the remote loads;
-//   * tiles are interleaved over masters so that concurrent CTAs pull from different peers.
+//   * tiles are interleaved over masters so that concurrent CTAs pull from different peers; they go
+//     expert by expert where all replicas lie in this device's memory.
 // The CTA budget (SMs used while the backward pass runs next to it) is the caller's knob
 // (grad_reduce_num_sms); each CTA holds about 215 KiB of shared memory.
 
@@ -49,7 +51,7 @@ constexpr int kReduceStages = 9;                       // ring of remote replica
 constexpr int kMasterStages = 3;                       // ring of local master tiles
 constexpr int kReduceVecPerThread = kReduceTileElems / 4 / kReduceConsumers;  // float4 per thread per tile
 constexpr int kMaxPulls = kMaxExportsPerDomain;
-constexpr int kMaxOwned = 64;  // used replica slots of the hosted ranks
+constexpr int kMaxOwned = 64;  // used replica slots of the hosted ranks (a lane of a warp asks for two)
 
 struct ReduceShared {
     int n_active, total_reps, vector_ok;
@@ -57,13 +59,16 @@ struct ReduceShared {
     int n_owned, s_go;
     volatile long long done_items;                 // items of this CTA whose replica tiles have all been consumed
     volatile int pull_finished;                    // the pull phase of this CTA is over (all items, or given up)
+    int n_hosted;                                  // replicas that lie on ranks of this launch
+    int n_away;                                    // replicas on other devices
     unsigned long long epoch;
     int w_a[kReduceThreads / 32], w_r[kReduceThreads / 32];
-    unsigned pull_mask[kMaxLocalRanks][3];         // per hosted rank: ranks it pulls replica gradients from
+    unsigned pull_mask[kMaxLocalRanks][3];         // per hosted rank: ranks on other devices it pulls replica gradients from
     float* own_base[kMaxOwned];                    // used local replica slots: base of the slot ...
     const uint64_t* own_flag[kMaxOwned];           // ... and the progress word its master's rank writes
     short rep_start[kMaxExpertsPerDomain + 1];
     float* rep_base[kMaxPulls];                    // replica slot base in the peer's grad buffer (null: skip)
+    unsigned char rep_hosted[kMaxPulls];           // 1: that peer is a rank of this launch, so the pulling CTA clears what it read
     float* master[kMaxExpertsPerDomain][2];        // [n_active][fc1, fc2] master gradient base
     __align__(8) uint64_t full[kReduceStages];     // a remote tile has landed in the stage
     __align__(8) uint64_t empty[kReduceStages];    // all eight consumer warps are done with the stage
@@ -79,11 +84,11 @@ struct ReduceItem {
 };
 
 __device__ __forceinline__ ReduceItem decode_item(int64_t idx, int n_active, int64_t fc1_numel, int64_t fc2_numel,
-                                                  int tiles_fc1) {
+                                                  int tiles_fc1, int expert_tiles) {
     ReduceItem it;
     const int idx32 = static_cast<int>(idx);
-    it.active = idx32 % n_active;
-    const int tile = idx32 / n_active;
+    it.active = expert_tiles > 0 ? idx32 / expert_tiles : idx32 % n_active;
+    const int tile = expert_tiles > 0 ? idx32 - it.active * expert_tiles : idx32 / n_active;
     it.shard = tile < tiles_fc1 ? 0 : 1;
     const int t = it.shard == 0 ? tile : tile - tiles_fc1;
     it.offset = static_cast<int64_t>(t) * kReduceTileElems;
@@ -117,6 +122,8 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
         sm.vector_ok = ((fc1 & 3) == 0 && (fc2 & 3) == 0) ? 1 : 0;
         sm.error = 0;
         sm.n_owned = 0;
+        sm.n_hosted = 0;
+        sm.n_away = 0;
         sm.done_items = 0;
         sm.pull_finished = 0;
         sm.epoch = *call.reduce_epoch + 1;  // ranks hosted together share the first one's counter
@@ -135,6 +142,13 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
     fence_proxy_async_smem();
     __syncthreads();
 
+    auto hosted_here = [&](int rank) {
+        if (call.owners_clear) return false;
+        for (int lr = 0; lr < nlocal; ++lr) {
+            if (call.my_rank[lr] == rank) return true;
+        }
+        return false;
+    };
     // pull list: masters of the hosted ranks with replicas, and where each replica lives.
     // Hosted ranks pool their tiles over all CTAs of the launch.
     const int total_masters = nlocal * M;
@@ -183,8 +197,11 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
                     report_error(rk.status, UEP_DEV_BAD_PLAN, l);
                     sm.rep_base[rs + j] = nullptr;
                 } else {
+                    const bool hosted = hosted_here(prank);
                     sm.rep_base[rs + j] = rk.peer_replica_grad[prank] + static_cast<int64_t>(pslot) * total_numel;
-                    atomicOr(&sm.pull_mask[lr][prank >> 5], 1u << (prank & 31));
+                    sm.rep_hosted[rs + j] = hosted ? 1 : 0;
+                    if (!hosted) atomicOr(&sm.pull_mask[lr][prank >> 5], 1u << (prank & 31));
+                    atomicAdd(hosted ? &sm.n_hosted : &sm.n_away, 1);
                 }
             }
             const uintptr_t p1 = static_cast<uintptr_t>(call.fc1_grad_ptrs[lr][m]);
@@ -201,13 +218,14 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
         __syncthreads();
     }
     if (tid == 0) sm.rep_start[sm.n_active] = static_cast<short>(sm.total_reps < kMaxPulls ? sm.total_reps : kMaxPulls);
-    // The used replica slots of the hosted ranks: this launch clears them once their master's rank has pulled them.
+    // The used replica slots of the hosted ranks whose master's rank is on another device: this launch clears them once that
+    // rank has pulled them.
     {
         const int i = tid;
         const bool in = i < nlocal * R && nlocal * R <= kMaxOwned;
         int l = -1;
         if (in) l = call.plan[i / R].p2l[call.my_rank[i / R] * Lp + M + i % R];
-        const bool used = in && l >= 0 && l / M < N;
+        const bool used = in && l >= 0 && l / M < N && !hosted_here(l / M);
         const unsigned has = __ballot_sync(kFullMask, used);
         const int lane = tid & 31, warp = tid >> 5;
         if (lane == 0) sm.w_a[warp] = __popc(has);
@@ -234,6 +252,11 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
     const int tiles_fc1 = static_cast<int>((fc1 + kReduceTileElems - 1) / kReduceTileElems);
     const int tiles_fc2 = static_cast<int>((fc2 + kReduceTileElems - 1) / kReduceTileElems);
     const int tiles_total = tiles_fc1 + tiles_fc2;
+    // Items go expert by expert where every replica is in this device's memory: at any time the CTAs of the launch then read
+    // and write a contiguous stretch of one expert, which suits the DRAM better than a tile of every expert at once (kernel
+    // time 86 and 78 us with 128 experts of 4.7 M elements on eight ranks, 294 and 257 with 18.9 M). Replicas on other devices
+    // are interleaved over the masters, so that concurrent CTAs pull from different peers.
+    const int expert_tiles = sm.n_away == 0 ? tiles_total : 0;
     const int64_t total_items = static_cast<int64_t>(n_active) * tiles_total;
     const int64_t first = blockIdx.x, step = gridDim.x;
     const int64_t count = first < total_items ? (total_items - first + step - 1) / step : 0;
@@ -243,7 +266,7 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
     // One thread per CTA reports progress: `done` of this CTA's items are consumed. When the CTA has passed a
     // segment it bumps that segment's counter; the CTA that completes the count tells every rank the launch pulls
     // from, and the one that completes the last segment closes the epoch.
-    int seg_next = 0;
+    int seg_next = sm.n_away > 0 ? 0 : kReduceSegments - 1;  // nobody to tell: only the epoch is left to close
     auto report_progress = [&](int64_t done) {
         while (seg_next < kReduceSegments) {
             const int64_t boundary = static_cast<int64_t>(seg_end(seg_next)) * n_active;  // first item index behind the segment
@@ -270,6 +293,14 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
     };
     auto master_ptr = [&](const ReduceItem& it) -> float* { return sm.master[it.active][it.shard] + it.offset; };
 
+    auto clear_tile = [&](float* dst, int elems) {  // one thread, 16-byte aligned
+        const uint32_t bytes = static_cast<uint32_t>(elems) * 4u;
+        for (uint32_t o = 0; o < bytes; o += kReduceZeroBytes) {
+            bulk_store(reinterpret_cast<char*>(dst) + o, zero_tile, bytes - o < kReduceZeroBytes ? bytes - o : kReduceZeroBytes);
+        }
+        bulk_commit();
+    };
+
     // ---- clearing warp: the used replica slots hosted here, segment by segment as their master's rank releases
     //      them; runs beside the pulls of this CTA (every CTA of the launch takes every gridDim-th tile) ----------
     if (tid >= kReduceConsumers + 96) {
@@ -280,7 +311,7 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
             const uint64_t t_begin = global_timer_ns();
             while (true) {
                 const int fin = sm.pull_finished;
-                const long long done = fin ? static_cast<long long>(count) : sm.done_items;
+                const long long done = fin || sm.n_away == 0 ? static_cast<long long>(count) : sm.done_items;
                 report_progress(done);
                 if (fin || seg_next >= kReduceSegments) break;
                 if (global_timer_ns() - t_begin > 4 * call.timeout_ns) {
@@ -300,18 +331,20 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
         // the last segment of the first slot held the clearing of all the others back until the pulls were over: backward of
         // eight hosted ranks, 128 experts of 4.7 M elements, 189 us; 143 like this. Experts of 18.9 M: 350 and 310.)
         for (int sg = 0; sg < kReduceSegments && ok; ++sg) {
-            for (int u = 0; u < n_owned && ok; ++u) {
+            // one lane per slot asks, so that a segment costs one round trip and not one per slot
+            unsigned here[kMaxOwned / 32];
+#pragma unroll
+            for (int h = 0; h < kMaxOwned / 32; ++h) {
+                const int u = 32 * h + lane;
+                const bool waits = u < n_owned;
+                const bool came = waits && wait_flag_ge_relaxed(sm.own_flag[u], epoch * kReduceFlagRadix + static_cast<uint64_t>(sg + 1), call.timeout_ns);
+                if (waits && !came) report_error(status0, UEP_DEV_TIMEOUT_SYNC, u);  // the slot keeps what it holds; no further wait runs
+                here[h] = __ballot_sync(kFullMask, came);
+                ok = ok && __all_sync(kFullMask, came || !waits);
+            }
+            for (int u = 0; u < n_owned; ++u) {
+                if (!((u < 32 ? here[0] : here[1]) >> (u & 31) & 1u)) continue;
                 float* base = sm.own_base[u];
-                int go = 1;
-                if (lane == 0 && !wait_flag_ge_relaxed(sm.own_flag[u], epoch * kReduceFlagRadix + static_cast<uint64_t>(sg + 1), call.timeout_ns)) {
-                    report_error(status0, UEP_DEV_TIMEOUT_SYNC, u);  // the slot keeps what it holds; no further wait runs
-                    go = 0;
-                }
-                go = __shfl_sync(kFullMask, go, 0);
-                if (!go) {
-                    ok = false;
-                    break;
-                }
                 const int t0 = sg == 0 ? 0 : seg_end(sg - 1), t1 = seg_end(sg);
                 for (int t = t0 + static_cast<int>(blockIdx.x); t < t1; t += static_cast<int>(gridDim.x)) {
                     const bool in1 = t < tiles_fc1;
@@ -321,13 +354,7 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
                     const int elems = static_cast<int>(left < kReduceTileElems ? left : kReduceTileElems);
                     float* dst = base + off;
                     if (vec_zero) {
-                        if (lane == 0) {
-                            const uint32_t bytes = static_cast<uint32_t>(elems) * 4u;
-                            for (uint32_t o = 0; o < bytes; o += kReduceZeroBytes) {
-                                bulk_store(reinterpret_cast<char*>(dst) + o, zero_tile, bytes - o < kReduceZeroBytes ? bytes - o : kReduceZeroBytes);
-                            }
-                            bulk_commit();
-                        }
+                        if (lane == 0) clear_tile(dst, elems);
                     } else {
                         for (int i = lane; i < elems; i += 32) dst[i] = 0.f;
                     }
@@ -338,14 +365,16 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
     } else if (!sm.vector_ok) {
         // element-wise path for sizes / pointers that are not multiples of 16 bytes
         for (int64_t k = 0; k < count; ++k) {
-            const ReduceItem it = decode_item(first + k * step, n_active, fc1, fc2, tiles_fc1);
+            const ReduceItem it = decode_item(first + k * step, n_active, fc1, fc2, tiles_fc1, expert_tiles);
             float* mp = master_ptr(it);
             const int r0 = sm.rep_start[it.active], r1 = sm.rep_start[it.active + 1];
             for (int i = tid; i < it.elems; i += kReduceConsumers + 64) {  // every thread but the clearing and reporting warps
                 float acc = mp[i];
                 for (int r = r0; r < r1; ++r) {
                     if (sm.rep_base[r] == nullptr) continue;
-                    acc = __fadd_rn(acc, __ldcg(replica_ptr(it, r) + i));
+                    float* from = replica_ptr(it, r) + i;
+                    acc = __fadd_rn(acc, __ldcg(from));
+                    if (sm.rep_hosted[r]) *from = 0.f;
                 }
                 mp[i] = acc;
             }
@@ -366,7 +395,7 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
                         break;
                     }
                 }
-                const ReduceItem it = decode_item(first + m_issued * step, n_active, fc1, fc2, tiles_fc1);
+                const ReduceItem it = decode_item(first + m_issued * step, n_active, fc1, fc2, tiles_fc1, expert_tiles);
                 const uint32_t bytes = static_cast<uint32_t>(it.elems) * 4u;
                 mbar_expect_tx(&sm.m_full[s], bytes);
                 bulk_load(master_ring + s * kReduceTileBytes, master_ptr(it), bytes, &sm.m_full[s]);
@@ -389,7 +418,7 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
                 while (true) {
                     if (r_issue < 0) {
                         if (k_rep >= count) return false;
-                        it_rep = decode_item(first + k_rep * step, n_active, fc1, fc2, tiles_fc1);
+                        it_rep = decode_item(first + k_rep * step, n_active, fc1, fc2, tiles_fc1, expert_tiles);
                         r_issue = sm.rep_start[it_rep.active];
                         r_issue_end = sm.rep_start[it_rep.active + 1];
                     }
@@ -441,6 +470,19 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
                 }
             }
             sm.pull_finished = 1;
+            // Replicas of ranks of this launch: the CTA that pulled a tile clears it, once it has pulled all of its tiles. The
+            // clearing is then mostly a phase of writes behind the phase of pulls; clearing a tile as soon as it has been read
+            // took 273 us for 257, in batches of 16 items 273, of 64 268 (18.9 M elements; at 4.7 M 78 us each).
+            if (sm.n_hosted > 0 && !sm.error) {
+                for (int64_t k = 0; k < count; ++k) {
+                    const ReduceItem it = decode_item(first + k * step, n_active, fc1, fc2, tiles_fc1, expert_tiles);
+                    const int r0 = sm.rep_start[it.active], r1 = sm.rep_start[it.active + 1];
+                    for (int r = r0; r < r1; ++r) {
+                        if (sm.rep_base[r] != nullptr && sm.rep_hosted[r]) clear_tile(replica_ptr(it, r), it.elems);
+                    }
+                }
+                bulk_wait_all<0>();
+            }
         }
     } else {
         // ---- consumer warps ---------------------------------------------------------------------
@@ -448,7 +490,7 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
         int64_t consumed = 0;
         stamp(2);
         for (int64_t k = 0; k < count; ++k) {
-            const ReduceItem it = decode_item(first + k * step, n_active, fc1, fc2, tiles_fc1);
+            const ReduceItem it = decode_item(first + k * step, n_active, fc1, fc2, tiles_fc1, expert_tiles);
             const int nvec = it.elems >> 2;
             float4 acc[kReduceVecPerThread];
             {
@@ -508,9 +550,9 @@ cudaError_t launch_grad_reduce(const ReduceCall& call, cudaStream_t stream) {
     if (call.nlocal * call.R > kMaxOwned) return cudaErrorInvalidValue;  // more replica slots per launch than the kernel's table holds
     count_launch();
     const dim3 grid(call.nlocal * call.ctas_per_rank), block(kReduceThreads);
-    if (call.nlocal > 1) {
+    if (call.nlocal > 1 && call.owners_clear) {
         // hosted ranks clear their slots behind other hosted ranks' pulls inside this one launch: the CTAs that
-        // wait and the CTAs they wait for must be resident together
+        // wait and the CTAs they wait for must be resident together. (Else no CTA waits for another one of its launch.)
         ReduceCall copy = call;
         void* args[] = {&copy};
         return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(grad_reduce_kernel), grid, block, args, smem, stream);

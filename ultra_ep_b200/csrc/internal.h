@@ -109,6 +109,7 @@ struct ReduceCall {
     int64_t fc1_numel, fc2_numel;
     uint64_t timeout_ns;
     int ctas_per_rank;
+    int owners_clear;           // test hook: replicas of hosted ranks are cleared by their owners too, as on other devices
     uint64_t* reduce_epoch;     // the reduce epoch counter of the first hosted rank
     unsigned long long* trace;  // optional: 8 globaltimer stamps per CTA (tuning aid), or null
 };
