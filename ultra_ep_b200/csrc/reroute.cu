@@ -548,34 +548,109 @@ __device__ __forceinline__ float routed_grad(const float* __restrict__ grad_expa
     return 0.f;
 }
 
-// Backward of a tile of `tile_rows` tokens (a multiple of eight, at most 64): the expanded map as bit columns, then four
-// logical columns of eight rows per thread. Which instance a row took is found for eight rows at a time, an AND per
-// instance, and kept as the bit planes of the instance number, so all the gradients a thread needs are asked for at once.
-// It reads the expanded map as a stream where the kernel below fetches a sector per routed cell and instance: 26 us against
-// 35 for eight ranks of 8192 tokens and 128 experts, behind a gradient reduce. (Walking only the set cells of a thread: 33.)
-// Needs L a multiple of four, a 4-byte aligned map and 16-byte aligned gradients.
-constexpr int kDenseBwdThreads = 128;
-constexpr int64_t kDenseBwdTileCells = 1 << 22;
+// The marked cells of a warp's 32 words of row bits (one word per lane), 32 cells at a time: every lane gets the lane that
+// holds its cell and the bit there. The few marked cells are so shared evenly by the lanes; a loop over the bits of the own
+// word runs as long as the fullest of 32 words.
+template <typename F>
+__device__ __forceinline__ void for_each_marked(uint32_t word, F&& cell) {
+    const int lane = threadIdx.x & 31;
+    int upto = __popc(word);
+#pragma unroll
+    for (int d = 1; d < kWarp; d <<= 1) {
+        const int x = __shfl_up_sync(kFullMask, upto, d);
+        if (lane >= d) upto += x;
+    }
+    const int total = __shfl_sync(kFullMask, upto, kWarp - 1);
+    for (int first = 0; first < total; first += kWarp) {
+        int n = first + lane, src = 0;  // the first lane whose inclusive sum is above n
+#pragma unroll
+        for (int d = kWarp / 2; d > 0; d >>= 1) src += __shfl_sync(kFullMask, upto, src + d - 1) <= n ? d : 0;
+        const bool active = n < total;
+        const uint32_t w = __shfl_sync(kFullMask, word, src);
+        n -= __shfl_sync(kFullMask, upto, src) - __popc(w);
+        int bit = 0;  // of the n-th marked cell of w
+#pragma unroll
+        for (int width = 16; width > 0; width >>= 1) {
+            const int c = __popc((w >> bit) & ((1u << width) - 1u));
+            if (n >= c) {
+                n -= c;
+                bit += width;
+            }
+        }
+        cell(active, src, bit & 31);
+    }
+}
 
-__host__ __device__ inline size_t dense_bwd_smem_bytes(int L, int P) {
-    return static_cast<size_t>(pad4(L)) * (kStagedReps + 1) * 4 + static_cast<size_t>(pad4(P)) * kDenseSegs;
+// Zeros by all threads of the CTA, 16 bytes a store but for the ends.
+__device__ __forceinline__ void zero_fill(void* where, int bytes) {
+    char* p = static_cast<char*>(where);
+    const int head = min(bytes, static_cast<int>((16u - (reinterpret_cast<uintptr_t>(p) & 15u)) & 15u));
+    const int vecs = (bytes - head) / 16, tail = head + vecs * 16;
+    if (static_cast<int>(threadIdx.x) < head) p[threadIdx.x] = 0;
+    uint4* v = reinterpret_cast<uint4*>(p + head) + threadIdx.x;
+    int left = vecs - static_cast<int>(threadIdx.x);
+    for (; left > 3 * static_cast<int>(blockDim.x); left -= 4 * blockDim.x, v += 4 * blockDim.x) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u * blockDim.x] = make_uint4(0, 0, 0, 0);
+    }
+    for (; left > 0; left -= blockDim.x, v += blockDim.x) *v = make_uint4(0, 0, 0, 0);
+    if (static_cast<int>(threadIdx.x) < bytes - tail) p[tail + threadIdx.x] = 0;
+}
+
+// `bytes` bytes into shared memory (16-byte aligned there), asynchronously where the source is aligned.
+__device__ __forceinline__ void stage_bytes(uint8_t* dst, const uint8_t* __restrict__ src, int bytes) {
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(src) | static_cast<uintptr_t>(bytes);
+    if ((bits & 15u) == 0) {
+        for (int i = threadIdx.x * 16; i < bytes; i += blockDim.x * 16) cp_async_16(dst + i, src + i);
+    } else if ((bits & 3u) == 0) {
+        for (int i = threadIdx.x * 4; i < bytes; i += blockDim.x * 4) cp_async_4(dst + i, src + i);
+    } else {
+        for (int i = threadIdx.x; i < bytes; i += blockDim.x) dst[i] = __ldg(src + i);
+    }
+}
+
+// Which of the 32 columns from `c` on are marked in a row of `cols` bytes in shared memory (rows stand `cols` bytes apart).
+__device__ __forceinline__ uint32_t row_bits(const uint8_t* row, int c, int cols) {
+    uint32_t bits = 0;
+    if (cols % 4 == 0) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t marks = c + 4 * k < cols ? nonzero_bytes(*reinterpret_cast<const uint32_t*>(row + c + 4 * k)) : 0u;
+            bits |= (marks * 0x10204080u) >> 28 << (4 * k);  // four bytes of 0 or 1 to four bits
+        }
+    } else {
+        for (int k = 0; k < 32 && c + k < cols; ++k) bits |= (row[c + k] != 0 ? 1u : 0u) << k;
+    }
+    return bits;
+}
+
+// Backward of a tile of `tile_rows` tokens: the rows of both maps are copied to shared memory, the output is filled with
+// zeros, and the marked cells (topk of them a token) are shared by the lanes: a cell looks its instances up in the expanded
+// row, fetches one gradient and stores it over the zero. Full occupancy (32 registers), since every step waits for memory.
+// Both maps as bit columns and four columns of eight rows per thread took 14 M instructions a call of eight ranks of 8192
+// tokens and 128 experts, two thirds of the issue slots: 24.8 us a call, 18.3 like this (20.7 with four CTAs an SM); one
+// rank of 16384 tokens and 256 experts 12.3 (a thread per four cells 19.3).
+constexpr int kDenseBwdThreads = 256;
+
+__host__ __device__ inline size_t dense_bwd_smem_bytes(int L, int P, int tile_rows) {
+    return static_cast<size_t>(pad4(L)) * (kStagedReps + 1) * 4 + static_cast<size_t>(tile_rows) * (L + P) + 16;
 }
 __global__ void __launch_bounds__(kDenseBwdThreads, 8)
 dense_backward_tile_kernel(Batch<DenseBwdArgs> batch, int L, int P, int D, int tile_rows) {
     const DenseBwdArgs& a = batch.a[blockIdx.y];
     const int first = static_cast<int>(blockIdx.x) * tile_rows;
-    // Rows from here to the rank's last one, not cut to the tile: everything below compares with it and none of it goes beyond
-    // tile_rows. With min(a.T - r0, tile_rows) and a 64-bit r0 the compiler (12.9.86, under this launch bound) took
-    // tile_rows for the last tile too, so that a height that is no multiple of the tile's wrote behind the output.
-    const int rows = a.T - first;
+    const int rows = min(a.T - first, tile_rows);
     if (rows <= 0) return;
     const int64_t r0 = first;
     extern __shared__ __align__(128) char smem_raw[];
     int32_t* l2p_s = reinterpret_cast<int32_t*>(smem_raw);
     int32_t* count_s = l2p_s + pad4(L) * kStagedReps;
-    uint8_t* bits = reinterpret_cast<uint8_t*>(count_s + pad4(L));
-    const int Pq = pad4(P), quads = L / 4, tasks = quads * (tile_rows / 8);
-    const uint8_t* map = a.map + r0 * L;
+    uint8_t* map_s = reinterpret_cast<uint8_t*>(count_s + pad4(L));
+    uint8_t* expanded_s = map_s + (tile_rows * L + 15) / 16 * 16;
+    const float* grads = a.grad_expanded + r0 * P;
+    float* out = a.grad_probs + r0 * L;
+    stage_bytes(map_s, a.map + r0 * L, rows * L);
+    stage_bytes(expanded_s, a.expanded_map + r0 * P, rows * P);
     for (int e = threadIdx.x; e < L; e += blockDim.x) cp_async_4(count_s + e, a.lcnts + e);
     if (D >= kStagedReps && D % 4 == 0 && (reinterpret_cast<uintptr_t>(a.l2p) & 15u) == 0) {
         for (int i = threadIdx.x; i < L * (kStagedReps / 4); i += blockDim.x) {
@@ -586,57 +661,38 @@ dense_backward_tile_kernel(Batch<DenseBwdArgs> batch, int L, int P, int D, int t
             if (i % kStagedReps < D) cp_async_4(l2p_s + i, a.l2p + static_cast<int64_t>(i / kStagedReps) * D + i % kStagedReps);
         }
     }
-    uint32_t word = threadIdx.x < tasks ? segment_bits<uint32_t>(map, rows, L, threadIdx.x / quads, threadIdx.x % quads) : 0u;
-    tile_bit_columns(a.expanded_map + r0 * P, rows, tile_rows / 8, P, bits);
+    zero_fill(out, rows * L * 4);
     cp_async_wait();
-    __syncthreads();
-    for (int i = threadIdx.x; i < tasks; i += blockDim.x) {
-        const int seg = i / quads, q = i - seg * quads;
-        if (i != threadIdx.x) word = segment_bits<uint32_t>(map, rows, L, seg, q);
-        const float* grads = a.grad_expanded + (r0 + 8 * seg) * P;
-        float v[8][4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int l = 4 * q + k;
-            const int32_t* phys_of = l2p_s + l * kStagedReps;
-            uint32_t open = (word >> (8 * k)) & 0xFFu;  // rows that have not found their instance
-            uint32_t found = 0, plane[3] = {0, 0, 0};
-            const int C = open ? count_s[l] : 0;
-#pragma unroll
-            for (int j = 0; j < kStagedReps; ++j) {
-                if (j < C && open) {
-                    const int phys = phys_of[j];
-                    const uint32_t hit = phys >= 0 && phys < P ? open & bits[seg * Pq + phys] : 0u;
-                    open &= ~hit;
-                    found |= hit;
-#pragma unroll
-                    for (int b = 0; b < 3; ++b) plane[b] |= (j >> b) & 1 ? hit : 0u;
+    __syncthreads();  // the zeros are in front of the stores below, too
+    const int groups = (L + 31) / 32, tasks = rows * groups, lane = threadIdx.x & 31;
+    float held = 0.f;  // a lane's last gradient, stored once its next one is on the way
+    int held_at = -1;
+    for (int i0 = threadIdx.x - lane; i0 < tasks; i0 += blockDim.x) {
+        const int i = i0 + lane, my_row = i / groups, my_group = i - my_row * groups;
+        const uint32_t word = i < tasks ? row_bits(map_s + my_row * L, 32 * my_group, L) : 0u;
+        for_each_marked(word, [&](bool active, int src, int bit) {
+            const int place = __shfl_sync(kFullMask, my_row << 16 | my_group, src);
+            float g = 0.f;
+            int at = -1;
+            if (active) {
+                const int row = place >> 16, l = 32 * (place & 0xFFFF) + bit, C = count_s[l];
+                const uint8_t* took = expanded_s + row * P;
+                int phys = -1;
+                for (int j = 0; j < C && phys < 0; ++j) {
+                    const int p = j < kStagedReps ? l2p_s[l * kStagedReps + j] : __ldg(a.l2p + static_cast<int64_t>(l) * D + j);
+                    if (p >= 0 && p < P && took[p] != 0) phys = p;
+                }
+                if (phys >= 0) {
+                    g = __ldg(grads + row * P + phys);
+                    at = row * L + l;
                 }
             }
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                v[r][k] = 0.f;
-                if ((found >> r) & 1u) {
-                    const int j = ((plane[0] >> r) & 1u) | ((plane[1] >> r) & 1u) << 1 | ((plane[2] >> r) & 1u) << 2;
-                    v[r][k] = __ldg(grads + static_cast<int64_t>(r) * P + phys_of[j]);
-                }
-            }
-            for (int j = kStagedReps; j < C && open; ++j) {  // instances behind the staged ones
-                const int phys = __ldg(a.l2p + static_cast<int64_t>(l) * D + j);
-                const uint32_t hit = phys >= 0 && phys < P ? open & bits[seg * Pq + phys] : 0u;
-                open &= ~hit;
-#pragma unroll
-                for (int r = 0; r < 8; ++r) {
-                    if ((hit >> r) & 1u) v[r][k] = __ldg(grads + static_cast<int64_t>(r) * P + phys);
-                }
-            }
-        }
-        float* out = a.grad_probs + (r0 + 8 * seg) * L + 4 * q;
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            if (8 * seg + r < rows) *reinterpret_cast<float4*>(out + static_cast<int64_t>(r) * L) = make_float4(v[r][0], v[r][1], v[r][2], v[r][3]);
-        }
+            if (held_at >= 0) out[held_at] = held;
+            held = g;
+            held_at = at;
+        });
     }
+    if (held_at >= 0) out[held_at] = held;
 }
 
 // One thread per four logical experts of a token when the rows allow it (L a multiple of 4, map rows 4-byte and
@@ -1156,30 +1212,35 @@ cudaError_t launch_dense_backward(const Batch<DenseBwdArgs>& b, int L, int P, in
     int max_T = 0;
     for (int i = 0; i < b.n; ++i) max_T = b.a[i].T > max_T ? b.a[i].T : max_T;
     if (max_T == 0) return cudaSuccess;
-    // The tile kernel pays for its staging where the launch is bound by memory; below, the thread-per-four-cells kernel has
-    // the shorter chain (events around one cold launch, tiles against cells: 16384 tokens x 256 experts 18.6 and 22.6 us,
-    // 16384 x 128 15.4 and 14.6, 8192 x 128 14.4 and 12.2).
+    // The tile kernel pays where a launch is more than a few waves of latency, and where a row of the map is more than two
+    // words, so that a tile keeps all of its threads busy (events around calls over 11 states, tiles against cells: one rank
+    // of 4096 x 128 6.3 and 6.3, 8191 x 128 8.3 and 8.3, 4096 x 256 6.3 and 8.5, 8191 x 256 8.4 and 12.6, 16384 x 128 10.4
+    // and 12.5; eight ranks of 1024 x 128 8.1 and 8.3, 2048 x 128 9.4 and 12.9; 64 experts: eight ranks of 2048 tokens 10.4
+    // and 8.3, of 8192 14.0 and 16.5 with the kernel before). Very wide layers: the staged plan rows are more than the few
+    // rows that share them.
     int64_t cells = 0;
     for (int i = 0; i < b.n; ++i) cells += static_cast<int64_t>(b.a[i].T) * L;
-    // Wider layers than a task a thread: the staged plan rows are more than the eight rows that share them (1000 experts,
-    // 8192 and 16384 tokens: tiles 31.5 and 48, cells 26.7 and 43).
-    bool tiles = cells >= kDenseBwdTileCells && L % 4 == 0 && L <= 4 * kDenseBwdThreads && dense_bwd_smem_bytes(L, P) <= kMaxCtaSmem;
+    const int groups = (L + 31) / 32;
+    // a word of a row a thread: 64 rows at 128 experts (32 rows 18.6 us for 18.3, 128 20.9); fewer where that leaves SMs
+    // without two CTAs (8191 x 256: 16 rows 8.4 us, 64 rows 10.4), or where wide rows fill the shared memory
+    const int sms = std::max(device_sm_count(), 1);
+    int rows = groups <= 4 ? 64 : (groups <= 8 ? 32 : 16);
+    while (rows > 16 && static_cast<int64_t>((max_T + rows - 1) / rows) * b.n < 2 * sms) rows /= 2;
+    while (rows > 8 && dense_bwd_smem_bytes(L, P, rows) > kMaxCtaSmem / 4) rows /= 2;
+    const size_t smem = dense_bwd_smem_bytes(L, P, rows);
+    bool tiles = cells >= (L > 64 ? 1 << 20 : 1 << 22) && L % 4 == 0 && L <= 512 && smem <= kMaxCtaSmem;
     for (int i = 0; i < b.n; ++i) {
         tiles = tiles && ((reinterpret_cast<uintptr_t>(b.a[i].map) & 3u) == 0) && ((reinterpret_cast<uintptr_t>(b.a[i].grad_probs) & 15u) == 0);
     }
     count_launch();
     if (tiles) {
-        const size_t smem = dense_bwd_smem_bytes(L, P);
         cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(dense_backward_tile_kernel), smem);
         if (e != cudaSuccess) return e;
-        // a task (four columns, eight rows) per thread
-        const int segs = std::min(kDenseBwdThreads / (L / 4), kDenseSegs), rows = 8 * segs;
         dense_backward_tile_kernel<<<dim3((max_T + rows - 1) / rows, b.n), kDenseBwdThreads, smem, stream>>>(b, L, P, D, rows);
         return cudaGetLastError();
     }
     int64_t blocks = (static_cast<int64_t>(max_T) * L / 4 + kRerouteThreads - 1) / kRerouteThreads + 1;
-    const int64_t sms = device_sm_count() > 0 ? device_sm_count() : 1;
-    const int64_t cap = (sms * 16) / b.n > 1 ? (sms * 16) / b.n : 1;
+    const int64_t cap = std::max(sms * 16 / b.n, 1);
     if (blocks > cap) blocks = cap;
     dense_backward_kernel<<<dim3(static_cast<unsigned>(blocks), b.n), kRerouteThreads, 0, stream>>>(b, L, P, D);
     return cudaGetLastError();
