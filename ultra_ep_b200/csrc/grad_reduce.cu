@@ -105,12 +105,13 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
     extern __shared__ __align__(128) char smem_raw[];  // kReduceStages replica tiles, kMasterStages master tiles, the zero tile
     __shared__ ReduceShared sm;
 
+    const GroupDev& group = call.group;
     const int M = call.M, R = call.R, D = call.D, Lp = M + R, N = call.N, nlocal = call.nlocal;
     const int tid = threadIdx.x;
     const int64_t fc1 = call.fc1_numel, fc2 = call.fc2_numel, total_numel = fc1 + fc2;
     char* master_ring = smem_raw + kReduceStages * kReduceTileBytes;
     char* zero_tile = master_ring + kMasterStages * kReduceTileBytes;
-    DeviceStatus* status0 = call.rank[0]->status;
+    DeviceStatus* status0 = group.status[0];
     auto stamp = [&](int slot) {
         if (call.trace != nullptr && tid == 0) call.trace[blockIdx.x * 8 + slot] = global_timer_ns();
     };
@@ -145,7 +146,7 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
     auto hosted_here = [&](int rank) {
         if (call.owners_clear) return false;
         for (int lr = 0; lr < nlocal; ++lr) {
-            if (call.my_rank[lr] == rank) return true;
+            if (group.my_rank[lr] == rank) return true;
         }
         return false;
     };
@@ -156,9 +157,8 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
         const int gm = g0 + tid;
         const int lr = gm < total_masters ? gm / M : 0;
         const int m = gm < total_masters ? gm % M : 0;
-        const RankDev& rk = *call.rank[lr];
         const PlanPtrs& plan = call.plan[lr];
-        const int me = call.my_rank[lr];
+        const int me = group.my_rank[lr];
         int reps = 0;
         if (gm < total_masters) {
             reps = plan.lcnts[me * M + m] - 1;
@@ -194,11 +194,11 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
                 const int phys = plan.l2p[static_cast<int64_t>(l) * D + 1 + j];
                 const int prank = phys / Lp, pslot = phys % Lp - M;
                 if (phys < 0 || prank >= N || pslot < 0 || pslot >= R) {
-                    report_error(rk.status, UEP_DEV_BAD_PLAN, l);
+                    report_error(group.status[lr], UEP_DEV_BAD_PLAN, l);
                     sm.rep_base[rs + j] = nullptr;
                 } else {
                     const bool hosted = hosted_here(prank);
-                    sm.rep_base[rs + j] = rk.peer_replica_grad[prank] + static_cast<int64_t>(pslot) * total_numel;
+                    sm.rep_base[rs + j] = group.grad_of(prank) + static_cast<int64_t>(pslot) * total_numel;
                     sm.rep_hosted[rs + j] = hosted ? 1 : 0;
                     if (!hosted) atomicOr(&sm.pull_mask[lr][prank >> 5], 1u << (prank & 31));
                     atomicAdd(hosted ? &sm.n_hosted : &sm.n_away, 1);
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
         const int i = tid;
         const bool in = i < nlocal * R && nlocal * R <= kMaxOwned;
         int l = -1;
-        if (in) l = call.plan[i / R].p2l[call.my_rank[i / R] * Lp + M + i % R];
+        if (in) l = call.plan[i / R].p2l[group.my_rank[i / R] * Lp + M + i % R];
         const bool used = in && l >= 0 && l / M < N && !hosted_here(l / M);
         const unsigned has = __ballot_sync(kFullMask, used);
         const int lane = tid & 31, warp = tid >> 5;
@@ -233,10 +233,9 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
         int f = __popc(has & ((1u << lane) - 1u));
         for (int w = 0; w < warp; ++w) f += sm.w_a[w];
         if (used) {
-            const int lr = i / R, me = call.my_rank[lr];
-            const RankDev& rk = *call.rank[lr];
-            sm.own_base[f] = rk.peer_replica_grad[me] + static_cast<int64_t>(i % R) * total_numel;
-            sm.own_flag[f] = rk.peer_reduce_flags[me] + l / M;
+            const int lr = i / R, me = group.my_rank[lr];
+            sm.own_base[f] = group.grad_of(me) + static_cast<int64_t>(i % R) * total_numel;
+            sm.own_flag[f] = group.reduce_flags_of(me) + l / M;
         }
         if (tid == 0) {
             int n = 0;
@@ -272,14 +271,13 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
             const int64_t boundary = static_cast<int64_t>(seg_end(seg_next)) * n_active;  // first item index behind the segment
             if (done < count && first + done * step < boundary) break;
             __threadfence();
-            int* counters = call.rank[0]->reduce_counters;
+            int* counters = call.counters;
             if (atomicAdd(&counters[seg_next], 1) == static_cast<int>(gridDim.x) - 1) {
                 counters[seg_next] = 0;
                 const uint64_t word = epoch * kReduceFlagRadix + static_cast<uint64_t>(seg_next + 1);
                 for (int lr = 0; lr < nlocal; ++lr) {
-                    const RankDev& rk = *call.rank[lr];
                     for (int p = 0; p < N; ++p) {
-                        if (sm.pull_mask[lr][p >> 5] & (1u << (p & 31))) st_relaxed_sys_u64(rk.peer_reduce_flags[p] + call.my_rank[lr], word);
+                        if (sm.pull_mask[lr][p >> 5] & (1u << (p & 31))) st_relaxed_sys_u64(group.reduce_flags_of(p) + group.my_rank[lr], word);
                     }
                 }
                 if (seg_next == kReduceSegments - 1) *call.reduce_epoch = epoch;

@@ -16,31 +16,30 @@ constexpr int kMaxPeers = kMaxRanksPerDomain;
 constexpr int kReduceSegments = 16;  // a replica's gradient is released for zeroing in this many pieces
 constexpr unsigned long long kReduceFlagRadix = 64;  // progress word = epoch * radix + segments done
 
-// Device-resident, per hosted rank, immutable after connect. Peer tables are indexed
-// by global rank; entry [my_rank] is this rank's own buffer.
 constexpr int kPlanMaxCtas = 32;  // CTAs of one rank in the plan kernel
 
-struct RankDev {
-    int my_rank;
-    int num_ranks;
-    // plan exchange
-    uint64_t* hist_parts;    // [kPlanMaxCtas][Lpad] words, (epoch tag << 32) | partial count of one CTA of the plan kernel
-    uint64_t* peer_gather[kMaxPeers];  // each: [2][N][Lpad] words, (epoch tag << 32) | token count
-    int32_t* global_loads;   // [L]
-    int32_t* loads_per_rank; // [N][L] latest gathered matrix (contiguous copy)
-    // weight sync / grad reduce
-    int* sync_ticket;        // zero between calls
-    uint8_t* peer_replica_weight[kMaxPeers];
-    uint8_t* peer_replica_scale[kMaxPeers];
-    float* peer_replica_grad[kMaxPeers];
-    uint64_t* peer_sync_flags[kMaxPeers];  // each: [N], entry [src] = last epoch src finished sending to that rank
-    uint64_t* peer_relay_flags[kMaxPeers]; // each: [R][relay_cap], entry [slot][tile] = epoch in which the master delivered that tile
-    uint64_t* peer_reduce_flags[kMaxPeers]; // each: [N], entry [src] = epoch * 64 + segments of its pulls master rank src has finished
-    int* reduce_counters;    // [kReduceSegments]: CTAs of the running Wgrad reduce that have passed each segment; zero between calls
-    DeviceStatus* status;    // mapped pinned host memory
-    // [0] plan epoch, [1] sync epoch, [2] Wgrad-reduce epoch: counted on the device (by one CTA of every launch), not
-    // passed by value, so that a captured CUDA graph can be replayed: every replay is a new epoch
-    uint64_t* epochs;
+// Where the group's buffers are. By value in the kernels' parameters, so that the first load of a kernel is of data and not
+// of a pointer to it (each of the two is a miss: the tables were last read a layer ago). Fixed once connected. With a table
+// per rank in device memory, and the plan's epoch and weight_sync's first unit waited for before the first load of data, the
+// step of eight ranks (8192 tokens, 128 experts, fp8 weights of 19 MB) took 70.0 us, 64.6 like this; plan kernel 19.0 and
+// 17.3.
+struct GroupDev {
+    uint8_t* arena[kMaxPeers];  // of every rank of the group, as the hosted ranks see them (all of them the same)
+    int64_t gather, sync_flags, relay_flags, reduce_flags, replica_weight, replica_scale, replica_grad;  // offsets in an arena
+    int my_rank[kMaxLocalRanks];
+    DeviceStatus* status[kMaxLocalRanks];  // mapped pinned host memory
+
+    // [2][N][Lpad] words, (epoch tag << 32) | token count
+    __device__ __forceinline__ uint64_t* gather_of(int rank) const { return reinterpret_cast<uint64_t*>(arena[rank] + gather); }
+    // [N], entry [src] = last epoch src finished sending to that rank
+    __device__ __forceinline__ uint64_t* sync_flags_of(int rank) const { return reinterpret_cast<uint64_t*>(arena[rank] + sync_flags); }
+    // [R][relay_cap], entry [slot][chunk] = epoch in which the master delivered that chunk
+    __device__ __forceinline__ uint64_t* relay_flags_of(int rank) const { return reinterpret_cast<uint64_t*>(arena[rank] + relay_flags); }
+    // [N], entry [src] = epoch * 64 + segments of its pulls master rank src has finished
+    __device__ __forceinline__ uint64_t* reduce_flags_of(int rank) const { return reinterpret_cast<uint64_t*>(arena[rank] + reduce_flags); }
+    __device__ __forceinline__ uint8_t* weight_of(int rank) const { return arena[rank] + replica_weight; }
+    __device__ __forceinline__ uint8_t* scale_of(int rank) const { return arena[rank] + replica_scale; }
+    __device__ __forceinline__ float* grad_of(int rank) const { return reinterpret_cast<float*>(arena[rank] + replica_grad); }
 };
 
 struct PlanPtrs {
@@ -59,7 +58,13 @@ struct ShardLayout {  // bytes of the four weight shards and their place inside 
 void count_launch(int n = 1);
 
 struct PlanCall {
-    const RankDev* rank[kMaxLocalRanks];
+    GroupDev group;
+    uint64_t* hist_parts[kMaxLocalRanks];    // [kPlanMaxCtas][Lpad] words, (epoch tag << 32) | partial count of one CTA
+    // Counted on the device (by one CTA of every launch), not passed by value, so that a captured CUDA graph can be
+    // replayed: every replay is a new epoch. The same for the epochs of weight_sync and of the Wgrad reduce.
+    uint64_t* epoch[kMaxLocalRanks];
+    int32_t* global_loads[kMaxLocalRanks];   // [L]
+    int32_t* loads_per_rank[kMaxLocalRanks]; // [N][L] latest gathered matrix (contiguous copy)
     const void* input[kMaxLocalRanks];
     int T[kMaxLocalRanks];
     PlanPtrs plan[kMaxLocalRanks];
@@ -78,8 +83,7 @@ cudaError_t launch_plan(const PlanCall& call, cudaStream_t stream);
 int plan_ctas_per_rank(int input_kind, int max_T, int K_or_L, int nlocal, int num_sms);
 
 struct SyncCall {
-    const RankDev* rank[kMaxLocalRanks];
-    int my_rank[kMaxLocalRanks];  // rank ids by value: one pointer hop less in every CTA's set-up
+    GroupDev group;
     PlanPtrs plan[kMaxLocalRanks];
     const int64_t* src_ptrs[kMaxLocalRanks][4];  // device int64[M] tables; scale tables may be null
     int nlocal;
@@ -92,15 +96,15 @@ struct SyncCall {
                              // replicas are scattered over them and forwarded replica to replica
     int relay_adaptive;      // 1: also relay the experts of ranks that send more than any rank receives (see weight_sync.cu)
     int relay_cap;           // chunks per slot the ready-flag table has room for
-    uint64_t* sync_epoch;    // the sync epoch counter of the first hosted rank (by value: one load, not two)
+    uint64_t* sync_epoch;    // the sync epoch counter of the first hosted rank
+    int* ticket;             // [2], zero between calls: CTAs that have finished, units handed out
     unsigned long long* trace;  // optional: 8 globaltimer stamps per CTA (tuning aid), or null
 };
 cudaError_t launch_weight_sync(const SyncCall& call, cudaStream_t stream);
 int weight_sync_max_ctas_per_rank(int nlocal, int num_sms);
 
 struct ReduceCall {
-    const RankDev* rank[kMaxLocalRanks];
-    int my_rank[kMaxLocalRanks];
+    GroupDev group;
     PlanPtrs plan[kMaxLocalRanks];
     const int64_t* fc1_grad_ptrs[kMaxLocalRanks];
     const int64_t* fc2_grad_ptrs[kMaxLocalRanks];
@@ -111,6 +115,7 @@ struct ReduceCall {
     int ctas_per_rank;
     int owners_clear;           // test hook: replicas of hosted ranks are cleared by their owners too, as on other devices
     uint64_t* reduce_epoch;     // the reduce epoch counter of the first hosted rank
+    int* counters;              // [kReduceSegments]: CTAs of this launch that have passed each segment; zero between calls
     unsigned long long* trace;  // optional: 8 globaltimer stamps per CTA (tuning aid), or null
 };
 cudaError_t launch_grad_reduce(const ReduceCall& call, cudaStream_t stream);

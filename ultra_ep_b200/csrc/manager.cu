@@ -122,7 +122,6 @@ struct RankHost {
     int32_t* loads_per_rank = nullptr;          // [N][L]
     DeviceStatus* status_host = nullptr;        // mapped pinned
     DeviceStatus* status_dev = nullptr;
-    RankDev* dev = nullptr;
     // reroute scratch (per-tile expert counts), one buffer per form so that a dense and a sparse
     // reroute of different layers never share one: [0] dense, [1] sparse
     int32_t* scratch[2] = {nullptr, nullptr};
@@ -141,6 +140,7 @@ struct uep_manager {
     int64_t scale_fc2_offset = 0, scale_stride = 0, weight_stride = 0, total_numel = 0;
     int64_t layer_stride = 0;  // int32 elements per layer in plan_blob
     ArenaLayout arena{};
+    GroupDev group{};  // as the kernels take it
     std::vector<RankHost> ranks;
     cudaStream_t comm_stream = nullptr;
     cudaEvent_t order_event = nullptr;  // reusable event for stream-to-stream ordering
@@ -212,30 +212,25 @@ int ensure_scratch(RankHost& r, int which, int64_t elems) {
     return UEP_OK;
 }
 
-int upload_rank_dev(uep_manager* m, RankHost& r) {
-    RankDev d;
+// What the kernels need to know of the group, once every arena is mapped.
+int describe_group(uep_manager* m) {
+    GroupDev& d = m->group;
     std::memset(&d, 0, sizeof(d));
-    d.my_rank = r.rank;
-    d.num_ranks = m->N;
-    d.hist_parts = r.hist_parts;
-    d.sync_ticket = r.tickets + 1;
-    d.reduce_counters = r.tickets + 4;
-    d.epochs = r.epochs;
-    d.global_loads = r.global_loads;
-    d.loads_per_rank = r.loads_per_rank;
-    d.status = r.status_dev;
     for (int p = 0; p < m->N; ++p) {
-        uint8_t* base = static_cast<uint8_t*>(r.peer_arena[p]);
-        if (base == nullptr) return fail(UEP_ERR_STATE, "connect: a peer arena is not mapped");
-        d.peer_gather[p] = reinterpret_cast<uint64_t*>(base + m->arena.gather);
-        d.peer_sync_flags[p] = reinterpret_cast<uint64_t*>(base + m->arena.sync_flags);
-        d.peer_reduce_flags[p] = reinterpret_cast<uint64_t*>(base + m->arena.reduce_flags);
-        d.peer_relay_flags[p] = reinterpret_cast<uint64_t*>(base + m->arena.relay_flags);
-        d.peer_replica_weight[p] = base + m->arena.replica_weight;
-        d.peer_replica_scale[p] = base + m->arena.replica_scale;
-        d.peer_replica_grad[p] = reinterpret_cast<float*>(base + m->arena.replica_grad);
+        d.arena[p] = static_cast<uint8_t*>(m->ranks[0].peer_arena[p]);
+        if (d.arena[p] == nullptr) return fail(UEP_ERR_STATE, "connect: a peer arena is not mapped");
     }
-    UEP_CUDA_TRY(cudaMemcpy(r.dev, &d, sizeof(d), cudaMemcpyHostToDevice));
+    d.gather = static_cast<int64_t>(m->arena.gather);
+    d.sync_flags = static_cast<int64_t>(m->arena.sync_flags);
+    d.relay_flags = static_cast<int64_t>(m->arena.relay_flags);
+    d.reduce_flags = static_cast<int64_t>(m->arena.reduce_flags);
+    d.replica_weight = static_cast<int64_t>(m->arena.replica_weight);
+    d.replica_scale = static_cast<int64_t>(m->arena.replica_scale);
+    d.replica_grad = static_cast<int64_t>(m->arena.replica_grad);
+    for (int i = 0; i < m->nlocal; ++i) {
+        d.my_rank[i] = m->ranks[i].rank;
+        d.status[i] = m->ranks[i].status_dev;
+    }
     return UEP_OK;
 }
 
@@ -255,7 +250,6 @@ void free_rank(RankHost& r, int my_rank_count) {
     cudaFree(r.epochs);
     cudaFree(r.global_loads);
     cudaFree(r.loads_per_rank);
-    cudaFree(r.dev);
     cudaFree(r.scratch[0]);
     cudaFree(r.scratch[1]);
     if (r.status_host != nullptr) cudaFreeHost(r.status_host);
@@ -408,7 +402,6 @@ int uep_manager_create(const uep_config* cfg, uep_manager** out) {
         UEP_TRY_BAIL(cudaMemset(r.global_loads, 0, sizeof(int32_t) * m->L));
         UEP_TRY_BAIL(cudaMalloc(&r.loads_per_rank, sizeof(int32_t) * static_cast<size_t>(N) * m->L));
         UEP_TRY_BAIL(cudaMemset(r.loads_per_rank, 0, sizeof(int32_t) * static_cast<size_t>(N) * m->L));
-        UEP_TRY_BAIL(cudaMalloc(&r.dev, sizeof(RankDev)));
         UEP_TRY_BAIL(cudaHostAlloc(&r.status_host, sizeof(DeviceStatus), cudaHostAllocMapped));
         r.status_host->code = 0;
         r.status_host->detail = 0;
@@ -456,8 +449,6 @@ int uep_manager_connect(uep_manager* m, const void* all_handles) {
     if (m->nlocal > 1) {
         for (auto& r : m->ranks) {
             for (int p = 0; p < m->N; ++p) r.peer_arena[p] = m->ranks[p].arena;
-            const int rc = upload_rank_dev(m, r);
-            if (rc != UEP_OK) return rc;
         }
     } else {
         RankHost& r = m->ranks[0];
@@ -475,9 +466,9 @@ int uep_manager_connect(uep_manager* m, const void* all_handles) {
             r.peer_arena[p] = ptr;
             r.peer_opened[p] = true;
         }
-        const int rc = upload_rank_dev(m, r);
-        if (rc != UEP_OK) return rc;
     }
+    const int rc = describe_group(m);
+    if (rc != UEP_OK) return rc;
     UEP_CUDA_TRY(cudaDeviceSynchronize());
     m->connected = true;
     return UEP_OK;
@@ -628,11 +619,16 @@ int uep_update_placement(uep_manager* m, int layer_id, int input_kind, const voi
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     PlanCall call;
     std::memset(&call, 0, sizeof(call));
+    call.group = m->group;
     int max_T = 0;
     for (int i = 0; i < m->nlocal; ++i) {
         if (T[i] < 0) return fail(UEP_ERR_INVALID, "update_placement: negative token count");
         if (T[i] > 0 && K_or_L > 0 && inputs[i] == nullptr) return fail(UEP_ERR_INVALID, "update_placement: null input");
-        call.rank[i] = m->ranks[i].dev;
+        const RankHost& r = m->ranks[i];
+        call.hist_parts[i] = r.hist_parts;
+        call.epoch[i] = r.epochs;
+        call.global_loads[i] = r.global_loads;
+        call.loads_per_rank[i] = r.loads_per_rank;
         call.input[i] = inputs[i];
         call.T[i] = T[i];
         call.plan[i] = plan_ptrs(m, m->ranks[i], layer_id);
@@ -677,10 +673,10 @@ int uep_weight_sync(uep_manager* m, int layer_id, const int64_t* const* fc1_ptrs
 
     SyncCall call;
     std::memset(&call, 0, sizeof(call));
+    call.group = m->group;
+    call.ticket = m->ranks[0].tickets + 1;
     for (int i = 0; i < m->nlocal; ++i) {
         if (fc1_ptrs[i] == nullptr || fc2_ptrs[i] == nullptr) return fail(UEP_ERR_INVALID, "weight_sync: null pointer table");
-        call.rank[i] = m->ranks[i].dev;
-        call.my_rank[i] = m->ranks[i].rank;
         call.plan[i] = plan_ptrs(m, m->ranks[i], layer_id);
         call.src_ptrs[i][0] = fc1_ptrs[i];
         call.src_ptrs[i][1] = fc2_ptrs[i];
@@ -733,10 +729,10 @@ int uep_grad_reduce(uep_manager* m, int layer_id, const int64_t* const* fc1_grad
     }
     ReduceCall call;
     std::memset(&call, 0, sizeof(call));
+    call.group = m->group;
+    call.counters = m->ranks[0].tickets + 4;
     for (int i = 0; i < m->nlocal; ++i) {
         if (fc1_grad_ptrs[i] == nullptr || fc2_grad_ptrs[i] == nullptr) return fail(UEP_ERR_INVALID, "grad_reduce: null pointer table");
-        call.rank[i] = m->ranks[i].dev;
-        call.my_rank[i] = m->ranks[i].rank;
         call.plan[i] = plan_ptrs(m, m->ranks[i], layer_id);
         call.fc1_grad_ptrs[i] = fc1_grad_ptrs[i];
         call.fc2_grad_ptrs[i] = fc2_grad_ptrs[i];

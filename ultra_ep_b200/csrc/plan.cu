@@ -245,7 +245,8 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(PlanCall call) {
 
     const int local = blockIdx.x / call.ctas_per_rank;
     const int part = blockIdx.x % call.ctas_per_rank;
-    const RankDev& rk = *call.rank[local];
+    const GroupDev& group = call.group;
+    uint64_t* const hist_parts = call.hist_parts[local];
     const int N = call.N, M = call.M;
     const int L = N * M;
     const int Lpad = (L + 3) / 4 * 4;
@@ -261,19 +262,21 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(PlanCall call) {
     for (int i = tid; i < L; i += blockDim.x) hist[i] = 0;
     if (tid == 0) {
         s_timeout_peer = -1;
-        // the epoch this launch opens: the owner stores it once it holds every partial, so every CTA of the
-        // launch reads the same value here
-        s_epoch = *reinterpret_cast<volatile uint64_t*>(rk.epochs) + 1;
     }
+    // the epoch this launch opens: the owner stores it once it holds every partial, so every CTA of the launch reads the
+    // same value here
+    uint64_t last_epoch = 0;
+    if (tid == 0) last_epoch = ld_relaxed_sys_u64(call.epoch[local]);  // on its way while the slice is counted
     __syncthreads();
     histogram_slice(call.input_kind, call.input[local], call.T[local], call.K_or_L, L, part, call.ctas_per_rank, hist);
+    if (tid == 0) s_epoch = last_epoch + 1;
     __syncthreads();
     const uint64_t epoch = s_epoch;
     // never zero (the buffers start zeroed), period 2^32 - 1: an odd period, so the word that carried the same
     // tag one period ago sat in the other parity slot and cannot be mistaken for this epoch's
     const uint32_t tag = static_cast<uint32_t>(epoch % 0xFFFFFFFFull) + 1u;
     if (part != 0) {
-        uint64_t* row = rk.hist_parts + static_cast<int64_t>(part) * Lpad;
+        uint64_t* row = hist_parts + static_cast<int64_t>(part) * Lpad;
         for (int i = tid; i < L; i += blockDim.x) st_relaxed_sys_u64(row + i, tag_word(tag, static_cast<uint32_t>(hist[i])));
         return;
     }
@@ -292,16 +295,16 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(PlanCall call) {
 #pragma unroll
                 for (int u = 0; u < kPartBatch; ++u) {
                     const int c = c0 + u * parts;
-                    if (c <= rest) w[u] = ld_relaxed_sys_u64(rk.hist_parts + static_cast<int64_t>(c) * Lpad + i);
+                    if (c <= rest) w[u] = ld_relaxed_sys_u64(hist_parts + static_cast<int64_t>(c) * Lpad + i);
                 }
 #pragma unroll
                 for (int u = 0; u < kPartBatch; ++u) {
                     const int c = c0 + u * parts;
                     if (c <= rest) {
                         if (static_cast<uint32_t>(w[u] >> 32) != tag &&
-                            !wait_tagged_word(rk.hist_parts + static_cast<int64_t>(c) * Lpad + i, tag,
+                            !wait_tagged_word(hist_parts + static_cast<int64_t>(c) * Lpad + i, tag,
                                               *reinterpret_cast<volatile int*>(&s_timeout_peer) >= 0 ? 0 : call.timeout_ns, w[u])) {
-                            atomicMax(&s_timeout_peer, rk.my_rank);
+                            atomicMax(&s_timeout_peer, group.my_rank[local]);
                             w[u] = 0;
                         }
                         total += static_cast<int32_t>(static_cast<uint32_t>(w[u]));
@@ -312,9 +315,9 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(PlanCall call) {
         }
     }
     __syncthreads();
-    if (tid == 0) *rk.epochs = epoch;  // every CTA of the launch has read the old value: its partial carried the tag
+    if (tid == 0) *call.epoch[local] = epoch;  // every CTA of the launch has read the old value: its partial carried the tag
     if (s_timeout_peer >= 0) {  // a CTA of this very launch never delivered
-        if (tid == 0) report_error(rk.status, UEP_DEV_TIMEOUT_GATHER, s_timeout_peer);
+        if (tid == 0) report_error(group.status[local], UEP_DEV_TIMEOUT_GATHER, s_timeout_peer);
         return;
     }
     stamp(0);
@@ -323,11 +326,11 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(PlanCall call) {
     //    count, so a row needs neither a fence nor a flag: one NVLink crossing, and the reader knows a word
     //    is this layer's when it sees it.
     const int slot = static_cast<int>(epoch & 1ull);
-    const int me = rk.my_rank;
+    const int me = group.my_rank[local];
     if (me != call.withhold_rank) {
         for (int idx = tid; idx < N * L; idx += blockDim.x) {
             const int p = idx / L, i = idx % L;
-            st_relaxed_sys_u64(rk.peer_gather[p] + (static_cast<int64_t>(slot) * N + me) * Lpad + i,
+            st_relaxed_sys_u64(group.gather_of(p) + (static_cast<int64_t>(slot) * N + me) * Lpad + i,
                                tag_word(tag, static_cast<uint32_t>(hist[i])));
         }
     }
@@ -342,7 +345,7 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(PlanCall call) {
     // 3. collect every rank's row (bounded), expose the matrix, reduce. A thread owns one expert:
     //    it first issues the loads of eight ranks' words together and only then looks at them,
     //    so the common case (all rows already here) costs one memory round trip.
-    const uint64_t* gathered = rk.peer_gather[me] + static_cast<int64_t>(slot) * N * Lpad;
+    const uint64_t* gathered = group.gather_of(me) + static_cast<int64_t>(slot) * N * Lpad;
     for (int i = tid; i < L; i += blockDim.x) {
         int32_t total = 0;
         for (int r0 = 0; r0 < N; r0 += 8) {
@@ -362,13 +365,13 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(PlanCall call) {
                         w[u] = 0;
                     }
                     const int32_t v = static_cast<int32_t>(static_cast<uint32_t>(w[u]));
-                    rk.loads_per_rank[static_cast<int64_t>(r0 + u) * L + i] = v;
+                    call.loads_per_rank[local][static_cast<int64_t>(r0 + u) * L + i] = v;
                     if (staged) matrix[(r0 + u) * L + i] = v;
                     total += v;
                 }
             }
         }
-        rk.global_loads[i] = total;
+        call.global_loads[local][i] = total;
         if (preload) {
             solver_sm.my_loads[i] = hist[i];
             solver_sm.loads[i] = total;  // (hist[i] itself)
@@ -377,15 +380,15 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(PlanCall call) {
     __threadfence_block();
     __syncthreads();
     if (s_timeout_peer >= 0) {
-        if (tid == 0) report_error(rk.status, UEP_DEV_TIMEOUT_GATHER, s_timeout_peer);
+        if (tid == 0) report_error(group.status[local], UEP_DEV_TIMEOUT_GATHER, s_timeout_peer);
         return;  // plan of this layer is left as it was; the host raises on the status word
     }
 
     stamp(2);
     stamp(3);
     SolveArgs a;
-    a.global_loads = rk.global_loads;
-    a.loads_per_rank = rk.loads_per_rank;
+    a.global_loads = call.global_loads[local];
+    a.loads_per_rank = call.loads_per_rank[local];
     const PlanPtrs& pp = call.plan[local];
     a.p2l = pp.p2l; a.l2p = pp.l2p; a.lcnts = pp.lcnts; a.quota = pp.quota; a.quota_prefix = pp.quota_prefix;
     a.rank_quota_prefix = pp.rank_quota_prefix;
@@ -402,7 +405,7 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(PlanCall call) {
     a.staged_loads = staged ? matrix : nullptr;
     a.trace = call.trace != nullptr ? call.trace + (kMaxLocalRanks + local) * 8 : nullptr;
     const int num_domains = N / call.G;
-    for (int d = 0; d < num_domains; ++d) solve_domain_dispatch(a, d, smem_raw, rk.status);
+    for (int d = 0; d < num_domains; ++d) solve_domain_dispatch(a, d, smem_raw, group.status[local]);
     stamp(4);
 }
 

@@ -104,11 +104,6 @@ struct SyncShared {
     uint8_t* dst_weight[kMaxSends];               // replica slot base in the peer's weight buffer (null: skip)
     uint8_t* dst_scale[kMaxSends];                // replica slot base in the peer's scale buffer
     uint64_t* dst_flags[kMaxSends];               // that slot's row of ready flags on the peer (relay)
-    // replica buffer bases of every (hosted rank, peer): nlocal * N entries (at most 72: several
-    // hosted ranks mean a simulated group of at most 8)
-    uint8_t* peer_weight[kMaxPeers];
-    uint8_t* peer_scale[kMaxPeers];
-    uint64_t* peer_flags[kMaxPeers];
     // forward entries: one per local replica slot that holds a relayed expert
     uint8_t* fwd_src_w[kMaxFwd];        // the slot itself
     uint8_t* fwd_src_s[kMaxFwd];
@@ -175,6 +170,7 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
     int* shard_tiles = sm.shard_tiles;
 
     const ShardLayout& sh = call.shards;
+    const GroupDev& group = call.group;
     const int M = call.M, R = call.R, D = call.D, Lp = M + R, N = call.N, nlocal = call.nlocal;
     const int tid = threadIdx.x;
     // Relaying needs a forward entry per local replica slot and a ready flag per chunk; the limits depend on
@@ -219,10 +215,10 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
     }
     __syncthreads();
     // Every global read of the set-up is issued here, before anything depends on one of them, so
-    // that they share one memory round trip instead of forming a chain (counts -> l2p rows ->
-    // peer tables): the plan rows of the first 128 masters (speculatively the whole l2p row when
-    // it has at most 8 entries), their source addresses, the peers' buffer bases and the
-    // owners of this rank's redundant slots.
+    // that they share one memory round trip instead of forming a chain (counts -> l2p rows): the plan
+    // rows of the first 128 masters (speculatively the whole l2p row when it has at most 8 entries),
+    // their source addresses and the owners of this rank's redundant slots. Where the peers' buffers
+    // are comes with the parameters.
     const int total_masters = nlocal * M;
     const bool row_cached = D <= 8;
     int pre_reps = 0, pre_row[7];
@@ -230,7 +226,7 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
     {
         const bool valid = tid < total_masters;
         const int lr = valid ? tid / M : 0, m = valid ? tid % M : 0;
-        const int l = call.my_rank[lr] * M + m;
+        const int l = group.my_rank[lr] * M + m;
         const PlanPtrs& plan = call.plan[lr];
         pre_reps = valid ? plan.lcnts[l] - 1 : 0;
 #pragma unroll
@@ -241,30 +237,17 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
             pre_src[sh_i] = present ? static_cast<uintptr_t>(call.src_ptrs[lr][sh_i][m]) : 0;
         }
     }
-    uint8_t *pre_pw = nullptr, *pre_ps = nullptr;
-    uint64_t* pre_pf = nullptr;
-    if (tid < nlocal * N) {
-        const RankDev& rk = *call.rank[tid / N];
-        pre_pw = rk.peer_replica_weight[tid % N];
-        pre_ps = rk.peer_replica_scale[tid % N];
-        if (kRelay) pre_pf = rk.peer_relay_flags[tid % N];
-    }
     // Ranks hosted together share the first one's epoch counter: they always run in the same launches.
     // The CTA that finishes last stores the new value; nobody reads the counter after that.
     unsigned long long pre_epoch = 0;
     if (tid == 0) pre_epoch = *call.sync_epoch;
     int pre_owner = -1;
-    if (tid < nlocal * R) pre_owner = call.plan[tid / R].p2l[call.my_rank[tid / R] * Lp + M + tid % R];
+    if (tid < nlocal * R) pre_owner = call.plan[tid / R].p2l[group.my_rank[tid / R] * Lp + M + tid % R];
     // relay decision: the replica count of logical expert `tid` and the owner of redundant slot `tid` of the group
     int pre_lc = 1, pre_slot_owner = -1;
     if (kRelay && relay_on) {
         if (tid < N * M) pre_lc = call.plan[0].lcnts[tid];
         if (call.relay_adaptive && tid < N * R) pre_slot_owner = call.plan[0].p2l[(tid / R) * Lp + M + tid % R];
-    }
-    if (tid < nlocal * N) {
-        sm.peer_weight[tid] = pre_pw;
-        sm.peer_scale[tid] = pre_ps;
-        sm.peer_flags[tid] = pre_pf;
     }
     if (tid == 0) sm.epoch = pre_epoch + 1;
 
@@ -325,9 +308,8 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
         const int gm = g0 + tid;
         const int lr = gm < total_masters ? gm / M : 0;
         const int m = gm < total_masters ? gm % M : 0;
-        const RankDev& rk = *call.rank[lr];
         const PlanPtrs& plan = call.plan[lr];
-        const int me = call.my_rank[lr];
+        const int me = group.my_rank[lr];
         int reps = 0;
         if (gm < total_masters) {
             reps = g0 == 0 ? pre_reps : plan.lcnts[me * M + m] - 1;
@@ -364,15 +346,15 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
             auto place = [&](int j, int phys) {
                 const int drank = phys / Lp, dslot = phys % Lp - M;
                 if (phys < 0 || drank >= N || dslot < 0 || dslot >= R) {  // never store outside a slot table
-                    report_error(rk.status, UEP_DEV_BAD_PLAN, l);
+                    report_error(group.status[lr], UEP_DEV_BAD_PLAN, l);
                     sm.dst_weight[rs + j] = nullptr;
                     sm.dst_scale[rs + j] = nullptr;
                     if (kRelay) sm.dst_flags[rs + j] = nullptr;
                 } else {
                     atomicOr(&sm.send_mask[lr][drank >> 5], 1u << (drank & 31));
-                    sm.dst_weight[rs + j] = sm.peer_weight[lr * N + drank] + static_cast<int64_t>(dslot) * sh.weight_slot_stride;
-                    sm.dst_scale[rs + j] = sm.peer_scale[lr * N + drank] + static_cast<int64_t>(dslot) * sh.scale_slot_stride;
-                    if (kRelay) sm.dst_flags[rs + j] = sm.peer_flags[lr * N + drank] + static_cast<int64_t>(dslot) * call.relay_cap;
+                    sm.dst_weight[rs + j] = group.weight_of(drank) + static_cast<int64_t>(dslot) * sh.weight_slot_stride;
+                    sm.dst_scale[rs + j] = group.scale_of(drank) + static_cast<int64_t>(dslot) * sh.scale_slot_stride;
+                    if (kRelay) sm.dst_flags[rs + j] = group.relay_flags_of(drank) + static_cast<int64_t>(dslot) * call.relay_cap;
                 }
             };
             if (g0 == 0 && row_cached) {
@@ -422,7 +404,7 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
     int my_fwd_r = 0, my_fwd_k = -1, my_l = -1;
     for (int i = tid; i < nlocal * R; i += blockDim.x) {
         const int lr = i / R, slot = i % R;
-        const int me = call.my_rank[lr];
+        const int me = group.my_rank[lr];
         const int l = i == tid ? pre_owner : call.plan[lr].p2l[me * Lp + M + slot];
         if (l >= 0) {
             const int src = l / M;
@@ -452,10 +434,10 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
         for (int w = 0; w < warp; ++w) f += sm.w_a[w];
         if (my_fwd_r > 0) {
             const int lr = tid / R, slot = tid % R;
-            const int me = call.my_rank[lr];
-            sm.fwd_src_w[f] = sm.peer_weight[lr * N + me] + static_cast<int64_t>(slot) * sh.weight_slot_stride;
-            sm.fwd_src_s[f] = sm.peer_scale[lr * N + me] + static_cast<int64_t>(slot) * sh.scale_slot_stride;
-            sm.fwd_flags[f] = sm.peer_flags[lr * N + me] + static_cast<int64_t>(slot) * call.relay_cap;
+            const int me = group.my_rank[lr];
+            sm.fwd_src_w[f] = group.weight_of(me) + static_cast<int64_t>(slot) * sh.weight_slot_stride;
+            sm.fwd_src_s[f] = group.scale_of(me) + static_cast<int64_t>(slot) * sh.scale_slot_stride;
+            sm.fwd_flags[f] = group.relay_flags_of(me) + static_cast<int64_t>(slot) * call.relay_cap;
             sm.fwd_r[f] = static_cast<unsigned char>(my_fwd_r);
             sm.fwd_k[f] = static_cast<unsigned char>(my_fwd_k);
             sm.fwd_lr[f] = static_cast<unsigned char>(lr);
@@ -475,7 +457,7 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
         __syncthreads();
         if (my_fwd_r > 0) {
             const int lr = tid / R;
-            const int me = call.my_rank[lr];
+            const int me = group.my_rank[lr];
             int o = sm.fwd_dst_start[f];
             for (int j = 0; j < my_fwd_r; ++j) {
                 const int phys = call.plan[lr].l2p[static_cast<int64_t>(my_l) * D + 1 + j];
@@ -488,8 +470,8 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
                     sm.fwd_dst_s[o] = nullptr;
                 } else {
                     atomicOr(&sm.send_mask[lr][drank >> 5], 1u << (drank & 31));
-                    sm.fwd_dst_w[o] = sm.peer_weight[lr * N + drank] + static_cast<int64_t>(dslot) * sh.weight_slot_stride;
-                    sm.fwd_dst_s[o] = sm.peer_scale[lr * N + drank] + static_cast<int64_t>(dslot) * sh.scale_slot_stride;
+                    sm.fwd_dst_w[o] = group.weight_of(drank) + static_cast<int64_t>(dslot) * sh.weight_slot_stride;
+                    sm.fwd_dst_s[o] = group.scale_of(drank) + static_cast<int64_t>(dslot) * sh.scale_slot_stride;
                 }
                 ++o;
             }
@@ -503,8 +485,8 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
     // that neither scatters nor forwards anything in this launch takes the compact one: the kernel runs once per
     // layer from a cold instruction cache, and every extra line of code on the path of the first tiles is a miss.
     const uint64_t epoch = sm.epoch;
-    DeviceStatus* status0 = call.rank[0]->status;
-    int* unit_counter = call.rank[0]->sync_ticket + 1;
+    DeviceStatus* status0 = group.status[0];
+    int* unit_counter = call.ticket + 1;
     auto run_copy = [&](auto relay_tag) {
         constexpr bool kR = decltype(relay_tag)::value;
         const int n_relay = kR ? sm.n_relay : 0;
@@ -512,6 +494,9 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
         const int relay_units = n_relay * chunks_per_expert;
         const int send_units = relay_units + n_direct * tiles_per_expert;
         const int total_units = send_units + (kR ? sm.fwd_units : 0);
+        // A CTA's first unit is its own number where nothing is relayed, so that its first load does not wait for the
+        // counter's round trip. (A unit that others wait for may not be held for a CTA that has not started.)
+        const int first_shared = kR ? 0 : static_cast<int>(gridDim.x);
         // Work is handed out by an atomic counter: CTAs that run on busy SMs (the reroute and the
         // model's own kernels run next to this one) simply take less, and replica counts that differ
         // between masters cannot leave some CTAs with several times the work of others.
@@ -558,7 +543,7 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
             bool ok = true;
             if (!wait_flag_ge_relaxed(sm.fwd_flags[un.who] + un.chunk, epoch, call.timeout_ns)) {
                 ok = false;
-                report_error(call.rank[sm.fwd_lr[un.who]]->status, UEP_DEV_TIMEOUT_SYNC, un.chunk);
+                report_error(group.status[sm.fwd_lr[un.who]], UEP_DEV_TIMEOUT_SYNC, un.chunk);
             }
             (void)ld_acquire_sys_u64(sm.fwd_flags[un.who] + un.chunk);  // acquire side of the flag
             fence_proxy_async_global();                                 // ... also for the bulk copies that read the chunk next
@@ -622,7 +607,7 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
                 };
                 // The index of the next unit is requested one load ahead, so the round trip of the
                 // atomic overlaps with the copies instead of sitting in front of every load.
-                int pending = atomicAdd(unit_counter, 1);
+                int pending = kR ? atomicAdd(unit_counter, 1) : static_cast<int>(blockIdx.x);
                 Unit cur{};
                 int cur_tile = 0;
                 bool have_cur = false;
@@ -651,7 +636,7 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
                             cur = decode_unit(pending);
                             cur_tile = cur.tile;
                             have_cur = true;
-                            pending = atomicAdd(unit_counter, 1);
+                            pending = first_shared + atomicAdd(unit_counter, 1);
                             if (kR && cur.kind == 2 && cur_tile < cur.tile_end) {
                                 if (!chunk_arrived(cur)) {
                                     deferred = true;
@@ -793,9 +778,9 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
                 }
             }
         } else {
-            while (true) {
+            for (bool first = true;; first = false) {
                 __syncthreads();
-                if (tid == 0) sm.s_unit = atomicAdd(unit_counter, 1);
+                if (tid == 0) sm.s_unit = first && !kR ? static_cast<int>(blockIdx.x) : first_shared + atomicAdd(unit_counter, 1);
                 __syncthreads();
                 const int u = sm.s_unit;
                 if (u >= total_units) break;
@@ -843,7 +828,7 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
 
     // ---- completion: the last CTA of the launch signals the receivers of every hosted rank
     // and waits for their senders
-    int* ticket_ptr = call.rank[0]->sync_ticket;
+    int* ticket_ptr = call.ticket;
     if (tid == 0) {
         const int ticket = atomicAdd(ticket_ptr, 1);
         if (ticket == static_cast<int>(gridDim.x) - 1) {
@@ -869,11 +854,10 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
         if (tid == 0) {
             __threadfence_system();
             for (int lr = 0; lr < nlocal; ++lr) {
-                const int me = call.my_rank[lr];
+                const int me = group.my_rank[lr];
                 if (me == call.withhold_rank) continue;
-                const RankDev& rk = *call.rank[lr];
                 for (int p = 0; p < N; ++p) {
-                    if (sm.send_mask[lr][p >> 5] & (1u << (p & 31))) st_relaxed_sys_u64(rk.peer_sync_flags[p] + me, epoch);
+                    if (sm.send_mask[lr][p >> 5] & (1u << (p & 31))) st_relaxed_sys_u64(group.sync_flags_of(p) + me, epoch);
                 }
             }
         }
@@ -887,10 +871,9 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
         for (int i = tid; i < nlocal * N; i += blockDim.x) {
             const int lr = i / N, p = i % N;
             if (sm.recv_mask[lr][p >> 5] & (1u << (p & 31))) {
-                const RankDev& rk = *call.rank[lr];
-                if (!wait_flag_ge_relaxed(rk.peer_sync_flags[call.my_rank[lr]] + p, epoch, call.timeout_ns)) {
+                if (!wait_flag_ge_relaxed(group.sync_flags_of(group.my_rank[lr]) + p, epoch, call.timeout_ns)) {
                     atomicMax(&sm.timeout_peer, p);
-                    report_error(rk.status, UEP_DEV_TIMEOUT_SYNC, p);
+                    report_error(group.status[lr], UEP_DEV_TIMEOUT_SYNC, p);
                 }
             }
         }
