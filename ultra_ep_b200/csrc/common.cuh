@@ -115,6 +115,13 @@ __device__ __forceinline__ bool wait_flag_ge_relaxed(const uint64_t* flag, uint6
     }
 }
 
+// Programmatic dependent launch: a kernel that is launched with the stream-serialisation attribute may start once every CTA
+// of the kernel in front of it has passed `pdl_launch_dependents`; what does not need that kernel's output then overlaps it.
+// `pdl_wait` returns once that kernel has completed and its writes are visible; without the launch attribute both
+// instructions do nothing.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------------
 // mbarrier + bulk async copies (non-multicast, 1-D). Addresses and sizes must be
 // multiples of 16 bytes; callers check and take a plain-load path otherwise.

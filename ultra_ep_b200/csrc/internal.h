@@ -151,12 +151,16 @@ struct Batch {
 };
 int64_t dense_scratch_elems(int T, int L);
 int64_t sparse_scratch_elems(int64_t entries, int L);
+// behind_plan: the plan kernel may be the one in front of it in the stream, and its end is not waited for before the tokens
+// are counted (a kernel, a copy or an event wait in between is waited for). Eight ranks, plan and reroute: 33 tokens of 64
+// experts 20.6 -> 16.8 us, 4096 tokens 30.2 -> 27.5. Not beside a weight_sync: the reroute then runs while weight_sync's CTAs
+// read their tables (16384 tokens of 256 experts, fp8 weights: 119 -> 128 us; 8192 bool rows of 128, bf16 68.6 -> 71.3).
 cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int D, int quota_mode, int interleave,
-                                 cudaStream_t stream);
+                                 bool behind_plan, cudaStream_t stream);
 cudaError_t launch_dense_backward(const Batch<DenseBwdArgs>& b, int L, int P, int D, cudaStream_t stream);
 // beside_sync: a weight_sync was launched beside it
 cudaError_t launch_sparse_reroute(const Batch<SparseArgs>& b, int ids_kind, int K, int L, int D, int interleave, bool beside_sync,
-                                  cudaStream_t stream);
+                                  bool behind_plan, cudaStream_t stream);
 
 int device_sm_count();  // of the current device; launch sizes are multiples of it
 // Lets a kernel use that much dynamic shared memory on the current device (and, once, ask for the largest carve-out).

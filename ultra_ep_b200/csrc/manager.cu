@@ -774,7 +774,8 @@ int uep_reroute_dense_forward(uep_manager* m, int layer_id, const uint8_t* const
                               expanded_maps[i], expanded_probs[i], T[i]};
     }
     // legacy placement has no quotas: its reroute is round-robin over an expert's instances
-    UEP_CUDA_TRY(launch_dense_forward(b, m->L, m->P, m->D, m->cfg.legacy_placement ? 0 : 1, m->cfg.solver.reroute_interleave, stream));
+    UEP_CUDA_TRY(launch_dense_forward(b, m->L, m->P, m->D, m->cfg.legacy_placement ? 0 : 1, m->cfg.solver.reroute_interleave,
+                                      m->sync_beside[plan_slot(m, layer_id)] == 0, stream));
     return UEP_OK;
 }
 
@@ -816,8 +817,9 @@ int uep_reroute_sparse(uep_manager* m, int layer_id, int ids_kind, const void* c
         const PlanPtrs p = plan_ptrs(m, m->ranks[i], layer_id);
         b.a[i] = SparseArgs{ids[i], out[i], p.l2p, p.lcnts, p.rank_quota_prefix, m->ranks[i].scratch[1], T[i]};
     }
+    const bool beside_sync = m->sync_beside[plan_slot(m, layer_id)] != 0;
     UEP_CUDA_TRY(launch_sparse_reroute(b, ids_kind, K, m->L, m->D, m->cfg.legacy_placement ? 2 : m->cfg.solver.reroute_interleave,
-                                       m->sync_beside[plan_slot(m, layer_id)] != 0, stream));
+                                       beside_sync, !beside_sync, stream));
     return UEP_OK;
 }
 

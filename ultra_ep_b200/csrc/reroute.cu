@@ -200,7 +200,7 @@ __device__ __forceinline__ bool dense_fast_path(const uint8_t* map, const void* 
            ((reinterpret_cast<uintptr_t>(map) | reinterpret_cast<uintptr_t>(scratch)) & 15u) == 0;
 }
 
-__global__ void __launch_bounds__(kRerouteThreads) dense_count_kernel(Batch<DenseFwdArgs> batch, int L) {
+__global__ void __launch_bounds__(kRerouteThreads) dense_count_kernel(Batch<DenseFwdArgs> batch, int L, int behind_plan) {
     pdl_launch_dependents();  // the scatter kernel may start its prologue now
     extern __shared__ __align__(128) char smem_raw[];  // [pad4(L)] counts, one byte each
     const DenseFwdArgs& a = batch.a[blockIdx.y];
@@ -208,6 +208,7 @@ __global__ void __launch_bounds__(kRerouteThreads) dense_count_kernel(Batch<Dens
     const int tile = blockIdx.x;
     const int r0 = tile * kDenseTileRows, r1 = min(r0 + kDenseTileRows, T);
     if (r0 >= T) return;
+    const bool holds = behind_plan && tile == 0;  // this grid ends behind the plan's: its first tiles see to it
     uint8_t* counts = reinterpret_cast<uint8_t*>(a.scratch) + static_cast<int64_t>(tile) * L;
     const uint8_t* src = a.map + static_cast<int64_t>(r0) * L;
     uint32_t* cnt = reinterpret_cast<uint32_t*>(smem_raw);
@@ -237,6 +238,7 @@ __global__ void __launch_bounds__(kRerouteThreads) dense_count_kernel(Batch<Dens
         }
         __syncthreads();
         for (int i = threadIdx.x; i < L / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(counts)[i] = cnt[i];
+        if (holds) pdl_wait();
         return;
     }
     const int quads = pad4(L) / 4;
@@ -251,6 +253,7 @@ __global__ void __launch_bounds__(kRerouteThreads) dense_count_kernel(Batch<Dens
     }
     __syncthreads();
     for (int e = threadIdx.x; e < L; e += blockDim.x) counts[e] = reinterpret_cast<const uint8_t*>(cnt)[e];
+    if (holds) pdl_wait();
 }
 
 // Adds the counts of the tiles in front of `tile` to base_of[L] (shared memory, zeroed), all threads of the CTA.
@@ -737,10 +740,11 @@ __global__ void __launch_bounds__(kRerouteThreads) dense_backward_kernel(Batch<D
 
 // ---------------------------------------------------------------------------- sparse
 template <typename IdT>
-__global__ void __launch_bounds__(kOrdThreads) sparse_count_kernel(Batch<SparseArgs> batch, int K, int L, int tile_entries) {
+__global__ void __launch_bounds__(kOrdThreads) sparse_count_kernel(Batch<SparseArgs> batch, int K, int L, int tile_entries, int behind_plan) {
     pdl_launch_dependents();  // the reroute kernel may start on everything that does not read the table
     const SparseArgs& a = batch.a[blockIdx.y];
     count_tile<IdT>(static_cast<const IdT*>(a.ids), static_cast<int64_t>(a.T) * K, L, false, tile_entries, a.scratch);
+    if (behind_plan && blockIdx.x == 0) pdl_wait();  // this grid ends behind the plan's
 }
 
 // shared memory: prefix rows [L][8] i32 | l2p rows [L][8] i32 (both only where they fit) | ordinals | routers[L]
@@ -753,7 +757,7 @@ size_t sparse_smem_bytes(int L, bool rows_staged) {
 // CTA occupies.
 template <int EPT, typename IdT>
 __global__ void __launch_bounds__(kOrdThreads) __maxnreg__(EPT > 4 ? 96 : 64)
-sparse_reroute_kernel(Batch<SparseArgs> batch, int ctas, int K, int L, int D, int interleave, int rows_staged, int use_table) {
+sparse_reroute_kernel(Batch<SparseArgs> batch, int ctas, int K, int L, int D, int interleave, int rows_staged, int use_table, int behind_plan) {
     extern __shared__ __align__(128) char smem_raw[];
     const SparseArgs& a = batch.a[blockIdx.y];
     const IdT* ids = static_cast<const IdT*>(a.ids);
@@ -766,13 +770,18 @@ sparse_reroute_kernel(Batch<SparseArgs> batch, int ctas, int K, int L, int D, in
     const OrdShared o = carve_ord_smem(rows_staged ? reinterpret_cast<char*>(l2p_s + static_cast<size_t>(L) * kStagedReps) : smem_raw, L);
     FastRouter* routers = reinterpret_cast<FastRouter*>(o.counters + kOrdWarps * ord_row(L));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (rows_staged) stage_plan_rows_async(a.lcnts, a.rqp, a.l2p, L, D, quota_mode, routers, prefix_s, l2p_s);
+    if (rows_staged && !behind_plan) stage_plan_rows_async(a.lcnts, a.rqp, a.l2p, L, D, quota_mode, routers, prefix_s, l2p_s);
 
     int64_t begin, end;
     int iters;
     uint32_t packed[EPT];
     cluster_ordinals<EPT, false, IdT>(
         ids, n, L, false, ctas, use_table ? a.scratch : nullptr, o, begin, end, iters, packed,
+        [&]() {
+            if (!behind_plan) return;
+            pdl_wait();  // the entries are counted: from here on it needs the plan
+            if (rows_staged) stage_plan_rows_async(a.lcnts, a.rqp, a.l2p, L, D, quota_mode, routers, prefix_s, l2p_s);
+        },
         [&]() {
             for (int e = tid; e < L; e += kOrdThreads) {
                 const int C = rows_staged ? routers[e].C : a.lcnts[e];
@@ -814,7 +823,7 @@ __host__ __device__ __forceinline__ size_t walk_smem_bytes(int L) {
     return static_cast<size_t>(L) * (2 * kStagedReps * 4 + sizeof(FastRouter) + 4 + kWalkWarps * 4);
 }
 template <typename IdT>
-__global__ void __launch_bounds__(kWalkThreads) sparse_walk_count_kernel(Batch<SparseArgs> batch, int K, int L) {
+__global__ void __launch_bounds__(kWalkThreads) sparse_walk_count_kernel(Batch<SparseArgs> batch, int K, int L, int behind_plan) {
     extern __shared__ __align__(128) char smem_raw[];
     const SparseArgs& a = batch.a[blockIdx.y];
     const IdT* keys = static_cast<const IdT*>(a.ids);
@@ -831,6 +840,7 @@ __global__ void __launch_bounds__(kWalkThreads) sparse_walk_count_kernel(Batch<S
     }
     __syncthreads();
     for (int i = threadIdx.x; i < L; i += blockDim.x) a.scratch[static_cast<int64_t>(blockIdx.x) * L + i] = hist[i];
+    if (behind_plan && blockIdx.x == 0) pdl_wait();  // this grid ends behind the plan's
 }
 
 template <typename IdT>
@@ -934,6 +944,7 @@ template <int EPT>
 __global__ void __launch_bounds__(kOrdThreads) __maxnreg__(EPT > 4 ? 128 : 80)
 dispatch_positions_kernel(const int32_t* phys, int64_t n, int ctas, int P, const int32_t* __restrict__ table, int32_t* pos,
                           int32_t* __restrict__ expert_offsets) {
+    pdl_launch_dependents();  // the gather behind it may set itself up
     extern __shared__ __align__(128) char smem_raw[];
     __shared__ int warp_tot[kOrdWarps];
     const int nb = P + 1;
@@ -944,7 +955,7 @@ dispatch_positions_kernel(const int32_t* phys, int64_t n, int ctas, int P, const
     int iters;
     uint32_t packed[EPT];
     cluster_ordinals<EPT, true, int32_t>(
-        phys, n, P, true, ctas, table, o, begin, end, iters, packed, []() {},
+        phys, n, P, true, ctas, table, o, begin, end, iters, packed, []() {}, []() {},
         [&](int b, int base, int all) {
             o.base[b] = base;
             all_of[b] = all;
@@ -1043,7 +1054,7 @@ __global__ void __launch_bounds__(32) gather_rows_kernel(const uint8_t* __restri
                 const int64_t item = first + k * step;
                 row = whole ? (item << shift) + (i & (rows_per_item - 1)) : item / chunks_per_row;
             }
-            p[u] = row < num_rows ? __ldg(pos + row) : 0;
+            p[u] = row < num_rows ? __ldcg(pos + row) : 0;
         }
     };
     auto keep = [&](int batch, const int32_t (&p)[kGatherBatch / 32]) {
@@ -1076,6 +1087,7 @@ __global__ void __launch_bounds__(32) gather_rows_kernel(const uint8_t* __restri
     };
 
     int32_t ahead[kGatherBatch / 32];
+    pdl_wait();  // the positions may be the output of the kernel in front
     fetch(0, ahead);
     keep(0, ahead);
     __syncwarp();
@@ -1181,7 +1193,7 @@ cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, s
 }
 
 cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int D, int quota_mode, int interleave,
-                                 cudaStream_t stream) {
+                                 bool behind_plan, cudaStream_t stream) {
     int max_T = 0;
     for (int i = 0; i < b.n; ++i) max_T = b.a[i].T > max_T ? b.a[i].T : max_T;
     if (max_T == 0) return cudaSuccess;
@@ -1195,8 +1207,10 @@ cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int
     e = ensure_smem_attr(reinterpret_cast<const void*>(dense_count_kernel), smem_count);
     if (e != cudaSuccess) return e;
     count_launch(2);
-    dense_count_kernel<<<grid, kRerouteThreads, smem_count, stream>>>(b, L);
-    e = cudaGetLastError();
+    // Behind the plan of several ranks the count does not wait for it. (The scatter kernel of one rank starts with the count
+    // and reads plan rows at once, so there the count must be behind the plan.)
+    behind_plan = behind_plan && b.n > 1 && pdl_enabled();
+    e = launch_dependent(dense_count_kernel, grid, dim3(kRerouteThreads), smem_count, stream, behind_plan, b, L, behind_plan ? 1 : 0);
     if (e != cudaSuccess) return e;
     // With one rank per launch the pair is latency-bound and the overlap pays; a launch that hosts several ranks
     // fills the device with the first kernel alone, and early CTAs of the second only get in its way.
@@ -1340,7 +1354,8 @@ bool walk_pays(int64_t n, int L, bool beside_sync) {
 
 template <typename IdT>
 static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L, int D, int interleave, bool beside_sync,
-                                       cudaStream_t stream) {
+                                       bool behind_plan, cudaStream_t stream) {
+    behind_plan = behind_plan && pdl_enabled();
     int64_t max_n = 0;
     bool in_place = false;
     for (int i = 0; i < b.n; ++i) {
@@ -1358,8 +1373,8 @@ static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L,
         e = ensure_smem_attr(reinterpret_cast<const void*>(sparse_walk_kernel<IdT>), walk_smem_bytes(L));
         if (e != cudaSuccess) return e;
         count_launch(2);
-        sparse_walk_count_kernel<IdT><<<grid, kWalkThreads, sizeof(int32_t) * L, stream>>>(b, K, L);
-        e = cudaGetLastError();
+        e = launch_dependent(sparse_walk_count_kernel<IdT>, grid, dim3(kWalkThreads), sizeof(int32_t) * L, stream, behind_plan, b, K, L,
+                             behind_plan ? 1 : 0);
         if (e != cudaSuccess) return e;
         sparse_walk_kernel<IdT><<<grid, kWalkThreads, walk_smem_bytes(L), stream>>>(b, K, L, D, interleave);
         return cudaGetLastError();
@@ -1374,20 +1389,23 @@ static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L,
         cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(sparse_count_kernel<IdT>), sizeof(int32_t) * L);
         if (e != cudaSuccess) return e;
         count_launch();
-        sparse_count_kernel<IdT><<<dim3(g.ctas * g.clusters, b.n), kOrdThreads, sizeof(int32_t) * L, stream>>>(b, K, L, g.per_lane * kOrdThreads);
-        e = cudaGetLastError();
+        // (of one rank: the reroute kernel starts with the count and reads plan rows at once)
+        const bool early = behind_plan && b.n > 1;
+        e = launch_dependent(sparse_count_kernel<IdT>, dim3(g.ctas * g.clusters, b.n), dim3(kOrdThreads), sizeof(int32_t) * L, stream, early, b,
+                             K, L, g.per_lane * kOrdThreads, early ? 1 : 0);
         if (e != cudaSuccess) return e;
     }
     return with_lanes(g, [&](auto per_lane) {
-        return launch_clusters(sparse_reroute_kernel<decltype(per_lane)::value, IdT>, g, b.n, smem, stream, overlap, b, g.ctas, K, L, D,
-                               interleave, staged, g.table ? 1 : 0);
+        const bool early = behind_plan && !g.table;
+        return launch_clusters(sparse_reroute_kernel<decltype(per_lane)::value, IdT>, g, b.n, smem, stream, overlap || early, b, g.ctas, K, L, D,
+                               interleave, staged, g.table ? 1 : 0, early ? 1 : 0);
     });
 }
 
 cudaError_t launch_sparse_reroute(const Batch<SparseArgs>& b, int ids_kind, int K, int L, int D, int interleave, bool beside_sync,
-                                  cudaStream_t stream) {
-    if (ids_kind == 2) return launch_sparse_typed<long long>(b, K, L, D, interleave, beside_sync, stream);
-    return launch_sparse_typed<int32_t>(b, K, L, D, interleave, beside_sync, stream);
+                                  bool behind_plan, cudaStream_t stream) {
+    if (ids_kind == 2) return launch_sparse_typed<long long>(b, K, L, D, interleave, beside_sync, behind_plan, stream);
+    return launch_sparse_typed<int32_t>(b, K, L, D, interleave, beside_sync, behind_plan, stream);
 }
 
 }  // namespace uep
@@ -1414,7 +1432,7 @@ int uep_dense_reroute_forward(const uint8_t* routing_map, const float* probs, co
     Batch<DenseFwdArgs> b{};
     b.n = 1;
     b.a[0] = DenseFwdArgs{routing_map, probs, l2p, lcnts, rank_quota_prefix, scratch, expanded_map, expanded_probs, T};
-    UEP_CUDA_TRY(launch_dense_forward(b, L, P, D, quota_mode, interleave, static_cast<cudaStream_t>(stream_)));
+    UEP_CUDA_TRY(launch_dense_forward(b, L, P, D, quota_mode, interleave, false, static_cast<cudaStream_t>(stream_)));
     return UEP_OK;
 }
 
@@ -1447,7 +1465,7 @@ static int sparse_common(int kind, const void* ids, void* out, int T, int K, int
     Batch<SparseArgs> b{};
     b.n = 1;
     b.a[0] = SparseArgs{ids, out, l2p, lcnts, rqp, scratch, T};
-    UEP_CUDA_TRY(launch_sparse_reroute(b, kind, K, L, D, interleave, false, static_cast<cudaStream_t>(stream_)));
+    UEP_CUDA_TRY(launch_sparse_reroute(b, kind, K, L, D, interleave, false, false, static_cast<cudaStream_t>(stream_)));
     return UEP_OK;
 }
 
@@ -1571,9 +1589,9 @@ int uep_gather_rows(const void* in, const int32_t* pos, void* out, int64_t num_r
         while (rows < 32 && 2 * rows * row_bytes <= kGatherChunk && num_rows >= 8 * rows * 2 * sms) rows *= 2;
         int64_t ctas = chunks > 1 ? num_rows * chunks : (num_rows + rows - 1) / rows;
         if (ctas > 2 * sms) ctas = 2 * sms;  // two CTAs of one warp per SM
-        gather_rows_kernel<<<static_cast<int>(ctas), 32, smem, stream>>>(
-            static_cast<const uint8_t*>(in), pos, static_cast<uint8_t*>(out), num_rows, row_bytes, rows, chunks,
-            num_src_rows, 2000000000ull, st);
+        UEP_CUDA_TRY(launch_dependent(gather_rows_kernel, dim3(static_cast<unsigned>(ctas)), dim3(32), smem, stream, true,
+                                      static_cast<const uint8_t*>(in), pos, static_cast<uint8_t*>(out), num_rows, row_bytes, rows, chunks,
+                                      num_src_rows, static_cast<uint64_t>(2000000000ull), st));
     } else {
         const int64_t sms = device_sm_count() > 0 ? device_sm_count() : 1;
         int64_t ctas = num_rows > sms * 8 ? sms * 8 : num_rows;
