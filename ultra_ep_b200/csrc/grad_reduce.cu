@@ -291,10 +291,12 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
     };
     auto master_ptr = [&](const ReduceItem& it) -> float* { return sm.master[it.active][it.shard] + it.offset; };
 
-    auto clear_tile = [&](float* dst, int elems) {  // one thread, 16-byte aligned
+    // one thread, 16-byte aligned; the zeros are not read again for long (82.1 us -> 80.7, 278.9 -> 275.2 with the two sizes above)
+    auto clear_tile = [&](float* dst, int elems) {
+        const uint64_t policy = l2_first();
         const uint32_t bytes = static_cast<uint32_t>(elems) * 4u;
         for (uint32_t o = 0; o < bytes; o += kReduceZeroBytes) {
-            bulk_store(reinterpret_cast<char*>(dst) + o, zero_tile, bytes - o < kReduceZeroBytes ? bytes - o : kReduceZeroBytes);
+            bulk_store(reinterpret_cast<char*>(dst) + o, zero_tile, bytes - o < kReduceZeroBytes ? bytes - o : kReduceZeroBytes, policy);
         }
         bulk_commit();
     };
