@@ -153,7 +153,7 @@ int64_t dense_scratch_elems(int T, int L);
 int64_t sparse_scratch_elems(int64_t entries, int L);
 // behind_plan: the plan kernel may be the one in front of it in the stream, and its end is not waited for before the tokens
 // are counted (a kernel, a copy or an event wait in between is waited for). Eight ranks, plan and reroute: 33 tokens of 64
-// experts 20.6 -> 16.8 us, 4096 tokens 30.2 -> 27.5. Not beside a weight_sync: the reroute then runs while weight_sync's CTAs
+// experts 20.6 -> 16.8 us, 4096 tokens 30.2 -> 24.7 (27.2 with the count alone started early). Not beside a weight_sync: the reroute then runs while weight_sync's CTAs
 // read their tables (16384 tokens of 256 experts, fp8 weights: 119 -> 128 us; 8192 bool rows of 128, bf16 68.6 -> 71.3).
 cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int D, int quota_mode, int interleave,
                                  bool behind_plan, cudaStream_t stream);

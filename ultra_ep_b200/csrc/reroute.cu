@@ -453,6 +453,9 @@ __device__ __forceinline__ void write_dense_chunk(const DenseShared& s, const fl
     }
 }
 
+// kBehindPlan: the plan may still be being made when it starts. A kernel of its own: with the choice made inside, the step
+// beside weight_sync was 2 us longer (68.1 and 70.0).
+template <bool kBehindPlan>
 __global__ void __launch_bounds__(kDenseMaxThreads, 2)
 dense_scatter_kernel(Batch<DenseFwdArgs> batch, int L, int P, int D, int quota_mode, int interleave, int chunk_cols,
                      int overlapped) {
@@ -467,11 +470,15 @@ dense_scatter_kernel(Batch<DenseFwdArgs> batch, int L, int P, int D, int quota_m
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, Lq = pad4(L);
 
     // ---- nothing here depends on the count kernel ------------------------------------------------
-    stage_plan_rows_async(a.lcnts, a.rqp, a.l2p, L, D, quota_mode != 0, s.routers, s.prefix, s.l2p);
+    if (!kBehindPlan) stage_plan_rows_async(a.lcnts, a.rqp, a.l2p, L, D, quota_mode != 0, s.routers, s.prefix, s.l2p);
     for (int e = tid; e < L; e += blockDim.x) s.base[e] = 0;
     for (int i = tid; i < pad4(chunk_cols) / 4 * kDenseSegs; i += blockDim.x) reinterpret_cast<uint32_t*>(s.phys_bits)[i] = 0;
     if (tid == 0) n_several = 0;
     tile_bit_columns(a.map + static_cast<int64_t>(r0) * L, rows, kDenseSegs, L, s.bits);
+    if (kBehindPlan) {
+        pdl_wait();
+        stage_plan_rows_async(a.lcnts, a.rqp, a.l2p, L, D, quota_mode != 0, s.routers, s.prefix, s.l2p);
+    }
     cp_async_wait();
     __syncthreads();
     for (int e = tid; e < L; e += blockDim.x) {
@@ -484,7 +491,7 @@ dense_scatter_kernel(Batch<DenseFwdArgs> batch, int L, int P, int D, int quota_m
             if (any) s.several[atomicAdd(&n_several, 1)] = static_cast<uint16_t>(e);
         }
     }
-    if (overlapped) pdl_wait();
+    if (!kBehindPlan && overlapped) pdl_wait();
     sum_earlier_tiles(a, L, tile, s.base);
     __syncthreads();
 
@@ -1205,23 +1212,23 @@ cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int
     const dim3 grid(dense_tiles(max_T), b.n);
     const int chunk = P > kDenseMaxChunkCols ? kDenseMaxChunkCols : P;
     const size_t smem_count = pad4(L), smem = dense_smem_bytes(L, chunk);
-    cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(dense_scatter_kernel), smem);
+    behind_plan = behind_plan && pdl_enabled();  // both kernels start while the plan is made
+    const auto scatter = behind_plan ? dense_scatter_kernel<true> : dense_scatter_kernel<false>;
+    cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(scatter), smem);
     if (e != cudaSuccess) return e;
     e = ensure_smem_attr(reinterpret_cast<const void*>(dense_count_kernel), smem_count);
     if (e != cudaSuccess) return e;
     count_launch(2);
-    // Behind the plan of several ranks the count does not wait for it. (The scatter kernel of one rank starts with the count
-    // and reads plan rows at once, so there the count must be behind the plan.)
-    behind_plan = behind_plan && b.n > 1 && pdl_enabled();
     e = launch_dependent(dense_count_kernel, grid, dim3(kRerouteThreads), smem_count, stream, behind_plan, b, L, behind_plan ? 1 : 0);
     if (e != cudaSuccess) return e;
     // With one rank per launch the pair is latency-bound and the overlap pays; a launch that hosts several ranks
-    // fills the device with the first kernel alone, and early CTAs of the second only get in its way.
-    const bool overlap = b.n == 1 && pdl_enabled();
+    // fills the device with the first kernel alone, and early CTAs of the second only get in its way, unless both start while
+    // the plan is made.
+    const bool overlap = (b.n == 1 || behind_plan) && pdl_enabled();
     // up to two tiles per SM the kernel is a chain of phases: more threads shorten each
     const int sms = std::max(device_sm_count(), 1);
     const int threads = static_cast<int64_t>(grid.x) * b.n <= 2 * sms ? kDenseMaxThreads : kRerouteThreads;
-    return launch_dependent(dense_scatter_kernel, grid, dim3(threads), smem, stream, overlap, b, L, P, D, quota_mode,
+    return launch_dependent(scatter, grid, dim3(threads), smem, stream, overlap, b, L, P, D, quota_mode,
                             interleave, chunk, overlap ? 1 : 0);
 }
 
@@ -1386,22 +1393,19 @@ static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L,
     const size_t smem = sparse_smem_bytes(L, staged != 0);
     const OrdGrid g = ord_grid(max_n, L, b.n, in_place, kOrdThreads, false);
     // One rank per launch is latency-bound and the overlap with the count kernel pays; several ranks fill the device
-    // with the first kernel alone.
-    const bool overlap = g.table && b.n == 1 && pdl_enabled();
+    // with the first kernel alone, unless both start while the plan is made.
+    const bool overlap = behind_plan || (g.table && b.n == 1 && pdl_enabled());
     if (g.table) {
         cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(sparse_count_kernel<IdT>), sizeof(int32_t) * L);
         if (e != cudaSuccess) return e;
         count_launch();
-        // (of one rank: the reroute kernel starts with the count and reads plan rows at once)
-        const bool early = behind_plan && b.n > 1;
-        e = launch_dependent(sparse_count_kernel<IdT>, dim3(g.ctas * g.clusters, b.n), dim3(kOrdThreads), sizeof(int32_t) * L, stream, early, b,
-                             K, L, g.per_lane * kOrdThreads, early ? 1 : 0);
+        e = launch_dependent(sparse_count_kernel<IdT>, dim3(g.ctas * g.clusters, b.n), dim3(kOrdThreads), sizeof(int32_t) * L, stream, behind_plan, b,
+                             K, L, g.per_lane * kOrdThreads, behind_plan ? 1 : 0);
         if (e != cudaSuccess) return e;
     }
     return with_lanes(g, [&](auto per_lane) {
-        const bool early = behind_plan && !g.table;
-        return launch_clusters(sparse_reroute_kernel<decltype(per_lane)::value, IdT>, g, b.n, smem, stream, overlap || early, b, g.ctas, K, L, D,
-                               interleave, staged, g.table ? 1 : 0, early ? 1 : 0);
+        return launch_clusters(sparse_reroute_kernel<decltype(per_lane)::value, IdT>, g, b.n, smem, stream, overlap, b, g.ctas, K, L, D,
+                               interleave, staged, g.table ? 1 : 0, behind_plan ? 1 : 0);
     });
 }
 
