@@ -1,11 +1,14 @@
-"""The reroute may count its tokens while the plan in front of it in the stream is still being made. It must use that plan all the
-same, and the ids as the stream leaves them: eager, behind a kernel or another stream's event in between, and replayed as a graph."""
+"""The reroute may be on its SMs while the plan in front of it in the stream is still being made. It must use that plan all the
+same, and the ids or maps as the stream leaves them: eager, behind a kernel or another stream's event in between, and replayed as
+a graph. A kernel in between may itself start its dependents early."""
+
+import ctypes as C
 
 import pytest
 import torch
 
 import gpu_util as G
-from ultra_ep_b200 import sim
+from ultra_ep_b200 import capi, sim
 
 pytestmark = pytest.mark.gpu
 
@@ -128,3 +131,197 @@ def test_gather_behind_positions(native_lib, cuda_device):
         torch.cuda.synchronize()
         assert not status.any()
         assert torch.equal(out, rows[pos.long()])
+
+
+# Lets its dependents start at once, waits for what it depends on itself, and writes its bytes 30 us later (at most 2^16 looks at
+# the clock).
+LATE_WRITER = r"""
+extern "C" __global__ void late_writer(unsigned char* dst, const unsigned char* src, long long bytes) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    unsigned long long begin, now;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(begin));
+    for (int i = 0; i < 65536; ++i) {
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+        if (now - begin > 30000) break;
+    }
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < bytes; i += (long long)gridDim.x * blockDim.x) dst[i] = src[i];
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def late_write():
+    """late_write(dst, src, dependent): on the current stream, as an ordinary launch or as a programmatic dependent one."""
+    from cuda.bindings import driver, nvrtc
+
+    def ok(result):
+        assert int(result[0]) == 0, result[0]
+        return result[1] if len(result) == 2 else result[1:]
+
+    torch.cuda.synchronize()  # the context is there
+    program = ok(nvrtc.nvrtcCreateProgram(LATE_WRITER.encode(), b"late_writer.cu", 0, [], []))
+    ok(nvrtc.nvrtcCompileProgram(program, 1, [b"--gpu-architecture=sm_100a"]))
+    image = b" " * ok(nvrtc.nvrtcGetCUBINSize(program))
+    ok(nvrtc.nvrtcGetCUBIN(program, image))
+    module = ok(driver.cuModuleLoadData(image))
+    kernel = ok(driver.cuModuleGetFunction(module, b"late_writer"))
+
+    def launch(dst, src, dependent):
+        assert dst.is_contiguous() and src.is_contiguous() and dst.nbytes == src.nbytes
+        config = driver.CUlaunchConfig()
+        config.gridDimX, config.gridDimY, config.gridDimZ = 16, 1, 1
+        config.blockDimX, config.blockDimY, config.blockDimZ = 256, 1, 1
+        config.hStream = driver.CUstream(torch.cuda.current_stream().cuda_stream)
+        attribute = driver.CUlaunchAttribute()
+        attribute.id = driver.CUlaunchAttributeID.CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION
+        attribute.value.programmaticStreamSerializationAllowed = 1
+        config.attrs, config.numAttrs = ([attribute], 1) if dependent else ([], 0)
+        values = (dst.data_ptr(), src.data_ptr(), dst.nbytes)
+        ok(driver.cuLaunchKernelEx(config, kernel, (values, (C.c_void_p, C.c_void_p, C.c_longlong)), 0))
+
+    yield launch
+    torch.cuda.synchronize()
+    ok(driver.cuModuleUnload(module))
+
+
+def _flat(parts):
+    """One buffer behind all ranks' tensors (one of them empty), and the ranks' views of it."""
+    flat = torch.cat([x.reshape(-1) for x in parts])
+    views, at = [], 0
+    for x in parts:
+        views.append(flat[at:at + x.numel()].view(x.shape))
+        at += x.numel()
+    return flat, views
+
+
+def _ranks_draw(ranks, tokens, dtype, seed, device):
+    parts = _draw(tokens, dtype, seed, device)[:ranks]
+    if ranks > 3:
+        parts[3] = parts[3][:0].contiguous()  # a rank without tokens
+    return parts
+
+
+# eight ranks: one launch, a count kernel in front, the walk; one rank: the same without the walk
+@pytest.mark.parametrize("ranks,tokens", [(RANKS, 33), (RANKS, 4099), (RANKS, 9000), (1, 33), (1, 4099), (1, 40000)])
+@pytest.mark.parametrize("dependent", [False, True])
+def test_sparse_behind_an_early_kernel(native_lib, cuda_device, late_write, ranks, tokens, dependent):
+    group = sim.SimGroup(sim.make_config(ranks, L // ranks, 2, 1, is_train=False, sim=True))
+    for seed in range(4):
+        flat, ids = _flat(_ranks_draw(ranks, tokens, torch.int32, seed, cuda_device))
+        late_flat, late = _flat(_ranks_draw(ranks, tokens, torch.int32, seed + 50, cuda_device))
+        group.update_placement(0, ids)
+        late_write(flat, late_flat, dependent)
+        got = group.reroute_sparse(0, ids)
+        for r, (a, b) in enumerate(zip(got, _expect_of(group, late))):
+            assert torch.equal(a, b), (seed, r)
+        torch.cuda.synchronize()
+        late_write(flat, late_flat.flip(0).contiguous(), dependent)  # the kept plan again
+        got = group.reroute_sparse(0, ids)
+        for r, (a, b) in enumerate(zip(got, _expect_of(group, [x.clone() for x in ids]))):
+            assert torch.equal(a, b), (seed, r)
+    group.destroy()
+
+
+@pytest.mark.parametrize("ranks,tokens", [(RANKS, 65), (RANKS, 3000), (1, 65), (1, 9000)])
+@pytest.mark.parametrize("between", ["late", "late dependent", "copy", "event", "nothing"])
+def test_dense_maps_change_behind_the_plan(native_lib, cuda_device, late_write, ranks, tokens, between):
+    group = sim.SimGroup(sim.make_config(ranks, L // ranks, 2, 1, is_train=True, sim=True))
+    other = torch.cuda.Stream()
+    to_map = lambda x: torch.zeros((x.shape[0], L), dtype=torch.bool, device=cuda_device).scatter_(1, x, True)
+    for seed in range(4):
+        flat, maps = _flat([to_map(x) for x in _ranks_draw(ranks, tokens, torch.int64, seed, cuda_device)])
+        late_flat, late = _flat([to_map(x) for x in _ranks_draw(ranks, tokens, torch.int64, seed + 50, cuda_device)])
+        probs = [torch.rand(m.shape, device=cuda_device) for m in maps]
+        torch.cuda.synchronize()
+        group.update_placement(0, maps)
+        if between.startswith("late"):
+            late_write(flat, late_flat, between.endswith("dependent"))
+        elif between == "copy":
+            flat.copy_(late_flat)
+        elif between == "event":
+            with torch.cuda.stream(other):
+                other.wait_stream(torch.cuda.current_stream())
+                torch.cuda._sleep(200_000)
+                flat.copy_(late_flat)
+            torch.cuda.current_stream().wait_stream(other)
+        got_probs, got_maps = group.reroute_dense(0, maps, probs)
+        want = maps if between == "nothing" else late
+        _check_dense(group, want, probs, got_probs, got_maps, seed)
+    group.destroy()
+
+
+def test_dense_replayed(native_lib, cuda_device):
+    group = sim.SimGroup(sim.make_config(RANKS, L // RANKS, 2, 1, is_train=True, sim=True))
+    to_map = lambda x: torch.zeros((x.shape[0], L), dtype=torch.bool, device=cuda_device).scatter_(1, x, True)
+    draw = lambda seed: _flat([to_map(x) for x in _ranks_draw(RANKS, 700, torch.int64, seed, cuda_device)])
+    flat, maps = draw(0)
+    next_flat = flat.clone()
+    probs = [torch.rand(m.shape, device=cuda_device) for m in maps]
+
+    def step():
+        group.update_placement(0, maps)
+        flat.copy_(next_flat)
+        return group.reroute_dense(0, maps, probs)
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        step()  # sizes the scratch
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got_probs, got_maps = step()
+    for seed in range(1, 5):
+        next_flat.copy_(draw(seed)[0])
+        graph.replay()
+        graph.replay()
+        _check_dense(group, maps, probs, got_probs, got_maps, seed)
+    group.destroy()
+
+
+def _expect_of(group, ids):
+    torch.cuda.synchronize()
+    group.check_status()
+    out = []
+    for r, x in enumerate(ids):
+        p = group.plan(r, 0)
+        out.append(G.cuda_sparse_reroute(x, p["l2p"].contiguous(), p["lcnts"].contiguous(), p["rank_quota_prefix"].contiguous())
+                   if x.numel() else x)
+    return out
+
+
+def _check_dense(group, maps, probs, got_probs, got_maps, what):
+    torch.cuda.synchronize()
+    group.check_status()
+    for r, m in enumerate(maps):
+        if m.numel() == 0:
+            assert got_probs[r].numel() == 0 and got_maps[r].numel() == 0
+            continue
+        p = group.plan(r, 0)
+        want_probs, want_map = G.cuda_dense_reroute(m, probs[r], p["l2p"].contiguous(), p["lcnts"].contiguous(),
+                                                    p["rank_quota_prefix"].contiguous(), group.P)
+        assert torch.equal(got_probs[r], want_probs) and torch.equal(got_maps[r], want_map), (what, r)
+
+
+# in one launch, in two (n > 2^18), and in place
+@pytest.mark.parametrize("n", [4096, 262145, 300001])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_gather_behind_positions_of_many(native_lib, cuda_device, n, in_place):
+    gen = torch.Generator(device=cuda_device).manual_seed(n)
+    rows = torch.randn((n, 8), generator=gen, device=cuda_device)
+    phys = torch.randint(-1, 80, (n,), generator=gen, device=cuda_device, dtype=torch.int32)
+    want = torch.empty_like(phys)
+    keys = torch.where(phys < 0, 80, phys)
+    want[torch.argsort(keys, stable=True)] = torch.arange(n, dtype=torch.int32, device=cuda_device)
+    lib = capi.lib()
+    pos = phys if in_place else torch.empty_like(phys)
+    scratch = torch.empty(lib.uep_dispatch_scratch_elems(n, 80), dtype=torch.int32, device=cuda_device)
+    out = torch.empty_like(rows)
+    status = torch.zeros(2, dtype=torch.int32, device=cuda_device)
+    torch.cuda.synchronize()
+    capi.check(lib.uep_dispatch_positions(phys.data_ptr(), n, 80, pos.data_ptr(), None, scratch.data_ptr(), G.stream_ptr()))
+    capi.check(lib.uep_gather_rows(rows.data_ptr(), pos.data_ptr(), out.data_ptr(), n, n, 32, status.data_ptr(), G.stream_ptr()))
+    torch.cuda.synchronize()
+    assert not status.any()
+    assert torch.equal(pos, want) and torch.equal(out, rows[want.long()])

@@ -151,10 +151,13 @@ struct Batch {
 };
 int64_t dense_scratch_elems(int T, int L);
 int64_t sparse_scratch_elems(int64_t entries, int L);
-// behind_plan: the plan kernel may be the one in front of it in the stream, and its end is not waited for before the tokens
-// are counted (a kernel, a copy or an event wait in between is waited for). Eight ranks, plan and reroute: 33 tokens of 64
-// experts 20.6 -> 16.8 us, 4096 tokens 30.2 -> 24.7 (27.2 with the count alone started early). Not beside a weight_sync: the reroute then runs while weight_sync's CTAs
-// read their tables (16384 tokens of 256 experts, fp8 weights: 119 -> 128 us; 8192 bool rows of 128, bf16 68.6 -> 71.3).
+// behind_plan: several ranks, and the kernel in front in the stream may be the plan: the first kernel is launched as a dependent
+// of whatever is in front, so that its CTAs are on the SMs when that ends. They read nothing but their parameters before they have
+// waited for it: the kernel in front may as well be one of the caller's that starts its dependents early and writes the ids
+// after that. Plan and reroute of eight ranks, ordinary launches and like this (us): 33 tokens of 64 experts 20.5 and 18.5, 4096
+// tokens 30.2 and 28.9, 8192 of 128 experts 34.3 and 31.6; bool rows, 4096 of 128 experts 46.5 and 42.9. Not beside a
+// weight_sync, whose CTAs read their tables in the microseconds in which the reroute would start (step with fp8 weights,
+// 16384 tokens of 256 experts 117.6 and 130.7; bf16, 8192 bool rows of 128 67.8 and 72.8).
 cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int D, int quota_mode, int interleave,
                                  bool behind_plan, cudaStream_t stream);
 cudaError_t launch_dense_backward(const Batch<DenseBwdArgs>& b, int L, int P, int D, cudaStream_t stream);

@@ -164,16 +164,16 @@ __device__ __forceinline__ void add_rows(const int32_t* __restrict__ table, int 
 // Run by all threads of every CTA of the rank's clusters (`ctas` CTAs each). Fills packed[i] of the calling thread's entries
 // begin + i * 32 + lane < end: (position among the warp's entries of the bucket) << 16 | bucket, 0xFFFFFFFF for an
 // entry without a bucket; and, once finish(b, base, all) has been called for every bucket by one thread of the CTA, the
-// ordinal of an entry is base + counters[warp][b] + position. `counted` runs when the keys are no longer waited for;
-// `staged` runs once the caller's own cp.async copies have landed, all threads. With kAll, `all` is the number of entries of the bucket in the whole input (else 0).
+// ordinal of an entry is base + counters[warp][b] + position. `staged` runs once the caller's own cp.async copies have
+// landed, all threads. With kAll, `all` is the number of entries of the bucket in the whole input (else 0).
 // `table`: the counts of the kernel in front (tiles of EPT entries a thread), or null. Without a table and with more than
 // one cluster the keys must not be overwritten. Ends with a CTA barrier.
 // No CTA may leave while another one may still read its totals: with ctas > 1 the caller arrives on the cluster barrier
 // behind this and waits on it before it exits.
-template <int EPT, bool kAll, typename IdT, typename Counted, typename Staged, typename Finish>
+template <int EPT, bool kAll, typename IdT, typename Staged, typename Finish>
 __device__ __forceinline__ void cluster_ordinals(const IdT* keys, int64_t n, int nb_valid, bool tail_bucket, int ctas,
                                                  const int32_t* __restrict__ table, const OrdShared& o, int64_t& begin,
-                                                 int64_t& end, int& iters, uint32_t (&packed)[EPT], Counted counted, Staged staged, Finish finish) {
+                                                 int64_t& end, int& iters, uint32_t (&packed)[EPT], Staged staged, Finish finish) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nthreads = blockDim.x, warps = nthreads / kWarp;
     const int nb = nb_valid + (tail_bucket ? 1 : 0), row = ord_row(nb);
     const int clusters = gridDim.x / ctas, chunk = blockIdx.x / ctas, cta = blockIdx.x % ctas;
@@ -247,7 +247,6 @@ __device__ __forceinline__ void cluster_ordinals(const IdT* keys, int64_t n, int
         add_rows(table, nb, cta, min(static_cast<int64_t>(chunk) * ctas, tiles), ctas, o.base);
         if (kAll) add_rows(table, nb, static_cast<int64_t>(chunk + 1) * ctas + cta, tiles, ctas, o.behind);
     }
-    counted();
     cp_async_wait();
     __syncthreads();
     staged();

@@ -247,7 +247,9 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(PlanCall call) {
     const int part = blockIdx.x % call.ctas_per_rank;
     const GroupDev& group = call.group;
     uint64_t* const hist_parts = call.hist_parts[local];
-    pdl_launch_dependents();  // the reroute behind it may count its tokens while the plan is made
+    // The next kernel of the stream may be on its SMs when the plan ends. Only where every rank of the group is in this launch:
+    // a plan that waits for other devices must not have the SMs held meanwhile by CTAs that wait for it.
+    if (call.nlocal == call.N) pdl_launch_dependents();
     const int N = call.N, M = call.M;
     const int L = N * M;
     const int Lpad = (L + 3) / 4 * 4;

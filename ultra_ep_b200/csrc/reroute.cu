@@ -201,6 +201,7 @@ __device__ __forceinline__ bool dense_fast_path(const uint8_t* map, const void* 
 }
 
 __global__ void __launch_bounds__(kRerouteThreads) dense_count_kernel(Batch<DenseFwdArgs> batch, int L, int behind_plan) {
+    if (behind_plan) pdl_wait();  // ahead of every read: the kernel in front may still be writing the map
     pdl_launch_dependents();  // the scatter kernel may start its prologue now
     extern __shared__ __align__(128) char smem_raw[];  // [pad4(L)] counts, one byte each
     const DenseFwdArgs& a = batch.a[blockIdx.y];
@@ -208,7 +209,6 @@ __global__ void __launch_bounds__(kRerouteThreads) dense_count_kernel(Batch<Dens
     const int tile = blockIdx.x;
     const int r0 = tile * kDenseTileRows, r1 = min(r0 + kDenseTileRows, T);
     if (r0 >= T) return;
-    const bool holds = behind_plan && tile == 0;  // this grid ends behind the plan's: its first tiles see to it
     uint8_t* counts = reinterpret_cast<uint8_t*>(a.scratch) + static_cast<int64_t>(tile) * L;
     const uint8_t* src = a.map + static_cast<int64_t>(r0) * L;
     uint32_t* cnt = reinterpret_cast<uint32_t*>(smem_raw);
@@ -238,7 +238,6 @@ __global__ void __launch_bounds__(kRerouteThreads) dense_count_kernel(Batch<Dens
         }
         __syncthreads();
         for (int i = threadIdx.x; i < L / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(counts)[i] = cnt[i];
-        if (holds) pdl_wait();
         return;
     }
     const int quads = pad4(L) / 4;
@@ -253,7 +252,6 @@ __global__ void __launch_bounds__(kRerouteThreads) dense_count_kernel(Batch<Dens
     }
     __syncthreads();
     for (int e = threadIdx.x; e < L; e += blockDim.x) counts[e] = reinterpret_cast<const uint8_t*>(cnt)[e];
-    if (holds) pdl_wait();
 }
 
 // Adds the counts of the tiles in front of `tile` to base_of[L] (shared memory, zeroed), all threads of the CTA.
@@ -453,12 +451,10 @@ __device__ __forceinline__ void write_dense_chunk(const DenseShared& s, const fl
     }
 }
 
-// kBehindPlan: the plan may still be being made when it starts. A kernel of its own: with the choice made inside, the step
-// beside weight_sync was 2 us longer (68.1 and 70.0).
-template <bool kBehindPlan>
 __global__ void __launch_bounds__(kDenseMaxThreads, 2)
 dense_scatter_kernel(Batch<DenseFwdArgs> batch, int L, int P, int D, int quota_mode, int interleave, int chunk_cols,
-                     int overlapped) {
+                     int overlapped, int behind_plan) {
+    if (behind_plan) pdl_wait();  // the count kernel waited for the plan, this one for both
     const DenseFwdArgs& a = batch.a[blockIdx.y];
     const int T = a.T;
     const int tile = blockIdx.x;
@@ -470,15 +466,11 @@ dense_scatter_kernel(Batch<DenseFwdArgs> batch, int L, int P, int D, int quota_m
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, Lq = pad4(L);
 
     // ---- nothing here depends on the count kernel ------------------------------------------------
-    if (!kBehindPlan) stage_plan_rows_async(a.lcnts, a.rqp, a.l2p, L, D, quota_mode != 0, s.routers, s.prefix, s.l2p);
+    stage_plan_rows_async(a.lcnts, a.rqp, a.l2p, L, D, quota_mode != 0, s.routers, s.prefix, s.l2p);
     for (int e = tid; e < L; e += blockDim.x) s.base[e] = 0;
     for (int i = tid; i < pad4(chunk_cols) / 4 * kDenseSegs; i += blockDim.x) reinterpret_cast<uint32_t*>(s.phys_bits)[i] = 0;
     if (tid == 0) n_several = 0;
     tile_bit_columns(a.map + static_cast<int64_t>(r0) * L, rows, kDenseSegs, L, s.bits);
-    if (kBehindPlan) {
-        pdl_wait();
-        stage_plan_rows_async(a.lcnts, a.rqp, a.l2p, L, D, quota_mode != 0, s.routers, s.prefix, s.l2p);
-    }
     cp_async_wait();
     __syncthreads();
     for (int e = tid; e < L; e += blockDim.x) {
@@ -491,7 +483,7 @@ dense_scatter_kernel(Batch<DenseFwdArgs> batch, int L, int P, int D, int quota_m
             if (any) s.several[atomicAdd(&n_several, 1)] = static_cast<uint16_t>(e);
         }
     }
-    if (!kBehindPlan && overlapped) pdl_wait();
+    if (overlapped) pdl_wait();
     sum_earlier_tiles(a, L, tile, s.base);
     __syncthreads();
 
@@ -748,10 +740,10 @@ __global__ void __launch_bounds__(kRerouteThreads) dense_backward_kernel(Batch<D
 // ---------------------------------------------------------------------------- sparse
 template <typename IdT>
 __global__ void __launch_bounds__(kOrdThreads) sparse_count_kernel(Batch<SparseArgs> batch, int K, int L, int tile_entries, int behind_plan) {
-    pdl_launch_dependents();  // the reroute kernel may start on everything that does not read the table
+    if (behind_plan) pdl_wait();  // ahead of every read: the kernel in front may still be writing the ids
+    pdl_launch_dependents();      // the reroute kernel may start on everything that does not read the table
     const SparseArgs& a = batch.a[blockIdx.y];
     count_tile<IdT>(static_cast<const IdT*>(a.ids), static_cast<int64_t>(a.T) * K, L, false, tile_entries, a.scratch);
-    if (behind_plan && blockIdx.x == 0) pdl_wait();  // this grid ends behind the plan's
 }
 
 // shared memory: prefix rows [L][8] i32 | l2p rows [L][8] i32 (both only where they fit) | ordinals | routers[L]
@@ -766,6 +758,7 @@ template <int EPT, typename IdT>
 __global__ void __launch_bounds__(kOrdThreads) __maxnreg__(EPT > 4 ? 96 : 64)
 sparse_reroute_kernel(Batch<SparseArgs> batch, int ctas, int K, int L, int D, int interleave, int rows_staged, int use_table, int behind_plan) {
     extern __shared__ __align__(128) char smem_raw[];
+    if (behind_plan) pdl_wait();  // ahead of every read
     const SparseArgs& a = batch.a[blockIdx.y];
     const IdT* ids = static_cast<const IdT*>(a.ids);
     IdT* out = static_cast<IdT*>(a.out);
@@ -777,18 +770,13 @@ sparse_reroute_kernel(Batch<SparseArgs> batch, int ctas, int K, int L, int D, in
     const OrdShared o = carve_ord_smem(rows_staged ? reinterpret_cast<char*>(l2p_s + static_cast<size_t>(L) * kStagedReps) : smem_raw, L);
     FastRouter* routers = reinterpret_cast<FastRouter*>(o.counters + kOrdWarps * ord_row(L));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (rows_staged && !behind_plan) stage_plan_rows_async(a.lcnts, a.rqp, a.l2p, L, D, quota_mode, routers, prefix_s, l2p_s);
+    if (rows_staged) stage_plan_rows_async(a.lcnts, a.rqp, a.l2p, L, D, quota_mode, routers, prefix_s, l2p_s);
 
     int64_t begin, end;
     int iters;
     uint32_t packed[EPT];
     cluster_ordinals<EPT, false, IdT>(
         ids, n, L, false, ctas, use_table ? a.scratch : nullptr, o, begin, end, iters, packed,
-        [&]() {
-            if (!behind_plan) return;
-            pdl_wait();  // the entries are counted: from here on it needs the plan
-            if (rows_staged) stage_plan_rows_async(a.lcnts, a.rqp, a.l2p, L, D, quota_mode, routers, prefix_s, l2p_s);
-        },
         [&]() {
             for (int e = tid; e < L; e += kOrdThreads) {
                 const int C = rows_staged ? routers[e].C : a.lcnts[e];
@@ -832,6 +820,7 @@ __host__ __device__ __forceinline__ size_t walk_smem_bytes(int L) {
 template <typename IdT>
 __global__ void __launch_bounds__(kWalkThreads) sparse_walk_count_kernel(Batch<SparseArgs> batch, int K, int L, int behind_plan) {
     extern __shared__ __align__(128) char smem_raw[];
+    if (behind_plan) pdl_wait();  // ahead of every read
     const SparseArgs& a = batch.a[blockIdx.y];
     const IdT* keys = static_cast<const IdT*>(a.ids);
     const int64_t n = static_cast<int64_t>(a.T) * K;
@@ -847,7 +836,6 @@ __global__ void __launch_bounds__(kWalkThreads) sparse_walk_count_kernel(Batch<S
     }
     __syncthreads();
     for (int i = threadIdx.x; i < L; i += blockDim.x) a.scratch[static_cast<int64_t>(blockIdx.x) * L + i] = hist[i];
-    if (behind_plan && blockIdx.x == 0) pdl_wait();  // this grid ends behind the plan's
 }
 
 template <typename IdT>
@@ -962,7 +950,7 @@ dispatch_positions_kernel(const int32_t* phys, int64_t n, int ctas, int P, const
     int iters;
     uint32_t packed[EPT];
     cluster_ordinals<EPT, true, int32_t>(
-        phys, n, P, true, ctas, table, o, begin, end, iters, packed, []() {}, []() {},
+        phys, n, P, true, ctas, table, o, begin, end, iters, packed, []() {},
         [&](int b, int base, int all) {
             o.base[b] = base;
             all_of[b] = all;
@@ -1212,9 +1200,8 @@ cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int
     const dim3 grid(dense_tiles(max_T), b.n);
     const int chunk = P > kDenseMaxChunkCols ? kDenseMaxChunkCols : P;
     const size_t smem_count = pad4(L), smem = dense_smem_bytes(L, chunk);
-    behind_plan = behind_plan && pdl_enabled();  // both kernels start while the plan is made
-    const auto scatter = behind_plan ? dense_scatter_kernel<true> : dense_scatter_kernel<false>;
-    cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(scatter), smem);
+    behind_plan = behind_plan && b.n > 1 && pdl_enabled();
+    cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(dense_scatter_kernel), smem);
     if (e != cudaSuccess) return e;
     e = ensure_smem_attr(reinterpret_cast<const void*>(dense_count_kernel), smem_count);
     if (e != cudaSuccess) return e;
@@ -1222,14 +1209,14 @@ cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int
     e = launch_dependent(dense_count_kernel, grid, dim3(kRerouteThreads), smem_count, stream, behind_plan, b, L, behind_plan ? 1 : 0);
     if (e != cudaSuccess) return e;
     // With one rank per launch the pair is latency-bound and the overlap pays; a launch that hosts several ranks
-    // fills the device with the first kernel alone, and early CTAs of the second only get in its way, unless both start while
-    // the plan is made.
+    // fills the device with the first kernel alone, and early CTAs of the second only get in its way, unless they do nothing
+    // but wait.
     const bool overlap = (b.n == 1 || behind_plan) && pdl_enabled();
     // up to two tiles per SM the kernel is a chain of phases: more threads shorten each
     const int sms = std::max(device_sm_count(), 1);
     const int threads = static_cast<int64_t>(grid.x) * b.n <= 2 * sms ? kDenseMaxThreads : kRerouteThreads;
-    return launch_dependent(scatter, grid, dim3(threads), smem, stream, overlap, b, L, P, D, quota_mode,
-                            interleave, chunk, overlap ? 1 : 0);
+    return launch_dependent(dense_scatter_kernel, grid, dim3(threads), smem, stream, overlap, b, L, P, D, quota_mode,
+                            interleave, chunk, overlap ? 1 : 0, behind_plan ? 1 : 0);
 }
 
 cudaError_t launch_dense_backward(const Batch<DenseBwdArgs>& b, int L, int P, int D, cudaStream_t stream) {
@@ -1365,7 +1352,7 @@ bool walk_pays(int64_t n, int L, bool beside_sync) {
 template <typename IdT>
 static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L, int D, int interleave, bool beside_sync,
                                        bool behind_plan, cudaStream_t stream) {
-    behind_plan = behind_plan && pdl_enabled();
+    behind_plan = behind_plan && b.n > 1 && pdl_enabled();
     int64_t max_n = 0;
     bool in_place = false;
     for (int i = 0; i < b.n; ++i) {
@@ -1393,7 +1380,7 @@ static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L,
     const size_t smem = sparse_smem_bytes(L, staged != 0);
     const OrdGrid g = ord_grid(max_n, L, b.n, in_place, kOrdThreads, false);
     // One rank per launch is latency-bound and the overlap with the count kernel pays; several ranks fill the device
-    // with the first kernel alone, unless both start while the plan is made.
+    // with the first kernel alone (behind a plan the second one is there early and does nothing but wait).
     const bool overlap = behind_plan || (g.table && b.n == 1 && pdl_enabled());
     if (g.table) {
         cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(sparse_count_kernel<IdT>), sizeof(int32_t) * L);
