@@ -298,8 +298,8 @@ int uep_poll_status(uep_manager* m, int local_rank, int* code, int* detail);
 int uep_clear_status(uep_manager* m);
 
 /* Failure-detection test hook, host side only: from the next call on, the hosted rank `rank`
- * completes its work but does not publish its load row / completion flags, so the ranks
- * that wait for it run into their time limit and report UEP_DEV_TIMEOUT_*; -1 switches the
+ * completes its work but does not publish its load row, its completion flags or the progress of
+ * its Wgrad reduce, so the ranks that wait for it run into their time limit and report UEP_DEV_TIMEOUT_*; -1 switches the
  * hook off. No device fault is involved. No counterpart in the reference (its waits are
  * unbounded, csrc/kernels/weight_sync.cu:666-677, csrc/kernels/ptx.cuh:73-86). While the hook is on
  * (with any rank, one outside the group too), hosted ranks treat each other as ranks of other devices do:

@@ -276,6 +276,7 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
                 counters[seg_next] = 0;
                 const uint64_t word = epoch * kReduceFlagRadix + static_cast<uint64_t>(seg_next + 1);
                 for (int lr = 0; lr < nlocal; ++lr) {
+                    if (group.my_rank[lr] == call.withhold_rank) continue;
                     for (int p = 0; p < N; ++p) {
                         if (sm.pull_mask[lr][p >> 5] & (1u << (p & 31))) st_relaxed_sys_u64(group.reduce_flags_of(p) + group.my_rank[lr], word);
                     }
@@ -326,40 +327,76 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
         const int lane = tid & 31;
         const int n_owned = sm.n_owned;
         const bool vec_zero = ((fc1 & 3) == 0) && ((fc2 & 3) == 0);
-        bool ok = true;
-        // Segment by segment over all slots: their masters' launches pull all of them at about the same pace. (Slot by slot,
-        // the last segment of the first slot held the clearing of all the others back until the pulls were over: backward of
-        // eight hosted ranks, 128 experts of 4.7 M elements, 189 us; 143 like this. Experts of 18.9 M: 350 and 310.)
-        for (int sg = 0; sg < kReduceSegments && ok; ++sg) {
-            // one lane per slot asks, so that a segment costs one round trip and not one per slot
-            unsigned here[kMaxOwned / 32];
-#pragma unroll
-            for (int h = 0; h < kMaxOwned / 32; ++h) {
-                const int u = 32 * h + lane;
-                const bool waits = u < n_owned;
-                const bool came = waits && wait_flag_ge_relaxed(sm.own_flag[u], epoch * kReduceFlagRadix + static_cast<uint64_t>(sg + 1), call.timeout_ns);
-                if (waits && !came) report_error(status0, UEP_DEV_TIMEOUT_SYNC, u);  // the slot keeps what it holds; no further wait runs
-                here[h] = __ballot_sync(kFullMask, came);
-                ok = ok && __all_sync(kFullMask, came || !waits);
-            }
-            for (int u = 0; u < n_owned; ++u) {
-                if (!((u < 32 ? here[0] : here[1]) >> (u & 31) & 1u)) continue;
-                float* base = sm.own_base[u];
-                const int t0 = sg == 0 ? 0 : seg_end(sg - 1), t1 = seg_end(sg);
-                for (int t = t0 + static_cast<int>(blockIdx.x); t < t1; t += static_cast<int>(gridDim.x)) {
-                    const bool in1 = t < tiles_fc1;
-                    const int64_t off = in1 ? static_cast<int64_t>(t) * kReduceTileElems
-                                            : fc1 + static_cast<int64_t>(t - tiles_fc1) * kReduceTileElems;
-                    const int64_t left = (in1 ? fc1 : total_numel) - off;
-                    const int elems = static_cast<int>(left < kReduceTileElems ? left : kReduceTileElems);
-                    float* dst = base + off;
-                    if (vec_zero) {
-                        if (lane == 0) clear_tile(dst, elems);
-                    } else {
-                        for (int i = lane; i < elems; i += 32) dst[i] = 0.f;
-                    }
+        // Every slot at its own pace: whatever its master's rank has released since the last look, so that what holds one rank up,
+        // or ends it, holds back that rank's slots only. One lane asks for two slots: a look at all of them costs one round
+        // trip. (Slot by slot, the last segment of the first slot held the clearing of all the others back until the pulls were
+        // over: backward of eight hosted ranks that clear as ranks of other devices do, 128 experts of 4.7 M elements, 189 us
+        // against 143. Segment by segment over all slots, the slowest rank held them back; where all keep the same pace it
+        // takes as long as this, the reduce alone 96.1 and 97.2 us, with experts of 18.9 M 267 and 264.)
+        auto clear_segment = [&](int u, int sg) {
+            float* base = sm.own_base[u];
+            const int t0 = sg == 0 ? 0 : seg_end(sg - 1), t1 = seg_end(sg);
+            for (int t = t0 + static_cast<int>(blockIdx.x); t < t1; t += static_cast<int>(gridDim.x)) {
+                const bool in1 = t < tiles_fc1;
+                const int64_t off = in1 ? static_cast<int64_t>(t) * kReduceTileElems
+                                        : fc1 + static_cast<int64_t>(t - tiles_fc1) * kReduceTileElems;
+                const int64_t left = (in1 ? fc1 : total_numel) - off;
+                const int elems = static_cast<int>(left < kReduceTileElems ? left : kReduceTileElems);
+                float* dst = base + off;
+                if (vec_zero) {
+                    if (lane == 0) clear_tile(dst, elems);
+                } else {
+                    for (int i = lane; i < elems; i += 32) dst[i] = 0.f;
                 }
             }
+        };
+        constexpr int kSlotsPerLane = kMaxOwned / kWarp;
+        int cleared[kSlotsPerLane];  // segments done with, of slot 32 * h + lane; all of them where there is no slot
+        uint64_t since[kSlotsPerLane];  // when that last changed
+#pragma unroll
+        for (int h = 0; h < kSlotsPerLane; ++h) {
+            cleared[h] = kWarp * h + lane < n_owned ? 0 : kReduceSegments;
+            since[h] = global_timer_ns();
+        }
+        while (true) {
+            bool open = false;
+#pragma unroll
+            for (int h = 0; h < kSlotsPerLane; ++h) open = open || cleared[h] < kReduceSegments;
+            if (!__any_sync(kFullMask, open)) break;
+            int released[kSlotsPerLane];
+#pragma unroll
+            for (int h = 0; h < kSlotsPerLane; ++h) {
+                released[h] = cleared[h];
+                if (cleared[h] < kReduceSegments) {
+                    const int64_t told = static_cast<int64_t>(ld_relaxed_sys_u64(sm.own_flag[kWarp * h + lane]) - epoch * kReduceFlagRadix);
+                    if (told > cleared[h]) released[h] = static_cast<int>(told < kReduceSegments ? told : kReduceSegments);
+                }
+            }
+            unsigned any_news = 0;
+#pragma unroll
+            for (int h = 0; h < kSlotsPerLane; ++h) {
+                const unsigned news = __ballot_sync(kFullMask, released[h] > cleared[h]);
+                any_news |= news;
+                for (unsigned rest = news; rest != 0; rest &= rest - 1) {
+                    const int src = __ffs(rest) - 1;
+                    const int s0 = __shfl_sync(kFullMask, cleared[h], src), s1 = __shfl_sync(kFullMask, released[h], src);
+                    for (int sg = s0; sg < s1; ++sg) clear_segment(kWarp * h + src, sg);
+                }
+                if (released[h] > cleared[h]) {
+                    cleared[h] = released[h];
+                    since[h] = global_timer_ns();
+                }
+            }
+            if (any_news != 0) continue;
+            const uint64_t now = global_timer_ns();
+#pragma unroll
+            for (int h = 0; h < kSlotsPerLane; ++h) {
+                if (cleared[h] < kReduceSegments && now - since[h] > call.timeout_ns) {
+                    report_error(status0, UEP_DEV_TIMEOUT_SYNC, kWarp * h + lane);
+                    cleared[h] = kReduceSegments;  // given up: the slot keeps what it holds
+                }
+            }
+            __nanosleep(100);
         }
         if (lane == 0) bulk_wait_all<0>();
     } else if (!sm.vector_ok) {

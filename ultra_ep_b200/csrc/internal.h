@@ -114,6 +114,7 @@ struct ReduceCall {
     uint64_t timeout_ns;
     int ctas_per_rank;
     int owners_clear;           // test hook: replicas of hosted ranks are cleared by their owners too, as on other devices
+    int withhold_rank;          // test hook: this rank reports no progress (-1: off)
     uint64_t* reduce_epoch;     // the reduce epoch counter of the first hosted rank
     int* counters;              // [kReduceSegments]: CTAs of this launch that have passed each segment; zero between calls
     unsigned long long* trace;  // optional: 8 globaltimer stamps per CTA (tuning aid), or null

@@ -747,6 +747,7 @@ int uep_grad_reduce(uep_manager* m, int layer_id, const int64_t* const* fc1_grad
     call.trace = m->sync_trace;
     call.reduce_epoch = m->ranks[0].epochs + 2;
     call.owners_clear = m->withhold_rank >= 0 ? 1 : 0;
+    call.withhold_rank = m->withhold_rank;
     // a group of one rank has no replicas
     if (m->R > 0 && m->N > 1 && m->total_numel > 0) UEP_CUDA_TRY(launch_grad_reduce(call, m->comm_stream));
     return finish_sync_op(m, async_finish, current, done_event);
