@@ -200,7 +200,10 @@ __device__ __forceinline__ void bulk_store(void* gdst, const void* smem_src, uin
                  : "memory");
 }
 // The same with an L2 priority. `l2_first`: the lines are the first to go, so that a stream of data that is longer than L2
-// does not push out what the kernels around it come back to.
+// does not push out what the kernels around it come back to. What comes next finds less of a shorter one there, and of one that
+// is read from its start again: weight_sync has the line, and why the Wgrad reduce's zeros and the row gather keep the usual
+// priority stands there.
+constexpr int64_t kL2Bytes = 126ll << 20;
 __device__ __forceinline__ uint64_t l2_normal() {
     uint64_t policy;
     asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));

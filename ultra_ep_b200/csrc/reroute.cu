@@ -1059,9 +1059,8 @@ __global__ void __launch_bounds__(32) gather_rows_kernel(const uint8_t* __restri
     Cursor load = whole ? Cursor{first << shift, 0} : Cursor{first / chunks_per_row, static_cast<int>(first % chunks_per_row)};
     Cursor store = load;
     int issued = 0, load_stage = 0, load_slot = 0, load_half = 0;
-    // A row that is read once need not stay in L2 (65536 rows of 8 KiB with their positions 187.5 us -> 184.7; the stores
-    // too: 188). With fewer rows than reads some are read again.
-    const uint64_t policy = num_src_rows >= num_rows ? l2_first() : l2_normal();
+    // (Loads whose lines are the first to leave L2: the gather alone 178.5 -> 176.4 us, 65536 rows of 8 KiB, and gather and a
+    // kernel that reads its output 335 -> 340, 16384 rows 95 -> 96.)
     auto issue_load = [&]() {
         const int n = rows_of(load);
         const uint32_t bytes = row_part(load);
@@ -1073,7 +1072,7 @@ __global__ void __launch_bounds__(32) gather_rows_kernel(const uint8_t* __restri
                 report_error(status, UEP_DEV_BAD_PLAN, static_cast<int>(load.row + lane));
                 src_row = 0;
             }
-            bulk_load(smem_raw + load_stage * kGatherChunk + lane * bytes, in + src_row * row_bytes + offset(load), bytes, &bars[load_stage], policy);
+            bulk_load(smem_raw + load_stage * kGatherChunk + lane * bytes, in + src_row * row_bytes + offset(load), bytes, &bars[load_stage]);
         }
         advance(load);
         ++issued;

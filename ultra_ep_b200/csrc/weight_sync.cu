@@ -583,10 +583,16 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
         if (sm.all_aligned) {
             if (tid == 0) {
                 // Masters and replicas of ranks on this device are one stream through its L2, as the plain path's streaming
-                // loads and stores are: the step of eight ranks (8192 tokens, 128 experts, fp8 weights) 64.1 -> 59.7 us,
-                // the copy itself 42.0 -> 40.9; loads or stores alone change nothing. (Not measured over NVLink, and a
-                // relayed chunk is read again where it lands: there the priority is the usual one.)
-                const uint64_t policy = !kR && nlocal > 1 ? l2_first() : l2_normal();
+                // loads and stores are. Where it is longer than L2 its lines are the first to leave, so that ids and tables
+                // stay: the step of eight ranks (8192 tokens, 128 experts, eight replicas), in us with the usual priority and
+                // like this, alone and with a kernel behind it that reads the replicas: 8 MB each 49.0 and 44.4, 76.4 and
+                // 74.8; 16 MB 62.8 and 58.5, 115.4 and 116.2; 19 MB 67.8 and 63.8, 121 and 119.7. A shorter one is still
+                // there when the experts are used: 4 MB each 46.0 and 44.2, but 68.4 and 71.3; 2 MB 42.8 and 43.0, 64.4 and
+                // 64.6. Loads or stores alone change nothing. (Not measured over NVLink, and a relayed chunk is read again
+                // where it lands: there the priority is the usual one.)
+                const int64_t expert_bytes = sh.bytes[0] + sh.bytes[1] + sh.bytes[2] + sh.bytes[3];
+                const bool streams = !kR && nlocal > 1 && (sm.n_active + sm.total_reps) * expert_bytes > kL2Bytes;
+                const uint64_t policy = streams ? l2_first() : l2_normal();
                 TileRef* ring = sm.ring;
                 int* ring_valid = sm.ring_valid;
                 uint64_t** ring_flag = sm.ring_flag;
