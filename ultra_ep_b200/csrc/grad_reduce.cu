@@ -56,7 +56,7 @@ constexpr int kMaxOwned = 64;  // used replica slots of the hosted ranks (a lane
 struct ReduceShared {
     int n_active, total_reps, vector_ok;
     volatile int error;
-    int n_owned, s_go;
+    int n_owned;
     volatile long long done_items;                 // items of this CTA whose replica tiles have all been consumed
     volatile int pull_finished;                    // the pull phase of this CTA is over (all items, or given up)
     int n_hosted;                                  // replicas that lie on ranks of this launch

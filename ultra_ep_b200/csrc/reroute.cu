@@ -583,20 +583,15 @@ __device__ __forceinline__ void for_each_marked(uint32_t word, F&& cell) {
     }
 }
 
-// Zeros by all threads of the CTA, 16 bytes a store but for the ends.
-__device__ __forceinline__ void zero_fill(void* where, int bytes) {
-    char* p = static_cast<char*>(where);
-    const int head = min(bytes, static_cast<int>((16u - (reinterpret_cast<uintptr_t>(p) & 15u)) & 15u));
-    const int vecs = (bytes - head) / 16, tail = head + vecs * 16;
-    if (static_cast<int>(threadIdx.x) < head) p[threadIdx.x] = 0;
-    uint4* v = reinterpret_cast<uint4*>(p + head) + threadIdx.x;
+// Zeros by all threads of the CTA, 16 bytes a store: `where` is 16-byte aligned.
+__device__ __forceinline__ void zero_fill(void* where, int vecs) {
+    uint4* v = static_cast<uint4*>(where) + threadIdx.x;
     int left = vecs - static_cast<int>(threadIdx.x);
     for (; left > 3 * static_cast<int>(blockDim.x); left -= 4 * blockDim.x, v += 4 * blockDim.x) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) v[u * blockDim.x] = make_uint4(0, 0, 0, 0);
     }
     for (; left > 0; left -= blockDim.x, v += blockDim.x) *v = make_uint4(0, 0, 0, 0);
-    if (static_cast<int>(threadIdx.x) < bytes - tail) p[tail + threadIdx.x] = 0;
 }
 
 // `bytes` bytes into shared memory (16-byte aligned there), asynchronously where the source is aligned.
@@ -611,24 +606,22 @@ __device__ __forceinline__ void stage_bytes(uint8_t* dst, const uint8_t* __restr
     }
 }
 
-// Which of the 32 columns from `c` on are marked in a row of `cols` bytes in shared memory (rows stand `cols` bytes apart).
+// Which of the 32 columns from `c` on are marked in a row of `cols` bytes, a multiple of four, in shared memory.
 __device__ __forceinline__ uint32_t row_bits(const uint8_t* row, int c, int cols) {
     uint32_t bits = 0;
-    if (cols % 4 == 0) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const uint32_t marks = c + 4 * k < cols ? nonzero_bytes(*reinterpret_cast<const uint32_t*>(row + c + 4 * k)) : 0u;
-            bits |= (marks * 0x10204080u) >> 28 << (4 * k);  // four bytes of 0 or 1 to four bits
-        }
-    } else {
-        for (int k = 0; k < 32 && c + k < cols; ++k) bits |= (row[c + k] != 0 ? 1u : 0u) << k;
+    for (int k = 0; k < 8; ++k) {
+        const uint32_t marks = c + 4 * k < cols ? nonzero_bytes(*reinterpret_cast<const uint32_t*>(row + c + 4 * k)) : 0u;
+        bits |= (marks * 0x10204080u) >> 28 << (4 * k);  // four bytes of 0 or 1 to four bits
     }
     return bits;
 }
 
 // Backward of a tile of `tile_rows` tokens: the rows of both maps are copied to shared memory, the output is filled with
 // zeros, and the marked cells (topk of them a token) are shared by the lanes: a cell looks its instances up in the expanded
-// row, fetches one gradient and stores it over the zero. Full occupancy (32 registers), since every step waits for memory.
+// row, fetches one gradient and stores it over the zero. L is a multiple of four and the output 16-byte aligned. Every step
+// waits for memory, so occupancy counts: 32 registers, and eight CTAs an SM up to 28 KB of staged rows (23 KB at 128 experts
+// and 160 slots; four CTAs at the 56 KB that the dispatch allows rows of more than eight tokens).
 // Both maps as bit columns and four columns of eight rows per thread took 14 M instructions a call of eight ranks of 8192
 // tokens and 128 experts, two thirds of the issue slots: 24.8 us a call, 18.3 like this (20.7 with four CTAs an SM); one
 // rank of 16384 tokens and 256 experts 12.3 (a thread per four cells 19.3).
@@ -663,7 +656,7 @@ dense_backward_tile_kernel(Batch<DenseBwdArgs> batch, int L, int P, int D, int t
             if (i % kStagedReps < D) cp_async_4(l2p_s + i, a.l2p + static_cast<int64_t>(i / kStagedReps) * D + i % kStagedReps);
         }
     }
-    zero_fill(out, rows * L * 4);
+    zero_fill(out, rows * L / 4);
     cp_async_wait();
     __syncthreads();  // the zeros are in front of the stores below, too
     const int groups = (L + 31) / 32, tasks = rows * groups, lane = threadIdx.x & 31;
