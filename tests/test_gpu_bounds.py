@@ -41,10 +41,11 @@ class Guarded:
         return all(bool((raw[:GUARD] == self.fill).all()) and bool((raw[GUARD + n:] == self.fill).all()) for raw, n in self.made)
 
 
-BACKWARD = [  # T, L, P, D: either side of 2^22 cells, a last tile of any height
+BACKWARD = [  # T, L, P, D: either side of 2^20 cells (2^22 up to 64 experts), tiles of 64, 32, 16 and 8 rows, a last tile of any height
     (1, 8, 12, 4), (1030, 128, 161, 8), (513, 37, 50, 6), (32769, 128, 192, 8), (32771, 128, 160, 8), (32790, 128, 160, 8), (32799, 128, 160, 8),
     (65601, 64, 128, 8), (65599, 64, 80, 8), (16385, 256, 320, 8), (16391, 256, 320, 8), (43700, 96, 98, 3), (3131, 1340, 1400, 8), (116600, 36, 60, 8),
     (8195, 512, 544, 8), (8130, 516, 540, 8),
+    (8191, 128, 160, 8), (8193, 128, 161, 8), (8251, 256, 322, 8), (2077, 512, 800, 16), (2100, 500, 4099, 8), (20001, 128, 160, 8), (10951, 96, 131, 3),
 ]
 
 
