@@ -35,6 +35,24 @@ def inputs(manager, cuda_device):
     return layer, probs.requires_grad_(True), rmap
 
 
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+def test_plan_from_ids_that_are_not_contiguous(manager, cuda_device, dtype):
+    """The plan reads a copy of them on the communication stream; memory that is asked for meanwhile must not be that copy."""
+    gen = torch.Generator(device=cuda_device).manual_seed(9)
+    ids = torch.randint(0, L, (6, 700), generator=gen, device=cuda_device, dtype=dtype).t()
+    want = torch.bincount(ids.reshape(-1), minlength=L).int()
+    layer = manager.allocate_microbatch_slot(1)
+    manager.update_placement_sparse(layer, ids)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(manager.get_comm_stream()):
+        torch.cuda._sleep(40_000_000)  # the plan waits for work in front of it
+    manager.update_placement_sparse(layer, ids)
+    others = [torch.zeros((700, 6), device=cuda_device, dtype=dtype) for _ in range(8)]
+    torch.cuda.synchronize()
+    assert torch.equal(manager.runtime.get_global_logical_expert_loads_tensor(), want)
+    assert all(not x.any() for x in others)
+
+
 def test_forward_mode_is_refused(manager, inputs):
     layer, probs, rmap = inputs
     with fwAD.dual_level():

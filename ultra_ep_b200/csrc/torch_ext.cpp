@@ -243,6 +243,8 @@ public:
         auto ids = topk_ids.contiguous();
         // as the reference: on the communication stream, after the current stream (csrc/ultra_ep.cpp:757-759)
         void* comm = uep_manager_comm_stream(m_);
+        // a copy belongs to nobody else: it has to outlive the plan on that stream
+        if (!topk_ids.is_contiguous()) ids.record_stream(at::cuda::getStreamFromExternal(static_cast<cudaStream_t>(comm), device_).unwrap());
         uep_event* ev = nullptr;
         check(uep_event_record(current_stream(), &ev), "update_placement_sparse");
         const int rc = uep_event_stream_wait(ev, comm);
