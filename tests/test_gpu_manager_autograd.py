@@ -1,5 +1,5 @@
 """Manager.reroute as autograd sees it, on a group of one rank: the gradients that reach the node, and the forms of
-differentiation that it refuses."""
+differentiation that it refuses; and a plan from ids that are not contiguous."""
 
 import pytest
 import torch

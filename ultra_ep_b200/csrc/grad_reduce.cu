@@ -16,10 +16,10 @@
 //     zeroes it in its own memory: the master's launch reports its progress in 16 segments
 //     (a counter per segment that every CTA bumps when it has consumed its items of the segment;
 //     the CTA that completes a segment stores "epoch, segments done" into a flag word on every
-//     rank it pulls from), and the host rank's launch, once its own pulls are done, clears each
-//     segment of its used slots as soon as the flag allows, from a warp of its own that runs beside
-//     the pulls (bulk stores from a zero tile into local memory). A replica that lies on a rank
-//     of the same launch needs none of that: the CTA that pulled a tile clears it;
+//     rank it pulls from), and the host rank's launch clears each segment of each used slot as
+//     soon as its flag allows, from a warp of its own that runs beside that launch's pulls (bulk
+//     stores from a zero tile into local memory). A replica that lies on a rank of the same launch
+//     needs none of that: the CTA that pulled a tile clears it;
 //   * roles are split. Two producer warps (one lane each) only issue bulk loads: one feeds the
 //     ring of replica tiles, the other the ring of master tiles. Eight
 //     consumer warps wait on a stage's "full" mbarrier, add it into accumulators in registers
@@ -33,7 +33,7 @@
 //   * tiles are interleaved over masters so that concurrent CTAs pull from different peers; they go
 //     expert by expert where all replicas lie in this device's memory.
 // The CTA budget (SMs used while the backward pass runs next to it) is the caller's knob
-// (grad_reduce_num_sms); each CTA holds about 215 KiB of shared memory.
+// (grad_reduce_num_sms); each CTA holds about 215 KB of shared memory (twelve stages and the zero tile are 200 KiB).
 
 #include "internal.h"
 

@@ -21,7 +21,7 @@ constexpr int kPlanMaxCtas = 32;  // CTAs of one rank in the plan kernel
 // Where the group's buffers are. By value in the kernels' parameters, so that the first load of a kernel is of data and not
 // of a pointer to it (each of the two is a miss: the tables were last read a layer ago). Fixed once connected. With a table
 // per rank in device memory, and the plan's epoch and weight_sync's first unit waited for before the first load of data, the
-// step of eight ranks (8192 tokens, 128 experts, fp8 weights of 19 MB) took 70.0 us, 64.6 like this; plan kernel 19.0 and
+// step of eight ranks (8192 tokens, 128 experts, fp8 weights of 19 MB) took 67.2 us, 63.2 like this; plan kernel 19.0 and
 // 17.3.
 struct GroupDev {
     uint8_t* arena[kMaxPeers];  // of every rank of the group, as the hosted ranks see them (all of them the same)

@@ -742,7 +742,7 @@ int uep_grad_reduce(uep_manager* m, int layer_id, const int64_t* const* fc1_grad
     call.fc1_numel = m->cfg.expert_fc1_numel;
     call.fc2_numel = m->cfg.expert_fc2_numel;
     call.timeout_ns = m->timeout_ns;
-    // one CTA per SM at most (128 KiB of shared memory each): hosted ranks share the device's SMs
+    // one CTA per SM at most (200 KiB of shared memory each): hosted ranks share the device's SMs
     call.ctas_per_rank = std::max(1, std::min(m->grad_reduce_ctas, m->num_sms / m->nlocal));
     call.trace = m->sync_trace;
     call.reduce_epoch = m->ranks[0].epochs + 2;
