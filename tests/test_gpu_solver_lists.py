@@ -1,0 +1,50 @@
+"""The placement solver where its lists of ranks can go wrong: thresholds on both sides of 2^24, from which on a rank's key takes 64
+bits; ranks that come back with equal slack; one redundant slot, so that nobody comes back; more experts with replicas than warps;
+floors that fail. Against the CPU oracle, whole numbers: bit-exact."""
+
+import numpy as np
+import pytest
+
+import cases as Cs
+import gpu_util as G
+from oracle import uep_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(loads, M, R, what, **kw):
+    N = loads.shape[0]
+    case = Cs.SolveCase(what, np.ascontiguousarray(loads, dtype=np.int32), M, R, N, ranks=(0, N - 1), **kw)
+    for rank in case.ranks:
+        out = G.cuda_solve(case, rank)
+        assert out["status"].tolist() == [0, 0]
+        plan = O.solve_placement(case.loads_per_rank, M, R, N, rank, G.oracle_params(case))
+        for f in G.PLAN_FIELDS:
+            assert np.array_equal(out[f].cpu().numpy(), getattr(plan, f)), (what, rank, f)
+
+
+# Mean load of a rank. (The oracle adds slack up in 32 bits: ranks^2 times the mean stays below 2^31.)
+@pytest.mark.parametrize("mean", [(1 << 24) - 40000, (1 << 24) - 1, 1 << 24, (1 << 24) + 3, 3 << 23])
+@pytest.mark.parametrize("N,M,R", [(2, 3, 1), (4, 2, 2), (8, 5, 3)])
+def test_keys_on_both_sides_of_32_bits(native_lib, cuda_device, mean, N, M, R):
+    rng = np.random.default_rng(mean % 1000003 + N)
+    for eps in (0.0, 0.01):
+        w = rng.dirichlet(np.full(N * M, 0.3))
+        total = np.floor(w * mean * N).astype(np.int64)
+        total[0] += mean * N - total.sum()
+        split = np.stack([total // N + (np.arange(N * M) % N == r) for r in range(N)])
+        split[0] += total - split.sum(0)
+        _check(np.maximum(split, 0), M, R, f"mean {mean}", eps=eps, min_tokens=1 if eps else 1024)
+
+
+@pytest.mark.parametrize("N,M,R", [(8, 4, 2), (16, 2, 1), (33, 3, 2), (72, 4, 4)])
+@pytest.mark.parametrize("min_tokens,bt", [(1, 1.0), (64, 1.0), (4096, 1.0), (256, 1.3)])
+def test_equal_slack_and_floors(native_lib, cuda_device, N, M, R, min_tokens, bt):
+    rng = np.random.default_rng(N + min_tokens)
+    for i in range(3):
+        loads = np.zeros((N, N * M), np.int64)
+        hot = rng.choice(N, size=max(1, N // 3), replace=False)
+        for r in hot:  # sources of several exports each, everyone else equal
+            loads[:, r * M:r * M + M] = rng.integers(1, 5, size=M) * 64
+        loads[:, rng.choice(N) * M] += 16 * i
+        _check(loads, M, R, f"equal {i}", min_tokens=min_tokens, balance_threshold=bt, allow_zero=i == 1)

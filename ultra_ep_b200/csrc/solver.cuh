@@ -5,20 +5,20 @@
 // (csrc/kernels/placement.cu:788-1482 of the reference): same fp32 threshold
 // arithmetic, same tie-breaks, same probe schedule of the threshold search, same
 // largest-remainder splits. The execution is different:
-//   * the ranks with slack are kept sorted in the lanes of a warp (1-3 per lane), and one step
-//     makes all the exports of an expert;
-//   * an expert is drained once, from its one home rank, so a build keeps no occupancy table
-//     and no exported sums: a source's masters sit in the lanes, and the walk over the sources
-//     ends at the first one below the threshold;
+//   * the ranks with slack wait in two sorted lists, and an expert is drained once, from its one home rank, so a build keeps no
+//     occupancy table and no exported sums, and the walk over the sources ends at the first one below the threshold;
 //   * the three builds of the fast path and the capacity pre-check run side by side on four
-//     warps (the serial search takes the first that is feasible), while the other warps clear
-//     the outputs;
+//     warps (the serial search takes the first that is feasible), while the other warps write
+//     the outputs of all experts as they are without replicas;
+//   * an export carries its redundant slot and so its physical id: behind the build the experts with replicas are written
+//     over side by side, a warp or two each;
 //   * each rank's masters are ranked by counting instead of a serial insertion sort;
 //   * the loads come in shared memory from the caller, and with one domain the per-rank load matrix
 //     too where it fits (plan.cu); else the few entries of it that are needed are read through L2.
-//     Without the matrix shared memory stays under 48 KB at the static limits.
-// All of it is latency of one CTA. Kernel time of uep_solve_placement on one B200: 64 ranks x 4 experts x 2 slots 25.3 us
-// (39.5 with the outputs cleared first, one build after another and one warp maximum per export), of which the build 14.
+// All of it is latency of one CTA: dependent instructions of some ten cycles each, so what counts is how many of them follow one
+// another. Calls of uep_solve_placement among others on one B200: 64 ranks x 4 experts x 2 slots 20.5 us (25.9 with the lists in
+// the lanes of a warp, slots handed out and experts split behind the build); plan and reroute of eight ranks, 33 tokens of 64
+// experts each, 16.7 (18.4).
 #pragma once
 
 #include <climits>
@@ -27,11 +27,17 @@
 
 namespace uep {
 
+// An export: tokens moved to a redundant slot. `place`: the slot's physical id inside the domain << 8 | its rank.
 struct ExportEntry {
-    int expert_local;
-    int target_rank_local;
     int quota;
+    int place;
 };
+
+// All the exports of one expert, which follow one another in the plan: expert, first entry, entries, rank of the master.
+__device__ __forceinline__ uint32_t pack_batch(int expert, int first, int count, int rank) {
+    return static_cast<uint32_t>(expert | first << 9 | count << 18) | static_cast<uint32_t>(rank) << 25;
+}
+static_assert(kMaxExpertsPerDomain <= 1 << 9 && kMaxExportsPerDomain <= 1 << 9 && kMaxRanksPerDomain < 1 << 7, "pack_batch");
 
 struct SolveArgs {
     const int32_t* global_loads;    // [L]
@@ -57,50 +63,52 @@ struct SolveArgs {
 };
 
 constexpr int kSolverProbeWarps = 4;
+constexpr int kMaxListed = kMaxRanksPerDomain + 2;  // ranks of a list, and its end
 
 // Control words in shared memory.
 enum SolverCtrl {
-    kCtlLo = 0, kCtlHi, kCtlStop0, kCtlNumExports = kCtlStop0 + kSolverProbeWarps, kCtlSmallRange,
+    kCtlLo = 0, kCtlHi, kCtlTotal, kCtlStop0, kCtlNumBatches = kCtlStop0 + kSolverProbeWarps, kCtlSmallRange,
     kCtlProbe0, kCtlValid0 = kCtlProbe0 + kSolverProbeWarps, kCtlFeasible0 = kCtlValid0 + kSolverProbeWarps,
-    kCtlExports0 = kCtlFeasible0 + kSolverProbeWarps, kCtlMultiCount = kCtlExports0 + kSolverProbeWarps, kCtlCount
+    kCtlBatches0 = kCtlFeasible0 + kSolverProbeWarps, kCtlCount = kCtlBatches0 + kSolverProbeWarps
 };
 static_assert(kCtlCount <= 32, "control words");
 
 struct SolverSmem {
-    int32_t* loads;           // [E]
-    int32_t* my_loads;        // [E]
-    int32_t* sorted_experts;  // [E]
-    int32_t* expert_slot;     // [E]
-    int32_t* rank_load;       // [Gp]
-    int32_t* source_order;    // [Gp] ranks by load, largest first, ties to the lower one
-    int32_t* sink_order;      // [Gp] smallest first, likewise
-    int32_t* next_slot;       // [Gp]
-    int32_t* export_sum;      // [4][E] of the four warps that build plans
-    ExportEntry* plan;        // [4][kMaxExportsPerDomain]
-    int* ctrl;                // [kCtlCount]
+    int32_t* loads;      // [E]
+    int32_t* my_loads;   // [E]
+    int2* masters;       // [E] rank after rank: {load, expert}, largest load first, ties to the lower expert
+    int2* source;        // [G] {load, rank}, largest load first, ties to the lower rank
+    int2* sink;          // [G] {load, rank}, smallest first, likewise
+    int32_t* rank_load;  // [G]
+    ExportEntry* plan;   // [4][kMaxExportsPerDomain] of the four warps that build plans
+    uint32_t* batches;   // [4][kMaxExportsPerDomain]
+    long long* fresh;    // [4][kMaxListed] lists of ranks of the four warps
+    longlong2* again;    // [4][kMaxListed]
+    int* ctrl;           // [kCtlCount]
 };
 
 __host__ __device__ inline int solver_ns(int G) { return (G + 31) / 32; }
-__host__ __device__ inline int solver_gpad(int G) { return (G + 3) / 4 * 4; }
+__host__ __device__ inline int solver_pad(int n) { return (n + 3) / 4 * 4; }
 __host__ __device__ inline size_t solver_smem_bytes(int E, int G) {
-    return sizeof(int32_t) * (4 * static_cast<size_t>(E) + 4 * solver_gpad(G) + kSolverProbeWarps * static_cast<size_t>(E)) +
-           kSolverProbeWarps * sizeof(ExportEntry) * kMaxExportsPerDomain + sizeof(int) * 32;
+    return sizeof(int32_t) * (4 * static_cast<size_t>(solver_pad(E)) + 5 * solver_pad(G)) +
+           kSolverProbeWarps * ((sizeof(ExportEntry) + sizeof(uint32_t)) * kMaxExportsPerDomain + 3 * sizeof(long long) * kMaxListed) +
+           sizeof(int) * 32;
 }
 
 __device__ inline SolverSmem carve_solver_smem(char* raw, int E, int G) {
-    const int gp = solver_gpad(G);
+    const int ep = solver_pad(E), gp = solver_pad(G);
     SolverSmem s;
     int32_t* p = reinterpret_cast<int32_t*>(raw);
-    s.loads = p; p += E;
-    s.my_loads = p; p += E;
-    s.sorted_experts = p; p += E;
-    s.expert_slot = p; p += E;
+    s.loads = p; p += ep;
+    s.my_loads = p; p += ep;
+    s.masters = reinterpret_cast<int2*>(p); p += 2 * ep;
+    s.source = reinterpret_cast<int2*>(p); p += 2 * gp;
+    s.sink = reinterpret_cast<int2*>(p); p += 2 * gp;
     s.rank_load = p; p += gp;
-    s.source_order = p; p += gp;
-    s.sink_order = p; p += gp;
-    s.next_slot = p; p += gp;
-    s.export_sum = p; p += kSolverProbeWarps * E;
-    s.plan = reinterpret_cast<ExportEntry*>(p); p += kSolverProbeWarps * 3 * kMaxExportsPerDomain;
+    s.plan = reinterpret_cast<ExportEntry*>(p); p += kSolverProbeWarps * 2 * kMaxExportsPerDomain;
+    s.batches = reinterpret_cast<uint32_t*>(p); p += kSolverProbeWarps * kMaxExportsPerDomain;
+    s.again = reinterpret_cast<longlong2*>(p); p += kSolverProbeWarps * 4 * kMaxListed;
+    s.fresh = reinterpret_cast<long long*>(p); p += kSolverProbeWarps * 2 * kMaxListed;
     s.ctrl = reinterpret_cast<int*>(p);
     return s;
 }
@@ -114,154 +122,153 @@ __device__ __forceinline__ int warp_inclusive_scan(int v, int lane) {
     return v;
 }
 
+// A rank that an export has used already and that has slack and slots left, as a key (below) and the slots used.
+template <typename Key>
+struct WaitingRank {
+    Key key;
+    int slots;
+};
+static_assert(sizeof(WaitingRank<long long>) == 16, "two words of two");
+
 // Greedy export plan for one threshold, by one warp. Returns feasibility (uniform over
 // the warp). Semantics of csrc/kernels/placement.cu:337-667 of the reference.
 //
 // An expert's exports go to the ranks by slack, largest first, ties to the lower rank, each rank once; every one of them is
-// filled up except the last. So the ranks are kept sorted in the lanes (slot 32 s + lane), with inclusive sums of their
-// slack, and one step per expert finds all its exports: lane i takes part while the slack in front of it is less than what
-// is to be moved and its share passes the floor. The filled ranks leave at the front, and the last one, if slack and
-// slots are left, moves back to its place. (One export at a time, a warp maximum each: 325 ns an export.)
-// `stop`: raised by a warp whose result makes this build pointless.
-template <int NS, bool STORE>
-__device__ bool warp_build_plan(const SolverSmem& sm, int32_t* export_sum, ExportEntry* plan, int& num_exports, int thr, int E,
-                                int G, int M, int R, int min_tokens, bool allow_zero_master, bool dynamic_floor, int lane,
-                                const volatile int* stop = nullptr) {
-    num_exports = 0;
-    if (STORE) {
-        __syncwarp();  // an earlier build of this warp may still be storing its sums
-        for (int e = lane; e < E; e += kWarp) export_sum[e] = 0;
-        __syncwarp();
-    }
-    int slack[NS], meta[NS], upto[NS];  // meta: free slots << 8 | rank; upto: slack of this slot and all in front of it
-    int order[NS], order_load[NS];      // the sources
-    int end = 0;                        // slots with slack are [head, end)
-    int local_excess = 0, total_slack = 0;
-#pragma unroll
-    for (int s = 0; s < NS; ++s) {
-        const int i = lane + kWarp * s;
-        const int sink = i < G ? sm.sink_order[i] : 0;
-        slack[s] = i < G ? max(thr - sm.rank_load[sink], 0) : 0;
-        meta[s] = R << 8 | sink;
-        order[s] = i < G ? sm.source_order[i] : 0;
-        order_load[s] = i < G ? sm.rank_load[order[s]] : thr;
-        local_excess += max(order_load[s] - thr, 0);
-        end += __popc(__ballot_sync(kFullMask, slack[s] > 0));
-        upto[s] = warp_inclusive_scan(slack[s], lane) + total_slack;
-        total_slack = __shfl_sync(kFullMask, upto[s], kWarp - 1);
-    }
-    const int total_excess = warp_sum(local_excess);
-    if (total_excess == 0) return true;
-    // Every export takes the same from both, so the slack left always covers the excess left.
-    if (total_excess > total_slack) return false;
-
-    auto at = [&](const int (&v)[NS], int slot) {
-        int x = __shfl_sync(kFullMask, v[0], slot & 31);
-#pragma unroll
-        for (int s = 1; s < NS; ++s) {
-            const int y = __shfl_sync(kFullMask, v[s], slot & 31);
-            x = slot >> 5 == s ? y : x;
-        }
-        return x;
-    };
-    auto masters = [&](int src, int base, int& e, int& load) {  // 32 of the source's masters, one per lane
-        e = base + lane < M ? sm.sorted_experts[src * M + base + lane] : 0;
-        load = base + lane < M ? sm.loads[e] : 0;
-    };
-    int head = 0, gone = 0;  // gone: slack in front of slot `head`, as `upto` counts it
-    int src = at(order, 0), src_load = at(order_load, 0), first_e, first_load;
-    masters(src, 0, first_e, first_load);
-    for (int ord = 0; ord < G; ++ord) {
-        int need = src_load - thr;
-        if (need <= 0) break;  // sources come by load: no later one is above the threshold
-        if (stop != nullptr && __shfl_sync(kFullMask, *stop, 0) != 0) return false;
-        const int this_src = src;
-        int my_e = first_e, my_load = first_load;
-        const int next_ord = min(ord + 1, G - 1);  // fetched while this one is drained
-        src = at(order, next_ord);
-        src_load = at(order_load, next_ord);
-        masters(src, 0, first_e, first_load);
-        bool drained = false;  // the masters come by load too: no later one has anything to give
-        for (int base = 0; base < M && need > 0 && !drained; base += kWarp) {
-            if (base > 0) masters(this_src, base, my_e, my_load);
-            const int in_chunk = min(M - base, kWarp);
-            for (int pos = 0; pos < in_chunk && need > 0; ++pos) {
-                const int load_e = __shfl_sync(kFullMask, my_load, pos);
-                const int avail = load_e - ((!allow_zero_master && load_e > 0) ? 1 : 0);
-                if (avail <= 0) {
-                    drained = true;
-                    break;
+// filled up except the last, which comes back with the slack it has left once the expert is placed. So the ranks wait in two
+// lists, both sorted: those that no export has used (`fresh`, in the order of sm.sink) and those that came back (`again`, the
+// best at its end), and an export takes the better of the two heads. A rank in a list is a key, slack << 7 | 127 - rank: the
+// larger one is the better one, and the ends of the lists are -1. A chain of dependent steps by nature, so one lane runs it,
+// with few instructions and branches an export, and what it will need next is asked for one export and one expert ahead. (The
+// lists in the lanes of a warp and all exports of an expert in one step: ballots, shuffles and the branches around them were
+// 1000 cycles an expert.) There are never more exports than redundant slots (kMaxExportsPerDomain).
+// Key: int where slack << 7 fits, long long beyond. `stop`: raised by a warp whose result makes this build pointless.
+template <typename Key, bool STORE>
+__device__ bool drain_sources(const SolverSmem& sm, int buffer, int& num_batches, int thr, int with_slack, int G, int M, int R,
+                              int min_tokens, bool allow_zero_master, bool dynamic_floor, const volatile int* stop) {
+    ExportEntry* const plan = sm.plan + buffer * kMaxExportsPerDomain;
+    uint32_t* const batches = sm.batches + buffer * kMaxExportsPerDomain;
+    const Key* const fresh_keys = reinterpret_cast<const Key*>(sm.fresh + buffer * kMaxListed);
+    WaitingRank<Key>* const again = reinterpret_cast<WaitingRank<Key>*>(sm.again + buffer * kMaxListed) + 2;  // [-2], [-1]: its end
+    const WaitingRank<Key> none{Key(-1), 0};
+    again[-2] = none;
+    again[-1] = none;
+    const int keep = allow_zero_master ? 0 : 1, by_count = dynamic_floor ? 1 : 0, Lp = M + R;
+    int used = 0, waiting = 0;  // of `fresh`; in `again`
+    Key fresh = fresh_keys[0], fresh_next = fresh_keys[1];
+    WaitingRank<Key> top = none, top_next = none;
+    int count = with_slack;  // ranks in both lists
+    int num_exports = 0, ord = 0, left = M;
+    int2 source = sm.source[0];
+    int need = source.x - thr, at_master = source.y * M;
+    int2 master = sm.masters[at_master];
+    int2 next_source = sm.source[min(1, G - 1)];
+    int2 next_first = sm.masters[next_source.y * M];
+    while (true) {
+        const int2 follow = sm.masters[min(at_master + 1, G * M - 1)];
+        if (stop != nullptr && *stop != 0) return false;
+        const int give = min(need, max(master.x - keep, 0));
+        if (give == 0) return false;  // the masters come by load: no later one of this source has anything to give
+        const int first = num_exports;
+        int move = give, q, slots, rest;
+        // an export is of at least min_tokens, or (dynamic) of ceil(what is still needed / the ranks that could still take part)
+        int times = dynamic_floor ? count : 1, floor = dynamic_floor ? need : max(min_tokens, 0);
+        Key best;
+        do {
+            best = max(fresh, top.key);
+            const int slack = static_cast<int>(best >> 7);
+            q = min(slack, move);
+            if (static_cast<Key>(q) * times < floor) {
+                // No later master of this source has more to give: where this one has made no export, or the best rank's slack is
+                // what is too small, the others fail in the same way. (A threshold with the static floor fails at its first source
+                // mostly; the walk over the other masters was the longest of the four builds.)
+                if (num_exports == first || q == slack) return false;
+                break;
+            }
+            const bool from_again = top.key > fresh;
+            slots = from_again ? top.slots : 0;
+            if (STORE) {
+                const int rank = 127 - static_cast<int>(best & 127);
+                plan[num_exports] = ExportEntry{q, (rank * Lp + M + slots) << 8 | rank};
+            }
+            ++num_exports;
+            times -= by_count;
+            floor -= by_count * q;
+            move -= q;
+            rest = slack - q;
+            waiting -= from_again ? 1 : 0;
+            used += from_again ? 0 : 1;
+            fresh = from_again ? fresh : fresh_next;
+            top.key = from_again ? top_next.key : top.key;
+            top.slots = from_again ? top_next.slots : top.slots;
+            top_next = again[waiting - 2];
+            fresh_next = fresh_keys[used + 1];
+        } while (move != 0);
+        if (num_exports > first) {
+            if (STORE) batches[num_batches++] = pack_batch(master.y, first, num_exports - first, source.y);
+            need -= give - move;
+            count -= num_exports - first;
+            if (move == 0 && rest > 0 && slots + 1 < R) {
+                const WaitingRank<Key> back{static_cast<Key>(rest) << 7 | (best & 127), slots + 1};
+                int place = waiting++;
+                for (; place > 0; --place) {
+                    const WaitingRank<Key> other = again[place - 1];
+                    if (other.key < back.key) break;
+                    again[place] = other;
                 }
-                const int move = min(need, avail);
-                int q[NS], next_slack[NS], next_meta[NS], next_upto[NS];
-                int first_out = kWarp * NS;  // the first slot from `head` on that takes nothing
-#pragma unroll
-                for (int s = NS - 1; s >= 0; --s) {
-                    const int slot = lane + kWarp * s;
-                    const int before = upto[s] - gone - slack[s];
-                    q[s] = min(slack[s], move - before);
-                    // dynamic floor: ceil(what is still needed / the ranks that could still take part)
-                    const bool enough = dynamic_floor ? static_cast<long long>(q[s]) * (end - slot) >= need - before : q[s] >= min_tokens;
-                    const unsigned out = __ballot_sync(kFullMask, slot >= head && !(slot < end && before < move && enough));
-                    if (out != 0u) first_out = kWarp * s + __ffs(out) - 1;
-                    next_slack[s] = __shfl_down_sync(kFullMask, slack[s], 1);
-                    next_meta[s] = __shfl_down_sync(kFullMask, meta[s], 1);
-                    next_upto[s] = __shfl_down_sync(kFullMask, upto[s], 1);
-                    if (s + 1 < NS) {
-                        const int a = __shfl_sync(kFullMask, slack[s + 1 < NS ? s + 1 : s], 0), b = __shfl_sync(kFullMask, meta[s + 1 < NS ? s + 1 : s], 0),
-                                  c = __shfl_sync(kFullMask, upto[s + 1 < NS ? s + 1 : s], 0);
-                        if (lane == kWarp - 1) {
-                            next_slack[s] = a;
-                            next_meta[s] = b;
-                            next_upto[s] = c;
-                        }
-                    }
-                }
-                const int exports = first_out - head;
-                if (exports == 0) continue;
-                const int last = first_out - 1;
-                const int last_upto = at(upto, last), last_meta = at(meta, last);
-                const int moved = min(last_upto - gone, move);
-                const int rest = last_upto - gone - moved;  // slack that the last rank keeps
-                const bool stays = rest > 0 && last_meta >> 8 > 1;
-                if (STORE) {
-                    if (num_exports + exports > kMaxExportsPerDomain) return false;
-                    const int e = __shfl_sync(kFullMask, my_e, pos);
-#pragma unroll
-                    for (int s = 0; s < NS; ++s) {
-                        const int slot = lane + kWarp * s;
-                        if (slot >= head && slot < first_out) plan[num_exports + slot - head] = ExportEntry{e, meta[s] & 255, q[s]};
-                    }
-                    if (lane == 0) export_sum[e] = moved;
-                    num_exports += exports;
-                }
-                int ahead = 0;  // slots that come in front of the last rank now
-#pragma unroll
-                for (int s = 0; s < NS; ++s) {
-                    const int slot = lane + kWarp * s;
-                    ahead += __popc(__ballot_sync(kFullMask, slot > last && slot < end && (slack[s] > rest || (slack[s] == rest &&
-                                                                                           (meta[s] & 255) < (last_meta & 255)))));
-                }
-#pragma unroll
-                for (int s = 0; s < NS; ++s) {
-                    const int slot = lane + kWarp * s;
-                    if (stays && slot >= last && slot < last + ahead) {
-                        slack[s] = next_slack[s];
-                        meta[s] = next_meta[s];
-                        upto[s] = next_upto[s] - rest;
-                    } else if (stays && slot == last + ahead) {
-                        slack[s] = rest;
-                        meta[s] = last_meta - 256;
-                    }
-                }
-                head = stays ? last : first_out;
-                gone = stays ? gone + moved : last_upto;
-                need -= moved;
+                again[place] = back;
+                top = again[waiting - 1];
+                top_next = again[waiting - 2];
+                ++count;
             }
         }
-        if (need > 0) return false;
+        if (need > 0) {
+            if (--left == 0) return false;
+            ++at_master;
+            master = follow;
+            continue;
+        }
+        // sources come by load: behind the first one that is not above the threshold there is none
+        if (++ord == G || (need = next_source.x - thr) <= 0) return true;
+        left = M;
+        source = next_source;
+        at_master = source.y * M;
+        master = next_first;
+        next_source = sm.source[min(ord + 1, G - 1)];
+        next_first = sm.masters[next_source.y * M];
     }
-    return true;
+}
+
+// `total`: of the domain's loads.
+template <bool STORE>
+__device__ bool warp_build_plan(const SolverSmem& sm, int buffer, int& num_batches, int thr, int total, int G, int M, int R,
+                                int min_tokens, bool allow_zero_master, bool dynamic_floor, int lane, const volatile int* stop = nullptr) {
+    num_batches = 0;
+    if (sm.source[0].x <= thr) return true;
+    // The excess has to fit the slack, and their difference is the sum of (load - threshold). Every export takes the same from
+    // both, so the slack left always covers the excess left.
+    if (total > static_cast<long long>(G) * thr) return false;
+    const bool narrow = thr < 1 << 24;  // (then a slack times a number of ranks is below 2^31, too)
+    int with_slack = 0;
+    __syncwarp();  // an earlier build of this warp has left its lists
+    for (int i0 = 0; i0 < G + 2; i0 += kWarp) {
+        const int i = i0 + lane;
+        const int2 sink = i < G ? sm.sink[i] : make_int2(thr, 0);
+        const int slack = max(thr - sink.x, 0);
+        const long long key = slack > 0 ? static_cast<long long>(slack) << 7 | (127 - sink.y) : -1;
+        if (i < G + 2) {
+            if (narrow) reinterpret_cast<int*>(sm.fresh + buffer * kMaxListed)[i] = static_cast<int>(key);
+            else sm.fresh[buffer * kMaxListed + i] = key;
+        }
+        with_slack += __popc(__ballot_sync(kFullMask, slack > 0));
+    }
+    __syncwarp();
+    int ok = 0, made = 0;
+    if (lane == 0) {
+        ok = narrow ? drain_sources<int, STORE>(sm, buffer, made, thr, with_slack, G, M, R, min_tokens, allow_zero_master, dynamic_floor, stop)
+                    : drain_sources<long long, STORE>(sm, buffer, made, thr, with_slack, G, M, R, min_tokens, allow_zero_master, dynamic_floor, stop);
+    }
+    num_batches = __shfl_sync(kFullMask, made, 0);
+    return __shfl_sync(kFullMask, ok, 0) != 0;
 }
 
 // x = a * b over d, for a, b >= 0 and d > 0: quotient and remainder. A float estimate of a quotient below 2^20 is off by
@@ -287,14 +294,30 @@ __device__ __forceinline__ void product_over(int a, int b, int d, int& quotient,
     }
 }
 
-// Split of this rank's tokens of one expert over the expert's replicas, as an inclusive
-// prefix. Semantics of csrc/kernels/placement.cu:1342-1481 / :669-786 of the reference.
-template <int MAXC>
-__device__ void build_rank_quota_prefix(const SolveArgs& a, int l_global, int C, int my_load, const int* phys,
-                                        const int* q, int Lp, int L) {
-    // phys[j] / q[j]: physical id and quota of replica j (j = 0 is the master), handed over from
-    // shared memory by the caller so that no plan row has to be read back from global memory.
+// Outputs of an expert with more than 32 replicas, by one thread: the split of this rank's tokens over the expert's replicas,
+// as an inclusive prefix. Semantics of csrc/kernels/placement.cu:1342-1481 / :669-786 of the reference. Not inlined: its
+// arrays and its code are for one rare case.
+__device__ __noinline__ void write_many_replicas(SolveArgs a, int first_rank, int e, int C, int load, int my_load, const ExportEntry* exports) {
+    constexpr int MAXC = kMaxRanksPerDomain;
+    const int Lp = a.M + a.R, L = a.N * a.M, l_global = first_rank * a.M + e;
     const int64_t row = static_cast<int64_t>(l_global) * a.D;
+    int phys[MAXC], q[MAXC];
+    phys[0] = (first_rank + e / a.M) * Lp + e % a.M;
+    q[0] = load;
+    for (int j = 1; j < C; ++j) {
+        phys[j] = first_rank * Lp + (exports[j - 1].place >> 8);
+        q[j] = exports[j - 1].quota;
+        q[0] -= q[j];
+        a.p2l[phys[j]] = l_global;
+        a.l2p[row + j] = phys[j];
+    }
+    int upto = 0;
+    for (int j = 0; j < C; ++j) {
+        upto += q[j];
+        a.quota[row + j] = q[j];
+        a.quota_prefix[row + j] = upto;
+        if (a.physical_loads != nullptr) a.physical_loads[phys[j]] = q[j];
+    }
     int host_rank[MAXC], my_alloc[MAXC];
     long long remainders[MAXC];
     for (int j = 0; j < C; ++j) {
@@ -389,7 +412,7 @@ __device__ void build_rank_quota_prefix(const SolveArgs& a, int l_global, int C,
     }
 }
 
-// The split of build_rank_quota_prefix for an expert with 2..32 replicas, by one warp: lane j
+// The same split for an expert with 2..32 replicas, by one warp: lane j
 // holds replica j on rank `host`, which has `own` tokens for the expert itself, and the sums and
 // arg-max searches are warp reductions. The hosts differ: an export never goes to a rank that
 // holds the expert already.
@@ -450,8 +473,7 @@ __device__ __forceinline__ void warp_rank_quota_prefix(const SolveArgs& a, int l
 
 // Solve one NVLink domain. All threads of the CTA must call it (blockDim.x >= 128,
 // multiple of 32). smem_raw must hold solver_smem_bytes(E, G) bytes, 16-byte aligned.
-template <int NS>
-__device__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, DeviceStatus* status) {
+__device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, DeviceStatus* status) {
     const int tid = threadIdx.x, nthreads = blockDim.x;
     const int warp = tid >> 5, lane = tid & 31;
     const int G = a.G, M = a.M, R = a.R, D = a.D;
@@ -464,69 +486,67 @@ __device__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, Dev
     };
     stamp(0);
 
-    // Every output of this domain as it is without replicas; run by `n` threads.
-    auto clear_outputs = [&](int t, int n) {
+    // Every output of this domain as it is without replicas (an expert then keeps all of this rank's tokens: every branch of
+    // the split reduces to that); run by `n` threads once the loads are in place. The experts with replicas are written over.
+    auto write_masters = [&](int t, int n) {
         for (int i = t; i < G * Lp; i += n) {
-            const int local = i % Lp;
-            a.p2l[domain_start_rank * Lp + i] = local < M ? domain_start_log + i / Lp * M + local : -1;
-            if (a.physical_loads != nullptr) a.physical_loads[domain_start_rank * Lp + i] = 0;
+            const int rank = i / Lp, local = i - rank * Lp, e = rank * M + local;
+            a.p2l[domain_start_rank * Lp + i] = local < M ? domain_start_log + e : -1;
+            if (a.physical_loads != nullptr) a.physical_loads[domain_start_rank * Lp + i] = local < M ? sm.loads[e] : 0;
         }
+        for (int e = t; e < E; e += n) a.lcnts[domain_start_log + e] = 1;
         const int64_t first = static_cast<int64_t>(domain_start_log) * D;
         auto master = [&](int e) { return (domain_start_rank + e / M) * Lp + e % M; };
         const uintptr_t align = reinterpret_cast<uintptr_t>(a.l2p) | reinterpret_cast<uintptr_t>(a.quota) |
                                 reinterpret_cast<uintptr_t>(a.quota_prefix) | reinterpret_cast<uintptr_t>(a.rank_quota_prefix);
         if (D % 4 == 0 && (align & 15u) == 0) {
             const int vecs = D / 4;
-            const int4 none = make_int4(0, 0, 0, 0);
             for (int i = t; i < E * vecs; i += n) {
                 const int e = i / vecs;
-                reinterpret_cast<int4*>(a.l2p + first)[i] = make_int4(i - e * vecs == 0 ? master(e) : -1, -1, -1, -1);
-                reinterpret_cast<int4*>(a.quota + first)[i] = none;
-                reinterpret_cast<int4*>(a.quota_prefix + first)[i] = none;
-                reinterpret_cast<int4*>(a.rank_quota_prefix + first)[i] = none;
+                const bool head = i - e * vecs == 0;
+                const int4 load = make_int4(head ? sm.loads[e] : 0, 0, 0, 0);
+                reinterpret_cast<int4*>(a.l2p + first)[i] = make_int4(head ? master(e) : -1, -1, -1, -1);
+                reinterpret_cast<int4*>(a.quota + first)[i] = load;
+                reinterpret_cast<int4*>(a.quota_prefix + first)[i] = load;
+                reinterpret_cast<int4*>(a.rank_quota_prefix + first)[i] = make_int4(head ? sm.my_loads[e] : 0, 0, 0, 0);
             }
         } else {
             for (int i = t; i < E * D; i += n) {
                 const int e = i / D;
-                a.l2p[first + i] = i - e * D == 0 ? master(e) : -1;
-                a.quota[first + i] = 0;
-                a.quota_prefix[first + i] = 0;
-                a.rank_quota_prefix[first + i] = 0;
+                const bool head = i - e * D == 0;
+                a.l2p[first + i] = head ? master(e) : -1;
+                a.quota[first + i] = head ? sm.loads[e] : 0;
+                a.quota_prefix[first + i] = head ? sm.loads[e] : 0;
+                a.rank_quota_prefix[first + i] = head ? sm.my_loads[e] : 0;
             }
         }
     };
-    for (int i = tid; i < E; i += nthreads) {
-        if (!a.preloaded) {
+    if (!a.preloaded) {
+        for (int i = tid; i < E; i += nthreads) {
             sm.loads[i] = __ldcg(a.global_loads + domain_start_log + i);
             sm.my_loads[i] = __ldcg(a.loads_per_rank + static_cast<int64_t>(a.my_rank) * L + domain_start_log + i);
         }
-        sm.expert_slot[i] = 1;
     }
-    if (tid == 0) sm.ctrl[kCtlNumExports] = 0;
     if (tid < kSolverProbeWarps) sm.ctrl[kCtlStop0 + tid] = 0;
     const bool do_search = (R > 0 && G > 1);
     stamp(1);
+    __syncthreads();
     if (!do_search) {
-        clear_outputs(tid, nthreads);
+        write_masters(tid, nthreads);
     } else {
-        __syncthreads();
-        for (int r = tid; r < G; r += nthreads) {
-            int sum = 0;
-#pragma unroll 8
-            for (int m = 0; m < M; ++m) sum += sm.loads[r * M + m];
-            sm.rank_load[r] = sum;
-            sm.next_slot[r] = 0;
-        }
-        for (int i = tid; i < E; i += nthreads) {  // each rank's masters by load descending, ties to the lower index
-            const int base = (i / M) * M;
+        // each rank's masters by load descending, ties to the lower index, and its load
+        for (int i = tid; i < E; i += nthreads) {
+            const int rank = i / M, base = rank * M;
             const int mine = sm.loads[i];
-            int pos = 0;
+            int pos = 0, sum = 0;
 #pragma unroll 8
             for (int j = base; j < base + M; ++j) {
                 const int other = sm.loads[j];
                 pos += (other > mine || (other == mine && j < i)) ? 1 : 0;
+                sum += other;
             }
-            sm.sorted_experts[base + pos] = i;
+            sm.masters[base + pos] = make_int2(mine, i);
+            if (i == base) sm.rank_load[rank] = sum;
         }
         __syncthreads();
         for (int i = tid; i < G; i += nthreads) {  // the ranks likewise
@@ -539,10 +559,10 @@ __device__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, Dev
                 below += other < mine ? 1 : 0;
                 equal += (other == mine && j < i) ? 1 : 0;
             }
-            sm.source_order[above + equal] = i;
-            sm.sink_order[below + equal] = i;
+            sm.source[above + equal] = make_int2(mine, i);
+            sm.sink[below + equal] = make_int2(mine, i);
         }
-        if (warp == 0) {
+        if (warp == kSolverProbeWarps - 1) {
             int total = 0, mx = 0;
             for (int r = lane; r < G; r += kWarp) {
                 total += sm.rank_load[r];
@@ -557,13 +577,14 @@ __device__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, Dev
             if (lane == 0) {
                 sm.ctrl[kCtlLo] = lo;
                 sm.ctrl[kCtlHi] = max(mx, lo);
+                sm.ctrl[kCtlTotal] = total;
             }
         }
         __syncthreads();
     }
     stamp(2);
     const bool allow0 = a.allow_zero_master != 0;
-    int winner = 0;  // the warp whose plan is taken
+    int winner = 0, num_batches = 0;  // the warp whose plan is taken
     if (do_search) {
         // The serial search is: up to three builds with the dynamic floor at rising thresholds; then one build at the
         // smallest threshold the capacities allow; then the probes below. The first four run at once, one warp each; one that
@@ -571,7 +592,6 @@ __device__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, Dev
         const int lo0 = sm.ctrl[kCtlLo], hi0 = sm.ctrl[kCtlHi];
         if (warp < kSolverProbeWarps) {
             int thr;
-            const volatile int* stop = sm.ctrl + kCtlStop0 + warp;
             const bool fast = warp < kSolverProbeWarps - 1;
             if (fast) {
                 const float eps = fmaxf(a.eps, 0.0f);
@@ -579,43 +599,33 @@ __device__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, Dev
                 const int step = max(1, (hi0 + 99) / 100);
                 for (int i = 0; i < warp; ++i) thr = min(hi0, thr + step);
             } else {
-                int lo = lo0, hi = hi0;
-                while (lo < hi && __shfl_sync(kFullMask, *stop, 0) == 0) {  // capacity bisection
-                    const int probe = lo + ((hi - lo) >> 1);
-                    int ex = 0, sl = 0;
-                    for (int r = lane; r < G; r += kWarp) {
-                        ex += max(sm.rank_load[r] - probe, 0);
-                        sl += max(probe - sm.rank_load[r], 0);
-                    }
-                    if (warp_sum(ex) <= warp_sum(sl)) hi = probe;
-                    else lo = probe + 1;
-                }
-                thr = lo;
+                // The smallest threshold from lo0 to hi0 whose excess fits its slack. Excess minus slack is the sum of
+                // (load - threshold): it fits from the mean load on. (The reference bisects, csrc/kernels/placement.cu:76-84.)
+                const int total = sm.ctrl[kCtlTotal];
+                thr = min(max(lo0, total / G + (total % G != 0 ? 1 : 0)), hi0);
             }
             int n = 0;
-            const bool ok = warp_build_plan<NS, true>(sm, sm.export_sum + warp * E, sm.plan + warp * kMaxExportsPerDomain, n, thr, E, G,
-                                                      M, R, a.min_tokens, allow0, fast, lane, stop);
+            const bool ok = warp_build_plan<true>(sm, warp, n, thr, sm.ctrl[kCtlTotal], G, M, R, a.min_tokens, allow0, fast, lane, sm.ctrl + kCtlStop0 + warp);
             if (ok && lane > warp && lane < kSolverProbeWarps) *(sm.ctrl + kCtlStop0 + lane) = 1;
             if (lane == 0) {
                 sm.ctrl[kCtlProbe0 + warp] = thr;
                 sm.ctrl[kCtlFeasible0 + warp] = ok ? 1 : 0;
-                sm.ctrl[kCtlExports0 + warp] = n;
+                sm.ctrl[kCtlBatches0 + warp] = n;
             }
         } else {
-            clear_outputs(tid - kSolverProbeWarps * kWarp, nthreads - kSolverProbeWarps * kWarp);
+            write_masters(tid - kSolverProbeWarps * kWarp, nthreads - kSolverProbeWarps * kWarp);
         }
-        if (nthreads == kSolverProbeWarps * kWarp) clear_outputs(tid, nthreads);
+        if (nthreads == kSolverProbeWarps * kWarp) write_masters(tid, nthreads);
         __syncthreads();
         winner = -1;
         for (int w = kSolverProbeWarps - 1; w >= 0; --w) {
             if (sm.ctrl[kCtlFeasible0 + w]) winner = w;
         }
-        const int precheck_thr = sm.ctrl[kCtlProbe0 + kSolverProbeWarps - 1];
-        const int num_exports = winner >= 0 ? sm.ctrl[kCtlExports0 + winner] : 0;
-        __syncthreads();  // everyone has read the four results
         if (winner >= 0) {
-            if (tid == 0) sm.ctrl[kCtlNumExports] = num_exports;
+            num_batches = sm.ctrl[kCtlBatches0 + winner];
         } else {
+            const int precheck_thr = sm.ctrl[kCtlProbe0 + kSolverProbeWarps - 1];
+            __syncthreads();  // everyone has read the four results
             if (tid == 0) sm.ctrl[kCtlLo] = min(precheck_thr + 1, hi0);
             winner = 0;
             __syncthreads();
@@ -642,8 +652,7 @@ __device__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, Dev
                 __syncthreads();
                 if (warp < kSolverProbeWarps && sm.ctrl[kCtlValid0 + warp]) {
                     int n = 0;
-                    const bool ok = warp_build_plan<NS, false>(sm, nullptr, nullptr, n, sm.ctrl[kCtlProbe0 + warp], E, G, M, R,
-                                                               a.min_tokens, allow0, false, lane);
+                    const bool ok = warp_build_plan<false>(sm, warp, n, sm.ctrl[kCtlProbe0 + warp], sm.ctrl[kCtlTotal], G, M, R, a.min_tokens, allow0, false, lane);
                     if (lane == 0) sm.ctrl[kCtlFeasible0 + warp] = ok ? 1 : 0;
                 }
                 __syncthreads();
@@ -682,144 +691,68 @@ __device__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, Dev
             }
             if (warp == 0) {
                 int n = 0;
-                const bool ok = warp_build_plan<NS, true>(sm, sm.export_sum, sm.plan, n, sm.ctrl[kCtlLo], E, G, M, R, a.min_tokens,
-                                                          allow0, false, lane);
+                const bool ok = warp_build_plan<true>(sm, 0, n, sm.ctrl[kCtlLo], sm.ctrl[kCtlTotal], G, M, R, a.min_tokens, allow0, false, lane);
                 if (lane == 0) {
-                    sm.ctrl[kCtlNumExports] = ok ? n : 0;
+                    sm.ctrl[kCtlNumBatches] = ok ? n : 0;
                     if (!ok) report_error(status, UEP_DEV_SOLVER_INFEASIBLE, sm.ctrl[kCtlLo]);
                 }
             }
+            __syncthreads();
+            num_batches = sm.ctrl[kCtlNumBatches];
         }
     }
-    __syncthreads();
-    const int32_t* export_sum = sm.export_sum + winner * E;
-    ExportEntry* plan = sm.plan + winner * kMaxExportsPerDomain;
-
     stamp(3);
-    // Emit: master quotas, then replicas in plan order. Two tables of the search are free by now
-    // and are reused: sorted_experts becomes "first plan entry of this expert" (an expert's
-    // exports are consecutive in the plan: they are all made while its one source rank is being
-    // drained), and another warp's sums become the list of experts that have replicas.
-    int* first_entry = sm.sorted_experts;
-    int* multi_list = sm.export_sum + (winner + 1) % kSolverProbeWarps * E;
-    for (int e = tid; e < E; e += nthreads) {
-        const int64_t row = static_cast<int64_t>(domain_start_log + e) * D;
-        const int master_quota = do_search ? (sm.loads[e] - export_sum[e]) : sm.loads[e];
-        a.quota[row] = master_quota;
-        if (a.physical_loads != nullptr) a.physical_loads[(domain_start_rank + e / M) * Lp + e % M] = master_quota;
-    }
-    if (tid == 0) sm.ctrl[kCtlMultiCount] = 0;
-    __syncthreads();
-    if (warp == 0) {
-        // 32 plan entries at a time: an entry's replica slot (and its target's redundant slot) is
-        // the counter left by the earlier chunks plus the number of lower lanes that name the same
-        // expert (the same target), which is exactly the creation order of a serial walk.
-        const int n = sm.ctrl[kCtlNumExports];
-        for (int base = 0; base < n; base += kWarp) {
-            const int k = base + lane;
-            const bool active = k < n;
-            const unsigned amask = __ballot_sync(kFullMask, active);
-            if (active) {
-                const ExportEntry entry = plan[k];
-                const unsigned same_e = __match_any_sync(amask, entry.expert_local);
-                const unsigned same_t = __match_any_sync(amask, entry.target_rank_local);
-                const unsigned below = (1u << lane) - 1u;
-                const int slot = sm.expert_slot[entry.expert_local] + __popc(same_e & below);
-                const int tslot = sm.next_slot[entry.target_rank_local] + __popc(same_t & below);
-                __syncwarp(amask);  // every lane has read the counters
-                if ((same_e >> lane) == 1u) sm.expert_slot[entry.expert_local] = slot + 1;  // highest lane of its group
-                if ((same_t >> lane) == 1u) sm.next_slot[entry.target_rank_local] = tslot + 1;
-                if (slot == 1) first_entry[entry.expert_local] = k;
-                const int l_global = domain_start_log + entry.expert_local;
-                const int64_t row = static_cast<int64_t>(l_global) * D;
-                const int phys = (domain_start_rank + entry.target_rank_local) * Lp + M + tslot;
-                if (slot >= D || phys >= (domain_start_rank + entry.target_rank_local + 1) * Lp) {
-                    report_error(status, UEP_DEV_BAD_PLAN, k);
-                } else {
-                    a.p2l[phys] = l_global;
-                    a.l2p[row + slot] = phys;
-                    a.quota[row + slot] = entry.quota;
-                    if (a.physical_loads != nullptr) a.physical_loads[phys] = entry.quota;
-                    plan[k].target_rank_local = phys;  // from here on the entry carries the physical id
+    // The experts with replicas, one per warp at a time, over what was written without them: lane 0 is the master, lane j the
+    // j-th export in the order of their creation.
+    const ExportEntry* plan = sm.plan + winner * kMaxExportsPerDomain;
+    const uint32_t* batches = sm.batches + winner * kMaxExportsPerDomain;
+    // Where there are warps enough, one writes an expert's rows and another one splits this rank's tokens.
+    const int warps = nthreads / kWarp, apart = 2 * num_batches <= warps ? 1 : 0;
+    for (int task = warp; task < num_batches << apart; task += warps) {
+        const uint32_t batch = batches[task >> apart];
+        const bool emits = apart == 0 || (task & 1) == 0, splits = apart == 0 || (task & 1) != 0;
+        const int e = batch & 511, first = batch >> 9 & 511, C = static_cast<int>(batch >> 18 & 127) + 1, home = batch >> 25;
+        const int l_global = domain_start_log + e;
+        const int64_t row = static_cast<int64_t>(l_global) * D;
+        const int my_load = sm.my_loads[e];
+        if (C > D) {
+            if (lane == 0) report_error(status, UEP_DEV_BAD_PLAN, l_global);
+            continue;
+        }
+        if (lane == 0 && emits) a.lcnts[l_global] = C;
+        if (C <= kWarp) {
+            const bool active = lane < C;
+            const ExportEntry entry = lane > 0 && active ? plan[first + lane - 1] : ExportEntry{0, 0};
+            const int moved = warp_sum(entry.quota);
+            const int host = domain_start_rank + (lane == 0 ? home : entry.place & 255);
+            const int q = lane == 0 ? sm.loads[e] - moved : entry.quota;
+            if (emits) {
+                const int phys = lane == 0 ? host * Lp + e - home * M : domain_start_rank * Lp + (entry.place >> 8);
+                const int prefix = warp_inclusive_scan(q, lane);
+                if (active) {
+                    a.quota[row + lane] = q;
+                    a.quota_prefix[row + lane] = prefix;
+                    if (a.physical_loads != nullptr) a.physical_loads[phys] = q;
+                    if (lane > 0) {
+                        a.p2l[phys] = l_global;
+                        a.l2p[row + lane] = phys;
+                    }
                 }
             }
-            __syncwarp();
+            if (splits) {
+                int own = 0;
+                if (a.locality && active) {
+                    const int64_t at = static_cast<int64_t>(host) * L + l_global;
+                    own = a.staged_loads != nullptr ? a.staged_loads[at] : __ldcg(a.loads_per_rank + at);
+                }
+                warp_rank_quota_prefix(a, l_global, C, my_load, active ? host : -1 - lane, q, own, lane);
+            }
+        } else if (lane == 0 && emits) {
+            write_many_replicas(a, domain_start_rank, e, C, sm.loads[e], my_load, plan + first);
         }
     }
     __syncthreads();
     stamp(4);
-    // Counts and prefixes. An expert without replicas keeps all of this rank's tokens (every
-    // branch of the split reduces to that), so one thread writes its row; the others go to the
-    // warps, one expert per warp at a time.
-    for (int e = tid; e < E; e += nthreads) {
-        const int l_global = domain_start_log + e;
-        const int64_t row = static_cast<int64_t>(l_global) * D;
-        const int C = min(sm.expert_slot[e], D);
-        a.lcnts[l_global] = C;
-        if (C == 1) {
-            a.quota_prefix[row] = do_search ? (sm.loads[e] - export_sum[e]) : sm.loads[e];
-            a.rank_quota_prefix[row] = sm.my_loads[e];
-        } else {
-            multi_list[atomicAdd(&sm.ctrl[kCtlMultiCount], 1)] = e;
-        }
-    }
-    __syncthreads();
-    const int n_multi = sm.ctrl[kCtlMultiCount];
-    // A lane's replica of the warp's next expert, its host's own load already on the way from L2.
-    struct Replica {
-        int e, C, phys, host, q, own;
-    };
-    auto fetch = [&](int idx) {
-        Replica r{-1, 0, 0, -1 - lane, 0, 0};
-        if (idx >= n_multi) return r;
-        r.e = multi_list[idx];
-        r.C = min(sm.expert_slot[r.e], D);
-        if (lane == 0) {
-            r.phys = (domain_start_rank + r.e / M) * Lp + r.e % M;
-            r.q = sm.loads[r.e] - export_sum[r.e];
-        } else if (lane < r.C && r.C <= kWarp) {
-            const ExportEntry entry = plan[first_entry[r.e] + lane - 1];
-            r.phys = entry.target_rank_local;
-            r.q = entry.quota;
-        }
-        if (lane < r.C && r.C <= kWarp) {
-            r.host = r.phys / Lp;
-            const int64_t at = static_cast<int64_t>(r.host) * L + domain_start_log + r.e;
-            if (a.locality) r.own = a.staged_loads != nullptr ? a.staged_loads[at] : __ldcg(a.loads_per_rank + at);
-        }
-        return r;
-    };
-    Replica next = fetch(warp);
-    for (int idx = warp; idx < n_multi; idx += nthreads / kWarp) {
-        const Replica r = next;
-        next = fetch(idx + nthreads / kWarp);
-        const int e = r.e, C = r.C;
-        const int l_global = domain_start_log + e;
-        const int64_t row = static_cast<int64_t>(l_global) * D;
-        if (C <= kWarp) {
-            const int qp = warp_inclusive_scan(r.q, lane);
-            if (lane < C) a.quota_prefix[row + lane] = qp;
-            warp_rank_quota_prefix(a, l_global, C, sm.my_loads[e], r.host, r.q, r.own, lane);
-        } else if (lane == 0) {  // more than 32 replicas: the serial version
-            int phys[kMaxRanksPerDomain], q[kMaxRanksPerDomain];
-            phys[0] = r.phys;
-            q[0] = r.q;
-            int prefix = 0;
-            const int first = first_entry[e];
-            for (int j = 0; j < C; ++j) {
-                if (j > 0) {
-                    phys[j] = plan[first + j - 1].target_rank_local;
-                    q[j] = plan[first + j - 1].quota;
-                }
-                prefix += q[j];
-                a.quota_prefix[row + j] = prefix;
-            }
-            build_rank_quota_prefix<kMaxRanksPerDomain>(a, l_global, C, sm.my_loads[e], phys, q, Lp, L);
-        }
-        __syncwarp();
-    }
-    __syncthreads();
-    stamp(5);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -837,8 +770,8 @@ __device__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, Dev
 // Shared memory: legacy_smem_bytes(E, G). All threads of the CTA must call it.
 // ---------------------------------------------------------------------------------------------
 __host__ __device__ inline size_t legacy_smem_bytes(int E, int G) {
-    return sizeof(double) * (static_cast<size_t>(E) + 2 * kMaxExportsPerDomain + solver_gpad(G)) +
-           sizeof(int32_t) * (3 * static_cast<size_t>(E) + 2 * kMaxExportsPerDomain + solver_gpad(G) + 8) +
+    return sizeof(double) * (static_cast<size_t>(E) + 2 * kMaxExportsPerDomain + solver_pad(G)) +
+           sizeof(int32_t) * (3 * static_cast<size_t>(E) + 2 * kMaxExportsPerDomain + solver_pad(G) + 8) +
            sizeof(uint32_t) * static_cast<size_t>(E) * solver_ns(G);
 }
 
@@ -850,13 +783,13 @@ __device__ __noinline__ void legacy_solve_domain(const SolveArgs& a, int domain,
     double* xkey = score + E;                                    // [512] extras: load per instance
     double* xkey_sorted = xkey + kMaxExportsPerDomain;           // [512]
     double* rank_load = xkey_sorted + kMaxExportsPerDomain;      // [Gpad]
-    int32_t* loads = reinterpret_cast<int32_t*>(rank_load + solver_gpad(G));  // [E]
+    int32_t* loads = reinterpret_cast<int32_t*>(rank_load + solver_pad(G));  // [E]
     int32_t* cnt = loads + E;                                    // [E] instances
     int32_t* placed = cnt + E;                                   // [E] instances placed so far (incl. master)
     int32_t* xid = placed + E;                                   // [512] extras: expert
     int32_t* xid_sorted = xid + kMaxExportsPerDomain;            // [512]
     int32_t* used = xid_sorted + kMaxExportsPerDomain;           // [Gpad] redundant slots used per rank
-    int32_t* ctl = used + solver_gpad(G);                        // [8]
+    int32_t* ctl = used + solver_pad(G);                        // [8]
     uint32_t* holds = reinterpret_cast<uint32_t*>(ctl + 8);      // [E][ns] ranks that hold the expert
 
     for (int i = tid; i < G * Lp; i += nthreads) {
@@ -1013,15 +946,13 @@ __device__ __noinline__ void legacy_solve_domain(const SolveArgs& a, int domain,
     __syncthreads();
 }
 
-__device__ inline void solve_domain_dispatch(const SolveArgs& a, int domain, char* smem_raw, DeviceStatus* status) {
+__device__ __forceinline__ void solve_domain_dispatch(const SolveArgs& a, int domain, char* smem_raw, DeviceStatus* status) {
     if (a.legacy) {
-        legacy_solve_domain(a, domain, smem_raw, status);
+        const SolveArgs copy = a;  // one whose address is taken, so that the other stays in registers and parameters
+        legacy_solve_domain(copy, domain, smem_raw, status);
         return;
     }
-    const int ns = solver_ns(a.G);
-    if (ns == 1) solve_domain<1>(a, domain, smem_raw, status);
-    else if (ns == 2) solve_domain<2>(a, domain, smem_raw, status);
-    else solve_domain<3>(a, domain, smem_raw, status);
+    solve_domain(a, domain, smem_raw, status);
 }
 
 }  // namespace uep
