@@ -74,13 +74,14 @@ struct PlanCall {
     int N, G, M, R, D;
     uep_solver_params params;
     uint64_t timeout_ns;
-    int ctas_per_rank;
+    int ctas_per_rank, threads;
     int withhold_rank;  // test hook: this rank does not publish its flags (-1: none)
     int legacy;         // 1: legacy placement solver (counts only; the reroute is then round-robin)
     unsigned long long* trace;  // optional: 8 globaltimer stamps per hosted rank (tuning aid), or null
 };
 cudaError_t launch_plan(const PlanCall& call, cudaStream_t stream);
 int plan_ctas_per_rank(int input_kind, int max_T, int K_or_L, int nlocal, int num_sms);
+int plan_threads(int input_kind, int max_T, int K_or_L, int ctas);
 
 struct SyncCall {
     GroupDev group;

@@ -641,6 +641,7 @@ int uep_update_placement(uep_manager* m, int layer_id, int input_kind, const voi
     call.params = m->cfg.solver;
     call.timeout_ns = m->timeout_ns;
     call.ctas_per_rank = plan_ctas_per_rank(input_kind, max_T, K_or_L, m->nlocal, m->num_sms);
+    call.threads = plan_threads(input_kind, max_T, K_or_L, call.ctas_per_rank);
     call.withhold_rank = m->withhold_rank;
     call.legacy = m->cfg.legacy_placement ? 1 : 0;
     call.trace = m->sync_trace ? m->sync_trace + 8 * 1000 : nullptr;  // the last rows of the trace buffer

@@ -33,14 +33,17 @@ namespace uep {
 
 namespace {
 
-constexpr int kPlanThreads = 256;
+constexpr int kPlanMaxThreads = 512;
+constexpr int kHistThreads = 256;
+constexpr int kIdLoads = 4;  // 16-byte loads of ids that a thread has in flight
 constexpr int kSolveThreads = 512;
 constexpr size_t kSolveMaxSmem = 200 * 1024;
 // Of the load matrix, where the plan kernel keeps it in shared memory: eight ranks of 512 experts, the largest group that one
 // device can host and the plan kernel could be timed with. The solver's own kernel has its SM to itself and takes what fits.
 constexpr size_t kPlanMatrixBytes = 16 * 1024;
 // Partial counts a thread asks for at once. The CTAs behind a rank's first one are shared by as many threads as an expert
-// can have: 17 of them (eight hosted ranks) by two threads up to 128 experts, one round each; other numbers take more rounds.
+// can have: 17 of them (eight hosted ranks) by two of 256 threads or four of 512 up to 128 experts, one round each; other numbers
+// take more rounds.
 constexpr int kPartBatch = 9;
 
 __device__ __forceinline__ void hist_add_swar(uint32_t word, int32_t* hist, int col) {
@@ -70,6 +73,7 @@ __device__ __noinline__ void histogram_slice(int input_kind, const void* input, 
             // plan kernel of eight ranks of 8192 x 128 took 28 us, against 22 with this and the present solver.)
             const int g = tid % groups;
             const int row_lane = tid / groups, row_lanes = nthreads / groups;
+            const int most = 8 * ceil_div_i(max(r1 - r0, 0), 8 * row_lanes);  // of a byte of a thread's sums
             uint4 acc = make_uint4(0, 0, 0, 0);
             int pending = 0;
             for (int r = row_lane < row_lanes ? r0 + row_lane : r1; r < r1; r += 8 * row_lanes) {
@@ -90,8 +94,23 @@ __device__ __noinline__ void histogram_slice(int input_kind, const void* input, 
                     pending = 0;
                 }
             }
-            hist_add_swar(acc.x, hist, g * 16); hist_add_swar(acc.y, hist, g * 16 + 4);
-            hist_add_swar(acc.z, hist, g * 16 + 8); hist_add_swar(acc.w, hist, g * 16 + 12);
+            if (groups <= 32 && (groups & (groups - 1)) == 0 && most * (32 / groups) < 256) {
+                // the lanes with the same columns add their bytes up first and then share the words: a fourth of the shared
+                // additions at 128 experts, and no two of a warp's at one address
+                for (int d = groups; d < 32; d <<= 1) {
+                    acc.x += __shfl_xor_sync(kFullMask, acc.x, d); acc.y += __shfl_xor_sync(kFullMask, acc.y, d);
+                    acc.z += __shfl_xor_sync(kFullMask, acc.z, d); acc.w += __shfl_xor_sync(kFullMask, acc.w, d);
+                }
+                const int subs = 32 / groups, sub = (tid & 31) / groups;
+                const uint32_t words[4] = {acc.x, acc.y, acc.z, acc.w};
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    if ((w & (subs - 1)) == sub) hist_add_swar(words[w], hist, g * 16 + 4 * w);
+                }
+            } else {
+                hist_add_swar(acc.x, hist, g * 16); hist_add_swar(acc.y, hist, g * 16 + 4);
+                hist_add_swar(acc.z, hist, g * 16 + 8); hist_add_swar(acc.w, hist, g * 16 + 12);
+            }
         } else {
             const int64_t begin = static_cast<int64_t>(r0) * L, end = static_cast<int64_t>(r1) * L;
             for (int64_t i = begin + tid; i < end; i += nthreads) {
@@ -110,15 +129,15 @@ __device__ __noinline__ void histogram_slice(int input_kind, const void* input, 
             if ((reinterpret_cast<uintptr_t>(ids) & 15u) == 0) {
                 const int64_t nvec = (end - begin) / 4;
                 const int4* v = reinterpret_cast<const int4*>(ids + begin);
-                for (int64_t j0 = 0; j0 < nvec; j0 += 4 * nthreads) {
-                    int4 x[4];
+                for (int64_t j0 = 0; j0 < nvec; j0 += kIdLoads * nthreads) {
+                    int4 x[kIdLoads];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
+                    for (int u = 0; u < kIdLoads; ++u) {
                         const int64_t j = j0 + tid + static_cast<int64_t>(u) * nthreads;
                         x[u] = j < nvec ? __ldg(v + j) : make_int4(-1, -1, -1, -1);
                     }
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
+                    for (int u = 0; u < kIdLoads; ++u) {
                         const int e[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
 #pragma unroll
                         for (int c = 0; c < 4; ++c) {
@@ -138,15 +157,15 @@ __device__ __noinline__ void histogram_slice(int input_kind, const void* input, 
             if ((reinterpret_cast<uintptr_t>(ids) & 15u) == 0) {
                 const int64_t nvec = (end - begin) / 2;
                 const longlong2* v = reinterpret_cast<const longlong2*>(ids + begin);
-                for (int64_t j0 = 0; j0 < nvec; j0 += 4 * nthreads) {
-                    longlong2 x[4];
+                for (int64_t j0 = 0; j0 < nvec; j0 += kIdLoads * nthreads) {
+                    longlong2 x[kIdLoads];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
+                    for (int u = 0; u < kIdLoads; ++u) {
                         const int64_t j = j0 + tid + static_cast<int64_t>(u) * nthreads;
                         x[u] = j < nvec ? __ldg(v + j) : make_longlong2(-1, -1);
                     }
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
+                    for (int u = 0; u < kIdLoads; ++u) {
                         if (x[u].x >= 0 && x[u].x < L) atomicAdd(hist + static_cast<int>(x[u].x), 1);
                         if (x[u].y >= 0 && x[u].y < L) atomicAdd(hist + static_cast<int>(x[u].y), 1);
                     }
@@ -161,7 +180,7 @@ __device__ __noinline__ void histogram_slice(int input_kind, const void* input, 
     }
 }
 
-__global__ void __launch_bounds__(kPlanThreads) histogram_kernel(int input_kind, const void* input, int T, int K_or_L,
+__global__ void __launch_bounds__(kHistThreads) histogram_kernel(int input_kind, const void* input, int T, int K_or_L,
                                                                  int L, int32_t* loads) {
     extern __shared__ __align__(128) char smem_raw[];
     int32_t* hist = reinterpret_cast<int32_t*>(smem_raw);
@@ -238,7 +257,7 @@ __host__ __device__ inline size_t plan_matrix_bytes(int N, int L) {
 }
 
 // The fused per-layer plan kernel. gridDim.x = nlocal * ctas_per_rank.
-__global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(PlanCall call) {
+__global__ void __launch_bounds__(kPlanMaxThreads, 1) plan_kernel(PlanCall call) {
     extern __shared__ __align__(128) char smem_raw[];
     __shared__ int s_timeout_peer;
     __shared__ uint64_t s_epoch;
@@ -331,10 +350,9 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(PlanCall call) {
     const int slot = static_cast<int>(epoch & 1ull);
     const int me = group.my_rank[local];
     if (me != call.withhold_rank) {
-        for (int idx = tid; idx < N * L; idx += blockDim.x) {
-            const int p = idx / L, i = idx % L;
-            st_relaxed_sys_u64(group.gather_of(p) + (static_cast<int64_t>(slot) * N + me) * Lpad + i,
-                               tag_word(tag, static_cast<uint32_t>(hist[i])));
+        for (int i = tid; i < L; i += blockDim.x) {
+            const uint64_t word = tag_word(tag, static_cast<uint32_t>(hist[i]));
+            for (int p = 0; p < N; ++p) st_relaxed_sys_u64(group.gather_of(p) + (static_cast<int64_t>(slot) * N + me) * Lpad + i, word);
         }
     }
 
@@ -424,6 +442,14 @@ std::atomic<int64_t> g_launches{0};
 
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
+// Twice the threads where a CTA's slice of the input would be several rounds of loads. Steps of eight ranks with 256 and 512
+// threads (us): 16384 int64 tokens of 256 experts (57 KB a CTA) 114.5 and 112.1, 8192 bool rows of 128 (57 KB) 69.6 and 69.2;
+// 8192 int32 tokens (15 KB) 31.3 and 32.0, 33 tokens 17.1 and 17.9.
+int plan_threads(int input_kind, int max_T, int K_or_L, int ctas) {
+    const int64_t bytes = static_cast<int64_t>(max_T) * K_or_L * (input_kind == 0 ? 1 : (input_kind == 1 ? 4 : 8));
+    return bytes > static_cast<int64_t>(ctas) * 16 * 1024 ? kPlanMaxThreads : kPlanMaxThreads / 2;
+}
+
 int plan_ctas_per_rank(int input_kind, int max_T, int K_or_L, int nlocal, int num_sms) {
     const int64_t bytes = static_cast<int64_t>(max_T) * K_or_L * (input_kind == 0 ? 1 : (input_kind == 1 ? 4 : 8));
     int ctas = static_cast<int>((bytes + 16 * 1024 - 1) / (16 * 1024));
@@ -437,7 +463,7 @@ cudaError_t launch_plan(const PlanCall& call, cudaStream_t stream) {
     const size_t smem = plan_smem_bytes(call.N, call.G, call.M);
     cudaError_t e = allow_smem(reinterpret_cast<const void*>(plan_kernel), smem);
     if (e != cudaSuccess) return e;
-    const dim3 grid(call.nlocal * call.ctas_per_rank), block(kPlanThreads);
+    const dim3 grid(call.nlocal * call.ctas_per_rank), block(call.threads);
     count_launch();
     if (call.nlocal > 1) {
         // ranks wait for each other inside the kernel: co-residency is required
@@ -472,7 +498,7 @@ static int histogram_common(int kind, const void* input, int T, int K_or_L, int 
     const size_t smem = sizeof(int32_t) * L;
     UEP_CUDA_TRY(allow_smem(reinterpret_cast<const void*>(histogram_kernel), smem));
     count_launch();
-    histogram_kernel<<<ctas, kPlanThreads, smem, stream>>>(kind, input, T, K_or_L, L, loads);
+    histogram_kernel<<<ctas, kHistThreads, smem, stream>>>(kind, input, T, K_or_L, L, loads);
     UEP_CUDA_TRY(cudaGetLastError());
     return UEP_OK;
 }
