@@ -1,0 +1,36 @@
+"""Plans of hosted groups whose inputs are large: 512 threads a CTA, bytes of the bool map summed in a warp before they are counted, and
+a CTA that rehearses the solver on a problem of its own beside them. The widths of the map decide how the lanes share the sums; the
+smallest group is smaller than the rehearsal's. Loads and plan against the CPU oracle, bit-exact, twice in a row."""
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import uep_oracle as O
+from ultra_ep_b200 import sim
+
+pytestmark = pytest.mark.gpu
+
+# ranks, masters, slots, tokens: the input of a rank is more than 16 KB for each CTA that the plan has for it
+SHAPES = [(2, 1, 1, 300000), (2, 8, 1, 40000), (3, 32, 2, 9000), (5, 5, 2, 25000), (7, 16, 0, 5000), (8, 4, 2, 12000), (8, 64, 8, 1500)]
+
+
+@pytest.mark.parametrize("N,M,R,T", SHAPES)
+def test_large_maps(native_lib, cuda_device, N, M, R, T):
+    L = N * M
+    group = sim.SimGroup(sim.make_config(N, M, R, 1, fc1_numel=64, fc2_numel=64, is_train=True, sim=True))
+    for seed in (1, 2):
+        gen = torch.Generator(device=cuda_device).manual_seed(seed)
+        popular = torch.rand(L, generator=gen, device=cuda_device) ** 4
+        maps = [torch.rand((T - 17 * r, L), generator=gen, device=cuda_device) < popular for r in range(N)]
+        maps[0][:, 0] = True  # a byte of every row: the largest sums
+        group.update_placement(0, maps)
+        torch.cuda.synchronize()
+        loads = np.stack([m.sum(0).cpu().numpy() for m in maps]).astype(np.int32)
+        for r in range(N):
+            want = O.solve_placement(loads, M, R, N, r)
+            got = group.plan(r, 0)
+            for f in ("p2l", "l2p", "lcnts", "quota", "quota_prefix", "rank_quota_prefix"):
+                assert np.array_equal(got[f].cpu().numpy().reshape(-1), getattr(want, f).reshape(-1)), (seed, r, f)
+    group.check_status()
+    group.destroy()

@@ -17,6 +17,7 @@ constexpr int kReduceSegments = 16;  // a replica's gradient is released for zer
 constexpr unsigned long long kReduceFlagRadix = 64;  // progress word = epoch * radix + segments done
 
 constexpr int kPlanMaxCtas = 32;  // CTAs of one rank in the plan kernel
+constexpr int kPlanMaxThreads = 512;
 
 // Where the group's buffers are. By value in the kernels' parameters, so that the first load of a kernel is of data and not
 // of a pointer to it (each of the two is a miss: the tables were last read a layer ago). Fixed once connected. With a table
@@ -75,6 +76,7 @@ struct PlanCall {
     uep_solver_params params;
     uint64_t timeout_ns;
     int ctas_per_rank, threads;
+    int rehearsal;      // 1: one more CTA, which runs the solver on a problem of its own (plan.cu)
     int withhold_rank;  // test hook: this rank does not publish its flags (-1: none)
     int legacy;         // 1: legacy placement solver (counts only; the reroute is then round-robin)
     unsigned long long* trace;  // optional: 8 globaltimer stamps per hosted rank (tuning aid), or null
