@@ -38,6 +38,7 @@
 // then the forward chunks: a CTA that waits (bounded) for a ready flag waits for a chunk that a
 // running CTA, on this or another device, is already sending.
 
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <type_traits>
@@ -48,7 +49,7 @@ namespace uep {
 
 namespace {
 
-constexpr int kSyncThreads = 128;
+constexpr int kSyncThreads = 128, kSyncMaxThreads = 256;  // launch_weight_sync
 constexpr int kMaxSends = kMaxExportsPerDomain;  // replicas of one rank's masters never exceed G*R <= 512
 constexpr int kMaxFwd = 64;                       // replica slots of the hosted ranks that may forward
 constexpr int kMaxRelayReplicas = 16;
@@ -91,27 +92,13 @@ struct SyncShared {
     int s_unit;
     unsigned long long epoch;
     int shard_tiles[4];
-    int w_a[kSyncThreads / 32], w_r[kSyncThreads / 32];
-    int rank_out[kMaxPeers], rank_in[kMaxPeers];  // adaptive relay: experts each rank sends / receives under this plan
+    int w_a[kSyncMaxThreads / 32], w_r[kSyncMaxThreads / 32];
     short rep_start[kMaxExpertsPerDomain + 1];  // [n_active+1] offsets into dst_*
-    short order[kMaxExpertsPerDomain];          // hand-out order of the active masters: relayed ones first
-    unsigned char relay_r[kMaxExpertsPerDomain];  // [n_active] 0: direct, else the replica count of a relayed expert
-    unsigned char relay_of[kMaxExpertsPerDomain]; // [logical expert of the domain] the same for every expert of the plan
-    unsigned char reps_of[kMaxExpertsPerDomain];  // [logical expert of the domain] its replica count (capped at 255)
     // Addresses are resolved once per CTA: the issuing thread must not chase pointers
     // through global memory for every 32 KiB tile.
     const uint8_t* src[kMaxExpertsPerDomain][4];  // [n_active][shard] master shard base
     uint8_t* dst_weight[kMaxSends];               // replica slot base in the peer's weight buffer (null: skip)
     uint8_t* dst_scale[kMaxSends];                // replica slot base in the peer's scale buffer
-    uint64_t* dst_flags[kMaxSends];               // that slot's row of ready flags on the peer (relay)
-    // forward entries: one per local replica slot that holds a relayed expert
-    uint8_t* fwd_src_w[kMaxFwd];        // the slot itself
-    uint8_t* fwd_src_s[kMaxFwd];
-    const uint64_t* fwd_flags[kMaxFwd]; // its row of ready flags
-    unsigned char fwd_r[kMaxFwd], fwd_k[kMaxFwd], fwd_lr[kMaxFwd];
-    short fwd_dst_start[kMaxFwd + 1];
-    uint8_t* fwd_dst_w[kMaxFwdDst];
-    uint8_t* fwd_dst_s[kMaxFwdDst];
     __align__(8) uint64_t bars[8];
     // State of the issuing thread's ring, kept here rather than in its local memory: the kernels that run
     // next to this one evict the L1 lines a stack frame lives in, and every miss would sit on the critical
@@ -124,6 +111,22 @@ struct SyncShared {
     uint64_t* ring_flag[8];  // ready flag to raise once that stage's tile is stored (last tile of a chunk)
     uint64_t* owed[8];       // ready flag owed for the k-th stored tile, slot k % stages
     int ring_valid[8];
+    // ---- from here on for the relay-capable kernel only: the other one is launched without room for it (22 KB, which the kernels
+    // that run next to it can use)
+    uint64_t* dst_flags[kMaxSends];               // that slot's row of ready flags on the peer (relay)
+    int rank_out[kMaxPeers], rank_in[kMaxPeers];  // adaptive relay: experts each rank sends / receives under this plan
+    short order[kMaxExpertsPerDomain];          // hand-out order of the active masters: relayed ones first
+    unsigned char relay_r[kMaxExpertsPerDomain];  // [n_active] 0: direct, else the replica count of a relayed expert
+    unsigned char relay_of[kMaxExpertsPerDomain]; // [logical expert of the domain] the same for every expert of the plan
+    unsigned char reps_of[kMaxExpertsPerDomain];  // [logical expert of the domain] its replica count (capped at 255)
+    // forward entries: one per local replica slot that holds a relayed expert
+    uint8_t* fwd_src_w[kMaxFwd];        // the slot itself
+    uint8_t* fwd_src_s[kMaxFwd];
+    const uint64_t* fwd_flags[kMaxFwd]; // its row of ready flags
+    unsigned char fwd_r[kMaxFwd], fwd_k[kMaxFwd], fwd_lr[kMaxFwd];
+    short fwd_dst_start[kMaxFwd + 1];
+    uint8_t* fwd_dst_w[kMaxFwdDst];
+    uint8_t* fwd_dst_s[kMaxFwdDst];
 };
 
 template <int kSyncTile>
@@ -163,7 +166,7 @@ __device__ void copy_plain(const uint8_t* src, uint8_t* dst, int bytes, bool str
 // its per-tile bookkeeping (the kernel runs once per layer from a cold instruction cache, and the one
 // issuing thread per CTA is on the critical path of every tile).
 template <int kSyncTile, int kSyncStages, bool kRelay>
-__global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call) {
+__global__ void __launch_bounds__(kSyncMaxThreads) weight_sync_kernel(SyncCall call) {
     extern __shared__ __align__(128) char smem_raw[];  // kSyncStages * kSyncTile, then SyncShared
     SyncShared& sm = *reinterpret_cast<SyncShared*>(smem_raw + static_cast<size_t>(kSyncStages) * kSyncTile);
     uint64_t* bars = sm.bars;
@@ -446,7 +449,7 @@ __global__ void __launch_bounds__(kSyncThreads) weight_sync_kernel(SyncCall call
         __syncthreads();
         if (tid == 0) {
             int nf = 0;
-            for (int w = 0; w < kSyncThreads / 32; ++w) nf += sm.w_a[w];
+            for (int w = 0; w < static_cast<int>(blockDim.x) / 32; ++w) nf += sm.w_a[w];
             sm.fwd_dst_start[0] = 0;
             for (int e = 0; e < nf; ++e) sm.fwd_dst_start[e + 1] = static_cast<short>(sm.fwd_dst_start[e + 1] + sm.fwd_dst_start[e]);
             sm.n_fwd = nf;
@@ -925,15 +928,15 @@ const SyncGeometry& sync_geometry() {
     return *chosen;
 }
 
-size_t sync_smem_bytes(const SyncGeometry& g) {
-    return static_cast<size_t>(g.stages) * g.tile_kib * 1024 + sizeof(SyncShared);
+size_t sync_smem_bytes(const SyncGeometry& g, bool relay) {
+    return static_cast<size_t>(g.stages) * g.tile_kib * 1024 + (relay ? sizeof(SyncShared) : offsetof(SyncShared, dst_flags));
 }
 
 }  // namespace
 
 int weight_sync_max_ctas_per_rank(int nlocal, int num_sms) {
     // CTAs that fit one wave: shared memory bounds the CTAs per SM; hosted ranks share the device
-    const size_t smem = sync_smem_bytes(sync_geometry()) + 1024;
+    const size_t smem = sync_smem_bytes(sync_geometry(), true) + 1024;
     int per_sm = static_cast<int>((227 * 1024) / smem);
     per_sm = per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm);
     const int per = num_sms * per_sm / (nlocal > 0 ? nlocal : 1);
@@ -944,18 +947,20 @@ int weight_sync_tile_bytes() { return sync_geometry().tile_kib * 1024; }
 
 cudaError_t launch_weight_sync(const SyncCall& call, cudaStream_t stream) {
     const SyncGeometry& g = sync_geometry();
-    const size_t smem = sync_smem_bytes(g);
     // two ranks: an expert has at most one replica away from its master, nothing can be relayed; the
     // compact kernel is the same on every rank because N is
     const bool relay = call.relay_min_replicas > 0 && call.N > 2;
     const void* fn = relay ? g.fn_relay : g.fn;
+    const size_t smem = sync_smem_bytes(g, relay);
     cudaError_t e = allow_smem(fn, smem);
     if (e != cudaSuccess) return e;
     // Hosted ranks pool their work over all CTAs. Without relaying, the only waits are those of the
     // last CTA, on flags that peers on other devices write. With relaying, CTAs that forward wait for
     // CTAs that send; when both are in this launch (ranks hosted together) they must be co-resident,
     // which a cooperative launch guarantees.
-    const dim3 grid(call.nlocal * call.ctas_per_rank), block(kSyncThreads);
+    // A thread per master of the hosted ranks asks for all that its set-up reads at once; a second round of masters is a chain of
+    // three more round trips (eight ranks, 256 experts: set-up 6.5 us, 128 experts 3.6).
+    const dim3 grid(call.nlocal * call.ctas_per_rank), block(call.nlocal * call.M > kSyncThreads ? kSyncMaxThreads : kSyncThreads);
     count_launch();
     SyncCall copy = call;
     void* args[] = {&copy};
