@@ -200,31 +200,43 @@ __device__ __forceinline__ bool dense_fast_path(const uint8_t* map, const void* 
            ((reinterpret_cast<uintptr_t>(map) | reinterpret_cast<uintptr_t>(scratch)) & 15u) == 0;
 }
 
-__global__ void __launch_bounds__(kRerouteThreads) dense_count_kernel(Batch<DenseFwdArgs> batch, int L, int behind_plan) {
-    if (behind_plan) pdl_wait();  // ahead of every read: the kernel in front may still be writing the map
+// TILES tiles a CTA: one or four (launch_dense_forward).
+template <int TILES>
+__global__ void __launch_bounds__(kRerouteThreads) dense_count_kernel(Batch<DenseFwdArgs> batch, int L, int wait_first) {
+    if (wait_first) pdl_wait();  // ahead of every read: the kernel in front may still be writing the map
     pdl_launch_dependents();  // the scatter kernel may start its prologue now
-    extern __shared__ __align__(128) char smem_raw[];  // [pad4(L)] counts, one byte each
+    extern __shared__ __align__(128) char smem_raw[];  // [TILES][pad4(L)] counts, one byte each
+    constexpr int kThreads = kRerouteThreads / TILES;  // of a tile: whole warps
     const DenseFwdArgs& a = batch.a[blockIdx.y];
     const int T = a.T;
-    const int tile = blockIdx.x;
-    const int r0 = tile * kDenseTileRows, r1 = min(r0 + kDenseTileRows, T);
-    if (r0 >= T) return;
-    uint8_t* counts = reinterpret_cast<uint8_t*>(a.scratch) + static_cast<int64_t>(tile) * L;
+    const int first = blockIdx.x * TILES * kDenseTileRows;
+    if (first >= T) return;
+    const int mine = threadIdx.x / kThreads, tid = threadIdx.x % kThreads, words = pad4(L) / 4;
+    const int r0 = min(first + mine * kDenseTileRows, T), rows = min(T - r0, kDenseTileRows);
     const uint8_t* src = a.map + static_cast<int64_t>(r0) * L;
-    uint32_t* cnt = reinterpret_cast<uint32_t*>(smem_raw);
-    for (int i = threadIdx.x; i < pad4(L) / 4; i += blockDim.x) cnt[i] = 0;
+    uint32_t* cnt = reinterpret_cast<uint32_t*>(smem_raw) + mine * words;
+    for (int i = tid; i < words; i += kThreads) cnt[i] = 0;
     __syncthreads();
     // a byte never exceeds 64, so the packed adds below cannot carry into the next byte
-    if (dense_fast_path(a.map, a.scratch, L)) {
+    const bool fast = dense_fast_path(a.map, a.scratch, L);
+    if (fast) {
+        constexpr int kFlight = TILES == 1 ? 4 : 8;
         const int G = L / 16;
-        // vector i of the tile covers row i / G, columns 16 * (i % G) ..; blockDim is a multiple of G, so a
+        // vector i of the tile covers row i / G, columns 16 * (i % G) ..; kThreads is a multiple of G, so a
         // thread always meets the same column group and adds the 0/1 bytes of its rows as packed words
-        const int nvec = (r1 - r0) * G;
+        const int nvec = rows * G;
         uint4 acc = make_uint4(0, 0, 0, 0);
-#pragma unroll 4
-        for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
-            const uint4 v = ld_global_nc_v4(src + static_cast<int64_t>(i) * 16);
-            acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+        for (int i = tid; i < nvec; i += kFlight * kThreads) {
+            uint4 v[kFlight];
+#pragma unroll
+            for (int u = 0; u < kFlight; ++u) {
+                const int at = i + u * kThreads;
+                v[u] = at < nvec ? ld_global_nc_v4(src + static_cast<int64_t>(at) * 16) : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < kFlight; ++u) {
+                acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w;
+            }
         }
         // lanes with the same column group inside the warp
         for (int d = G; d < 32; d <<= 1) {
@@ -236,22 +248,25 @@ __global__ void __launch_bounds__(kRerouteThreads) dense_count_kernel(Batch<Dens
             atomicAdd(cnt + lane * 4 + 0, acc.x); atomicAdd(cnt + lane * 4 + 1, acc.y);
             atomicAdd(cnt + lane * 4 + 2, acc.z); atomicAdd(cnt + lane * 4 + 3, acc.w);
         }
-        __syncthreads();
-        for (int i = threadIdx.x; i < L / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(counts)[i] = cnt[i];
-        return;
-    }
-    const int quads = pad4(L) / 4;
-    const int load_bytes = map_load_bytes(src, L);
-    for (int i = threadIdx.x; i < quads * kDenseSegs; i += blockDim.x) {
-        const int s = i / quads, q = i - s * quads;
-        const uint32_t b = segment_bits_any(load_bytes, src, r1 - r0, L, s, q);
-        uint32_t packed = 0;
+    } else {
+        const int load_bytes = map_load_bytes(src, L);
+        for (int i = tid; i < words * kDenseSegs; i += kThreads) {
+            const int s = i / words, q = i - s * words;
+            const uint32_t b = segment_bits_any(load_bytes, src, rows, L, s, q);
+            uint32_t packed = 0;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) packed |= static_cast<uint32_t>(__popc((b >> (8 * k)) & 0xFFu)) << (8 * k);
-        if (packed) atomicAdd(cnt + q, packed);
+            for (int k = 0; k < 4; ++k) packed |= static_cast<uint32_t>(__popc((b >> (8 * k)) & 0xFFu)) << (8 * k);
+            if (packed) atomicAdd(cnt + q, packed);
+        }
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < L; e += blockDim.x) counts[e] = reinterpret_cast<const uint8_t*>(cnt)[e];
+    if (rows <= 0) return;
+    uint8_t* counts = reinterpret_cast<uint8_t*>(a.scratch) + static_cast<int64_t>(r0 / kDenseTileRows) * L;
+    if (fast) {
+        for (int i = tid; i < words; i += kThreads) reinterpret_cast<uint32_t*>(counts)[i] = cnt[i];
+    } else {
+        for (int e = tid; e < L; e += kThreads) counts[e] = reinterpret_cast<const uint8_t*>(cnt)[e];
+    }
 }
 
 // Adds the counts of the tiles in front of `tile` to base_of[L] (shared memory, zeroed), all threads of the CTA.
@@ -1191,21 +1206,26 @@ cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int
     if (L > kDenseMaxExperts) return cudaErrorInvalidValue;
     const dim3 grid(dense_tiles(max_T), b.n);
     const int chunk = P > kDenseMaxChunkCols ? kDenseMaxChunkCols : P;
-    const size_t smem_count = pad4(L), smem = dense_smem_bytes(L, chunk);
+    const int sms = std::max(device_sm_count(), 1);
+    // Four tiles a CTA where one each would be more CTAs than the device holds at once and four tiles are one round of loads.
+    // Plan and pair of eight ranks, tile by tile and by four (us): 8192 x 128 51.7 and 49.6; 4096 x 128 34.1 and 34.8, 8192 x 256
+    // (two rounds) 71.6 and 72.7.
+    const bool by_four = L <= 128 && static_cast<int64_t>(grid.x) * b.n > 6 * sms;
+    const auto count = by_four ? dense_count_kernel<4> : dense_count_kernel<1>;
+    const size_t smem_count = static_cast<size_t>(pad4(L)) * (by_four ? 4 : 1), smem = dense_smem_bytes(L, chunk);
     behind_plan = behind_plan && b.n > 1 && pdl_enabled();
     cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(dense_scatter_kernel), smem);
     if (e != cudaSuccess) return e;
-    e = ensure_smem_attr(reinterpret_cast<const void*>(dense_count_kernel), smem_count);
+    e = ensure_smem_attr(reinterpret_cast<const void*>(count), smem_count);
     if (e != cudaSuccess) return e;
     count_launch(2);
-    e = launch_dependent(dense_count_kernel, grid, dim3(kRerouteThreads), smem_count, stream, behind_plan, b, L, behind_plan ? 1 : 0);
+    e = launch_dependent(count, dim3(by_four ? (grid.x + 3) / 4 : grid.x, b.n), dim3(kRerouteThreads), smem_count, stream, behind_plan, b, L, behind_plan ? 1 : 0);
     if (e != cudaSuccess) return e;
     // With one rank per launch the pair is latency-bound and the overlap pays; a launch that hosts several ranks
     // fills the device with the first kernel alone, and early CTAs of the second only get in its way, unless they do nothing
     // but wait.
     const bool overlap = (b.n == 1 || behind_plan) && pdl_enabled();
     // up to two tiles per SM the kernel is a chain of phases: more threads shorten each
-    const int sms = std::max(device_sm_count(), 1);
     const int threads = static_cast<int64_t>(grid.x) * b.n <= 2 * sms ? kDenseMaxThreads : kRerouteThreads;
     return launch_dependent(dense_scatter_kernel, grid, dim3(threads), smem, stream, overlap, b, L, P, D, quota_mode,
                             interleave, chunk, overlap ? 1 : 0, behind_plan ? 1 : 0);
