@@ -499,6 +499,7 @@ dense_scatter_kernel(Batch<DenseFwdArgs> batch, int L, int P, int D, int quota_m
         }
     }
     if (overlapped) pdl_wait();
+    pdl_launch_dependents();
     sum_earlier_tiles(a, L, tile, s.base);
     __syncthreads();
 
@@ -646,7 +647,8 @@ __host__ __device__ inline size_t dense_bwd_smem_bytes(int L, int P, int tile_ro
     return static_cast<size_t>(pad4(L)) * (kStagedReps + 1) * 4 + static_cast<size_t>(tile_rows) * (L + P) + 16;
 }
 __global__ void __launch_bounds__(kDenseBwdThreads, 8)
-dense_backward_tile_kernel(Batch<DenseBwdArgs> batch, int L, int P, int D, int tile_rows) {
+dense_backward_tile_kernel(Batch<DenseBwdArgs> batch, int L, int P, int D, int tile_rows, int wait_first) {
+    if (wait_first) pdl_wait();  // ahead of every read
     const DenseBwdArgs& a = batch.a[blockIdx.y];
     const int first = static_cast<int>(blockIdx.x) * tile_rows;
     const int rows = min(a.T - first, tile_rows);
@@ -747,8 +749,8 @@ __global__ void __launch_bounds__(kRerouteThreads) dense_backward_kernel(Batch<D
 
 // ---------------------------------------------------------------------------- sparse
 template <typename IdT>
-__global__ void __launch_bounds__(kOrdThreads) sparse_count_kernel(Batch<SparseArgs> batch, int K, int L, int tile_entries, int behind_plan) {
-    if (behind_plan) pdl_wait();  // ahead of every read: the kernel in front may still be writing the ids
+__global__ void __launch_bounds__(kOrdThreads) sparse_count_kernel(Batch<SparseArgs> batch, int K, int L, int tile_entries, int wait_first) {
+    if (wait_first) pdl_wait();  // ahead of every read: the kernel in front may still be writing the ids
     pdl_launch_dependents();      // the reroute kernel may start on everything that does not read the table
     const SparseArgs& a = batch.a[blockIdx.y];
     count_tile<IdT>(static_cast<const IdT*>(a.ids), static_cast<int64_t>(a.T) * K, L, false, tile_entries, a.scratch);
@@ -764,9 +766,10 @@ size_t sparse_smem_bytes(int L, bool rows_staged) {
 // CTA occupies.
 template <int EPT, typename IdT>
 __global__ void __launch_bounds__(kOrdThreads) __maxnreg__(EPT > 4 ? 96 : 64)
-sparse_reroute_kernel(Batch<SparseArgs> batch, int ctas, int K, int L, int D, int interleave, int rows_staged, int use_table, int behind_plan) {
+sparse_reroute_kernel(Batch<SparseArgs> batch, int ctas, int K, int L, int D, int interleave, int rows_staged, int use_table, int wait_first) {
     extern __shared__ __align__(128) char smem_raw[];
-    if (behind_plan) pdl_wait();  // ahead of every read
+    if (wait_first) pdl_wait();  // ahead of every read
+    pdl_launch_dependents();
     const SparseArgs& a = batch.a[blockIdx.y];
     const IdT* ids = static_cast<const IdT*>(a.ids);
     IdT* out = static_cast<IdT*>(a.out);
@@ -1214,17 +1217,21 @@ cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int
     const auto count = by_four ? dense_count_kernel<4> : dense_count_kernel<1>;
     const size_t smem_count = static_cast<size_t>(pad4(L)) * (by_four ? 4 : 1), smem = dense_smem_bytes(L, chunk);
     behind_plan = behind_plan && b.n > 1 && pdl_enabled();
+    // The first kernel may be on its SMs when whatever is in front of it ends, too: it waits before its first read. (One rank, 8191
+    // tokens of 256 experts, sparse, dense and backward one behind the other: 34.1 us with ordinary launches, 32.8 like this. Of
+    // several ranks only behind a plan, as internal.h says.)
+    const bool early = behind_plan || (b.n == 1 && pdl_enabled());
     cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(dense_scatter_kernel), smem);
     if (e != cudaSuccess) return e;
     e = ensure_smem_attr(reinterpret_cast<const void*>(count), smem_count);
     if (e != cudaSuccess) return e;
     count_launch(2);
-    e = launch_dependent(count, dim3(by_four ? (grid.x + 3) / 4 : grid.x, b.n), dim3(kRerouteThreads), smem_count, stream, behind_plan, b, L, behind_plan ? 1 : 0);
+    e = launch_dependent(count, dim3(by_four ? (grid.x + 3) / 4 : grid.x, b.n), dim3(kRerouteThreads), smem_count, stream, early, b, L, early ? 1 : 0);
     if (e != cudaSuccess) return e;
     // With one rank per launch the pair is latency-bound and the overlap pays; a launch that hosts several ranks
     // fills the device with the first kernel alone, and early CTAs of the second only get in its way, unless they do nothing
     // but wait.
-    const bool overlap = (b.n == 1 || behind_plan) && pdl_enabled();
+    const bool overlap = early;
     // up to two tiles per SM the kernel is a chain of phases: more threads shorten each
     const int threads = static_cast<int64_t>(grid.x) * b.n <= 2 * sms ? kDenseMaxThreads : kRerouteThreads;
     return launch_dependent(dense_scatter_kernel, grid, dim3(threads), smem, stream, overlap, b, L, P, D, quota_mode,
@@ -1259,8 +1266,9 @@ cudaError_t launch_dense_backward(const Batch<DenseBwdArgs>& b, int L, int P, in
     if (tiles) {
         cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(dense_backward_tile_kernel), smem);
         if (e != cudaSuccess) return e;
-        dense_backward_tile_kernel<<<dim3((max_T + rows - 1) / rows, b.n), kDenseBwdThreads, smem, stream>>>(b, L, P, D, rows);
-        return cudaGetLastError();
+        const bool early = b.n == 1 && pdl_enabled();
+        return launch_dependent(dense_backward_tile_kernel, dim3((max_T + rows - 1) / rows, b.n), dim3(kDenseBwdThreads), smem, stream, early, b, L, P,
+                                D, rows, early ? 1 : 0);
     }
     int64_t blocks = (static_cast<int64_t>(max_T) * L / 4 + kRerouteThreads - 1) / kRerouteThreads + 1;
     const int64_t cap = std::max(sms * 16 / b.n, 1);
@@ -1365,6 +1373,7 @@ template <typename IdT>
 static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L, int D, int interleave, bool beside_sync,
                                        bool behind_plan, cudaStream_t stream) {
     behind_plan = behind_plan && b.n > 1 && pdl_enabled();
+    const bool early = behind_plan || (b.n == 1 && pdl_enabled());  // as in launch_dense_forward
     int64_t max_n = 0;
     bool in_place = false;
     for (int i = 0; i < b.n; ++i) {
@@ -1393,18 +1402,18 @@ static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L,
     const OrdGrid g = ord_grid(max_n, L, b.n, in_place, kOrdThreads, false);
     // One rank per launch is latency-bound and the overlap with the count kernel pays; several ranks fill the device
     // with the first kernel alone (behind a plan the second one is there early and does nothing but wait).
-    const bool overlap = behind_plan || (g.table && b.n == 1 && pdl_enabled());
+    const bool overlap = early;
     if (g.table) {
         cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(sparse_count_kernel<IdT>), sizeof(int32_t) * L);
         if (e != cudaSuccess) return e;
         count_launch();
-        e = launch_dependent(sparse_count_kernel<IdT>, dim3(g.ctas * g.clusters, b.n), dim3(kOrdThreads), sizeof(int32_t) * L, stream, behind_plan, b,
-                             K, L, g.per_lane * kOrdThreads, behind_plan ? 1 : 0);
+        e = launch_dependent(sparse_count_kernel<IdT>, dim3(g.ctas * g.clusters, b.n), dim3(kOrdThreads), sizeof(int32_t) * L, stream, early, b,
+                             K, L, g.per_lane * kOrdThreads, early ? 1 : 0);
         if (e != cudaSuccess) return e;
     }
     return with_lanes(g, [&](auto per_lane) {
         return launch_clusters(sparse_reroute_kernel<decltype(per_lane)::value, IdT>, g, b.n, smem, stream, overlap, b, g.ctas, K, L, D,
-                               interleave, staged, g.table ? 1 : 0, behind_plan ? 1 : 0);
+                               interleave, staged, g.table ? 1 : 0, behind_plan || (early && !g.table) ? 1 : 0);
     });
 }
 
