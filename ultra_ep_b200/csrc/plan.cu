@@ -36,7 +36,7 @@ namespace {
 constexpr int kHistThreads = 256;
 constexpr int kIdLoads = 4;  // 16-byte loads of ids that a thread has in flight
 constexpr int kSolveThreads = 512;
-constexpr size_t kSolveMaxSmem = 200 * 1024;
+constexpr size_t kSolveMaxSmem = 220 * 1024;
 // Of the load matrix, where the plan kernel keeps it in shared memory: eight ranks of 512 experts, the largest group that one
 // device can host and the plan kernel could be timed with. The solver's own kernel has its SM to itself and takes what fits.
 constexpr size_t kPlanMatrixBytes = 16 * 1024;
@@ -201,9 +201,9 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(SolveArgs a, in
     if (reduce_loads) {
         // Total load of this domain's experts over all ranks, and this rank's own, straight to where the solver keeps
         // them. The rows are shared by all the threads an expert can have, 16 loads of each in flight.
-        const SolverSmem sm = carve_solver_smem(smem_raw, E, a.G);
+        const SolverSmem sm = carve_solver_smem(smem_raw, E, a.G, a.R);
         const int parts = max(static_cast<int>(blockDim.x) / E, 1);
-        int32_t* matrix = reinterpret_cast<int32_t*>(smem_raw + solver_smem_bytes(E, a.G));
+        int32_t* matrix = reinterpret_cast<int32_t*>(smem_raw + solver_smem_bytes(E, a.G, a.R));
         for (int i = threadIdx.x; i < E; i += blockDim.x) sm.loads[i] = 0;
         __syncthreads();
         for (int i = threadIdx.x; i < E * parts; i += blockDim.x) {
@@ -265,13 +265,13 @@ constexpr int kRehearsalRanks = 4, kRehearsalMasters = 2, kRehearsalSlots = 2, k
 constexpr int kRehearsalExperts = kRehearsalRanks * kRehearsalMasters;
 constexpr int kRehearsalPhysical = kRehearsalRanks * (kRehearsalMasters + kRehearsalSlots);
 __host__ __device__ inline size_t rehearsal_smem_bytes() {
-    return solver_smem_bytes(kRehearsalExperts, kRehearsalRanks) +
+    return solver_smem_bytes(kRehearsalExperts, kRehearsalRanks, kRehearsalSlots) +
            sizeof(int32_t) * (kRehearsalRanks * kRehearsalExperts + 4 * kRehearsalExperts * kRehearsalD + kRehearsalExperts + 2 * kRehearsalPhysical);
 }
 // Two ranks above the mean and two below, so that every step of the solver is taken: an expert with two exports, ranks that come back.
 __device__ __forceinline__ void rehearsal_args(const PlanCall& call, char* smem_raw, SolveArgs& a) {
-    const SolverSmem sm = carve_solver_smem(smem_raw, kRehearsalExperts, kRehearsalRanks);
-    int32_t* matrix = reinterpret_cast<int32_t*>(smem_raw + solver_smem_bytes(kRehearsalExperts, kRehearsalRanks));
+    const SolverSmem sm = carve_solver_smem(smem_raw, kRehearsalExperts, kRehearsalRanks, kRehearsalSlots);
+    int32_t* matrix = reinterpret_cast<int32_t*>(smem_raw + solver_smem_bytes(kRehearsalExperts, kRehearsalRanks, kRehearsalSlots));
     for (int i = threadIdx.x; i < kRehearsalExperts; i += blockDim.x) {
         const int load = (i & 1) != 0 ? 100 : 6000 >> 2 * (i >> 2) * (i >> 1);  // 6000, 6000, 375, 93
         sm.loads[i] = load;
@@ -398,9 +398,9 @@ __device__ __forceinline__ bool gather_loads(const PlanCall& call, int local, in
 
     // With one domain the solver finds the loads in shared memory where it keeps them: its loads are where hist was.
     const bool preload = call.G == N && !call.legacy;
-    const SolverSmem solver_sm = carve_solver_smem(smem_raw, L, N);
+    const SolverSmem solver_sm = carve_solver_smem(smem_raw, L, N, call.R);
     const bool staged = preload && plan_matrix_bytes(N, L) > 0;
-    int32_t* matrix = reinterpret_cast<int32_t*>(smem_raw + solver_smem_bytes(L, N));
+    int32_t* matrix = reinterpret_cast<int32_t*>(smem_raw + solver_smem_bytes(L, N, call.R));
     __syncthreads();  // hist has been read by every thread
     stamp(1);
     // 3. collect every rank's row (bounded), expose the matrix, reduce. A thread owns one expert:
@@ -486,8 +486,8 @@ __global__ void __launch_bounds__(kPlanMaxThreads, 1) plan_kernel(PlanCall call)
     if (!rehearses && call.trace != nullptr && threadIdx.x == 0) call.trace[local * 8 + 4] = global_timer_ns();
 }
 
-size_t plan_smem_bytes(int N, int G, int M) {
-    const size_t solver = std::max(solver_smem_bytes(G * M, G) + (G == N ? plan_matrix_bytes(N, N * M) : 0), legacy_smem_bytes(G * M, G));
+size_t plan_smem_bytes(int N, int G, int M, int R) {
+    const size_t solver = std::max(solver_smem_bytes(G * M, G, R) + (G == N ? plan_matrix_bytes(N, N * M) : 0), legacy_smem_bytes(G * M, G));
     const size_t hist = sizeof(int32_t) * static_cast<size_t>(N) * M;
     return std::max(std::max(solver, hist), rehearsal_smem_bytes()) + 16;
 }
@@ -516,7 +516,7 @@ int plan_ctas_per_rank(int input_kind, int max_T, int K_or_L, int nlocal, int nu
 }
 
 cudaError_t launch_plan(const PlanCall& call, cudaStream_t stream) {
-    const size_t smem = plan_smem_bytes(call.N, call.G, call.M);
+    const size_t smem = plan_smem_bytes(call.N, call.G, call.M, call.R);
     cudaError_t e = allow_smem(reinterpret_cast<const void*>(plan_kernel), smem);
     if (e != cudaSuccess) return e;
     const dim3 grid(call.nlocal * call.ctas_per_rank + call.rehearsal), block(call.threads);
@@ -602,7 +602,7 @@ int uep_solve_placement(const int32_t* loads_per_rank, int32_t* global_loads_out
     a.preloaded = 0;
     a.staged_loads = nullptr;
     a.trace = nullptr;
-    size_t smem = solver_smem_bytes(nvl_ranks * M, nvl_ranks) + 16;
+    size_t smem = solver_smem_bytes(nvl_ranks * M, nvl_ranks, R) + 16;
     // with one domain the solver also keeps the load matrix it adds up, where that fits
     const size_t matrix = sizeof(int32_t) * num_ranks * num_ranks * static_cast<size_t>(M);
     const int staged = nvl_ranks == num_ranks && smem + matrix <= kSolveMaxSmem ? 1 : 0;

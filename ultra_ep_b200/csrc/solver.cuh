@@ -65,12 +65,10 @@ struct SolveArgs {
 constexpr int kSolverProbeWarps = 4;
 constexpr int kMaxListed = kMaxRanksPerDomain + 2;  // ranks of a list, and its end
 
-// Control words in shared memory.
-enum SolverCtrl {
-    kCtlLo = 0, kCtlHi, kCtlTotal, kCtlStop0, kCtlNumBatches = kCtlStop0 + kSolverProbeWarps, kCtlSmallRange,
-    kCtlProbe0, kCtlValid0 = kCtlProbe0 + kSolverProbeWarps, kCtlFeasible0 = kCtlValid0 + kSolverProbeWarps,
-    kCtlBatches0 = kCtlFeasible0 + kSolverProbeWarps, kCtlCount = kCtlBatches0 + kSolverProbeWarps
-};
+constexpr int kSolverBuffers = 2 * kSolverProbeWarps;  // plans: one the search may end with, and those of the present round
+
+// Control words in shared memory. kCtlBuilt0: of a buffer's plan, 0 if it is not feasible, else its batches plus one.
+enum SolverCtrl { kCtlLo = 0, kCtlHi, kCtlTotal, kCtlStop0, kCtlBuilt0 = kCtlStop0 + kSolverProbeWarps, kCtlCount = kCtlBuilt0 + kSolverBuffers };
 static_assert(kCtlCount <= 32, "control words");
 
 struct SolverSmem {
@@ -80,23 +78,24 @@ struct SolverSmem {
     int2* source;        // [G] {load, rank}, largest load first, ties to the lower rank
     int2* sink;          // [G] {load, rank}, smallest first, likewise
     int32_t* rank_load;  // [G]
-    ExportEntry* plan;   // [4][kMaxExportsPerDomain] of the four warps that build plans
-    uint32_t* batches;   // [4][kMaxExportsPerDomain]
+    ExportEntry* plan;   // [kSolverBuffers][slots]
+    uint32_t* batches;   // [kSolverBuffers][slots]
     long long* fresh;    // [4][kMaxListed] lists of ranks of the four warps
     longlong2* again;    // [4][kMaxListed]
     int* ctrl;           // [kCtlCount]
+    int slots;           // redundant slots of the domain, the most exports of a plan (rounded up)
 };
 
 __host__ __device__ inline int solver_ns(int G) { return (G + 31) / 32; }
 __host__ __device__ inline int solver_pad(int n) { return (n + 3) / 4 * 4; }
-__host__ __device__ inline size_t solver_smem_bytes(int E, int G) {
+__host__ __device__ inline size_t solver_smem_bytes(int E, int G, int R) {
     return sizeof(int32_t) * (4 * static_cast<size_t>(solver_pad(E)) + 5 * solver_pad(G)) +
-           kSolverProbeWarps * ((sizeof(ExportEntry) + sizeof(uint32_t)) * kMaxExportsPerDomain + 3 * sizeof(long long) * kMaxListed) +
-           sizeof(int) * 32;
+           kSolverBuffers * (sizeof(ExportEntry) + sizeof(uint32_t)) * solver_pad(G * R) +
+           kSolverProbeWarps * 3 * sizeof(long long) * kMaxListed + sizeof(int) * 32;
 }
 
-__device__ inline SolverSmem carve_solver_smem(char* raw, int E, int G) {
-    const int ep = solver_pad(E), gp = solver_pad(G);
+__device__ inline SolverSmem carve_solver_smem(char* raw, int E, int G, int R) {
+    const int ep = solver_pad(E), gp = solver_pad(G), slots = solver_pad(G * R);
     SolverSmem s;
     int32_t* p = reinterpret_cast<int32_t*>(raw);
     s.loads = p; p += ep;
@@ -105,11 +104,12 @@ __device__ inline SolverSmem carve_solver_smem(char* raw, int E, int G) {
     s.source = reinterpret_cast<int2*>(p); p += 2 * gp;
     s.sink = reinterpret_cast<int2*>(p); p += 2 * gp;
     s.rank_load = p; p += gp;
-    s.plan = reinterpret_cast<ExportEntry*>(p); p += kSolverProbeWarps * 2 * kMaxExportsPerDomain;
-    s.batches = reinterpret_cast<uint32_t*>(p); p += kSolverProbeWarps * kMaxExportsPerDomain;
+    s.plan = reinterpret_cast<ExportEntry*>(p); p += kSolverBuffers * 2 * slots;
+    s.batches = reinterpret_cast<uint32_t*>(p); p += kSolverBuffers * slots;
     s.again = reinterpret_cast<longlong2*>(p); p += kSolverProbeWarps * 4 * kMaxListed;
     s.fresh = reinterpret_cast<long long*>(p); p += kSolverProbeWarps * 2 * kMaxListed;
     s.ctrl = reinterpret_cast<int*>(p);
+    s.slots = slots;
     return s;
 }
 
@@ -142,13 +142,13 @@ static_assert(sizeof(WaitingRank<long long>) == 16, "two words of two");
 // lists in the lanes of a warp and all exports of an expert in one step: ballots, shuffles and the branches around them were
 // 1000 cycles an expert.) There are never more exports than redundant slots (kMaxExportsPerDomain).
 // Key: int where slack << 7 fits, long long beyond. `stop`: raised by a warp whose result makes this build pointless.
-template <typename Key, bool STORE>
-__device__ bool drain_sources(const SolverSmem& sm, int buffer, int& num_batches, int thr, int with_slack, int G, int M, int R,
+template <typename Key>
+__device__ bool drain_sources(const SolverSmem& sm, int warp, int buffer, int& num_batches, int thr, int with_slack, int G, int M, int R,
                               int min_tokens, bool allow_zero_master, bool dynamic_floor, const volatile int* stop) {
-    ExportEntry* const plan = sm.plan + buffer * kMaxExportsPerDomain;
-    uint32_t* const batches = sm.batches + buffer * kMaxExportsPerDomain;
-    const Key* const fresh_keys = reinterpret_cast<const Key*>(sm.fresh + buffer * kMaxListed);
-    WaitingRank<Key>* const again = reinterpret_cast<WaitingRank<Key>*>(sm.again + buffer * kMaxListed) + 2;  // [-2], [-1]: its end
+    ExportEntry* const plan = sm.plan + buffer * sm.slots;
+    uint32_t* const batches = sm.batches + buffer * sm.slots;
+    const Key* const fresh_keys = reinterpret_cast<const Key*>(sm.fresh + warp * kMaxListed);
+    WaitingRank<Key>* const again = reinterpret_cast<WaitingRank<Key>*>(sm.again + warp * kMaxListed) + 2;  // [-2], [-1]: its end
     const WaitingRank<Key> none{Key(-1), 0};
     again[-2] = none;
     again[-1] = none;
@@ -186,11 +186,8 @@ __device__ bool drain_sources(const SolverSmem& sm, int buffer, int& num_batches
             }
             const bool from_again = top.key > fresh;
             slots = from_again ? top.slots : 0;
-            if (STORE) {
-                const int rank = 127 - static_cast<int>(best & 127);
-                plan[num_exports] = ExportEntry{q, (rank * Lp + M + slots) << 8 | rank};
-            }
-            ++num_exports;
+            const int rank = 127 - static_cast<int>(best & 127);
+            plan[num_exports++] = ExportEntry{q, (rank * Lp + M + slots) << 8 | rank};
             times -= by_count;
             floor -= by_count * q;
             move -= q;
@@ -204,7 +201,7 @@ __device__ bool drain_sources(const SolverSmem& sm, int buffer, int& num_batches
             fresh_next = fresh_keys[used + 1];
         } while (move != 0);
         if (num_exports > first) {
-            if (STORE) batches[num_batches++] = pack_batch(master.y, first, num_exports - first, source.y);
+            batches[num_batches++] = pack_batch(master.y, first, num_exports - first, source.y);
             need -= give - move;
             count -= num_exports - first;
             if (move == 0 && rest > 0 && slots + 1 < R) {
@@ -238,9 +235,8 @@ __device__ bool drain_sources(const SolverSmem& sm, int buffer, int& num_batches
     }
 }
 
-// `total`: of the domain's loads.
-template <bool STORE>
-__device__ bool warp_build_plan(const SolverSmem& sm, int buffer, int& num_batches, int thr, int total, int G, int M, int R,
+// By warp `warp` of the first four, into plan buffer `buffer`. `total`: of the domain's loads.
+__device__ bool warp_build_plan(const SolverSmem& sm, int warp, int buffer, int& num_batches, int thr, int total, int G, int M, int R,
                                 int min_tokens, bool allow_zero_master, bool dynamic_floor, int lane, const volatile int* stop = nullptr) {
     num_batches = 0;
     if (sm.source[0].x <= thr) return true;
@@ -256,16 +252,16 @@ __device__ bool warp_build_plan(const SolverSmem& sm, int buffer, int& num_batch
         const int slack = max(thr - sink.x, 0);
         const long long key = slack > 0 ? static_cast<long long>(slack) << 7 | (127 - sink.y) : -1;
         if (i < G + 2) {
-            if (narrow) reinterpret_cast<int*>(sm.fresh + buffer * kMaxListed)[i] = static_cast<int>(key);
-            else sm.fresh[buffer * kMaxListed + i] = key;
+            if (narrow) reinterpret_cast<int*>(sm.fresh + warp * kMaxListed)[i] = static_cast<int>(key);
+            else sm.fresh[warp * kMaxListed + i] = key;
         }
         with_slack += __popc(__ballot_sync(kFullMask, slack > 0));
     }
     __syncwarp();
     int ok = 0, made = 0;
     if (lane == 0) {
-        ok = narrow ? drain_sources<int, STORE>(sm, buffer, made, thr, with_slack, G, M, R, min_tokens, allow_zero_master, dynamic_floor, stop)
-                    : drain_sources<long long, STORE>(sm, buffer, made, thr, with_slack, G, M, R, min_tokens, allow_zero_master, dynamic_floor, stop);
+        ok = narrow ? drain_sources<int>(sm, warp, buffer, made, thr, with_slack, G, M, R, min_tokens, allow_zero_master, dynamic_floor, stop)
+                    : drain_sources<long long>(sm, warp, buffer, made, thr, with_slack, G, M, R, min_tokens, allow_zero_master, dynamic_floor, stop);
     }
     num_batches = __shfl_sync(kFullMask, made, 0);
     return __shfl_sync(kFullMask, ok, 0) != 0;
@@ -472,7 +468,7 @@ __device__ __forceinline__ void warp_rank_quota_prefix(const SolveArgs& a, int l
 }
 
 // Solve one NVLink domain. All threads of the CTA must call it (blockDim.x >= 128,
-// multiple of 32). smem_raw must hold solver_smem_bytes(E, G) bytes, 16-byte aligned.
+// multiple of 32). smem_raw must hold solver_smem_bytes(E, G, R) bytes, 16-byte aligned.
 __device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, DeviceStatus* status) {
     const int tid = threadIdx.x, nthreads = blockDim.x;
     const int warp = tid >> 5, lane = tid & 31;
@@ -480,7 +476,7 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, cha
     const int E = G * M, Lp = M + R, L = a.N * M;
     const int domain_start_rank = domain * G;
     const int domain_start_log = domain_start_rank * M;
-    SolverSmem sm = carve_solver_smem(smem_raw, E, G);
+    SolverSmem sm = carve_solver_smem(smem_raw, E, G, R);
     auto stamp = [&](int slot) {
         if (a.trace != nullptr && tid == 0) a.trace[slot] = global_timer_ns();
     };
@@ -584,128 +580,89 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, cha
     }
     stamp(2);
     const bool allow0 = a.allow_zero_master != 0;
-    int winner = 0, num_batches = 0;  // the warp whose plan is taken
+    int winner = 0, num_batches = 0;  // the buffer whose plan is taken
     if (do_search) {
         // The serial search is: up to three builds with the dynamic floor at rising thresholds; then one build at the
         // smallest threshold the capacities allow; then the probes below. The first four run at once, one warp each; one that
         // succeeds stops those behind it.
-        const int lo0 = sm.ctrl[kCtlLo], hi0 = sm.ctrl[kCtlHi];
+        const int lo0 = sm.ctrl[kCtlLo], hi0 = sm.ctrl[kCtlHi], total = sm.ctrl[kCtlTotal];
+        // The smallest threshold from lo0 to hi0 whose excess fits its slack. Excess minus slack is the sum of (load - threshold):
+        // it fits from the mean load on. (The reference bisects, csrc/kernels/placement.cu:76-84.)
+        const int fitting = min(max(lo0, total / G + (total % G != 0 ? 1 : 0)), hi0);
+        auto build = [&](int buffer, int thr, bool dynamic_floor, const volatile int* stop) {
+            int n = 0;
+            const bool ok = warp_build_plan(sm, warp, buffer, n, thr, total, G, M, R, a.min_tokens, allow0, dynamic_floor, lane, stop);
+            if (lane == 0) sm.ctrl[kCtlBuilt0 + buffer] = ok ? n + 1 : 0;
+            return ok;
+        };
+        auto first_feasible = [&](int buffer0) {  // of a round, -1: none; its batches go to num_batches
+            int first = -1;
+#pragma unroll
+            for (int w = kSolverProbeWarps - 1; w >= 0; --w) {
+                const int built = sm.ctrl[kCtlBuilt0 + buffer0 + w];
+                if (built != 0) {
+                    first = w;
+                    num_batches = built - 1;
+                }
+            }
+            return first;
+        };
         if (warp < kSolverProbeWarps) {
-            int thr;
             const bool fast = warp < kSolverProbeWarps - 1;
+            int thr = fitting;
             if (fast) {
                 const float eps = fmaxf(a.eps, 0.0f);
                 thr = max(static_cast<int>(ceilf(__fmul_rn(static_cast<float>(lo0), __fadd_rn(1.0f, eps)))), lo0);
                 const int step = max(1, (hi0 + 99) / 100);
                 for (int i = 0; i < warp; ++i) thr = min(hi0, thr + step);
-            } else {
-                // The smallest threshold from lo0 to hi0 whose excess fits its slack. Excess minus slack is the sum of
-                // (load - threshold): it fits from the mean load on. (The reference bisects, csrc/kernels/placement.cu:76-84.)
-                const int total = sm.ctrl[kCtlTotal];
-                thr = min(max(lo0, total / G + (total % G != 0 ? 1 : 0)), hi0);
             }
-            int n = 0;
-            const bool ok = warp_build_plan<true>(sm, warp, n, thr, sm.ctrl[kCtlTotal], G, M, R, a.min_tokens, allow0, fast, lane, sm.ctrl + kCtlStop0 + warp);
-            if (ok && lane > warp && lane < kSolverProbeWarps) *(sm.ctrl + kCtlStop0 + lane) = 1;
-            if (lane == 0) {
-                sm.ctrl[kCtlProbe0 + warp] = thr;
-                sm.ctrl[kCtlFeasible0 + warp] = ok ? 1 : 0;
-                sm.ctrl[kCtlBatches0 + warp] = n;
-            }
+            if (build(warp, thr, fast, sm.ctrl + kCtlStop0 + warp) && lane > warp && lane < kSolverProbeWarps) *(sm.ctrl + kCtlStop0 + lane) = 1;
         } else {
             write_masters(tid - kSolverProbeWarps * kWarp, nthreads - kSolverProbeWarps * kWarp);
         }
         if (nthreads == kSolverProbeWarps * kWarp) write_masters(tid, nthreads);
         __syncthreads();
-        winner = -1;
-        for (int w = kSolverProbeWarps - 1; w >= 0; --w) {
-            if (sm.ctrl[kCtlFeasible0 + w]) winner = w;
-        }
-        if (winner >= 0) {
-            num_batches = sm.ctrl[kCtlBatches0 + winner];
-        } else {
-            const int precheck_thr = sm.ctrl[kCtlProbe0 + kSolverProbeWarps - 1];
-            __syncthreads();  // everyone has read the four results
-            if (tid == 0) sm.ctrl[kCtlLo] = min(precheck_thr + 1, hi0);
-            winner = 0;
-            __syncthreads();
-            while (true) {
-                if (sm.ctrl[kCtlLo] >= sm.ctrl[kCtlHi]) break;
-                __syncthreads();  // everyone has read lo/hi before thread 0 rewrites the probe table
-                if (tid == 0) {
-                    const int lo = sm.ctrl[kCtlLo], hi = sm.ctrl[kCtlHi];
-                    const int range = hi - lo;
-                    const int small_range = (range <= kSolverProbeWarps) ? 1 : 0;
-                    sm.ctrl[kCtlSmallRange] = small_range;
-                    for (int w = 0; w < kSolverProbeWarps; ++w) {
-                        if (small_range) {
-                            sm.ctrl[kCtlProbe0 + w] = lo + w;
-                            sm.ctrl[kCtlValid0 + w] = (lo + w < hi) ? 1 : 0;
-                        } else {
-                            sm.ctrl[kCtlProbe0 + w] =
-                                lo + static_cast<int>((static_cast<long long>(range) * (w + 1)) / (kSolverProbeWarps + 1));
-                            sm.ctrl[kCtlValid0 + w] = 1;
-                        }
-                        sm.ctrl[kCtlFeasible0 + w] = 0;
-                    }
+        winner = first_feasible(0);
+        if (winner < 0) {
+            // Four probes a round. Every thread follows the interval, and a round's results are read behind its one barrier: the
+            // next round builds into the four buffers that do not hold the best plan so far, and the results of the round after
+            // that are written behind the next barrier. (Four barriers a round and the best threshold built again: 16 ranks x 2
+            // experts x 1 slot 20.0 us, 18.8 like this.)
+            int lo = min(fitting + 1, hi0), hi = hi0;
+            for (int set = kSolverProbeWarps; lo < hi;) {
+                const int range = hi - lo;
+                const bool each = range <= kSolverProbeWarps;
+                auto probe = [&](int w) {
+                    return lo + (each ? w : static_cast<int>((static_cast<long long>(range) * (w + 1)) / (kSolverProbeWarps + 1)));
+                };
+                if (warp < kSolverProbeWarps) {
+                    if (!each || warp < range) build(set + warp, probe(warp), false, nullptr);
+                    else if (lane == 0) sm.ctrl[kCtlBuilt0 + set + warp] = 0;
                 }
                 __syncthreads();
-                if (warp < kSolverProbeWarps && sm.ctrl[kCtlValid0 + warp]) {
-                    int n = 0;
-                    const bool ok = warp_build_plan<false>(sm, warp, n, sm.ctrl[kCtlProbe0 + warp], sm.ctrl[kCtlTotal], G, M, R, a.min_tokens, allow0, false, lane);
-                    if (lane == 0) sm.ctrl[kCtlFeasible0 + warp] = ok ? 1 : 0;
-                }
-                __syncthreads();
-                if (tid == 0) {
-                    if (sm.ctrl[kCtlSmallRange]) {
-                        int best = -1;
-                        for (int w = 0; w < kSolverProbeWarps; ++w) {
-                            if (sm.ctrl[kCtlValid0 + w] && sm.ctrl[kCtlFeasible0 + w]) {
-                                best = sm.ctrl[kCtlProbe0 + w];
-                                break;
-                            }
-                        }
-                        if (best >= 0) {
-                            sm.ctrl[kCtlLo] = best;
-                            sm.ctrl[kCtlHi] = best;
-                        } else {
-                            sm.ctrl[kCtlLo] = sm.ctrl[kCtlHi];
-                        }
-                    } else {
-                        int first = -1;
-                        for (int w = 0; w < kSolverProbeWarps; ++w) {
-                            if (sm.ctrl[kCtlFeasible0 + w]) {
-                                first = w;
-                                break;
-                            }
-                        }
-                        if (first >= 0) {
-                            sm.ctrl[kCtlHi] = sm.ctrl[kCtlProbe0 + first];
-                            if (first > 0) sm.ctrl[kCtlLo] = sm.ctrl[kCtlProbe0 + first - 1] + 1;
-                        } else {
-                            sm.ctrl[kCtlLo] = sm.ctrl[kCtlProbe0 + kSolverProbeWarps - 1] + 1;
-                        }
-                    }
-                }
-                __syncthreads();
-            }
-            if (warp == 0) {
-                int n = 0;
-                const bool ok = warp_build_plan<true>(sm, 0, n, sm.ctrl[kCtlLo], sm.ctrl[kCtlTotal], G, M, R, a.min_tokens, allow0, false, lane);
-                if (lane == 0) {
-                    sm.ctrl[kCtlNumBatches] = ok ? n : 0;
-                    if (!ok) report_error(status, UEP_DEV_SOLVER_INFEASIBLE, sm.ctrl[kCtlLo]);
+                const int first = first_feasible(set);
+                if (first >= 0) {
+                    hi = probe(first);
+                    winner = set + first;
+                    lo = each ? hi : (first > 0 ? probe(first - 1) + 1 : lo);
+                    set ^= kSolverProbeWarps;
+                } else {
+                    lo = each ? hi : probe(kSolverProbeWarps - 1) + 1;
+                    __syncthreads();  // the same buffers again
                 }
             }
-            __syncthreads();
-            num_batches = sm.ctrl[kCtlNumBatches];
+            // No probe succeeded: at the largest load nothing is to be moved.
+            if (winner < 0) {
+                winner = 0;
+                num_batches = 0;
+            }
         }
     }
     stamp(3);
     // The experts with replicas, one per warp at a time, over what was written without them: lane 0 is the master, lane j the
     // j-th export in the order of their creation.
-    const ExportEntry* plan = sm.plan + winner * kMaxExportsPerDomain;
-    const uint32_t* batches = sm.batches + winner * kMaxExportsPerDomain;
+    const ExportEntry* plan = sm.plan + winner * sm.slots;
+    const uint32_t* batches = sm.batches + winner * sm.slots;
     // Where there are warps enough, one writes an expert's rows and another one splits this rank's tokens.
     const int warps = nthreads / kWarp, apart = 2 * num_batches <= warps ? 1 : 0;
     for (int task = warp; task < num_batches << apart; task += warps) {
