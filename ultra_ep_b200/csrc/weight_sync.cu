@@ -94,6 +94,7 @@ struct SyncShared {
     int shard_tiles[4];
     int w_a[kSyncMaxThreads / 32], w_r[kSyncMaxThreads / 32];
     short rep_start[kMaxExpertsPerDomain + 1];  // [n_active+1] offsets into dst_*
+    short order[kMaxExpertsPerDomain];          // hand-out order of the active masters: relayed ones first; by_expert
     // Addresses are resolved once per CTA: the issuing thread must not chase pointers
     // through global memory for every 32 KiB tile.
     const uint8_t* src[kMaxExpertsPerDomain][4];  // [n_active][shard] master shard base
@@ -115,7 +116,6 @@ struct SyncShared {
     // that run next to it can use)
     uint64_t* dst_flags[kMaxSends];               // that slot's row of ready flags on the peer (relay)
     int rank_out[kMaxPeers], rank_in[kMaxPeers];  // adaptive relay: experts each rank sends / receives under this plan
-    short order[kMaxExpertsPerDomain];          // hand-out order of the active masters: relayed ones first
     unsigned char relay_r[kMaxExpertsPerDomain];  // [n_active] 0: direct, else the replica count of a relayed expert
     unsigned char relay_of[kMaxExpertsPerDomain]; // [logical expert of the domain] the same for every expert of the plan
     unsigned char reps_of[kMaxExpertsPerDomain];  // [logical expert of the domain] its replica count (capped at 255)
@@ -402,6 +402,24 @@ __global__ void __launch_bounds__(kSyncMaxThreads) weight_sync_kernel(SyncCall c
             }
         }
     }
+    // Hosted ranks' masters and replicas are one device's memory: expert by expert, the most replicated first, its streams are
+    // longer stretches, and the units that end last are those of one replica. Ranks of other devices are fed in turn instead, and
+    // so are streams that L2 holds. Step of eight ranks (us, in turn and like this): 256 experts of 44 MB 113.1 and 110.6, in the
+    // order of the masters 111.0; 128 of 19 MB 61.1 and 61.2; 9 MB, 100 MB in all, 67.3 and 67.6.
+    const bool longer_than_l2 = nlocal > 1 && (sm.n_active + sm.total_reps) * (sh.bytes[0] + sh.bytes[1] + sh.bytes[2] + sh.bytes[3]) > kL2Bytes;
+    const bool by_expert = !kRelay && longer_than_l2;
+    if (by_expert) {  // (the scan above has ended with a barrier; the one in front of the copy covers the order)
+        for (int i = tid; i < sm.n_active; i += blockDim.x) {
+            auto replicas = [&](int k) { return (k + 1 < sm.n_active ? sm.rep_start[k + 1] : sm.total_reps) - sm.rep_start[k]; };
+            const int mine = replicas(i);
+            int pos = 0;
+            for (int j = 0; j < sm.n_active; ++j) {
+                const int other = replicas(j);
+                pos += (other > mine || (other == mine && j < i)) ? 1 : 0;
+            }
+            sm.order[pos] = static_cast<short>(i);
+        }
+    }
     // Owners of the local replica slots: who sends to this rank; and, for relayed experts, what this
     // rank forwards. One thread per (hosted rank, slot).
     int my_fwd_r = 0, my_fwd_k = -1, my_l = -1;
@@ -516,9 +534,14 @@ __global__ void __launch_bounds__(kSyncMaxThreads) weight_sync_kernel(SyncCall c
             } else if (!kR || u < send_units) {
                 const int v = u - relay_units;
                 un.kind = 0;
-                un.who = kR ? sm.order[n_relay + v % n_direct] : v % n_direct;
                 un.chunk = 0;
-                un.tile = v / n_direct;
+                if (by_expert) {
+                    un.who = sm.order[v / tiles_per_expert];
+                    un.tile = v % tiles_per_expert;
+                } else {
+                    un.who = kR ? sm.order[n_relay + v % n_direct] : v % n_direct;
+                    un.tile = v / n_direct;
+                }
                 un.tile_end = un.tile + 1;
             } else {
                 const int v = u - send_units;
@@ -593,9 +616,7 @@ __global__ void __launch_bounds__(kSyncMaxThreads) weight_sync_kernel(SyncCall c
                 // there when the experts are used: 4 MB each 46.0 and 44.2, but 68.4 and 71.3; 2 MB 42.8 and 43.0, 64.4 and
                 // 64.6. Loads or stores alone change nothing. (Not measured over NVLink, and a relayed chunk is read again
                 // where it lands: there the priority is the usual one.)
-                const int64_t expert_bytes = sh.bytes[0] + sh.bytes[1] + sh.bytes[2] + sh.bytes[3];
-                const bool streams = !kR && nlocal > 1 && (sm.n_active + sm.total_reps) * expert_bytes > kL2Bytes;
-                const uint64_t policy = streams ? l2_first() : l2_normal();
+                const uint64_t policy = !kR && longer_than_l2 ? l2_first() : l2_normal();
                 TileRef* ring = sm.ring;
                 int* ring_valid = sm.ring_valid;
                 uint64_t** ring_flag = sm.ring_flag;
