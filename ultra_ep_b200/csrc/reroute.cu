@@ -190,14 +190,18 @@ __device__ __forceinline__ void tile_bit_columns(const uint8_t* __restrict__ til
     }
 }
 
-// The count of a (tile, expert) pair is at most kDenseTileRows = 64: it is kept in ONE BYTE, row-major
-// [tile][L] in the scratch buffer, so that the second kernel can add up the tiles in front of it sixteen
-// experts per load. `fast`: L is a multiple of 16 with L/16 in {1,2,4,...,32}, the map and the scratch are
-// 16-byte aligned: a thread then always meets the same sixteen columns and can add map bytes as packed words.
-__device__ __forceinline__ bool dense_fast_path(const uint8_t* map, const void* scratch, int L) {
+// The count of a (tile, expert) pair is at most kDenseTileRows = 64: it is kept in ONE BYTE of the scratch buffer, an expert's
+// tiles side by side, so that a warp of the second kernel adds up the tiles in front of its own four to a load and four to an
+// instruction, and only for the experts that need it. Rows of four tiles and more are padded to 16 bytes (the scratch has an
+// int32 for each pair).
+__host__ __device__ __forceinline__ int count_stride(int tiles) { return tiles >= 4 ? (tiles + 15) & ~15 : 4; }
+__host__ __device__ __forceinline__ int dense_tiles(int T) { return (T + kDenseTileRows - 1) / kDenseTileRows; }
+
+// L is a multiple of 16 with L/16 in {1,2,4,...,32} and the map 16-byte aligned: a thread then always meets the same sixteen
+// columns and can add map bytes as packed words.
+__device__ __forceinline__ bool dense_fast_path(const uint8_t* map, int L) {
     const int G = L / 16;
-    return (L % 16 == 0) && G <= 32 && (G & (G - 1)) == 0 &&
-           ((reinterpret_cast<uintptr_t>(map) | reinterpret_cast<uintptr_t>(scratch)) & 15u) == 0;
+    return (L % 16 == 0) && G <= 32 && (G & (G - 1)) == 0 && (reinterpret_cast<uintptr_t>(map) & 15u) == 0;
 }
 
 // TILES tiles a CTA: one or four (launch_dense_forward).
@@ -208,18 +212,17 @@ __global__ void __launch_bounds__(kRerouteThreads) dense_count_kernel(Batch<Dens
     extern __shared__ __align__(128) char smem_raw[];  // [TILES][pad4(L)] counts, one byte each
     constexpr int kThreads = kRerouteThreads / TILES;  // of a tile: whole warps
     const DenseFwdArgs& a = batch.a[blockIdx.y];
-    const int T = a.T;
-    const int first = blockIdx.x * TILES * kDenseTileRows;
-    if (first >= T) return;
-    const int mine = threadIdx.x / kThreads, tid = threadIdx.x % kThreads, words = pad4(L) / 4;
-    const int r0 = min(first + mine * kDenseTileRows, T), rows = min(T - r0, kDenseTileRows);
+    const int T = a.T, tiles = dense_tiles(T), words = pad4(L) / 4;
+    const int first = blockIdx.x * TILES;
+    if (first >= tiles) return;
+    const int mine = threadIdx.x / kThreads, tid = threadIdx.x % kThreads;
+    const int r0 = min((first + mine) * kDenseTileRows, T), rows = min(T - r0, kDenseTileRows);
     const uint8_t* src = a.map + static_cast<int64_t>(r0) * L;
-    uint32_t* cnt = reinterpret_cast<uint32_t*>(smem_raw) + mine * words;
-    for (int i = tid; i < words; i += kThreads) cnt[i] = 0;
+    for (int i = threadIdx.x; i < words * TILES; i += blockDim.x) reinterpret_cast<uint32_t*>(smem_raw)[i] = 0;
     __syncthreads();
+    uint32_t* cnt = reinterpret_cast<uint32_t*>(smem_raw) + mine * words;
     // a byte never exceeds 64, so the packed adds below cannot carry into the next byte
-    const bool fast = dense_fast_path(a.map, a.scratch, L);
-    if (fast) {
+    if (dense_fast_path(a.map, L)) {
         constexpr int kFlight = TILES == 1 ? 4 : 8;
         const int G = L / 16;
         // vector i of the tile covers row i / G, columns 16 * (i % G) ..; kThreads is a multiple of G, so a
@@ -260,149 +263,70 @@ __global__ void __launch_bounds__(kRerouteThreads) dense_count_kernel(Batch<Dens
         }
     }
     __syncthreads();
-    if (rows <= 0) return;
-    uint8_t* counts = reinterpret_cast<uint8_t*>(a.scratch) + static_cast<int64_t>(r0 / kDenseTileRows) * L;
-    if (fast) {
-        for (int i = tid; i < words; i += kThreads) reinterpret_cast<uint32_t*>(counts)[i] = cnt[i];
-    } else {
-        for (int e = tid; e < L; e += kThreads) counts[e] = reinterpret_cast<const uint8_t*>(cnt)[e];
+    const uint8_t* bytes = reinterpret_cast<const uint8_t*>(smem_raw);
+    const int stride = count_stride(tiles);
+    uint8_t* counts = reinterpret_cast<uint8_t*>(a.scratch) + first;
+    for (int e = threadIdx.x; e < L; e += blockDim.x) {
+        if (TILES == 1) {
+            counts[static_cast<int64_t>(e) * stride] = bytes[e];
+        } else {
+            uint32_t w = 0;
+#pragma unroll
+            for (int k = 0; k < TILES; ++k) w |= static_cast<uint32_t>(bytes[k * 4 * words + e]) << (8 * k);
+            *reinterpret_cast<uint32_t*>(counts + static_cast<int64_t>(e) * stride) = w;
+        }
     }
 }
 
-// Adds the counts of the tiles in front of `tile` to base_of[L] (shared memory, zeroed), all threads of the CTA.
-__device__ __forceinline__ void sum_earlier_tiles(const DenseFwdArgs& a, int L, int tile, int32_t* base_of) {
-    const uint8_t* counts = reinterpret_cast<const uint8_t*>(a.scratch);
-    const int tid = threadIdx.x;
-    if (dense_fast_path(a.map, a.scratch, L)) {
-        const int G = L / 16;
-        const int g = tid % G, sub = tid / G, nsub = blockDim.x / G;
-        // bytes are widened to 16-bit lanes; a lane overflows after 1024 tiles of 64 rows, so it is spilled before
-        uint32_t lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
-        const int lane = tid & 31;
-        auto spill = [&]() {
-            // lanes of the warp that hold the same sixteen columns first (their sum stays below 2^16), then one
-            // shared-memory add per column from the first of them
-            for (int d = G; d < 32; d <<= 1) {
-#pragma unroll
-                for (int w = 0; w < 4; ++w) {
-                    lo[w] += __shfl_xor_sync(kFullMask, lo[w], d);
-                    hi[w] += __shfl_xor_sync(kFullMask, hi[w], d);
-                }
-            }
-            if (lane < G) {
-#pragma unroll
-                for (int w = 0; w < 4; ++w) {
-                    const int e = g * 16 + w * 4;
-                    if (lo[w] & 0xFFFFu) atomicAdd(base_of + e, static_cast<int>(lo[w] & 0xFFFFu));
-                    if (hi[w] & 0xFFFFu) atomicAdd(base_of + e + 1, static_cast<int>(hi[w] & 0xFFFFu));
-                    if (lo[w] >> 16) atomicAdd(base_of + e + 2, static_cast<int>(lo[w] >> 16));
-                    if (hi[w] >> 16) atomicAdd(base_of + e + 3, static_cast<int>(hi[w] >> 16));
-                }
-            }
-#pragma unroll
-            for (int w = 0; w < 4; ++w) lo[w] = hi[w] = 0;
-        };
-        // every thread runs the same number of rounds (the shuffles above need the whole warp)
-        const int rounds = (tile + 4 * nsub - 1) / (4 * nsub);
-        int since = 0;
-        for (int rd = 0; rd < rounds; ++rd) {
-            const int tl0 = sub + rd * 4 * nsub;
-            uint4 v[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {  // four independent loads in flight
-                const int tl = tl0 + u * nsub;
-                v[u] = tl < tile ? __ldcg(reinterpret_cast<const uint4*>(counts + static_cast<int64_t>(tl) * L) + g)
-                                 : make_uint4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const uint32_t w4[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
-#pragma unroll
-                for (int w = 0; w < 4; ++w) {
-                    lo[w] += w4[w] & 0x00FF00FFu;
-                    hi[w] += (w4[w] >> 8) & 0x00FF00FFu;
-                }
-            }
-            since += 4;
-            if (since >= 4 * G) {  // at most (4G + 4) counts of at most 64 per lane, times 32 / G lanes in the shuffle: < 2^15
-                spill();
-                since = 0;
-            }
-        }
-        spill();
-        return;
+// Tokens of the tiles in front of `tile` in an expert's row of counts, by one warp.
+__device__ __forceinline__ int sum_earlier_tiles(const uint8_t* counts, int tile, int lane) {
+    uint32_t sum = 0;
+    for (int t = 4 * lane; t < tile; t += 4 * kWarp) {
+        uint32_t w = __ldcg(reinterpret_cast<const uint32_t*>(counts + t));
+        if (tile - t < 4) w &= (1u << (8 * (tile - t))) - 1u;
+        sum = __dp4a(w, 0x01010101u, sum);
     }
-    if (L % 4 == 0 && (reinterpret_cast<uintptr_t>(counts) & 3u) == 0) {
-        // other widths: a word of four columns per thread, the tiles shared among the threads of a word. A thread per
-        // column that walked all tiles was 16 round trips of eight tiles at 8192 rows.
-        const int quads = L / 4, parts = max(static_cast<int>(blockDim.x) / quads, 1);
-        for (int i = tid; i < quads * parts; i += blockDim.x) {
-            const int q = i % quads, part = i / quads;
-            for (int t0 = part; t0 < tile; t0 += 512 * parts) {  // 512 counts of at most 64 fit a 16-bit lane
-                const int t1 = min(t0 + 512 * parts, tile);
-                uint32_t lo = 0, hi = 0;
-                for (int t = t0; t < t1; t += 8 * parts) {
-                    uint32_t v[8];
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        const int tl = t + u * parts;
-                        v[u] = tl < t1 ? __ldcg(reinterpret_cast<const uint32_t*>(counts + static_cast<int64_t>(tl) * L) + q) : 0u;
-                    }
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        lo += v[u] & 0x00FF00FFu;
-                        hi += (v[u] >> 8) & 0x00FF00FFu;
-                    }
-                }
-                atomicAdd(base_of + 4 * q, static_cast<int>(lo & 0xFFFFu));
-                atomicAdd(base_of + 4 * q + 1, static_cast<int>(hi & 0xFFFFu));
-                atomicAdd(base_of + 4 * q + 2, static_cast<int>(lo >> 16));
-                atomicAdd(base_of + 4 * q + 3, static_cast<int>(hi >> 16));
-            }
-        }
-        return;
-    }
-    for (int e = tid; e < L; e += blockDim.x) {
-        int b = 0;
-#pragma unroll 8
-        for (int tl = 0; tl < tile; ++tl) b += __ldcg(counts + static_cast<int64_t>(tl) * L + e);
-        base_of[e] = b;
-    }
+    return warp_sum(static_cast<int>(sum));
 }
 
 // Second kernel: one CTA per tile of 64 tokens. The logical bit columns become physical ones (an expert with one
 // instance: its column is copied; with several: a warp resolves the column's marked rows), and then a thread owns four
-// physical columns of eight rows and writes them out of its registers: a probability is read where its bit is set,
-// zeros are written elsewhere. Shared memory holds bits and plan rows only (15 KB at 128 experts), so eight CTAs fit an
-// SM, and several still do beside a weight_sync CTA. Outputs wider than kDenseMaxChunkCols go in column chunks.
-// Building the output tile in shared memory took 71 KB per CTA and a walk of every column. Kernel time, before and after:
-// 8191 tokens, 256 experts, one rank 18.4 -> 10.3 us; eight ranks of 8192 tokens, 128 experts, beside weight_sync
-// 53..70 -> 38 us (the two share the memory); 4096 tokens, 64 experts 10.4 -> 5.9 us.
+// physical columns of four rows and writes them out of its registers: a probability is read where its bit is set,
+// zeros are written elsewhere. Outputs wider than kDenseMaxChunkCols go in column chunks.
+// Two thirds of the kernel's time is instructions, so what is done for every expert is little: its one physical column, or that it
+// has several. Plan rows, the router and the tiles in front are looked up for an expert with several that the tile routes to, by
+// the warp that resolves it, in a few words of its own; shared memory is 4 KB at 128 experts. With all plan rows staged, all
+// experts' tiles added up by every CTA (15 KB) and eight rows a thread, and like this (us): the pair for eight ranks of 8192 tokens
+// and 128 experts 30.0 and 27.3, of 4096 17.0 and 13.7; step of 8192 x 128 with bf16 experts of 9 MB 67.1 and 64.2, of 2000 x 256 with
+// 3 MB 52.3 and 49.4; one rank of 8191 x 256, sparse, dense and backward, 31.9 and 27.9. 64 registers: with 40 (six CTAs an SM) 17.7,
+// 32 are spills. Marked cells written over zeros in memory are partial sectors, and rows gathered in shared memory and sent as
+// bulk stores wait too long for each other: both slower.
 constexpr int kDenseMaxChunkCols = 4096;
 constexpr int kDenseMaxExperts = 1340;
 constexpr int kDenseMaxThreads = 512;
+constexpr int kNoPlace = -1, kSeveralPlaces = -2;
 
-struct DenseShared {
-    int32_t *prefix, *l2p;  // [L][kStagedReps]
-    FastRouter* routers;    // [L]
-    int32_t* base;          // [L] tokens routed to the expert in front of the tile
-    uint8_t* bits;          // [kDenseSegs][pad4(L)]
-    uint8_t* phys_bits;     // [kDenseSegs][pad4(chunk)]
-    uint16_t* expert_of;    // [pad4(chunk)] valid where a bit is set
-    uint16_t* several;      // [L] experts with several instances that the tile routes to
+struct DenseRows {  // of the expert that a warp resolves
+    int32_t prefix[kStagedReps], l2p[kStagedReps];
 };
-__host__ __device__ inline size_t dense_smem_bytes(int L, int chunk_cols) {
+struct DenseShared {
+    DenseRows* rows;      // [warps]
+    int32_t* place;       // [pad4(L)] physical id of an expert with one instance, or one of the constants above
+    uint8_t* bits;        // [kDenseSegs][pad4(L)]
+    uint8_t* phys_bits;   // [kDenseSegs][pad4(chunk)]
+    uint16_t* expert_of;  // [pad4(chunk)] valid where a bit is set
+    uint16_t* several;    // [L] experts with several instances that the tile routes to
+};
+__host__ __device__ inline size_t dense_smem_bytes(int L, int chunk_cols, int threads) {
     const size_t Lq = pad4(L), Cq = pad4(chunk_cols);
-    return Lq * (2 * kStagedReps * 4 + sizeof(FastRouter) + 4 + kDenseSegs + 2) + Cq * (kDenseSegs + 2);
+    return sizeof(DenseRows) * (threads / kWarp) + Lq * (4 + kDenseSegs + 2) + Cq * (kDenseSegs + 2);
 }
 __device__ __forceinline__ DenseShared carve_dense_smem(char* raw, int L, int chunk_cols) {
     const int Lq = pad4(L), Cq = pad4(chunk_cols);
     DenseShared s;
-    s.prefix = reinterpret_cast<int32_t*>(raw);
-    s.l2p = s.prefix + Lq * kStagedReps;
-    s.routers = reinterpret_cast<FastRouter*>(s.l2p + Lq * kStagedReps);
-    s.base = reinterpret_cast<int32_t*>(s.routers + Lq);
-    s.bits = reinterpret_cast<uint8_t*>(s.base + Lq);
+    s.rows = reinterpret_cast<DenseRows*>(raw);
+    s.place = reinterpret_cast<int32_t*>(s.rows + blockDim.x / kWarp);
+    s.bits = reinterpret_cast<uint8_t*>(s.place + Lq);
     s.phys_bits = s.bits + Lq * kDenseSegs;
     s.expert_of = reinterpret_cast<uint16_t*>(s.phys_bits + Cq * kDenseSegs);
     s.several = s.expert_of + Cq;
@@ -427,41 +351,43 @@ struct DenseVec<1> {
     using B = uint8_t;
 };
 
-// Columns [p_lo, p_lo + cols) of the tile's rows, V columns and eight rows per thread and turn.
+// Columns [p_lo, p_lo + cols) of the tile's rows, V columns and four rows per thread and turn.
 template <int V>
 __device__ __forceinline__ void write_dense_chunk(const DenseShared& s, const float* __restrict__ probs, float* __restrict__ out_probs,
                                                   uint8_t* __restrict__ out_map, int rows, int L, int P, int p_lo, int cols) {
+    using F = typename DenseVec<V>::F;
+    using B = typename DenseVec<V>::B;
+    constexpr int kRows = 4;
     const int groups = cols / V, Cq = pad4(cols);
-    const int segs = (rows + 7) / 8;
-    for (int i = threadIdx.x; i < groups * segs; i += blockDim.x) {
-        const int seg = i / groups, c = (i - seg * groups) * V;
-        uint32_t bits[V];
-        int e[V];
+    const int turns = groups * ((rows + kRows - 1) / kRows);
+    const uint32_t per_group = 0xFFFFFFFFu / static_cast<uint32_t>(groups) + 1u;  // i / groups, exact for i < 2^16; 0: one group
+    for (int i = threadIdx.x; i < turns; i += blockDim.x) {
+        const int strip = per_group != 0 ? static_cast<int>(__umulhi(static_cast<uint32_t>(i), per_group)) : i;
+        const int c = (i - strip * groups) * V, r0 = strip * kRows;
+        // byte k: the rows of column c + k
+        const uint32_t bits = static_cast<uint32_t>(*reinterpret_cast<const B*>(s.phys_bits + r0 / 8 * Cq + c)) >> r0 % 8;
+        unsigned from[V];
 #pragma unroll
-        for (int k = 0; k < V; ++k) {
-            bits[k] = s.phys_bits[seg * Cq + c + k];
-            e[k] = s.expert_of[c + k];
+        for (int k = 0; k < V; ++k) from[k] = static_cast<unsigned>(r0 * L) + s.expert_of[c + k];
+        float v[kRows][V];
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+#pragma unroll
+            for (int k = 0; k < V; ++k) v[r][k] = (bits >> (8 * k + r)) & 1u ? __ldg(probs + (from[k] + static_cast<unsigned>(r * L))) : 0.f;
         }
-        float v[8][V];
+        float* to = out_probs + static_cast<int64_t>(r0) * P + p_lo + c;
+        uint8_t* to_map = out_map + static_cast<int64_t>(r0) * P + p_lo + c;
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const float* row = probs + static_cast<int64_t>(8 * seg + r) * L;
-#pragma unroll
-            for (int k = 0; k < V; ++k) v[r][k] = (bits[k] >> r) & 1u ? __ldg(row + e[k]) : 0.f;
-        }
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            if (8 * seg + r < rows) {
-                const int64_t at = static_cast<int64_t>(8 * seg + r) * P + p_lo + c;
-                uint32_t m = 0;
-#pragma unroll
-                for (int k = 0; k < V; ++k) m |= ((bits[k] >> r) & 1u) << (8 * k);
-                typename DenseVec<V>::F f;
+        for (int r = 0; r < kRows; ++r) {
+            if (r0 + r < rows) {
+                F f;
 #pragma unroll
                 for (int k = 0; k < V; ++k) reinterpret_cast<float*>(&f)[k] = v[r][k];
-                *reinterpret_cast<typename DenseVec<V>::F*>(out_probs + at) = f;
-                *reinterpret_cast<typename DenseVec<V>::B*>(out_map + at) = static_cast<typename DenseVec<V>::B>(m);
+                *reinterpret_cast<F*>(to) = f;
+                *reinterpret_cast<B*>(to_map) = static_cast<B>((bits >> r) & 0x01010101u);
             }
+            to += P;
+            to_map += P;
         }
     }
 }
@@ -478,34 +404,31 @@ dense_scatter_kernel(Batch<DenseFwdArgs> batch, int L, int P, int D, int quota_m
     extern __shared__ __align__(128) char smem_raw[];
     __shared__ int n_several;
     const DenseShared s = carve_dense_smem(smem_raw, L, chunk_cols);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, Lq = pad4(L);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, warps = blockDim.x / kWarp, Lq = pad4(L);
 
     // ---- nothing here depends on the count kernel ------------------------------------------------
-    stage_plan_rows_async(a.lcnts, a.rqp, a.l2p, L, D, quota_mode != 0, s.routers, s.prefix, s.l2p);
-    for (int e = tid; e < L; e += blockDim.x) s.base[e] = 0;
     for (int i = tid; i < pad4(chunk_cols) / 4 * kDenseSegs; i += blockDim.x) reinterpret_cast<uint32_t*>(s.phys_bits)[i] = 0;
     if (tid == 0) n_several = 0;
+    for (int e = tid; e < L; e += blockDim.x) {
+        const int C = a.lcnts[e], p = a.l2p[static_cast<int64_t>(e) * D];
+        s.place[e] = C > 1 ? kSeveralPlaces : (C == 1 && p >= 0 && p < P ? p : kNoPlace);
+    }
     tile_bit_columns(a.map + static_cast<int64_t>(r0) * L, rows, kDenseSegs, L, s.bits);
-    cp_async_wait();
     __syncthreads();
     for (int e = tid; e < L; e += blockDim.x) {
-        const int C = s.routers[e].C;
-        s.routers[e] = make_fast_router(e, C, a.rqp, D, quota_mode != 0, interleave != 0, s.prefix + e * kStagedReps);
-        if (C > 1) {
+        if (s.place[e] == kSeveralPlaces) {
             uint32_t any = 0;
 #pragma unroll
             for (int g = 0; g < kDenseSegs; ++g) any |= s.bits[g * Lq + e];
             if (any) s.several[atomicAdd(&n_several, 1)] = static_cast<uint16_t>(e);
         }
     }
-    if (overlapped) pdl_wait();
-    pdl_launch_dependents();
-    sum_earlier_tiles(a, L, tile, s.base);
-    __syncthreads();
 
     const float* probs = a.probs + static_cast<int64_t>(r0) * L;
     float* out_probs = a.out_probs + static_cast<int64_t>(r0) * P;
     uint8_t* out_map = a.out_map + static_cast<int64_t>(r0) * P;
+    const uint8_t* counts = reinterpret_cast<const uint8_t*>(a.scratch);
+    const int stride = count_stride(dense_tiles(T));
     for (int p_lo = 0; p_lo < P; p_lo += chunk_cols) {
         const int cols = min(chunk_cols, P - p_lo), Cq = pad4(cols);
         if (p_lo > 0) {
@@ -513,21 +436,38 @@ dense_scatter_kernel(Batch<DenseFwdArgs> batch, int L, int P, int D, int quota_m
             for (int i = tid; i < Cq / 4 * kDenseSegs; i += blockDim.x) reinterpret_cast<uint32_t*>(s.phys_bits)[i] = 0;
             __syncthreads();
         }
-        for (int i = tid; i < L * kDenseSegs; i += blockDim.x) {  // experts with one instance
-            const int g = i / L, e = i - g * L;
-            if (s.routers[e].C != 1) continue;
-            const int p = s.l2p[e * kStagedReps] - p_lo;
-            const uint8_t b = s.bits[g * Lq + e];
-            if (b != 0 && p >= 0 && p < cols) {
-                s.phys_bits[g * Cq + p] = b;
-                s.expert_of[p] = static_cast<uint16_t>(e);
-            }
+        for (int e = tid; e < L; e += blockDim.x) {  // experts with one instance
+            const int p = s.place[e] - p_lo;
+            if (s.place[e] < 0 || p < 0 || p >= cols) continue;
+            s.expert_of[p] = static_cast<uint16_t>(e);
+#pragma unroll
+            for (int g = 0; g < kDenseSegs; ++g) s.phys_bits[g * Cq + p] = s.bits[g * Lq + e];
         }
-        __syncthreads();  // the bytes above share words with the atomics below
-        for (int i = warp; i < n_several; i += blockDim.x / kWarp) {
+        if (p_lo == 0 && overlapped) pdl_wait();
+        if (p_lo == 0) pdl_launch_dependents();
+        __syncthreads();  // the list of experts with several; the bytes above share words with the atomics below
+        for (int i = warp; i < n_several; i += warps) {
             const int e = s.several[i];
-            const FastRouter router = s.routers[e];
-            int before = s.base[e];
+            const int64_t row = static_cast<int64_t>(e) * D;
+            DenseRows& plan = s.rows[warp];
+            const int C = a.lcnts[e];
+            const int prefix = lane < min(D, kStagedReps) && quota_mode ? a.rqp[row + lane] : 0;
+            const int phys = lane < min(D, kStagedReps) ? a.l2p[row + lane] : -1;
+            int before = sum_earlier_tiles(counts + static_cast<int64_t>(e) * stride, tile, lane);
+            __syncwarp();  // the expert before this one has been resolved
+            if (lane < kStagedReps) {
+                plan.prefix[lane] = prefix;
+                plan.l2p[lane] = phys;
+            }
+            __syncwarp();
+            FastRouter router{};
+            if (lane == 0) router = make_fast_router(e, C, a.rqp, D, quota_mode != 0, interleave != 0, plan.prefix);
+            router.C = C;
+            router.total = __shfl_sync(kFullMask, router.total, 0);
+            router.stride = __shfl_sync(kFullMask, router.stride, 0);
+            router.offset = __shfl_sync(kFullMask, router.offset, 0);
+            router.recip = __shfl_sync(kFullMask, router.recip, 0);
+            __syncwarp();
 #pragma unroll
             for (int half = 0; half < 2; ++half) {  // lane t: row 32 * half + t
                 uint32_t m = 0;
@@ -535,9 +475,8 @@ dense_scatter_kernel(Batch<DenseFwdArgs> batch, int L, int P, int D, int quota_m
                 for (int g = 0; g < 4; ++g) m |= static_cast<uint32_t>(s.bits[(4 * half + g) * Lq + e]) << (8 * g);
                 if ((m >> lane) & 1u) {
                     const int ordinal = before + __popc(m & ((1u << lane) - 1u));
-                    const int j = fast_replica_index(router, ordinal, s.prefix + e * kStagedReps, a.rqp + static_cast<int64_t>(e) * D,
-                                                     quota_mode != 0);
-                    const int p = (j < kStagedReps ? s.l2p[e * kStagedReps + j] : a.l2p[static_cast<int64_t>(e) * D + j]) - p_lo;
+                    const int j = fast_replica_index(router, ordinal, plan.prefix, a.rqp + row, quota_mode != 0);
+                    const int p = (j < kStagedReps ? plan.l2p[j] : a.l2p[row + j]) - p_lo;
                     if (p >= 0 && p < cols) {
                         const int seg = 4 * half + lane / 8;
                         atomicOr(reinterpret_cast<uint32_t*>(s.phys_bits + seg * Cq) + p / 4, 1u << (8 * (p & 3) + (lane & 7)));
@@ -1164,7 +1103,6 @@ __global__ void __launch_bounds__(256) gather_rows_plain_kernel(const uint8_t* _
 // until it has drained.
 cudaError_t ensure_smem_attr(const void* fn, size_t bytes) { return allow_smem(fn, bytes, true); }
 
-int dense_tiles(int T) { return (T + kDenseTileRows - 1) / kDenseTileRows; }
 int64_t sparse_tiles(int64_t n) { return (n + kSparseTileEntries - 1) / kSparseTileEntries; }
 
 }  // namespace
@@ -1215,7 +1153,9 @@ cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int
     // (two rounds) 71.6 and 72.7.
     const bool by_four = L <= 128 && static_cast<int64_t>(grid.x) * b.n > 6 * sms;
     const auto count = by_four ? dense_count_kernel<4> : dense_count_kernel<1>;
-    const size_t smem_count = static_cast<size_t>(pad4(L)) * (by_four ? 4 : 1), smem = dense_smem_bytes(L, chunk);
+    // up to two tiles per SM the scatter kernel is a chain of phases: more threads shorten each
+    const int threads = static_cast<int64_t>(grid.x) * b.n <= 2 * sms ? kDenseMaxThreads : kRerouteThreads;
+    const size_t smem_count = static_cast<size_t>(pad4(L)) * (by_four ? 4 : 1), smem = dense_smem_bytes(L, chunk, threads);
     behind_plan = behind_plan && b.n > 1 && pdl_enabled();
     // The first kernel may be on its SMs when whatever is in front of it ends, too: it waits before its first read. (One rank, 8191
     // tokens of 256 experts, sparse, dense and backward one behind the other: 34.1 us with ordinary launches, 32.8 like this. Of
@@ -1232,8 +1172,6 @@ cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int
     // fills the device with the first kernel alone, and early CTAs of the second only get in its way, unless they do nothing
     // but wait.
     const bool overlap = early;
-    // up to two tiles per SM the kernel is a chain of phases: more threads shorten each
-    const int threads = static_cast<int64_t>(grid.x) * b.n <= 2 * sms ? kDenseMaxThreads : kRerouteThreads;
     return launch_dependent(dense_scatter_kernel, grid, dim3(threads), smem, stream, overlap, b, L, P, D, quota_mode,
                             interleave, chunk, overlap ? 1 : 0, behind_plan ? 1 : 0);
 }
