@@ -75,7 +75,7 @@ struct SolverSmem {
     int32_t* loads;      // [E]
     int32_t* my_loads;   // [E]
     int2* masters;       // [E] rank after rank: {load, expert}, largest load first, ties to the lower expert
-    int2* source;        // [G] {load, rank}, largest load first, ties to the lower rank
+    int4* source;        // [G] {load, rank, its largest master's load and number}, largest load first, ties to the lower rank
     int2* sink;          // [G] {load, rank}, smallest first, likewise
     int32_t* rank_load;  // [G]
     ExportEntry* plan;   // [kSolverBuffers][slots]
@@ -89,7 +89,7 @@ struct SolverSmem {
 __host__ __device__ inline int solver_ns(int G) { return (G + 31) / 32; }
 __host__ __device__ inline int solver_pad(int n) { return (n + 3) / 4 * 4; }
 __host__ __device__ inline size_t solver_smem_bytes(int E, int G, int R) {
-    return sizeof(int32_t) * (4 * static_cast<size_t>(solver_pad(E)) + 5 * solver_pad(G)) +
+    return sizeof(int32_t) * (4 * static_cast<size_t>(solver_pad(E)) + 7 * solver_pad(G)) +
            kSolverBuffers * (sizeof(ExportEntry) + sizeof(uint32_t)) * solver_pad(G * R) +
            kSolverProbeWarps * 3 * sizeof(long long) * kMaxListed + sizeof(int) * 32;
 }
@@ -101,7 +101,7 @@ __device__ inline SolverSmem carve_solver_smem(char* raw, int E, int G, int R) {
     s.loads = p; p += ep;
     s.my_loads = p; p += ep;
     s.masters = reinterpret_cast<int2*>(p); p += 2 * ep;
-    s.source = reinterpret_cast<int2*>(p); p += 2 * gp;
+    s.source = reinterpret_cast<int4*>(p); p += 4 * gp;
     s.sink = reinterpret_cast<int2*>(p); p += 2 * gp;
     s.rank_load = p; p += gp;
     s.plan = reinterpret_cast<ExportEntry*>(p); p += kSolverBuffers * 2 * slots;
@@ -157,15 +157,14 @@ __device__ bool drain_sources(const SolverSmem& sm, int warp, int buffer, int& n
     Key fresh = fresh_keys[0], fresh_next = fresh_keys[1];
     WaitingRank<Key> top = none, top_next = none;
     int count = with_slack;  // ranks in both lists
-    int num_exports = 0, ord = 0, left = M;
-    int2 source = sm.source[0];
+    int num_exports = 0, ord = 0, left = M, stopped = 0;
+    int4 source = sm.source[0], next_source = sm.source[min(1, G - 1)];
     int need = source.x - thr, at_master = source.y * M;
-    int2 master = sm.masters[at_master];
-    int2 next_source = sm.source[min(1, G - 1)];
-    int2 next_first = sm.masters[next_source.y * M];
+    int2 master = make_int2(source.z, source.w);
     while (true) {
         const int2 follow = sm.masters[min(at_master + 1, G * M - 1)];
-        if (stop != nullptr && *stop != 0) return false;
+        if (stopped != 0) return false;
+        if (stop != nullptr) stopped = *stop;
         const int give = min(need, max(master.x - keep, 0));
         if (give == 0) return false;  // the masters come by load: no later one of this source has anything to give
         const int first = num_exports;
@@ -207,15 +206,20 @@ __device__ bool drain_sources(const SolverSmem& sm, int warp, int buffer, int& n
             if (move == 0 && rest > 0 && slots + 1 < R) {
                 const WaitingRank<Key> back{static_cast<Key>(rest) << 7 | (best & 127), slots + 1};
                 int place = waiting++;
-                for (; place > 0; --place) {
-                    const WaitingRank<Key> other = again[place - 1];
-                    if (other.key < back.key) break;
-                    again[place] = other;
-                }
-                again[place] = back;
-                top = again[waiting - 1];
-                top_next = again[waiting - 2];
                 ++count;
+                if (back.key > top.key) {
+                    again[place] = back;
+                    top_next = top;
+                    top = back;
+                } else {
+                    for (; place > 0; --place) {
+                        const WaitingRank<Key> other = again[place - 1];
+                        if (other.key < back.key) break;
+                        again[place] = other;
+                    }
+                    again[place] = back;
+                    top_next = again[waiting - 2];
+                }
             }
         }
         if (need > 0) {
@@ -229,9 +233,8 @@ __device__ bool drain_sources(const SolverSmem& sm, int warp, int buffer, int& n
         left = M;
         source = next_source;
         at_master = source.y * M;
-        master = next_first;
+        master = make_int2(source.z, source.w);
         next_source = sm.source[min(ord + 1, G - 1)];
-        next_first = sm.masters[next_source.y * M];
     }
 }
 
@@ -249,11 +252,10 @@ __device__ bool warp_build_plan(const SolverSmem& sm, int warp, int buffer, int&
     for (int i0 = 0; i0 < G + 2; i0 += kWarp) {
         const int i = i0 + lane;
         const int2 sink = i < G ? sm.sink[i] : make_int2(thr, 0);
-        const int slack = max(thr - sink.x, 0);
-        const long long key = slack > 0 ? static_cast<long long>(slack) << 7 | (127 - sink.y) : -1;
+        const int slack = max(thr - sink.x, 0), code = 127 - sink.y;
         if (i < G + 2) {
-            if (narrow) reinterpret_cast<int*>(sm.fresh + warp * kMaxListed)[i] = static_cast<int>(key);
-            else sm.fresh[warp * kMaxListed + i] = key;
+            if (narrow) reinterpret_cast<int*>(sm.fresh + warp * kMaxListed)[i] = slack > 0 ? slack << 7 | code : -1;
+            else sm.fresh[warp * kMaxListed + i] = slack > 0 ? static_cast<long long>(slack) << 7 | code : -1;
         }
         with_slack += __popc(__ballot_sync(kFullMask, slack > 0));
     }
@@ -555,7 +557,8 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, cha
                 below += other < mine ? 1 : 0;
                 equal += (other == mine && j < i) ? 1 : 0;
             }
-            sm.source[above + equal] = make_int2(mine, i);
+            const int2 largest = sm.masters[i * M];
+            sm.source[above + equal] = make_int4(mine, i, largest.x, largest.y);
             sm.sink[below + equal] = make_int2(mine, i);
         }
         if (warp == kSolverProbeWarps - 1) {
