@@ -42,7 +42,7 @@ enum {
     UEP_DEV_TIMEOUT_GATHER = 1,     /* a peer's load row did not arrive in time       */
     UEP_DEV_TIMEOUT_SYNC = 2,       /* a peer's weight_sync completion flag timed out */
     UEP_DEV_TIMEOUT_COPY = 3,       /* an async bulk copy did not complete in time    */
-    UEP_DEV_SOLVER_INFEASIBLE = 4,  /* final plan rebuild infeasible (cannot happen on valid loads) */
+    UEP_DEV_SOLVER_INFEASIBLE = 4,  /* not reported: the search ends with a plan that it has built */
     UEP_DEV_BAD_PLAN = 5            /* plan entry outside its table                   */
 };
 
