@@ -255,12 +255,14 @@ __host__ __device__ inline size_t plan_matrix_bytes(int N, int L) {
     return bytes <= kPlanMatrixBytes ? bytes : 0;
 }
 
-// The solver's code runs once a layer, and what runs between two layers (weight copies, expanded outputs) leaves none of it in
-// L2: its instructions came from DRAM one line after another. Where the input is large, a CTA of its own solves a small problem of
-// its own from the kernel's start, while the others count and exchange, so that the owners find the lines in L2. Nothing waits
-// for it, and its outputs stay in its shared memory. Step of eight ranks, bool rows of 8192 x 128 and bf16 experts of 9 MB, without and
-// with it: 69.2 and 66.7 us (search 6.1 and 4.4); 16384 tokens of 256 experts 112.1 and 111.3. Where the counting is shorter than
-// the rehearsal, or copies leave L2 first (fp8 experts, 8192 int32 tokens), it takes as much as it gives: 59.6 and 60.5.
+// The solver's code runs once a layer, and what runs between two layers (weight copies, expanded outputs, the model) leaves none of
+// it in L2: its instructions came from DRAM one line after another. Where the input is more than eight CTAs' a rank, a CTA of its
+// own solves a small problem of its own from the kernel's start, while the others count and exchange, so that the owners find the
+// lines in L2. Nothing waits for it, and its outputs stay in its shared memory. Without and with it, eight ranks (us): behind an
+// L2 flush, 8192 int32 tokens of 128 experts, plan 24.1 and 21.5, step with fp8 experts of 19 MB 63.1 and 59.7; among passes of the
+// same step alone, whose streams leave L2 first and the code there, 58.9 and 59.3; 8192 bool rows of 128 with bf16 experts of 9 MB 66.7 and 64.5; 16384 int64
+// tokens of 256 110.7 and 109.9. Shorter inputs are counted before it has got anywhere: 4096 tokens of 64 experts (8 CTAs) 28.3 and 28.4,
+// 33 tokens 17.2 and 17.5.
 constexpr int kRehearsalRanks = 4, kRehearsalMasters = 2, kRehearsalSlots = 2, kRehearsalD = 4;
 constexpr int kRehearsalExperts = kRehearsalRanks * kRehearsalMasters;
 constexpr int kRehearsalPhysical = kRehearsalRanks * (kRehearsalMasters + kRehearsalSlots);
