@@ -238,6 +238,12 @@ __device__ bool drain_sources(const SolverSmem& sm, int warp, int buffer, int& n
     }
 }
 
+// Out of line: loads that need it are rare, and code that is jumped over is fetched all the same (below).
+__device__ __noinline__ bool drain_sources_wide(SolverSmem sm, int warp, int buffer, int& num_batches, int thr, int with_slack, int G, int M, int R,
+                                                int min_tokens, bool allow_zero_master, bool dynamic_floor, const volatile int* stop) {
+    return drain_sources<long long>(sm, warp, buffer, num_batches, thr, with_slack, G, M, R, min_tokens, allow_zero_master, dynamic_floor, stop);
+}
+
 // By warp `warp` of the first four, into plan buffer `buffer`. `total`: of the domain's loads.
 __device__ bool warp_build_plan(const SolverSmem& sm, int warp, int buffer, int& num_batches, int thr, int total, int G, int M, int R,
                                 int min_tokens, bool allow_zero_master, bool dynamic_floor, int lane, const volatile int* stop = nullptr) {
@@ -263,7 +269,7 @@ __device__ bool warp_build_plan(const SolverSmem& sm, int warp, int buffer, int&
     int ok = 0, made = 0;
     if (lane == 0) {
         ok = narrow ? drain_sources<int>(sm, warp, buffer, made, thr, with_slack, G, M, R, min_tokens, allow_zero_master, dynamic_floor, stop)
-                    : drain_sources<long long>(sm, warp, buffer, made, thr, with_slack, G, M, R, min_tokens, allow_zero_master, dynamic_floor, stop);
+                    : drain_sources_wide(sm, warp, buffer, made, thr, with_slack, G, M, R, min_tokens, allow_zero_master, dynamic_floor, stop);
     }
     num_batches = __shfl_sync(kFullMask, made, 0);
     return __shfl_sync(kFullMask, ok, 0) != 0;
@@ -529,9 +535,7 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, cha
     const bool do_search = (R > 0 && G > 1);
     stamp(1);
     __syncthreads();
-    if (!do_search) {
-        write_masters(tid, nthreads);
-    } else {
+    if (do_search) {
         // each rank's masters by load descending, ties to the lower index, and its load
         for (int i = tid; i < E; i += nthreads) {
             const int rank = i / M, base = rank * M;
@@ -583,21 +587,24 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, cha
     }
     stamp(2);
     const bool allow0 = a.allow_zero_master != 0;
+    // Without a search by all threads; else by the warps that build no plans (where there are any).
+    const int builders = do_search && nthreads > kSolverProbeWarps * kWarp ? kSolverProbeWarps * kWarp : 0;
+    if (tid >= builders) write_masters(tid - builders, nthreads - builders);
     int winner = 0, num_batches = 0;  // the buffer whose plan is taken
     if (do_search) {
         // The serial search is: up to three builds with the dynamic floor at rising thresholds; then one build at the
         // smallest threshold the capacities allow; then the probes below. The first four run at once, one warp each; one that
-        // succeeds stops those behind it.
+        // succeeds stops those behind it. Then four probes a round. Every thread follows the interval, and a round's results are
+        // read behind its one barrier: the next round builds into the four buffers that do not hold the best plan so far, and the
+        // results of the round after that are written behind the next barrier. (Four barriers a round and the best threshold
+        // built again: 16 ranks x 2 experts x 1 slot 20.0 us, 18.8 like this.)
+        // One loop, so that the build is compiled in once: mostly this code comes from DRAM, a line after the other. Plan of eight
+        // ranks behind an L2 flush, on the device (us), with a build in front of the loop and one inside it, for either width of the
+        // keys, and like this: 33 tokens of 64 experts 19.2 and 14.4, 4096 tokens 17.8 and 16.8; among other plans 10.3 and 9.7, 12.8 and 12.7.
         const int lo0 = sm.ctrl[kCtlLo], hi0 = sm.ctrl[kCtlHi], total = sm.ctrl[kCtlTotal];
         // The smallest threshold from lo0 to hi0 whose excess fits its slack. Excess minus slack is the sum of (load - threshold):
         // it fits from the mean load on. (The reference bisects, csrc/kernels/placement.cu:76-84.)
         const int fitting = min(max(lo0, total / G + (total % G != 0 ? 1 : 0)), hi0);
-        auto build = [&](int buffer, int thr, bool dynamic_floor, const volatile int* stop) {
-            int n = 0;
-            const bool ok = warp_build_plan(sm, warp, buffer, n, thr, total, G, M, R, a.min_tokens, allow0, dynamic_floor, lane, stop);
-            if (lane == 0) sm.ctrl[kCtlBuilt0 + buffer] = ok ? n + 1 : 0;
-            return ok;
-        };
         auto first_feasible = [&](int buffer0) {  // of a round, -1: none; its batches go to num_batches
             int first = -1;
 #pragma unroll
@@ -610,55 +617,52 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, cha
             }
             return first;
         };
-        if (warp < kSolverProbeWarps) {
-            const bool fast = warp < kSolverProbeWarps - 1;
-            int thr = fitting;
-            if (fast) {
-                const float eps = fmaxf(a.eps, 0.0f);
-                thr = max(static_cast<int>(ceilf(__fmul_rn(static_cast<float>(lo0), __fadd_rn(1.0f, eps)))), lo0);
-                const int step = max(1, (hi0 + 99) / 100);
-                for (int i = 0; i < warp; ++i) thr = min(hi0, thr + step);
+        winner = -1;
+        int lo = lo0, hi = hi0, set = 0;  // set: the buffers of the round
+        bool probing = false;
+        while (true) {
+            const int range = hi - lo;
+            const bool each = range <= kSolverProbeWarps;
+            auto probe = [&](int w) {
+                return lo + (each ? w : static_cast<int>((static_cast<long long>(range) * (w + 1)) / (kSolverProbeWarps + 1)));
+            };
+            if (warp < kSolverProbeWarps) {
+                const bool fast = !probing && warp < kSolverProbeWarps - 1, builds = !probing || !each || warp < range;
+                int thr = probing ? probe(warp) : fitting;
+                if (fast) {
+                    const float eps = fmaxf(a.eps, 0.0f);
+                    thr = max(static_cast<int>(ceilf(__fmul_rn(static_cast<float>(lo0), __fadd_rn(1.0f, eps)))), lo0);
+                    const int step = max(1, (hi0 + 99) / 100);
+                    for (int i = 0; i < warp; ++i) thr = min(hi0, thr + step);
+                }
+                int n = 0;
+                const bool ok = builds && warp_build_plan(sm, warp, set + warp, n, thr, total, G, M, R, a.min_tokens, allow0, fast, lane,
+                                                          probing ? nullptr : sm.ctrl + kCtlStop0 + warp);
+                if (lane == 0) sm.ctrl[kCtlBuilt0 + set + warp] = ok ? n + 1 : 0;
+                if (!probing && ok && lane > warp && lane < kSolverProbeWarps) *(sm.ctrl + kCtlStop0 + lane) = 1;
             }
-            if (build(warp, thr, fast, sm.ctrl + kCtlStop0 + warp) && lane > warp && lane < kSolverProbeWarps) *(sm.ctrl + kCtlStop0 + lane) = 1;
-        } else {
-            write_masters(tid - kSolverProbeWarps * kWarp, nthreads - kSolverProbeWarps * kWarp);
+            __syncthreads();
+            const int first = first_feasible(set);
+            if (first >= 0) winner = set + first;
+            if (!probing) {
+                if (first >= 0) break;
+                probing = true;
+                lo = min(fitting + 1, hi0);
+                set = kSolverProbeWarps;
+            } else if (first >= 0) {
+                hi = probe(first);
+                lo = each ? hi : (first > 0 ? probe(first - 1) + 1 : lo);
+                set ^= kSolverProbeWarps;
+            } else {
+                lo = each ? hi : probe(kSolverProbeWarps - 1) + 1;
+                __syncthreads();  // the same buffers again
+            }
+            if (lo >= hi) break;
         }
-        if (nthreads == kSolverProbeWarps * kWarp) write_masters(tid, nthreads);
-        __syncthreads();
-        winner = first_feasible(0);
+        // No probe succeeded: at the largest load nothing is to be moved.
         if (winner < 0) {
-            // Four probes a round. Every thread follows the interval, and a round's results are read behind its one barrier: the
-            // next round builds into the four buffers that do not hold the best plan so far, and the results of the round after
-            // that are written behind the next barrier. (Four barriers a round and the best threshold built again: 16 ranks x 2
-            // experts x 1 slot 20.0 us, 18.8 like this.)
-            int lo = min(fitting + 1, hi0), hi = hi0;
-            for (int set = kSolverProbeWarps; lo < hi;) {
-                const int range = hi - lo;
-                const bool each = range <= kSolverProbeWarps;
-                auto probe = [&](int w) {
-                    return lo + (each ? w : static_cast<int>((static_cast<long long>(range) * (w + 1)) / (kSolverProbeWarps + 1)));
-                };
-                if (warp < kSolverProbeWarps) {
-                    if (!each || warp < range) build(set + warp, probe(warp), false, nullptr);
-                    else if (lane == 0) sm.ctrl[kCtlBuilt0 + set + warp] = 0;
-                }
-                __syncthreads();
-                const int first = first_feasible(set);
-                if (first >= 0) {
-                    hi = probe(first);
-                    winner = set + first;
-                    lo = each ? hi : (first > 0 ? probe(first - 1) + 1 : lo);
-                    set ^= kSolverProbeWarps;
-                } else {
-                    lo = each ? hi : probe(kSolverProbeWarps - 1) + 1;
-                    __syncthreads();  // the same buffers again
-                }
-            }
-            // No probe succeeded: at the largest load nothing is to be moved.
-            if (winner < 0) {
-                winner = 0;
-                num_batches = 0;
-            }
+            winner = 0;
+            num_batches = 0;
         }
     }
     stamp(3);
