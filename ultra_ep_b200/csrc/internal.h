@@ -84,6 +84,7 @@ struct PlanCall {
 cudaError_t launch_plan(const PlanCall& call, cudaStream_t stream);
 int plan_ctas_per_rank(int input_kind, int max_T, int K_or_L, int nlocal, int num_sms);
 int plan_threads(int input_kind, int max_T, int K_or_L, int ctas);
+bool plan_rehearses(const PlanCall& call, int num_sms);
 
 struct SyncCall {
     GroupDev group;

@@ -644,7 +644,7 @@ int uep_update_placement(uep_manager* m, int layer_id, int input_kind, const voi
     call.threads = plan_threads(input_kind, max_T, K_or_L, call.ctas_per_rank);
     call.withhold_rank = m->withhold_rank;
     call.legacy = m->cfg.legacy_placement ? 1 : 0;
-    call.rehearsal = call.ctas_per_rank > 8 && m->N > 1 && m->R > 0 && call.legacy == 0 && m->nlocal * call.ctas_per_rank < m->num_sms ? 1 : 0;
+    call.rehearsal = plan_rehearses(call, m->num_sms) ? 1 : 0;
     call.trace = m->sync_trace ? m->sync_trace + 8 * 1000 : nullptr;  // the last rows of the trace buffer
     UEP_CUDA_TRY(launch_plan(call, stream));
     const int slot = plan_slot(m, layer_id);

@@ -256,13 +256,11 @@ __host__ __device__ inline size_t plan_matrix_bytes(int N, int L) {
 }
 
 // The solver's code runs once a layer, and what runs between two layers (weight copies, expanded outputs, the model) leaves none of
-// it in L2: its instructions came from DRAM one line after another. Where the input is more than eight CTAs' a rank, a CTA of its
-// own solves a small problem of its own from the kernel's start, while the others count and exchange, so that the owners find the
-// lines in L2. Nothing waits for it, and its outputs stay in its shared memory. Without and with it, eight ranks (us): behind an
-// L2 flush, 8192 int32 tokens of 128 experts, plan 24.1 and 21.5, step with fp8 experts of 19 MB 63.1 and 59.7; among passes of the
-// same step alone, whose streams leave L2 first and the code there, 58.9 and 59.3; 8192 bool rows of 128 with bf16 experts of 9 MB 66.7 and 64.5; 16384 int64
-// tokens of 256 110.7 and 109.9. Shorter inputs are counted before it has got anywhere: 4096 tokens of 64 experts (8 CTAs) 28.3 and 28.4,
-// 33 tokens 17.2 and 17.5.
+// it in L2: its instructions came from DRAM one line after another. Where the input is long, a CTA of its own solves a small problem
+// of its own from the kernel's start, while the others count and exchange, so that the owners find the lines in L2. No owner waits
+// for it, but the launch ends with it too, and a cooperative one needs its SM free. It takes the way of the default parameters:
+// the sorts, the four builds side by side with an expert of two exports and ranks that come back, outputs and splits of experts
+// with replicas; not the rounds of probes nor more than 32 replicas. Outputs stay in its shared memory.
 constexpr int kRehearsalRanks = 4, kRehearsalMasters = 2, kRehearsalSlots = 2, kRehearsalD = 4;
 constexpr int kRehearsalExperts = kRehearsalRanks * kRehearsalMasters;
 constexpr int kRehearsalPhysical = kRehearsalRanks * (kRehearsalMasters + kRehearsalSlots);
@@ -270,7 +268,7 @@ __host__ __device__ inline size_t rehearsal_smem_bytes() {
     return solver_smem_bytes(kRehearsalExperts, kRehearsalRanks, kRehearsalSlots) +
            sizeof(int32_t) * (kRehearsalRanks * kRehearsalExperts + 4 * kRehearsalExperts * kRehearsalD + kRehearsalExperts + 2 * kRehearsalPhysical);
 }
-// Two ranks above the mean and two below, so that every step of the solver is taken: an expert with two exports, ranks that come back.
+// Two ranks above the mean and two below. The parameters are its own: a caller's threshold or floor could leave it without exports.
 __device__ __forceinline__ void rehearsal_args(const PlanCall& call, char* smem_raw, SolveArgs& a) {
     const SolverSmem sm = carve_solver_smem(smem_raw, kRehearsalExperts, kRehearsalRanks, kRehearsalSlots);
     int32_t* matrix = reinterpret_cast<int32_t*>(smem_raw + solver_smem_bytes(kRehearsalExperts, kRehearsalRanks, kRehearsalSlots));
@@ -291,11 +289,11 @@ __device__ __forceinline__ void rehearsal_args(const PlanCall& call, char* smem_
     a.global_loads = nullptr;
     a.loads_per_rank = nullptr;
     a.N = a.G = kRehearsalRanks; a.M = kRehearsalMasters; a.R = kRehearsalSlots; a.D = kRehearsalD;
-    a.balance_threshold = call.params.balance_threshold;
-    a.min_tokens = call.params.min_tokens_per_replica;
-    a.allow_zero_master = call.params.allow_zero_master_quota;
+    a.balance_threshold = 1.f;
+    a.min_tokens = 1;
+    a.allow_zero_master = 0;
     a.locality = call.params.locality_aware;
-    a.eps = call.params.oracle_eps;
+    a.eps = 0.01f;
     a.my_rank = 0;
     a.legacy = 0;
     a.preloaded = 1;
@@ -469,13 +467,15 @@ __device__ __forceinline__ bool gather_loads(const PlanCall& call, int local, in
     return true;
 }
 
-// The fused per-layer plan kernel. gridDim.x = nlocal * ctas_per_rank, and one more CTA where it is rehearsed.
-__global__ void __launch_bounds__(kPlanMaxThreads, 1) plan_kernel(PlanCall call) {
+// The fused per-layer plan kernel. gridDim.x = nlocal * ctas_per_rank, and one more CTA where it is rehearsed, which only the form
+// with more threads can be: without, every output's address is known to be global, and the registers are twice as many.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) plan_kernel(PlanCall call) {
     extern __shared__ __align__(128) char smem_raw[];
     // The next kernel of the stream may be on its SMs when the plan ends. Only where every rank of the group is in this launch:
     // a plan that waits for other devices must not have the SMs held meanwhile by CTAs that wait for it.
     if (call.nlocal == call.N) pdl_launch_dependents();
-    const bool rehearses = static_cast<int>(blockIdx.x) == call.nlocal * call.ctas_per_rank;
+    const bool rehearses = THREADS == kPlanMaxThreads && static_cast<int>(blockIdx.x) == call.nlocal * call.ctas_per_rank;
     const int local = rehearses ? 0 : blockIdx.x / call.ctas_per_rank;
     SolveArgs a;
     if (rehearses) {
@@ -500,9 +500,13 @@ std::atomic<int64_t> g_launches{0};
 
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
-// Twice the threads where a CTA's slice of the input would be several rounds of loads. Steps of eight ranks with 256 and 512
-// threads (us): 16384 int64 tokens of 256 experts (57 KB a CTA) 114.5 and 112.1, 8192 bool rows of 128 (57 KB) 69.6 and 69.2;
-// 8192 int32 tokens (15 KB) 31.3 and 32.0, 33 tokens 17.1 and 17.9.
+// Twice the threads where a CTA's slice of the input would be several rounds of loads, and a rehearsal with them. Steps of eight
+// ranks: 256 threads, 512, 512 and the rehearsal; among others / behind an L2 flush (us). Above the line: 2600 bool rows of 128
+// experts (18 KB a CTA) 42.7/49.2, 44.7/50.2, 42.9/47.4; 6500 rows 55.7/59.5, 56.8/59.7, 54.0/57.5; 8192 rows 64.6/67.9, 66.0/69.8,
+// 63.2/67.7; 9600 int32 tokens of 128 (17 KB) 46.1/51.4, 45.9/51.4, 44.7/49.2; 4800 int64 tokens of 64 (17 KB) 35.6/43.2, 36.0/45.2,
+// 35.9/41.1; 16384 of 256 (57 KB) 110.6/114.7, 109.9/114.6, 108.7/111.5. Below: 1600 bool rows 41.2/47.3, 42.8/49.4, 41.5/47.3; 3000
+// int64 tokens of 64 32.7/41.2, 34.5/43.2, 34.5/40.8; 4096 int32 tokens of 64, no experts, 27.2/33.8, 28.7/35.9, 28.7/33.8; 33 tokens
+// 16.2/23.4, 17.3/25.4, 17.6/23.5.
 int plan_threads(int input_kind, int max_T, int K_or_L, int ctas) {
     const int64_t bytes = static_cast<int64_t>(max_T) * K_or_L * (input_kind == 0 ? 1 : (input_kind == 1 ? 4 : 8));
     return bytes > static_cast<int64_t>(ctas) * 16 * 1024 ? kPlanMaxThreads : kPlanMaxThreads / 2;
@@ -517,9 +521,16 @@ int plan_ctas_per_rank(int input_kind, int max_T, int K_or_L, int nlocal, int nu
     return ctas > kPlanMaxCtas ? kPlanMaxCtas : (ctas < 1 ? 1 : ctas);
 }
 
+// Only where the ranks of a group are hosted together: with ranks on other devices it is not measured.
+bool plan_rehearses(const PlanCall& call, int num_sms) {
+    return call.threads == kPlanMaxThreads && call.nlocal == call.N && call.N > 1 && call.R > 0 && call.legacy == 0 &&
+           call.nlocal * call.ctas_per_rank < num_sms;
+}
+
 cudaError_t launch_plan(const PlanCall& call, cudaStream_t stream) {
     const size_t smem = plan_smem_bytes(call.N, call.G, call.M, call.R);
-    cudaError_t e = allow_smem(reinterpret_cast<const void*>(plan_kernel), smem);
+    const auto kernel = call.threads == kPlanMaxThreads ? plan_kernel<kPlanMaxThreads> : plan_kernel<kPlanMaxThreads / 2>;
+    cudaError_t e = allow_smem(reinterpret_cast<const void*>(kernel), smem);
     if (e != cudaSuccess) return e;
     const dim3 grid(call.nlocal * call.ctas_per_rank + call.rehearsal), block(call.threads);
     count_launch();
@@ -527,9 +538,9 @@ cudaError_t launch_plan(const PlanCall& call, cudaStream_t stream) {
         // ranks wait for each other inside the kernel: co-residency is required
         PlanCall copy = call;
         void* args[] = {&copy};
-        return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(plan_kernel), grid, block, args, smem, stream);
+        return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), grid, block, args, smem, stream);
     }
-    plan_kernel<<<grid, block, smem, stream>>>(call);
+    kernel<<<grid, block, smem, stream>>>(call);
     return cudaGetLastError();
 }
 
