@@ -439,9 +439,14 @@ dense_scatter_kernel(Batch<DenseFwdArgs> batch, int L, int P, int D, int quota_m
         for (int e = tid; e < L; e += blockDim.x) {  // experts with one instance
             const int p = s.place[e] - p_lo;
             if (s.place[e] < 0 || p < 0 || p >= cols) continue;
-            s.expert_of[p] = static_cast<uint16_t>(e);
+            bool any = false;  // a caller's table may have the column for another expert too, which the tile routes to
 #pragma unroll
-            for (int g = 0; g < kDenseSegs; ++g) s.phys_bits[g * Cq + p] = s.bits[g * Lq + e];
+            for (int g = 0; g < kDenseSegs; ++g) {
+                const uint8_t b = s.bits[g * Lq + e];
+                if (b != 0) s.phys_bits[g * Cq + p] = b;
+                any = any || b != 0;
+            }
+            if (any) s.expert_of[p] = static_cast<uint16_t>(e);
         }
         if (p_lo == 0 && overlapped) pdl_wait();
         if (p_lo == 0) pdl_launch_dependents();
