@@ -50,6 +50,9 @@ namespace uep {
 namespace {
 
 constexpr int kSyncThreads = 128, kSyncMaxThreads = 256;  // launch_weight_sync
+// Of the smaller rings: a launch whose CTAs wait for each other counts on them, so the registers have to allow them. (64 each; without
+// a bound the direct kernel took 48 and spilled: step of 8192 x 128 bool rows with bf16 experts 64.7 us and 64.2.)
+constexpr int kSyncMaxCtasPerSm = 4;
 constexpr int kMaxSends = kMaxExportsPerDomain;  // replicas of one rank's masters never exceed G*R <= 512
 constexpr int kMaxFwd = 64;                       // replica slots of the hosted ranks that may forward
 constexpr int kMaxRelayReplicas = 16;
@@ -166,7 +169,7 @@ __device__ void copy_plain(const uint8_t* src, uint8_t* dst, int bytes, bool str
 // its per-tile bookkeeping (the kernel runs once per layer from a cold instruction cache, and the one
 // issuing thread per CTA is on the critical path of every tile).
 template <int kSyncTile, int kSyncStages, bool kRelay>
-__global__ void __launch_bounds__(kSyncMaxThreads) weight_sync_kernel(SyncCall call) {
+__global__ void __launch_bounds__(kSyncMaxThreads, kSyncMaxCtasPerSm) weight_sync_kernel(SyncCall call) {
     extern __shared__ __align__(128) char smem_raw[];  // kSyncStages * kSyncTile, then SyncShared
     SyncShared& sm = *reinterpret_cast<SyncShared*>(smem_raw + static_cast<size_t>(kSyncStages) * kSyncTile);
     uint64_t* bars = sm.bars;
@@ -956,10 +959,10 @@ size_t sync_smem_bytes(const SyncGeometry& g, bool relay) {
 }  // namespace
 
 int weight_sync_max_ctas_per_rank(int nlocal, int num_sms) {
-    // CTAs that fit one wave: shared memory bounds the CTAs per SM; hosted ranks share the device
+    // CTAs that fit one wave: shared memory and kSyncMaxCtasPerSm bound the CTAs per SM; hosted ranks share the device
     const size_t smem = sync_smem_bytes(sync_geometry(), true) + 1024;
     int per_sm = static_cast<int>((227 * 1024) / smem);
-    per_sm = per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm);
+    per_sm = per_sm < 1 ? 1 : (per_sm > kSyncMaxCtasPerSm ? kSyncMaxCtasPerSm : per_sm);
     const int per = num_sms * per_sm / (nlocal > 0 ? nlocal : 1);
     return per < 1 ? 1 : per;
 }
