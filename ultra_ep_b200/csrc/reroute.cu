@@ -205,8 +205,9 @@ __device__ __forceinline__ bool dense_fast_path(const uint8_t* map, int L) {
 }
 
 // TILES tiles a CTA: one or four (launch_dense_forward).
+constexpr int kCountCtasPerSm = 5;  // at 48 registers
 template <int TILES>
-__global__ void __launch_bounds__(kRerouteThreads) dense_count_kernel(Batch<DenseFwdArgs> batch, int L, int wait_first) {
+__global__ void __launch_bounds__(kRerouteThreads, kCountCtasPerSm) dense_count_kernel(Batch<DenseFwdArgs> batch, int L, int wait_first) {
     if (wait_first) pdl_wait();  // ahead of every read: the kernel in front may still be writing the map
     pdl_launch_dependents();  // the scatter kernel may start its prologue now
     extern __shared__ __align__(128) char smem_raw[];  // [TILES][pad4(L)] counts, one byte each
@@ -298,8 +299,8 @@ __device__ __forceinline__ int sum_earlier_tiles(const uint8_t* counts, int tile
 // the warp that resolves it, in a few words of its own; shared memory is 4 KB at 128 experts. With all plan rows staged, all
 // experts' tiles added up by every CTA (15 KB) and eight rows a thread, and like this (us): the pair for eight ranks of 8192 tokens
 // and 128 experts 30.0 and 27.3, of 4096 17.0 and 13.7; step of 8192 x 128 with bf16 experts of 9 MB 67.1 and 64.2, of 2000 x 256 with
-// 3 MB 52.3 and 49.4; one rank of 8191 x 256, sparse, dense and backward, 31.9 and 27.9. 64 registers: with 40 (six CTAs an SM) 17.7,
-// 32 are spills. Marked cells written over zeros in memory are partial sectors, and rows gathered in shared memory and sent as
+// 3 MB 52.3 and 49.4; one rank of 8191 x 256, sparse, dense and backward, 31.9 and 27.9. 64 registers and one spilled word: with 40 (six CTAs an SM) 17.7,
+// with 32 28. Marked cells written over zeros in memory are partial sectors, and rows gathered in shared memory and sent as
 // bulk stores wait too long for each other: both slower.
 constexpr int kDenseMaxChunkCols = 4096;
 constexpr int kDenseMaxExperts = 1340;
@@ -1153,10 +1154,12 @@ cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int
     const dim3 grid(dense_tiles(max_T), b.n);
     const int chunk = P > kDenseMaxChunkCols ? kDenseMaxChunkCols : P;
     const int sms = std::max(device_sm_count(), 1);
-    // Four tiles a CTA where one each would be more CTAs than the device holds at once and four tiles are one round of loads.
-    // Plan and pair of eight ranks, tile by tile and by four (us): 8192 x 128 51.7 and 49.6; 4096 x 128 34.1 and 34.8, 8192 x 256
-    // (two rounds) 71.6 and 72.7.
-    const bool by_four = L <= 128 && static_cast<int64_t>(grid.x) * b.n > 6 * sms;
+    // Four tiles a CTA where one each would be more CTAs than the device holds at once (kCountCtasPerSm) and four tiles are one round
+    // of loads. Plan and pair of eight ranks of 128 experts, tile by tile and by four, among others / each alone (us): 4096 rows
+    // 30.8/38.7 and 31.2/38.5, 5500 37.6/46.0 and 38.3/45.5, above the line 6000 38.7/47.6 and 38.8/46.5, 7000 42.6/51.4 and 42.4/49.6,
+    // 8000 45.5/54.8 and 45.2/52.2; beside a weight_sync 6000 53.6/62.7 and 53.4/61.0, 7000 56.6/65.2 and 55.5/64.0. 8192 x 256 (two rounds)
+    // 71.6 and 72.7.
+    const bool by_four = L <= 128 && static_cast<int64_t>(grid.x) * b.n > kCountCtasPerSm * sms;
     const auto count = by_four ? dense_count_kernel<4> : dense_count_kernel<1>;
     // up to two tiles per SM the scatter kernel is a chain of phases: more threads shorten each
     const int threads = static_cast<int64_t>(grid.x) * b.n <= 2 * sms ? kDenseMaxThreads : kRerouteThreads;
@@ -1164,7 +1167,8 @@ cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int
     behind_plan = behind_plan && b.n > 1 && pdl_enabled();
     // The first kernel may be on its SMs when whatever is in front of it ends, too: it waits before its first read. (One rank, 8191
     // tokens of 256 experts, sparse, dense and backward one behind the other: 34.1 us with ordinary launches, 32.8 like this. Of
-    // several ranks only behind a plan, as internal.h says.)
+    // several ranks only behind a plan, as internal.h says; not beside a weight_sync, whose set-up the early CTAs would disturb. One
+    // rank beside a weight_sync has others on other devices: then the plan in front of this pair lets nothing start early.)
     const bool early = behind_plan || (b.n == 1 && pdl_enabled());
     cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(dense_scatter_kernel), smem);
     if (e != cudaSuccess) return e;
