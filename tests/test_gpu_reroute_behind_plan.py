@@ -1,13 +1,17 @@
 """The reroute may be on its SMs while the plan in front of it in the stream is still being made. It must use that plan all the
 same, and the ids or maps as the stream leaves them: eager, behind a kernel or another stream's event in between, and replayed as
-a graph. A kernel in between may itself start its dependents early."""
+a graph. A kernel in between may itself start its dependents early. One rank's kernels, forward and backward, one behind the other and
+behind such a kernel."""
 
 import ctypes as C
 
+import numpy as np
 import pytest
 import torch
 
 import gpu_util as G
+from oracle import uep_oracle as O
+from test_gpu_dense_tiles import _random_plan
 from ultra_ep_b200 import capi, sim
 
 pytestmark = pytest.mark.gpu
@@ -325,3 +329,64 @@ def test_gather_behind_positions_of_many(native_lib, cuda_device, n, in_place):
     torch.cuda.synchronize()
     assert not status.any()
     assert torch.equal(pos, want) and torch.equal(out, rows[want.long()])
+
+
+# One rank of eight, 1.2 million cells: the tiles of the backward, and a count kernel in front of both forwards. Each step's inputs are
+# written by the kernel in front of its first reroute, in the memory of the step before, and one scratch serves all of them.
+@pytest.mark.parametrize("dependent", [False, True])
+@pytest.mark.parametrize("backward_first", [False, True])
+def test_one_rank_back_to_back(native_lib, cuda_device, late_write, dependent, backward_first):
+    ranks, masters, slots, tokens, steps = 8, 16, 4, 9600, 5
+    experts, physical = ranks * masters, ranks * (masters + slots)
+    rng = np.random.default_rng(7)
+    popular = np.arange(1, experts + 1) ** -1.2
+    plan = _random_plan(experts, physical, ranks, 5, rng)
+    assert (plan.lcnts > 1).sum() > 10
+    draws, wanted = [], []
+    for step in range(steps):
+        keys = np.log(popular)[rng.permutation(experts)] + rng.gumbel(size=(tokens, experts))
+        ids = np.argsort(-keys, axis=1)[:, :K].astype(np.int32)
+        rmap = np.zeros((tokens, experts), bool)
+        np.put_along_axis(rmap, ids, True, 1)
+        probs = rng.random((tokens, experts), dtype=np.float32)
+        grad = rng.normal(size=(tokens, physical)).astype(np.float32)
+        out_probs, out_map = O.dense_reroute_forward(rmap, probs, plan, physical)
+        expanded = out_map & (rng.random((tokens, 1)) < 0.9)  # the backward's: not what the forward of this step writes
+        draws.append([grad, probs, ids, rmap, expanded])
+        wanted.append((O.sparse_reroute(ids, plan), out_probs, out_map, O.dense_reroute_backward(grad, rmap, expanded, plan)))
+    sources = [torch.cat([torch.from_numpy(np.ascontiguousarray(x)).view(torch.uint8).reshape(-1) for x in d]).to(cuda_device) for d in draws]
+    flat = torch.zeros_like(sources[0])
+    views, at = [], 0
+    for x in draws[0]:
+        part = flat[at:at + x.nbytes]
+        views.append(part.view({"f": torch.float32, "i": torch.int32, "b": torch.bool}[x.dtype.kind]).view(x.shape))
+        at += x.nbytes
+    grad, probs, ids, rmap, expanded = views
+    p = G.plan_to_device(plan, cuda_device)
+    lib, D = capi.lib(), plan.l2p.shape[1]
+    scratch = torch.empty(max(lib.uep_reroute_scratch_elems(tokens, 0, experts), lib.uep_reroute_scratch_elems(tokens, K, experts)),
+                          dtype=torch.int32, device=cuda_device)
+    outs = [(torch.empty((tokens, K), dtype=torch.int32, device=cuda_device), torch.empty((tokens, physical), device=cuda_device),
+             torch.empty((tokens, physical), dtype=torch.bool, device=cuda_device), torch.empty((tokens, experts), device=cuda_device))
+            for _ in range(steps)]
+    l2p, counts, prefix = p["l2p"].data_ptr(), p["lcnts"].data_ptr(), p["rank_quota_prefix"].data_ptr()
+
+    def backward(out):
+        capi.check(lib.uep_dense_reroute_backward(grad.data_ptr(), rmap.data_ptr(), expanded.data_ptr(), l2p, counts, out[3].data_ptr(), tokens,
+                                                  experts, physical, D, G.stream_ptr()))
+
+    torch.cuda.synchronize()
+    for source, out in zip(sources, outs):
+        late_write(flat, source, dependent)
+        if backward_first:
+            backward(out)
+        capi.check(lib.uep_sparse_reroute_i32(ids.data_ptr(), out[0].data_ptr(), tokens, K, experts, l2p, counts, prefix, D, 1, scratch.data_ptr(),
+                                              G.stream_ptr()))
+        capi.check(lib.uep_dense_reroute_forward(rmap.data_ptr(), probs.data_ptr(), l2p, counts, prefix, out[2].data_ptr(), out[1].data_ptr(),
+                                                 scratch.data_ptr(), tokens, experts, physical, D, 1, 1, G.stream_ptr()))
+        if not backward_first:
+            backward(out)
+    torch.cuda.synchronize()
+    for step, (out, want) in enumerate(zip(outs, wanted)):
+        for a, b in zip(out, want):
+            assert np.array_equal(a.cpu().numpy().view(np.uint8), np.ascontiguousarray(b).view(np.uint8)), step

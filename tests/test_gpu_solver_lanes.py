@@ -1,4 +1,4 @@
-"""The placement solver at the edges of its lane layout: 31 to 72 ranks (one, two and three ranks per lane), more than 32
+"""The placement solver where a warp fills its lists of ranks and adds loads up in one, two and three rounds (2 to 72 ranks), with many
 masters per rank, many equal loads, quotients beyond 2^20, several floors; and the plan's histogram at widths that do not
 divide its threads. Against the CPU oracle, whole numbers: bit-exact."""
 

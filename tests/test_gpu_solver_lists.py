@@ -48,3 +48,34 @@ def test_equal_slack_and_floors(native_lib, cuda_device, N, M, R, min_tokens, bt
             loads[:, r * M:r * M + M] = rng.integers(1, 5, size=M) * 64
         loads[:, rng.choice(N) * M] += 16 * i
         _check(loads, M, R, f"equal {i}", min_tokens=min_tokens, balance_threshold=bt, allow_zero=i == 1)
+
+
+def _draw(i):
+    rng = np.random.default_rng(i)
+    nvl = int(rng.choice([2, 3, 4, 8, 16, 31, 48, 72]))
+    N = 2 * nvl if nvl <= 8 and i % 3 == 0 else nvl
+    M, R = int(rng.integers(1, min(7, 512 // nvl) + 1)), int(rng.integers(1, min(4, 512 // nvl) + 1))
+    total = int(rng.integers(50, 30000))
+    if i % 2:
+        w = rng.permutation(np.arange(1, N * M + 1) ** -float(rng.uniform(0.5, 2.5)))
+    else:  # some ranks hold nearly everything in even masters: more exports than slots, or (four slots) exports below the dynamic floor
+        w = np.where(np.repeat(rng.random(N) < rng.uniform(0.3, 0.8), M), rng.uniform(0.5, 1.0, N * M), 0.01)
+        R = 1 if i % 4 else min(4, 512 // nvl)
+    loads = rng.multinomial(total, w / w.sum(), size=N).astype(np.int32)
+    return Cs.SolveCase(f"sweep {i}", loads, M, R, nvl, balance_threshold=[1.0, 1.0, 1.02, 1.5][i % 4], min_tokens=[-3, 0, 1, 16, 200, 1024][i // 2 % 6],
+                        allow_zero=i % 5 == 0, locality=i % 3 != 0, eps=[0.0, 0.01, 0.1][i % 3], ranks=(i % N,))
+
+
+def test_every_way_through_the_search(native_lib, cuda_device):
+    ways, rounds = set(), set()
+    for i in range(300):
+        case = _draw(i)
+        rank = case.ranks[0]
+        plan = O.solve_placement(case.loads_per_rank, case.M, case.R, case.nvl, rank, G.oracle_params(case))
+        out = G.cuda_solve(case, rank)
+        for f in G.PLAN_FIELDS:
+            assert np.array_equal(out[f].cpu().numpy(), getattr(plan, f)), (i, f)
+        assert out["status"].tolist() == [0, 0]
+        ways |= {int(x) & 15 for x in plan.path}
+        rounds |= {int(x) >> 12 & 255 for x in plan.path}
+    assert ways == {1, 2, 3} and max(rounds) >= 5  # the builds side by side, the capacity threshold, the probes and how many rounds of them
