@@ -56,8 +56,9 @@ __device__ __forceinline__ void hist_add_swar(uint32_t word, int32_t* hist, int 
 
 // Count this CTA's slice of the input into hist[L] (shared memory, zeroed by the caller).
 // part / nparts split the rows (dense) or the entries (sparse) evenly.
-// (not inlined: its vector-load registers must not add to the solver's register pressure in plan_kernel)
-__device__ __noinline__ void histogram_slice(int input_kind, const void* input, int T, int K_or_L, int L, int part, int nparts,
+// Inlined, so that a cold kernel does not jump for it first. Counts of 33 tokens of 64 experts behind an L2 flush, out of line and like
+// this: 4.2 us after the start and 2.2, 4096 tokens 5.1 and 3.6; among other plans 1.9 and 1.6, 3.4 and 3.0.
+__device__ __forceinline__ void histogram_slice(int input_kind, const void* input, int T, int K_or_L, int L, int part, int nparts,
                                 int32_t* hist) {
     const int tid = threadIdx.x, nthreads = blockDim.x;
     if (input_kind == 0) {

@@ -16,9 +16,9 @@
 //   * the loads come in shared memory from the caller, and with one domain the per-rank load matrix
 //     too where it fits (plan.cu); else the few entries of it that are needed are read through L2.
 // All of it is latency of one CTA: dependent instructions of some ten cycles each, so what counts is how many of them follow one
-// another. Calls of uep_solve_placement among others on one B200: 64 ranks x 4 experts x 2 slots 20.5 us (25.9 with the lists in
+// another. Calls of uep_solve_placement among others on one B200: 64 ranks x 4 experts x 2 slots 20.6 us (25.9 with the lists in
 // the lanes of a warp, slots handed out and experts split behind the build); plan and reroute of eight ranks, 33 tokens of 64
-// experts each, 16.7 (18.4).
+// experts each, 15.8 (18.4).
 #pragma once
 
 #include <climits>
@@ -239,8 +239,10 @@ __device__ bool drain_sources(const SolverSmem& sm, int warp, int buffer, int& n
 }
 
 // Out of line: loads that need it are rare, and code that is jumped over is fetched all the same (below).
-__device__ __noinline__ bool drain_sources_wide(SolverSmem sm, int warp, int buffer, int& num_batches, int thr, int with_slack, int G, int M, int R,
+__device__ __noinline__ bool drain_sources_wide(int warp, int buffer, int& num_batches, int thr, int with_slack, int G, int M, int R,
                                                 int min_tokens, bool allow_zero_master, bool dynamic_floor, const volatile int* stop) {
+    extern __shared__ __align__(128) char smem_raw[];  // the kernel's: as an argument its address would not be known to be shared
+    const SolverSmem sm = carve_solver_smem(smem_raw, G * M, G, R);
     return drain_sources<long long>(sm, warp, buffer, num_batches, thr, with_slack, G, M, R, min_tokens, allow_zero_master, dynamic_floor, stop);
 }
 
@@ -269,10 +271,63 @@ __device__ bool warp_build_plan(const SolverSmem& sm, int warp, int buffer, int&
     int ok = 0, made = 0;
     if (lane == 0) {
         ok = narrow ? drain_sources<int>(sm, warp, buffer, made, thr, with_slack, G, M, R, min_tokens, allow_zero_master, dynamic_floor, stop)
-                    : drain_sources_wide(sm, warp, buffer, made, thr, with_slack, G, M, R, min_tokens, allow_zero_master, dynamic_floor, stop);
+                    : drain_sources_wide(warp, buffer, made, thr, with_slack, G, M, R, min_tokens, allow_zero_master, dynamic_floor, stop);
     }
     num_batches = __shfl_sync(kFullMask, made, 0);
     return __shfl_sync(kFullMask, ok, 0) != 0;
+}
+
+// The first warp of a round whose plan is feasible, -1: none; its batches go to num_batches.
+__device__ __forceinline__ int first_feasible(const SolverSmem& sm, int buffer0, int& num_batches) {
+    int first = -1;
+#pragma unroll
+    for (int w = kSolverProbeWarps - 1; w >= 0; --w) {
+        const int built = sm.ctrl[kCtlBuilt0 + buffer0 + w];
+        if (built != 0) {
+            first = w;
+            num_batches = built - 1;
+        }
+    }
+    return first;
+}
+
+// The probes of the search: four a round. Every thread follows the interval, and a round's results are read behind its one barrier: the
+// next round builds into the four buffers that do not hold the best plan so far, and the results of the round after that are
+// written behind the next barrier. (Four barriers a round and the best threshold built again: 16 ranks x 2 experts x 1 slot
+// 20.0 us, 18.8 like this.) Returns the plan's buffer and its batches. All threads of the CTA; the first four warps' buffers hold nothing that counts.
+// Out of line, with a build of its own that knows its floor (one build, in one loop, for these and for the four in front of them: 16
+// ranks x 2 experts x 1 slot 27.4 us for 21.9).
+__device__ __noinline__ int2 probe_thresholds(int fitting, int hi0, int total, int G, int M, int R, int min_tokens, bool allow_zero_master) {
+    extern __shared__ __align__(128) char smem_raw[];  // the kernel's: as an argument its address would not be known to be shared
+    const SolverSmem sm = carve_solver_smem(smem_raw, G * M, G, R);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int lo = min(fitting + 1, hi0), hi = hi0, winner = -1, num_batches = 0;
+    for (int set = kSolverProbeWarps; lo < hi;) {
+        const int range = hi - lo;
+        const bool each = range <= kSolverProbeWarps;
+        auto probe = [&](int w) {
+            return lo + (each ? w : static_cast<int>((static_cast<long long>(range) * (w + 1)) / (kSolverProbeWarps + 1)));
+        };
+        if (warp < kSolverProbeWarps) {
+            int n = 0;
+            const bool ok = (!each || warp < range) &&
+                            warp_build_plan(sm, warp, set + warp, n, probe(warp), total, G, M, R, min_tokens, allow_zero_master, false, lane);
+            if (lane == 0) sm.ctrl[kCtlBuilt0 + set + warp] = ok ? n + 1 : 0;
+        }
+        __syncthreads();
+        const int first = first_feasible(sm, set, num_batches);
+        if (first >= 0) {
+            hi = probe(first);
+            winner = set + first;
+            lo = each ? hi : (first > 0 ? probe(first - 1) + 1 : lo);
+            set ^= kSolverProbeWarps;
+        } else {
+            lo = each ? hi : probe(kSolverProbeWarps - 1) + 1;
+            __syncthreads();  // the same buffers again
+        }
+    }
+    // no probe succeeded: at the largest load nothing is to be moved
+    return winner >= 0 ? make_int2(winner, num_batches) : make_int2(0, 0);
 }
 
 // x = a * b over d, for a, b >= 0 and d > 0: quotient and remainder. A float estimate of a quotient below 2^20 is off by
@@ -593,76 +648,36 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, cha
     int winner = 0, num_batches = 0;  // the buffer whose plan is taken
     if (do_search) {
         // The serial search is: up to three builds with the dynamic floor at rising thresholds; then one build at the
-        // smallest threshold the capacities allow; then the probes below. The first four run at once, one warp each; one that
-        // succeeds stops those behind it. Then four probes a round. Every thread follows the interval, and a round's results are
-        // read behind its one barrier: the next round builds into the four buffers that do not hold the best plan so far, and the
-        // results of the round after that are written behind the next barrier. (Four barriers a round and the best threshold
-        // built again: 16 ranks x 2 experts x 1 slot 20.0 us, 18.8 like this.)
-        // One loop, so that the build is compiled in once: mostly this code comes from DRAM, a line after the other. Plan of eight
-        // ranks behind an L2 flush, on the device (us), with a build in front of the loop and one inside it, for either width of the
-        // keys, and like this: 33 tokens of 64 experts 19.2 and 14.4, 4096 tokens 17.8 and 16.8; among other plans 10.3 and 9.7, 12.8 and 12.7.
+        // smallest threshold the capacities allow; then the probes. The first four run at once, one warp each; one that
+        // succeeds stops those behind it.
+        // Mostly this code comes from DRAM, a line after the other, and what is jumped over comes too: so what a call seldom needs is
+        // out of line (the probes, keys of 64 bits, more than 32 replicas, the legacy solver), and the outputs are compiled in once.
+        // Plan of eight ranks behind an L2 flush, on the device (us), with all builds and widths inlined and like this: 33 tokens of 64
+        // experts 19.3 and 13.3, 4096 tokens 17.8 and 15.7; among other plans 10.3 and 9.5, 12.8 and 11.8.
         const int lo0 = sm.ctrl[kCtlLo], hi0 = sm.ctrl[kCtlHi], total = sm.ctrl[kCtlTotal];
         // The smallest threshold from lo0 to hi0 whose excess fits its slack. Excess minus slack is the sum of (load - threshold):
         // it fits from the mean load on. (The reference bisects, csrc/kernels/placement.cu:76-84.)
         const int fitting = min(max(lo0, total / G + (total % G != 0 ? 1 : 0)), hi0);
-        auto first_feasible = [&](int buffer0) {  // of a round, -1: none; its batches go to num_batches
-            int first = -1;
-#pragma unroll
-            for (int w = kSolverProbeWarps - 1; w >= 0; --w) {
-                const int built = sm.ctrl[kCtlBuilt0 + buffer0 + w];
-                if (built != 0) {
-                    first = w;
-                    num_batches = built - 1;
-                }
+        if (warp < kSolverProbeWarps) {
+            const bool fast = warp < kSolverProbeWarps - 1;
+            int thr = fitting;
+            if (fast) {
+                const float eps = fmaxf(a.eps, 0.0f);
+                thr = max(static_cast<int>(ceilf(__fmul_rn(static_cast<float>(lo0), __fadd_rn(1.0f, eps)))), lo0);
+                const int step = max(1, (hi0 + 99) / 100);
+                for (int i = 0; i < warp; ++i) thr = min(hi0, thr + step);
             }
-            return first;
-        };
-        winner = -1;
-        int lo = lo0, hi = hi0, set = 0;  // set: the buffers of the round
-        bool probing = false;
-        while (true) {
-            const int range = hi - lo;
-            const bool each = range <= kSolverProbeWarps;
-            auto probe = [&](int w) {
-                return lo + (each ? w : static_cast<int>((static_cast<long long>(range) * (w + 1)) / (kSolverProbeWarps + 1)));
-            };
-            if (warp < kSolverProbeWarps) {
-                const bool fast = !probing && warp < kSolverProbeWarps - 1, builds = !probing || !each || warp < range;
-                int thr = probing ? probe(warp) : fitting;
-                if (fast) {
-                    const float eps = fmaxf(a.eps, 0.0f);
-                    thr = max(static_cast<int>(ceilf(__fmul_rn(static_cast<float>(lo0), __fadd_rn(1.0f, eps)))), lo0);
-                    const int step = max(1, (hi0 + 99) / 100);
-                    for (int i = 0; i < warp; ++i) thr = min(hi0, thr + step);
-                }
-                int n = 0;
-                const bool ok = builds && warp_build_plan(sm, warp, set + warp, n, thr, total, G, M, R, a.min_tokens, allow0, fast, lane,
-                                                          probing ? nullptr : sm.ctrl + kCtlStop0 + warp);
-                if (lane == 0) sm.ctrl[kCtlBuilt0 + set + warp] = ok ? n + 1 : 0;
-                if (!probing && ok && lane > warp && lane < kSolverProbeWarps) *(sm.ctrl + kCtlStop0 + lane) = 1;
-            }
-            __syncthreads();
-            const int first = first_feasible(set);
-            if (first >= 0) winner = set + first;
-            if (!probing) {
-                if (first >= 0) break;
-                probing = true;
-                lo = min(fitting + 1, hi0);
-                set = kSolverProbeWarps;
-            } else if (first >= 0) {
-                hi = probe(first);
-                lo = each ? hi : (first > 0 ? probe(first - 1) + 1 : lo);
-                set ^= kSolverProbeWarps;
-            } else {
-                lo = each ? hi : probe(kSolverProbeWarps - 1) + 1;
-                __syncthreads();  // the same buffers again
-            }
-            if (lo >= hi) break;
+            int n = 0;
+            const bool ok = warp_build_plan(sm, warp, warp, n, thr, total, G, M, R, a.min_tokens, allow0, fast, lane, sm.ctrl + kCtlStop0 + warp);
+            if (lane == 0) sm.ctrl[kCtlBuilt0 + warp] = ok ? n + 1 : 0;
+            if (ok && lane > warp && lane < kSolverProbeWarps) *(sm.ctrl + kCtlStop0 + lane) = 1;
         }
-        // No probe succeeded: at the largest load nothing is to be moved.
-        if (winner < 0) {
-            winner = 0;
-            num_batches = 0;
+        __syncthreads();
+        winner = first_feasible(sm, 0, num_batches);
+        if (__builtin_expect(winner < 0, 0)) {
+            const int2 found = probe_thresholds(fitting, hi0, total, G, M, R, a.min_tokens, allow0);
+            winner = found.x;
+            num_batches = found.y;
         }
     }
     stamp(3);
