@@ -4,10 +4,12 @@ floors that fail. Against the CPU oracle, whole numbers: bit-exact."""
 
 import numpy as np
 import pytest
+import torch
 
 import cases as Cs
 import gpu_util as G
 from oracle import uep_oracle as O
+from ultra_ep_b200 import sim
 
 pytestmark = pytest.mark.gpu
 
@@ -79,3 +81,47 @@ def test_every_way_through_the_search(native_lib, cuda_device):
         ways |= {int(x) & 15 for x in plan.path}
         rounds |= {int(x) >> 12 & 255 for x in plan.path}
     assert ways == {1, 2, 3} and max(rounds) >= 5  # the builds side by side, the capacity threshold, the probes and how many rounds of them
+
+
+# inputs for either kernel of the plan: 256 threads, and 512 with a rehearsal
+@pytest.mark.parametrize("scale", [1, 60])
+@pytest.mark.parametrize("M,R,legal", [(2, 1, {3}), (5, 1, {3}), (6, 4, {1, 2, 3})])
+def test_probes_of_hosted_plans(native_lib, cuda_device, scale, M, R, legal):
+    N = 8
+    group = sim.SimGroup(sim.make_config(N, M, R, 1, is_train=False, sim=True))
+    ways = set()
+    for seed in range(6):
+        rng = np.random.default_rng(seed)
+        w = np.where(np.repeat(rng.permutation(N) < 4 + seed % 3, M), rng.uniform(0.5, 1.0, N * M), 0.01)
+        loads = (rng.multinomial(12000, w / w.sum(), size=N) * scale).astype(np.int32)
+        ids = [torch.from_numpy(rng.permutation(np.repeat(np.arange(N * M, dtype=np.int32), row))[:, None].copy()).to(cuda_device) for row in loads]
+        group.update_placement(0, ids)
+        torch.cuda.synchronize()
+        group.check_status()
+        for r in range(N):
+            plan = O.solve_placement(loads, M, R, N, r)
+            ways |= {int(x) & 15 for x in plan.path}
+            got = group.plan(r, 0)
+            for f in G.PLAN_FIELDS:
+                assert np.array_equal(got[f].cpu().numpy().reshape(-1), getattr(plan, f).reshape(-1)), (seed, r, f)
+    assert ways <= legal and ways & {2, 3}
+    group.destroy()
+
+
+def test_wide_keys_of_hosted_plans(native_lib, cuda_device):
+    N, M, R = 2, 3, 2
+    loads = np.array([[9000001, 5000000, 4000000, 100, 0, 7], [9000001, 6000000, 2000000, 90, 3, 0]], np.int32)  # thresholds above 2^24
+    assert loads.sum() // N > 1 << 24
+    group = sim.SimGroup(sim.make_config(N, M, R, 1, is_train=False, sim=True))
+    experts = torch.arange(N * M, dtype=torch.int32, device=cuda_device)
+    ids = [torch.repeat_interleave(experts, torch.from_numpy(row).to(cuda_device))[:, None].contiguous() for row in loads]
+    group.update_placement(0, ids)
+    torch.cuda.synchronize()
+    group.check_status()
+    for r in range(N):
+        plan = O.solve_placement(loads, M, R, N, r)
+        assert plan.lcnts.max() == 2
+        got = group.plan(r, 0)
+        for f in G.PLAN_FIELDS:
+            assert np.array_equal(got[f].cpu().numpy().reshape(-1), getattr(plan, f).reshape(-1)), (r, f)
+    group.destroy()
