@@ -194,6 +194,7 @@ __global__ void __launch_bounds__(kHistThreads) histogram_kernel(int input_kind,
 }
 
 // Stateless solve: one CTA per NVLink domain.
+template <bool kLegacy>
 __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(SolveArgs a, int32_t* global_loads_out, int reduce_loads, int staged,
                                                                  DeviceStatus* status) {
     extern __shared__ __align__(128) char smem_raw[];
@@ -229,7 +230,8 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(SolveArgs a, in
         a.preloaded = 1;
         a.staged_loads = staged ? matrix : nullptr;
     }
-    solve_domain_dispatch(a, domain, smem_raw, status);
+    if (kLegacy) legacy_solve_domain(a, domain, smem_raw, status);
+    else solve_domain(a, domain, smem_raw, status);
 }
 
 __global__ void __launch_bounds__(256) init_master_kernel(int32_t* p2l, int32_t* l2p, int32_t* lcnts, int32_t* quota,
@@ -296,7 +298,6 @@ __device__ __forceinline__ void rehearsal_args(const PlanCall& call, char* smem_
     a.locality = call.params.locality_aware;
     a.eps = 0.01f;
     a.my_rank = 0;
-    a.legacy = 0;
     a.preloaded = 1;
     a.staged_loads = matrix;
     a.trace = nullptr;
@@ -305,6 +306,7 @@ __device__ __forceinline__ void rehearsal_args(const PlanCall& call, char* smem_
 
 // Steps 1 to 3 of a rank: counts, exchange, reduction. False: this CTA has handed its counts over and is done, or the loads did not
 // come; else `a` says what to solve.
+template <bool kLegacy>
 __device__ __forceinline__ bool gather_loads(const PlanCall& call, int local, int part, char* smem_raw, SolveArgs& a) {
     __shared__ int s_timeout_peer;
     __shared__ uint64_t s_epoch;
@@ -398,7 +400,7 @@ __device__ __forceinline__ bool gather_loads(const PlanCall& call, int local, in
     }
 
     // With one domain the solver finds the loads in shared memory where it keeps them: its loads are where hist was.
-    const bool preload = call.G == N && !call.legacy;
+    const bool preload = !kLegacy;
     const SolverSmem solver_sm = carve_solver_smem(smem_raw, L, N, call.R);
     const bool staged = preload && plan_matrix_bytes(N, L) > 0;
     int32_t* matrix = reinterpret_cast<int32_t*>(smem_raw + solver_smem_bytes(L, N, call.R));
@@ -461,7 +463,6 @@ __device__ __forceinline__ bool gather_loads(const PlanCall& call, int local, in
     a.locality = call.params.locality_aware;
     a.eps = call.params.oracle_eps;
     a.my_rank = me;
-    a.legacy = call.legacy;
     a.preloaded = preload ? 1 : 0;
     a.staged_loads = staged ? matrix : nullptr;
     a.trace = call.trace != nullptr ? call.trace + (kMaxLocalRanks + local) * 8 : nullptr;
@@ -470,22 +471,23 @@ __device__ __forceinline__ bool gather_loads(const PlanCall& call, int local, in
 
 // The fused per-layer plan kernel. gridDim.x = nlocal * ctas_per_rank, and one more CTA where it is rehearsed, which only the form
 // with more threads can be: without, every output's address is known to be global, and the registers are twice as many.
-template <int THREADS>
+template <int THREADS, bool kLegacy>
 __global__ void __launch_bounds__(THREADS, 1) plan_kernel(PlanCall call) {
     extern __shared__ __align__(128) char smem_raw[];
     // The next kernel of the stream may be on its SMs when the plan ends. Only where every rank of the group is in this launch:
     // a plan that waits for other devices must not have the SMs held meanwhile by CTAs that wait for it.
     if (call.nlocal == call.N) pdl_launch_dependents();
-    const bool rehearses = THREADS == kPlanMaxThreads && static_cast<int>(blockIdx.x) == call.nlocal * call.ctas_per_rank;
+    const bool rehearses = THREADS == kPlanMaxThreads && !kLegacy && static_cast<int>(blockIdx.x) == call.nlocal * call.ctas_per_rank;
     const int local = rehearses ? 0 : blockIdx.x / call.ctas_per_rank;
     SolveArgs a;
     if (rehearses) {
         rehearsal_args(call, smem_raw, a);
-    } else if (!gather_loads(call, local, blockIdx.x % call.ctas_per_rank, smem_raw, a)) {
+    } else if (!gather_loads<kLegacy>(call, local, blockIdx.x % call.ctas_per_rank, smem_raw, a)) {
         return;
     }
-    const int num_domains = a.N / a.G;
-    for (int d = 0; d < num_domains; ++d) solve_domain_dispatch(a, d, smem_raw, rehearses ? nullptr : call.group.status[local]);
+    DeviceStatus* const status = rehearses ? nullptr : call.group.status[local];
+    if (kLegacy) legacy_solve_domain(a, 0, smem_raw, status);
+    else solve_domain(a, 0, smem_raw, status);
     if (!rehearses && call.trace != nullptr && threadIdx.x == 0) call.trace[local * 8 + 4] = global_timer_ns();
 }
 
@@ -530,10 +532,11 @@ bool plan_rehearses(const PlanCall& call, int num_sms) {
 
 cudaError_t launch_plan(const PlanCall& call, cudaStream_t stream) {
     const size_t smem = plan_smem_bytes(call.N, call.G, call.M, call.R);
-    const auto kernel = call.threads == kPlanMaxThreads ? plan_kernel<kPlanMaxThreads> : plan_kernel<kPlanMaxThreads / 2>;
+    const auto kernel = call.legacy ? plan_kernel<kPlanMaxThreads / 2, true>
+                                    : (call.threads == kPlanMaxThreads ? plan_kernel<kPlanMaxThreads, false> : plan_kernel<kPlanMaxThreads / 2, false>);
     cudaError_t e = allow_smem(reinterpret_cast<const void*>(kernel), smem);
     if (e != cudaSuccess) return e;
-    const dim3 grid(call.nlocal * call.ctas_per_rank + call.rehearsal), block(call.threads);
+    const dim3 grid(call.nlocal * call.ctas_per_rank + call.rehearsal), block(call.legacy ? kPlanMaxThreads / 2 : call.threads);
     count_launch();
     if (call.nlocal > 1) {
         // ranks wait for each other inside the kernel: co-residency is required
@@ -612,7 +615,6 @@ int uep_solve_placement(const int32_t* loads_per_rank, int32_t* global_loads_out
     a.locality = params->locality_aware;
     a.eps = params->oracle_eps;
     a.my_rank = my_rank;
-    a.legacy = 0;
     a.preloaded = 0;
     a.staged_loads = nullptr;
     a.trace = nullptr;
@@ -621,10 +623,10 @@ int uep_solve_placement(const int32_t* loads_per_rank, int32_t* global_loads_out
     const size_t matrix = sizeof(int32_t) * num_ranks * num_ranks * static_cast<size_t>(M);
     const int staged = nvl_ranks == num_ranks && smem + matrix <= kSolveMaxSmem ? 1 : 0;
     if (staged) smem += matrix;
-    UEP_CUDA_TRY(allow_smem(reinterpret_cast<const void*>(solve_kernel), smem));
+    UEP_CUDA_TRY(allow_smem(reinterpret_cast<const void*>(solve_kernel<false>), smem));
     count_launch();
-    solve_kernel<<<num_ranks / nvl_ranks, kSolveThreads, smem, stream>>>(a, global_loads_out, 1, staged,
-                                                                          reinterpret_cast<DeviceStatus*>(status));
+    solve_kernel<false><<<num_ranks / nvl_ranks, kSolveThreads, smem, stream>>>(a, global_loads_out, 1, staged,
+                                                                                 reinterpret_cast<DeviceStatus*>(status));
     UEP_CUDA_TRY(cudaGetLastError());
     return UEP_OK;
 }
@@ -647,11 +649,10 @@ int uep_legacy_solve_placement(const int32_t* global_loads, int32_t* p2l, int32_
     a.rank_quota_prefix = rank_quota_prefix;
     a.N = num_ranks; a.G = nvl_ranks; a.M = M; a.R = R; a.D = D;
     a.balance_threshold = balance_threshold;
-    a.legacy = 1;
     const size_t smem = legacy_smem_bytes(nvl_ranks * M, nvl_ranks) + 16;
-    UEP_CUDA_TRY(allow_smem(reinterpret_cast<const void*>(solve_kernel), smem));
+    UEP_CUDA_TRY(allow_smem(reinterpret_cast<const void*>(solve_kernel<true>), smem));
     count_launch();
-    solve_kernel<<<num_ranks / nvl_ranks, kSolveThreads, smem, stream>>>(a, nullptr, 0, 0, reinterpret_cast<DeviceStatus*>(status));
+    solve_kernel<true><<<num_ranks / nvl_ranks, kSolveThreads, smem, stream>>>(a, nullptr, 0, 0, reinterpret_cast<DeviceStatus*>(status));
     UEP_CUDA_TRY(cudaGetLastError());
     return UEP_OK;
 }

@@ -5,8 +5,8 @@
 // (csrc/kernels/placement.cu:788-1482 of the reference): same fp32 threshold
 // arithmetic, same tie-breaks, same probe schedule of the threshold search, same
 // largest-remainder splits. The execution is different:
-//   * the ranks with slack wait in two sorted lists, and an expert is drained once, from its one home rank, so a build keeps no
-//     occupancy table and no exported sums, and the walk over the sources ends at the first one below the threshold;
+//   * the ranks wait in the lanes of a warp, which finds the next source and the next taker by a reduction, and an expert is drained
+//     once, from its one home rank, so a build sorts no ranks and keeps no occupancy table and no exported sums;
 //   * the three builds of the fast path and the capacity pre-check run side by side on four
 //     warps (the serial search takes the first that is feasible), while the other warps write
 //     the outputs of all experts as they are without replicas;
@@ -15,10 +15,10 @@
 //   * each rank's masters are ranked by counting instead of a serial insertion sort;
 //   * the loads come in shared memory from the caller, and with one domain the per-rank load matrix
 //     too where it fits (plan.cu); else the few entries of it that are needed are read through L2.
-// All of it is latency of one CTA: dependent instructions of some ten cycles each, so what counts is how many of them follow one
-// another. Calls of uep_solve_placement among others on one B200: 64 ranks x 4 experts x 2 slots 20.6 us (25.9 with the lists in
-// the lanes of a warp, slots handed out and experts split behind the build); plan and reroute of eight ranks, 33 tokens of 64
-// experts each, 15.8 (18.4).
+// All of it is latency of one CTA: what counts is how many dependent instructions follow one another, how many of them branch, and
+// how much code there is, since each line of it is fetched once a launch. Calls of uep_solve_placement among others on one B200: 64
+// ranks x 4 experts x 2 slots 18.6 us (20.6 with sorted lists of ranks, which one lane walked); plan and reroute of eight ranks, 33
+// tokens of 64 experts each, 13.1 (15.6).
 #pragma once
 
 #include <climits>
@@ -28,7 +28,7 @@
 namespace uep {
 
 // An export: tokens moved to a redundant slot. `place`: the slot's physical id inside the domain << 8 | its rank.
-struct ExportEntry {
+struct alignas(8) ExportEntry {
     int quota;
     int place;
 };
@@ -58,30 +58,23 @@ struct SolveArgs {
     int my_rank;
     const int32_t* staged_loads;  // loads_per_rank[N, L] in shared memory, or null
     int preloaded;  // 1: the shared-memory loads and my_loads of the (only) domain are in place already
-    int legacy;  // 1: legacy placement (counts-only greedy, round-robin reroute) instead of the quota solver
     unsigned long long* trace;  // optional: 8 globaltimer stamps of the solver phases (tuning aid), or null
 };
 
 constexpr int kSolverProbeWarps = 4;
-constexpr int kMaxListed = kMaxRanksPerDomain + 2;  // ranks of a list, and its end
-
 constexpr int kSolverBuffers = 2 * kSolverProbeWarps;  // plans: one the search may end with, and those of the present round
 
 // Control words in shared memory. kCtlBuilt0: of a buffer's plan, 0 if it is not feasible, else its batches plus one.
-enum SolverCtrl { kCtlLo = 0, kCtlHi, kCtlTotal, kCtlStop0, kCtlBuilt0 = kCtlStop0 + kSolverProbeWarps, kCtlCount = kCtlBuilt0 + kSolverBuffers };
+enum SolverCtrl { kCtlFitting = 0, kCtlHi, kCtlTotal, kCtlLargest, kCtlStop0, kCtlBuilt0 = kCtlStop0 + kSolverProbeWarps, kCtlCount = kCtlBuilt0 + kSolverBuffers };
 static_assert(kCtlCount <= 32, "control words");
 
 struct SolverSmem {
     int32_t* loads;      // [E]
     int32_t* my_loads;   // [E]
     int2* masters;       // [E] rank after rank: {load, expert}, largest load first, ties to the lower expert
-    int4* source;        // [G] {load, rank, its largest master's load and number}, largest load first, ties to the lower rank
-    int2* sink;          // [G] {load, rank}, smallest first, likewise
     int32_t* rank_load;  // [G]
     ExportEntry* plan;   // [kSolverBuffers][slots]
     uint32_t* batches;   // [kSolverBuffers][slots]
-    long long* fresh;    // [4][kMaxListed] lists of ranks of the four warps
-    longlong2* again;    // [4][kMaxListed]
     int* ctrl;           // [kCtlCount]
     int slots;           // redundant slots of the domain, the most exports of a plan (rounded up)
 };
@@ -89,9 +82,8 @@ struct SolverSmem {
 __host__ __device__ inline int solver_ns(int G) { return (G + 31) / 32; }
 __host__ __device__ inline int solver_pad(int n) { return (n + 3) / 4 * 4; }
 __host__ __device__ inline size_t solver_smem_bytes(int E, int G, int R) {
-    return sizeof(int32_t) * (4 * static_cast<size_t>(solver_pad(E)) + 7 * solver_pad(G)) +
-           kSolverBuffers * (sizeof(ExportEntry) + sizeof(uint32_t)) * solver_pad(G * R) +
-           kSolverProbeWarps * 3 * sizeof(long long) * kMaxListed + sizeof(int) * 32;
+    return sizeof(int32_t) * (4 * static_cast<size_t>(solver_pad(E)) + solver_pad(G)) +
+           kSolverBuffers * (sizeof(ExportEntry) + sizeof(uint32_t)) * solver_pad(G * R) + sizeof(int) * 32;
 }
 
 __device__ inline SolverSmem carve_solver_smem(char* raw, int E, int G, int R) {
@@ -101,13 +93,9 @@ __device__ inline SolverSmem carve_solver_smem(char* raw, int E, int G, int R) {
     s.loads = p; p += ep;
     s.my_loads = p; p += ep;
     s.masters = reinterpret_cast<int2*>(p); p += 2 * ep;
-    s.source = reinterpret_cast<int4*>(p); p += 4 * gp;
-    s.sink = reinterpret_cast<int2*>(p); p += 2 * gp;
     s.rank_load = p; p += gp;
     s.plan = reinterpret_cast<ExportEntry*>(p); p += kSolverBuffers * 2 * slots;
     s.batches = reinterpret_cast<uint32_t*>(p); p += kSolverBuffers * slots;
-    s.again = reinterpret_cast<longlong2*>(p); p += kSolverProbeWarps * 4 * kMaxListed;
-    s.fresh = reinterpret_cast<long long*>(p); p += kSolverProbeWarps * 2 * kMaxListed;
     s.ctrl = reinterpret_cast<int*>(p);
     s.slots = slots;
     return s;
@@ -122,159 +110,164 @@ __device__ __forceinline__ int warp_inclusive_scan(int v, int lane) {
     return v;
 }
 
-// A rank that an export has used already and that has slack and slots left, as a key (below) and the slots used.
-template <typename Key>
-struct WaitingRank {
-    Key key;
-    int slots;
-};
-static_assert(sizeof(WaitingRank<long long>) == 16, "two words of two");
-
 // Greedy export plan for one threshold, by one warp. Returns feasibility (uniform over
 // the warp). Semantics of csrc/kernels/placement.cu:337-667 of the reference.
 //
-// An expert's exports go to the ranks by slack, largest first, ties to the lower rank, each rank once; every one of them is
-// filled up except the last, which comes back with the slack it has left once the expert is placed. So the ranks wait in two
-// lists, both sorted: those that no export has used (`fresh`, in the order of sm.sink) and those that came back (`again`, the
-// best at its end), and an export takes the better of the two heads. A rank in a list is a key, slack << 7 | 127 - rank: the
-// larger one is the better one, and the ends of the lists are -1. A chain of dependent steps by nature, so one lane runs it,
-// with few instructions and branches an export, and what it will need next is asked for one export and one expert ahead. (The
-// lists in the lanes of a warp and all exports of an expert in one step: ballots, shuffles and the branches around them were
-// 1000 cycles an expert.) There are never more exports than redundant slots (kMaxExportsPerDomain).
-// Key: int where slack << 7 fits, long long beyond. `stop`: raised by a warp whose result makes this build pointless.
-template <typename Key>
-__device__ bool drain_sources(const SolverSmem& sm, int warp, int buffer, int& num_batches, int thr, int with_slack, int G, int M, int R,
-                              int min_tokens, bool allow_zero_master, bool dynamic_floor, const volatile int* stop) {
+// The ranks above the threshold give experts away, largest load first, ties to the lower rank, and of each its masters, likewise. An
+// expert's exports go to the ranks below it by slack, largest first, ties to the lower rank, each rank once; every one of them is
+// filled up except the last, which comes back with the slack it has left once the expert is placed. A chain of dependent steps by
+// nature. A lane holds the ranks lane, lane + 32, .. as keys, amount << 7 | 127 - rank, -1 where there is none, so that the next rank is
+// the warp's largest key: one reduction, and its lane notices by itself that it was chosen. All the rest of an export is the same few
+// instructions in every lane, with one branch, and the next source and its master are asked for beside the exports of this one.
+// An export takes some 55 cycles, a source 290 (sorted lists in shared memory, walked by one lane: several loads and selects an
+// export. By group, ranks x experts x slots, calls among others with the lists and like this (us): 16 x 7 x 4 10.4 and 10.2, 32 x 4 x 2
+// 12.5 and 10.6, 48 x 7 x 4 19.2 and 17.0, 72 x 7 x 1 22.7 and 21.8, 72 x 7 x 4 28.1 and 23.9; with rounds of probes, 16 x 2 x 1, 21.3 both. All
+// exports of an expert in one step, by ballots and shuffles: 1000 cycles an expert. The list of up to eight ranks in the registers
+// of one lane, the best one first: builds of a plan of eight ranks 2.7 us, 2.0 like this.)
+// kKeys: keys a lane. kWide: a key is the amount alone, where amount << 7 does not fit 31 bits, and the rank is a second reduction.
+// kProbe: the floor is static, and nobody stops the build; else `stop` is raised by a warp whose result makes it pointless.
+template <int kKeys, bool kWide, bool kProbe>
+__device__ __forceinline__ bool drain_sources(const SolverSmem& sm, int buffer, int& num_batches, int thr, int G, int M, int R, int min_tokens,
+                                              bool allow_zero_master, bool dynamic_floor, int lane, const volatile int* stop) {
     ExportEntry* const plan = sm.plan + buffer * sm.slots;
     uint32_t* const batches = sm.batches + buffer * sm.slots;
-    const Key* const fresh_keys = reinterpret_cast<const Key*>(sm.fresh + warp * kMaxListed);
-    WaitingRank<Key>* const again = reinterpret_cast<WaitingRank<Key>*>(sm.again + warp * kMaxListed) + 2;  // [-2], [-1]: its end
-    const WaitingRank<Key> none{Key(-1), 0};
-    again[-2] = none;
-    again[-1] = none;
-    const int keep = allow_zero_master ? 0 : 1, by_count = dynamic_floor ? 1 : 0, Lp = M + R;
-    int used = 0, waiting = 0;  // of `fresh`; in `again`
-    Key fresh = fresh_keys[0], fresh_next = fresh_keys[1];
-    WaitingRank<Key> top = none, top_next = none;
-    int count = with_slack;  // ranks in both lists
-    int num_exports = 0, ord = 0, left = M, stopped = 0;
-    int4 source = sm.source[0], next_source = sm.source[min(1, G - 1)];
-    int need = source.x - thr, at_master = source.y * M;
-    int2 master = make_int2(source.z, source.w);
+    const int keep = allow_zero_master ? 0 : 1, Lp = M + R;
+    auto encode = [](int amount, int rank) { return kWide ? amount : amount << 7 | (127 - rank); };
+    auto amount_of = [](int key) { return kWide ? key : key >> 7; };
+    auto largest = [&](const int (&key)[kKeys]) {
+        int mine = key[0];
+#pragma unroll
+        for (int k = 1; k < kKeys; ++k) mine = max(mine, key[k]);
+        return __reduce_max_sync(kFullMask, mine);
+    };
+    auto rank_of = [&](const int (&key)[kKeys], int best) {
+        if (!kWide) return 127 - (best & 127);
+        int r = INT_MAX;  // the lowest one that has it
+#pragma unroll
+        for (int k = kKeys - 1; k >= 0; --k) r = key[k] == best ? lane + k * kWarp : r;
+        return __reduce_min_sync(kFullMask, r);
+    };
+    int above[kKeys], below[kKeys];  // keys of the excess, of the slack
+    int place[kKeys], last[kKeys];   // of the rank's next redundant slot, as the plan has it, and of the one behind its last
+#pragma unroll
+    for (int k = 0; k < kKeys; ++k) {
+        const int rank = lane + k * kWarp, load = rank < G ? sm.rank_load[rank] : thr;
+        above[k] = load > thr ? encode(load - thr, rank) : -1;
+        below[k] = load < thr ? encode(thr - load, rank) : -1;
+        place[k] = (rank * Lp + M) << 8 | rank;
+        last[k] = place[k] + (R << 8);
+    }
+    const int first_source = largest(above);
+    int need = amount_of(first_source), from = rank_of(above, first_source), at_master = from * M;
+    int2 master = sm.masters[at_master];
+    int num_exports = 0, left = M, stopped = 0;
+    num_batches = 0;
     while (true) {
-        const int2 follow = sm.masters[min(at_master + 1, G * M - 1)];
-        if (stopped != 0) return false;
-        if (stop != nullptr) stopped = *stop;
+        // what only the next expert needs: its source if this one is the source's last, its master; and whether to go on at all
+#pragma unroll
+        for (int k = 0; k < kKeys; ++k) above[k] = from == lane + k * kWarp ? -1 : above[k];
+        const int next_source = largest(above);
+        int count = 0;  // ranks with slack and slots
+        if (!kProbe) {
+#pragma unroll
+            for (int k = 0; k < kKeys; ++k) count += __popc(__ballot_sync(kFullMask, below[k] >= 0));
+            if (__any_sync(kFullMask, stopped != 0)) return false;
+            stopped = *stop;
+        }
+        const int next_from = next_source >= 0 ? rank_of(above, next_source) : 0;
+        const int2 next_master = sm.masters[next_from * M], follow = sm.masters[min(at_master + 1, G * M - 1)];
+
         const int give = min(need, max(master.x - keep, 0));
         if (give == 0) return false;  // the masters come by load: no later one of this source has anything to give
-        const int first = num_exports;
-        int move = give, q, slots, rest;
         // an export is of at least min_tokens, or (dynamic) of ceil(what is still needed / the ranks that could still take part)
-        int times = dynamic_floor ? count : 1, floor = dynamic_floor ? need : max(min_tokens, 0);
-        Key best;
+        const int by_count = !kProbe && dynamic_floor ? 1 : 0;
+        int times = by_count != 0 ? count : 1, floor = by_count != 0 ? need : max(min_tokens, 0);
+        int move = give, made = 0, best, q;
+        bool small, hit[kKeys];
         do {
-            best = max(fresh, top.key);
-            const int slack = static_cast<int>(best >> 7);
+            best = largest(below);
+            const int slack = amount_of(best), rank = kWide ? rank_of(below, best) : 0;
             q = min(slack, move);
-            if (static_cast<Key>(q) * times < floor) {
-                // No later master of this source has more to give: where this one has made no export, or the best rank's slack is
-                // what is too small, the others fail in the same way. (A threshold with the static floor fails at its first source
-                // mostly; the walk over the other masters was the longest of the four builds.)
-                if (num_exports == first || q == slack) return false;
-                break;
+            small = kWide ? static_cast<long long>(q) * times < floor : q * times < floor;  // with no rank left, too
+#pragma unroll
+            for (int k = 0; k < kKeys; ++k) {
+                hit[k] = kWide ? rank == lane + k * kWarp : below[k] == best;
+                if (hit[k]) plan[num_exports + made] = ExportEntry{q, place[k]};
+                place[k] += hit[k] ? 1 << 8 : 0;
+                below[k] = hit[k] ? -1 : below[k];
             }
-            const bool from_again = top.key > fresh;
-            slots = from_again ? top.slots : 0;
-            const int rank = 127 - static_cast<int>(best & 127);
-            plan[num_exports++] = ExportEntry{q, (rank * Lp + M + slots) << 8 | rank};
+            ++made;
             times -= by_count;
             floor -= by_count * q;
-            move -= q;
-            rest = slack - q;
-            waiting -= from_again ? 1 : 0;
-            used += from_again ? 0 : 1;
-            fresh = from_again ? fresh : fresh_next;
-            top.key = from_again ? top_next.key : top.key;
-            top.slots = from_again ? top_next.slots : top.slots;
-            top_next = again[waiting - 2];
-            fresh_next = fresh_keys[used + 1];
-        } while (move != 0);
-        if (num_exports > first) {
-            batches[num_batches++] = pack_batch(master.y, first, num_exports - first, source.y);
-            need -= give - move;
-            count -= num_exports - first;
-            if (move == 0 && rest > 0 && slots + 1 < R) {
-                const WaitingRank<Key> back{static_cast<Key>(rest) << 7 | (best & 127), slots + 1};
-                int place = waiting++;
-                ++count;
-                if (back.key > top.key) {
-                    again[place] = back;
-                    top_next = top;
-                    top = back;
-                } else {
-                    for (; place > 0; --place) {
-                        const WaitingRank<Key> other = again[place - 1];
-                        if (other.key < back.key) break;
-                        again[place] = other;
-                    }
-                    again[place] = back;
-                    top_next = again[waiting - 2];
+            move -= slack;
+        } while (move > 0 && !small);
+        const int rest = -move;  // of the last one's slack
+        if (small) {
+            // The last one is too small, and is taken back. No later master of this source has more to give: where this one has made
+            // no export, or the best rank's slack is what is too small, the others fail in the same way. (A threshold with the
+            // static floor fails at its first source mostly; the walk over the other masters was the longest of the four builds.)
+            if (made == 1 || rest <= 0) return false;
+            --made;
+            need += q;
+#pragma unroll
+            for (int k = 0; k < kKeys; ++k) {
+                if (hit[k]) {
+                    below[k] = best;
+                    place[k] -= 1 << 8;
                 }
             }
+        } else {
+#pragma unroll
+            for (int k = 0; k < kKeys; ++k) {
+                if (hit[k]) below[k] = rest > 0 && place[k] < last[k] ? encode(rest, lane + k * kWarp) : -1;
+            }
         }
+        if (lane == 0) batches[num_batches] = pack_batch(master.y, num_exports, made, from);
+        ++num_batches;
+        num_exports += made;
+        need -= give;
         if (need > 0) {
             if (--left == 0) return false;
             ++at_master;
             master = follow;
             continue;
         }
-        // sources come by load: behind the first one that is not above the threshold there is none
-        if (++ord == G || (need = next_source.x - thr) <= 0) return true;
+        if (next_source < 0) return true;
         left = M;
-        source = next_source;
-        at_master = source.y * M;
-        master = make_int2(source.z, source.w);
-        next_source = sm.source[min(ord + 1, G - 1)];
+        need = amount_of(next_source);
+        from = next_from;
+        at_master = from * M;
+        master = next_master;
     }
 }
 
-// Out of line: loads that need it are rare, and code that is jumped over is fetched all the same (below).
-__device__ __noinline__ bool drain_sources_wide(int warp, int buffer, int& num_batches, int thr, int with_slack, int G, int M, int R,
-                                                int min_tokens, bool allow_zero_master, bool dynamic_floor, const volatile int* stop) {
+// Out of line: groups and loads that need it are rare where the plan is short of time, and code that is jumped over is fetched all the
+// same (below).
+template <int kKeys, bool kWide, bool kProbe>
+__device__ __noinline__ bool drain_sources_apart(int buffer, int& num_batches, int thr, int G, int M, int R, int min_tokens, bool allow_zero_master,
+                                                 bool dynamic_floor, int lane, const volatile int* stop) {
     extern __shared__ __align__(128) char smem_raw[];  // the kernel's: as an argument its address would not be known to be shared
     const SolverSmem sm = carve_solver_smem(smem_raw, G * M, G, R);
-    return drain_sources<long long>(sm, warp, buffer, num_batches, thr, with_slack, G, M, R, min_tokens, allow_zero_master, dynamic_floor, stop);
+    return drain_sources<kKeys, kWide, kProbe>(sm, buffer, num_batches, thr, G, M, R, min_tokens, allow_zero_master, dynamic_floor, lane, stop);
 }
+constexpr int kMostKeys = (kMaxRanksPerDomain + kWarp - 1) / kWarp;
 
-// By warp `warp` of the first four, into plan buffer `buffer`. `total`: of the domain's loads.
-__device__ bool warp_build_plan(const SolverSmem& sm, int warp, int buffer, int& num_batches, int thr, int total, int G, int M, int R,
-                                int min_tokens, bool allow_zero_master, bool dynamic_floor, int lane, const volatile int* stop = nullptr) {
+// By one warp, into plan buffer `buffer`. `total`, `largest`: of the ranks' loads. kProbe: a static floor, and nobody stops it.
+template <bool kProbe>
+__device__ __forceinline__ bool warp_build_plan(const SolverSmem& sm, int buffer, int& num_batches, int thr, int total, int largest, int G, int M, int R,
+                                                int min_tokens, bool allow_zero_master, bool dynamic_floor, int lane, const volatile int* stop) {
     num_batches = 0;
-    if (sm.source[0].x <= thr) return true;
+    if (largest <= thr) return true;
     // The excess has to fit the slack, and their difference is the sum of (load - threshold). Every export takes the same from
     // both, so the slack left always covers the excess left.
     if (total > static_cast<long long>(G) * thr) return false;
-    const bool narrow = thr < 1 << 24;  // (then a slack times a number of ranks is below 2^31, too)
-    int with_slack = 0;
-    __syncwarp();  // an earlier build of this warp has left its lists
-    for (int i0 = 0; i0 < G + 2; i0 += kWarp) {
-        const int i = i0 + lane;
-        const int2 sink = i < G ? sm.sink[i] : make_int2(thr, 0);
-        const int slack = max(thr - sink.x, 0), code = 127 - sink.y;
-        if (i < G + 2) {
-            if (narrow) reinterpret_cast<int*>(sm.fresh + warp * kMaxListed)[i] = slack > 0 ? slack << 7 | code : -1;
-            else sm.fresh[warp * kMaxListed + i] = slack > 0 ? static_cast<long long>(slack) << 7 | code : -1;
-        }
-        with_slack += __popc(__ballot_sync(kFullMask, slack > 0));
+    const bool narrow = largest < 1 << 24;  // (then a slack times a number of ranks is below 2^31, too)
+    if (narrow && G <= kWarp) {
+        return drain_sources<1, false, kProbe>(sm, buffer, num_batches, thr, G, M, R, min_tokens, allow_zero_master, dynamic_floor, lane, stop);
     }
-    __syncwarp();
-    int ok = 0, made = 0;
-    if (lane == 0) {
-        ok = narrow ? drain_sources<int>(sm, warp, buffer, made, thr, with_slack, G, M, R, min_tokens, allow_zero_master, dynamic_floor, stop)
-                    : drain_sources_wide(warp, buffer, made, thr, with_slack, G, M, R, min_tokens, allow_zero_master, dynamic_floor, stop);
-    }
-    num_batches = __shfl_sync(kFullMask, made, 0);
-    return __shfl_sync(kFullMask, ok, 0) != 0;
+    if (!narrow) return drain_sources_apart<kMostKeys, true, kProbe>(buffer, num_batches, thr, G, M, R, min_tokens, allow_zero_master, dynamic_floor, lane, stop);
+    if (G <= 2 * kWarp) return drain_sources_apart<2, false, kProbe>(buffer, num_batches, thr, G, M, R, min_tokens, allow_zero_master, dynamic_floor, lane, stop);
+    return drain_sources_apart<kMostKeys, false, kProbe>(buffer, num_batches, thr, G, M, R, min_tokens, allow_zero_master, dynamic_floor, lane, stop);
 }
 
 // The first warp of a round whose plan is feasible, -1: none; its batches go to num_batches.
@@ -297,7 +290,7 @@ __device__ __forceinline__ int first_feasible(const SolverSmem& sm, int buffer0,
 // 20.0 us, 18.8 like this.) Returns the plan's buffer and its batches. All threads of the CTA; the first four warps' buffers hold nothing that counts.
 // Out of line, with a build of its own that knows its floor (one build, in one loop, for these and for the four in front of them: 16
 // ranks x 2 experts x 1 slot 27.4 us for 21.9).
-__device__ __noinline__ int2 probe_thresholds(int fitting, int hi0, int total, int G, int M, int R, int min_tokens, bool allow_zero_master) {
+__device__ __noinline__ int2 probe_thresholds(int fitting, int hi0, int total, int largest, int G, int M, int R, int min_tokens, bool allow_zero_master) {
     extern __shared__ __align__(128) char smem_raw[];  // the kernel's: as an argument its address would not be known to be shared
     const SolverSmem sm = carve_solver_smem(smem_raw, G * M, G, R);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -311,7 +304,7 @@ __device__ __noinline__ int2 probe_thresholds(int fitting, int hi0, int total, i
         if (warp < kSolverProbeWarps) {
             int n = 0;
             const bool ok = (!each || warp < range) &&
-                            warp_build_plan(sm, warp, set + warp, n, probe(warp), total, G, M, R, min_tokens, allow_zero_master, false, lane);
+                            warp_build_plan<true>(sm, set + warp, n, probe(warp), total, largest, G, M, R, min_tokens, allow_zero_master, false, lane, nullptr);
             if (lane == 0) sm.ctrl[kCtlBuilt0 + set + warp] = ok ? n + 1 : 0;
         }
         __syncthreads();
@@ -591,52 +584,31 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, cha
     stamp(1);
     __syncthreads();
     if (do_search) {
-        // each rank's masters by load descending, ties to the lower index, and its load
+        // each rank's masters by load descending, ties to the lower index, and its load; four masters a load where they lie so
+        const bool fours = (M & 3) == 0;
         for (int i = tid; i < E; i += nthreads) {
             const int rank = i / M, base = rank * M;
-            const int mine = sm.loads[i];
+            const unsigned mine = static_cast<unsigned>(sm.loads[i]);
             int pos = 0, sum = 0;
-#pragma unroll 8
-            for (int j = base; j < base + M; ++j) {
-                const int other = sm.loads[j];
-                pos += (other > mine || (other == mine && j < i)) ? 1 : 0;
+            auto look = [&](int j, int other) {
+                pos += static_cast<unsigned>(other) + (j < i ? 1u : 0u) > mine ? 1 : 0;
                 sum += other;
-            }
-            sm.masters[base + pos] = make_int2(mine, i);
-            if (i == base) sm.rank_load[rank] = sum;
-        }
-        __syncthreads();
-        for (int i = tid; i < G; i += nthreads) {  // the ranks likewise
-            const int mine = sm.rank_load[i];
-            int above = 0, below = 0, equal = 0;
+            };
+            if (fours) {
+#pragma unroll 4
+                for (int j = base; j < base + M; j += 4) {
+                    const int4 v = *reinterpret_cast<const int4*>(sm.loads + j);
+                    look(j, v.x);
+                    look(j + 1, v.y);
+                    look(j + 2, v.z);
+                    look(j + 3, v.w);
+                }
+            } else {
 #pragma unroll 8
-            for (int j = 0; j < G; ++j) {
-                const int other = sm.rank_load[j];
-                above += other > mine ? 1 : 0;
-                below += other < mine ? 1 : 0;
-                equal += (other == mine && j < i) ? 1 : 0;
+                for (int j = base; j < base + M; ++j) look(j, sm.loads[j]);
             }
-            const int2 largest = sm.masters[i * M];
-            sm.source[above + equal] = make_int4(mine, i, largest.x, largest.y);
-            sm.sink[below + equal] = make_int2(mine, i);
-        }
-        if (warp == kSolverProbeWarps - 1) {
-            int total = 0, mx = 0;
-            for (int r = lane; r < G; r += kWarp) {
-                total += sm.rank_load[r];
-                mx = max(mx, sm.rank_load[r]);
-            }
-            total = warp_sum(total);
-            mx = warp_max(mx);
-            // fp32, in the reference's order: ceilf((float(total) / G) * bt)
-            const float bt = fmaxf(a.balance_threshold, 1.0f);
-            const float mean = __fdiv_rn(static_cast<float>(total), static_cast<float>(G));
-            const int lo = static_cast<int>(ceilf(__fmul_rn(mean, bt)));
-            if (lane == 0) {
-                sm.ctrl[kCtlLo] = lo;
-                sm.ctrl[kCtlHi] = max(mx, lo);
-                sm.ctrl[kCtlTotal] = total;
-            }
+            sm.masters[base + pos] = make_int2(static_cast<int>(mine), i);
+            if (i == base) sm.rank_load[rank] = sum;
         }
         __syncthreads();
     }
@@ -654,28 +626,45 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, cha
         // out of line (the probes, keys of 64 bits, more than 32 replicas, the legacy solver), and the outputs are compiled in once.
         // Plan of eight ranks behind an L2 flush, on the device (us), with all builds and widths inlined and like this: 33 tokens of 64
         // experts 19.3 and 13.3, 4096 tokens 17.8 and 15.7; among other plans 10.3 and 9.5, 12.8 and 11.8.
-        const int lo0 = sm.ctrl[kCtlLo], hi0 = sm.ctrl[kCtlHi], total = sm.ctrl[kCtlTotal];
-        // The smallest threshold from lo0 to hi0 whose excess fits its slack. Excess minus slack is the sum of (load - threshold):
-        // it fits from the mean load on. (The reference bisects, csrc/kernels/placement.cu:76-84.)
-        const int fitting = min(max(lo0, total / G + (total % G != 0 ? 1 : 0)), hi0);
         if (warp < kSolverProbeWarps) {
+            int total = 0, largest = 0;
+            for (int r = lane; r < G; r += kWarp) {
+                total += sm.rank_load[r];
+                largest = max(largest, sm.rank_load[r]);
+            }
+            total = warp_sum(total);
+            largest = warp_max(largest);
+            // fp32, in the reference's order: ceilf((float(total) / G) * bt). A power of two divides by a multiplication.
+            const float bt = fmaxf(a.balance_threshold, 1.0f), sum = static_cast<float>(total), ranks = static_cast<float>(G);
+            const float mean = (G & (G - 1)) == 0 ? __fmul_rn(sum, __uint_as_float(0x7F000000u - __float_as_uint(ranks))) : __fdiv_rn(sum, ranks);
+            const int lo0 = static_cast<int>(ceilf(__fmul_rn(mean, bt))), hi0 = max(largest, lo0);
             const bool fast = warp < kSolverProbeWarps - 1;
-            int thr = fitting;
+            int thr;
             if (fast) {
                 const float eps = fmaxf(a.eps, 0.0f);
                 thr = max(static_cast<int>(ceilf(__fmul_rn(static_cast<float>(lo0), __fadd_rn(1.0f, eps)))), lo0);
                 const int step = max(1, (hi0 + 99) / 100);
                 for (int i = 0; i < warp; ++i) thr = min(hi0, thr + step);
+            } else {
+                // The smallest threshold from lo0 to hi0 whose excess fits its slack. Excess minus slack is the sum of (load - threshold):
+                // it fits from the mean load on. (The reference bisects, csrc/kernels/placement.cu:76-84.)
+                thr = min(max(lo0, static_cast<int>((static_cast<unsigned>(total) + G - 1) / G)), hi0);
+                if (lane == 0) {
+                    sm.ctrl[kCtlFitting] = thr;
+                    sm.ctrl[kCtlHi] = hi0;
+                    sm.ctrl[kCtlTotal] = total;
+                    sm.ctrl[kCtlLargest] = largest;
+                }
             }
             int n = 0;
-            const bool ok = warp_build_plan(sm, warp, warp, n, thr, total, G, M, R, a.min_tokens, allow0, fast, lane, sm.ctrl + kCtlStop0 + warp);
+            const bool ok = warp_build_plan<false>(sm, warp, n, thr, total, largest, G, M, R, a.min_tokens, allow0, fast, lane, sm.ctrl + kCtlStop0 + warp);
             if (lane == 0) sm.ctrl[kCtlBuilt0 + warp] = ok ? n + 1 : 0;
             if (ok && lane > warp && lane < kSolverProbeWarps) *(sm.ctrl + kCtlStop0 + lane) = 1;
         }
         __syncthreads();
         winner = first_feasible(sm, 0, num_batches);
         if (__builtin_expect(winner < 0, 0)) {
-            const int2 found = probe_thresholds(fitting, hi0, total, G, M, R, a.min_tokens, allow0);
+            const int2 found = probe_thresholds(sm.ctrl[kCtlFitting], sm.ctrl[kCtlHi], sm.ctrl[kCtlTotal], sm.ctrl[kCtlLargest], G, M, R, a.min_tokens, allow0);
             winner = found.x;
             num_batches = found.y;
         }
@@ -923,15 +912,6 @@ __device__ __noinline__ void legacy_solve_domain(const SolveArgs& a, int domain,
     __syncthreads();
     for (int e = tid; e < E; e += nthreads) a.lcnts[log0 + e] = cnt[e];
     __syncthreads();
-}
-
-__device__ __forceinline__ void solve_domain_dispatch(const SolveArgs& a, int domain, char* smem_raw, DeviceStatus* status) {
-    if (a.legacy) {
-        const SolveArgs copy = a;  // one whose address is taken, so that the other stays in registers and parameters
-        legacy_solve_domain(copy, domain, smem_raw, status);
-        return;
-    }
-    solve_domain(a, domain, smem_raw, status);
 }
 
 }  // namespace uep
