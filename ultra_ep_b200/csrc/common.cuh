@@ -174,6 +174,28 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint64
         if (global_timer_ns() - start > timeout_ns) return false;
     }
 }
+// ---- thread-block clusters: the CTA's number, the barrier, a place of the own shared memory as it lies in another CTA's
+__device__ __forceinline__ int cluster_cta() {
+    int r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ uint32_t cluster_addr(const void* own, int cta) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(own)), "r"(cta));
+    return a;
+}
+// Words into another CTA's shared memory, their bytes counted on an mbarrier beside them.
+__device__ __forceinline__ void push_word(uint32_t to, int32_t v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(to), "r"(v), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void push_v4(uint32_t to, int4 v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(to), "r"(v.x), "r"(v.y),
+                 "r"(v.z), "r"(v.w), "r"(bar)
+                 : "memory");
+}
 __device__ __forceinline__ void fence_mbar_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }

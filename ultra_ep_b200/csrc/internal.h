@@ -17,7 +17,7 @@ constexpr int kReduceSegments = 16;  // a replica's gradient is released for zer
 constexpr unsigned long long kReduceFlagRadix = 64;  // progress word = epoch * radix + segments done
 
 constexpr int kPlanMaxCtas = 32;  // CTAs of one rank in the plan kernel
-constexpr int kPlanMaxThreads = 512;
+constexpr int kRehearsalOut = 256;  // words that the rehearsal of a plan writes
 
 // Where the group's buffers are. By value in the kernels' parameters, so that the first load of a kernel is of data and not
 // of a pointer to it (each of the two is a miss: the tables were last read a layer ago). Fixed once connected. With a table
@@ -76,15 +76,18 @@ struct PlanCall {
     uep_solver_params params;
     uint64_t timeout_ns;
     int ctas_per_rank, threads;
-    int rehearsal;      // 1: one more CTA, which runs the solver on a problem of its own (plan.cu)
+    int rehearsal_smem;      // where its crew's shared memory begins (set by launch_plan)
+    int32_t* rehearsal_out;  // [hosted ranks][kRehearsalOut]
+    int in_cluster;          // 1: the ranks hand each other their rows through the shared memory of their cluster (set by launch_plan)
     int withhold_rank;  // test hook: this rank does not publish its flags (-1: none)
     int legacy;         // 1: legacy placement solver (counts only; the reroute is then round-robin)
     unsigned long long* trace;  // optional: 8 globaltimer stamps per hosted rank (tuning aid), or null
 };
 cudaError_t launch_plan(const PlanCall& call, cudaStream_t stream);
-int plan_ctas_per_rank(int input_kind, int max_T, int K_or_L, int nlocal, int num_sms);
+cudaError_t plan_most_ctas(int nlocal, int N, int G, int M, int R, int* ctas);
+int plan_ctas_per_rank(int input_kind, int max_T, int K_or_L, int cap);
+
 int plan_threads(int input_kind, int max_T, int K_or_L, int ctas);
-bool plan_rehearses(const PlanCall& call, int num_sms);
 
 struct SyncCall {
     GroupDev group;
@@ -156,20 +159,22 @@ struct Batch {
 };
 int64_t dense_scratch_elems(int T, int L);
 int64_t sparse_scratch_elems(int64_t entries, int L);
-// behind_plan: several ranks, and the kernel in front in the stream may be the plan: the first kernel is launched as a dependent
-// of whatever is in front, so that its CTAs are on the SMs when that ends. They read nothing but their parameters before they have
-// waited for it: the kernel in front may as well be one of the caller's that starts its dependents early and writes the ids
-// after that. Plan and reroute of eight ranks, ordinary launches and like this (us): 33 tokens of 64 experts 20.5 and 18.5, 4096
-// tokens 30.2 and 28.9, 8192 of 128 experts 34.3 and 31.6; bool rows, 4096 of 128 experts 46.5 and 42.9. Not beside a
-// weight_sync, whose CTAs read their tables in the microseconds in which the reroute would start (step with fp8 weights,
-// 16384 tokens of 256 experts 117.6 and 130.7; bf16, 8192 bool rows of 128 67.8 and 72.8).
+// Kernels are launched as dependents of whatever is in front of them in their stream, and wait for it before they read anything but
+// parameters (it may as well be a kernel of the caller's that starts its dependents early and writes the ids after that). An ordinary
+// launch starts on the next tick of some 2 us from the start of the kernel in front, 1.8 us at least behind its end; a dependent one is
+// past its wait 0.8 us behind that end whether or not the kernel in front says when it may start. So no kernel here says it, except to
+// one that has something to do before its wait: CTAs that only wait take the place of others. Plan and reroute of eight ranks among
+// others, ordinary launches of the plan and both that start their dependents early, and like this (us): 33 tokens of 64 experts 13.5 and
+// 11.4, 4096 tokens 25.1 and 18.1, bool rows 4096 of 128 experts 28.6 and 24.3; one rank's sparse, dense and backward, 8191 x 256,
+// 28.5 and 25.4. beside_sync, beside_bytes: several ranks and a weight_sync of the plan was launched, which writes at most so many
+// bytes: where its CTAs' first microseconds count, the reroute's launches are ordinary ones (reroute.cu).
 cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int D, int quota_mode, int interleave,
-                                 bool behind_plan, cudaStream_t stream);
+                                 bool beside_sync, cudaStream_t stream);
 cudaError_t launch_dense_backward(const Batch<DenseBwdArgs>& b, int L, int P, int D, cudaStream_t stream);
-// beside_sync: a weight_sync was launched beside it
-cudaError_t launch_sparse_reroute(const Batch<SparseArgs>& b, int ids_kind, int K, int L, int D, int interleave, bool beside_sync,
-                                  bool behind_plan, cudaStream_t stream);
+cudaError_t launch_sparse_reroute(const Batch<SparseArgs>& b, int ids_kind, int K, int L, int D, int interleave, int64_t beside_bytes,
+                                  cudaStream_t stream);
 
+bool pdl_enabled();      // programmatic dependent launches are on (UEP_DISABLE_PDL=1 turns them off)
 int device_sm_count();  // of the current device; launch sizes are multiples of it
 // Lets a kernel use that much dynamic shared memory on the current device (and, once, ask for the largest carve-out).
 cudaError_t allow_smem(const void* fn, size_t bytes, bool largest_carveout = false);

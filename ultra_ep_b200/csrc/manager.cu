@@ -152,8 +152,10 @@ struct uep_manager {
     bool connected = false;
     int grad_reduce_ctas = 42;
     int weight_sync_ctas = 0;
+    int plan_ctas = 1;  // most CTAs of a rank in the plan kernel
     int withhold_rank = -1;
     int relay_cap = 0;  // ready-flag words per replica slot
+    int32_t* rehearsal_out = nullptr;  // written by the plans' rehearsals, read by nobody
     unsigned long long* sync_trace = nullptr;  // UEP_SYNC_TRACE=1: per-CTA phase stamps of the last weight_sync
 };
 
@@ -337,6 +339,7 @@ int uep_manager_create(const uep_config* cfg, uep_manager** out) {
         if (m->comm_stream) cudaStreamDestroy(m->comm_stream);
         if (m->order_event) cudaEventDestroy(m->order_event);
         for (auto e : m->plan_ready) cudaEventDestroy(e);
+        cudaFree(m->rehearsal_out);
         delete m;
         return rc;
     };
@@ -380,6 +383,9 @@ int uep_manager_create(const uep_config* cfg, uep_manager** out) {
     m->plan_recorded.assign(slots, 0);
     m->sync_beside.assign(slots, 0);
     for (int i = 0; i < slots; ++i) UEP_TRY_BAIL(cudaEventCreateWithFlags(&m->plan_ready[i], cudaEventDisableTiming));
+
+    UEP_TRY_BAIL(plan_most_ctas(nlocal, N, G, M, R, &m->plan_ctas));
+    UEP_TRY_BAIL(cudaMalloc(&m->rehearsal_out, sizeof(int32_t) * kRehearsalOut * nlocal));
 
     m->ranks.resize(nlocal);
     for (int i = 0; i < nlocal; ++i) {
@@ -482,6 +488,7 @@ int uep_manager_destroy(uep_manager* m) {
     if (m->order_event) cudaEventDestroy(m->order_event);
     for (auto e : m->plan_ready) cudaEventDestroy(e);
     cudaFree(m->sync_trace);
+    cudaFree(m->rehearsal_out);
     delete m;
     event_pool().manager_gone();
     return UEP_OK;
@@ -640,11 +647,11 @@ int uep_update_placement(uep_manager* m, int layer_id, int input_kind, const voi
     call.N = m->N; call.G = m->G; call.M = m->M; call.R = m->R; call.D = m->D;
     call.params = m->cfg.solver;
     call.timeout_ns = m->timeout_ns;
-    call.ctas_per_rank = plan_ctas_per_rank(input_kind, max_T, K_or_L, m->nlocal, m->num_sms);
+    call.ctas_per_rank = plan_ctas_per_rank(input_kind, max_T, K_or_L, m->plan_ctas);
     call.threads = plan_threads(input_kind, max_T, K_or_L, call.ctas_per_rank);
     call.withhold_rank = m->withhold_rank;
     call.legacy = m->cfg.legacy_placement ? 1 : 0;
-    call.rehearsal = plan_rehearses(call, m->num_sms) ? 1 : 0;
+    call.rehearsal_out = m->rehearsal_out;
     call.trace = m->sync_trace ? m->sync_trace + 8 * 1000 : nullptr;  // the last rows of the trace buffer
     UEP_CUDA_TRY(launch_plan(call, stream));
     const int slot = plan_slot(m, layer_id);
@@ -778,7 +785,7 @@ int uep_reroute_dense_forward(uep_manager* m, int layer_id, const uint8_t* const
     }
     // legacy placement has no quotas: its reroute is round-robin over an expert's instances
     UEP_CUDA_TRY(launch_dense_forward(b, m->L, m->P, m->D, m->cfg.legacy_placement ? 0 : 1, m->cfg.solver.reroute_interleave,
-                                      m->sync_beside[plan_slot(m, layer_id)] == 0, stream));
+                                      m->sync_beside[plan_slot(m, layer_id)] != 0, stream));
     return UEP_OK;
 }
 
@@ -820,9 +827,9 @@ int uep_reroute_sparse(uep_manager* m, int layer_id, int ids_kind, const void* c
         const PlanPtrs p = plan_ptrs(m, m->ranks[i], layer_id);
         b.a[i] = SparseArgs{ids[i], out[i], p.l2p, p.lcnts, p.rank_quota_prefix, m->ranks[i].scratch[1], T[i]};
     }
-    const bool beside_sync = m->sync_beside[plan_slot(m, layer_id)] != 0;
+    const int64_t beside_bytes = m->sync_beside[plan_slot(m, layer_id)] != 0 ? std::max<int64_t>(static_cast<int64_t>(m->N) * m->R * (m->weight_stride + m->scale_stride), 1) : 0;
     UEP_CUDA_TRY(launch_sparse_reroute(b, ids_kind, K, m->L, m->D, m->cfg.legacy_placement ? 2 : m->cfg.solver.reroute_interleave,
-                                       beside_sync, !beside_sync, stream));
+                                       beside_bytes, stream));
     return UEP_OK;
 }
 

@@ -31,8 +31,6 @@ __device__ __forceinline__ void cp_async_4(void* smem_dst, const void* gsrc) {
 }
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 // the four words at the same place of another CTA's shared memory
 __device__ __forceinline__ int4 ld_cluster_v4(const int4* own, int cta) {
     uint32_t a;

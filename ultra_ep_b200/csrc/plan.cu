@@ -16,10 +16,9 @@
 // The gather buffers are double-buffered by epoch parity: a peer can be at most one
 // call ahead, because it cannot pass call e+1 without this rank's row for e+1.
 //
-// With several ranks hosted on one device (simulated EP) the same kernel runs all of
-// them in one cooperative launch, so the ranks that wait for each other are co-resident.
-
-#include <cooperative_groups.h>
+// With several ranks hosted on one device (simulated EP) the same kernel runs all of them in one launch of clusters, a CTA of
+// every rank in each: the first CTAs of the ranks, the only ones that wait for each other, are one cluster and so co-resident,
+// and hand their rows over through its shared memory.
 
 #include <atomic>
 
@@ -34,6 +33,8 @@ namespace uep {
 namespace {
 
 constexpr int kHistThreads = 256;
+constexpr int kPlanThreads = 256;       // of a CTA of the plan kernel
+constexpr int kRehearsalThreads = 128;  // and, where the solver is rehearsed, of its second crew
 constexpr int kIdLoads = 4;  // 16-byte loads of ids that a thread has in flight
 constexpr int kSolveThreads = 512;
 constexpr size_t kSolveMaxSmem = 220 * 1024;
@@ -59,8 +60,8 @@ __device__ __forceinline__ void hist_add_swar(uint32_t word, int32_t* hist, int 
 // Inlined, so that a cold kernel does not jump for it first. Counts of 33 tokens of 64 experts behind an L2 flush, out of line and like
 // this: 4.2 us after the start and 2.2, 4096 tokens 5.1 and 3.6; among other plans 1.9 and 1.6, 3.4 and 3.0.
 __device__ __forceinline__ void histogram_slice(int input_kind, const void* input, int T, int K_or_L, int L, int part, int nparts,
-                                int32_t* hist) {
-    const int tid = threadIdx.x, nthreads = blockDim.x;
+                                int32_t* hist, int nthreads) {
+    const int tid = threadIdx.x;
     if (input_kind == 0) {
         const uint8_t* map = static_cast<const uint8_t*>(input);
         const int rows_per = ceil_div_i(T, nparts);
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(kHistThreads) histogram_kernel(int input_kind,
     int32_t* hist = reinterpret_cast<int32_t*>(smem_raw);
     for (int i = threadIdx.x; i < L; i += blockDim.x) hist[i] = 0;
     __syncthreads();
-    histogram_slice(input_kind, input, T, K_or_L, L, blockIdx.x, gridDim.x, hist);
+    histogram_slice(input_kind, input, T, K_or_L, L, blockIdx.x, gridDim.x, hist, blockDim.x);
     __syncthreads();
     for (int i = threadIdx.x; i < L; i += blockDim.x) {
         if (hist[i]) atomicAdd(loads + i, hist[i]);
@@ -200,6 +201,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(SolveArgs a, in
     extern __shared__ __align__(128) char smem_raw[];
     const int domain = blockIdx.x;
     const int E = a.G * a.M, L = a.N * a.M;
+    pdl_wait();  // ahead of every read
     if (reduce_loads) {
         // Total load of this domain's experts over all ranks, and this rank's own, straight to where the solver keeps
         // them. The rows are shared by all the threads an expert can have, 16 loads of each in flight.
@@ -231,7 +233,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(SolveArgs a, in
         a.staged_loads = staged ? matrix : nullptr;
     }
     if (kLegacy) legacy_solve_domain(a, domain, smem_raw, status);
-    else solve_domain(a, domain, smem_raw, status);
+    else solve_domain(a, Crew{static_cast<int>(threadIdx.x), static_cast<int>(blockDim.x), 0}, domain, smem_raw, status);
 }
 
 __global__ void __launch_bounds__(256) init_master_kernel(int32_t* p2l, int32_t* l2p, int32_t* lcnts, int32_t* quota,
@@ -259,63 +261,69 @@ __host__ __device__ inline size_t plan_matrix_bytes(int N, int L) {
 }
 
 // The solver's code runs once a layer, and what runs between two layers (weight copies, expanded outputs, the model) leaves none of
-// it in L2: its instructions came from DRAM one line after another. Where the input is long, a CTA of its own solves a small problem
-// of its own from the kernel's start, while the others count and exchange, so that the owners find the lines in L2. No owner waits
-// for it, but the launch ends with it too, and a cooperative one needs its SM free. It takes the way of the default parameters:
-// the sorts, the four builds side by side with an expert of two exports and ranks that come back, outputs and splits of experts
-// with replicas; not the rounds of probes nor more than 32 replicas. Outputs stay in its shared memory.
+// it in L2: its instructions came from DRAM one line after another, and from L2 to the SM likewise where they were still there. So the
+// CTA that owns a rank has a second crew of threads, which solves a small problem from the kernel's start, while the first one counts
+// and exchanges, with the same instructions. Nobody waits for it. It takes the way of the default parameters: the sort, the four
+// builds side by side with an expert of two exports and ranks that come back, outputs and splits of experts with replicas; not the rounds
+// of probes nor more than 32 replicas. Its outputs go to a place of their own. Step of eight ranks among others without it and like
+// this (us): bf16 experts of 9 MB, 8192 bool rows of 128 64.3 and 59.2; fp8 experts of 19 MB, 8192 int32 tokens of 128 56.1 and 54.4; plan and
+// reroute of 4096 tokens of 64 18.8 and 18.1, of 33 11.6 and 11.4. (A CTA of its own warms L2 alone: the plan's builds 2.2 us instead of
+// 1.8; half of the ranks with the outputs first 59.2 and 59.3.)
 constexpr int kRehearsalRanks = 4, kRehearsalMasters = 2, kRehearsalSlots = 2, kRehearsalD = 4;
 constexpr int kRehearsalExperts = kRehearsalRanks * kRehearsalMasters;
 constexpr int kRehearsalPhysical = kRehearsalRanks * (kRehearsalMasters + kRehearsalSlots);
+static_assert(4 * kRehearsalExperts * kRehearsalD + kRehearsalExperts + 2 * kRehearsalPhysical <= kRehearsalOut, "room for its outputs");
 __host__ __device__ inline size_t rehearsal_smem_bytes() {
-    return solver_smem_bytes(kRehearsalExperts, kRehearsalRanks, kRehearsalSlots) +
-           sizeof(int32_t) * (kRehearsalRanks * kRehearsalExperts + 4 * kRehearsalExperts * kRehearsalD + kRehearsalExperts + 2 * kRehearsalPhysical);
+    return solver_smem_bytes(kRehearsalExperts, kRehearsalRanks, kRehearsalSlots) + sizeof(int32_t) * kRehearsalRanks * kRehearsalExperts;
 }
 // Two ranks above the mean and two below. The parameters are its own: a caller's threshold or floor could leave it without exports.
-__device__ __forceinline__ void rehearsal_args(const PlanCall& call, char* smem_raw, SolveArgs& a) {
+__device__ __forceinline__ void rehearsal_args(const PlanCall& call, const Crew& crew, int local, char* smem_raw, SolveArgs& a) {
     const SolverSmem sm = carve_solver_smem(smem_raw, kRehearsalExperts, kRehearsalRanks, kRehearsalSlots);
     int32_t* matrix = reinterpret_cast<int32_t*>(smem_raw + solver_smem_bytes(kRehearsalExperts, kRehearsalRanks, kRehearsalSlots));
-    for (int i = threadIdx.x; i < kRehearsalExperts; i += blockDim.x) {
+    for (int i = crew.tid; i < kRehearsalExperts; i += crew.threads) {
         const int load = (i & 1) != 0 ? 100 : 6000 >> 2 * (i >> 2) * (i >> 1);  // 6000, 6000, 375, 93
         sm.loads[i] = load;
         sm.my_loads[i] = load / 4;
         for (int r = 0; r < kRehearsalRanks; ++r) matrix[r * kRehearsalExperts + i] = load / 4;
     }
-    int32_t* out = matrix + kRehearsalRanks * kRehearsalExperts;
-    a.l2p = out; out += kRehearsalExperts * kRehearsalD;
-    a.quota = out; out += kRehearsalExperts * kRehearsalD;
-    a.quota_prefix = out; out += kRehearsalExperts * kRehearsalD;
-    a.rank_quota_prefix = out; out += kRehearsalExperts * kRehearsalD;
-    a.lcnts = out; out += kRehearsalExperts;
-    a.p2l = out; out += kRehearsalPhysical;
-    a.physical_loads = out;
-    a.global_loads = nullptr;
-    a.loads_per_rank = nullptr;
-    a.N = a.G = kRehearsalRanks; a.M = kRehearsalMasters; a.R = kRehearsalSlots; a.D = kRehearsalD;
-    a.balance_threshold = 1.f;
-    a.min_tokens = 1;
-    a.allow_zero_master = 0;
-    a.locality = call.params.locality_aware;
-    a.eps = 0.01f;
-    a.my_rank = 0;
-    a.preloaded = 1;
-    a.staged_loads = matrix;
-    a.trace = nullptr;
-    __syncthreads();
+    if (crew.tid == 0) {
+        int32_t* out = call.rehearsal_out + local * kRehearsalOut;
+        a.l2p = out; out += kRehearsalExperts * kRehearsalD;
+        a.quota = out; out += kRehearsalExperts * kRehearsalD;
+        a.quota_prefix = out; out += kRehearsalExperts * kRehearsalD;
+        a.rank_quota_prefix = out; out += kRehearsalExperts * kRehearsalD;
+        a.lcnts = out; out += kRehearsalExperts;
+        a.p2l = out; out += kRehearsalPhysical;
+        a.physical_loads = out;
+        a.global_loads = nullptr;
+        a.loads_per_rank = nullptr;
+        a.N = a.G = kRehearsalRanks; a.M = kRehearsalMasters; a.R = kRehearsalSlots; a.D = kRehearsalD;
+        a.balance_threshold = 1.f;
+        a.min_tokens = 1;
+        a.allow_zero_master = 0;
+        a.locality = call.params.locality_aware;
+        a.eps = 0.01f;
+        a.my_rank = 0;
+        a.preloaded = 1;
+        a.staged_loads = matrix;
+        a.trace = nullptr;
+    }
+    crew.sync();
 }
 
 // Steps 1 to 3 of a rank: counts, exchange, reduction. False: this CTA has handed its counts over and is done, or the loads did not
 // come; else `a` says what to solve.
 template <bool kLegacy>
-__device__ __forceinline__ bool gather_loads(const PlanCall& call, int local, int part, char* smem_raw, SolveArgs& a) {
+__device__ __forceinline__ bool gather_loads(const PlanCall& call, const Crew& crew, int local, int part, char* smem_raw, SolveArgs& a) {
     __shared__ int s_timeout_peer;
     __shared__ uint64_t s_epoch;
+    __shared__ __align__(8) uint64_t s_rows;  // the other ranks' rows, where they are pushed
     const GroupDev& group = call.group;
     uint64_t* const hist_parts = call.hist_parts[local];
     const int N = call.N, M = call.M;
     const int L = N * M;
     const int Lpad = (L + 3) / 4 * 4;
-    const int tid = threadIdx.x;
+    const int tid = crew.tid;
     const unsigned long long t_start = call.trace != nullptr ? global_timer_ns() : 0ull;
     auto stamp = [&](int slot) {
         if (call.trace != nullptr && tid == 0) call.trace[local * 8 + slot] = global_timer_ns();
@@ -327,32 +335,72 @@ __device__ __forceinline__ bool gather_loads(const PlanCall& call, int local, in
     //    after it was stored. The owner waits (bounded) for CTAs of its own launch; none of them waits for it,
     //    so they need not be resident at the same time.
     int32_t* hist = reinterpret_cast<int32_t*>(smem_raw);
-    for (int i = tid; i < L; i += blockDim.x) hist[i] = 0;
+    const int me = group.my_rank[local];
+    const bool preload = !kLegacy;
+    const bool staged = preload && plan_matrix_bytes(N, L) > 0;
+    int32_t* matrix = reinterpret_cast<int32_t*>(smem_raw + solver_smem_bytes(L, N, call.R));
+    for (int i = tid; i < L; i += crew.threads) hist[i] = 0;
+    const bool owner = part == 0, pushes = call.in_cluster != 0;
     if (tid == 0) {
         s_timeout_peer = -1;
+        if (owner && pushes) {
+            mbar_init(&s_rows, 1);
+            fence_mbar_init();
+            mbar_expect_tx(&s_rows, static_cast<uint32_t>((N - 1) * L * sizeof(int32_t)));
+        }
     }
+    if (owner && pushes) cluster_arrive();  // (the owners are a cluster of their own)
+    pdl_wait();  // ahead of every read: what is in front may still be writing the input
     // the epoch this launch opens: the owner stores it once it holds every partial, so every CTA of the launch reads the
     // same value here
     uint64_t last_epoch = 0;
     if (tid == 0) last_epoch = ld_relaxed_sys_u64(call.epoch[local]);  // on its way while the slice is counted
-    __syncthreads();
-    histogram_slice(call.input_kind, call.input[local], call.T[local], call.K_or_L, L, part, call.ctas_per_rank, hist);
+    crew.sync();
+    histogram_slice(call.input_kind, call.input[local], call.T[local], call.K_or_L, L, part, call.ctas_per_rank, hist, crew.threads);
     if (tid == 0) s_epoch = last_epoch + 1;
-    __syncthreads();
+    crew.sync();
     const uint64_t epoch = s_epoch;
     // never zero (the buffers start zeroed), period 2^32 - 1: an odd period, so the word that carried the same
     // tag one period ago sat in the other parity slot and cannot be mistaken for this epoch's
     const uint32_t tag = static_cast<uint32_t>(epoch % 0xFFFFFFFFull) + 1u;
     if (part != 0) {
         uint64_t* row = hist_parts + static_cast<int64_t>(part) * Lpad;
-        for (int i = tid; i < L; i += blockDim.x) st_relaxed_sys_u64(row + i, tag_word(tag, static_cast<uint32_t>(hist[i])));
+        for (int i = tid; i < L; i += crew.threads) st_relaxed_sys_u64(row + i, tag_word(tag, static_cast<uint32_t>(hist[i])));
         return false;
     }
     if (call.trace != nullptr && tid == 0) call.trace[local * 8 + 5] = t_start;  // when this CTA started
+    if (pushes) cluster_wait();  // every owner has started and its barrier for the rows is there
+    // An owner that gives up stays until nobody can push to it any more.
+    auto leave = [&]() {
+        if (pushes) {
+            cluster_arrive();
+            cluster_wait();
+        }
+    };
+    // What the solver needs of the parameters goes into shared memory while this CTA waits for the others: of one rank they were last
+    // read a layer ago, and each line of them comes from memory.
+    if (tid == crew.threads - 1) {
+        a.global_loads = call.global_loads[local];
+        a.loads_per_rank = call.loads_per_rank[local];
+        const PlanPtrs& pp = call.plan[local];
+        a.p2l = pp.p2l; a.l2p = pp.l2p; a.lcnts = pp.lcnts; a.quota = pp.quota; a.quota_prefix = pp.quota_prefix;
+        a.rank_quota_prefix = pp.rank_quota_prefix;
+        a.physical_loads = pp.physical_loads;
+        a.N = N; a.G = N; a.M = M; a.R = call.R; a.D = call.D;
+        a.balance_threshold = call.params.balance_threshold;
+        a.min_tokens = call.params.min_tokens_per_replica;
+        a.allow_zero_master = call.params.allow_zero_master_quota;
+        a.locality = call.params.locality_aware;
+        a.eps = call.params.oracle_eps;
+        a.my_rank = me;
+        a.preloaded = preload ? 1 : 0;
+        a.staged_loads = staged ? matrix : nullptr;
+        a.trace = call.trace != nullptr ? call.trace + (kMaxLocalRanks + local) * 8 : nullptr;
+    }
     {   // an expert's partials are shared by all the threads it can have, so that one round of loads fetches them
         const int rest = call.ctas_per_rank - 1;
-        const int parts = max(min(static_cast<int>(blockDim.x) / L, rest), 1);
-        for (int idx = tid; idx < L * parts; idx += blockDim.x) {
+        const int parts = max(min(crew.threads / L, rest), 1);
+        for (int idx = tid; idx < L * parts; idx += crew.threads) {
             const int i = idx % L, part = idx / L;
             int32_t total = 0;
             for (int c0 = 1 + part; c0 <= rest; c0 += kPartBatch * parts) {
@@ -379,122 +427,152 @@ __device__ __forceinline__ bool gather_loads(const PlanCall& call, int local, in
             if (rest > 0) atomicAdd(hist + i, total);
         }
     }
-    __syncthreads();
+    crew.sync();
     if (tid == 0) *call.epoch[local] = epoch;  // every CTA of the launch has read the old value: its partial carried the tag
     if (s_timeout_peer >= 0) {  // a CTA of this very launch never delivered
         if (tid == 0) report_error(group.status[local], UEP_DEV_TIMEOUT_GATHER, s_timeout_peer);
+        leave();
         return false;
     }
     stamp(0);
 
-    // 2. publish the row to every rank (itself included). Every 64-bit word carries the epoch beside its
-    //    count, so a row needs neither a fence nor a flag: one NVLink crossing, and the reader knows a word
-    //    is this layer's when it sees it.
-    const int slot = static_cast<int>(epoch & 1ull);
-    const int me = group.my_rank[local];
-    if (me != call.withhold_rank) {
-        for (int i = tid; i < L; i += blockDim.x) {
-            const uint64_t word = tag_word(tag, static_cast<uint32_t>(hist[i]));
-            for (int p = 0; p < N; ++p) st_relaxed_sys_u64(group.gather_of(p) + (static_cast<int64_t>(slot) * N + me) * Lpad + i, word);
-        }
-    }
-
     // With one domain the solver finds the loads in shared memory where it keeps them: its loads are where hist was.
-    const bool preload = !kLegacy;
     const SolverSmem solver_sm = carve_solver_smem(smem_raw, L, N, call.R);
-    const bool staged = preload && plan_matrix_bytes(N, L) > 0;
-    int32_t* matrix = reinterpret_cast<int32_t*>(smem_raw + solver_smem_bytes(L, N, call.R));
-    __syncthreads();  // hist has been read by every thread
-    stamp(1);
-    // 3. collect every rank's row (bounded), expose the matrix, reduce. A thread owns one expert:
-    //    it first issues the loads of eight ranks' words together and only then looks at them,
-    //    so the common case (all rows already here) costs one memory round trip.
-    const uint64_t* gathered = group.gather_of(me) + static_cast<int64_t>(slot) * N * Lpad;
-    for (int i = tid; i < L; i += blockDim.x) {
-        int32_t total = 0;
-        for (int r0 = 0; r0 < N; r0 += 8) {
-            uint64_t w[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                if (r0 + u < N) w[u] = ld_relaxed_sys_u64(gathered + static_cast<int64_t>(r0 + u) * Lpad + i);
+    if (pushes) {
+        // 2, 3. The ranks of one cluster write their rows straight into each other's matrix, a warp per rank; the bytes are counted
+        //    where they land. (Words through memory, as below, take a store, a look and their two ways through L2: 1.5 us more.)
+        const int warp = tid >> 5, lane = tid & 31, warps = crew.threads / kWarp;
+        const bool vec = (L & 3) == 0;
+        int32_t* row = matrix + me * L;
+        for (int p = warp; p < N; p += warps) {
+            if (p == local) {
+                for (int i = lane; i < L; i += kWarp) row[i] = hist[i];
+                continue;
             }
+            const uint32_t to = cluster_addr(row, p), bar = cluster_addr(&s_rows, p);
+            if (vec) {
+                for (int i = lane * 4; i < L; i += kWarp * 4) push_v4(to + i * 4, *reinterpret_cast<const int4*>(hist + i), bar);
+            } else {
+                for (int i = lane; i < L; i += kWarp) push_word(to + i * 4, hist[i], bar);
+            }
+        }
+        crew.sync();  // hist has been read by every thread, this rank's own row is there
+        stamp(1);
+        if (!mbar_wait(&s_rows, 0, call.timeout_ns)) atomicMax(&s_timeout_peer, me);
+        crew.sync();
+        if (s_timeout_peer >= 0) {
+            if (tid == 0) report_error(group.status[local], UEP_DEV_TIMEOUT_GATHER, s_timeout_peer);
+            leave();
+            return false;
+        }
+        for (int i = tid; i < L; i += crew.threads) {
+            int32_t total = 0;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                if (r0 + u < N) {
-                    // one time limit for the whole gather: once a wait has run out, no other word is waited for
-                    if (static_cast<uint32_t>(w[u] >> 32) != tag &&
-                        !wait_tagged_word(gathered + static_cast<int64_t>(r0 + u) * Lpad + i, tag,
-                                          *reinterpret_cast<volatile int*>(&s_timeout_peer) >= 0 ? 0 : call.timeout_ns, w[u])) {
-                        atomicMax(&s_timeout_peer, r0 + u);
-                        w[u] = 0;
-                    }
-                    const int32_t v = static_cast<int32_t>(static_cast<uint32_t>(w[u]));
-                    call.loads_per_rank[local][static_cast<int64_t>(r0 + u) * L + i] = v;
-                    if (staged) matrix[(r0 + u) * L + i] = v;
+            for (int r = 0; r < kMaxLocalRanks; ++r) {
+                if (r < N) {
+                    const int32_t v = matrix[r * L + i];
+                    call.loads_per_rank[local][r * L + i] = v;
                     total += v;
                 }
             }
+            call.global_loads[local][i] = total;
+            if (preload) {
+                solver_sm.my_loads[i] = hist[i];
+                solver_sm.loads[i] = total;  // (hist[i] itself)
+            }
         }
-        call.global_loads[local][i] = total;
-        if (preload) {
-            solver_sm.my_loads[i] = hist[i];
-            solver_sm.loads[i] = total;  // (hist[i] itself)
+        __threadfence_block();
+        crew.sync();
+    } else {
+        const int slot = static_cast<int>(epoch & 1ull);
+        // 2. publish the row to every rank (itself included). Every 64-bit word carries the epoch beside its
+        //    count, so a row needs neither a fence nor a flag: one NVLink crossing, and the reader knows a word
+        //    is this layer's when it sees it.
+        if (me != call.withhold_rank) {
+            for (int i = tid; i < L; i += crew.threads) {
+                const uint64_t word = tag_word(tag, static_cast<uint32_t>(hist[i]));
+                for (int p = 0; p < N; ++p) st_relaxed_sys_u64(group.gather_of(p) + (static_cast<int64_t>(slot) * N + me) * Lpad + i, word);
+            }
         }
-    }
-    __threadfence_block();
-    __syncthreads();
-    if (s_timeout_peer >= 0) {
-        if (tid == 0) report_error(group.status[local], UEP_DEV_TIMEOUT_GATHER, s_timeout_peer);
-        return false;  // plan of this layer is left as it was; the host raises on the status word
-    }
 
+        crew.sync();  // hist has been read by every thread
+        stamp(1);
+        // 3. collect every rank's row (bounded), expose the matrix, reduce. A thread owns one expert:
+        //    it first issues the loads of eight ranks' words together and only then looks at them,
+        //    so the common case (all rows already here) costs one memory round trip.
+        const uint64_t* gathered = group.gather_of(me) + static_cast<int64_t>(slot) * N * Lpad;
+        for (int i = tid; i < L; i += crew.threads) {
+            int32_t total = 0;
+            for (int r0 = 0; r0 < N; r0 += 8) {
+                uint64_t w[8];
+    #pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    if (r0 + u < N) w[u] = ld_relaxed_sys_u64(gathered + static_cast<int64_t>(r0 + u) * Lpad + i);
+                }
+    #pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    if (r0 + u < N) {
+                        // one time limit for the whole gather: once a wait has run out, no other word is waited for
+                        if (static_cast<uint32_t>(w[u] >> 32) != tag &&
+                            !wait_tagged_word(gathered + static_cast<int64_t>(r0 + u) * Lpad + i, tag,
+                                              *reinterpret_cast<volatile int*>(&s_timeout_peer) >= 0 ? 0 : call.timeout_ns, w[u])) {
+                            atomicMax(&s_timeout_peer, r0 + u);
+                            w[u] = 0;
+                        }
+                        const int32_t v = static_cast<int32_t>(static_cast<uint32_t>(w[u]));
+                        call.loads_per_rank[local][static_cast<int64_t>(r0 + u) * L + i] = v;
+                        if (staged) matrix[(r0 + u) * L + i] = v;
+                        total += v;
+                    }
+                }
+            }
+            call.global_loads[local][i] = total;
+            if (preload) {
+                solver_sm.my_loads[i] = hist[i];
+                solver_sm.loads[i] = total;  // (hist[i] itself)
+            }
+        }
+        __threadfence_block();
+        crew.sync();
+        if (s_timeout_peer >= 0) {
+            if (tid == 0) report_error(group.status[local], UEP_DEV_TIMEOUT_GATHER, s_timeout_peer);
+            return false;  // plan of this layer is left as it was; the host raises on the status word
+        }
+    }
     stamp(2);
     stamp(3);
-    a.global_loads = call.global_loads[local];
-    a.loads_per_rank = call.loads_per_rank[local];
-    const PlanPtrs& pp = call.plan[local];
-    a.p2l = pp.p2l; a.l2p = pp.l2p; a.lcnts = pp.lcnts; a.quota = pp.quota; a.quota_prefix = pp.quota_prefix;
-    a.rank_quota_prefix = pp.rank_quota_prefix;
-    a.physical_loads = pp.physical_loads;
-    a.N = N; a.G = call.G; a.M = M; a.R = call.R; a.D = call.D;
-    a.balance_threshold = call.params.balance_threshold;
-    a.min_tokens = call.params.min_tokens_per_replica;
-    a.allow_zero_master = call.params.allow_zero_master_quota;
-    a.locality = call.params.locality_aware;
-    a.eps = call.params.oracle_eps;
-    a.my_rank = me;
-    a.preloaded = preload ? 1 : 0;
-    a.staged_loads = staged ? matrix : nullptr;
-    a.trace = call.trace != nullptr ? call.trace + (kMaxLocalRanks + local) * 8 : nullptr;
     return true;
 }
 
-// The fused per-layer plan kernel. gridDim.x = nlocal * ctas_per_rank, and one more CTA where it is rehearsed, which only the form
-// with more threads can be: without, every output's address is known to be global, and the registers are twice as many.
-template <int THREADS, bool kLegacy>
-__global__ void __launch_bounds__(THREADS, 1) plan_kernel(PlanCall call) {
+// The fused per-layer plan kernel: ctas_per_rank clusters of a CTA of every hosted rank. The ranks' first CTAs come last, behind those that
+// they wait for. The threads behind kThreads are there where it is rehearsed.
+template <int kThreads, bool kLegacy>
+__global__ void __launch_bounds__(kThreads + kRehearsalThreads, 1) plan_kernel(PlanCall call) {
     extern __shared__ __align__(128) char smem_raw[];
-    // The next kernel of the stream may be on its SMs when the plan ends. Only where every rank of the group is in this launch:
-    // a plan that waits for other devices must not have the SMs held meanwhile by CTAs that wait for it.
-    if (call.nlocal == call.N) pdl_launch_dependents();
-    const bool rehearses = THREADS == kPlanMaxThreads && !kLegacy && static_cast<int>(blockIdx.x) == call.nlocal * call.ctas_per_rank;
-    const int local = rehearses ? 0 : blockIdx.x / call.ctas_per_rank;
-    SolveArgs a;
+    const int local = cluster_cta();
+    const int part = call.ctas_per_rank - 1 - (call.nlocal > 1 ? static_cast<int>(blockIdx.x) / call.nlocal : static_cast<int>(blockIdx.x));
+    const bool rehearses = !kLegacy && threadIdx.x >= kThreads;
+    const Crew crew = rehearses ? Crew{static_cast<int>(threadIdx.x) - kThreads, kRehearsalThreads, 2} : Crew{static_cast<int>(threadIdx.x), kThreads, 1};
+    char* const smem = rehearses ? smem_raw + call.rehearsal_smem : smem_raw;
+    __shared__ SolveArgs args[2];  // of each crew
+    SolveArgs& a = args[rehearses ? 1 : 0];
     if (rehearses) {
-        rehearsal_args(call, smem_raw, a);
-    } else if (!gather_loads<kLegacy>(call, local, blockIdx.x % call.ctas_per_rank, smem_raw, a)) {
+        if (part != 0) return;
+        if (call.in_cluster) cluster_arrive();  // the other crew's barrier counts every thread
+        rehearsal_args(call, crew, local, smem, a);
+    } else if (!gather_loads<kLegacy>(call, crew, local, part, smem, a)) {
         return;
     }
     DeviceStatus* const status = rehearses ? nullptr : call.group.status[local];
-    if (kLegacy) legacy_solve_domain(a, 0, smem_raw, status);
-    else solve_domain(a, 0, smem_raw, status);
+    if (kLegacy) legacy_solve_domain(a, 0, smem, status);
+    else solve_domain(a, crew, 0, smem, status);
     if (!rehearses && call.trace != nullptr && threadIdx.x == 0) call.trace[local * 8 + 4] = global_timer_ns();
 }
 
 size_t plan_smem_bytes(int N, int G, int M, int R) {
     const size_t solver = std::max(solver_smem_bytes(G * M, G, R) + (G == N ? plan_matrix_bytes(N, N * M) : 0), legacy_smem_bytes(G * M, G));
     const size_t hist = sizeof(int32_t) * static_cast<size_t>(N) * M;
-    return std::max(std::max(solver, hist), rehearsal_smem_bytes()) + 16;
+    return (std::max(solver, hist) + 15) / 16 * 16;
 }
 
 std::atomic<int64_t> g_launches{0};
@@ -503,49 +581,90 @@ std::atomic<int64_t> g_launches{0};
 
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
-// Twice the threads where a CTA's slice of the input would be several rounds of loads, and a rehearsal with them. Steps of eight
-// ranks: 256 threads, 512, 512 and the rehearsal; among others / behind an L2 flush (us). Above the line: 2600 bool rows of 128
-// experts (18 KB a CTA) 42.7/49.2, 44.7/50.2, 42.9/47.4; 6500 rows 55.7/59.5, 56.8/59.7, 54.0/57.5; 8192 rows 64.6/67.9, 66.0/69.8,
-// 63.2/67.7; 9600 int32 tokens of 128 (17 KB) 46.1/51.4, 45.9/51.4, 44.7/49.2; 4800 int64 tokens of 64 (17 KB) 35.6/43.2, 36.0/45.2,
-// 35.9/41.1; 16384 of 256 (57 KB) 110.6/114.7, 109.9/114.6, 108.7/111.5. Below: 1600 bool rows 41.2/47.3, 42.8/49.4, 41.5/47.3; 3000
-// int64 tokens of 64 32.7/41.2, 34.5/43.2, 34.5/40.8; 4096 int32 tokens of 64, no experts, 27.2/33.8, 28.7/35.9, 28.7/33.8; 33 tokens
-// 16.2/23.4, 17.3/25.4, 17.6/23.5.
+// Twice the threads where a CTA's slice of the input would be several rounds of loads. Step of eight ranks with 256 threads and 512 (us),
+// above the line: 16384 int64 tokens of 256 experts (70 KB a CTA) 106.8 and 104.5, 2600 bool rows of 256 (44 KB) 53.4 and 51.8, 8192 bool rows
+// of 128 (70 KB) 59.3 and 59.4; below it, where nothing is left to share, smaller blocks start sooner.
 int plan_threads(int input_kind, int max_T, int K_or_L, int ctas) {
     const int64_t bytes = static_cast<int64_t>(max_T) * K_or_L * (input_kind == 0 ? 1 : (input_kind == 1 ? 4 : 8));
-    return bytes > static_cast<int64_t>(ctas) * 16 * 1024 ? kPlanMaxThreads : kPlanMaxThreads / 2;
+    return bytes > static_cast<int64_t>(ctas) * 16 * 1024 ? 2 * kPlanThreads : kPlanThreads;
 }
 
-int plan_ctas_per_rank(int input_kind, int max_T, int K_or_L, int nlocal, int num_sms) {
+int plan_ctas_per_rank(int input_kind, int max_T, int K_or_L, int cap) {
     const int64_t bytes = static_cast<int64_t>(max_T) * K_or_L * (input_kind == 0 ? 1 : (input_kind == 1 ? 4 : 8));
-    int ctas = static_cast<int>((bytes + 16 * 1024 - 1) / (16 * 1024));
-    const int cap = nlocal > 1 ? (num_sms / nlocal) : kPlanMaxCtas;
-    ctas = ctas < 1 ? 1 : ctas;
-    ctas = ctas > cap ? cap : ctas;
-    return ctas > kPlanMaxCtas ? kPlanMaxCtas : (ctas < 1 ? 1 : ctas);
+    const int64_t ctas = (bytes + 16 * 1024 - 1) / (16 * 1024);
+    return static_cast<int>(std::max<int64_t>(std::min<int64_t>(ctas, std::min(cap, kPlanMaxCtas)), 1));
 }
 
-// Only where the ranks of a group are hosted together: with ranks on other devices it is not measured.
-bool plan_rehearses(const PlanCall& call, int num_sms) {
-    return call.threads == kPlanMaxThreads && call.nlocal == call.N && call.N > 1 && call.R > 0 && call.legacy == 0 &&
-           call.nlocal * call.ctas_per_rank < num_sms;
+namespace {
+
+const void* plan_kernel_of(bool legacy, int threads) {
+    if (legacy) return reinterpret_cast<const void*>(plan_kernel<kPlanThreads, true>);
+    return threads == kPlanThreads ? reinterpret_cast<const void*>(plan_kernel<kPlanThreads, false>)
+                                   : reinterpret_cast<const void*>(plan_kernel<2 * kPlanThreads, false>);
+}
+
+cudaLaunchAttribute dependent_launch() {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    return attr;
+}
+
+cudaLaunchAttribute plan_cluster(int nlocal) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = nlocal;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    return attr;
+}
+
+}  // namespace
+
+// The most CTAs of a rank that the device holds at once, a CTA of every hosted rank being a cluster (clusters of eight: 15 of the 18 that
+// 148 SMs could hold, since a cluster's SMs are of one GPC).
+cudaError_t plan_most_ctas(int nlocal, int N, int G, int M, int R, int* ctas) {
+    *ctas = kPlanMaxCtas;
+    if (nlocal == 1) return cudaSuccess;
+    const void* kernel = plan_kernel_of(false, kPlanThreads);
+    const size_t smem = plan_smem_bytes(N, G, M, R) + rehearsal_smem_bytes();
+    cudaError_t e = allow_smem(kernel, smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute attr[1] = {plan_cluster(nlocal)};
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(nlocal);
+    cfg.blockDim = dim3(kPlanThreads + kRehearsalThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    e = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg);
+    if (e != cudaSuccess) return e;
+    *ctas = std::max(clusters, 1);
+    return cudaSuccess;
 }
 
 cudaError_t launch_plan(const PlanCall& call, cudaStream_t stream) {
-    const size_t smem = plan_smem_bytes(call.N, call.G, call.M, call.R);
-    const auto kernel = call.legacy ? plan_kernel<kPlanMaxThreads / 2, true>
-                                    : (call.threads == kPlanMaxThreads ? plan_kernel<kPlanMaxThreads, false> : plan_kernel<kPlanMaxThreads / 2, false>);
-    cudaError_t e = allow_smem(reinterpret_cast<const void*>(kernel), smem);
+    const bool rehearses = call.N > 1 && call.R > 0 && !call.legacy;
+    PlanCall copy = call;
+    copy.rehearsal_smem = static_cast<int>(plan_smem_bytes(call.N, call.G, call.M, call.R));
+    copy.in_cluster = call.nlocal == call.N && call.withhold_rank < 0 ? 1 : 0;
+    const size_t smem = copy.rehearsal_smem + (rehearses ? rehearsal_smem_bytes() : 0);
+    const void* kernel = plan_kernel_of(call.legacy != 0, call.threads);
+    cudaError_t e = allow_smem(kernel, smem);
     if (e != cudaSuccess) return e;
-    const dim3 grid(call.nlocal * call.ctas_per_rank + call.rehearsal), block(call.legacy ? kPlanMaxThreads / 2 : call.threads);
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(call.nlocal * call.ctas_per_rank);
+    cfg.blockDim = dim3((call.legacy ? kPlanThreads : call.threads) + (rehearses ? kRehearsalThreads : 0));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    if (call.nlocal > 1) attr[cfg.numAttrs++] = plan_cluster(call.nlocal);
+    if (pdl_enabled()) attr[cfg.numAttrs++] = dependent_launch();
+    void* args[] = {&copy};
     count_launch();
-    if (call.nlocal > 1) {
-        // ranks wait for each other inside the kernel: co-residency is required
-        PlanCall copy = call;
-        void* args[] = {&copy};
-        return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), grid, block, args, smem, stream);
-    }
-    kernel<<<grid, block, smem, stream>>>(call);
-    return cudaGetLastError();
+    return cudaLaunchKernelExC(&cfg, kernel, args);
 }
 
 }  // namespace uep
@@ -567,7 +686,7 @@ static int histogram_common(int kind, const void* input, int T, int K_or_L, int 
     const int64_t n = static_cast<int64_t>(T) * K_or_L;
     if (n == 0) return UEP_OK;
     if (input == nullptr) return fail(UEP_ERR_INVALID, "histogram: null input");
-    const int ctas = plan_ctas_per_rank(kind, T, K_or_L, 1, std::max(device_sm_count(), 1));
+    const int ctas = plan_ctas_per_rank(kind, T, K_or_L, kPlanMaxCtas);
     const size_t smem = sizeof(int32_t) * L;
     UEP_CUDA_TRY(allow_smem(reinterpret_cast<const void*>(histogram_kernel), smem));
     count_launch();
@@ -625,9 +744,15 @@ int uep_solve_placement(const int32_t* loads_per_rank, int32_t* global_loads_out
     if (staged) smem += matrix;
     UEP_CUDA_TRY(allow_smem(reinterpret_cast<const void*>(solve_kernel<false>), smem));
     count_launch();
-    solve_kernel<false><<<num_ranks / nvl_ranks, kSolveThreads, smem, stream>>>(a, global_loads_out, 1, staged,
-                                                                                 reinterpret_cast<DeviceStatus*>(status));
-    UEP_CUDA_TRY(cudaGetLastError());
+    cudaLaunchAttribute attr[1] = {dependent_launch()};
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(num_ranks / nvl_ranks);
+    cfg.blockDim = dim3(kSolveThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    UEP_CUDA_TRY(cudaLaunchKernelEx(&cfg, solve_kernel<false>, a, global_loads_out, 1, staged, reinterpret_cast<DeviceStatus*>(status)));
     return UEP_OK;
 }
 

@@ -207,9 +207,9 @@ __device__ __forceinline__ bool dense_fast_path(const uint8_t* map, int L) {
 // TILES tiles a CTA: one or four (launch_dense_forward).
 constexpr int kCountCtasPerSm = 5;  // at 48 registers
 template <int TILES>
-__global__ void __launch_bounds__(kRerouteThreads, kCountCtasPerSm) dense_count_kernel(Batch<DenseFwdArgs> batch, int L, int wait_first) {
+__global__ void __launch_bounds__(kRerouteThreads, kCountCtasPerSm) dense_count_kernel(Batch<DenseFwdArgs> batch, int L, int wait_first, int next_early) {
     if (wait_first) pdl_wait();  // ahead of every read: the kernel in front may still be writing the map
-    pdl_launch_dependents();  // the scatter kernel may start its prologue now
+    if (next_early) pdl_launch_dependents();  // the scatter kernel may start its prologue now
     extern __shared__ __align__(128) char smem_raw[];  // [TILES][pad4(L)] counts, one byte each
     constexpr int kThreads = kRerouteThreads / TILES;  // of a tile: whole warps
     const DenseFwdArgs& a = batch.a[blockIdx.y];
@@ -395,8 +395,8 @@ __device__ __forceinline__ void write_dense_chunk(const DenseShared& s, const fl
 
 __global__ void __launch_bounds__(kDenseMaxThreads, 2)
 dense_scatter_kernel(Batch<DenseFwdArgs> batch, int L, int P, int D, int quota_mode, int interleave, int chunk_cols,
-                     int overlapped, int behind_plan) {
-    if (behind_plan) pdl_wait();  // the count kernel waited for the plan, this one for both
+                     int overlapped, int wait_first) {
+    if (wait_first) pdl_wait();  // the count kernel waited for what was in front of it, this one for both
     const DenseFwdArgs& a = batch.a[blockIdx.y];
     const int T = a.T;
     const int tile = blockIdx.x;
@@ -450,7 +450,6 @@ dense_scatter_kernel(Batch<DenseFwdArgs> batch, int L, int P, int D, int quota_m
             if (any) s.expert_of[p] = static_cast<uint16_t>(e);
         }
         if (p_lo == 0 && overlapped) pdl_wait();
-        if (p_lo == 0) pdl_launch_dependents();
         __syncthreads();  // the list of experts with several; the bytes above share words with the atomics below
         for (int i = warp; i < n_several; i += warps) {
             const int e = s.several[i];
@@ -655,7 +654,8 @@ dense_backward_tile_kernel(Batch<DenseBwdArgs> batch, int L, int P, int D, int t
 // One thread per four logical experts of a token when the rows allow it (L a multiple of 4, map rows 4-byte and
 // gradient rows 16-byte aligned): the routing map is read a word at a time and the gradients leave as float4.
 // Most entries are not routed, so the kernel is a zero fill plus a few gathers.
-__global__ void __launch_bounds__(kRerouteThreads) dense_backward_kernel(Batch<DenseBwdArgs> batch, int L, int P, int D) {
+__global__ void __launch_bounds__(kRerouteThreads) dense_backward_kernel(Batch<DenseBwdArgs> batch, int L, int P, int D, int wait_first) {
+    if (wait_first) pdl_wait();  // ahead of every read
     const DenseBwdArgs& a = batch.a[blockIdx.y];
     const float* __restrict__ grad_expanded = a.grad_expanded;
     const uint8_t* __restrict__ map = a.map;
@@ -694,9 +694,10 @@ __global__ void __launch_bounds__(kRerouteThreads) dense_backward_kernel(Batch<D
 
 // ---------------------------------------------------------------------------- sparse
 template <typename IdT>
-__global__ void __launch_bounds__(kOrdThreads) sparse_count_kernel(Batch<SparseArgs> batch, int K, int L, int tile_entries, int wait_first) {
+__global__ void __launch_bounds__(kOrdThreads) sparse_count_kernel(Batch<SparseArgs> batch, int K, int L, int tile_entries, int wait_first,
+                                                                   int next_early) {
     if (wait_first) pdl_wait();  // ahead of every read: the kernel in front may still be writing the ids
-    pdl_launch_dependents();      // the reroute kernel may start on everything that does not read the table
+    if (next_early) pdl_launch_dependents();  // the reroute kernel may start on everything that does not read the table
     const SparseArgs& a = batch.a[blockIdx.y];
     count_tile<IdT>(static_cast<const IdT*>(a.ids), static_cast<int64_t>(a.T) * K, L, false, tile_entries, a.scratch);
 }
@@ -714,7 +715,6 @@ __global__ void __launch_bounds__(kOrdThreads) __maxnreg__(EPT > 4 ? 96 : 64)
 sparse_reroute_kernel(Batch<SparseArgs> batch, int ctas, int K, int L, int D, int interleave, int rows_staged, int use_table, int wait_first) {
     extern __shared__ __align__(128) char smem_raw[];
     if (wait_first) pdl_wait();  // ahead of every read
-    pdl_launch_dependents();
     const SparseArgs& a = batch.a[blockIdx.y];
     const IdT* ids = static_cast<const IdT*>(a.ids);
     IdT* out = static_cast<IdT*>(a.out);
@@ -774,9 +774,9 @@ __host__ __device__ __forceinline__ size_t walk_smem_bytes(int L) {
     return static_cast<size_t>(L) * (2 * kStagedReps * 4 + sizeof(FastRouter) + 4 + kWalkWarps * 4);
 }
 template <typename IdT>
-__global__ void __launch_bounds__(kWalkThreads) sparse_walk_count_kernel(Batch<SparseArgs> batch, int K, int L, int behind_plan) {
+__global__ void __launch_bounds__(kWalkThreads) sparse_walk_count_kernel(Batch<SparseArgs> batch, int K, int L, int wait_first) {
     extern __shared__ __align__(128) char smem_raw[];
-    if (behind_plan) pdl_wait();  // ahead of every read
+    if (wait_first) pdl_wait();  // ahead of every read
     const SparseArgs& a = batch.a[blockIdx.y];
     const IdT* keys = static_cast<const IdT*>(a.ids);
     const int64_t n = static_cast<int64_t>(a.T) * K;
@@ -795,8 +795,9 @@ __global__ void __launch_bounds__(kWalkThreads) sparse_walk_count_kernel(Batch<S
 }
 
 template <typename IdT>
-__global__ void __launch_bounds__(kWalkThreads) sparse_walk_kernel(Batch<SparseArgs> batch, int K, int L, int D, int interleave) {
+__global__ void __launch_bounds__(kWalkThreads) sparse_walk_kernel(Batch<SparseArgs> batch, int K, int L, int D, int interleave, int wait_first) {
     extern __shared__ __align__(128) char smem_raw[];
+    if (wait_first) pdl_wait();
     const SparseArgs& a = batch.a[blockIdx.y];
     const IdT* ids = static_cast<const IdT*>(a.ids);
     IdT* out = static_cast<IdT*>(a.out);
@@ -884,6 +885,7 @@ __global__ void __launch_bounds__(kWalkThreads) sparse_walk_kernel(Batch<SparseA
 // ------------------------------------------------------------- dispatch positions
 __global__ void __launch_bounds__(kOrdThreads) dispatch_count_kernel(const int32_t* __restrict__ phys, int64_t n, int P, int tile_entries,
                                                                      int32_t* __restrict__ table) {
+    pdl_wait();  // ahead of every read
     pdl_launch_dependents();
     count_tile<int32_t>(phys, n, P, true, tile_entries, table);
 }
@@ -895,7 +897,7 @@ template <int EPT>
 __global__ void __launch_bounds__(kOrdThreads) __maxnreg__(EPT > 4 ? 128 : 80)
 dispatch_positions_kernel(const int32_t* phys, int64_t n, int ctas, int P, const int32_t* __restrict__ table, int32_t* pos,
                           int32_t* __restrict__ expert_offsets) {
-    pdl_launch_dependents();  // the gather behind it may set itself up
+    if (table == nullptr) pdl_wait();  // ahead of every read; the count kernel in front waited, and its table is waited for where it is read
     extern __shared__ __align__(128) char smem_raw[];
     __shared__ int warp_tot[kOrdWarps];
     const int nb = P + 1;
@@ -1145,7 +1147,7 @@ cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, s
 }
 
 cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int D, int quota_mode, int interleave,
-                                 bool behind_plan, cudaStream_t stream) {
+                                 bool beside_sync, cudaStream_t stream) {
     int max_T = 0;
     for (int i = 0; i < b.n; ++i) max_T = b.a[i].T > max_T ? b.a[i].T : max_T;
     if (max_T == 0) return cudaSuccess;
@@ -1164,25 +1166,24 @@ cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int
     // up to two tiles per SM the scatter kernel is a chain of phases: more threads shorten each
     const int threads = static_cast<int64_t>(grid.x) * b.n <= 2 * sms ? kDenseMaxThreads : kRerouteThreads;
     const size_t smem_count = static_cast<size_t>(pad4(L)) * (by_four ? 4 : 1), smem = dense_smem_bytes(L, chunk, threads);
-    behind_plan = behind_plan && b.n > 1 && pdl_enabled();
-    // The first kernel may be on its SMs when whatever is in front of it ends, too: it waits before its first read. (One rank, 8191
-    // tokens of 256 experts, sparse, dense and backward one behind the other: 34.1 us with ordinary launches, 32.8 like this. Of
-    // several ranks only behind a plan, as internal.h says; not beside a weight_sync, whose set-up the early CTAs would disturb. One
-    // rank beside a weight_sync has others on other devices: then the plan in front of this pair lets nothing start early.)
-    const bool early = behind_plan || (b.n == 1 && pdl_enabled());
+    // Both kernels are dependents of whatever is in front of them, as internal.h says; several ranks not beside a weight_sync, whose set-up
+    // the early CTAs disturb (step of 8192 bool rows of 128 experts with bf16 experts of 9 MB 59.5 us, first kernel, second and both
+    // as dependents 60.1, 60.2 and 60.3; of 8000 with 5 MB 54.0, 54.9, 54.0 and 54.5; of 1000 of 64 with 3 MB 29.9, 29.6, 30.0 and 30.7).
+    const bool dependent = pdl_enabled() && (b.n == 1 || !beside_sync);
+    // One rank's pair is latency: the second kernel has its prologue beside the first one. Several ranks fill the device with the
+    // first kernel alone; their second one starts behind it and waits first (started early it does nothing but wait: plan and
+    // pair of eight ranks, 4096 rows of 128 experts, 24.4 us and 25.6, 8192 rows 38.4 and 39.7).
+    const bool prologue = dependent && b.n == 1;
     cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(dense_scatter_kernel), smem);
     if (e != cudaSuccess) return e;
     e = ensure_smem_attr(reinterpret_cast<const void*>(count), smem_count);
     if (e != cudaSuccess) return e;
     count_launch(2);
-    e = launch_dependent(count, dim3(by_four ? (grid.x + 3) / 4 : grid.x, b.n), dim3(kRerouteThreads), smem_count, stream, early, b, L, early ? 1 : 0);
+    e = launch_dependent(count, dim3(by_four ? (grid.x + 3) / 4 : grid.x, b.n), dim3(kRerouteThreads), smem_count, stream, dependent, b, L,
+                         dependent ? 1 : 0, prologue ? 1 : 0);
     if (e != cudaSuccess) return e;
-    // With one rank per launch the pair is latency-bound and the overlap pays; a launch that hosts several ranks
-    // fills the device with the first kernel alone, and early CTAs of the second only get in its way, unless they do nothing
-    // but wait.
-    const bool overlap = early;
-    return launch_dependent(dense_scatter_kernel, grid, dim3(threads), smem, stream, overlap, b, L, P, D, quota_mode,
-                            interleave, chunk, overlap ? 1 : 0, behind_plan ? 1 : 0);
+    return launch_dependent(dense_scatter_kernel, grid, dim3(threads), smem, stream, dependent, b, L, P, D, quota_mode,
+                            interleave, chunk, prologue ? 1 : 0, dependent && !prologue ? 1 : 0);
 }
 
 cudaError_t launch_dense_backward(const Batch<DenseBwdArgs>& b, int L, int P, int D, cudaStream_t stream) {
@@ -1213,15 +1214,13 @@ cudaError_t launch_dense_backward(const Batch<DenseBwdArgs>& b, int L, int P, in
     if (tiles) {
         cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(dense_backward_tile_kernel), smem);
         if (e != cudaSuccess) return e;
-        const bool early = b.n == 1 && pdl_enabled();
-        return launch_dependent(dense_backward_tile_kernel, dim3((max_T + rows - 1) / rows, b.n), dim3(kDenseBwdThreads), smem, stream, early, b, L, P,
-                                D, rows, early ? 1 : 0);
+        return launch_dependent(dense_backward_tile_kernel, dim3((max_T + rows - 1) / rows, b.n), dim3(kDenseBwdThreads), smem, stream, true, b, L, P,
+                                D, rows, 1);
     }
     int64_t blocks = (static_cast<int64_t>(max_T) * L / 4 + kRerouteThreads - 1) / kRerouteThreads + 1;
     const int64_t cap = std::max(sms * 16 / b.n, 1);
     if (blocks > cap) blocks = cap;
-    dense_backward_kernel<<<dim3(static_cast<unsigned>(blocks), b.n), kRerouteThreads, 0, stream>>>(b, L, P, D);
-    return cudaGetLastError();
+    return launch_dependent(dense_backward_kernel, dim3(static_cast<unsigned>(blocks), b.n), dim3(kRerouteThreads), 0, stream, true, b, L, P, D, 1);
 }
 
 // How an input of n entries is cut: a cluster of CTAs with at most per_lane entries a thread, and as many clusters as it
@@ -1316,11 +1315,18 @@ bool walk_pays(int64_t n, int L, bool beside_sync) {
     return n > kOrdRecountMax || (beside_sync ? n * L <= 1 << 23 : n > 1 << 16);
 }
 
+// Several ranks beside a weight_sync of at most so many bytes: the reroute is then the longer one of the two, and both of its kernels
+// are dependents like elsewhere; beside a longer one their early CTAs disturb its set-up. Step of eight ranks, ordinary launches and
+// dependents (us): fp8 experts in 16 slots of 1.5 MB, 8000 int32 tokens of 128 experts 34.4 and 31.2, 4800 int64 tokens of 64 31.2 and
+// 27.2; 16 slots of 3 MB, 3000 tokens of 64 31.0 and 28.6; above the line 32 slots of 3 MB, 1000 tokens 27.8 and 27.6; 32 of 19 MB, 8192
+// tokens 54.3 and 54.9; 64 of 44 MB, 16384 of 256 104.0 and 107.4.
+constexpr int64_t kShortSyncBytes = 64ll << 20;
+
 template <typename IdT>
-static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L, int D, int interleave, bool beside_sync,
-                                       bool behind_plan, cudaStream_t stream) {
-    behind_plan = behind_plan && b.n > 1 && pdl_enabled();
-    const bool early = behind_plan || (b.n == 1 && pdl_enabled());  // as in launch_dense_forward
+static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L, int D, int interleave, int64_t beside_bytes,
+                                       cudaStream_t stream) {
+    const bool beside_sync = beside_bytes > 0;
+    const bool dependent = pdl_enabled() && (b.n == 1 || beside_bytes <= kShortSyncBytes);
     int64_t max_n = 0;
     bool in_place = false;
     for (int i = 0; i < b.n; ++i) {
@@ -1338,36 +1344,34 @@ static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L,
         e = ensure_smem_attr(reinterpret_cast<const void*>(sparse_walk_kernel<IdT>), walk_smem_bytes(L));
         if (e != cudaSuccess) return e;
         count_launch(2);
-        e = launch_dependent(sparse_walk_count_kernel<IdT>, grid, dim3(kWalkThreads), sizeof(int32_t) * L, stream, behind_plan, b, K, L,
-                             behind_plan ? 1 : 0);
+        e = launch_dependent(sparse_walk_count_kernel<IdT>, grid, dim3(kWalkThreads), sizeof(int32_t) * L, stream, dependent, b, K, L,
+                             dependent ? 1 : 0);
         if (e != cudaSuccess) return e;
-        sparse_walk_kernel<IdT><<<grid, kWalkThreads, walk_smem_bytes(L), stream>>>(b, K, L, D, interleave);
-        return cudaGetLastError();
+        return launch_dependent(sparse_walk_kernel<IdT>, grid, dim3(kWalkThreads), walk_smem_bytes(L), stream, dependent, b, K, L, D, interleave,
+                                dependent ? 1 : 0);
     }
     const int staged = sparse_smem_bytes(L, true) <= kMaxCtaSmem ? 1 : 0;
     const size_t smem = sparse_smem_bytes(L, staged != 0);
     const OrdGrid g = ord_grid(max_n, L, b.n, in_place, kOrdThreads, false);
-    // One rank per launch is latency-bound and the overlap with the count kernel pays; several ranks fill the device
-    // with the first kernel alone (behind a plan the second one is there early and does nothing but wait).
-    const bool overlap = early;
+    const bool prologue = dependent && g.table && b.n == 1;  // as in launch_dense_forward
     if (g.table) {
         cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(sparse_count_kernel<IdT>), sizeof(int32_t) * L);
         if (e != cudaSuccess) return e;
         count_launch();
-        e = launch_dependent(sparse_count_kernel<IdT>, dim3(g.ctas * g.clusters, b.n), dim3(kOrdThreads), sizeof(int32_t) * L, stream, early, b,
-                             K, L, g.per_lane * kOrdThreads, early ? 1 : 0);
+        e = launch_dependent(sparse_count_kernel<IdT>, dim3(g.ctas * g.clusters, b.n), dim3(kOrdThreads), sizeof(int32_t) * L, stream, dependent, b,
+                             K, L, g.per_lane * kOrdThreads, dependent ? 1 : 0, prologue ? 1 : 0);
         if (e != cudaSuccess) return e;
     }
     return with_lanes(g, [&](auto per_lane) {
-        return launch_clusters(sparse_reroute_kernel<decltype(per_lane)::value, IdT>, g, b.n, smem, stream, overlap, b, g.ctas, K, L, D,
-                               interleave, staged, g.table ? 1 : 0, behind_plan || (early && !g.table) ? 1 : 0);
+        return launch_clusters(sparse_reroute_kernel<decltype(per_lane)::value, IdT>, g, b.n, smem, stream, dependent, b, g.ctas, K, L, D,
+                               interleave, staged, g.table ? 1 : 0, dependent && !prologue ? 1 : 0);
     });
 }
 
-cudaError_t launch_sparse_reroute(const Batch<SparseArgs>& b, int ids_kind, int K, int L, int D, int interleave, bool beside_sync,
-                                  bool behind_plan, cudaStream_t stream) {
-    if (ids_kind == 2) return launch_sparse_typed<long long>(b, K, L, D, interleave, beside_sync, behind_plan, stream);
-    return launch_sparse_typed<int32_t>(b, K, L, D, interleave, beside_sync, behind_plan, stream);
+cudaError_t launch_sparse_reroute(const Batch<SparseArgs>& b, int ids_kind, int K, int L, int D, int interleave, int64_t beside_bytes,
+                                  cudaStream_t stream) {
+    if (ids_kind == 2) return launch_sparse_typed<long long>(b, K, L, D, interleave, beside_bytes, stream);
+    return launch_sparse_typed<int32_t>(b, K, L, D, interleave, beside_bytes, stream);
 }
 
 }  // namespace uep
@@ -1427,7 +1431,7 @@ static int sparse_common(int kind, const void* ids, void* out, int T, int K, int
     Batch<SparseArgs> b{};
     b.n = 1;
     b.a[0] = SparseArgs{ids, out, l2p, lcnts, rqp, scratch, T};
-    UEP_CUDA_TRY(launch_sparse_reroute(b, kind, K, L, D, interleave, false, false, static_cast<cudaStream_t>(stream_)));
+    UEP_CUDA_TRY(launch_sparse_reroute(b, kind, K, L, D, interleave, 0, static_cast<cudaStream_t>(stream_)));
     return UEP_OK;
 }
 
@@ -1516,16 +1520,15 @@ int uep_dispatch_positions(const int32_t* phys_ids, int64_t num_entries, int P, 
     const bool in_place = x < y + bytes && y < x + bytes;
     const OrdGrid g = ord_grid(num_entries, P + 1, 1, in_place, ord_smem_bytes(P + 1, kOrdThreads) <= kMaxCtaSmem ? kOrdThreads : kOrdFewThreads, true);
     const size_t smem = ord_smem_bytes(P + 1, g.threads), smem1 = sizeof(int32_t) * (P + 1);
-    const bool overlap = g.table && pdl_enabled();
     if (g.table) {
         UEP_CUDA_TRY(ensure_smem_attr(reinterpret_cast<const void*>(dispatch_count_kernel), smem1));
         count_launch();
-        dispatch_count_kernel<<<g.ctas * g.clusters, g.threads, smem1, stream>>>(phys_ids, num_entries, P, g.per_lane * g.threads, scratch);
-        UEP_CUDA_TRY(cudaGetLastError());
+        UEP_CUDA_TRY(launch_dependent(dispatch_count_kernel, dim3(g.ctas * g.clusters), dim3(g.threads), smem1, stream, true, phys_ids, num_entries, P,
+                                      g.per_lane * g.threads, scratch));
     }
     const int32_t* table = g.table ? scratch : nullptr;
     UEP_CUDA_TRY(with_lanes(g, [&](auto per_lane) {
-        return launch_clusters(dispatch_positions_kernel<decltype(per_lane)::value>, g, 1, smem, stream, overlap, phys_ids, num_entries, g.ctas, P,
+        return launch_clusters(dispatch_positions_kernel<decltype(per_lane)::value>, g, 1, smem, stream, pdl_enabled(), phys_ids, num_entries, g.ctas, P,
                                table, pos, expert_offsets);
     }));
     return UEP_OK;

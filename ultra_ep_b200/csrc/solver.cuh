@@ -27,6 +27,13 @@
 
 namespace uep {
 
+// The threads of a CTA that solve a problem together: their number among them, how many, and their barrier (0 to 15). A CTA can hold
+// two of them.
+struct Crew {
+    int tid, threads, barrier;
+    __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(barrier), "r"(threads) : "memory"); }
+};
+
 // An export: tokens moved to a redundant slot. `place`: the slot's physical id inside the domain << 8 | its rank.
 struct alignas(8) ExportEntry {
     int quota;
@@ -60,6 +67,12 @@ struct SolveArgs {
     int preloaded;  // 1: the shared-memory loads and my_loads of the (only) domain are in place already
     unsigned long long* trace;  // optional: 8 globaltimer stamps of the solver phases (tuning aid), or null
 };
+
+// The arguments may lie in shared memory, where a pointer does not show that it is of global memory.
+template <typename T>
+__device__ __forceinline__ T* as_global(T* p) {
+    return static_cast<T*>(__cvta_global_to_generic(__cvta_generic_to_global(p)));
+}
 
 constexpr int kSolverProbeWarps = 4;
 constexpr int kSolverBuffers = 2 * kSolverProbeWarps;  // plans: one the search may end with, and those of the present round
@@ -189,13 +202,15 @@ __device__ __forceinline__ bool drain_sources(const SolverSmem& sm, int buffer, 
             const int slack = amount_of(best), rank = kWide ? rank_of(below, best) : 0;
             q = min(slack, move);
             small = kWide ? static_cast<long long>(q) * times < floor : q * times < floor;  // with no rank left, too
+            int at = -1;
 #pragma unroll
             for (int k = 0; k < kKeys; ++k) {
                 hit[k] = kWide ? rank == lane + k * kWarp : below[k] == best;
-                if (hit[k]) plan[num_exports + made] = ExportEntry{q, place[k]};
+                at = hit[k] ? place[k] : at;
                 place[k] += hit[k] ? 1 << 8 : 0;
                 below[k] = hit[k] ? -1 : below[k];
             }
+            if (at >= 0) plan[num_exports + made] = ExportEntry{q, at};
             ++made;
             times -= by_count;
             floor -= by_count * q;
@@ -290,10 +305,11 @@ __device__ __forceinline__ int first_feasible(const SolverSmem& sm, int buffer0,
 // 20.0 us, 18.8 like this.) Returns the plan's buffer and its batches. All threads of the CTA; the first four warps' buffers hold nothing that counts.
 // Out of line, with a build of its own that knows its floor (one build, in one loop, for these and for the four in front of them: 16
 // ranks x 2 experts x 1 slot 27.4 us for 21.9).
-__device__ __noinline__ int2 probe_thresholds(int fitting, int hi0, int total, int largest, int G, int M, int R, int min_tokens, bool allow_zero_master) {
+__device__ __noinline__ int2 probe_thresholds(Crew crew, int fitting, int hi0, int total, int largest, int G, int M, int R, int min_tokens,
+                                              bool allow_zero_master) {
     extern __shared__ __align__(128) char smem_raw[];  // the kernel's: as an argument its address would not be known to be shared
     const SolverSmem sm = carve_solver_smem(smem_raw, G * M, G, R);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = crew.tid >> 5, lane = crew.tid & 31;
     int lo = min(fitting + 1, hi0), hi = hi0, winner = -1, num_batches = 0;
     for (int set = kSolverProbeWarps; lo < hi;) {
         const int range = hi - lo;
@@ -307,7 +323,7 @@ __device__ __noinline__ int2 probe_thresholds(int fitting, int hi0, int total, i
                             warp_build_plan<true>(sm, set + warp, n, probe(warp), total, largest, G, M, R, min_tokens, allow_zero_master, false, lane, nullptr);
             if (lane == 0) sm.ctrl[kCtlBuilt0 + set + warp] = ok ? n + 1 : 0;
         }
-        __syncthreads();
+        crew.sync();
         const int first = first_feasible(sm, set, num_batches);
         if (first >= 0) {
             hi = probe(first);
@@ -316,7 +332,7 @@ __device__ __noinline__ int2 probe_thresholds(int fitting, int hi0, int total, i
             set ^= kSolverProbeWarps;
         } else {
             lo = each ? hi : probe(kSolverProbeWarps - 1) + 1;
-            __syncthreads();  // the same buffers again
+            crew.sync();  // the same buffers again
         }
     }
     // no probe succeeded: at the largest load nothing is to be moved
@@ -520,13 +536,14 @@ __device__ __forceinline__ void warp_rank_quota_prefix(const SolveArgs& a, int l
         }
     }
     const int prefix = warp_inclusive_scan(my_alloc, lane);
-    if (active) a.rank_quota_prefix[static_cast<int64_t>(l_global) * a.D + lane] = prefix;
+    if (active) as_global(a.rank_quota_prefix)[static_cast<int64_t>(l_global) * a.D + lane] = prefix;
 }
 
-// Solve one NVLink domain. All threads of the CTA must call it (blockDim.x >= 128,
-// multiple of 32). smem_raw must hold solver_smem_bytes(E, G, R) bytes, 16-byte aligned.
-__device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, char* smem_raw, DeviceStatus* status) {
-    const int tid = threadIdx.x, nthreads = blockDim.x;
+// Solve one NVLink domain. All threads of the crew must call it (128 at least,
+// multiple of 32). smem_raw must hold solver_smem_bytes(E, G, R) bytes, 16-byte aligned; more than 32 ranks, loads from 2^24 on and
+// probes take the CTA's dynamic shared memory for it.
+__device__ __forceinline__ void solve_domain(const SolveArgs& a, const Crew& crew, int domain, char* smem_raw, DeviceStatus* status) {
+    const int tid = crew.tid, nthreads = crew.threads;
     const int warp = tid >> 5, lane = tid & 31;
     const int G = a.G, M = a.M, R = a.R, D = a.D;
     const int E = G * M, Lp = M + R, L = a.N * M;
@@ -537,39 +554,43 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, cha
         if (a.trace != nullptr && tid == 0) a.trace[slot] = global_timer_ns();
     };
     stamp(0);
+    int32_t *const out_p2l = as_global(a.p2l), *const out_l2p = as_global(a.l2p), *const out_lcnts = as_global(a.lcnts);
+    int32_t *const out_quota = as_global(a.quota), *const out_quota_prefix = as_global(a.quota_prefix);
+    int32_t *const out_rank_quota_prefix = as_global(a.rank_quota_prefix);
+    int32_t* const out_physical_loads = a.physical_loads != nullptr ? as_global(a.physical_loads) : nullptr;
 
     // Every output of this domain as it is without replicas (an expert then keeps all of this rank's tokens: every branch of
     // the split reduces to that); run by `n` threads once the loads are in place. The experts with replicas are written over.
     auto write_masters = [&](int t, int n) {
         for (int i = t; i < G * Lp; i += n) {
             const int rank = i / Lp, local = i - rank * Lp, e = rank * M + local;
-            a.p2l[domain_start_rank * Lp + i] = local < M ? domain_start_log + e : -1;
-            if (a.physical_loads != nullptr) a.physical_loads[domain_start_rank * Lp + i] = local < M ? sm.loads[e] : 0;
+            out_p2l[domain_start_rank * Lp + i] = local < M ? domain_start_log + e : -1;
+            if (out_physical_loads != nullptr) out_physical_loads[domain_start_rank * Lp + i] = local < M ? sm.loads[e] : 0;
         }
-        for (int e = t; e < E; e += n) a.lcnts[domain_start_log + e] = 1;
+        for (int e = t; e < E; e += n) out_lcnts[domain_start_log + e] = 1;
         const int64_t first = static_cast<int64_t>(domain_start_log) * D;
         auto master = [&](int e) { return (domain_start_rank + e / M) * Lp + e % M; };
-        const uintptr_t align = reinterpret_cast<uintptr_t>(a.l2p) | reinterpret_cast<uintptr_t>(a.quota) |
-                                reinterpret_cast<uintptr_t>(a.quota_prefix) | reinterpret_cast<uintptr_t>(a.rank_quota_prefix);
+        const uintptr_t align = reinterpret_cast<uintptr_t>(out_l2p) | reinterpret_cast<uintptr_t>(out_quota) |
+                                reinterpret_cast<uintptr_t>(out_quota_prefix) | reinterpret_cast<uintptr_t>(out_rank_quota_prefix);
         if (D % 4 == 0 && (align & 15u) == 0) {
             const int vecs = D / 4;
             for (int i = t; i < E * vecs; i += n) {
                 const int e = i / vecs;
                 const bool head = i - e * vecs == 0;
                 const int4 load = make_int4(head ? sm.loads[e] : 0, 0, 0, 0);
-                reinterpret_cast<int4*>(a.l2p + first)[i] = make_int4(head ? master(e) : -1, -1, -1, -1);
-                reinterpret_cast<int4*>(a.quota + first)[i] = load;
-                reinterpret_cast<int4*>(a.quota_prefix + first)[i] = load;
-                reinterpret_cast<int4*>(a.rank_quota_prefix + first)[i] = make_int4(head ? sm.my_loads[e] : 0, 0, 0, 0);
+                reinterpret_cast<int4*>(out_l2p + first)[i] = make_int4(head ? master(e) : -1, -1, -1, -1);
+                reinterpret_cast<int4*>(out_quota + first)[i] = load;
+                reinterpret_cast<int4*>(out_quota_prefix + first)[i] = load;
+                reinterpret_cast<int4*>(out_rank_quota_prefix + first)[i] = make_int4(head ? sm.my_loads[e] : 0, 0, 0, 0);
             }
         } else {
             for (int i = t; i < E * D; i += n) {
                 const int e = i / D;
                 const bool head = i - e * D == 0;
-                a.l2p[first + i] = head ? master(e) : -1;
-                a.quota[first + i] = head ? sm.loads[e] : 0;
-                a.quota_prefix[first + i] = head ? sm.loads[e] : 0;
-                a.rank_quota_prefix[first + i] = head ? sm.my_loads[e] : 0;
+                out_l2p[first + i] = head ? master(e) : -1;
+                out_quota[first + i] = head ? sm.loads[e] : 0;
+                out_quota_prefix[first + i] = head ? sm.loads[e] : 0;
+                out_rank_quota_prefix[first + i] = head ? sm.my_loads[e] : 0;
             }
         }
     };
@@ -582,7 +603,7 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, cha
     if (tid < kSolverProbeWarps) sm.ctrl[kCtlStop0 + tid] = 0;
     const bool do_search = (R > 0 && G > 1);
     stamp(1);
-    __syncthreads();
+    crew.sync();
     if (do_search) {
         // each rank's masters by load descending, ties to the lower index, and its load; four masters a load where they lie so
         const bool fours = (M & 3) == 0;
@@ -610,7 +631,7 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, cha
             sm.masters[base + pos] = make_int2(static_cast<int>(mine), i);
             if (i == base) sm.rank_load[rank] = sum;
         }
-        __syncthreads();
+        crew.sync();
     }
     stamp(2);
     const bool allow0 = a.allow_zero_master != 0;
@@ -661,10 +682,10 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, cha
             if (lane == 0) sm.ctrl[kCtlBuilt0 + warp] = ok ? n + 1 : 0;
             if (ok && lane > warp && lane < kSolverProbeWarps) *(sm.ctrl + kCtlStop0 + lane) = 1;
         }
-        __syncthreads();
+        crew.sync();
         winner = first_feasible(sm, 0, num_batches);
         if (__builtin_expect(winner < 0, 0)) {
-            const int2 found = probe_thresholds(sm.ctrl[kCtlFitting], sm.ctrl[kCtlHi], sm.ctrl[kCtlTotal], sm.ctrl[kCtlLargest], G, M, R, a.min_tokens, allow0);
+            const int2 found = probe_thresholds(crew, sm.ctrl[kCtlFitting], sm.ctrl[kCtlHi], sm.ctrl[kCtlTotal], sm.ctrl[kCtlLargest], G, M, R, a.min_tokens, allow0);
             winner = found.x;
             num_batches = found.y;
         }
@@ -687,7 +708,7 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, cha
             if (lane == 0) report_error(status, UEP_DEV_BAD_PLAN, l_global);
             continue;
         }
-        if (lane == 0 && emits) a.lcnts[l_global] = C;
+        if (lane == 0 && emits) out_lcnts[l_global] = C;
         if (C <= kWarp) {
             const bool active = lane < C;
             const ExportEntry entry = lane > 0 && active ? plan[first + lane - 1] : ExportEntry{0, 0};
@@ -698,12 +719,12 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, cha
                 const int phys = lane == 0 ? host * Lp + e - home * M : domain_start_rank * Lp + (entry.place >> 8);
                 const int prefix = warp_inclusive_scan(q, lane);
                 if (active) {
-                    a.quota[row + lane] = q;
-                    a.quota_prefix[row + lane] = prefix;
-                    if (a.physical_loads != nullptr) a.physical_loads[phys] = q;
+                    out_quota[row + lane] = q;
+                    out_quota_prefix[row + lane] = prefix;
+                    if (out_physical_loads != nullptr) out_physical_loads[phys] = q;
                     if (lane > 0) {
-                        a.p2l[phys] = l_global;
-                        a.l2p[row + lane] = phys;
+                        out_p2l[phys] = l_global;
+                        out_l2p[row + lane] = phys;
                     }
                 }
             }
@@ -719,7 +740,7 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, int domain, cha
             write_many_replicas(a, domain_start_rank, e, C, sm.loads[e], my_load, plan + first);
         }
     }
-    __syncthreads();
+    crew.sync();
     stamp(4);
 }
 
