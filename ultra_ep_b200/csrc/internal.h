@@ -17,7 +17,7 @@ constexpr int kReduceSegments = 16;  // a replica's gradient is released for zer
 constexpr unsigned long long kReduceFlagRadix = 64;  // progress word = epoch * radix + segments done
 
 constexpr int kPlanMaxCtas = 32;  // CTAs of one rank in the plan kernel
-constexpr int kRehearsalOut = 256;  // words that the rehearsal of a plan writes
+constexpr int kRehearsalOut = 512;  // words that the rehearsal of a plan writes
 
 // Where the group's buffers are. By value in the kernels' parameters, so that the first load of a kernel is of data and not
 // of a pointer to it (each of the two is a miss: the tables were last read a layer ago). Fixed once connected. With a table

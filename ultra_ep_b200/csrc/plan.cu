@@ -265,11 +265,11 @@ __host__ __device__ inline size_t plan_matrix_bytes(int N, int L) {
 // CTA that owns a rank has a second crew of threads, which solves a small problem from the kernel's start, while the first one counts
 // and exchanges, with the same instructions. Nobody waits for it. It takes the way of the default parameters: the sort, the four
 // builds side by side with an expert of two exports and ranks that come back, outputs and splits of experts with replicas; not the rounds
-// of probes nor more than 32 replicas. Its outputs go to a place of their own. Step of eight ranks among others without it and like
+// of probes nor more than 32 replicas, nor masters and replicas that do not come in fours. Its outputs go to a place of their own. Step of eight ranks among others without it and like
 // this (us): bf16 experts of 9 MB, 8192 bool rows of 128 64.3 and 59.2; fp8 experts of 19 MB, 8192 int32 tokens of 128 56.1 and 54.4; plan and
 // reroute of 4096 tokens of 64 18.8 and 18.1, of 33 11.6 and 11.4. (A CTA of its own warms L2 alone: the plan's builds 2.2 us instead of
 // 1.8; half of the ranks with the outputs first 59.2 and 59.3.)
-constexpr int kRehearsalRanks = 4, kRehearsalMasters = 2, kRehearsalSlots = 2, kRehearsalD = 4;
+constexpr int kRehearsalRanks = 4, kRehearsalMasters = 4, kRehearsalSlots = 2, kRehearsalD = 4;
 constexpr int kRehearsalExperts = kRehearsalRanks * kRehearsalMasters;
 constexpr int kRehearsalPhysical = kRehearsalRanks * (kRehearsalMasters + kRehearsalSlots);
 static_assert(4 * kRehearsalExperts * kRehearsalD + kRehearsalExperts + 2 * kRehearsalPhysical <= kRehearsalOut, "room for its outputs");
@@ -281,7 +281,8 @@ __device__ __forceinline__ void rehearsal_args(const PlanCall& call, const Crew&
     const SolverSmem sm = carve_solver_smem(smem_raw, kRehearsalExperts, kRehearsalRanks, kRehearsalSlots);
     int32_t* matrix = reinterpret_cast<int32_t*>(smem_raw + solver_smem_bytes(kRehearsalExperts, kRehearsalRanks, kRehearsalSlots));
     for (int i = crew.tid; i < kRehearsalExperts; i += crew.threads) {
-        const int load = (i & 1) != 0 ? 100 : 6000 >> 2 * (i >> 2) * (i >> 1);  // 6000, 6000, 375, 93
+        const int rank = i / kRehearsalMasters;
+        const int load = i % kRehearsalMasters != 0 ? 100 : (rank < 2 ? 6000 : 375 >> 2 * (rank - 2));
         sm.loads[i] = load;
         sm.my_loads[i] = load / 4;
         for (int r = 0; r < kRehearsalRanks; ++r) matrix[r * kRehearsalExperts + i] = load / 4;

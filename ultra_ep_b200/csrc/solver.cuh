@@ -114,9 +114,10 @@ __device__ inline SolverSmem carve_solver_smem(char* raw, int E, int G, int R) {
     return s;
 }
 
-__device__ __forceinline__ int warp_inclusive_scan(int v, int lane) {
-#pragma unroll
-    for (int off = 1; off < kWarp; off <<= 1) {
+// Over the first n lanes.
+__device__ __forceinline__ int warp_inclusive_scan(int v, int lane, int n) {
+#pragma unroll 1
+    for (int off = 1; off < n; off <<= 1) {
         const int t = __shfl_up_sync(kFullMask, v, off);
         if (lane >= off) v += t;
     }
@@ -535,7 +536,7 @@ __device__ __forceinline__ void warp_rank_quota_prefix(const SolveArgs& a, int l
             }
         }
     }
-    const int prefix = warp_inclusive_scan(my_alloc, lane);
+    const int prefix = warp_inclusive_scan(my_alloc, lane, C);
     if (active) as_global(a.rank_quota_prefix)[static_cast<int64_t>(l_global) * a.D + lane] = prefix;
 }
 
@@ -695,11 +696,12 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, const Crew& cre
     // j-th export in the order of their creation.
     const ExportEntry* plan = sm.plan + winner * sm.slots;
     const uint32_t* batches = sm.batches + winner * sm.slots;
-    // Where there are warps enough, one writes an expert's rows and another one splits this rank's tokens.
-    const int warps = nthreads / kWarp, apart = 2 * num_batches <= warps ? 1 : 0;
-    for (int task = warp; task < num_batches << apart; task += warps) {
-        const uint32_t batch = batches[task >> apart];
-        const bool emits = apart == 0 || (task & 1) == 0, splits = apart == 0 || (task & 1) != 0;
+    // Where there are warps enough, one of its own splits this rank's tokens, which takes longest, and the others write the rows.
+    const int warps = nthreads / kWarp;
+    const bool apart = num_batches < warps, split_only = apart && warp < num_batches, emit_only = apart && !split_only;
+    for (int task = emit_only ? warp - num_batches : warp; task < num_batches; task += emit_only ? warps - num_batches : warps) {
+        const uint32_t batch = batches[task];
+        const bool emits = !split_only, splits = !emit_only;
         const int e = batch & 511, first = batch >> 9 & 511, C = static_cast<int>(batch >> 18 & 127) + 1, home = batch >> 25;
         const int l_global = domain_start_log + e;
         const int64_t row = static_cast<int64_t>(l_global) * D;
@@ -717,7 +719,7 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, const Crew& cre
             const int q = lane == 0 ? sm.loads[e] - moved : entry.quota;
             if (emits) {
                 const int phys = lane == 0 ? host * Lp + e - home * M : domain_start_rank * Lp + (entry.place >> 8);
-                const int prefix = warp_inclusive_scan(q, lane);
+                const int prefix = warp_inclusive_scan(q, lane, C);
                 if (active) {
                     out_quota[row + lane] = q;
                     out_quota_prefix[row + lane] = prefix;
