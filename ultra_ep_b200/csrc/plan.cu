@@ -582,12 +582,14 @@ std::atomic<int64_t> g_launches{0};
 
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
-// Twice the threads where a CTA's slice of the input would be several rounds of loads. Step of eight ranks with 256 threads and 512 (us),
-// above the line: 16384 int64 tokens of 256 experts (70 KB a CTA) 106.8 and 104.5, 2600 bool rows of 256 (44 KB) 53.4 and 51.8, 8192 bool rows
-// of 128 (70 KB) 59.3 and 59.4; below it, where nothing is left to share, smaller blocks start sooner.
+// Twice the threads where a CTA's slice of the input is long enough to pay for the larger block. Step of eight ranks with 256 threads and
+// 512 (us), below the line: 2200 bool rows of 128 experts (18.3 KB a CTA) 36.5 and 38.2, 2600 (21.7 KB) 35.3 and 36.4, 8192 int32 tokens of 128
+// (17 KB) 52.5 and 52.7, 9600 (20 KB) 39.65 and 39.6, 4800 int64 tokens of 64 (20 KB) 27.9 and 28.1; above it 11000 int32 tokens (23 KB) 40.75
+// and 40.3, 2600 bool rows of 256 (43 KB) 53.4 and 51.8, 16384 int64 tokens of 256 (68 KB) 106.8 and 104.5.
+constexpr int kFewThreadsBytes = 22 * 1024;
 int plan_threads(int input_kind, int max_T, int K_or_L, int ctas) {
     const int64_t bytes = static_cast<int64_t>(max_T) * K_or_L * (input_kind == 0 ? 1 : (input_kind == 1 ? 4 : 8));
-    return bytes > static_cast<int64_t>(ctas) * 16 * 1024 ? 2 * kPlanThreads : kPlanThreads;
+    return bytes > static_cast<int64_t>(ctas) * kFewThreadsBytes ? 2 * kPlanThreads : kPlanThreads;
 }
 
 int plan_ctas_per_rank(int input_kind, int max_T, int K_or_L, int cap) {
