@@ -117,6 +117,28 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
     };
     stamp(0);
 
+    // Every global read of the set-up is asked for here, before anything depends on one of them: a master's count, its row of
+    // instances (up to eight of them) and its gradients' addresses by a thread each, the owner of a redundant slot, the epoch. One
+    // memory round trip then, where the count, each instance, the addresses and the owner came one behind the other.
+    const int total_masters = nlocal * M;
+    const bool row_cached = D <= 8;
+    int pre_reps = 0, pre_row[7], pre_owner = -1;
+    uintptr_t pre_grad[2] = {0, 0};
+    {
+        const bool valid = tid < total_masters;
+        const int lr = valid ? tid / M : 0, m = valid ? tid % M : 0, l = group.my_rank[lr] * M + m;
+        const PlanPtrs& plan = call.plan[lr];
+        if (valid) pre_reps = plan.lcnts[l] - 1;
+#pragma unroll
+        for (int j = 0; j < 7; ++j) pre_row[j] = valid && row_cached && j < D - 1 ? plan.l2p[static_cast<int64_t>(l) * D + 1 + j] : -1;
+        if (valid) {
+            pre_grad[0] = static_cast<uintptr_t>(call.fc1_grad_ptrs[lr][m]);
+            pre_grad[1] = static_cast<uintptr_t>(call.fc2_grad_ptrs[lr][m]);
+        }
+        if (tid < nlocal * R && nlocal * R <= kMaxOwned) pre_owner = call.plan[tid / R].p2l[group.my_rank[tid / R] * Lp + M + tid % R];
+    }
+    unsigned long long pre_epoch = 0;
+    if (tid == 0) pre_epoch = *call.reduce_epoch;
     if (tid == 0) {
         sm.n_active = 0;
         sm.total_reps = 0;
@@ -127,7 +149,7 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
         sm.n_away = 0;
         sm.done_items = 0;
         sm.pull_finished = 0;
-        sm.epoch = *call.reduce_epoch + 1;  // ranks hosted together share the first one's counter
+        sm.epoch = pre_epoch + 1;  // ranks hosted together share the first one's counter
         for (int s = 0; s < kReduceStages; ++s) {
             mbar_init(&sm.full[s], 1);
             mbar_init(&sm.empty[s], kReduceConsumers / 32);
@@ -152,7 +174,6 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
     };
     // pull list: masters of the hosted ranks with replicas, and where each replica lives.
     // Hosted ranks pool their tiles over all CTAs of the launch.
-    const int total_masters = nlocal * M;
     for (int g0 = 0; g0 < total_masters; g0 += blockDim.x) {
         const int gm = g0 + tid;
         const int lr = gm < total_masters ? gm / M : 0;
@@ -161,7 +182,7 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
         const int me = group.my_rank[lr];
         int reps = 0;
         if (gm < total_masters) {
-            reps = plan.lcnts[me * M + m] - 1;
+            reps = g0 == 0 ? pre_reps : plan.lcnts[me * M + m] - 1;
             reps = reps < 0 ? 0 : (reps > D - 1 ? D - 1 : reps);
         }
         const int act = reps > 0 ? 1 : 0;
@@ -190,8 +211,7 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
             const int rs = r_off + r_incl - reps;
             sm.rep_start[ai] = static_cast<short>(rs);
             const int l = me * M + m;
-            for (int j = 0; j < reps && rs + j < kMaxPulls; ++j) {
-                const int phys = plan.l2p[static_cast<int64_t>(l) * D + 1 + j];
+            auto place = [&](int j, int phys) {
                 const int prank = phys / Lp, pslot = phys % Lp - M;
                 if (phys < 0 || prank >= N || pslot < 0 || pslot >= R) {
                     report_error(group.status[lr], UEP_DEV_BAD_PLAN, l);
@@ -203,9 +223,17 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
                     if (!hosted) atomicOr(&sm.pull_mask[lr][prank >> 5], 1u << (prank & 31));
                     atomicAdd(hosted ? &sm.n_hosted : &sm.n_away, 1);
                 }
+            };
+            if (g0 == 0 && row_cached) {
+#pragma unroll
+                for (int j = 0; j < 7; ++j) {
+                    if (j < reps && rs + j < kMaxPulls) place(j, pre_row[j]);
+                }
+            } else {
+                for (int j = 0; j < reps && rs + j < kMaxPulls; ++j) place(j, plan.l2p[static_cast<int64_t>(l) * D + 1 + j]);
             }
-            const uintptr_t p1 = static_cast<uintptr_t>(call.fc1_grad_ptrs[lr][m]);
-            const uintptr_t p2 = static_cast<uintptr_t>(call.fc2_grad_ptrs[lr][m]);
+            const uintptr_t p1 = g0 == 0 ? pre_grad[0] : static_cast<uintptr_t>(call.fc1_grad_ptrs[lr][m]);
+            const uintptr_t p2 = g0 == 0 ? pre_grad[1] : static_cast<uintptr_t>(call.fc2_grad_ptrs[lr][m]);
             sm.master[ai][0] = reinterpret_cast<float*>(p1);
             sm.master[ai][1] = reinterpret_cast<float*>(p2);
             if ((p1 & 15u) || (p2 & 15u)) atomicAnd(&sm.vector_ok, 0);
@@ -223,8 +251,7 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
     {
         const int i = tid;
         const bool in = i < nlocal * R && nlocal * R <= kMaxOwned;
-        int l = -1;
-        if (in) l = call.plan[i / R].p2l[group.my_rank[i / R] * Lp + M + i % R];
+        const int l = pre_owner;
         const bool used = in && l >= 0 && l / M < N && !hosted_here(l / M);
         const unsigned has = __ballot_sync(kFullMask, used);
         const int lane = tid & 31, warp = tid >> 5;
