@@ -31,9 +31,12 @@
 //     hold a stage as long as a remote tile does, and with one replica per master half of the
 //     ring would be taken away from the remote loads;
 //   * tiles are interleaved over masters so that concurrent CTAs pull from different peers; they go
-//     expert by expert where all replicas lie in this device's memory.
+//     expert by expert where all replicas lie in this device's memory, and long streams of those
+//     are handed out as CTAs ask for more.
 // The CTA budget (SMs used while the backward pass runs next to it) is the caller's knob
-// (grad_reduce_num_sms); each CTA holds about 215 KB of shared memory (twelve stages and the zero tile are 200 KiB).
+// (grad_reduce_num_sms); each CTA holds about 225 KB of shared memory (twelve stages and the zero tile are 200 KiB).
+
+#include <climits>
 
 #include "internal.h"
 
@@ -51,6 +54,13 @@ constexpr int kReduceStages = 9;                       // ring of remote replica
 constexpr int kMasterStages = 3;                       // ring of local master tiles
 constexpr int kReduceVecPerThread = kReduceTileElems / 4 / kReduceConsumers;  // float4 per thread per tile
 constexpr int kMaxPulls = kMaxExportsPerDomain;
+// Items handed out as CTAs ask for them, in runs: a CTA keeps those that it took, for the clearing, at most so many; half as many is its
+// even share.
+constexpr int kMaxRuns = 1024, kLeastRun = 2, kRunsAhead = 2;
+constexpr int kHandOutItems = 64;    // of a CTA's even share, at least
+constexpr int kHandOutTiles = 2048;  // of an expert, at least
+constexpr int kItemRing = 32;  // items between the thread that takes them and the warps that add them up: at most the stages of both rings and two
+static_assert(kItemRing >= kReduceStages + kMasterStages + 4, "an item is not overwritten while it is looked up");
 constexpr int kMaxOwned = 64;  // used replica slots of the hosted ranks (a lane of a warp asks for two)
 
 struct ReduceShared {
@@ -59,6 +69,9 @@ struct ReduceShared {
     int n_owned;
     volatile long long done_items;                 // items of this CTA whose replica tiles have all been consumed
     volatile int pull_finished;                    // the pull phase of this CTA is over (all items, or given up)
+    int2 items[kItemRing];                         // handed out: {active, tile} of the k-th item of this CTA at k mod its size; active -1 behind the last one
+    volatile int items_ready;                      // how many of them there are so far
+    int runs[kMaxRuns];                            // the first items of the runs that this CTA took
     int n_hosted;                                  // replicas that lie on ranks of this launch
     int n_away;                                    // replicas on other devices
     unsigned long long epoch;
@@ -140,6 +153,9 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
+// kHandOut: items may be handed out to CTAs as they ask for them. A kernel of its own, because short streams lose by the code for it
+// (backward of eight ranks, 20 and 15 items a CTA 46.5 and 47.9 us without it, 46.8 and 48.2 with it there and not taken).
+template <bool kHandOut>
 __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCall call) {
     extern __shared__ __align__(128) char smem_raw[];  // kReduceStages replica tiles, kMasterStages master tiles, the zero tile
     __shared__ ReduceShared sm;
@@ -188,6 +204,7 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
         sm.n_away = 0;
         sm.done_items = 0;
         sm.pull_finished = 0;
+        sm.items_ready = 0;
         sm.epoch = pre_epoch + 1;  // ranks hosted together share the first one's counter
         for (int s = 0; s < kReduceStages; ++s) {
             mbar_init(&sm.full[s], 1);
@@ -325,6 +342,17 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
     const int64_t total_items = static_cast<int64_t>(n_active) * tiles_total;
     const int64_t first = blockIdx.x, step = gridDim.x;
     const int64_t count = first < total_items ? (total_items - first + step - 1) / step : 0;
+    // Where all replicas lie in this device's memory, and there are items enough, CTAs take them as they get on: of even shares the median
+    // CTA was through after 169 us and the last one after 202, like this after 173 and 176 (128 experts of 18.9 M elements). Backward of
+    // eight ranks, even shares and like this (us): 192 items a CTA of 4608 tiles an expert 276 and 259, 140 of 3240 211 and 191, 80 of 2304
+    // 146.2 and 144.8; below the lines 60 of 1620 98.7 and 99.3, 1536 tiles 102.0 and 102.7, 20 of 576 48.2 and 48.7, 15 of 384 46.4 and
+    // 46.8. (One item at a time 282 for 259, four the same.) Ranks of other devices are told how far each CTA has come in an order that
+    // they know: there the shares are fixed.
+    const bool handed_out = kHandOut && sm.n_away == 0 && sm.n_owned == 0 && sm.vector_ok != 0 && total_items >= kHandOutItems * step && total_items < 1 << 30;
+    int run = kLeastRun;  // items at a time
+    if (handed_out && total_items > step * (kLeastRun * kMaxRuns / 2)) {
+        run = static_cast<int>((static_cast<unsigned>(total_items) + gridDim.x * (kMaxRuns / 2) - 1) / (gridDim.x * (kMaxRuns / 2)));
+    }
     const ItemCursor start(static_cast<int>(first), static_cast<int>(step), n_active, expert_tiles);
     // segment s covers the tiles [seg_end(s-1), seg_end(s)) of an expert; items come tile after tile
     auto seg_end = [&](int s) -> int { return static_cast<int>(static_cast<int64_t>(s + 1) * tiles_total / kReduceSegments); };
@@ -372,7 +400,9 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
 
     // ---- clearing warp: the used replica slots hosted here, segment by segment as their master's rank releases
     //      them; runs beside the pulls of this CTA (every CTA of the launch takes every gridDim-th tile) ----------
-    if (tid >= kReduceConsumers + 96) {
+    if (handed_out && tid >= kReduceConsumers + 64) {
+        // nothing to report and nothing to wait for: the thread that takes items closes the epoch, and clears
+    } else if (tid >= kReduceConsumers + 96) {
         // ---- reporting warp: keeps the atomics and the flag stores of the progress report off the threads that
         //      feed the rings (each costs a round trip to memory) -----------------------------------------------
         if (tid == kReduceConsumers + 96) {
@@ -494,15 +524,37 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
             int64_t m_issued = 0;
             ItemCursor cursor = start;
             RingPlace<kMasterStages> place;
-            for (; m_issued < count; ++m_issued, place.advance(), cursor.advance(n_active, expert_tiles)) {
+            for (; handed_out || m_issued < count; ++m_issued, place.advance(), cursor.advance(n_active, expert_tiles)) {
                 const int s = place.stage;
-                const ReduceItem it = cursor.item(fc1, fc2, tiles_fc1);
-                const float* from = master_ptr(it);
+                if (handed_out) {
+                    const uint64_t t_begin = global_timer_ns();
+                    bool there = sm.items_ready > m_issued;
+                    while (!there) {  // (the thread that takes them ends with a -1, whatever happens)
+                        if (global_timer_ns() - t_begin > 2 * call.timeout_ns) break;
+                        there = sm.items_ready > m_issued;
+                    }
+                    __threadfence_block();
+                    const int2 next = there ? sm.items[m_issued % kItemRing] : make_int2(-1, 0);
+                    cursor.active = next.x;
+                    cursor.tile = next.y;
+                }
+                const bool end = cursor.active < 0;
+                ReduceItem it{};
+                const float* from = nullptr;
+                if (!end) {
+                    it = cursor.item(fc1, fc2, tiles_fc1);
+                    from = master_ptr(it);
+                }
                 if (m_issued >= kMasterStages) {  // the stage's previous tile has been read by every consumer warp
                     if (!mbar_wait(&sm.m_empty[s], place.parity ^ 1u, sm.error ? 0 : call.timeout_ns)) {
                         sm.error = 1;
                         break;
                     }
+                }
+                if (end) {  // the consumers find it where an item would be
+                    sm.items[m_issued % kItemRing] = make_int2(-1, 0);
+                    mbar_arrive(&sm.m_full[s]);
+                    break;
                 }
                 const uint32_t bytes = static_cast<uint32_t>(it.elems) * 4u;
                 mbar_expect_tx(&sm.m_full[s], bytes);
@@ -524,12 +576,57 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
             ItemCursor cursor = start;
             RingPlace<kReduceStages> fill, drain;
             bool last_of_item = false;
+            // Handed out: the first run is the CTA's own number, the next ones are asked for ahead. Items without a replica to add (a plan with
+            // bad entries) stay as they are.
+            int taken = 0, left = 0, published = 0, asked = 1;
+            int ahead[kRunsAhead];  // runs asked for
+            auto ask = [&]() { return handed_out && asked++ < kMaxRuns ? static_cast<int>(gridDim.x) + atomicAdd(call.counters, 1) : INT_MAX; };
+            ahead[0] = static_cast<int>(blockIdx.x);
+#pragma unroll
+            for (int i = 1; i < kRunsAhead; ++i) ahead[i] = ask();
+            auto publish = [&](int active, int tile) {
+                sm.items[published % kItemRing] = make_int2(active, tile);
+                __threadfence_block();
+                sm.items_ready = ++published;
+            };
+            // The next item of this CTA into it_rep; false: none.
+            auto next_item = [&]() -> bool {
+                if (!handed_out) {
+                    if (k_rep >= count) return false;
+                    it_rep = cursor.item(fc1, fc2, tiles_fc1);
+                    cursor.advance(n_active, expert_tiles);
+                    return true;
+                }
+                while (true) {
+                    if (left > 0) {
+                        if (++cursor.tile == expert_tiles) {
+                            cursor.tile = 0;
+                            ++cursor.active;
+                        }
+                    } else {
+                        const int64_t at = static_cast<int64_t>(ahead[0]) * run;
+                        if (at >= total_items) return false;
+                        cursor.active = static_cast<int>(at) / expert_tiles;
+                        cursor.tile = static_cast<int>(at) - cursor.active * expert_tiles;
+                        left = min(run, static_cast<int>(total_items - at));
+                        sm.runs[taken++] = static_cast<int>(at);
+#pragma unroll
+                        for (int i = 0; i + 1 < kRunsAhead; ++i) ahead[i] = ahead[i + 1];
+                        ahead[kRunsAhead - 1] = ask();  // (whoever has twice an even share asks for no more: the others have room for the rest)
+                    }
+                    --left;
+                    bool any = false;
+                    for (int r = sm.rep_start[cursor.active]; r < sm.rep_start[cursor.active + 1] && !any; ++r) any = sm.rep_base[r] != nullptr;
+                    if (!any) continue;
+                    publish(cursor.active, cursor.tile);
+                    it_rep = cursor.item(fc1, fc2, tiles_fc1);
+                    return true;
+                }
+            };
             auto next_replica = [&](float*& src, int& elems) -> bool {
                 while (true) {
                     if (r_issue < 0) {
-                        if (k_rep >= count) return false;
-                        it_rep = cursor.item(fc1, fc2, tiles_fc1);
-                        cursor.advance(n_active, expert_tiles);
+                        if (!next_item()) return false;
                         r_issue = sm.rep_start[it_rep.active];
                         r_issue_end = sm.rep_start[it_rep.active + 1];
                     }
@@ -582,18 +679,46 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
                     mbar_wait(&sm.full[j % kReduceStages], static_cast<uint32_t>((j / kReduceStages) & 1), call.timeout_ns);
                 }
             }
+            if (handed_out) {
+                publish(-1, 0);
+                // When everybody has asked for the last time, the counters go back and the epoch is closed. (The fence: what was
+                // asked for ahead and never looked at must have been counted before.)
+                __threadfence();
+                if (atomicAdd(&call.counters[kReduceSegments - 1], 1) == static_cast<int>(gridDim.x) - 1) {
+                    __threadfence();
+                    call.counters[0] = 0;
+                    call.counters[kReduceSegments - 1] = 0;
+                    *call.reduce_epoch = epoch;
+                }
+            }
             sm.pull_finished = 1;
             // Replicas of ranks of this launch: the CTA that pulled a tile clears it, once it has pulled all of its tiles. The
             // clearing is then mostly a phase of writes behind the phase of pulls; clearing a tile as soon as it has been read
             // took 273 us for 257, in batches of 16 items 273, of 64 268 (18.9 M elements; at 4.7 M 78 us each).
             if (sm.n_hosted > 0 && !sm.error) {
-                cursor = start;
-                for (int64_t k = 0; k < count; ++k, cursor.advance(n_active, expert_tiles)) {
+                auto clear_item = [&]() {
                     const ReduceItem it = cursor.item(fc1, fc2, tiles_fc1);
                     const int r0 = sm.rep_start[it.active], r1 = sm.rep_start[it.active + 1];
                     for (int r = r0; r < r1; ++r) {
                         if (sm.rep_base[r] != nullptr && sm.rep_hosted[r]) clear_tile(replica_ptr(it, r), it.elems);
                     }
+                };
+                if (handed_out) {
+                    for (int k = 0; k < taken; ++k) {
+                        const int at = sm.runs[k];
+                        cursor.active = at / expert_tiles;
+                        cursor.tile = at - cursor.active * expert_tiles;
+                        for (int i = min(run, static_cast<int>(total_items) - at); i > 0; --i) {
+                            clear_item();
+                            if (++cursor.tile == expert_tiles) {
+                                cursor.tile = 0;
+                                ++cursor.active;
+                            }
+                        }
+                    }
+                } else {
+                    cursor = start;
+                    for (int64_t k = 0; k < count; ++k, cursor.advance(n_active, expert_tiles)) clear_item();
                 }
                 bulk_wait_all<0>();
             }
@@ -603,17 +728,25 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
         const int lane = tid & 31;
         ItemCursor cursor = start;
         RingPlace<kMasterStages> m_place;
+        const uint64_t wait_ns = handed_out ? 2 * call.timeout_ns : call.timeout_ns;
         RingPlace<kReduceStages> place;
         stamp(2);
-        for (int64_t k = 0; k < count; ++k, m_place.advance(), cursor.advance(n_active, expert_tiles)) {
-            const ReduceItem it = cursor.item(fc1, fc2, tiles_fc1);
+        for (int64_t k = 0; handed_out || k < count; ++k, m_place.advance(), cursor.advance(n_active, expert_tiles)) {
+            ReduceItem it{};
+            if (!handed_out) it = cursor.item(fc1, fc2, tiles_fc1);  // beside the wait
+            const bool there = mbar_wait(&sm.m_full[m_place.stage], m_place.parity, sm.error ? 0 : wait_ns);
+            if (!there) sm.error = 1;  // keep the control flow uniform; the result of this tile is void
+            if (handed_out) {  // an item is there before its master's tile is
+                const int2 next = __all_sync(kFullMask, there) ? sm.items[k % kItemRing] : make_int2(-1, 0);
+                if (next.x < 0) break;
+                cursor.active = next.x;
+                cursor.tile = next.y;
+                it = cursor.item(fc1, fc2, tiles_fc1);
+            }
             const int nvec = it.elems >> 2;
             float4 acc[kReduceVecPerThread];
             {
                 const int s = m_place.stage;
-                if (!mbar_wait(&sm.m_full[s], m_place.parity, sm.error ? 0 : call.timeout_ns)) {
-                    sm.error = 1;  // keep the control flow uniform; the result of this tile is void
-                }
                 const float4* stage = reinterpret_cast<const float4*>(master_ring + s * kReduceTileBytes);
 #pragma unroll
                 for (int u = 0; u < kReduceVecPerThread; ++u) {
@@ -660,20 +793,24 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
 }  // namespace
 
 cudaError_t launch_grad_reduce(const ReduceCall& call, cudaStream_t stream) {
+    const dim3 grid(call.nlocal * call.ctas_per_rank), block(kReduceThreads);
+    // Whether items may be handed out goes by the size of an expert: how many experts have replicas is not known here.
+    const int64_t tiles = (call.fc1_numel + kReduceTileElems - 1) / kReduceTileElems + (call.fc2_numel + kReduceTileElems - 1) / kReduceTileElems;
+    const bool hand_out = call.nlocal == call.N && !call.owners_clear && tiles >= kHandOutTiles;
+    void (*const kernel)(ReduceCall) = hand_out ? grad_reduce_kernel<true> : grad_reduce_kernel<false>;
     const size_t smem = static_cast<size_t>(kReduceStages + kMasterStages) * kReduceTileBytes + kReduceZeroBytes;
-    cudaError_t e = allow_smem(reinterpret_cast<const void*>(grad_reduce_kernel), smem);
+    cudaError_t e = allow_smem(reinterpret_cast<const void*>(kernel), smem);
     if (e != cudaSuccess) return e;
     if (call.nlocal * call.R > kMaxOwned) return cudaErrorInvalidValue;  // more replica slots per launch than the kernel's table holds
     count_launch();
-    const dim3 grid(call.nlocal * call.ctas_per_rank), block(kReduceThreads);
     if (call.nlocal > 1 && call.owners_clear) {
         // hosted ranks clear their slots behind other hosted ranks' pulls inside this one launch: the CTAs that
         // wait and the CTAs they wait for must be resident together. (Else no CTA waits for another one of its launch.)
         ReduceCall copy = call;
         void* args[] = {&copy};
-        return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(grad_reduce_kernel), grid, block, args, smem, stream);
+        return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), grid, block, args, smem, stream);
     }
-    grad_reduce_kernel<<<grid, block, smem, stream>>>(call);
+    kernel<<<grid, block, smem, stream>>>(call);
     return cudaGetLastError();
 }
 
