@@ -294,14 +294,15 @@ __device__ __forceinline__ int sum_earlier_tiles(const uint8_t* counts, int tile
 // instance: its column is copied; with several: a warp resolves the column's marked rows), and then a thread owns four
 // physical columns of four rows and writes them out of its registers: a probability is read where its bit is set,
 // zeros are written elsewhere. Outputs wider than kDenseMaxChunkCols go in column chunks.
-// Two thirds of the kernel's time is instructions, so what is done for every expert is little: its one physical column, or that it
+// What is done for every expert is little: its one physical column, or that it
 // has several. Plan rows, the router and the tiles in front are looked up for an expert with several that the tile routes to, by
 // the warp that resolves it, in a few words of its own; shared memory is 4 KB at 128 experts. With all plan rows staged, all
 // experts' tiles added up by every CTA (15 KB) and eight rows a thread, and like this (us): the pair for eight ranks of 8192 tokens
 // and 128 experts 30.0 and 27.3, of 4096 17.0 and 13.7; step of 8192 x 128 with bf16 experts of 9 MB 67.1 and 64.2, of 2000 x 256 with
-// 3 MB 52.3 and 49.4; one rank of 8191 x 256, sparse, dense and backward, 31.9 and 27.9. 64 registers and one spilled word: with 40 (six CTAs an SM) 17.7,
+// 3 MB 52.3 and 49.4; one rank of 8191 x 256, sparse, dense and backward, 31.9 and 27.9. 64 registers and three spilled words: with 40 (six CTAs an SM) 17.7,
 // with 32 28. Marked cells written over zeros in memory are partial sectors, and rows gathered in shared memory and sent as
-// bulk stores wait too long for each other: both slower.
+// bulk stores wait too long for each other: both slower. So were all experts with several resolved together, marks shared by the lanes
+// (38.0 to 38.9), though that is fewer instructions. A tile's 9.8 us among 591 others: 4 until its bits are physical, 5 to write.
 constexpr int kDenseMaxChunkCols = 4096;
 constexpr int kDenseMaxExperts = 1340;
 constexpr int kDenseMaxThreads = 512;
@@ -410,20 +411,18 @@ dense_scatter_kernel(Batch<DenseFwdArgs> batch, int L, int P, int D, int quota_m
     // ---- nothing here depends on the count kernel ------------------------------------------------
     for (int i = tid; i < pad4(chunk_cols) / 4 * kDenseSegs; i += blockDim.x) reinterpret_cast<uint32_t*>(s.phys_bits)[i] = 0;
     if (tid == 0) n_several = 0;
-    for (int e = tid; e < L; e += blockDim.x) {
-        const int C = a.lcnts[e], p = a.l2p[static_cast<int64_t>(e) * D];
-        s.place[e] = C > 1 ? kSeveralPlaces : (C == 1 && p >= 0 && p < P ? p : kNoPlace);
-    }
-    tile_bit_columns(a.map + static_cast<int64_t>(r0) * L, rows, kDenseSegs, L, s.bits);
-    __syncthreads();
-    for (int e = tid; e < L; e += blockDim.x) {
-        if (s.place[e] == kSeveralPlaces) {
-            uint32_t any = 0;
-#pragma unroll
-            for (int g = 0; g < kDenseSegs; ++g) any |= s.bits[g * Lq + e];
-            if (any) s.several[atomicAdd(&n_several, 1)] = static_cast<uint16_t>(e);
+    {
+        auto place_of = [&](int C, int p) { return C > 1 ? kSeveralPlaces : (C == 1 && p >= 0 && p < P ? p : kNoPlace); };
+        int C = 0, p = 0;  // asked for beside the map
+        if (tid < L) {
+            C = a.lcnts[tid];
+            p = a.l2p[static_cast<int64_t>(tid) * D];
         }
+        tile_bit_columns(a.map + static_cast<int64_t>(r0) * L, rows, kDenseSegs, L, s.bits);
+        if (tid < L) s.place[tid] = place_of(C, p);
+        for (int e = tid + blockDim.x; e < L; e += blockDim.x) s.place[e] = place_of(a.lcnts[e], a.l2p[static_cast<int64_t>(e) * D]);
     }
+    __syncthreads();
 
     const float* probs = a.probs + static_cast<int64_t>(r0) * L;
     float* out_probs = a.out_probs + static_cast<int64_t>(r0) * P;
@@ -437,17 +436,26 @@ dense_scatter_kernel(Batch<DenseFwdArgs> batch, int L, int P, int D, int quota_m
             for (int i = tid; i < Cq / 4 * kDenseSegs; i += blockDim.x) reinterpret_cast<uint32_t*>(s.phys_bits)[i] = 0;
             __syncthreads();
         }
-        for (int e = tid; e < L; e += blockDim.x) {  // experts with one instance
-            const int p = s.place[e] - p_lo;
-            if (s.place[e] < 0 || p < 0 || p >= cols) continue;
-            bool any = false;  // a caller's table may have the column for another expert too, which the tile routes to
+        for (int e = tid; e < L; e += blockDim.x) {  // experts with one instance; the first time also the list of the others
+            const int place = s.place[e], p = place - p_lo;
+            const bool single = place >= 0 && p >= 0 && p < cols;
+            if (!single && (p_lo > 0 || place != kSeveralPlaces)) continue;
+            uint32_t b[kDenseSegs], any = 0;
 #pragma unroll
             for (int g = 0; g < kDenseSegs; ++g) {
-                const uint8_t b = s.bits[g * Lq + e];
-                if (b != 0) s.phys_bits[g * Cq + p] = b;
-                any = any || b != 0;
+                b[g] = s.bits[g * Lq + e];
+                any |= b[g];
             }
-            if (any) s.expert_of[p] = static_cast<uint16_t>(e);
+            if (any == 0) continue;  // a caller's table may have the column for another expert too, which the tile routes to
+            if (!single) {
+                s.several[atomicAdd(&n_several, 1)] = static_cast<uint16_t>(e);
+                continue;
+            }
+#pragma unroll
+            for (int g = 0; g < kDenseSegs; ++g) {
+                if (b[g] != 0) s.phys_bits[g * Cq + p] = static_cast<uint8_t>(b[g]);
+            }
+            s.expert_of[p] = static_cast<uint16_t>(e);
         }
         if (p_lo == 0 && overlapped) pdl_wait();
         __syncthreads();  // the list of experts with several; the bytes above share words with the atomics below
@@ -1163,8 +1171,14 @@ cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int
     // 71.6 and 72.7.
     const bool by_four = L <= 128 && static_cast<int64_t>(grid.x) * b.n > kCountCtasPerSm * sms;
     const auto count = by_four ? dense_count_kernel<4> : dense_count_kernel<1>;
-    // up to two tiles per SM the scatter kernel is a chain of phases: more threads shorten each
-    const int threads = static_cast<int64_t>(grid.x) * b.n <= 2 * sms ? kDenseMaxThreads : kRerouteThreads;
+    // Up to two tiles an SM the scatter kernel is a chain of phases: more threads shorten each. Of 256 threads (64 registers) an SM
+    // holds four tiles, of 128 eight: between the two all tiles are under way at once with 128, and their phases, of which only the last one
+    // writes, fill each other's gaps; with 256 the first wave writes when the second one has not begun. Plan and pair of eight ranks, 256 and
+    // 128 threads (us): 4800 rows of 128 experts 29.8 and 27.8, 8192 40.1 and 38.0, of 64 experts 28.5 and 25.7, of 256 61.2 and 60.5; beside
+    // a weight_sync 8192 x 128 with bf16 experts of 9 MB 58.0 and 56.8, 6500 x 64 with fp8 of 5 MB 41.6 and 39.6. In one wave either way, 4096
+    // x 128 25.3 and 25.9; in two, 12000 x 128 52.7 and 54.1.
+    const int64_t all_tiles = static_cast<int64_t>(grid.x) * b.n;
+    const int threads = all_tiles <= 2 * sms ? kDenseMaxThreads : (all_tiles > 4 * sms && all_tiles <= 8 * sms ? kRerouteThreads / 2 : kRerouteThreads);
     const size_t smem_count = static_cast<size_t>(pad4(L)) * (by_four ? 4 : 1), smem = dense_smem_bytes(L, chunk, threads);
     // Both kernels are dependents of whatever is in front of them, as internal.h says; several ranks not beside a weight_sync, whose set-up
     // the early CTAs disturb (step of 8192 bool rows of 128 experts with bf16 experts of 9 MB 59.5 us, first kernel, second and both
