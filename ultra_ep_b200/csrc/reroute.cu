@@ -1367,7 +1367,11 @@ static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L,
     const int staged = sparse_smem_bytes(L, true) <= kMaxCtaSmem ? 1 : 0;
     const size_t smem = sparse_smem_bytes(L, staged != 0);
     const OrdGrid g = ord_grid(max_n, L, b.n, in_place, kOrdThreads, false);
-    const bool prologue = dependent && g.table && b.n == 1;  // as in launch_dense_forward
+    // The second kernel has its ids, its plan rows and its positions inside the warps while the first one counts: single CTAs, of
+    // which few fill the device. Plan and reroute of eight ranks, second kernel behind the first and beside it (us): 2100 int64 tokens, top 8 of 64
+    // 17.8 and 16.5, 4096 int32 of 64 17.9 and 16.8, 5000 top 6 of 128 18.5 and 17.4, 8192 of 128 22.9 and 22.1, of 256 25.3 and 24.4; with a
+    // weight_sync of 25 MB 6000 of 256 32.8 and 31.2.
+    const bool prologue = dependent && g.table;
     if (g.table) {
         cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(sparse_count_kernel<IdT>), sizeof(int32_t) * L);
         if (e != cudaSuccess) return e;
