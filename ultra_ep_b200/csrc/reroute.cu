@@ -7,7 +7,7 @@
 // outputs twice (zero-fill, then scatter): csrc/kernels/reroute.cu:21-51, 138-264 and
 // csrc/ultra_ep.cpp:891-892 of the reference. Here:
 //   * sparse: one launch (ordinals.cuh); a cluster of CTAs keeps its entries in registers and
-//     counts again what lies in front of it. In place, with several ranks or with very many
+//     counts again what lies in front of it, where there is more than one. In place, with several ranks or with very many
 //     entries a count kernel goes in front;
 //   * dense: pass 1 counts per (tile, expert) from coalesced row reads; pass 2 turns the counts of
 //     the preceding tiles into a base per expert, holds the tile as bit columns, turns logical
@@ -1259,12 +1259,17 @@ struct OrdGrid {
 // `totals`: the grand totals are wanted too (the positions). Every CTA of a cluster then reads every other one's totals: with
 // many buckets a thread takes four entries before the cluster grows (4096 entries, 320 and 1024 buckets: 10.2 and 12.3 us,
 // on eight CTAs 12.3 and 19.7).
-OrdGrid ord_grid(int64_t n, int buckets, int ranks, bool in_place, int threads, bool totals) {
+// one_cluster: up to eight entries a thread in one cluster (launch_sparse_typed).
+OrdGrid ord_grid(int64_t n, int buckets, int ranks, bool in_place, int threads, bool totals, bool one_cluster = false) {
     OrdGrid g{threads, 1, 1, 1, false};
     const int64_t grow = static_cast<int64_t>(threads) * (totals && buckets > 256 ? 4 : 1);
     while (g.ctas < kOrdMaxCluster && n > g.ctas * grow) g.ctas *= 2;
     int64_t row = static_cast<int64_t>(g.ctas) * threads;  // one entry per thread of a cluster
     if (n <= row) return g;
+    if (one_cluster && n > 4 * row && n <= 8 * row) {
+        g.per_lane = 8;
+        return g;
+    }
     g.per_lane = 4;
     g.table = n > 4 * row && (in_place || ranks > 1 || n > kOrdRecountMax);
     if (g.table && totals) {
@@ -1315,11 +1320,12 @@ template <typename Launch>
 cudaError_t with_lanes(const OrdGrid& g, Launch launch) {
     if (g.per_lane == 1) return launch(std::integral_constant<int, 1>{});
     if (g.per_lane == 4) return launch(std::integral_constant<int, 4>{});
+    if (g.per_lane == 8) return launch(std::integral_constant<int, 8>{});
     return launch(std::integral_constant<int, 16>{});
 }
 
-// Several ranks in one launch, n entries of the longest (up to one cluster's the other kernel is one launch): does the walk
-// pay? Beside weight_sync while the walk's sums over the earlier tiles stay short, n / 2048 * L up to 4096 (whole step, walk
+// Several ranks in one launch, n entries of the longest (up to one cluster's the other kernel is one launch, and up to two beside a
+// weight_sync that is not long): does the walk pay? Beside weight_sync while the walk's sums over the earlier tiles stay short, n / 2048 * L up to 4096 (whole step, walk
 // and table: 128 experts, 65536 entries 72.5 and 75.2, 131072 80 and 74; 256 experts, 32768 entries 76.7 and 78.7, 65536 int64
 // 84.9 and 81.3; 64 experts, 131072 entries 57.8 and 60.1). Alone from 65536 entries on, where the launch fills the device
 // either way (131072 entries of 128 experts 27.6 and 31.7; 32768 entries 18 and 14.3). Behind kOrdRecountMax always
@@ -1336,6 +1342,16 @@ bool walk_pays(int64_t n, int L, bool beside_sync) {
 // tokens 54.3 and 54.9; 64 of 44 MB, 16384 of 256 104.0 and 107.4.
 constexpr int64_t kShortSyncBytes = 64ll << 20;
 
+// Several ranks of up to 32768 entries beside a weight_sync of at most so many bytes: one cluster a rank with up to eight entries a
+// thread, one launch where the walk is two, each of which starts on a tick of 2 us. Step of eight ranks, walk and one cluster (us): 2100
+// tokens of 64 experts with 25 MB 23.9 and 22.6, 4096 int64 of 64 with 38 MB 27.6 and 25.9, 4000 of 256 with 71 MB 36.7 and 30.6, 4096 of 64
+// with 201 MB of bf16 31.0 and 27.1, 2500 int64 of 128 with 151 MB 36.5 and 30.9. Above the line the reroute is over before the
+// weight_sync, whose set-up the cluster's burst of loads disturbs: 302 MB in 64 slots 36.2 and 31.0, in 32 42.5 and 41.0, in 16 51.6 and
+// 52.0, 604 MB 50.8 and 51.2, 2.4 GB 80.5 and 81.3. With sixteen entries a thread longer inputs lose too: 5000 of 128 with 151 MB 35.1 and
+// 36.0, 8000 of 128 with 25 MB 30.9 and 34.4. Alone the pair with its counts is the better one, 16.9 and 18.9.
+constexpr int64_t kOneClusterSyncBytes = 256ll << 20;
+constexpr int64_t kOneClusterEntries = 8LL * kOrdMaxCluster * kOrdThreads;
+
 template <typename IdT>
 static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L, int D, int interleave, int64_t beside_bytes,
                                        cudaStream_t stream) {
@@ -1351,7 +1367,8 @@ static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L,
         in_place = in_place || (n > 0 && x < y + bytes && y < x + bytes);
     }
     if (max_n == 0) return cudaSuccess;
-    if (b.n > 1 && walk_pays(max_n, L, beside_sync) && walk_smem_bytes(L) <= kMaxCtaSmem) {
+    const bool one_cluster = b.n > 1 && beside_sync && beside_bytes <= kOneClusterSyncBytes && max_n <= kOneClusterEntries;
+    if (b.n > 1 && !one_cluster && walk_pays(max_n, L, beside_sync) && walk_smem_bytes(L) <= kMaxCtaSmem) {
         const dim3 grid(static_cast<unsigned>(sparse_tiles(max_n)), b.n);
         cudaError_t e = ensure_smem_attr(reinterpret_cast<const void*>(sparse_walk_count_kernel<IdT>), sizeof(int32_t) * L);
         if (e != cudaSuccess) return e;
@@ -1366,7 +1383,7 @@ static cudaError_t launch_sparse_typed(const Batch<SparseArgs>& b, int K, int L,
     }
     const int staged = sparse_smem_bytes(L, true) <= kMaxCtaSmem ? 1 : 0;
     const size_t smem = sparse_smem_bytes(L, staged != 0);
-    const OrdGrid g = ord_grid(max_n, L, b.n, in_place, kOrdThreads, false);
+    const OrdGrid g = ord_grid(max_n, L, b.n, in_place, kOrdThreads, false, one_cluster);
     // The second kernel has its ids, its plan rows and its positions inside the warps while the first one counts: single CTAs, of
     // which few fill the device. Plan and reroute of eight ranks, second kernel behind the first and beside it (us): 2100 int64 tokens, top 8 of 64
     // 17.8 and 16.5, 4096 int32 of 64 17.9 and 16.8, 5000 top 6 of 128 18.5 and 17.4, 8192 of 128 22.9 and 22.1, of 256 25.3 and 24.4; with a
