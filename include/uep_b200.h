@@ -303,8 +303,15 @@ int uep_clear_status(uep_manager* m);
  * hook off. No device fault is involved. No counterpart in the reference (its waits are
  * unbounded, csrc/kernels/weight_sync.cu:666-677, csrc/kernels/ptx.cuh:73-86). While the hook is on
  * (with any rank, one outside the group too), hosted ranks treat each other as ranks of other devices do:
- * completion flags are written and waited for, and a replica's gradient is cleared by its owner. */
+ * completion flags are written and waited for, a replica's gradient is cleared by its owner, and load rows go through memory. */
 int uep_debug_withhold_rank(uep_manager* m, int rank);
+
+/* The same hook for the exchange of a group that is hosted whole, whose ranks hand their load rows over inside a cluster: from the next
+ * plan on, rank `rank` hands its row to nobody, and the others report UEP_DEV_TIMEOUT_GATHER with its number; -1 switches it off. */
+int uep_debug_withhold_row(uep_manager* m, int rank);
+/* The form of the next plan (tests assert which one they run): 1 if the ranks hand their rows over inside a cluster, 0 if through
+ * memory; negative: UEP_ERR_*. */
+int uep_debug_plan_form(uep_manager* m);
 
 /* Tuning aid: with UEP_SYNC_TRACE=1 in the environment when the manager is created, the
  * weight_sync kernel records eight %globaltimer stamps per CTA (start, set-up done, copies

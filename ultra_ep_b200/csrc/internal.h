@@ -80,9 +80,13 @@ struct PlanCall {
     int32_t* rehearsal_out;  // [hosted ranks][kRehearsalOut]
     int in_cluster;          // 1: the ranks hand each other their rows through the shared memory of their cluster (set by launch_plan)
     int withhold_rank;  // test hook: this rank does not publish its flags (-1: none)
+    int withhold_row;   // test hook: in a cluster, this rank does not hand over its row (-1: none)
     int legacy;         // 1: legacy placement solver (counts only; the reroute is then round-robin)
     unsigned long long* trace;  // optional: 8 globaltimer stamps per hosted rank (tuning aid), or null
 };
+// Whether the ranks hand their rows over inside a cluster: a group hosted whole. With the hook that withholds a rank they do it through
+// memory, like ranks of several devices.
+inline bool plan_in_cluster(int nlocal, int N, int withhold_rank) { return nlocal == N && withhold_rank < 0; }
 cudaError_t launch_plan(const PlanCall& call, cudaStream_t stream);
 cudaError_t plan_most_ctas(int nlocal, int N, int G, int M, int R, int* ctas);
 int plan_ctas_per_rank(int input_kind, int max_T, int K_or_L, int cap);

@@ -341,7 +341,7 @@ template <bool kLegacy>
 __device__ __forceinline__ bool gather_loads(const PlanCall& call, const Crew& crew, int local, int part, char* smem_raw, SolveArgs& a) {
     __shared__ int s_timeout_peer;
     __shared__ uint64_t s_epoch;
-    __shared__ __align__(8) uint64_t s_rows;  // the other ranks' rows, where they are pushed
+    __shared__ __align__(8) uint64_t s_rows[kMaxLocalRanks];  // a barrier for each other rank's row, where they are pushed
     const GroupDev& group = call.group;
     uint64_t* const hist_parts = call.hist_parts[local];
     const int N = call.N, M = call.M;
@@ -365,13 +365,11 @@ __device__ __forceinline__ bool gather_loads(const PlanCall& call, const Crew& c
     int32_t* matrix = reinterpret_cast<int32_t*>(smem_raw + solver_smem_bytes(L, N, call.R));
     for (int i = tid; i < L; i += crew.threads) hist[i] = 0;
     const bool owner = part == 0, pushes = call.in_cluster != 0;
-    if (tid == 0) {
-        s_timeout_peer = -1;
-        if (owner && pushes) {
-            mbar_init(&s_rows, 1);
-            fence_mbar_init();
-            mbar_expect_tx(&s_rows, static_cast<uint32_t>((N - 1) * L * sizeof(int32_t)));
-        }
+    if (tid == 0) s_timeout_peer = -1;
+    if (owner && pushes && tid < N && tid != local) {
+        mbar_init(&s_rows[tid], 1);
+        fence_mbar_init();
+        mbar_expect_tx(&s_rows[tid], static_cast<uint32_t>(L * sizeof(int32_t)));
     }
     if (owner && pushes) cluster_arrive();  // (the owners are a cluster of their own)
     pdl_wait();  // ahead of every read: what is in front may still be writing the input
@@ -464,7 +462,7 @@ __device__ __forceinline__ bool gather_loads(const PlanCall& call, const Crew& c
     const SolverSmem solver_sm = carve_solver_smem(smem_raw, L, N, call.R);
     if (pushes) {
         // 2, 3. The ranks of one cluster write their rows straight into each other's matrix, a warp per rank; the bytes are counted
-        //    where they land. (Words through memory, as below, take a store, a look and their two ways through L2: 1.5 us more.)
+        //    where they land, row by row, so that a rank whose row does not come can be named. (Words through memory, as below, take a store, a look and their two ways through L2: 1.5 us more.)
         const int warp = tid >> 5, lane = tid & 31, warps = crew.threads / kWarp;
         const bool vec = (L & 3) == 0;
         int32_t* row = matrix + me * L;
@@ -473,7 +471,8 @@ __device__ __forceinline__ bool gather_loads(const PlanCall& call, const Crew& c
                 for (int i = lane; i < L; i += kWarp) row[i] = hist[i];
                 continue;
             }
-            const uint32_t to = cluster_addr(row, p), bar = cluster_addr(&s_rows, p);
+            if (me == call.withhold_row) continue;
+            const uint32_t to = cluster_addr(row, p), bar = cluster_addr(&s_rows[local], p);
             if (vec) {
                 for (int i = lane * 4; i < L; i += kWarp * 4) push_v4(to + i * 4, *reinterpret_cast<const int4*>(hist + i), bar);
             } else {
@@ -482,7 +481,7 @@ __device__ __forceinline__ bool gather_loads(const PlanCall& call, const Crew& c
         }
         crew.sync();  // hist has been read by every thread, this rank's own row is there
         stamp(1);
-        if (!mbar_wait(&s_rows, 0, call.timeout_ns)) atomicMax(&s_timeout_peer, me);
+        if (tid < N && tid != local && !mbar_wait(&s_rows[tid], 0, call.timeout_ns)) atomicMax(&s_timeout_peer, group.my_rank[tid]);
         crew.sync();
         if (s_timeout_peer >= 0) {
             if (tid == 0) report_error(group.status[local], UEP_DEV_TIMEOUT_GATHER, s_timeout_peer);
@@ -674,7 +673,7 @@ cudaError_t launch_plan(const PlanCall& call, cudaStream_t stream) {
     const bool rehearses = call.N > 1 && call.R > 0 && !call.legacy;
     PlanCall copy = call;
     copy.rehearsal_smem = static_cast<int>(plan_smem_bytes(call.N, call.G, call.M, call.R));
-    copy.in_cluster = call.nlocal == call.N && call.withhold_rank < 0 ? 1 : 0;
+    copy.in_cluster = plan_in_cluster(call.nlocal, call.N, call.withhold_rank) ? 1 : 0;
     const size_t smem = copy.rehearsal_smem + (rehearses ? rehearsal_smem_bytes() : 0);
     const void* kernel = plan_kernel_of(call.legacy != 0, call.threads);
     cudaError_t e = allow_smem(kernel, smem);
