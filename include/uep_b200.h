@@ -309,6 +309,9 @@ int uep_debug_withhold_rank(uep_manager* m, int rank);
 /* The same hook for the exchange of a group that is hosted whole, whose ranks hand their load rows over inside a cluster: from the next
  * plan on, rank `rank` hands its row to nobody, and the others report UEP_DEV_TIMEOUT_GATHER with its number; -1 switches it off. */
 int uep_debug_withhold_row(uep_manager* m, int rank);
+/* Test hook: the small problem that the plan kernel solves beside the real one, to have the solver's code at hand, becomes one that no
+ * build of the fast path solves (1), or of loads of 2^24 and more (2); 0 as usual. The plan is the same. */
+int uep_debug_hard_rehearsal(uep_manager* m, int kind);
 /* The form of the next plan (tests assert which one they run): 1 if the ranks hand their rows over inside a cluster, 0 if through
  * memory; negative: UEP_ERR_*. */
 int uep_debug_plan_form(uep_manager* m);

@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from oracle import uep_oracle as O
-from ultra_ep_b200 import sim
+from ultra_ep_b200 import capi, sim
 
 pytestmark = pytest.mark.gpu
 
@@ -33,4 +33,25 @@ def test_large_maps(native_lib, cuda_device, N, M, R, T):
             for f in ("p2l", "l2p", "lcnts", "quota", "quota_prefix", "rank_quota_prefix"):
                 assert np.array_equal(got[f].cpu().numpy().reshape(-1), getattr(want, f).reshape(-1)), (seed, r, f)
     group.check_status()
+    group.destroy()
+
+
+@pytest.mark.parametrize("kind", [1, 2])
+@pytest.mark.parametrize("N,M,R,T,K", [(2, 3, 1, 50, 2), (3, 5, 2, 4000, 4), (8, 16, 4, 8192, 8), (8, 64, 8, 33, 8), (8, 2, 1, 9000, 4)])
+def test_rehearsal_of_what_is_out_of_line(native_lib, cuda_device, kind, N, M, R, T, K):
+    """A rehearsal that comes to the probes or to wide keys, whose code takes the shared memory of the plan beside it, leaves that alone."""
+    L = N * M
+    group = sim.SimGroup(sim.make_config(N, M, R, 1, is_train=True, sim=True))
+    capi.check(group.lib.uep_debug_hard_rehearsal(group.handle, kind))
+    for seed in range(4):
+        rng = np.random.default_rng(seed)
+        ids = [np.minimum(rng.geometric(0.15, size=(T, K)) - 1, L - 1).astype(np.int32) for _ in range(N)]
+        group.update_placement(0, [torch.from_numpy(x).to(cuda_device) for x in ids])
+        torch.cuda.synchronize()
+        group.check_status()
+        loads = np.stack([np.bincount(x.reshape(-1), minlength=L) for x in ids]).astype(np.int32)
+        for r in range(N):
+            want, got = O.solve_placement(loads, M, R, N, r), group.plan(r, 0)
+            for f in ("p2l", "l2p", "lcnts", "quota", "quota_prefix", "rank_quota_prefix"):
+                assert np.array_equal(got[f].cpu().numpy().reshape(-1), getattr(want, f).reshape(-1)), (seed, r, f)
     group.destroy()

@@ -110,6 +110,7 @@ SIGNATURES = {
     "uep_clear_status": (_i, [_vp]),
     "uep_debug_withhold_rank": (_i, [_vp, _i]),
     "uep_debug_withhold_row": (_i, [_vp, _i]),
+    "uep_debug_hard_rehearsal": (_i, [_vp, _i]),
     "uep_debug_plan_form": (_i, [_vp]),
     "uep_debug_sync_trace": (_i, [_vp, _vp, _i]),
     "uep_launch_count": (_i64, []),

@@ -81,6 +81,7 @@ struct PlanCall {
     int in_cluster;          // 1: the ranks hand each other their rows through the shared memory of their cluster (set by launch_plan)
     int withhold_rank;  // test hook: this rank does not publish its flags (-1: none)
     int withhold_row;   // test hook: in a cluster, this rank does not hand over its row (-1: none)
+    int hard_rehearsal; // test hook: the rehearsal comes to the probes (1) or the wide keys (2)
     int legacy;         // 1: legacy placement solver (counts only; the reroute is then round-robin)
     unsigned long long* trace;  // optional: 8 globaltimer stamps per hosted rank (tuning aid), or null
 };

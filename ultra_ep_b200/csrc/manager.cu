@@ -153,7 +153,7 @@ struct uep_manager {
     int grad_reduce_ctas = 42;
     int weight_sync_ctas = 0;
     int plan_ctas = 1;  // most CTAs of a rank in the plan kernel
-    int withhold_rank = -1, withhold_row = -1;
+    int withhold_rank = -1, withhold_row = -1, hard_rehearsal = 0;
     int relay_cap = 0;  // ready-flag words per replica slot
     int32_t* rehearsal_out = nullptr;  // written by the plans' rehearsals, read by nobody
     unsigned long long* sync_trace = nullptr;  // UEP_SYNC_TRACE=1: per-CTA phase stamps of the last weight_sync
@@ -651,6 +651,7 @@ int uep_update_placement(uep_manager* m, int layer_id, int input_kind, const voi
     call.threads = plan_threads(input_kind, max_T, K_or_L, call.ctas_per_rank);
     call.withhold_rank = m->withhold_rank;
     call.withhold_row = m->withhold_row;
+    call.hard_rehearsal = m->hard_rehearsal;
     call.legacy = m->cfg.legacy_placement ? 1 : 0;
     call.rehearsal_out = m->rehearsal_out;
     call.trace = m->sync_trace ? m->sync_trace + 8 * 1000 : nullptr;  // the last rows of the trace buffer
@@ -902,6 +903,12 @@ int uep_debug_withhold_rank(uep_manager* m, int rank) {
 int uep_debug_withhold_row(uep_manager* m, int rank) {
     if (m == nullptr) return fail(UEP_ERR_INVALID, "debug_withhold_row: null manager");
     m->withhold_row = rank;
+    return UEP_OK;
+}
+
+int uep_debug_hard_rehearsal(uep_manager* m, int kind) {
+    if (m == nullptr || kind < 0 || kind > 2) return fail(UEP_ERR_INVALID, "debug_hard_rehearsal: bad argument");
+    m->hard_rehearsal = kind;
     return UEP_OK;
 }
 

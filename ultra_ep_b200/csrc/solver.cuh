@@ -28,9 +28,13 @@
 namespace uep {
 
 // The threads of a CTA that solve a problem together: their number among them, how many, and their barrier (0 to 15). A CTA can hold
-// two of them.
+// two of them; the second one has its shared memory behind the first one's, and what is out of line (below) takes the first one's, so
+// it is closed to the second. (With the place as an argument it was open, and the plan's registers spilled: step of eight ranks of 8192
+// bool rows of 128 with bf16 experts of 9 MB 57.7 us like this and 59.5.)
+constexpr int kSecondCrewBarrier = 2;
 struct Crew {
     int tid, threads, barrier;
+    __device__ __forceinline__ bool second() const { return barrier == kSecondCrewBarrier; }
     __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(barrier), "r"(threads) : "memory"); }
 };
 
@@ -270,7 +274,7 @@ constexpr int kMostKeys = (kMaxRanksPerDomain + kWarp - 1) / kWarp;
 
 // By one warp, into plan buffer `buffer`. `total`, `largest`: of the ranks' loads. kProbe: a static floor, and nobody stops it.
 template <bool kProbe>
-__device__ __forceinline__ bool warp_build_plan(const SolverSmem& sm, int buffer, int& num_batches, int thr, int total, int largest, int G, int M, int R,
+__device__ __forceinline__ bool warp_build_plan(const Crew& crew, const SolverSmem& sm, int buffer, int& num_batches, int thr, int total, int largest, int G, int M, int R,
                                                 int min_tokens, bool allow_zero_master, bool dynamic_floor, int lane, const volatile int* stop) {
     num_batches = 0;
     if (largest <= thr) return true;
@@ -281,6 +285,7 @@ __device__ __forceinline__ bool warp_build_plan(const SolverSmem& sm, int buffer
     if (narrow && G <= kWarp) {
         return drain_sources<1, false, kProbe>(sm, buffer, num_batches, thr, G, M, R, min_tokens, allow_zero_master, dynamic_floor, lane, stop);
     }
+    if (crew.second()) return false;
     if (!narrow) return drain_sources_apart<kMostKeys, true, kProbe>(buffer, num_batches, thr, G, M, R, min_tokens, allow_zero_master, dynamic_floor, lane, stop);
     if (G <= 2 * kWarp) return drain_sources_apart<2, false, kProbe>(buffer, num_batches, thr, G, M, R, min_tokens, allow_zero_master, dynamic_floor, lane, stop);
     return drain_sources_apart<kMostKeys, false, kProbe>(buffer, num_batches, thr, G, M, R, min_tokens, allow_zero_master, dynamic_floor, lane, stop);
@@ -321,7 +326,7 @@ __device__ __noinline__ int2 probe_thresholds(Crew crew, int fitting, int hi0, i
         if (warp < kSolverProbeWarps) {
             int n = 0;
             const bool ok = (!each || warp < range) &&
-                            warp_build_plan<true>(sm, set + warp, n, probe(warp), total, largest, G, M, R, min_tokens, allow_zero_master, false, lane, nullptr);
+                            warp_build_plan<true>(crew, sm, set + warp, n, probe(warp), total, largest, G, M, R, min_tokens, allow_zero_master, false, lane, nullptr);
             if (lane == 0) sm.ctrl[kCtlBuilt0 + set + warp] = ok ? n + 1 : 0;
         }
         crew.sync();
@@ -541,8 +546,8 @@ __device__ __forceinline__ void warp_rank_quota_prefix(const SolveArgs& a, int l
 }
 
 // Solve one NVLink domain. All threads of the crew must call it (128 at least,
-// multiple of 32). smem_raw must hold solver_smem_bytes(E, G, R) bytes, 16-byte aligned; more than 32 ranks, loads from 2^24 on and
-// probes take the CTA's dynamic shared memory for it.
+// multiple of 32). smem_raw must hold solver_smem_bytes(E, G, R) bytes, 16-byte aligned; of a first crew it is the start of the CTA's dynamic
+// shared memory. A second crew leaves a problem as it is that needs more than 32 ranks, loads from 2^24 on or probes.
 __device__ __forceinline__ void solve_domain(const SolveArgs& a, const Crew& crew, int domain, char* smem_raw, DeviceStatus* status) {
     const int tid = crew.tid, nthreads = crew.threads;
     const int warp = tid >> 5, lane = tid & 31;
@@ -679,13 +684,14 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, const Crew& cre
                 }
             }
             int n = 0;
-            const bool ok = warp_build_plan<false>(sm, warp, n, thr, total, largest, G, M, R, a.min_tokens, allow0, fast, lane, sm.ctrl + kCtlStop0 + warp);
+            const bool ok = warp_build_plan<false>(crew, sm, warp, n, thr, total, largest, G, M, R, a.min_tokens, allow0, fast, lane, sm.ctrl + kCtlStop0 + warp);
             if (lane == 0) sm.ctrl[kCtlBuilt0 + warp] = ok ? n + 1 : 0;
             if (ok && lane > warp && lane < kSolverProbeWarps) *(sm.ctrl + kCtlStop0 + lane) = 1;
         }
         crew.sync();
         winner = first_feasible(sm, 0, num_batches);
         if (__builtin_expect(winner < 0, 0)) {
+            if (crew.second()) return;
             const int2 found = probe_thresholds(crew, sm.ctrl[kCtlFitting], sm.ctrl[kCtlHi], sm.ctrl[kCtlTotal], sm.ctrl[kCtlLargest], G, M, R, a.min_tokens, allow0);
             winner = found.x;
             num_batches = found.y;
