@@ -312,8 +312,8 @@ int uep_debug_withhold_row(uep_manager* m, int rank);
 /* Test hook: the small problem that the plan kernel solves beside the real one, to have the solver's code at hand, becomes one that no
  * build of the fast path solves (1), or of loads of 2^24 and more (2); 0 as usual. The plan is the same. */
 int uep_debug_hard_rehearsal(uep_manager* m, int kind);
-/* The form of the next plan (tests assert which one they run): 1 if the ranks hand their rows over inside a cluster, 0 if through
- * memory; negative: UEP_ERR_*. */
+/* The form of the next plan (tests assert which one they run): 1 if the ranks hand their rows over inside a cluster and not through
+ * memory, plus 2 if the solver is rehearsed beside it; negative: UEP_ERR_*. */
 int uep_debug_plan_form(uep_manager* m);
 
 /* Tuning aid: with UEP_SYNC_TRACE=1 in the environment when the manager is created, the

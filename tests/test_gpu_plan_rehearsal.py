@@ -2,6 +2,8 @@
 and a CTA that rehearses the solver on a problem of its own beside them. The widths of the map decide how the lanes share the sums; the
 smallest group is smaller than the rehearsal's. Loads and plan against the CPU oracle, bit-exact, twice in a row."""
 
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -34,6 +36,21 @@ def test_large_maps(native_lib, cuda_device, N, M, R, T):
                 assert np.array_equal(got[f].cpu().numpy().reshape(-1), getattr(want, f).reshape(-1)), (seed, r, f)
     group.check_status()
     group.destroy()
+
+
+def test_who_rehearses(native_lib, cuda_device):
+    """A group that is hosted whole and has something to solve by quotas; not one rank among ranks on other devices."""
+    def form(N, R, hosted, legacy=0):
+        cfg = sim.make_config(N, 4, R, 1, is_train=True, sim=hosted)
+        cfg.legacy_placement = legacy
+        handle = C.c_void_p()
+        capi.check(capi.lib().uep_manager_create(C.byref(cfg), C.byref(handle)))
+        got = capi.lib().uep_debug_plan_form(handle)
+        capi.check(capi.lib().uep_manager_destroy(handle))
+        return got
+
+    assert [form(2, 1, True), form(8, 2, True), form(8, 0, True), form(1, 2, True), form(8, 2, True, legacy=1)] == [3, 3, 1, 1, 1]
+    assert [form(2, 1, False), form(8, 2, False), form(1, 2, False)] == [0, 0, 1]
 
 
 @pytest.mark.parametrize("kind", [1, 2])

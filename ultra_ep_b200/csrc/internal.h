@@ -88,6 +88,9 @@ struct PlanCall {
 // Whether the ranks hand their rows over inside a cluster: a group hosted whole. With the hook that withholds a rank they do it through
 // memory, like ranks of several devices.
 inline bool plan_in_cluster(int nlocal, int N, int withhold_rank) { return nlocal == N && withhold_rank < 0; }
+// Whether the owners' CTAs rehearse the solver: a group hosted whole. Of one rank among ranks on other devices it is not measured, and its
+// CTAs keep their size.
+inline bool plan_rehearses(int nlocal, int N, int R, bool legacy) { return nlocal == N && N > 1 && R > 0 && !legacy; }
 cudaError_t launch_plan(const PlanCall& call, cudaStream_t stream);
 cudaError_t plan_most_ctas(int nlocal, int N, int G, int M, int R, int* ctas);
 int plan_ctas_per_rank(int input_kind, int max_T, int K_or_L, int cap);

@@ -914,7 +914,7 @@ int uep_debug_hard_rehearsal(uep_manager* m, int kind) {
 
 int uep_debug_plan_form(uep_manager* m) {
     if (m == nullptr) return fail(UEP_ERR_INVALID, "debug_plan_form: null manager");
-    return plan_in_cluster(m->nlocal, m->N, m->withhold_rank) ? 1 : 0;
+    return (plan_in_cluster(m->nlocal, m->N, m->withhold_rank) ? 1 : 0) | (plan_rehearses(m->nlocal, m->N, m->R, m->cfg.legacy_placement != 0) ? 2 : 0);
 }
 
 int uep_clear_status(uep_manager* m) {

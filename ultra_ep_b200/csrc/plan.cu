@@ -673,7 +673,7 @@ cudaError_t plan_most_ctas(int nlocal, int N, int G, int M, int R, int* ctas) {
 }
 
 cudaError_t launch_plan(const PlanCall& call, cudaStream_t stream) {
-    const bool rehearses = call.N > 1 && call.R > 0 && !call.legacy;
+    const bool rehearses = plan_rehearses(call.nlocal, call.N, call.R, call.legacy != 0);
     PlanCall copy = call;
     copy.rehearsal_smem = static_cast<int>(plan_smem_bytes(call.N, call.G, call.M, call.R));
     copy.in_cluster = plan_in_cluster(call.nlocal, call.N, call.withhold_rank) ? 1 : 0;
