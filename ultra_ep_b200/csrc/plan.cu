@@ -610,7 +610,8 @@ void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 // Twice the threads where a CTA's slice of the input is long enough to pay for the larger block. Step of eight ranks with 256 threads and
 // 512 (us), below the line: 2200 bool rows of 128 experts (18.3 KB a CTA) 36.5 and 38.2, 2600 (21.7 KB) 35.3 and 36.4, 8192 int32 tokens of 128
 // (17 KB) 52.5 and 52.7, 9600 (20 KB) 39.65 and 39.6, 4800 int64 tokens of 64 (20 KB) 27.9 and 28.1; above it 11000 int32 tokens (23 KB) 40.75
-// and 40.3, 2600 bool rows of 256 (43 KB) 53.4 and 51.8, 16384 int64 tokens of 256 (68 KB) 106.8 and 104.5.
+// and 40.3, 2600 bool rows of 256 (43 KB) 53.4 and 51.8, 16384 int64 tokens of 256 (68 KB) 106.8 and 104.5. Legacy plans the same: with the
+// dense reroute 8192 rows of 256 191.4 and 188.5, of 512 180.5 and 175.6; one rank's plan of 8192 x 256 9.5 and 8.1, of 16384 x 64 6.3 and 6.7.
 constexpr int kFewThreadsBytes = 22 * 1024;
 int plan_threads(int input_kind, int max_T, int K_or_L, int ctas) {
     const int64_t bytes = static_cast<int64_t>(max_T) * K_or_L * (input_kind == 0 ? 1 : (input_kind == 1 ? 4 : 8));
@@ -626,9 +627,10 @@ int plan_ctas_per_rank(int input_kind, int max_T, int K_or_L, int cap) {
 namespace {
 
 const void* plan_kernel_of(bool legacy, int threads) {
-    if (legacy) return reinterpret_cast<const void*>(plan_kernel<kPlanThreads, true>);
-    return threads == kPlanThreads ? reinterpret_cast<const void*>(plan_kernel<kPlanThreads, false>)
-                                   : reinterpret_cast<const void*>(plan_kernel<2 * kPlanThreads, false>);
+    if (threads == kPlanThreads) {
+        return legacy ? reinterpret_cast<const void*>(plan_kernel<kPlanThreads, true>) : reinterpret_cast<const void*>(plan_kernel<kPlanThreads, false>);
+    }
+    return legacy ? reinterpret_cast<const void*>(plan_kernel<2 * kPlanThreads, true>) : reinterpret_cast<const void*>(plan_kernel<2 * kPlanThreads, false>);
 }
 
 cudaLaunchAttribute dependent_launch() {
@@ -684,7 +686,7 @@ cudaError_t launch_plan(const PlanCall& call, cudaStream_t stream) {
     cudaLaunchAttribute attr[2];
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(call.nlocal * call.ctas_per_rank);
-    cfg.blockDim = dim3((call.legacy ? kPlanThreads : call.threads) + (rehearses ? kRehearsalThreads : 0));
+    cfg.blockDim = dim3(call.threads + (rehearses ? kRehearsalThreads : 0));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = attr;
