@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(SolveArgs a, in
         a.preloaded = 1;
         a.staged_loads = staged ? matrix : nullptr;
     }
-    if (kLegacy) legacy_solve_domain(a, domain, smem_raw, status);
+    if (kLegacy) legacy_solve(a, domain, smem_raw, status);
     else solve_domain(a, Crew{static_cast<int>(threadIdx.x), static_cast<int>(blockDim.x), 0}, domain, smem_raw, status);
 }
 
@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(kThreads + kRehearsalThreads, 1) plan_kernel(P
         return;
     }
     DeviceStatus* const status = rehearses ? nullptr : call.group.status[local];
-    if (kLegacy) legacy_solve_domain(a, 0, smem, status);
+    if (kLegacy) legacy_solve_apart(a, 0, smem, status);
     else solve_domain(a, crew, 0, smem, status);
     if (!rehearses && call.trace != nullptr && threadIdx.x == 0) call.trace[local * 8 + 4] = global_timer_ns();
 }
