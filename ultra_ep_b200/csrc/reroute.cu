@@ -1176,9 +1176,13 @@ cudaError_t launch_dense_forward(const Batch<DenseFwdArgs>& b, int L, int P, int
     // writes, fill each other's gaps; with 256 the first wave writes when the second one has not begun. Plan and pair of eight ranks, 256 and
     // 128 threads (us): 4800 rows of 128 experts 29.8 and 27.8, 8192 40.1 and 38.0, of 64 experts 28.5 and 25.7, of 256 61.2 and 60.5; beside
     // a weight_sync 8192 x 128 with bf16 experts of 9 MB 58.0 and 56.8, 6500 x 64 with fp8 of 5 MB 41.6 and 39.6. In one wave either way, 4096
-    // x 128 25.3 and 25.9; in two, 12000 x 128 52.7 and 54.1.
+    // x 128 25.3 and 25.9; in two, 12000 x 128 52.7 and 54.1. With more experts the tiles are longer and the last wave of 256 threads is filled
+    // from seven tiles an SM on: pair of eight ranks, 256 and 128 threads, 8169 x 192 (6.9 tiles) 39.8 and 39.1, 8643 x 192 (7.3) 41.2 and 41.4,
+    // 9353 x 256 (7.9) 50.5 and 51.0, quota plans, 51.9 and 52.9, legacy ones. One rank: 73000 x 192 (7.7) 38.2 and 37.2, 44000 x 256 30.5 and
+    // 31.1, 57000 x 256 38.5 and 39.9, 55000 x 512 64.0 and 66.4 (50000 x 256 35.4 and 34.2).
     const int64_t all_tiles = static_cast<int64_t>(grid.x) * b.n;
-    const int threads = all_tiles <= 2 * sms ? kDenseMaxThreads : (all_tiles > 4 * sms && all_tiles <= 8 * sms ? kRerouteThreads / 2 : kRerouteThreads);
+    const int one_wave = L <= 128 ? 8 : (b.n > 1 ? 7 : (L < 256 ? 8 : 0));  // tiles an SM
+    const int threads = all_tiles <= 2 * sms ? kDenseMaxThreads : (all_tiles > 4 * sms && all_tiles <= one_wave * sms ? kRerouteThreads / 2 : kRerouteThreads);
     const size_t smem_count = static_cast<size_t>(pad4(L)) * (by_four ? 4 : 1), smem = dense_smem_bytes(L, chunk, threads);
     // Both kernels are dependents of whatever is in front of them, as internal.h says; several ranks not beside a weight_sync, whose set-up
     // the early CTAs disturb (step of 8192 bool rows of 128 experts with bf16 experts of 9 MB 59.5 us, first kernel, second and both
