@@ -2,12 +2,17 @@
 memory, as ranks of several devices do (which the hook that withholds a rank asks for, also with a rank that does not exist). To a good
 end against the CPU oracle, bit-exact, in turn on one group; and with one rank's row missing, which the others name."""
 
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
 
 from oracle import uep_oracle as O
 from test_gpu_dependents import FIELDS, _group_input
+from test_gpu_reroute_behind_plan import late_write  # noqa: F401  (fixture)
 from test_gpu_sync_repeats import _ids
 from ultra_ep_b200 import capi, sim
 
@@ -121,3 +126,38 @@ def test_weights_behind_tickets_and_flags(native_lib, cuda_device, N, M, R, offs
                 assert torch.equal(replicas[r][s], want), (kind, r, s)
     assert seen > 0
     group.destroy()
+
+
+@pytest.mark.parametrize("N,M,R", [(2, 3, 1), (8, 16, 4)])
+@pytest.mark.parametrize("kind,T", [("int64", 9), ("map", 2600)])
+def test_legacy_plan_behind_an_early_kernel(native_lib, cuda_device, late_write, N, M, R, kind, T):  # noqa: F811
+    """Counts-only plans through the cluster, behind a kernel that starts its dependents early and writes the input later."""
+    cfg = sim.make_config(N, M, R, 1, is_train=True, sim=True)
+    cfg.legacy_placement = 1
+    group = sim.SimGroup(cfg)
+    for seed in range(3):
+        data, shapes, _ = _group_input(kind, N, N * M, T, seed)
+        late, _, loads = _group_input(kind, N, N * M, T, seed + 10)
+        flat, source = torch.from_numpy(data).to(cuda_device), torch.from_numpy(late).to(cuda_device)
+        views, at = [], 0
+        for shape in shapes:
+            views.append(flat[at:at + shape[0] * shape[1]].view(shape))
+            at += shape[0] * shape[1]
+        late_write(flat.view(torch.uint8), source.view(torch.uint8), seed % 2 == 1)
+        group.update_placement(0, views)
+        torch.cuda.synchronize()
+        group.check_status()
+        for r in range(N):
+            _assert_plan(group, 0, O.legacy_solve_placement(loads.sum(0), N, M, R, N, 1.0), r)
+    group.destroy()
+
+
+def test_without_dependent_launches(native_lib, cuda_device):
+    """UEP_DISABLE_PDL=1, which a process reads once: both exchanges, plan and reroute, solves and positions as ordinary launches."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    chosen = ["test_gpu_plan_exchange.py::test_both_forms_in_turn", "test_gpu_reroute_behind_plan.py::test_sparse",
+              "test_gpu_reroute_behind_plan.py::test_dense", "test_gpu_dependents.py::test_solve_behind_an_early_kernel",
+              "test_gpu_dependents.py::test_positions_behind_an_early_kernel"]
+    run = subprocess.run([sys.executable, "-m", "pytest", "-x", "-q", "-m", "gpu", "-p", "no:cacheprovider", *(os.path.join(here, c) for c in chosen)],
+                         env=dict(os.environ, UEP_DISABLE_PDL="1"), capture_output=True, text=True, timeout=600)
+    assert run.returncode == 0 and " passed" in run.stdout and "failed" not in run.stdout, run.stdout[-3000:] + run.stderr[-1000:]

@@ -1,6 +1,7 @@
-"""Plans of hosted groups whose inputs are large: 256 or 512 threads a CTA, bytes of the bool map summed in a warp before they are counted,
-and a CTA that rehearses the solver on a problem of its own beside them. The widths of the map decide how the lanes share the sums; the
-smallest group is smaller than the rehearsal's. Loads and plan against the CPU oracle, bit-exact, twice in a row."""
+"""Plans of hosted groups whose inputs are large: 256 or 512 threads that count, bytes of the bool map summed in a warp before they are
+counted, and a second crew of threads in the owners' CTAs that rehearses the solver on a problem of its own beside them. The widths of the map
+decide how the lanes share the sums; the smallest group is smaller than the rehearsal's. Loads and plan against the CPU oracle,
+bit-exact, twice in a row."""
 
 import ctypes as C
 
@@ -13,8 +14,10 @@ from ultra_ep_b200 import capi, sim
 
 pytestmark = pytest.mark.gpu
 
-# ranks, masters, slots, tokens: more than 16 KB for each CTA that a rank has, but for the first, which has nine CTAs of less
-SHAPES = [(8, 16, 4, 1100), (2, 1, 1, 300000), (2, 8, 1, 40000), (3, 32, 2, 9000), (5, 5, 2, 25000), (7, 16, 0, 5000), (8, 4, 2, 12000), (8, 64, 8, 1500)]
+# ranks, masters, slots, tokens. 512 threads count from 22 KB of input for each CTA that a rank has (two ranks have 32 each, eight 15): the last
+# two are on either side of that line
+SHAPES = [(8, 16, 4, 1100), (2, 1, 1, 300000), (2, 8, 1, 40000), (3, 32, 2, 9000), (5, 5, 2, 25000), (7, 16, 0, 5000), (8, 4, 2, 12000), (8, 64, 8, 1500),
+          (2, 1, 1, 400000), (2, 8, 1, 50000), (8, 16, 4, 9000), (2, 8, 1, 45056), (2, 8, 1, 45057)]
 
 
 @pytest.mark.parametrize("N,M,R,T", SHAPES)
