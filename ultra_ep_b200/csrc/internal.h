@@ -172,7 +172,7 @@ int64_t sparse_scratch_elems(int64_t entries, int L);
 // launch starts on the next tick of some 2 us from the start of the kernel in front, 1.8 us at least behind its end; a dependent one is
 // past its wait 0.8 us behind that end whether or not the kernel in front says when it may start. So no kernel here says it, except to
 // one that has something to do before its wait: CTAs that only wait take the place of others. Plan and reroute of eight ranks among
-// others, ordinary launches of the plan and both that start their dependents early, and like this (us): 33 tokens of 64 experts 13.5 and
+// others, before every launch was a dependent one and right behind that change (us): 33 tokens of 64 experts 13.5 and
 // 11.4, 4096 tokens 25.1 and 16.9, bool rows 4096 of 128 experts 28.6 and 24.3; one rank's sparse, dense and backward, 8191 x 256,
 // 28.5 and 25.4. beside_sync, beside_bytes: several ranks and a weight_sync of the plan was launched, which writes at most so many
 // bytes: where its CTAs' first microseconds count, the reroute's launches are ordinary ones (reroute.cu).

@@ -41,9 +41,9 @@ constexpr size_t kSolveMaxSmem = 220 * 1024;
 // Of the load matrix, where the plan kernel keeps it in shared memory: eight ranks of 512 experts, the largest group that one
 // device can host and the plan kernel could be timed with. The solver's own kernel has its SM to itself and takes what fits.
 constexpr size_t kPlanMatrixBytes = 16 * 1024;
-// Partial counts a thread asks for at once. The CTAs behind a rank's first one are shared by as many threads as an expert
-// can have: 17 of them (eight hosted ranks) by two of 256 threads or four of 512 up to 128 experts, one round each; other numbers
-// take more rounds.
+// Partial counts a thread asks for at once. The CTAs behind a rank's first one are shared by as many threads as an expert can have: 14
+// of them at most (eight hosted ranks) by two of 256 threads or four of 512 up to 128 experts, 31 (one rank) by four of 256 up to 64, one
+// round each; more experts take more rounds.
 constexpr int kPartBatch = 9;
 
 __device__ __forceinline__ void hist_add_swar(uint32_t word, int32_t* hist, int col) {

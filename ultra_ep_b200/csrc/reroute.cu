@@ -1341,18 +1341,16 @@ bool walk_pays(int64_t n, int L, bool beside_sync) {
 
 // Several ranks beside a weight_sync of at most so many bytes: the reroute is then the longer one of the two, and both of its kernels
 // are dependents like elsewhere; beside a longer one their early CTAs disturb its set-up. Step of eight ranks, ordinary launches and
-// dependents (us): fp8 experts in 16 slots of 1.5 MB, 8000 int32 tokens of 128 experts 34.4 and 31.2, 4800 int64 tokens of 64 31.2 and
-// 27.2; 16 slots of 3 MB, 3000 tokens of 64 31.0 and 28.6; above the line 32 slots of 3 MB, 1000 tokens 27.8 and 27.6; 32 of 19 MB, 8192
-// tokens 54.3 and 54.9; 64 of 44 MB, 16384 of 256 104.0 and 107.4.
+// dependents (us): fp8 experts in 16 slots of 3 MB, 3000 tokens of 64 31.0 and 28.6; above the line 32 slots of 19 MB, 8192 tokens 54.3 and
+// 54.9, 64 of 44 MB, 16384 of 256 104.0 and 107.4.
 constexpr int64_t kShortSyncBytes = 64ll << 20;
 
 // Several ranks of up to 32768 entries beside a weight_sync of at most so many bytes: one cluster a rank with up to eight entries a
-// thread, one launch where the walk is two, each of which starts on a tick of 2 us. Step of eight ranks, walk and one cluster (us): 2100
-// tokens of 64 experts with 25 MB 23.9 and 22.6, 4096 int64 of 64 with 38 MB 27.6 and 25.9, 4000 of 256 with 71 MB 36.7 and 30.6, 4096 of 64
-// with 201 MB of bf16 31.0 and 27.1, 2500 int64 of 128 with 151 MB 36.5 and 30.9. Above the line the reroute is over before the
-// weight_sync, whose set-up the cluster's burst of loads disturbs: 302 MB in 64 slots 36.2 and 31.0, in 32 42.5 and 41.0, in 16 51.6 and
-// 52.0, 604 MB 50.8 and 51.2, 2.4 GB 80.5 and 81.3. With sixteen entries a thread longer inputs lose too: 5000 of 128 with 151 MB 35.1 and
-// 36.0, 8000 of 128 with 25 MB 30.9 and 34.4. Alone the pair with its counts is the better one, 16.9 and 18.9.
+// thread, one launch where the walk is two, each of which starts on a tick of 2 us. Step of eight ranks, walk and one cluster (us): 4000
+// tokens of 256 experts with 71 MB 36.7 and 30.6, 4096 of 64 with 201 MB of bf16 31.0 and 27.1. Above the line the reroute is over before the
+// weight_sync, whose set-up the cluster's burst of loads disturbs: 302 MB in 16 slots 51.6 and 52.0, 2.4 GB 80.5 and 81.3. With sixteen
+// entries a thread longer inputs lose too: 8000 of 128 with 25 MB 30.9 and 34.4. Alone the pair with its counts is the better one, 16.9
+// and 18.9.
 constexpr int64_t kOneClusterSyncBytes = 256ll << 20;
 constexpr int64_t kOneClusterEntries = 8LL * kOrdMaxCluster * kOrdThreads;
 

@@ -17,8 +17,8 @@
 //     too where it fits (plan.cu); else the few entries of it that are needed are read through L2.
 // All of it is latency of one CTA: what counts is how many dependent instructions follow one another, how many of them branch, and
 // how much code there is, since each line of it is fetched once a launch. Calls of uep_solve_placement among others on one B200: 64
-// ranks x 4 experts x 2 slots 18.6 us (20.6 with sorted lists of ranks, which one lane walked); plan and reroute of eight ranks, 33
-// tokens of 64 experts each, 13.1 (15.6).
+// ranks x 4 experts x 2 slots 15.5 us; plan and reroute of eight ranks, 33 tokens of 64 experts each, 10.9. (With sorted lists of ranks,
+// which one lane walked, and all else as it then was, 20.6 for 18.6 and 15.6 for 13.1.)
 #pragma once
 
 #include <climits>
@@ -137,11 +137,9 @@ __device__ __forceinline__ int warp_inclusive_scan(int v, int lane, int n) {
 // nature. A lane holds the ranks lane, lane + 32, .. as keys, amount << 7 | 127 - rank, -1 where there is none, so that the next rank is
 // the warp's largest key: one reduction, and its lane notices by itself that it was chosen. All the rest of an export is the same few
 // instructions in every lane, with one branch, and the next source and its master are asked for beside the exports of this one.
-// An export takes some 55 cycles, a source 290 (sorted lists in shared memory, walked by one lane: several loads and selects an
-// export. By group, ranks x experts x slots, calls among others with the lists and like this (us): 16 x 7 x 4 10.4 and 10.2, 32 x 4 x 2
-// 12.5 and 10.6, 48 x 7 x 4 19.2 and 17.0, 72 x 7 x 1 22.7 and 21.8, 72 x 7 x 4 28.1 and 23.9; with rounds of probes, 16 x 2 x 1, 21.3 both. All
-// exports of an expert in one step, by ballots and shuffles: 1000 cycles an expert. The list of up to eight ranks in the registers
-// of one lane, the best one first: builds of a plan of eight ranks 2.7 us, 2.0 like this.)
+// An export takes some 55 cycles, a source 290. (Sorted lists in shared memory, walked by one lane: several loads and selects an
+// export; ranks x experts x slots, calls among others with the lists and when they were replaced by this (us), 72 x 7 x 4 28.1 and 23.9,
+// 32 x 4 x 2 12.5 and 10.6, with rounds of probes, 16 x 2 x 1, 21.3 both.)
 // kKeys: keys a lane. kWide: a key is the amount alone, where amount << 7 does not fit 31 bits, and the rank is a second reduction.
 // kProbe: the floor is static, and nobody stops the build; else `stop` is raised by a warp whose result makes it pointless.
 template <int kKeys, bool kWide, bool kProbe>
@@ -650,9 +648,9 @@ __device__ __forceinline__ void solve_domain(const SolveArgs& a, const Crew& cre
         // smallest threshold the capacities allow; then the probes. The first four run at once, one warp each; one that
         // succeeds stops those behind it.
         // Mostly this code comes from DRAM, a line after the other, and what is jumped over comes too: so what a call seldom needs is
-        // out of line (the probes, keys of 64 bits, more than 32 replicas, the legacy solver), and the outputs are compiled in once.
-        // Plan of eight ranks behind an L2 flush, on the device (us), with all builds and widths inlined and like this: 33 tokens of 64
-        // experts 19.3 and 13.3, 4096 tokens 17.8 and 15.7; among other plans 10.3 and 9.5, 12.8 and 11.8.
+        // out of line (the probes, the wide and the many keys, more than 32 replicas), and the outputs are compiled in once.
+        // Plan of eight ranks behind an L2 flush, on the device (us), with all builds and widths inlined and when that was changed: 33
+        // tokens of 64 experts 19.3 and 13.3, 4096 tokens 17.8 and 15.7; among other plans 10.3 and 9.5, 12.8 and 11.8.
         if (warp < kSolverProbeWarps) {
             int total = 0, largest = 0;
             for (int r = lane; r < G; r += kWarp) {
