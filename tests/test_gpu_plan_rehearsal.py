@@ -9,15 +9,17 @@ import numpy as np
 import pytest
 import torch
 
+import gpu_util as G
 from oracle import uep_oracle as O
 from ultra_ep_b200 import capi, sim
 
 pytestmark = pytest.mark.gpu
 
-# ranks, masters, slots, tokens. 512 threads count from 22 KB of input for each CTA that a rank has (two ranks have 32 each, eight 15): the last
-# two are on either side of that line
+# ranks, masters, slots, tokens. 512 threads count from 22 KB of input for each CTA that a rank has (two ranks have 32 each, eight 15):
+# 45056 and 45057 are on either side of that line. The last ones' rows are no whole vectors, and are counted byte by byte.
 SHAPES = [(8, 16, 4, 1100), (2, 1, 1, 300000), (2, 8, 1, 40000), (3, 32, 2, 9000), (5, 5, 2, 25000), (7, 16, 0, 5000), (8, 4, 2, 12000), (8, 64, 8, 1500),
-          (2, 1, 1, 400000), (2, 8, 1, 50000), (8, 16, 4, 9000), (2, 8, 1, 45056), (2, 8, 1, 45057)]
+          (2, 1, 1, 400000), (2, 8, 1, 50000), (8, 16, 4, 9000), (2, 8, 1, 45056), (2, 8, 1, 45057),
+          (6, 20, 2, 4000), (3, 40, 2, 5561), (7, 10, 2, 1000), (8, 15, 2, 8192), (5, 1, 1, 70000), (2, 255, 1, 3000)]
 
 
 @pytest.mark.parametrize("N,M,R,T", SHAPES)
@@ -75,3 +77,17 @@ def test_rehearsal_of_what_is_out_of_line(native_lib, cuda_device, kind, N, M, R
             for f in ("p2l", "l2p", "lcnts", "quota", "quota_prefix", "rank_quota_prefix"):
                 assert np.array_equal(got[f].cpu().numpy().reshape(-1), getattr(want, f).reshape(-1)), (seed, r, f)
     group.destroy()
+
+
+# around eight rounds of a CTA's threads and the last one's rest, one column to more than threads, rows that begin anywhere in memory
+@pytest.mark.parametrize("T,L", [(1, 1), (255, 1), (2049, 1), (3, 5), (700, 7), (4099, 24), (1000, 100), (33, 257), (9, 5001), (300, 64)])
+@pytest.mark.parametrize("offset", [0, 1, 7])
+def test_counts_byte_by_byte(native_lib, cuda_device, T, L, offset):
+    gen = torch.Generator(device=cuda_device).manual_seed(T * L + offset)
+    flat = torch.rand(T * L + offset, generator=gen, device=cuda_device) < 0.3
+    flat.view(torch.uint8)[::3] *= 255  # any byte but zero counts once
+    rmap = flat[offset:].view(T, L)
+    want = (rmap.view(torch.uint8) != 0).sum(0, dtype=torch.int32)
+    if L % 16 == 0 and offset == 0:
+        pytest.skip("whole vectors")
+    assert torch.equal(G.cuda_histogram(rmap, L, "map"), want)

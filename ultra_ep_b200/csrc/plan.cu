@@ -55,7 +55,28 @@ __device__ __forceinline__ void hist_add_swar(uint32_t word, int32_t* hist, int 
     if (c3) atomicAdd(hist + col + 3, c3);
 }
 
-// Count this CTA's slice of the input into hist[L] (shared memory, zeroed by the caller).
+// Bytes [begin, end) of a map whose rows are not whole vectors, into the counts at the start of the CTA's shared memory; `begin` is a row's
+// first. Eight loads in flight, the column by additions. Out of line: most maps do not come here. (One load and a division at a time: plan of
+// six ranks of 4000 x 120 33.5 us and 14.3, of eight of 8192 x 120 46.8 and 23.0, of three of 5561 x 120 37.1 and 19.5.)
+__device__ __noinline__ void count_bytes(const uint8_t* __restrict__ map, int64_t begin, int64_t end, int L, int tid, int nthreads) {
+    extern __shared__ __align__(128) char smem_raw[];
+    int32_t* const hist = reinterpret_cast<int32_t*>(smem_raw);
+    const int step = nthreads % L;
+    int column = tid % L;
+    for (int64_t i = begin + tid; i < end; i += 8 * nthreads) {
+        uint8_t v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = i + u * nthreads < end ? map[i + u * nthreads] : 0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            if (v[u] != 0) atomicAdd(hist + column, 1);
+            column += step;
+            column -= column >= L ? L : 0;
+        }
+    }
+}
+
+// Count this CTA's slice of the input into hist[L] (the start of its shared memory, zeroed by the caller).
 // part / nparts split the rows (dense) or the entries (sparse) evenly.
 // Inlined, so that a cold kernel does not jump for it first. Counts of 33 tokens of 64 experts behind an L2 flush, out of line and like
 // this: 4.2 us after the start and 2.2, 4096 tokens 5.1 and 3.6; among other plans 1.9 and 1.6, 3.4 and 3.0.
@@ -113,10 +134,7 @@ __device__ __forceinline__ void histogram_slice(int input_kind, const void* inpu
                 hist_add_swar(acc.z, hist, g * 16 + 8); hist_add_swar(acc.w, hist, g * 16 + 12);
             }
         } else {
-            const int64_t begin = static_cast<int64_t>(r0) * L, end = static_cast<int64_t>(r1) * L;
-            for (int64_t i = begin + tid; i < end; i += nthreads) {
-                if (map[i]) atomicAdd(hist + static_cast<int>(i % L), 1);
-            }
+            count_bytes(map, static_cast<int64_t>(r0) * L, static_cast<int64_t>(r1) * L, L, tid, nthreads);
         }
     } else {
         const int64_t n = static_cast<int64_t>(T) * K_or_L;
@@ -612,10 +630,13 @@ void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 // (17 KB) 52.5 and 52.7, 9600 (20 KB) 39.65 and 39.6, 4800 int64 tokens of 64 (20 KB) 27.9 and 28.1; above it 11000 int32 tokens (23 KB) 40.75
 // and 40.3, 2600 bool rows of 256 (43 KB) 53.4 and 51.8, 16384 int64 tokens of 256 (68 KB) 106.8 and 104.5. Legacy plans the same: with the
 // dense reroute 8192 rows of 256 191.4 and 188.5, of 512 180.5 and 175.6; one rank's plan of 8192 x 256 9.5 and 8.1, of 16384 x 64 6.3 and 6.7.
-constexpr int kFewThreadsBytes = 22 * 1024;
+// Maps that are counted byte by byte take longer: 512 threads from 16 KB on (plan of six ranks of 4000 x 120, 20.9 KB, 17.3 and 14.3; of seven of
+// 4000 x 70 15.2 and 13.1).
+constexpr int kFewThreadsBytes = 22 * 1024, kFewThreadsBytesSingle = 16 * 1024;
 int plan_threads(int input_kind, int max_T, int K_or_L, int ctas) {
     const int64_t bytes = static_cast<int64_t>(max_T) * K_or_L * (input_kind == 0 ? 1 : (input_kind == 1 ? 4 : 8));
-    return bytes > static_cast<int64_t>(ctas) * kFewThreadsBytes ? 2 * kPlanThreads : kPlanThreads;
+    const int line = input_kind == 0 && K_or_L % 16 != 0 ? kFewThreadsBytesSingle : kFewThreadsBytes;
+    return bytes > static_cast<int64_t>(ctas) * line ? 2 * kPlanThreads : kPlanThreads;
 }
 
 int plan_ctas_per_rank(int input_kind, int max_T, int K_or_L, int cap) {
