@@ -794,9 +794,13 @@ __global__ void __launch_bounds__(kReduceThreads, 1) grad_reduce_kernel(ReduceCa
 
 cudaError_t launch_grad_reduce(const ReduceCall& call, cudaStream_t stream) {
     const dim3 grid(call.nlocal * call.ctas_per_rank), block(kReduceThreads);
-    // Whether items may be handed out goes by the size of an expert: how many experts have replicas is not known here.
+    // Whether items may be handed out goes by the size of an expert (how many experts have replicas is not known here) and by the CTAs: six
+    // sevenths of the SMs at least. Fewer of them bound the kernel and not the memory, and keep pace with each other, and each
+    // run that is asked for is a wait. Reduce of 28.3 M elements an expert, even shares and handed out (us): two ranks, a replica, on 84 CTAs 92
+    // and 117, four ranks, four replicas, on 80 317 and 400, on 112 269 and 291, on 128 264 and 258, on 144 272 and 247; three ranks of 42 M on 126
+    // 165 and 170.
     const int64_t tiles = (call.fc1_numel + kReduceTileElems - 1) / kReduceTileElems + (call.fc2_numel + kReduceTileElems - 1) / kReduceTileElems;
-    const bool hand_out = call.nlocal == call.N && !call.owners_clear && tiles >= kHandOutTiles;
+    const bool hand_out = call.nlocal == call.N && !call.owners_clear && tiles >= kHandOutTiles && static_cast<int>(grid.x) * 7 >= device_sm_count() * 6;
     void (*const kernel)(ReduceCall) = hand_out ? grad_reduce_kernel<true> : grad_reduce_kernel<false>;
     const size_t smem = static_cast<size_t>(kReduceStages + kMasterStages) * kReduceTileBytes + kReduceZeroBytes;
     cudaError_t e = allow_smem(reinterpret_cast<const void*>(kernel), smem);
